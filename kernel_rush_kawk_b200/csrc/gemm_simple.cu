@@ -1,17 +1,27 @@
 // C[M, N] = A[M, K] * W[N, K]^T with float32 multiply-adds on the CUDA cores.
 //
 // This is the matrix product of the true 32-bit path: no tensor cores, no
-// reduced-precision mode, and every output element is one thread's sum over k
-// in ascending order, so a row's result does not depend on how many other rows
-// the call has. Weights are [out, in] as in the reference (y = x W^T, no bias:
+// reduced-precision mode, and every output element is one chain of fused
+// multiply-adds over k in ascending order, whichever kernel below computes it, so
+// a row's result does not depend on how many other rows the call has. Weights are
+// [out, in] as in the reference (y = x W^T, no bias:
 // engine/model.py:295,299,301 of willzeng274/kernel-rush-kawk).
 //
-// It also serves, with bfloat16 inputs and float32 output, for output-head
-// logits at many positions, where the serving path would otherwise round its
-// logits to bfloat16.
+// Three kernels share that sum:
 //
-// 64x64 output tile, k in slices of 16, 256 threads with a 4x4 micro-tile each.
-#include "common.cuh"
+// * gemm_f32_tile: more than 16 float32 rows. Bound by the multiply-add pipe and, close behind it, by shared-memory reads,
+//   so a thread holds up to 8 x 8 outputs, operands come k-major through two shared-memory buffers, and the next slice
+//   is in registers while this one is multiplied. 1,024 rows of 19,456 x 2,560: 1.99 ms, 51 of the pipe's 72 TFLOP/s
+//   (measured with independent chains); 360 rows of 6,144 x 2,560: 259 us, 44 TFLOP/s (the general kernel: 2.0 ms).
+//   Packed multiply-adds (fma.rn.f32x2) were measured and are slower here (274 to 294 us): the copies that pair an
+//   operand with itself cost more than the pipe's register reads gain.
+// * gemm_f32_few: up to 16 float32 rows. Bound by the weights' bytes: each is read once, by asynchronous 16-byte copies
+//   several slices ahead; a thread owns one or two output columns of one or two rows. One row of 151,936 x 2,560: 252 us,
+//   6.2 TB/s; three rows 361 us, of 2,560 x 4,096 26 us (the general kernel: 1.9 ms and 570 us).
+// * gemm_nt: everything else (bfloat16 inputs with float32 output at odd sizes, for output-head logits at many
+//   positions; float32 rows whose size or alignment does not allow 16-byte accesses). 64x64 output tile, k in slices of
+//   16, 256 threads with a 4x4 micro-tile each.
+#include "mma.cuh"  // cp.async
 
 namespace {
 
@@ -73,11 +83,279 @@ int launch(void* C, const void* A, const void* W, int M, int N, int K, int lda, 
   return 0;
 }
 
+// ---- float32, more than 16 rows --------------------------------------------------------------------------------
+// 128 threads; thread (ty, tx) of 8 x 16 holds MG groups of 4 rows and NG groups of 4 columns, the groups 32 rows (64
+// columns) apart. A warp covers 4 x 8 of the threads' places, neighbouring lanes sharing a column or differing in their
+// row alone: a warp's 16-byte read then takes 2 cycles of the SM's shared memory (measured; 4 where every fourth lane
+// shares). The fragments of the next k are read before this one's are multiplied.
+constexpr int TK = 16;  // k per slice
+
+template <int MG, int NG>
+__global__ void __launch_bounds__(128, MG * NG == 4 ? 3 : 4)
+gemm_f32_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W, int M, int N, int K,
+                     int lda, int ldw, int ldc) {
+  constexpr int TM = 32 * MG, TN = 64 * NG;
+  // Row k of a slice starts 8 floats further for every four k, so that the 32 stores of a warp (8 rows or columns of four
+  // k that are four apart) fall into different banks; rows stay on 16-byte boundaries.
+  constexpr int AP = TM + 28, WP = TN + 28;
+#define KRK_SKEW(k) (8 * (((k) >> 2) & 3))
+  __shared__ __align__(16) float As[2][TK][AP];
+  __shared__ __align__(16) float Ws[2][TK][WP];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tx = (warp >> 1) * 8 + ((lane & 15) >> 1), ty = (warp & 1) * 4 + (lane & 1) + 2 * (lane >> 4);
+  const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
+  const int lk = (tid & 3) * 4, lr = tid >> 2;  // this thread loads k = lk..lk+3 of rows lr, lr + 32, ...
+  float acc[4 * MG][4 * NG];
+#pragma unroll
+  for (int i = 0; i < 4 * MG; ++i)
+#pragma unroll
+    for (int j = 0; j < 4 * NG; ++j) acc[i][j] = 0.f;
+  float4 ar[MG], wr[2 * NG];
+  auto fetch = [&](int k0) {  // zeros beyond the matrices' ends (K is a multiple of 4)
+    const bool in = k0 + lk < K;
+#pragma unroll
+    for (int i = 0; i < MG; ++i) {
+      const int m = m0 + lr + 32 * i;
+      ar[i] = in && m < M ? *reinterpret_cast<const float4*>(A + (size_t)m * lda + k0 + lk) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < 2 * NG; ++i) {
+      const int n = n0 + lr + 32 * i;
+      wr[i] = in && n < N ? *reinterpret_cast<const float4*>(W + (size_t)n * ldw + k0 + lk) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  auto stage = [&](int b) {
+    const int at = lr + KRK_SKEW(lk);
+#pragma unroll
+    for (int i = 0; i < MG; ++i) {
+      As[b][lk][at + 32 * i] = ar[i].x; As[b][lk + 1][at + 32 * i] = ar[i].y;
+      As[b][lk + 2][at + 32 * i] = ar[i].z; As[b][lk + 3][at + 32 * i] = ar[i].w;
+    }
+#pragma unroll
+    for (int i = 0; i < 2 * NG; ++i) {
+      Ws[b][lk][at + 32 * i] = wr[i].x; Ws[b][lk + 1][at + 32 * i] = wr[i].y;
+      Ws[b][lk + 2][at + 32 * i] = wr[i].z; Ws[b][lk + 3][at + 32 * i] = wr[i].w;
+    }
+  };
+  fetch(0);
+  stage(0);
+  __syncthreads();
+  const int slices = (K + TK - 1) / TK;
+  for (int s = 0; s < slices; ++s) {
+    const int b = s & 1;
+    if (s + 1 < slices) fetch((s + 1) * TK);
+    float4 w[2][NG];
+    float4 a[2][MG];
+    auto read = [&](int f, int k) {
+#pragma unroll
+      for (int g = 0; g < NG; ++g) w[f][g] = *reinterpret_cast<const float4*>(&Ws[b][k][64 * g + 4 * tx + KRK_SKEW(k)]);
+#pragma unroll
+      for (int g = 0; g < MG; ++g) a[f][g] = *reinterpret_cast<const float4*>(&As[b][k][32 * g + 4 * ty + KRK_SKEW(k)]);
+    };
+    read(0, 0);
+#pragma unroll
+    for (int k = 0; k < TK; ++k) {
+      if (k + 1 < TK) read((k + 1) & 1, k + 1);
+#pragma unroll
+      for (int g = 0; g < MG; ++g) {
+        const float4 v = a[k & 1][g];
+        const float av[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < NG; ++j) {
+            const float4 u = w[k & 1][j];
+            acc[4 * g + i][4 * j] = fmaf(av[i], u.x, acc[4 * g + i][4 * j]);
+            acc[4 * g + i][4 * j + 1] = fmaf(av[i], u.y, acc[4 * g + i][4 * j + 1]);
+            acc[4 * g + i][4 * j + 2] = fmaf(av[i], u.z, acc[4 * g + i][4 * j + 2]);
+            acc[4 * g + i][4 * j + 3] = fmaf(av[i], u.w, acc[4 * g + i][4 * j + 3]);
+          }
+      }
+    }
+    if (s + 1 < slices) {
+      stage(b ^ 1);  // the slice before, which was there, was multiplied before the last barrier
+      __syncthreads();
+    }
+  }
+#undef KRK_SKEW
+  const bool wide = (ldc & 3) == 0;  // C's rows start on 16-byte boundaries (its base does: the caller checks)
+#pragma unroll
+  for (int g = 0; g < MG; ++g)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int m = m0 + 32 * g + 4 * ty + i;
+      if (m >= M) continue;
+#pragma unroll
+      for (int h = 0; h < NG; ++h) {
+        const int n = n0 + 64 * h + 4 * tx;
+        float* c = C + (size_t)m * ldc + n;
+        const float4 v = make_float4(acc[4 * g + i][4 * h], acc[4 * g + i][4 * h + 1], acc[4 * g + i][4 * h + 2], acc[4 * g + i][4 * h + 3]);
+        if (wide && n + 4 <= N) {
+          *reinterpret_cast<float4*>(c) = v;
+        } else {
+          const float* f = reinterpret_cast<const float*>(&v);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (n + j < N) c[j] = f[j];
+        }
+      }
+    }
+}
+
+// ---- float32, up to 16 rows ------------------------------------------------------------------------------------
+// A block owns 16 * CPT columns (a thread c, c + 16); its 8 groups of 16 threads take RPT rows each. A slice is 128 k of
+// the columns' weights and of the rows; DEPTH slices are on the way, 40 or 80 KB of weights a block, which is what an SM
+// has to have in flight to draw its share of the memory's bandwidth. Beyond 8 rows, where shared-memory reads are the
+// bound, a thread's two rows of two columns read half as much for a multiply-add as one of one.
+constexpr int FEW_K = 128, FEW_PITCH = FEW_K + 4, FEW_DEPTH = 6;
+
+template <int RPT, int CPT>
+__global__ void __launch_bounds__(128)
+gemm_f32_few_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W, int M, int N, int K,
+                    int lda, int ldw, int ldc) {
+  constexpr int COLS = 16 * CPT;
+  extern __shared__ __align__(16) float sm[];
+  const int stage_floats = (COLS + M) * FEW_PITCH;
+  // neighbouring lanes share a column and differ in their rows: a warp's 16-byte reads of W and of x then take 2 cycles
+  // of the SM's shared memory each, 4 where neighbours' columns differ
+  const int tid = threadIdx.x, col = (tid & 31) >> 1, group = 2 * (tid >> 5) + (tid & 1);
+  const int n0 = blockIdx.x * COLS;
+  const int slices = (K + FEW_K - 1) / FEW_K;
+  const uint64_t policy = l2_evict_first_policy();
+  const int ck = (tid & 31) * 4, cr = tid >> 5;  // this thread copies k = ck..ck+3 of rows cr, cr + 4, ...
+  auto request = [&](int s) {
+    const int k = s * FEW_K + ck;
+    if (k < K) {  // what lies beyond K is never read: the loops below end there
+      float* dst = sm + (s % FEW_DEPTH) * stage_floats + ck;
+#pragma unroll
+      for (int r = 0; r < COLS; r += 4)
+        if (n0 + cr + r < N) cp_async_16_stream(dst + (cr + r) * FEW_PITCH, W + (size_t)(n0 + cr + r) * ldw + k, policy);
+      for (int r = cr; r < M; r += 4) cp_async_16(dst + (COLS + r) * FEW_PITCH, A + (size_t)r * lda + k);
+    }
+    cp_async_commit();  // one group a slice, empty beyond the last, so that the count of waits holds
+  };
+  for (int s = 0; s < FEW_DEPTH - 1; ++s) request(s);
+  float acc[RPT][CPT];
+#pragma unroll
+  for (int r = 0; r < RPT; ++r)
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) acc[r][c] = 0.f;
+  const int row0 = group * RPT;
+  const bool live = row0 < M;
+  int xat[RPT];
+#pragma unroll
+  for (int r = 0; r < RPT; ++r) xat[r] = (COLS + min(row0 + r, M - 1)) * FEW_PITCH;
+  for (int s = 0; s < slices; ++s) {
+    cp_async_wait<FEW_DEPTH - 2>();
+    __syncthreads();  // slice s is here for everyone, and the slice before it is no longer read
+    request(s + FEW_DEPTH - 1);
+    if (!live) continue;
+    const float* base = sm + (s % FEW_DEPTH) * stage_floats;
+    const float* w = base + col * FEW_PITCH;
+    constexpr int AHEAD = 4;  // pieces of four k in registers while as many are multiplied
+    const int kn = min(FEW_K, K - s * FEW_K);
+    float4 w4[2][AHEAD][CPT], x4[2][AHEAD][RPT];
+    auto read = [&](int b, int k0) {
+#pragma unroll
+      for (int i = 0; i < AHEAD; ++i) {
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) w4[b][i][c] = *reinterpret_cast<const float4*>(w + 16 * c * FEW_PITCH + k0 + 4 * i);
+#pragma unroll
+        for (int r = 0; r < RPT; ++r) x4[b][i][r] = *reinterpret_cast<const float4*>(base + xat[r] + k0 + 4 * i);
+      }
+    };
+    auto multiply = [&](int b, int i) {
+#pragma unroll
+      for (int r = 0; r < RPT; ++r)
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) acc[r][c] = fmaf(x4[b][i][r].x, w4[b][i][c].x, acc[r][c]);
+#pragma unroll
+      for (int r = 0; r < RPT; ++r)
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) acc[r][c] = fmaf(x4[b][i][r].y, w4[b][i][c].y, acc[r][c]);
+#pragma unroll
+      for (int r = 0; r < RPT; ++r)
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) acc[r][c] = fmaf(x4[b][i][r].z, w4[b][i][c].z, acc[r][c]);
+#pragma unroll
+      for (int r = 0; r < RPT; ++r)
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) acc[r][c] = fmaf(x4[b][i][r].w, w4[b][i][c].w, acc[r][c]);
+    };
+    if (kn == FEW_K) {
+      read(0, 0);
+#pragma unroll
+      for (int p = 0; p < FEW_K / (4 * AHEAD); ++p) {
+        if (p + 1 < FEW_K / (4 * AHEAD)) read((p + 1) & 1, (p + 1) * 4 * AHEAD);
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) multiply(p & 1, i);
+      }
+    } else {
+      for (int k = 0; k < kn; k += 4) {
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) w4[0][0][c] = *reinterpret_cast<const float4*>(w + 16 * c * FEW_PITCH + k);
+#pragma unroll
+        for (int r = 0; r < RPT; ++r) x4[0][0][r] = *reinterpret_cast<const float4*>(base + xat[r] + k);
+        multiply(0, 0);
+      }
+    }
+  }
+  cp_async_wait<0>();
+#pragma unroll
+  for (int r = 0; r < RPT; ++r)
+#pragma unroll
+    for (int c = 0; c < CPT; ++c)
+      if (row0 + r < M && n0 + col + 16 * c < N) C[(size_t)(row0 + r) * ldc + n0 + col + 16 * c] = acc[r][c];
+}
+
+template <int MG, int NG>
+int launch_tile(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
+  dim3 grid((N + 64 * NG - 1) / (64 * NG), (M + 32 * MG - 1) / (32 * MG));
+  if (grid.y > 65535) return -3;
+  gemm_f32_tile_kernel<MG, NG><<<grid, 128, 0, stream>>>(C, A, W, M, N, K, lda, ldw, ldc);
+  KRK_CHECK_LAUNCH();
+  return 0;
+}
+
+template <int RPT, int CPT>
+int launch_few(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
+  const size_t smem = (size_t)FEW_DEPTH * (16 * CPT + M) * FEW_PITCH * sizeof(float);  // 54 to 152 KB
+  cudaFuncSetAttribute(gemm_f32_few_kernel<RPT, CPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  gemm_f32_few_kernel<RPT, CPT><<<(N + 16 * CPT - 1) / (16 * CPT), 128, smem, stream>>>(C, A, W, M, N, K, lda, ldw, ldc);
+  KRK_CHECK_LAUNCH();
+  return 0;
+}
+
+// float32 in and out with 16-byte rows. -2: not of that kind.
+int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
+  if (M == 0 || N == 0) return 0;
+  if (K < 4 || K % 4 || lda % 4 || ldw % 4 || (((uintptr_t)A | (uintptr_t)W | (uintptr_t)C) & 15)) return -2;
+  // Cycles per k on the busiest SM, from the times measured at 17 to 1,024 rows of five matrices: a block alone is bound by
+  // its own latency (the first number), several by what a block takes of the SM.
+  auto cost = [&](int tm, int tn, int alone, int each) {
+    const long long tiles = (long long)((M + tm - 1) / tm) * ((N + tn - 1) / tn);
+    const long long all = (tiles + 147) / 148 * each;
+    return all > alone ? all : alone;
+  };
+  const long long c22 = cost(64, 128, 120, 89), c21 = cost(64, 64, 88, 47), c12 = cost(32, 128, 96, 49);
+  const long long best = min(c22, min(c21, c12));
+  if (M <= 8) return launch_few<1, 1>(C, A, W, M, N, K, lda, ldw, ldc, stream);
+  // 9 to 16 rows: 17 cycles a block (115 us at 16 rows of 19,456 x 2,560 against the tiles' 192; 740 against 641 at 151,936)
+  if (M <= 16 && ((long long)(N + 31) / 32 + 147) / 148 * 17 <= best) return launch_few<2, 2>(C, A, W, M, N, K, lda, ldw, ldc, stream);
+  if (best == c22) return launch_tile<2, 2>(C, A, W, M, N, K, lda, ldw, ldc, stream);
+  if (best == c21) return launch_tile<2, 1>(C, A, W, M, N, K, lda, ldw, ldc, stream);
+  return launch_tile<1, 2>(C, A, W, M, N, K, lda, ldw, ldc, stream);
+}
+
 }  // namespace
 
 // in_dtype / out_dtype: KRK_DTYPE_F32 or KRK_DTYPE_BF16. Supported: f32->f32, bf16->f32, bf16->bf16.
 KRK_API int krk_gemm_nt(void* C, const void* A, const void* W, int M, int N, int K, int lda, int ldw, int ldc,
                         int in_dtype, int out_dtype, cudaStream_t stream) {
+  if (in_dtype == KRK_DTYPE_F32 && out_dtype == KRK_DTYPE_F32) {
+    const int rc = launch_f32((float*)C, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldc, stream);
+    if (rc != -2) return rc;
+  }
   if (in_dtype == KRK_DTYPE_F32 && out_dtype == KRK_DTYPE_F32)
     return launch<float, float>(C, A, W, M, N, K, lda, ldw, ldc, stream);
   if (in_dtype == KRK_DTYPE_BF16 && out_dtype == KRK_DTYPE_F32)

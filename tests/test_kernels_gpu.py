@@ -92,6 +92,26 @@ def test_linear(ops, dtype, mnk):
     close(ops.linear(x, w, out_float32=True), ref.linear(x, w, out_float32=True), dtype, f"linear {mnk}, float32 out")
 
 
+@pytest.mark.parametrize("nk", [(301, 132), (64, 4), (129, 20), (2560, 272)])
+def test_float32_products_sum_in_one_order_whatever_the_rows(ops, nk):
+    """Every 32-bit product, by whichever kernel (few rows, the tiles of more rows, the general one that a row offset of
+    one element leads to), is the same chain of multiply-adds over k: equal to the bit, at the edges of row groups,
+    tiles and slices; and within that chain's rounding (K + 1 half steps of the sum of magnitudes) of 64 bits."""
+    n, k = nk
+    x, w = rand((260, k), torch.float32, 71), rand((n, k), torch.float32, 72)
+    odd = torch.empty((260, k + 1), device="cuda")
+    odd[:, 1:] = x
+    want = ops.linear(odd[:, 1:], w)
+    exact = x.double() @ w.double().T
+    bound = (x.double().abs() @ w.double().abs().T) * (k + 1) * 2.0 ** -24
+    assert ((want.double() - exact).abs() <= bound).all()
+    for m in (1, 2, 7, 8, 9, 15, 16, 17, 32, 33, 64, 65, 260):
+        assert torch.equal(ops.linear(x[:m], w), want[:m]), f"{m} rows"
+    wide = torch.zeros((40, 2 * k), device="cuda")
+    wide[:, :k] = x[:40]
+    assert torch.equal(ops.linear(wide[:, :k], w), want[:40]), "rows of a wider buffer"
+
+
 @pytest.mark.parametrize("mnk", [(1, 2560, 9728), (8, 2560, 4096), (16, 2560, 9728), (13, 1000, 2080), (3, 48, 2048),
                                  (9, 2000, 4128)])
 def test_few_row_products_that_split_k_over_a_cluster(ops, mnk):
