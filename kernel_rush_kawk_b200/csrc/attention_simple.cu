@@ -1,8 +1,12 @@
 // Causal grouped-query attention over the paged cache, one warp per (row, head),
-// one key after the other. This is the kernel of the true 32-bit path; it is
-// slow and its result for a row depends on nothing but that row's own keys, in
+// the keys' sums one after the other. This is the kernel of the true 32-bit path; its
+// result for a row depends on nothing but that row's own keys, in
 // their order, so it is the same however the tokens were cut into steps or
 // batched.
+//
+// A warp is bound by the latency of one key's chain (load, sum over the lanes, exponentials, sum), so the rows of
+// KEYS keys and values are requested together and their scores' sums over the lanes interleave; the running maximum
+// and the sums still take the keys in order.
 //
 // s = (q . k) * scale; a query at position p sees keys max(0, p - window + 1)..p
 // (window 0: all keys 0..p); running max and sum in float32; the probability is
@@ -22,6 +26,7 @@ namespace {
 
 constexpr int D = KRK_HEAD_DIM;
 constexpr int PER_LANE = (D + 31) / 32;
+constexpr int KEYS = PER_LANE <= 4 ? 8 : 4;  // in flight; divides a page, so that they lie in one
 
 template <typename T>
 __global__ void attention_simple_kernel(T* __restrict__ out, const T* __restrict__ q, int q_row_stride, int HQ, int HKV,
@@ -47,30 +52,48 @@ __global__ void attention_simple_kernel(T* __restrict__ out, const T* __restrict
   }
   float m = -INFINITY, l = 0.f;
   int page = -1, page_index = -1;
-  for (int key = first; key <= pos; ++key) {
-    if (key / KRK_PAGE != page_index) {
-      page_index = key / KRK_PAGE;
-      page = page_of(table, width, slot, key);
+  for (int key0 = first - first % KEYS; key0 <= pos; key0 += KEYS) {
+    if (key0 / KRK_PAGE != page_index) {
+      page_index = key0 / KRK_PAGE;
+      page = page_of(table, width, slot, key0);
     }
-    const size_t base = (((size_t)page * HKV + kh) * KRK_PAGE + (key % KRK_PAGE)) * D;
-    float dot = 0.f;
+    const size_t base = (((size_t)page * HKV + kh) * KRK_PAGE + (key0 % KRK_PAGE)) * D;
+    float kv[KEYS][PER_LANE], vv[KEYS][PER_LANE], s[KEYS];
 #pragma unroll
-    for (int i = 0; i < PER_LANE; ++i) {
-      const int d = lane + 32 * i;
-      if (d < D) dot += qv[i] * to_float<T>(k_cache[base + d]);
-    }
-    const float s = warp_sum(dot) * scale;
-    const float m_new = fmaxf(m, s);
-    const float alpha = expf(m - m_new);  // exp(-inf) = 0 on the first key
-    const float p = expf(s - m_new);
-    l = l * alpha + p;
-    const float pr = round_to<T>(p);
+    for (int j = 0; j < KEYS; ++j) {
+      const bool seen = key0 + j >= first && key0 + j <= pos;
 #pragma unroll
-    for (int i = 0; i < PER_LANE; ++i) {
-      const int d = lane + 32 * i;
-      if (d < D) acc[i] = acc[i] * alpha + pr * to_float<T>(v_cache[base + d]);
+      for (int i = 0; i < PER_LANE; ++i) {
+        const int d = lane + 32 * i;
+        const bool in = seen && d < D;
+        kv[j][i] = in ? to_float<T>(k_cache[base + (size_t)j * D + d]) : 0.f;
+        vv[j][i] = in ? to_float<T>(v_cache[base + (size_t)j * D + d]) : 0.f;
+      }
     }
-    m = m_new;
+#pragma unroll
+    for (int j = 0; j < KEYS; ++j) {
+      float dot = 0.f;
+#pragma unroll
+      for (int i = 0; i < PER_LANE; ++i) dot += qv[i] * kv[j][i];
+      s[j] = dot;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int j = 0; j < KEYS; ++j) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
+#pragma unroll
+    for (int j = 0; j < KEYS; ++j) {
+      if (key0 + j < first || key0 + j > pos) continue;
+      const float sj = s[j] * scale;
+      const float m_new = fmaxf(m, sj);
+      const float alpha = expf(m - m_new);  // exp(-inf) = 0 on the first key
+      const float p = expf(sj - m_new);
+      l = l * alpha + p;
+      const float pr = round_to<T>(p);
+#pragma unroll
+      for (int i = 0; i < PER_LANE; ++i) acc[i] = acc[i] * alpha + pr * vv[j][i];
+      m = m_new;
+    }
   }
 #pragma unroll
   for (int i = 0; i < PER_LANE; ++i) {
