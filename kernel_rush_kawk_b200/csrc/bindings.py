@@ -119,6 +119,10 @@ _SCAN_SIGNATURES = {
     "krk_linear_recurrence": [c_int, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, _P, _P, _P, _P,
                               _P, _P, c_int, c_int, _P, _P, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_int,
                               c_int, _P, _P, _P, c_int, _P, _P, c_int, _P],
+    "krk_recurrence_chunk_tokens": [c_int, c_int, c_int, c_float, _P],
+    "krk_recurrence_chunks": [c_int, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, _P, _P, _P, _P, _P, _P,
+                              c_int, c_int, _P, _P, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_int, _P, _P, _P,
+                              c_int, c_int, _P, _P],
     "krk_causal_conv_silu": [_P, _P, c_int, _P, _P, _P, c_int, c_int, c_int, c_int, _P, _P, _P, _P, c_int, _P],
     "krk_ssd_scan": [_P, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int,
                      c_int, _P, _P, _P, c_int, _P, _P, c_int, _P],
@@ -1239,6 +1243,23 @@ class Kernels:
                                           batch.seq_slot.data_ptr(), _code(h.dtype), self._stream(), int(store)), "token shift")
         return out
 
+    RECURRENCE_CHUNK_MIN = 40  # tokens of a step's longest sequence from which a bfloat16 scan of such mixers may run in chunks
+    RECURRENCE_SCRATCH = 256 << 20  # bytes
+
+    def _recurrence_in_chunks(self, kind, heads, batch) -> bool:
+        """Time mixing gains at every size measured from 40 tokens on (one sequence of 40 at 24 heads: 60 -> 55 us a layer's mixer, 16
+        of 64: 130 -> 95, one of 2,048 and more: several times). The delta rule has more work a chunk: where sequences and
+        heads fill the SMs, the scan token by token keeps up (8 heads, 16 sequences of 128: 145 us against 157; of 64: 85
+        against 95), so the two are estimated from their measured parts: 0.57 us a token for each round of blocks, against 0.18 us a
+        chunk and head, 0.5 us a chunk of the longest sequence and 12 us."""
+        longest = batch.max_q_len
+        if longest < self.RECURRENCE_CHUNK_MIN:
+            return False
+        if kind == "wkv":
+            return True
+        items = heads * sum(-(-n // 32) for n in batch.q_lens)
+        return 0.57 * longest * -(-batch.n_seqs * heads // 148) > 12.0 + 0.18 * items + 0.5 * longest / 32
+
     def linear_recurrence(self, kind, r, k, v, gate, lora, w2, w0, heads, dim, norm_w, eps, state, batch, out, out_col,
                           out_scale, rate=None, rate_bias=None, decay_scale=1.0, bonus=None, last_rows=None):
         """The scan of a matrix-state mixer over a step's rows ("wkv" or "delta"); see csrc/recurrent.cu."""
@@ -1252,13 +1273,36 @@ class Kernels:
         if state.dtype != torch.float32 or not state.is_contiguous() or not w2.is_contiguous() or w2.dtype != r.dtype:
             raise KernelError("the recurrence keeps a contiguous float32 state and reads W2 in the path's dtype")
         rows = r.shape[0]
+        rule = {"wkv": 0, "delta": 1}[kind]
+        if (r.dtype == torch.bfloat16 and not batch.is_decode and not self.split_recurrence
+                and self._recurrence_in_chunks(kind, heads, batch)):
+            item = c_int(0)
+            tokens = self.scan.krk_recurrence_chunk_tokens(rule, dim, lora.shape[1], float(decay_scale), ctypes.byref(item))
+            chunks = -(-batch.max_q_len // tokens) if tokens else 0
+            # a long step goes through its chunks in portions, so that the scratch stays within RECURRENCE_SCRATCH
+            portion = max(1, min(chunks, self.RECURRENCE_SCRATCH // (4 * item.value * batch.n_seqs * heads)))
+            scratch = torch.empty(portion * batch.n_seqs * heads * item.value if tokens else 0, dtype=torch.float32, device=r.device)
+            rc = 0 if tokens else -2
+            for first in range(0, chunks, portion):
+                rc = self.scan.krk_recurrence_chunks(
+                    rule, *views[0], *views[1], *views[2], *views[3], *rate_v, *lora_v, w2.data_ptr(), w0.data_ptr(),
+                    _ptr(rate_bias), _ptr(bonus), norm_w.data_ptr(), state.data_ptr(), last_ptr, last_stride, C,
+                    _ptr(last_state), optr, ostride, out_col, float(out_scale), float(eps), float(decay_scale), heads,
+                    lora.shape[1], batch.n_seqs, batch.cu_q.data_ptr(), batch.seq_qlen.data_ptr(), batch.seq_slot.data_ptr(),
+                    first, min(portion, chunks - first), scratch.data_ptr(), self._stream())
+                if rc == -2:  # odd strides or offsets: the first portion already says so, and nothing was done
+                    break
+                self._ok(rc, f"{kind} recurrence in chunks")
+                self.launches += 2
+            if rc == 0:
+                return
         prep = o_raw = None
         if not batch.is_decode and dim % 4 == 0 and self.split_recurrence:
             # steps of many tokens: decays and gates over all rows at once, the scan between them (float32 scratch)
             prep = torch.empty(rows * heads * 6 * dim, dtype=torch.float32, device=r.device)
             o_raw = torch.empty(rows * heads * dim, dtype=torch.float32, device=r.device)
         rc = self.scan.krk_linear_recurrence(
-            {"wkv": 0, "delta": 1}[kind], views[0][0], views[0][1], views[1][0], views[1][1], views[2][0], views[2][1],
+            rule, views[0][0], views[0][1], views[1][0], views[1][1], views[2][0], views[2][1],
             views[3][0], views[3][1], rate_v[0], rate_v[1], lora_v[0], lora_v[1], w2.data_ptr(), w0.data_ptr(),
             _ptr(rate_bias), _ptr(bonus), norm_w.data_ptr(), state.data_ptr(), last_ptr, last_stride, C,
             _ptr(last_state), optr, ostride, out_col, float(out_scale), float(eps), float(decay_scale), heads, dim,

@@ -1,0 +1,718 @@
+// The recurrences of recurrent.cu over a step's many tokens in chunks of 32, for bfloat16 rows and heads of 64 channels.
+//
+// The scan of recurrent.cu takes a sequence's tokens one after the other: 0.57 us a token (delta rule) or 0.40 (time
+// mixing) whatever the batch, on as many SMs as there are heads and sequences. Here a chunk's tokens become small matrix
+// products, and all chunks but for one walk run side by side. Everything is float32 on the CUDA cores, as it is there; only
+// the order of the sums differs. With the state S before the chunk, c_t the log decays summed from the chunk's first
+// token to t, and rows of the chunk's tokens:
+//
+//   time mixing:  o_t = (r_t e^{c_{t-1}}) . S + sum_{s<t} [sum_n r_tn k_sn e^{c_{t-1,n} - c_{s,n}}] v_s + (r_t . bonus k_t) v_t
+//                 S' = e^{c_last} S + sum_s (k_s e^{c_last - c_s}) v_s^T
+//
+//   delta rule, u the unit keys, a the removal rates, y_t = u_t . S_{t-1} (what token t removes along its key):
+//     y_t = (u_t e^{c_{t-1}}) . S + sum_{s<t} (B_ts v_s - D_ts y_s),  B_ts = (u_t e^{c_{t-1}}) . (k_s e^{-c_s}), D with a_s u_s for k_s
+//     o_t = (r_t e^{c_t}) . S + sum_{s<=t} (P_ts v_s - R_ts y_s),      P, R likewise from r_t e^{c_t}
+//     S'  = e^{c_last} (S + sum_s (k_s e^{-c_s}) v_s^T - (a_s u_s e^{-c_s}) y_s^T)
+//   y is linear in S: Y = X S + Z with (I + D) X = U and (I + D) Z = B V, U the rows u_t e^{c_{t-1}}. So
+//     O = Q S + O_own with Q = Rows - R X, O_own = P V - R Z;   S' = M S + G with M = e^{c_last} (I - A^T X),
+//     G = e^{c_last} (K^T V - A^T Z).
+//
+// Three passes: (1) per (sequence, chunk, head) M, G, Q and O_own (time mixing: G and the summed decays alone); (2) the walk over
+// a sequence's chunks, S' = M S + G, split over the value columns, which are independent of one another; it leaves each chunk
+// its starting state in G's place and the sequence its final one; (3) per (sequence, chunk, head) the outputs with their norm,
+// weight and gate. Chunks of 32: a chunk of 64 needs twice the multiply-adds a token in pass 1 and halves the walk's steps.
+//
+// Measured: one prompt of 2,048 tokens, delta rule of 8 heads, 1,171 -> 107 us (the passes 62, 34 and 11); three prompts of
+// 2,553 tokens in all, time mixing of 40 heads, 405 -> 180 us (59, 13, 109). Passes 1 and 3 are bound by instruction issue
+// and shared-memory latency (a 0.4 to 0.5 share of the issue slots, 12 to 16 warps an SM), the walk by the chain of its steps.
+//
+// e^{-c_s} must stay in range. The delta rule's decay is at least e^{-decay_scale} a token, so a chunk's is bounded by the
+// parameter (the caller asks krk_recurrence_chunk_tokens). Time mixing's has no bound: a chunk in which some channel decays by
+// more than e^-80 forms its pair sums from e^{c_{t-1} - c_s} one by one, right for any decay and slower.
+#include "mma.cuh"  // cp.async
+
+namespace {
+
+constexpr int L = 32;         // tokens per chunk
+constexpr int N = 64;         // channels of a head
+constexpr int PITCH = N + 4;  // rows on 16-byte boundaries; eight neighbouring rows' pieces fall into different banks
+constexpr int THREADS = 128;
+constexpr float SAFE = 80.f;
+constexpr float FORGOTTEN = 120.f;
+constexpr int WALK_COLS = 4;    // value columns a block of pass 2 walks with
+constexpr int WALK_STAGES = 6;  // chunks whose M are on the way, and the one at hand
+
+struct ChunkArgs {
+  const bf16 *r, *k, *v, *g, *rate, *lora;
+  int r_stride, k_stride, v_stride, g_stride, rate_stride, lora_stride;
+  const bf16* w2;
+  const float *w0, *rate_bias, *bonus, *norm_w;
+  float* state;  // [slots, H, N, N]
+  const bf16* last_rows;
+  int last_stride, C;
+  float* last_state;
+  bf16* out;
+  int out_stride, out_col;
+  float out_scale, eps, decay_scale;
+  int H, R;
+  const int *cu_q, *seq_qlen, *seq_slot;
+  int chunk0, n_chunks;  // the chunks of every sequence that this launch takes
+  float* scratch;        // per (sequence, chunk, head): delta M, G, Q, O_own; time mixing G, summed decays
+};
+constexpr int ITEM_DELTA = 2 * N * N + 2 * L * N, ITEM_MIX = N * N + L * N;
+
+__device__ __forceinline__ float sigmoid_f(float z) { return 1.0f / (1.0f + expf(-z)); }
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ float4 widen4(const bf16* p) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&raw.x), b = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
+  return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
+}
+__device__ __forceinline__ void fma4(float4& d, float a, float4 b) {
+  d.x = fmaf(a, b.x, d.x); d.y = fmaf(a, b.y, d.y); d.z = fmaf(a, b.z, d.z); d.w = fmaf(a, b.w, d.w);
+}
+__device__ __forceinline__ float dot4(float4 a, float4 b, float d) {
+  return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, d))));
+}
+
+// The chunk's log decays, summed over its tokens, into cs [L][PITCH] (zero decay beyond the last token). A thread takes
+// one channel of half the tokens; `total` is [2][N]. With `rest` (delta rule) what the running sums round off goes
+// there: a sum of 18 rounds at 1e-6, which e^c would multiply everything by. Ends with a barrier.
+template <int RULE>
+__device__ __forceinline__ void summed_decays(const ChunkArgs& a, float* cs, float* rest, float* total, const float* th_s, int ch0, int nt) {
+  constexpr int HALF = L / 2;
+  const int ch = threadIdx.x & (N - 1), half = threadIdx.x / N, t0 = half * HALF, RP = (a.R + 7) & ~7;
+  const bf16* w2 = a.w2 + (size_t)(ch0 + ch) * a.R;
+  float z[HALF];
+#pragma unroll
+  for (int t = 0; t < HALF; ++t) z[t] = 0.f;
+  for (int m = 0; m < RP; m += 8) {
+    float w[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[i] = m + i < a.R ? __bfloat162float(w2[m + i]) : 0.f;
+#pragma unroll
+    for (int t = 0; t < HALF; ++t) {
+      const float4 x = ld4(th_s + (t0 + t) * RP + m), y = ld4(th_s + (t0 + t) * RP + m + 4);
+      z[t] = fmaf(x.w, w[3], fmaf(x.z, w[2], fmaf(x.y, w[1], fmaf(x.x, w[0], z[t]))));
+      z[t] = fmaf(y.w, w[7], fmaf(y.z, w[6], fmaf(y.y, w[5], fmaf(y.x, w[4], z[t]))));
+    }
+  }
+  const float w0 = a.w0[ch0 + ch];
+  float run = 0.f, lost = 0.f, low[HALF];
+#pragma unroll
+  for (int t = 0; t < HALF; ++t) {
+    float x = RULE == 1 ? -a.decay_scale * sigmoid_f(z[t] + w0) : -expf(z[t] + w0);
+    if (x < -FORGOTTEN) x = -FORGOTTEN;  // a decay that is zero in 32 bits either way; -infinity would not add up
+    if (t0 + t >= nt) x = 0.f;
+    const float sum = run + x;
+    if (RULE == 1) {
+      const float y = sum - run;
+      lost += (run - (sum - y)) + (x - y);
+      low[t] = lost;
+    }
+    z[t] = run = sum;
+  }
+  if (half == 0) {
+    total[ch] = run;
+    total[N + ch] = lost;
+  }
+  __syncthreads();
+  const float before = half ? total[ch] : 0.f, before_low = half && RULE == 1 ? total[N + ch] : 0.f;
+#pragma unroll
+  for (int t = 0; t < HALF; ++t) {
+    const float sum = before + z[t];
+    cs[(t0 + t) * PITCH + ch] = sum;
+    if (RULE == 1) {
+      const float y = sum - before;
+      rest[(t0 + t) * PITCH + ch] = low[t] + before_low + ((before - (sum - y)) + (z[t] - y));
+    }
+  }
+  __syncthreads();
+}
+
+// tanh of the low-rank input in the path's precision, [L][R rounded up to 8], zeros beyond the tokens and R
+__device__ __forceinline__ void load_tanh(const ChunkArgs& a, float* th_s, size_t row0, int nt) {
+  const int RP = (a.R + 7) & ~7;
+  for (int t = threadIdx.x >> 3; t < L; t += THREADS / 8)
+    for (int m = threadIdx.x & 7; m < RP; m += 8)
+      th_s[t * RP + m] = t < nt && m < a.R ? round_to<bf16>(tanhf(__bfloat162float(a.lora[(row0 + t) * a.lora_stride + m]))) : 0.f;
+}
+__device__ __forceinline__ void load_rows(float* dst, const bf16* src, int stride, size_t row0, int ch0, int nt) {
+#pragma unroll
+  for (int i = threadIdx.x; i < L * (N / 4); i += THREADS) {
+    const int t = i / (N / 4), c = (i % (N / 4)) * 4;
+    st4(dst + t * PITCH + c, t < nt ? widen4(src + (row0 + t) * stride + ch0 + c) : make_float4(0.f, 0.f, 0.f, 0.f));
+  }
+}
+
+// A warp's place in a product of 64 columns: 16 columns a warp, lanes 8 x 4, neighbouring lanes sharing a row or a column
+// (a warp's 16-byte read of shared memory then takes 2 cycles, not 4).
+struct Place {
+  int ty, col;
+  __device__ Place() {
+    const int lane = threadIdx.x & 31;
+    ty = (lane & 15) >> 1;
+    col = (threadIdx.x >> 5) * 16 + 4 * ((lane & 1) + 2 * (lane >> 4));
+  }
+};
+
+// ---- pass 1, delta rule ----------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(THREADS, 3) delta_chunk_kernel(ChunkArgs a) {
+  extern __shared__ __align__(16) float sm[];
+  float* us = sm;                  // [L][PITCH] u_t e^{c_{t-1}}; then X
+  float* rs = us + L * PITCH;      // [L][PITCH] r_t e^{c_t} (behind us: one matrix of 2 L rows)
+  float* ks = rs + L * PITCH;      // [L][PITCH] k_s e^{-c_s}
+  float* as = ks + L * PITCH;      // [L][PITCH] a_s u_s e^{-c_s} (behind ks)
+  float* vs = as + L * PITCH;      // [L][PITCH]
+  float* zs = vs + L * PITCH;      // [L][PITCH] c, then Z
+  float* es = zs + L * PITCH;      // [2 L][PITCH] products of us, rs with ks, as: B, D above P, R; before, the rest of c
+  float* last = es + 2 * L * PITCH;  // [N] e^{c_last}
+  float* inv = last + N;           // [L] 1 / |k|
+  float* th_s = us;                // [L][R rounded up]; gone before us is written
+  const int h = blockIdx.x, ci = blockIdx.y, seq = blockIdx.z, ch0 = h * N;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  grid_dependency_wait();
+  const int first = (a.chunk0 + ci) * L, nt = min(L, a.seq_qlen[seq] - first);
+  if (nt <= 0) return;
+  const size_t row0 = (size_t)a.cu_q[seq] + first;
+  load_rows(rs, a.r, a.r_stride, row0, ch0, nt);
+  load_rows(ks, a.k, a.k_stride, row0, ch0, nt);
+  load_rows(vs, a.v, a.v_stride, row0, ch0, nt);
+  load_rows(as, a.rate, a.rate_stride, row0, ch0, nt);
+  load_tanh(a, th_s, row0, nt);
+  __syncthreads();
+  for (int t = warp; t < L; t += THREADS / 32) {
+    const float x = ks[t * PITCH + lane], y = ks[t * PITCH + lane + 32];
+    const float sq = warp_sum(x * x + y * y);
+    if (lane == 0) inv[t] = rsqrtf(sq + 1e-6f);
+  }
+  summed_decays<1>(a, zs, es, es + L * PITCH, th_s, ch0, nt);
+  {
+    const int ch = tid & 63;
+    const float bias = a.rate_bias[ch0 + ch];
+#pragma unroll 4
+    for (int t = tid >> 6; t < L; t += 2) {
+      const int at = t * PITCH + ch;
+      const float c = zs[at], c1 = es[at];
+      const float k = ks[at], u = k * inv[t], back = expf(-c) * (1.f - c1);
+      const float before = t ? zs[at - PITCH] : 0.f, before1 = t ? es[at - PITCH] : 0.f;
+      us[at] = u * (expf(before) * (1.f + before1));
+      rs[at] *= expf(c) * (1.f + c1);
+      as[at] = sigmoid_f(as[at] + bias) * u * back;
+      ks[at] = k * back;
+      if (t == L - 1) last[ch] = expf(c) * (1.f + c1);
+    }
+  }
+  __syncthreads();
+  {  // [us; rs] [ks; as]^T, 4 rows (16 apart) x 8 columns (8 apart) a thread; what looks ahead is zeroed
+    const int ty = (warp & 1) * 8 + ((lane & 15) >> 1), tx = (warp >> 1) * 4 + (lane & 1) + 2 * (lane >> 4);
+    float e[4][8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) e[i][j] = 0.f;
+#pragma unroll 2
+    for (int n = 0; n < N; n += 4) {
+      float4 x[4], y[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = ld4(us + (ty + 16 * i) * PITCH + n);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) y[j] = ld4(ks + (tx + 8 * j) * PITCH + n);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) e[i][j] = dot4(x[i], y[j], e[i][j]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int row = ty + 16 * i, col = tx + 8 * j, t = row & (L - 1), s = col & (L - 1);
+        es[row * PITCH + col] = s < t || (s == t && row >= L) ? e[i][j] : 0.f;
+      }
+  }
+  __syncthreads();
+  {  // forward substitution, a column of [X | Z] a thread; four partial sums a row
+    float x[L];
+    if (warp < 2) {
+#pragma unroll
+      for (int t = 0; t < L; ++t) {
+        float p[4] = {us[t * PITCH + tid], 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int s = 0; s < t; s += 4) {
+          const float4 d = ld4(es + t * PITCH + L + s);
+          p[0] = fmaf(-d.x, x[s], p[0]);
+          if (s + 1 < t) p[1] = fmaf(-d.y, x[s + 1], p[1]);
+          if (s + 2 < t) p[2] = fmaf(-d.z, x[s + 2], p[2]);
+          if (s + 3 < t) p[3] = fmaf(-d.w, x[s + 3], p[3]);
+        }
+        x[t] = (p[0] + p[1]) + (p[2] + p[3]);
+      }
+#pragma unroll
+      for (int t = 0; t < L; ++t) us[t * PITCH + tid] = x[t];
+    } else {
+      const int p0 = tid - N;
+      float v[L];
+#pragma unroll
+      for (int t = 0; t < L; ++t) v[t] = vs[t * PITCH + p0];
+#pragma unroll
+      for (int t = 0; t < L; ++t) {
+        float p[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int s = 0; s < t; s += 4) {
+          const float4 b = ld4(es + t * PITCH + s), d = ld4(es + t * PITCH + L + s);
+          p[0] = fmaf(-d.x, x[s], fmaf(b.x, v[s], p[0]));
+          if (s + 1 < t) p[1] = fmaf(-d.y, x[s + 1], fmaf(b.y, v[s + 1], p[1]));
+          if (s + 2 < t) p[2] = fmaf(-d.z, x[s + 2], fmaf(b.z, v[s + 2], p[2]));
+          if (s + 3 < t) p[3] = fmaf(-d.w, x[s + 3], fmaf(b.w, v[s + 3], p[3]));
+        }
+        x[t] = (p[0] + p[1]) + (p[2] + p[3]);
+      }
+#pragma unroll
+      for (int t = 0; t < L; ++t) zs[t * PITCH + p0] = x[t];
+    }
+  }
+  __syncthreads();
+  // only now: a block of the walk that waited from the start would hold the shared memory that this kernel's blocks need
+  grid_launch_dependents();
+  float* item = a.scratch + (((size_t)seq * a.n_chunks + ci) * a.H + h) * ITEM_DELTA;
+  const Place at;
+  {  // Q and O_own: rows ty, ty + 8, ... of the chunk
+    float4 q[4], o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      q[i] = ld4(rs + (at.ty + 8 * i) * PITCH + at.col);
+      o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll 2
+    for (int s = 0; s < L; s += 4) {
+      float p[4][4], r[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        st4(p[i], ld4(es + (L + at.ty + 8 * i) * PITCH + s));
+        st4(r[i], ld4(es + (L + at.ty + 8 * i) * PITCH + L + s));
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float4 x = ld4(us + (s + j) * PITCH + at.col), v = ld4(vs + (s + j) * PITCH + at.col), z = ld4(zs + (s + j) * PITCH + at.col);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (s + j <= at.ty + 8 * i) {  // a later token's infinities stay its own
+            fma4(q[i], -r[i][j], x);
+            fma4(o[i], p[i][j], v);
+            fma4(o[i], -r[i][j], z);
+          }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      st4(item + 2 * N * N + (at.ty + 8 * i) * N + at.col, q[i]);
+      st4(item + 2 * N * N + L * N + (at.ty + 8 * i) * N + at.col, o[i]);
+    }
+  }
+  {  // M and G: key channels 4 ty .. and 32 + 4 ty ..
+    float4 m[8], g[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m[i] = g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+    for (int s = 0; s < L; ++s) {
+      float ar[8], kr[8];
+      st4(ar, ld4(as + s * PITCH + 4 * at.ty));
+      st4(ar + 4, ld4(as + s * PITCH + 32 + 4 * at.ty));
+      st4(kr, ld4(ks + s * PITCH + 4 * at.ty));
+      st4(kr + 4, ld4(ks + s * PITCH + 32 + 4 * at.ty));
+      const float4 x = ld4(us + s * PITCH + at.col), v = ld4(vs + s * PITCH + at.col), z = ld4(zs + s * PITCH + at.col);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        fma4(m[i], -ar[i], x);
+        fma4(g[i], kr[i], v);
+        fma4(g[i], -ar[i], z);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int n = 32 * (i >> 2) + 4 * at.ty + (i & 3);
+      const float w = last[n];
+      m[i].x += n == at.col ? 1.f : 0.f; m[i].y += n == at.col + 1 ? 1.f : 0.f;
+      m[i].z += n == at.col + 2 ? 1.f : 0.f; m[i].w += n == at.col + 3 ? 1.f : 0.f;
+      st4(item + n * N + at.col, make_float4(w * m[i].x, w * m[i].y, w * m[i].z, w * m[i].w));
+      st4(item + N * N + n * N + at.col, make_float4(w * g[i].x, w * g[i].y, w * g[i].z, w * g[i].w));
+    }
+  }
+}
+
+// ---- pass 1, time mixing ---------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(THREADS) mix_chunk_kernel(ChunkArgs a) {
+  extern __shared__ __align__(16) float sm[];
+  float* ks = sm;                // [L][PITCH] k_s e^{c_last - c_s}
+  float* vs = ks + L * PITCH;    // [L][PITCH]
+  float* cs = vs + L * PITCH;    // [L][PITCH]
+  float* th_s = cs + L * PITCH;  // [L][R rounded up]
+  float* total = th_s + L * ((a.R + 7) & ~7);  // [2][N]
+  const int h = blockIdx.x, ci = blockIdx.y, seq = blockIdx.z, ch0 = h * N;
+  grid_dependency_wait();
+  const int first = (a.chunk0 + ci) * L, nt = min(L, a.seq_qlen[seq] - first);
+  if (nt <= 0) return;
+  const size_t row0 = (size_t)a.cu_q[seq] + first;
+  load_rows(ks, a.k, a.k_stride, row0, ch0, nt);
+  load_rows(vs, a.v, a.v_stride, row0, ch0, nt);
+  load_tanh(a, th_s, row0, nt);
+  __syncthreads();
+  summed_decays<0>(a, cs, nullptr, total, th_s, ch0, nt);
+  grid_launch_dependents();
+  float* item = a.scratch + (((size_t)seq * a.n_chunks + ci) * a.H + h) * ITEM_MIX;
+  for (int i = threadIdx.x; i < L * (N / 4); i += THREADS) {
+    const int t = i / (N / 4), n = (i % (N / 4)) * 4;
+    const float4 c = ld4(cs + t * PITCH + n), e = ld4(cs + (L - 1) * PITCH + n);
+    st4(item + N * N + t * N + n, c);
+    float4 k = ld4(ks + t * PITCH + n);
+    k.x *= expf(e.x - c.x); k.y *= expf(e.y - c.y); k.z *= expf(e.z - c.z); k.w *= expf(e.w - c.w);
+    st4(ks + t * PITCH + n, k);
+  }
+  __syncthreads();
+  const Place at;
+  float4 g[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int s = 0; s < L; ++s) {
+    float kr[8];
+    st4(kr, ld4(ks + s * PITCH + 4 * at.ty));
+    st4(kr + 4, ld4(ks + s * PITCH + 32 + 4 * at.ty));
+    const float4 v = ld4(vs + s * PITCH + at.col);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) fma4(g[i], kr[i], v);
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) st4(item + (32 * (i >> 2) + 4 * at.ty + (i & 3)) * N + at.col, g[i]);
+}
+
+// ---- pass 2 ----------------------------------------------------------------------------------------------------
+// Delta rule: a block walks WALK_COLS value columns of one (sequence, head). A lane holds the sums of two key channels over
+// its warp's quarter of M's columns; the warps' shares meet in shared memory. M comes by asynchronous copies, five chunks ahead.
+__global__ void __launch_bounds__(THREADS) delta_walk_kernel(ChunkArgs a) {
+  extern __shared__ __align__(16) float sm[];
+  float* ms = sm;                                          // [WALK_STAGES][N][PITCH]
+  float* gs = ms + WALK_STAGES * N * PITCH;                // [WALK_STAGES][N][4]
+  float* ss = gs + WALK_STAGES * N * WALK_COLS;            // [N][4] the state's columns
+  float* part = ss + N * WALK_COLS;                        // [4][N][4]
+  grid_dependency_wait();
+  const int p0 = blockIdx.x * WALK_COLS, h = blockIdx.y, seq = blockIdx.z;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n_chunks = min(a.n_chunks, (a.seq_qlen[seq] + L - 1) / L - a.chunk0);
+  if (n_chunks <= 0) return;
+  float* items = a.scratch + ((size_t)seq * a.n_chunks * a.H + h) * ITEM_DELTA;
+  const size_t step = (size_t)a.H * ITEM_DELTA;
+  float* st = a.state + ((size_t)a.seq_slot[seq] * a.H + h) * N * N + p0;
+  auto request = [&](int c) {
+    if (c < n_chunks) {
+      const float* m = items + c * step;
+      const int b = c % WALK_STAGES;
+#pragma unroll
+      for (int i = 0; i < N * N / 4 / THREADS; ++i) {
+        const int e = i * THREADS + tid, n = e / (N / 4), j = (e % (N / 4)) * 4;
+        cp_async_16(ms + (b * N + n) * PITCH + j, m + n * N + j);
+      }
+      if (tid < N) cp_async_16(gs + (b * N + tid) * WALK_COLS, m + N * N + tid * N + p0);
+    }
+    cp_async_commit();
+  };
+  for (int c = 0; c < WALK_STAGES - 1; ++c) request(c);
+  if (tid < N) st4(ss + tid * WALK_COLS, ld4(st + (size_t)tid * N));
+  for (int c = 0; c < n_chunks; ++c) {
+    cp_async_wait<WALK_STAGES - 2>();
+    __syncthreads();  // chunk c's M and G and the state are here; the buffers of the chunk before are no longer read
+    request(c + WALK_STAGES - 1);
+    const int b = c % WALK_STAGES;
+    float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+#pragma unroll
+    for (int j = 0; j < N / 4; j += 4) {
+      const int k = warp * (N / 4) + j;
+      float x[4], y[4];
+      st4(x, ld4(ms + (b * N + lane) * PITCH + k));
+      st4(y, ld4(ms + (b * N + 32 + lane) * PITCH + k));
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 s = ld4(ss + (k + i) * WALK_COLS);
+        fma4(lo, x[i], s);
+        fma4(hi, y[i], s);
+      }
+    }
+    st4(part + (warp * N + lane) * 4, lo);
+    st4(part + (warp * N + 32 + lane) * 4, hi);
+    __syncthreads();
+    if (tid < N) {
+      const float4 p = ld4(part + tid * 4), q = ld4(part + (N + tid) * 4), r = ld4(part + (2 * N + tid) * 4), s = ld4(part + (3 * N + tid) * 4);
+      const float4 g = ld4(gs + (b * N + tid) * WALK_COLS);
+      st4(items + c * step + N * N + tid * N + p0, ld4(ss + tid * WALK_COLS));  // the chunk's starting state, in G's place
+      st4(ss + tid * WALK_COLS, make_float4(g.x + ((p.x + q.x) + (r.x + s.x)), g.y + ((p.y + q.y) + (r.y + s.y)),
+                                            g.z + ((p.z + q.z) + (r.z + s.z)), g.w + ((p.w + q.w) + (r.w + s.w))));
+    }
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  grid_launch_dependents();
+  if (tid < N) st4(st + (size_t)tid * N, ld4(ss + tid * WALK_COLS));
+}
+
+// Time mixing: every element of the state by itself, four neighbours a thread.
+__global__ void mix_walk_kernel(ChunkArgs a) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int h = blockIdx.y, seq = blockIdx.z;
+  const int n_chunks = min(a.n_chunks, (a.seq_qlen[seq] + L - 1) / L - a.chunk0);
+  if (n_chunks <= 0) return;
+  const int e = 4 * (blockIdx.x * blockDim.x + threadIdx.x), n = e / N;
+  float* st = a.state + ((size_t)a.seq_slot[seq] * a.H + h) * N * N + e;
+  float* items = a.scratch + ((size_t)seq * a.n_chunks * a.H + h) * ITEM_MIX;
+  const size_t step = (size_t)a.H * ITEM_MIX;
+  float4 run = ld4(st);
+  for (int c0 = 0; c0 < n_chunks; c0 += 8) {
+    float4 own[8];
+    float decay[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (c0 + i < n_chunks) {
+        own[i] = __ldcg(reinterpret_cast<const float4*>(items + (c0 + i) * step + e));
+        decay[i] = __ldcg(items + (c0 + i) * step + N * N + (L - 1) * N + n);
+      }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (c0 + i < n_chunks) {
+        st4(items + (c0 + i) * step + e, run);
+        const float w = expf(decay[i]);
+        run = make_float4(fmaf(w, run.x, own[i].x), fmaf(w, run.y, own[i].y), fmaf(w, run.z, own[i].z), fmaf(w, run.w, own[i].w));
+      }
+  }
+  st4(st, run);
+}
+
+// ---- pass 3 ----------------------------------------------------------------------------------------------------
+template <int RULE>
+__global__ void __launch_bounds__(THREADS) chunk_finish_kernel(ChunkArgs a) {
+  extern __shared__ __align__(16) float sm[];
+  float* qs = sm;                 // [L][PITCH] rows that meet the state
+  float* red = qs + L * PITCH;    // [4][L] sums of squares of a warp's columns
+  float* ks = red + 4 * L;        // time mixing: [L][PITCH] k_s e^{-c_s}
+  float* vs = ks + L * PITCH;     // [L][PITCH]
+  float* cs = vs + L * PITCH;     // [L][PITCH], where a channel forgets too much
+  float* ps = cs + L * PITCH;     // [L][L + 4] pair sums
+  constexpr int PP = L + 4;
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int h = blockIdx.x, ci = blockIdx.y, seq = blockIdx.z, ch0 = h * N;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int first = (a.chunk0 + ci) * L, qlen = a.seq_qlen[seq], nt = min(L, qlen - first);
+  if (nt <= 0) return;
+  const size_t row0 = (size_t)a.cu_q[seq] + first;
+  const size_t index = ((size_t)seq * a.n_chunks + ci) * a.H + h;
+  const float* item = a.scratch + index * (RULE == 1 ? ITEM_DELTA : ITEM_MIX);
+  const Place at;
+  // the state before the chunk: a value column is one warp's alone, so it is read from memory where it is used
+  const float* start = item + (RULE == 1 ? N * N : 0) + at.col;
+  auto state4 = [&](int n) { return __ldcg(reinterpret_cast<const float4*>(start + n * N)); };
+  float4 o[4], s0[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) s0[j] = state4(j);
+  if (RULE == 1) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[i] = __ldcg(reinterpret_cast<const float4*>(item + 2 * N * N + L * N + (at.ty + 8 * i) * N + at.col));
+    for (int i = tid; i < L * (N / 4); i += THREADS)
+      cp_async_16(qs + (i / (N / 4)) * PITCH + (i % (N / 4)) * 4, item + 2 * N * N + 4 * i);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float* cum = item + N * N;
+    const int n = (tid % (N / 4)) * 4;  // this thread's four channels of tokens tid / 16, 8 further on, ...
+    constexpr int EACH = L * (N / 4) / THREADS;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 end = __ldcg(reinterpret_cast<const float4*>(cum + (L - 1) * N + n)), by = ld4(a.bonus + ch0 + n);
+    float4 q[EACH], k[EACH], c[EACH], b[EACH];
+    load_rows(vs, a.v, a.v_stride, row0, ch0, nt);
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) {
+      const int t = tid / (N / 4) + i * (THREADS / (N / 4));
+      q[i] = t < nt ? widen4(a.r + (row0 + t) * a.r_stride + ch0 + n) : zero;
+      k[i] = t < nt ? widen4(a.k + (row0 + t) * a.k_stride + ch0 + n) : zero;
+      c[i] = __ldcg(reinterpret_cast<const float4*>(cum + t * N + n));
+      b[i] = t ? __ldcg(reinterpret_cast<const float4*>(cum + (t - 1) * N + n)) : zero;
+    }
+    const bool safe = !__syncthreads_or(!(end.x > -SAFE) || !(end.y > -SAFE) || !(end.z > -SAFE) || !(end.w > -SAFE));
+    if (!safe) {  // pair by pair: a token against every fourth one before it
+#pragma unroll
+      for (int i = 0; i < EACH; ++i) {
+        const int at4 = (tid / (N / 4) + i * (THREADS / (N / 4))) * PITCH + n;
+        st4(qs + at4, q[i]);
+        st4(ks + at4, k[i]);
+        st4(cs + at4, c[i]);
+      }
+      __syncthreads();
+      const int t = tid >> 2, piece = tid & 3;
+      for (int s = piece; s < L; s += 4) {
+        float d = 0.f;
+        if (s < t)
+          for (int m = 0; m < N; ++m)
+            d += qs[t * PITCH + m] * ks[s * PITCH + m] * expf(cs[(t - 1) * PITCH + m] - cs[s * PITCH + m]);
+        if (s != t) ps[t * PP + s] = d;
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) {
+      const int t = tid / (N / 4) + i * (THREADS / (N / 4));
+      float bonus = q[i].x * by.x * k[i].x + q[i].y * by.y * k[i].y + q[i].z * by.z * k[i].z + q[i].w * by.w * k[i].w;
+#pragma unroll
+      for (int off = 1; off < N / 4; off <<= 1) bonus += __shfl_xor_sync(0xffffffffu, bonus, off);
+      if (n == 0) ps[t * PP + t] = bonus;
+      st4(qs + t * PITCH + n, make_float4(q[i].x * expf(b[i].x), q[i].y * expf(b[i].y), q[i].z * expf(b[i].z), q[i].w * expf(b[i].w)));
+      if (safe)
+        st4(ks + t * PITCH + n, make_float4(k[i].x * expf(-c[i].x), k[i].y * expf(-c[i].y), k[i].z * expf(-c[i].z), k[i].w * expf(-c[i].w)));
+    }
+    __syncthreads();
+    if (safe) {  // rows ty, ty + 8, ...; columns x, x + 16 of the pair sums
+      const int x = at.col / 4;
+      float e[4][2];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) e[i][0] = e[i][1] = 0.f;
+#pragma unroll 4
+      for (int m = 0; m < N; m += 4) {
+        const float4 k0 = ld4(ks + x * PITCH + m), k1 = ld4(ks + (x + 16) * PITCH + m);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float4 r = ld4(qs + (at.ty + 8 * i) * PITCH + m);
+          e[i][0] = dot4(r, k0, e[i][0]);
+          e[i][1] = dot4(r, k1, e[i][1]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int u = at.ty + 8 * i, s = x + 16 * j;
+          if (s != u) ps[u * PP + s] = s < u ? e[i][j] : 0.f;
+        }
+      __syncthreads();
+    }
+  }
+#pragma unroll 2
+  for (int n = 0; n < N; n += 4) {
+    float4 s1[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s1[j] = n + 4 < N ? state4(n + 4 + j) : s0[j];  // the next four rows are on the way
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float4 q = ld4(qs + (at.ty + 8 * i) * PITCH + n);
+      fma4(o[i], q.x, s0[0]);
+      fma4(o[i], q.y, s0[1]);
+      fma4(o[i], q.z, s0[2]);
+      fma4(o[i], q.w, s0[3]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s0[j] = s1[j];
+  }
+  if (RULE == 0) {
+#pragma unroll 2
+    for (int s = 0; s < L; s += 4) {
+      float p[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) st4(p[i], ld4(ps + (at.ty + 8 * i) * PP + s));
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float4 v = ld4(vs + (s + j) * PITCH + at.col);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (s + j <= at.ty + 8 * i) fma4(o[i], p[i][j], v);  // a later token's infinities stay its own
+      }
+    }
+  }
+  // per head: divide by the root mean square, weight, gate, scale
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float sq = o[i].x * o[i].x + o[i].y * o[i].y + o[i].z * o[i].z + o[i].w * o[i].w;
+    sq += __shfl_xor_sync(0xffffffffu, sq, 1);
+    sq += __shfl_xor_sync(0xffffffffu, sq, 16);
+    if ((tid & 17) == 0) red[warp * L + at.ty + 8 * i] = sq;
+  }
+  __syncthreads();
+  const float4 w = ld4(a.norm_w + ch0 + at.col);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int t = at.ty + 8 * i;
+    if (t >= nt) continue;
+    const float sum = (red[t] + red[L + t]) + (red[2 * L + t] + red[3 * L + t]);
+    const float by = rsqrtf(sum / (float)N + a.eps) * a.out_scale;
+    const float4 g = widen4(a.g + (row0 + t) * a.g_stride + ch0 + at.col);
+    auto gate = [](float x) { return RULE == 1 ? sigmoid_f(x) : x * sigmoid_f(x); };
+    uint2 raw;
+    raw.x = pack_bf16x2(o[i].x * by * w.x * gate(g.x), o[i].y * by * w.y * gate(g.y));
+    raw.y = pack_bf16x2(o[i].z * by * w.z * gate(g.z), o[i].w * by * w.w * gate(g.w));
+    *reinterpret_cast<uint2*>(a.out + (row0 + t) * a.out_stride + a.out_col + ch0 + at.col) = raw;
+  }
+  if (a.last_rows && h == 0 && first + nt == qlen) {  // the sequence's last row, for the next step's token shift
+    const bf16* row = a.last_rows + (row0 + nt - 1) * a.last_stride;
+    float* dst = a.last_state + (size_t)a.seq_slot[seq] * a.C;
+    for (int c = tid; c < a.C; c += THREADS) dst[c] = __bfloat162float(row[c]);
+  }
+}
+
+template <typename Kernel>
+int run(Kernel kernel, dim3 grid, int threads, size_t floats, const ChunkArgs& a, cudaStream_t stream) {
+  const size_t smem = floats * sizeof(float);
+  if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return (int)launch_pdl(kernel, grid, dim3(threads), smem, stream, a);
+}
+
+}  // namespace
+
+// Tokens per chunk where a step's scan may run in chunks, else 0; *item_floats: scratch of a (sequence, chunk, head).
+KRK_API int krk_recurrence_chunk_tokens(int rule, int head, int R, float decay_scale, int* item_floats) {
+  *item_floats = rule == 1 ? ITEM_DELTA : ITEM_MIX;
+  if (head != N || R < 1 || R > 64) return 0;
+  // the delta rule: e^{decay_scale * 32} is what keys and rates are multiplied by at most
+  if (rule == 1 && !(decay_scale >= 0.f && decay_scale * L <= 40.f)) return 0;
+  return L;
+}
+
+// krk_linear_recurrence over chunks chunk0 .. chunk0 + n_chunks - 1 of every sequence, bfloat16 (float32 state), from and to the
+// stored state; the caller goes through a step's chunks in order. Rows of four elements on 8-byte boundaries.
+KRK_API int krk_recurrence_chunks(int rule, const void* r, int r_stride, const void* k, int k_stride, const void* v, int v_stride,
+                                  const void* g, int g_stride, const void* rate, int rate_stride, const void* lora,
+                                  int lora_stride, const void* w2, const float* w0, const float* rate_bias, const float* bonus,
+                                  const float* norm_w, float* state, const void* last_rows, int last_stride, int C,
+                                  float* last_state, void* out, int out_stride, int out_col, float out_scale, float eps,
+                                  float decay_scale, int H, int R, int n_seqs, const int* cu_q, const int* seq_qlen,
+                                  const int* seq_slot, int chunk0, int n_chunks, float* scratch, cudaStream_t stream) {
+  if (n_seqs == 0 || n_chunks == 0) return 0;
+  int item;
+  const uintptr_t rows = (uintptr_t)r | (uintptr_t)k | (uintptr_t)v | (uintptr_t)g | (uintptr_t)rate | (uintptr_t)out;
+  const uintptr_t floats = (uintptr_t)norm_w | (uintptr_t)state | (uintptr_t)scratch;
+  const int strides = r_stride | k_stride | v_stride | g_stride | rate_stride | out_stride | out_col;
+  if ((rule != 0 && rule != 1) || (rule == 1 && (!rate || !rate_bias)) || (rule == 0 && !bonus) || !scratch ||
+      !krk_recurrence_chunk_tokens(rule, N, R, decay_scale, &item) || (rows & 7) || (strides & 3) || (floats & 15) ||
+      n_chunks > 65535 || n_seqs > 65535 || H > 65535)
+    return -2;
+  ChunkArgs a;
+  a.r = (const bf16*)r; a.k = (const bf16*)k; a.v = (const bf16*)v; a.g = (const bf16*)g; a.rate = (const bf16*)rate;
+  a.lora = (const bf16*)lora; a.r_stride = r_stride; a.k_stride = k_stride; a.v_stride = v_stride; a.g_stride = g_stride;
+  a.rate_stride = rate_stride; a.lora_stride = lora_stride; a.w2 = (const bf16*)w2; a.w0 = w0; a.rate_bias = rate_bias;
+  a.bonus = bonus; a.norm_w = norm_w; a.state = state; a.last_rows = (const bf16*)last_rows; a.last_stride = last_stride;
+  a.C = C; a.last_state = last_state; a.out = (bf16*)out; a.out_stride = out_stride; a.out_col = out_col; a.out_scale = out_scale;
+  a.eps = eps; a.decay_scale = decay_scale; a.H = H; a.R = R; a.cu_q = cu_q; a.seq_qlen = seq_qlen; a.seq_slot = seq_slot;
+  a.chunk0 = chunk0; a.n_chunks = n_chunks; a.scratch = scratch;
+  const dim3 items((unsigned)H, (unsigned)n_chunks, (unsigned)n_seqs);
+  int rc;
+  const size_t RP = (size_t)((R + 7) & ~7);
+  if (rule == 1) {
+    if ((rc = run(delta_chunk_kernel, items, THREADS, 8 * (size_t)L * PITCH + N + L, a, stream))) return rc;
+    const size_t walk = (size_t)WALK_STAGES * N * (PITCH + WALK_COLS) + N * WALK_COLS + 4 * N * 4;
+    if ((rc = run(delta_walk_kernel, dim3(N / WALK_COLS, (unsigned)H, (unsigned)n_seqs), THREADS, walk, a, stream))) return rc;
+    return run(chunk_finish_kernel<1>, items, THREADS, (size_t)L * PITCH + 4 * L, a, stream);
+  }
+  if ((rc = run(mix_chunk_kernel, items, THREADS, 3 * (size_t)L * PITCH + L * RP + 2 * N, a, stream))) return rc;
+  if ((rc = run(mix_walk_kernel, dim3(N * N / 4 / 64, (unsigned)H, (unsigned)n_seqs), 64, 0, a, stream))) return rc;
+  return run(chunk_finish_kernel<0>, items, THREADS, 4 * (size_t)L * PITCH + 4 * L + (size_t)L * (L + 4), a, stream);
+}

@@ -300,6 +300,95 @@ def test_scans_do_not_depend_on_the_cut_to_the_bit():
         rt.ops.split_recurrence = False
 
 
+def scan_inputs(kind, lens, heads, decays, seed):
+    """bfloat16 rows with the spread that trained models show, or with decays that forget everything in a token."""
+    rows, HN, R = sum(lens), heads * 64, 16
+    w0 = {"mild": -3.0, "spread": None, "strong": 3.0}[decays]
+    bf = lambda t: t.to(torch.bfloat16).cuda()
+    x = {k: bf(rand((rows, HN), seed + i)) for i, k in enumerate(("r", "k", "v", "g", "rate"))}
+    x["lora"], x["w2"] = bf(rand((rows, R), seed + 5)), bf(rand((HN, R), seed + 6, 0.2))
+    x["w0"] = (torch.linspace(-6.0, 4.0, HN) if w0 is None else torch.full((HN,), w0)).cuda()
+    x["bias"], x["norm"], x["u"] = rand((HN,), seed + 7).cuda(), (1 + rand((HN,), seed + 8, 0.1)).cuda(), rand((HN,), seed + 9).cuda()
+    return x
+
+
+def run_scan(rt, kind, x, lens, heads, state, decay_scale=0.6):
+    rows, HN = x["r"].shape
+    ctx = context(rt, list(range(len(lens))), [0] * len(lens), lens, None)
+    out = torch.zeros((rows, HN + 8), dtype=torch.bfloat16, device="cuda")
+    more = {"rate": x["rate"], "rate_bias": x["bias"], "decay_scale": decay_scale} if kind == "delta" else {"bonus": x["u"]}
+    rt.ops.linear_recurrence(kind, x["r"], x["k"], x["v"], x["g"], x["lora"], x["w2"], x["w0"], heads, 64, x["norm"], 1e-6,
+                             state, ctx.batch, out, 8, 0.5, **more)
+    return out[:, 8:]
+
+
+def scan_in_64_bits(kind, x, lens, heads, state, decay_scale=0.6):
+    d = {k: v.double().cpu() for k, v in x.items()}
+    z = torch.tanh(x["lora"].float()).to(torch.bfloat16).double().cpu() @ d["w2"].T + d["w0"]
+    head = lambda t: t.view(-1, heads, 64)
+    r, k, v = head(d["r"]), head(d["k"]), head(d["v"])
+    outs, states, row = [], [], 0
+    for i, n in enumerate(lens):
+        cut = slice(row, row + n)
+        if kind == "delta":
+            decay, rate = torch.exp(-decay_scale * torch.sigmoid(z)), torch.sigmoid(d["rate"] + d["bias"])
+            o, S = plain.delta_rule_scan(r[cut], k[cut], v[cut], head(decay)[cut], head(rate)[cut], state[i].double().cpu())
+        else:
+            o, S = plain.wkv_scan(r[cut], k[cut], v[cut], head(torch.exp(-torch.exp(z)))[cut], d["u"].view(heads, 64), state[i].double().cpu())
+        outs.append(o)
+        states.append(S)
+        row += n
+    o = plain.unit_rms(torch.cat(outs), 1e-6).reshape(row, -1) * d["norm"]
+    gate = torch.sigmoid(d["g"]) * (1.0 if kind == "delta" else d["g"])
+    return 0.5 * o * gate, torch.stack(states)
+
+
+@pytest.mark.parametrize("decays", ["mild", "spread", "strong"])
+@pytest.mark.parametrize("lens", [[64], [65, 31, 1, 96], [200, 33]])
+@pytest.mark.parametrize("kind", ["delta", "wkv"])
+def test_scans_in_chunks(kind, lens, decays, monkeypatch):
+    """Steps of many tokens in bfloat16 with heads of 64 channels: chunks of 32 tokens, whole and cut into portions of one
+    chunk (little scratch), from a state that is not zero; against 64 bits, and no further from it than the scan token by
+    token: the outputs within a bfloat16 rounding (2^-8 of a value, and of the row's size for what cancels), the
+    32-bit state within 8e-6 of its size (the decays' sums over a chunk round at 2^-24 of up to 80)."""
+    rt = runtime(torch.bfloat16)
+    heads = 3
+    x = scan_inputs(kind, lens, heads, decays, 60)
+    start = rand((len(lens), heads, 64, 64), 70).cuda()
+    want, want_state = scan_in_64_bits(kind, x, lens, heads, start)
+    off = {}
+    for name, in_chunks, scratch in (("tokens", False, 1 << 28), ("chunks", True, 1 << 28), ("portions", True, 1)):
+        monkeypatch.setattr(type(rt.ops), "_recurrence_in_chunks", lambda *_, yes=in_chunks: yes)
+        monkeypatch.setattr(type(rt.ops), "RECURRENCE_SCRATCH", scratch)
+        state = start.clone()
+        got = run_scan(rt, kind, x, lens, heads, state)
+        size = want.pow(2).mean().sqrt()
+        assert ((got.double().cpu() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-3 * size).all(), name
+        off[name] = ((state.double().cpu() - want_state).norm() / want_state.norm()).item()
+        assert off[name] < 8e-6, (name, off)
+        if name == "chunks":
+            whole = got, state
+    assert torch.equal(got, whole[0]) and torch.equal(state, whole[1]), "portions are the same sums"
+    assert off["chunks"] < 2 * off["tokens"] + 1e-7, off
+
+
+@pytest.mark.parametrize("kind", ["delta", "wkv"])
+def test_a_tokens_infinities_reach_no_earlier_token(kind, monkeypatch):
+    """An infinite value in the middle of a chunk: the tokens before it and the value channels beside it are untouched."""
+    rt = runtime(torch.bfloat16)
+    monkeypatch.setattr(type(rt.ops), "_recurrence_in_chunks", lambda *_: True)
+    x = scan_inputs(kind, [96], 2, "mild", 80)
+    start = rand((1, 2, 64, 64), 90).cuda()
+    states = [start.clone(), start.clone()]
+    clean = run_scan(rt, kind, x, [96], 2, states[0])
+    x["v"] = x["v"].clone()
+    x["v"][41, 5] = float("inf")
+    got = run_scan(rt, kind, x, [96], 2, states[1])
+    assert torch.equal(got[:41], clean[:41]) and torch.equal(got[:, 64:], clean[:, 64:])
+    rest = [p for p in range(64) if p != 5]
+    assert torch.equal(states[1][0, :, :, rest], states[0][0, :, :, rest]) and not torch.isfinite(states[1][0, 0, :, 5]).any()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_parallel_mixer_alone(dtype):
     """Two branches on one input: one stacked input product, one output product over both branches' columns."""
