@@ -146,6 +146,26 @@ def test_token_shift_keeps_the_last_row_of_every_sequence(dtype):
     assert (state[2] == 7.0).all()
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("store", [False, True])
+def test_token_shift_of_many_rows(dtype, store):
+    """Five blends of 64 rows and more: 16-byte pieces, sequences that start anywhere in a block's sixteen rows (one of a
+    single row among them), a width that fills no block. The same bits as the kernel of single elements, which rows that
+    start off a 16-byte boundary take."""
+    rt = runtime(dtype)
+    C, lens = 520, [15, 1, 33, 48, 7]
+    rows = sum(lens)
+    h = rand((rows, C), 10).to(dtype).cuda()
+    odd = torch.empty((rows, C + 1), dtype=dtype, device="cuda")
+    odd[:, 1:] = h
+    mu, start = rand((5, C), 3).cuda(), rand((6, C), 4).cuda()
+    states = [start.clone(), start.clone()]
+    ctx = context(rt, [1, 0, 4, 3, 5], [0] * 5, [[0] * n for n in lens], None)
+    got = rt.ops.token_shift(h, states[0], mu, ctx.batch, store=store)
+    want = rt.ops.token_shift(odd[:, 1:], states[1], mu, ctx.batch, store=store)
+    assert torch.equal(got, want) and torch.equal(states[0], states[1])
+
+
 LEFT_SHAPES = [  # hidden, heads, kv heads, dim, vdim, block, rotated, base, factor
     (64, 4, 2, 16, 32, 10, 8, 100.0, 2.0),
     (48, 2, 2, 24, 8, 37, 24, 5000.0, 1.0),
