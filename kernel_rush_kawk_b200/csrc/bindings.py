@@ -108,6 +108,9 @@ _MEMORY_SIGNATURES = {
     "krk_memory_chunk_decays": [_P, _P, c_int, _P, _P, c_float, c_int, c_int, c_int, c_int, _P, _P, _P],
     "krk_memory_chunks": [_P, _P, _P, c_int, _P, c_int, _P, c_int, c_float, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int,
                           _P, _P, _P, _P],
+    "krk_ssd_steps": [_P, _P, c_int, _P, _P, c_int, c_int, _P],
+    "krk_ssd_chunks": [_P, _P, c_int, _P, c_int, _P, c_int, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
+                       _P, _P, _P, _P],
     "krk_memory_finish": [_P, c_int, c_int, c_float, _P, _P, _P, _P, c_int, _P, c_int, c_int, c_float, c_int, c_int, _P],
 }
 _LATENT_SIGNATURES = {
@@ -1443,6 +1446,10 @@ class Kernels:
         if state.dtype != torch.float32 or not state.is_contiguous() or state.shape[1:] != (heads, N, P):
             raise KernelError("the scan keeps a contiguous float32 state [slots, heads, N, P]")
         y = torch.empty((rows, heads * P), dtype=torch.float32, device=x.device)
+        if x.dtype == torch.bfloat16 and not batch.is_decode and batch.max_q_len >= self.SSD_TENSOR_MIN:
+            tokens = int(self.memory.krk_memory_chunk_tokens(N, P, 1))
+            if tokens and self._ssd_chunks(views, dt_bias, a_log, skip, heads, P, N, groups, state, batch, y, tokens):
+                return y
         chunk, cs, cd = 0, None, None
         if not batch.is_decode and batch.max_q_len >= 2 * self.SSD_CHUNK:
             chunk = self.SSD_CHUNK
@@ -1457,6 +1464,37 @@ class Kernels:
                                         batch.seq_slot.data_ptr(), chunk, _ptr(cs), _ptr(cd), _code(x.dtype),
                                         self._stream()), "state-space scan (a head's state must fit a block's registers)")
         return y
+
+    # tokens of a step's longest sequence from which a bfloat16 scan runs in chunks on the tensor cores (48 heads of 64 x 128, a
+    # whole mixer: one sequence of 33 tokens 41.1 us token by token and 43.1 in chunks, of 64 63 and 53, of 255 188 and 70;
+    # 16 sequences of 64 143 and 135)
+    SSD_TENSOR_MIN = 64
+    SSD_SCRATCH = 256 << 20  # bytes of chunk states
+
+    def _ssd_chunks(self, views, dt_bias, a_log, skip, heads, P, N, groups, state, batch, y, tokens) -> bool:
+        """The scan in chunks on the tensor cores (csrc/matrix_memory_chunks.cu); False, with nothing done, where rows do not
+        start on 16-byte boundaries."""
+        (xp, xs), (bp, bs), (cp, cs_), (dp, ds) = views
+        if any(p % 16 or s % 8 for p, s in views[:3]) or state.data_ptr() % 16:
+            return False
+        rows = y.shape[0]
+        steps = torch.empty((rows, heads, 2), dtype=torch.float32, device=y.device)
+        self._ok(self.memory.krk_ssd_steps(steps.data_ptr(), dp, ds, dt_bias.data_ptr(), a_log.data_ptr(), rows, heads,
+                                           self._stream()), "step sizes and decays")
+        chunks = -(-batch.max_q_len // tokens)
+        # a long step goes through its chunks in portions, so that their states stay within SSD_SCRATCH
+        portion = max(1, min(chunks, 65535 // heads, self.SSD_SCRATCH // (4 * batch.n_seqs * heads * N * P)))
+        items = portion * batch.n_seqs * heads
+        sums = torch.empty((items, N * P), dtype=torch.float32, device=y.device)
+        decays = torch.empty((items, N), dtype=torch.float32, device=y.device)
+        for first in range(0, chunks, portion):
+            self._ok(self.memory.krk_ssd_chunks(y.data_ptr(), xp, xs, bp, bs, cp, cs_, steps.data_ptr(), skip.data_ptr(),
+                                                state.data_ptr(), sums.data_ptr(), decays.data_ptr(), heads, P, N, groups,
+                                                batch.n_seqs, first, min(portion, chunks - first), batch.cu_q.data_ptr(),
+                                                batch.seq_qlen.data_ptr(), batch.seq_slot.data_ptr(), self._stream()),
+                     "state-space scan in chunks")
+            self.launches += 2
+        return True
 
     def gated_group_norm(self, y, gate_rows, weight, parts, eps, out, out_col, out_scale):
         """out[:, out_col:...] = group_norm(y * silu(gate_rows)) * weight * out_scale; y float32, ``parts`` equal parts

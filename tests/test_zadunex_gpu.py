@@ -170,6 +170,111 @@ def test_state_space_mixer_alone(dtype, shape):
         close(got, want, dtype, f"state-space mixer {shape}, pieces {pieces[:4]}, prior {len(prior)}")
 
 
+def ssd_in_64_bits(x, B, C, dt, bias, a_log, skip, groups, lens, start):
+    rows, H = dt.shape
+    d = torch.nn.functional.softplus(dt.double() + bias.double())
+    decay = torch.exp(-torch.exp(a_log.double()) * d)
+    xx, per = x.double().view(rows, H, -1), H // groups
+    bb, cc = (t.double().view(rows, groups, -1).repeat_interleave(per, 1) for t in (B, C))
+    y, states, row = torch.empty_like(xx), [], 0
+    for i, n in enumerate(lens):
+        S = start[i].double()
+        for t in range(row, row + n):
+            S = decay[t][:, None, None] * S + (d[t][:, None] * bb[t])[:, :, None] * xx[t][:, None, :]
+            y[t] = torch.einsum("hn,hnp->hp", cc[t], S) + skip.double()[:, None] * xx[t]
+        states.append(S)
+        row += n
+    return y.view(rows, -1), torch.stack(states)
+
+
+@pytest.mark.parametrize("rate", [-6.0, 0.0, 3.0, "trained"])
+@pytest.mark.parametrize("lens", [[96], [131, 64, 1, 33], [300, 65]])
+@pytest.mark.parametrize("shape", [(4, 64, 128, 2), (3, 80, 16, 1), (2, 16, 48, 2)])  # heads, head size, state rows, groups
+def test_state_space_scans_on_the_tensor_cores(shape, lens, rate, monkeypatch):
+    """Chunks of 64 tokens, whole and in portions of one chunk (little scratch), from a state that is not zero, with decays
+    from almost none to everything within a token: outputs and state no further from 64 bits than twice what the scan
+    token by token is (and 2e-7, a few roundings at 2^-24)."""
+    rt = runtime(torch.bfloat16)
+    H, P, N, G = shape
+    rows = sum(lens)
+    buf = rand((rows, H * P + 2 * G * N), 31).to(torch.bfloat16).cuda()
+    x, B, C = buf[:, :H * P], buf[:, H * P:H * P + G * N], buf[:, H * P + G * N:]
+    dt, bias = rand((rows, H), 32).to(torch.bfloat16).cuda(), rand((H,), 33).cuda()
+    a_log, skip = rand((H,), 34, 0.3).cuda(), rand((H,), 35).cuda()
+    if rate == "trained":  # rates of 1 to 16, steps of 0.001 to 0.1
+        a_log, dt = torch.linspace(0.0, 2.77, H).cuda(), dt * 0.2
+        bias = torch.log(torch.expm1(torch.exp(torch.linspace(-2.3, -6.9, H)))).cuda()
+    else:
+        a_log += rate
+    start = rand((len(lens), H, N, P), 36).cuda()
+    want, want_state = ssd_in_64_bits(x, B, C, dt, bias, a_log, skip, G, lens, start)
+    ctx = context(rt, list(range(len(lens))), [0] * len(lens), lens, None)
+    off = {}
+    for name, least, scratch in (("tokens", 1 << 30, 1 << 28), ("chunks", 1, 1 << 28), ("portions", 1, 1)):
+        monkeypatch.setattr(type(rt.ops), "SSD_TENSOR_MIN", least)
+        monkeypatch.setattr(type(rt.ops), "SSD_SCRATCH", scratch)
+        state = start.clone()
+        y = rt.ops.ssd_scan(x, B, C, dt, bias, a_log, skip, H, P, N, G, state, ctx.batch)
+        off[name] = [((a.double() - b).norm() / b.norm()).item() for a, b in ((y, want), (state, want_state))]
+        if name == "chunks":
+            whole = y, state
+    assert torch.equal(y, whole[0]) and torch.equal(state, whole[1]), "portions are the same sums"
+    assert all(c <= 2 * t + 2e-7 for c, t in zip(off["chunks"], off["tokens"])), off
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_convolution_of_many_rows(dtype):
+    """64 rows and more with four taps: sequences that start anywhere in a thread's sixteen rows, shorter than the taps, channels
+    that fill no block. The same bits as the kernel of single elements, which rows off a 16-byte boundary take."""
+    rt = runtime(dtype)
+    ch, lens = 520, [15, 1, 2, 33, 48, 7]
+    rows = sum(lens)
+    x = rand((rows, ch), 50).to(dtype).cuda()
+    odd = torch.empty((rows, ch + 1), dtype=dtype, device="cuda")
+    odd[:, 1:] = x
+    w, b, tail = rand((4, ch), 51).cuda(), rand((ch,), 52).cuda(), rand((7, 3, ch), 53).to(dtype).cuda()
+    ctx = context(rt, [1, 0, 4, 3, 5, 6], [9] * 6, lens, None)
+    tails = [tail.clone(), tail.clone()]
+    got = rt.ops.causal_conv_silu(x, w, b, tails[0], ctx.batch)
+    want = rt.ops.causal_conv_silu(odd[:, 1:], w, b, tails[1], ctx.batch)
+    assert torch.equal(got, want) and torch.equal(tails[0], tails[1])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n", [4, 32, 124, 256, 260, 768, 772, 1024, 1028])
+def test_gated_norm_of_parts_of_any_size(dtype, n):
+    """Up to 1,024 elements a part a warp each, beyond that a block: within an element's rounding and a sum's of n terms."""
+    rt = runtime(dtype)
+    rows, parts = 5, 3
+    y, z = rand((rows, parts * n), 54).cuda(), rand((rows, parts * n), 55).to(dtype).cuda()
+    weight, out = (1 + rand((parts * n,), 56, 0.2)).cuda(), torch.zeros((rows, parts * n + 8), dtype=dtype, device="cuda")
+    rt.ops.gated_group_norm(y, z, weight, parts, 1e-5, out, 4, 0.5)
+    v = (y.double() * torch.nn.functional.silu(z.double())).view(rows, parts, n)
+    want = 0.5 * (v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-5)).view(rows, -1) * weight.double()
+    unit = 2.0 ** -8 if dtype == torch.bfloat16 else 2e-6
+    assert ((out[:, 4:-4].double() - want).abs() <= unit * want.abs() + 1e-12).all()
+    assert not out[:, :4].any() and not out[:, -4:].any()
+
+
+def test_a_tokens_infinities_reach_no_earlier_token_of_a_state_space_chunk(monkeypatch):
+    rt = runtime(torch.bfloat16)
+    monkeypatch.setattr(type(rt.ops), "SSD_TENSOR_MIN", 1)
+    H, P, N = 2, 64, 32
+    x, B, C = (rand((100, n), 40 + i).to(torch.bfloat16).cuda() for i, n in enumerate((H * P, N, N)))
+    dt, vec = rand((100, H), 43).to(torch.bfloat16).cuda(), rand((H,), 44).cuda()
+    ctx = context(rt, [0], [0], [100], None)
+    got = []
+    for value in (1.0, float("inf")):
+        x = x.clone()
+        x[41, 5] = value
+        state = torch.zeros((1, H, N, P), device="cuda")
+        got.append((rt.ops.ssd_scan(x, B, C, dt, vec, vec, vec, H, P, N, 1, state, ctx.batch), state))
+    (y0, s0), (y1, s1) = got
+    rest = [c for c in range(H * P) if c != 5]
+    assert torch.equal(y0[:41], y1[:41]) and torch.equal(y0[:, rest], y1[:, rest]) and not torch.isfinite(y1[41:, 5]).any()
+    assert torch.equal(s0[0, 1], s1[0, 1]) and not torch.isfinite(s1[0, 0, :, 5]).any()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_a_state_carries_one_loud_token_over_hundreds(dtype):
     """A head whose decay is almost one keeps a token that came hundreds of tokens (and several chunks and
