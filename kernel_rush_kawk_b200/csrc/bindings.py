@@ -92,6 +92,7 @@ _MOE_SIGNATURES = {
     "krk_moe_route_softmax_groups": [_P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P],
     "krk_moe_gate_up_pairs": [_P, _P, c_int, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_float, c_float, c_int, _P],
     "krk_moe_down_pairs": [_P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, _P, c_int, _P, c_int, _P],
+    "krk_few_experts": [_P, _P, c_int, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_float, c_float, _P],
     "krk_moe_sort": [_P, _P, _P, c_int, c_int, c_int, _P],
     "krk_moe_gather": [_P, _P, c_int, _P, _P, _P, c_int, c_int, c_int, c_int, _P, _P, c_int, _P],
     "krk_grouped_gemm": [_P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_float, c_float, _P, _P],
@@ -897,6 +898,18 @@ class Kernels:
         single = batch is not None and batch.is_decode  # such a step may be replayed from a graph: nothing comes to the host
         if single or rows * top <= max(self.MOE_PAIR_ROWS * top, 2 * E):
             pairs = torch.empty((rows * top, F), dtype=x.dtype, device=x.device)
+            if self._few_experts(x, K, F, C, rows, top):
+                # bfloat16: an expert's weights meet all its rows at once; the pairs' results are added up by their rows
+                self._ok(self.moe.krk_few_experts(pairs.data_ptr(), ptr, stride, w_gate_up.data_ptr(), experts.data_ptr(), rows, top,
+                                                  E, F, K, int(not gated), act, _ptr(w_in), float(limit), float(slope),
+                                                  self._stream()), "experts' first product of few rows")
+                y = torch.empty((rows * top, C), dtype=x.dtype, device=x.device)
+                self._ok(self.moe.krk_few_experts(y.data_ptr(), pairs.data_ptr(), F, w_down.data_ptr(), experts.data_ptr(), rows, top,
+                                                  E, C, F, 2, 0, None, 0.0, 0.0, self._stream()), "experts' second product of few rows")
+                self._ok(self.moe.krk_moe_combine(out.data_ptr(), _ptr(add), _ptr(add_gate), y.data_ptr(), None, experts.data_ptr(),
+                                                  None, 0, _ptr(w_out), rows, top, C, ptr, stride, _ptr(add_input),
+                                                  _code(x.dtype), self._stream()), "experts' sum")
+                return out
             self._ok(self.moe.krk_moe_gate_up_pairs(pairs.data_ptr(), ptr, stride, w_gate_up.data_ptr(), experts.data_ptr(),
                                                     rows, top, F, K, act, int(gated), _ptr(w_in), float(limit), float(slope),
                                                     _code(x.dtype), self._stream()), "experts' gate/up")
@@ -940,6 +953,12 @@ class Kernels:
                                           offsets.data_ptr(), cap, _ptr(w_out), rows, top, C, ptr, stride,
                                           _ptr(add_input), _code(x.dtype), self._stream()), "experts' sum")
         return out
+
+    @staticmethod
+    def _few_experts(x, K, F, C, rows, top) -> bool:
+        """Whether the experts' products of few rows run once per expert (csrc/few_experts.cu): type, sizes and alignment."""
+        return (x.dtype == torch.bfloat16 and K % 8 == 0 and F % 8 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
+                and rows * top <= 4096)
 
     @staticmethod
     def _use_grouped(x, K, F, C, gated, activation) -> bool:

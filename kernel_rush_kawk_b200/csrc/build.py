@@ -37,7 +37,7 @@ CORE_LIBS = ["-lcublasLt"]  # lt_gemm.cu; the process already holds the copy tha
 MIX_SOURCES = ["wide_rows.cu", "sink_attention.cu", "latent.cu", "hyper.cu", "mixed_attention.cu", "latent_decode.cu"]
 SCAN_SOURCES = ["recurrent.cu", "recurrent_chunks.cu", "ssd.cu"]
 MEMORY_SOURCES = ["matrix_memory.cu", "matrix_memory_chunks.cu", "matrix_memory_step.cu"]
-MOE_SOURCES = ["routed.cu", "grouped_gemm.cu"]
+MOE_SOURCES = ["routed.cu", "few_experts.cu", "grouped_gemm.cu"]
 SMALL_LIBRARIES = {"mix": MIX_SOURCES, "scan": SCAN_SOURCES, "memory": MEMORY_SOURCES, "moe": MOE_SOURCES}
 LATENT_SOURCES = ["latent_prefill.cu"]
 ATTN_SOURCES = ["attention_simple.cu", "attention_mma.cu", "attention_tcgen05.cu"]

@@ -16,14 +16,16 @@
 // identity weights goes to a buffer of its own; whoever adds up the experts' results also adds that number times the
 // row. Every kernel below takes -1 for "no expert".
 //
-// Few rows (single-token steps): a (row, chosen expert) pair reads its expert's weights once.
+// Few rows (single-token steps), 32-bit or sizes that few_experts.cu does not take: a (row, chosen expert) pair reads its
+// expert's weights by itself.
 //   krk_moe_gate_up_pairs: act[pair, f] = a(Wg_e[f] . x_r) * (Wu_e[f] . x_r), a warp per f, lanes over K.
 //   krk_moe_down_pairs: out[r, c] = add[r, c] + sum_j weight[r, j] * (Wd_e(j)[c] . act[(r, j)]), a warp per c;
 //   the sum over the chosen experts is float32, in the order of the choice.
 //
 // Many rows: pairs are counted per expert and ordered by expert on the device (krk_moe_sort: one block; offsets
 // and the pairs' places), krk_moe_gather copies the rows into that order, the experts' products run over
-// contiguous rows, and krk_moe_combine adds each row's weighted results onto `add`. With cap > 0 every expert's
+// contiguous rows, and krk_moe_combine adds each row's weighted results onto `add` (without places: results
+// in the pairs' own order). With cap > 0 every expert's
 // rows start at a multiple of cap (expert e's i-th pair sits in row e * cap + i), which is the layout a batched
 // batched product over [experts, cap, K] reads.
 //
@@ -399,6 +401,7 @@ __device__ __forceinline__ int row_of_pair(const int* __restrict__ place, const 
                                            const int* __restrict__ offsets, int cap, int pair) {
   const int e = experts[pair];
   if (e < 0) return -1;
+  if (!place) return pair;  // results in the pairs' own order
   if (cap <= 0) return place[pair];
   return e * cap + place[pair] - offsets[e];
 }

@@ -352,6 +352,52 @@ def test_routed_experts_alone(dtype, shape, rows):
         close(part.forward(ctx, h.cuda()), want, dtype, f"experts {shape}, {rows} rows, single-token step {decode}")
 
 
+@pytest.mark.parametrize("gated,activation,weigh_input", [(True, "silu", False), (True, "swish_clamped", True), (False, "relu2", False)])
+@pytest.mark.parametrize("sizes", [(40, 24, 8, 8), (264, 72, 136, 33), (512, 176, 200, 4)])  # K, F, C, experts
+@pytest.mark.parametrize("rows,top", [(1, 2), (5, 3), (17, 4), (50, 2)])
+def test_products_of_few_experts_rows(gated, activation, weigh_input, sizes, rows, top):
+    """Single-token steps in bfloat16, an expert's weights read once for all its rows: one row to more than sixteen rows an
+    expert, more pairs than experts and fewer, choices that are no expert, sizes off the tiles of 16 and 32; no further from
+    64 bits than the kernels that read an expert per pair are, within a rounding of the result."""
+    rt = runtime(torch.bfloat16)
+    K, F, C, E = sizes
+    bf = lambda t: t.to(torch.bfloat16).cuda()
+    x, w1, w2 = bf(rand((rows, K), 1)), bf(rand((E, (2 if gated else 1) * F, K), 2, 0.2)), bf(rand((E, C, F), 3, 0.3))
+    g = torch.Generator().manual_seed(rows)
+    experts = torch.stack([torch.randperm(min(E, 6), generator=g)[:top] for _ in range(rows)]).to(torch.int32)
+    experts[rows // 2, 0] = -1
+    weights, add, gate = rand((rows, top), 5).abs().cuda(), bf(rand((rows, C), 6)), rand((rows,), 7).cuda()
+    params = (2.0, 1.702) if activation == "swish_clamped" else None
+    want = torch.zeros((rows, C), dtype=torch.float64)
+    for r in range(rows):
+        want[r] = gate[r].item() * add[r].double().cpu()
+        for j in range(top):
+            e, a = int(experts[r, j]), weights[r, j].item()
+            if e < 0:
+                continue
+            z = w1[e].double().cpu() @ x[r].double().cpu() * (a if weigh_input else 1.0)
+            if activation == "swish_clamped":
+                p, u = z[:F].clamp(max=2.0), z[F:].clamp(-2.0, 2.0)
+                h = p * torch.sigmoid(1.702 * p) * (u + 1.0)
+            else:
+                h = torch.nn.functional.silu(z[:F]) * z[F:] if gated else z.clamp(min=0.0) ** 2
+            want[r] += (1.0 if weigh_input else a) * (w2[e].double().cpu() @ h)
+    off = {}
+    for few in (True, False):
+        ops = type(rt.ops)
+        kept = ops._few_experts
+        if not few:
+            ops._few_experts = staticmethod(lambda *_: False)
+        try:
+            got = rt.ops.moe_experts(x, w1, w2, experts.cuda(), weights, F, activation, add=add, add_gate=gate,
+                                     batch=SimpleNamespace(is_decode=True), gated=gated, act_params=params, weigh_input=weigh_input)
+        finally:
+            ops._few_experts = staticmethod(kept)
+        off[few] = ((got.double().cpu() - want).norm() / want.norm()).item()
+    assert off[True] <= 1.2 * off[False] + 2.0 ** -10, off
+    assert off[True] < 1e-2, off
+
+
 def test_routing_takes_the_lower_index_on_a_tie_and_weighs_by_the_chosen_logits_only():
     rt = runtime(torch.float32)
     x = torch.eye(4, device="cuda")
