@@ -29,6 +29,14 @@
 // member) pairs of one kv head, row R -> token R / G, head kh * G + R % G, so all G query heads of a
 // kv head share one read of K and V (attention.py:70-73). Every barrier wait is bounded.
 //
+// WIDE: attention whose softmax weights are 32-bit quantities (krk_sink_prefill_tcgen05). A weight reaches P V as two bfloat16
+// halves, p = hi + lo (16 bits of mantissa), which take the two halves of S's columns in tensor memory, and each instruction of
+// P V comes twice. A row may start from a softmax sink (maximum = its head's sink, sum 1, no value); rows of the output may lie
+// apart, are multiplied by a number and by the sigmoid of a gate per head or per element. SHAPED: scores are capped
+// (c tanh(s / c) = c (1 - 2 / (1 + e^(2 s / c)))) and lose a slope times the distance of query and key before the softmax.
+// 2,048 tokens, a window of 1,024, 16 heads of 128 in groups of four: 45 us against the mma.sync kernel's 116 (of 37 at that
+// instruction's measured rate, 550 TFLOP/s, for 19 GFLOP); 12 heads in groups of three, no slopes, 46 against 75.
+//
 // Compiled once per head size, for head sizes 64 and 128: -DKRK_HEAD_DIM=<D>.
 #include "tcgen05.cuh"
 
@@ -83,12 +91,23 @@ __device__ __forceinline__ TileRange tile_range(int row_begin, int n_rows, int G
   return t;
 }
 
+// What the wide form adds; see the opening text.
+struct Extras {
+  const float *sink, *slopes;  // per query head, either may be null
+  float cap_log2, in_cap;      // softcap in log2 units, and what an exponent of 2 (x, in log2 units) is multiplied by; 0: none
+  float out_scale;
+  const bf16* gate;
+  int gate_stride, gate_mode;  // 0: none, 1: a column per head, 2: a column per element
+  int out_stride;
+};
+
+template <bool WIDE, bool SHAPED>
 __global__ void __launch_bounds__(THREADS, 1)
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                          const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_o, int q_by_tma, bf16* __restrict__ out, const bf16* __restrict__ qkv, int q_stride, int HQ, int HKV,
                          const int* __restrict__ seq_slot, const int* __restrict__ seq_start,
                          const int* __restrict__ seq_qlen, const int* __restrict__ cu_q, const int* __restrict__ table,
-                         int width, float scale_log2, int window, int* __restrict__ error) {
+                         int width, float scale_log2, int window, int* __restrict__ error, const Extras ex) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* q_s = base;                    // two tiles
@@ -217,9 +236,13 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
       auto pv = [&](int t, int i, bool first) {  // O_t (+)= P_t V_i, 16 keys (8 columns of P) per instruction
         const unsigned char* v = v_s + (i & 1) * TILE_BYTES;
 #pragma unroll
-        for (int ks = 0; ks < KEYS / 16; ++ks)
+        for (int ks = 0; ks < KEYS / 16; ++ks) {
           umma_bf16_tmem_a(tmem + TMEM_O + t * D, tmem + t * 128 + ks * 8, umma_desc_sw128(v + ks * 16 * 128, SUB, 1024),
                            idesc_o, (first && ks == 0) ? 0u : 1u);
+          if constexpr (WIDE)  // the weights' low halves
+            umma_bf16_tmem_a(tmem + TMEM_O + t * D, tmem + t * 128 + 64 + ks * 8, umma_desc_sw128(v + ks * 16 * 128, SUB, 1024),
+                             idesc_o, 1u);
+        }
       };
       const TileRange rng[2] = {r0, r1};
       if (q_by_tma && !mbar_wait(bars + Q_FULL, 0)) give_up(14);
@@ -286,7 +309,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     const TileRange rng[2] = {r0, r1};
     bool valid[2];
     int tok[2], pos[2], lo[2];
-    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, slope[2] = {0.f, 0.f};
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
       const int R = pair * PAIR + t * ROWS + r;
@@ -294,6 +317,14 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
       tok[t] = valid[t] ? R / G : 0;
       pos[t] = valid[t] ? start + tok[t] : -1;  // -1: sees nothing
       lo[t] = (valid[t] && window > 0) ? max(0, pos[t] - window + 1) : 0;
+      if constexpr (WIDE) {
+        const int head = kh * G + (valid[t] ? R % G : 0);
+        if (ex.sink) {
+          m[t] = ex.sink[head] * LOG2E;
+          l[t] = half == 0 ? 1.f : 0.f;  // the two halves' sums are added at the end
+        }
+        if (SHAPED && ex.slopes) slope[t] = ex.slopes[head] * LOG2E;
+      }
     }
     auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory"); };
     bool ok = true, stores_pending = false;
@@ -323,6 +354,21 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
 #pragma unroll
           for (int q = 0; q < HALF / 32; ++q) tmem_ld_32x32(tmem_s + HALF * half + 32 * q, *reinterpret_cast<uint32_t(*)[32]>(s + 32 * q));
           tmem_wait_ld();
+          if constexpr (SHAPED) {  // in log2 units from here on; the slope's distance counted from the half's first key
+            const float away = slope[t] * (float)(pos[t] - key0);
+            if (ex.in_cap > 0.f) {
+#pragma unroll
+              for (int i = 0; i < HALF; ++i) {
+                const float x = __uint_as_float(s[i]) * scale_log2;
+                const float y = ex.cap_log2 * (1.f - __fdividef(2.f, 1.f + fast_exp2(x * ex.in_cap)));
+                s[i] = __float_as_uint(fmaf(slope[t], (float)i, y - away));
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < HALF; ++i)
+                s[i] = __float_as_uint(fmaf(slope[t], (float)i, fmaf(__uint_as_float(s[i]), scale_log2, -away)));
+            }
+          }
           if (whole) {
 #pragma unroll
             for (int i = 0; i < HALF; ++i) mx = fmaxf(mx, __uint_as_float(s[i]));
@@ -339,15 +385,16 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         pair_sync();
         if (gave_up[quad]) { ok = false; break; }
         mx = fmaxf(mx, xm[(half ^ 1) * ROWS + r]);
-        const float m_new = fmaxf(m[t], mx * scale_log2);
+        const float m_new = fmaxf(m[t], SHAPED ? mx : mx * scale_log2);
         const bool outgrown = m[t] != -INFINITY && m_new - m[t] > RESCALE_STEP;
         if (__any_sync(0xffffffffu, outgrown)) {
           // the warp moves its rows' reference maxima (its partner, with the same rows and maxima, decides the
           // same) and scales its half of the columns of O; the block's P.V has not been issued and the one
           // before it is complete (S of this block came after it), so nothing else touches these rows of O
           const float alpha = m[t] == -INFINITY ? 1.f : fast_exp2(m[t] - m_new);
+          // a row that starts from a sink may outgrow it in the tile's first block, when there is no O yet
 #pragma unroll
-          for (int c0 = 0; c0 < D / 2; c0 += 32) {
+          for (int c0 = 0; c0 < ((WIDE && c == 0) ? 0 : D / 2); c0 += 32) {
             uint32_t o[32];
             tmem_ld_32x32(tmem_o + half * (D / 2) + c0, o);
             tmem_wait_ld();
@@ -362,30 +409,33 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         }
         const float m_safe = m[t] == -INFINITY ? 0.f : m[t];
         float sum = 0.f;
-        uint32_t pk[HALF / 2];
+        uint32_t pk[HALF / 2], pl[WIDE ? HALF / 2 : 1];
+        auto weight = [&](int i) {
+          return fast_exp2(SHAPED ? __uint_as_float(s[i]) - m_safe : fmaf(__uint_as_float(s[i]), scale_log2, -m_safe));
+        };
+        auto keep = [&](int i, float p0, float p1) {
+          sum += p0 + p1;
+          const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
+          const uint32_t hi = *reinterpret_cast<const uint32_t*>(&h);
+          pk[i / 2] = hi;
+          if constexpr (WIDE) {
+            const __nv_bfloat162 d = __floats2bfloat162_rn(p0 - __uint_as_float(hi << 16), p1 - __uint_as_float(hi & 0xffff0000u));
+            pl[i / 2] = *reinterpret_cast<const uint32_t*>(&d);
+          }
+        };
         if (whole) {
 #pragma unroll
-          for (int i = 0; i < HALF; i += 2) {
-            const float p0 = fast_exp2(fmaf(__uint_as_float(s[i]), scale_log2, -m_safe));
-            const float p1 = fast_exp2(fmaf(__uint_as_float(s[i + 1]), scale_log2, -m_safe));
-            sum += p0 + p1;
-            const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
-            pk[i / 2] = *reinterpret_cast<const uint32_t*>(&h);
-          }
+          for (int i = 0; i < HALF; i += 2) keep(i, weight(i), weight(i + 1));
         } else {
 #pragma unroll
-          for (int i = 0; i < HALF; i += 2) {
-            const float p0 = ((unsigned)i - first <= span) ? fast_exp2(fmaf(__uint_as_float(s[i]), scale_log2, -m_safe)) : 0.f;
-            const float p1 = ((unsigned)(i + 1) - first <= span) ? fast_exp2(fmaf(__uint_as_float(s[i + 1]), scale_log2, -m_safe)) : 0.f;
-            sum += p0 + p1;
-            const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
-            pk[i / 2] = *reinterpret_cast<const uint32_t*>(&h);
-          }
+          for (int i = 0; i < HALF; i += 2)
+            keep(i, ((unsigned)i - first <= span) ? weight(i) : 0.f, ((unsigned)(i + 1) - first <= span) ? weight(i + 1) : 0.f);
         }
         l[t] += sum;
         __syncwarp();  // rows that see their whole half and rows at its edge took different paths
         // P's second half lands on score columns of the partner warp, which holds them in registers since the barrier
         tmem_st_32x32(tmem_s + (HALF / 2) * half, pk);
+        if constexpr (WIDE) tmem_st_32x32(tmem_s + HALF + (HALF / 2) * half, pl);
         tmem_wait_st();
         tc_fence_before();
         mbar_arrive(bars + P_READY + t);
@@ -410,7 +460,16 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
       if (fine) {
         tc_fence_after();
         const uint32_t tmem_o = tmem + TMEM_O + t * D + lane_addr;
-        const float inv = valid[t] ? 1.0f / l[t] : 0.f;
+        float inv = valid[t] ? (WIDE ? ex.out_scale : 1.0f) / l[t] : 0.f;
+        const bf16* gp = nullptr;  // this row's gates, one per element
+        if constexpr (WIDE) {
+          if (ex.gate_mode && valid[t]) {
+            const int head = kh * G + (pair * PAIR + t * ROWS + r) % G;
+            const bf16* g = ex.gate + (size_t)(row0 + tok[t]) * ex.gate_stride;
+            if (ex.gate_mode == 1) inv /= 1.0f + expf(-__bfloat162float(g[head]));
+            else gp = g + (size_t)head * D;
+          }
+        }
 #pragma unroll
         for (int c0 = 0; c0 < D / 2; c0 += 32) {
           uint32_t o[32];
@@ -418,6 +477,12 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
           tmem_wait_ld();
 #pragma unroll
           for (int c = 0; c < 32; c += 8) {
+            if constexpr (WIDE) {
+              if (gp)
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                  o[c + e] = __float_as_uint(__uint_as_float(o[c + e]) / (1.0f + expf(-__bfloat162float(gp[half * (D / 2) + c0 + c + e]))));
+            }
             uint4 pk;
             __nv_bfloat162* pp = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll
@@ -449,7 +514,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
           const int row = p / (D / 8), piece = p % (D / 8);
           const int R = row_begin + row;
           if (R < n_rows)
-            *reinterpret_cast<uint4*>(out + (size_t)(row0 + R / G) * HQ * D + (size_t)(kh * G + R % G) * D + piece * 8) =
+            *reinterpret_cast<uint4*>(out + (size_t)(row0 + R / G) * (WIDE ? ex.out_stride : HQ * D) + (size_t)(kh * G + R % G) * D + piece * 8) =
                 *reinterpret_cast<const uint4*>(stage + (piece / 8) * SUB + swz(row, piece % 8));
         }
       }
@@ -466,6 +531,43 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
 
 constexpr size_t SMEM_BYTES = 6 * TILE_BYTES + 1024 + N_BARS * 8 + 64 + PAGE_IDS * sizeof(int) + 8 * ROWS * sizeof(float) + 16;
 
+template <bool WIDE, bool SHAPED>
+int launch_tcgen05(bf16* out, const bf16* q, int q_stride, int HQ, int HKV, const int* seq_slot, const int* seq_start,
+                   const int* seq_qlen, const int* cu_q, const int* table, int width, const void* k_cache, const void* v_cache,
+                   int n_pages, int n_seqs, int max_q_len, int total_rows, float scale, int window, int* error, const Extras& ex,
+                   cudaStream_t stream) {
+  const int G = HQ / HKV;
+  const long long tiles = ((long long)max_q_len * G + PAIR - 1) / PAIR;
+  if (tiles * HKV > 0x7fffffffLL || n_seqs > 65535) return -3;
+  CUtensorMap map_k, map_v;
+  const long long rows = (long long)n_pages * HKV * KRK_PAGE;
+  int rc = make_map_bf16(&map_k, k_cache, rows, D, D, 64);
+  if (rc) return rc;
+  rc = make_map_bf16(&map_v, v_cache, rows, D, D, 64);
+  if (rc) return rc;
+  // the query tiles come by TMA when a tile is a whole number of tokens (the group size divides 128)
+  const int q_by_tma = (ROWS % G == 0) ? 1 : 0;
+  CUtensorMap map_q = map_k, map_o = map_k;
+  if (q_by_tma) {
+    rc = make_map_bf16_3d(&map_q, q, D, HQ, total_rows, D, q_stride, G, ROWS / G);
+    if (rc) return rc;
+    rc = make_map_bf16_3d(&map_o, out, D, HQ, total_rows, D, ex.out_stride, G, ROWS / G);
+    if (rc) return rc;
+  }
+  auto kern = attention_tcgen05_kernel<WIDE, SHAPED>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  kern<<<dim3((unsigned)(tiles * HKV), n_seqs, 1), THREADS, SMEM_BYTES, stream>>>(
+      map_k, map_v, map_q, map_o, q_by_tma, out, q, q_stride, HQ, HKV, seq_slot, seq_start, seq_qlen, cu_q, table, width,
+      scale * LOG2E, window, error, ex);
+  KRK_CHECK_LAUNCH();
+  return 0;
+}
+
 }  // namespace
 
 // Same arguments as krk_attention_prefill plus the cache's number of pages and the number of rows of qkv
@@ -476,40 +578,31 @@ KRK_API int krk_attention_prefill_tcgen05(void* out, const void* qkv, int q_stri
                                           const void* v_cache, int n_pages, int n_seqs, int max_q_len, int total_rows,
                                           float scale, int window, int* error, cudaStream_t stream) {
   if (n_seqs == 0 || max_q_len == 0) return 0;
-  const int G = HQ / HKV;
-  const long long tiles = ((long long)max_q_len * G + PAIR - 1) / PAIR;
-  if (tiles * HKV > 0x7fffffffLL || n_seqs > 65535) return -3;
   if ((q_stride % 8) || ((uintptr_t)qkv & 15) || ((uintptr_t)out & 15)) return -2;
-  CUtensorMap map_k, map_v;
-  const long long rows = (long long)n_pages * HKV * KRK_PAGE;
-  int rc = make_map_bf16(&map_k, k_cache, rows, D, D, 64);
-  if (rc) return rc;
-  rc = make_map_bf16(&map_v, v_cache, rows, D, D, 64);
-  if (rc) return rc;
-  // the query tiles come by TMA when a tile is a whole number of tokens (the group size divides 128)
-  const int q_by_tma = (ROWS % G == 0) ? 1 : 0;
-  CUtensorMap map_q = map_k;
-  if (q_by_tma) {
-    rc = make_map_bf16_3d(&map_q, qkv, D, HQ, total_rows, D, q_stride, G, ROWS / G);
-    if (rc) return rc;
-  }
-  CUtensorMap map_o = map_k;
-  if (q_by_tma) {
-    rc = make_map_bf16_3d(&map_o, out, D, HQ, total_rows, D, (long long)HQ * D, G, ROWS / G);
-    if (rc) return rc;
-  }
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attention_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
-  dim3 grid((unsigned)(tiles * HKV), n_seqs, 1);
-  attention_tcgen05_kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(
-      map_k, map_v, map_q, map_o, q_by_tma, (bf16*)out, (const bf16*)qkv, q_stride, HQ, HKV, seq_slot, seq_start, seq_qlen, cu_q, table, width,
-      scale * LOG2E, window, error);
-  KRK_CHECK_LAUNCH();
-  return 0;
+  Extras ex = {};
+  ex.out_stride = HQ * D;
+  return launch_tcgen05<false, false>((bf16*)out, (const bf16*)qkv, q_stride, HQ, HKV, seq_slot, seq_start, seq_qlen, cu_q, table, width,
+                                      k_cache, v_cache, n_pages, n_seqs, max_q_len, total_rows, scale, window, error, ex, stream);
+}
+
+// krk_sink_window_prefill (attention_mma.cu) on the 5th-generation tensor cores: the same arguments plus the cache's number of
+// pages, the number of rows of the queries and the error word, less the kept first keys, which it does not take. -2: rows or
+// columns off 16-byte boundaries, or a scale that is not positive (maxima are taken before it).
+KRK_API int krk_sink_prefill_tcgen05(void* out, int out_stride, float out_scale, const void* q, int q_stride, int HQ, int HKV,
+                                     const float* sink, const int* seq_slot, const int* seq_start, const int* seq_qlen,
+                                     const int* cu_q, const int* table, int width, const void* k_cache, const void* v_cache,
+                                     int n_pages, int n_seqs, int max_q_len, int total_rows, float scale, int window, const void* gate,
+                                     int gate_stride, int gate_mode, const float* slopes, float softcap, int* error,
+                                     cudaStream_t stream) {
+  if (n_seqs == 0 || max_q_len == 0) return 0;
+  if (q_stride % 8 || out_stride % 8 || ((uintptr_t)q & 15) || ((uintptr_t)out & 15) || !(scale > 0.f)) return -2;
+  Extras ex = {};
+  ex.sink = sink; ex.slopes = slopes; ex.out_scale = out_scale; ex.out_stride = out_stride;
+  ex.cap_log2 = softcap * LOG2E; ex.in_cap = softcap > 0.f ? 2.f / softcap : 0.f;
+  ex.gate = (const bf16*)gate; ex.gate_stride = gate_stride; ex.gate_mode = gate ? gate_mode : 0;
+  auto go = slopes || softcap > 0.f ? launch_tcgen05<true, true> : launch_tcgen05<true, false>;
+  return go((bf16*)out, (const bf16*)q, q_stride, HQ, HKV, seq_slot, seq_start, seq_qlen, cu_q, table, width, k_cache, v_cache, n_pages,
+            n_seqs, max_q_len, total_rows, scale, window, error, ex, stream);
 }
 
 #endif  // head sizes served by this kernel

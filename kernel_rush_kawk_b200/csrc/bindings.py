@@ -140,6 +140,8 @@ _ATTN_SIGNATURES = {
                               c_int, _P],
     "krk_sink_window_prefill": [_P, c_int, c_float, _P, c_int, c_int, c_int, _P, _P, _P, _P, _P, _P, c_int, _P, _P, c_int,
                                 c_int, c_float, c_int, c_int, c_int, _P, c_int, c_int, _P, c_float, _P],
+    "krk_sink_prefill_tcgen05": [_P, c_int, c_float, _P, c_int, c_int, c_int, _P, _P, _P, _P, _P, _P, c_int, _P, _P, c_int, c_int,
+                                 c_int, c_int, c_float, c_int, _P, c_int, c_int, _P, c_float, _P, _P],
     "krk_sink_window_decode": [_P, c_int, c_float, _P, c_int, c_int, c_int, _P, _P, _P, _P, c_int, _P, _P, c_int, c_float, c_int,
                                c_int, c_int, _P, c_int, c_int, _P, c_float, c_int, _P],
     "krk_mixed_prefill": [_P, c_int, c_float, _P, c_int, c_int, c_int, _P, _P, _P, _P, _P, _P, _P, c_int, _P, _P, c_int,
@@ -1038,6 +1040,12 @@ class Kernels:
         return self.sink_attention(proj, q_col, heads, dim, vdim, sink, scale, window, batch, cache, out, out_col, out_scale,
                                    fuse=(k_col, v_col, inv_freq, rot_dims, value_eps))
 
+    # Windowed prompts take the tcgen05 kernel from so many rows (tokens times heads of a group) of the longest sequence and so many
+    # keys in a row's sight: a block of it walks two tiles of 128 rows through blocks of 128 keys, which pays where the walk is
+    # long (a whole mixer of 16/4 heads of 128 with a window of 1,024, mma.sync and tcgen05: one prompt of 256 tokens 31 and 35 us, of
+    # 512 47 and 45, of 1,024 85 and 67; 64 tokens behind 1,400 62 and 56; 12/4 heads: 512 tokens 86 and 90, 1,024 147 and 134)
+    SINK_TCGEN05_ROWS, SINK_TCGEN05_KEYS = 192, 640
+
     def sink_attention(self, proj, q_col, heads, dim, vdim, sink, scale, window, batch, cache, out, out_col, out_scale,
                        fuse=None, keep_first=0, gate=None, gate_rows=None, slopes=None, softcap=None):
         """``slopes`` (float32, one per query head) and ``softcap``: a scaled score s becomes softcap * tanh(s / softcap) -
@@ -1105,6 +1113,18 @@ class Kernels:
         if tensor_cores and not batch.is_decode and hasattr(self.attn[dim], "krk_sink_window_prefill"):
             # many tokens per sequence: the tensor-core walk over whole pages
             esz = proj.element_size()
+            if (dim in (64, 128) and not keep_first and self.use_tcgen05_attention
+                    and batch.max_q_len * (heads // cache.kv_heads) >= self.SINK_TCGEN05_ROWS
+                    and min(batch.max_kv_len, int(window or 1 << 30)) >= self.SINK_TCGEN05_KEYS):
+                rc = self.attn[dim].krk_sink_prefill_tcgen05(
+                    optr + out_col * esz, ostride, float(out_scale), ptr + q_col * esz, stride, heads, cache.kv_heads, _ptr(sink),
+                    batch.seq_slot.data_ptr(), batch.seq_start.data_ptr(), batch.seq_qlen.data_ptr(), batch.cu_q.data_ptr(),
+                    cache.table.data_ptr(), cache.width, cache.k.data_ptr(), cache.v.data_ptr(), cache.k.shape[0], batch.n_seqs,
+                    batch.max_q_len, proj.shape[0], float(scale), int(window or 0), None if g_ptr is None else g_ptr + g_col * esz,
+                    g_stride, g_mode, *shape, self.error.data_ptr(), self._stream())
+                if rc != -2:  # -2: rows off 16-byte boundaries, or a scale that is not positive; the kernel below takes them
+                    self._ok(rc, "tcgen05 windowed attention with a sink")
+                    return
             rc = self.attn[dim].krk_sink_window_prefill(
                 optr + out_col * esz, ostride, float(out_scale), ptr + q_col * esz, stride, heads, cache.kv_heads,
                 _ptr(sink), batch.seq_slot.data_ptr(), batch.seq_start.data_ptr(), batch.seq_qlen.data_ptr(),

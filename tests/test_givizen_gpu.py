@@ -306,6 +306,87 @@ EDGES = [  # window, the loud token, total
 ]
 
 
+def attention_in_64_bits(q, k, v, first, scale, window, sink, slopes, cap):
+    T, H, _ = q.shape
+    G = k.shape[1]
+    k, v = (t.repeat_interleave(H // G, 1) for t in (k, v))
+    s = torch.einsum("thd,khd->htk", q, k) * scale
+    if cap:
+        s = cap * torch.tanh(s / cap)
+    gap = (first + torch.arange(T))[:, None] - torch.arange(k.shape[0])
+    if slopes is not None:
+        s = s - slopes[:, None, None] * gap
+    s = s.masked_fill((gap < 0) | (gap >= (window or 1 << 30)), -float("inf"))
+    if sink is not None:
+        s = torch.cat([s, sink[:, None, None].expand(H, T, 1)], -1)
+    return torch.einsum("htk,khd->thd", s.softmax(-1)[..., :k.shape[0]], v)
+
+
+@pytest.mark.parametrize("options", ["sink", "sink+slopes", "slopes+cap+head", "element", "sink+far"])
+@pytest.mark.parametrize("heads,kv_heads,D", [(8, 2, 64), (6, 2, 128), (16, 1, 128), (3, 3, 64)])
+@pytest.mark.parametrize("window", [None, 1, 100, 128, 300])
+def test_prompt_attention_on_the_tcgen05_cores(options, heads, kv_heads, D, window, monkeypatch):
+    """The wide form of the tcgen05 kernel over groups that divide a tile of 128 rows and groups that do not, windows from one key
+    to more than a tile's, unequal sequences (one of a single token, one whose tile is partly filled), a second step
+    that goes on from cached keys; output columns inside a wider row, times a number, times gates; a sink that the first block
+    outgrows by far. No further from 64 bits than the mma.sync kernel is, and both within the output's rounding."""
+    from kernel_rush_kawk_b200.cache import SequenceCache
+    from kernel_rush_kawk_b200.parts.base import KVNeed
+
+    rt = runtime(torch.bfloat16)
+    bf = lambda t: t.to(torch.bfloat16).cuda()
+    steps = [[130, 1, 300], [129, 260, 70]]
+    total = [sum(n) for n in zip(*steps)]
+    W = (heads + 2 * kv_heads) * D
+    gates = heads * D if options == "element" else heads
+    rows = [bf(rand((n, W + gates), 70 + i)) for i, n in enumerate(total)]
+    sink = rand((heads,), 75, 2.0).cuda() if "sink" in options else None
+    if "far" in options:
+        sink -= 60.0
+    slopes = (2.0 ** -torch.arange(1.0, heads + 1)).cuda() if "slopes" in options else None
+    cap = 5.0 if "cap" in options else None
+    gate = (W, "head" if "head" in options else "element") if ("head" in options or options == "element") else None
+    off = {}
+    for tcgen05 in (True, False):
+        cache = SequenceCache([KVNeed(kv_heads, D, window)], 2048, 3, 1024, rt.device, torch.bfloat16, step_tokens=512)
+        slots = [cache.alloc() for _ in total]
+        got, start = [[], [], []], [0, 0, 0]
+        monkeypatch.setattr(type(rt.ops), "SINK_TCGEN05_ROWS", 1)
+        monkeypatch.setattr(type(rt.ops), "SINK_TCGEN05_KEYS", 1 if tcgen05 else 1 << 30)
+        for lens in steps:
+            for slot, a, n in zip(slots, start, lens):
+                cache.reserve(slot, a + n)
+            cache.sync()
+            ctx = context(rt, slots, start, lens, cache)
+            proj = torch.cat([r[a:a + n] for r, a, n in zip(rows, start, lens)]).contiguous()
+            out = torch.zeros((proj.shape[0], heads * D + 16), dtype=torch.bfloat16, device="cuda")
+            freq = torch.zeros(2, device="cuda")
+            rt.ops.rotate_norm_write(proj, 0, heads * D, (heads + kv_heads) * D, heads, kv_heads, D, D, freq, 0, None, ctx.batch,
+                                     cache.view(0))
+            rt.ops.sink_attention(proj, 0, heads, D, D, sink, 0.3, window, ctx.batch, cache.view(0), out, 8, 0.5, gate=gate,
+                                  slopes=slopes, softcap=cap)
+            assert not out[:, :8].any() and not out[:, -8:].any()
+            at = 0
+            for i, (slot, n) in enumerate(zip(slots, lens)):
+                got[i].append(out[at:at + n, 8:-8])
+                cache.advance(slot, n)
+                at += n
+            start = [a + n for a, n in zip(start, lens)]
+        rt.ops.check()
+        err = size = 0.0
+        for i, r in enumerate(rows):
+            d = r.double().cpu()
+            q, k, v = d[:, :heads * D].view(-1, heads, D), d[:, heads * D:(heads + kv_heads) * D].view(-1, kv_heads, D), d[:, (heads + kv_heads) * D:W].view(-1, kv_heads, D)
+            want = 0.5 * attention_in_64_bits(q, k, v, 0, 0.3, window, *(None if t is None else t.double().cpu() for t in (sink, slopes)), cap)
+            if gate is not None:
+                want = want * torch.sigmoid(d[:, W:]).view(d.shape[0], heads, -1)
+            diff = torch.cat(got[i]).double().cpu() - want.reshape(d.shape[0], -1)
+            assert (diff.abs() <= 2.0 ** -8 * want.reshape(d.shape[0], -1).abs() + 1e-4).all(), (tcgen05, i, diff.abs().max())
+            err, size = err + diff.pow(2).sum().item(), size + want.pow(2).sum().item()
+        off[tcgen05] = (err / size) ** 0.5
+    assert off[True] <= 1.05 * off[False] + 1e-5, off
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("kind", ["attention", "attention_2"])
 @pytest.mark.parametrize("D", [16, 12])
