@@ -22,7 +22,7 @@
 //   krk_moe_down_pairs: out[r, c] = add[r, c] + sum_j weight[r, j] * (Wd_e(j)[c] . act[(r, j)]), a warp per c;
 //   the sum over the chosen experts is float32, in the order of the choice.
 //
-// Many rows: pairs are counted per expert and ordered by expert on the device (krk_moe_sort: one block; offsets
+// Many rows: pairs are counted per expert and ordered by expert on the device (krk_moe_sort: a block an expert; offsets
 // and the pairs' places), krk_moe_gather copies the rows into that order, the experts' products run over
 // contiguous rows, and krk_moe_combine adds each row's weighted results onto `add` (without places: results
 // in the pairs' own order). With cap > 0 every expert's
@@ -338,62 +338,43 @@ moe_down_pairs_kernel(T* __restrict__ out, const T* __restrict__ add, const floa
   }
 }
 
-// One block: counts per expert, offsets, each pair's place in the expert order (stable: pairs of one expert keep their
-// order). Every warp owns a run of the pairs and a row of counters; 32 pairs at a time, lanes with one expert find one
-// another and their rank (match), so a warp walks its run twice, once to count and once to place.
-__global__ void moe_sort_kernel(int* __restrict__ offsets, int* __restrict__ place, const int* __restrict__ experts,
-                                int pairs, int E) {
-  extern __shared__ int cnt[];  // [warps][E], then [E + 1]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
-  int* mine = cnt + (size_t)warp * E;
-  int* base = cnt + (size_t)n_warps * E;
-  for (int i = threadIdx.x; i < n_warps * E; i += blockDim.x) cnt[i] = 0;
+// A block per expert: its offset (how many pairs chose an expert of a lower number) and its own pairs' places, in their order.
+// Every block looks through all the pairs, a run a warp: counting one expert's pairs is a ballot of 32, where ordering all experts in
+// one block took a match of 32 numbers each time, which the hardware resolves one distinct number after another (12,288 pairs of
+// 64 experts: 24.5 us; this: 5.6).
+constexpr int SORT_WARPS = 32;
+__global__ void __launch_bounds__(SORT_WARPS * 32)
+moe_sort_kernel(int* __restrict__ offsets, int* __restrict__ place, const int* __restrict__ experts, int pairs, int E) {
+  __shared__ int own[SORT_WARPS], lower[SORT_WARPS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, mine = blockIdx.x;
   grid_dependency_wait();
-  __syncthreads();
-  const int run = ((pairs + n_warps - 1) / n_warps + 31) / 32 * 32;
+  const int run = ((pairs + SORT_WARPS - 1) / SORT_WARPS + 31) / 32 * 32;
   const int lo = warp * run, hi = min(pairs, lo + run);
-  for (int i0 = lo; i0 < hi; i0 += 32) {
-    const int e = i0 + lane < hi ? experts[i0 + lane] : -1;
-    const unsigned same = __match_any_sync(0xffffffffu, e);
-    if (e >= 0 && lane == __ffs(same) - 1) mine[e] += __popc(same);
-    __syncwarp();
+  int n_own = 0, n_lower = 0;
+#pragma unroll 8
+  for (int i = lo; i < hi; i += 32) {
+    const int e = i + lane < hi ? experts[i + lane] : -1;
+    n_own += __popc(__ballot_sync(0xffffffffu, e == mine));
+    n_lower += __popc(__ballot_sync(0xffffffffu, e >= 0 && e < mine));
+  }
+  if (lane == 0) {
+    own[warp] = n_own;
+    lower[warp] = n_lower;
   }
   __syncthreads();
-  // per expert: what the warps before counted; the total goes to base
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    int before = 0;
-    for (int w = 0; w < n_warps; ++w) {
-      const int c = cnt[(size_t)w * E + e];
-      cnt[(size_t)w * E + e] = before;
-      before += c;
-    }
-    base[e] = before;
+  const int o = own[lane], below = __reduce_add_sync(0xffffffffu, lower[lane]);  // lane: a warp of the block
+  int at = below + __reduce_add_sync(0xffffffffu, lane < warp ? o : 0);
+  if (threadIdx.x == 0) offsets[mine] = below;
+  if (mine == E - 1) {
+    const int all = below + __reduce_add_sync(0xffffffffu, o);
+    if (threadIdx.x == 0) offsets[E] = all;
   }
-  __syncthreads();
-  if (warp == 0) {  // totals to offsets
-    int carry = 0;
-    for (int e0 = 0; e0 < E; e0 += 32) {
-      const int c = e0 + lane < E ? base[e0 + lane] : 0;
-      int incl = c;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int p = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += p;
-      }
-      if (e0 + lane < E) base[e0 + lane] = offsets[e0 + lane] = carry + incl - c;
-      carry += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (lane == 0) offsets[E] = carry;
-  }
-  __syncthreads();
-  for (int i0 = lo; i0 < hi; i0 += 32) {
-    const int i = i0 + lane;
-    const int e = i < hi ? experts[i] : -1;
-    const unsigned same = __match_any_sync(0xffffffffu, e);
-    if (e >= 0) place[i] = base[e] + mine[e] + __popc(same & ((1u << lane) - 1u));
-    __syncwarp();
-    if (e >= 0 && lane == __ffs(same) - 1) mine[e] += __popc(same);
-    __syncwarp();
+  if (n_own == 0) return;
+  for (int i = lo; i < hi; i += 32) {
+    const bool is = i + lane < hi && experts[i + lane] == mine;
+    const unsigned same = __ballot_sync(0xffffffffu, is);
+    if (is) place[i + lane] = at + __popc(same & ((1u << lane) - 1u));
+    at += __popc(same);
   }
 }
 
@@ -564,12 +545,8 @@ KRK_API int krk_moe_down_pairs(void* out, const void* add, const float* add_gate
 
 KRK_API int krk_moe_sort(int* offsets, int* place, const int* experts, int rows, int top, int E, cudaStream_t stream) {
   if (rows == 0) return 0;
-  int warps = 32;
-  while (warps > 1 && (size_t)(warps + 1) * E * sizeof(int) > 200 * 1024) warps >>= 1;
-  const size_t smem = (size_t)(warps + 1) * E * sizeof(int);
-  if (smem > 200 * 1024) return -2;
-  if (smem > 48 * 1024) cudaFuncSetAttribute(moe_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  return (int)launch_pdl(moe_sort_kernel, dim3(1), dim3(warps * 32), smem, stream, offsets, place, experts, rows * top, E);
+  if (E < 1 || (long long)rows * top > 0x7fffff00LL) return -2;
+  return (int)launch_pdl(moe_sort_kernel, dim3(E), dim3(SORT_WARPS * 32), 0, stream, offsets, place, experts, rows * top, E);
 }
 
 // in_weights [rows * top] (may be null): with row_weights [rows of xg] they are written there, in row order; without, the

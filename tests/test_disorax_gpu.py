@@ -398,6 +398,25 @@ def test_products_of_few_experts_rows(gated, activation, weigh_input, sizes, row
     assert off[True] < 1e-2, off
 
 
+@pytest.mark.parametrize("rows,top,E", [(1, 1, 1), (40, 3, 7), (1000, 6, 64), (2048, 6, 64), (3000, 8, 33)])
+def test_expert_ordering_is_stable(rows, top, E):
+    """Offsets and places of pairs ordered by expert, pairs of one expert in their own order, choices that are no expert left out:
+    runs of one piece of 32 a warp and of several, warps without pairs."""
+    rt = runtime(torch.bfloat16)
+    g = torch.Generator().manual_seed(rows)
+    experts = torch.randint(-1, E, (rows, top), generator=g).to(torch.int32)
+    offsets, place = torch.zeros(E + 1, dtype=torch.int32, device="cuda"), torch.full((rows * top,), -1, dtype=torch.int32, device="cuda")
+    dev = experts.cuda()
+    assert rt.ops.moe.krk_moe_sort(offsets.data_ptr(), place.data_ptr(), dev.data_ptr(), rows, top, E, rt.ops._stream()) == 0
+    flat = experts.view(-1)
+    counts = torch.bincount(flat[flat >= 0].long(), minlength=E)
+    assert offsets.cpu().tolist() == [0] + torch.cumsum(counts, 0).tolist()
+    order = torch.argsort(flat[flat >= 0], stable=True)
+    want = torch.empty_like(order)
+    want[order] = torch.arange(order.numel())
+    assert torch.equal(place.cpu()[flat >= 0].long(), want) and (place.cpu()[flat < 0] == -1).all()
+
+
 def test_routing_takes_the_lower_index_on_a_tie_and_weighs_by_the_chosen_logits_only():
     rt = runtime(torch.float32)
     x = torch.eye(4, device="cuda")
