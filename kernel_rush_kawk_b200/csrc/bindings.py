@@ -1287,6 +1287,7 @@ class Kernels:
 
     RECURRENCE_CHUNK_MIN = 40  # tokens of a step's longest sequence from which a bfloat16 scan of such mixers may run in chunks
     RECURRENCE_SCRATCH = 256 << 20  # bytes
+    CHUNK_SCRATCH_MOST = 1 << 30    # a step of so many sequences that one chunk of each takes more is scanned token by token
 
     def _recurrence_in_chunks(self, kind, heads, batch) -> bool:
         """Time mixing gains at every size measured from 40 tokens on (one sequence of 40 at 24 heads: 60 -> 55 us a layer's mixer, 16
@@ -1320,6 +1321,8 @@ class Kernels:
                 and self._recurrence_in_chunks(kind, heads, batch)):
             item = c_int(0)
             tokens = self.scan.krk_recurrence_chunk_tokens(rule, dim, lora.shape[1], float(decay_scale), ctypes.byref(item))
+            if 4 * item.value * batch.n_seqs * heads > self.CHUNK_SCRATCH_MOST:
+                tokens = 0
             chunks = -(-batch.max_q_len // tokens) if tokens else 0
             # a long step goes through its chunks in portions, so that the scratch stays within RECURRENCE_SCRATCH
             portion = max(1, min(chunks, self.RECURRENCE_SCRATCH // (4 * item.value * batch.n_seqs * heads)))
@@ -1514,7 +1517,8 @@ class Kernels:
         """The scan in chunks on the tensor cores (csrc/matrix_memory_chunks.cu); False, with nothing done, where rows do not
         start on 16-byte boundaries."""
         (xp, xs), (bp, bs), (cp, cs_), (dp, ds) = views
-        if any(p % 16 or s % 8 for p, s in views[:3]) or state.data_ptr() % 16:
+        if (any(p % 16 or s % 8 for p, s in views[:3]) or state.data_ptr() % 16
+                or 4 * batch.n_seqs * heads * N * P > self.CHUNK_SCRATCH_MOST):
             return False
         rows = y.shape[0]
         steps = torch.empty((rows, heads, 2), dtype=torch.float32, device=y.device)
