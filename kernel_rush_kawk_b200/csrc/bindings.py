@@ -958,9 +958,11 @@ class Kernels:
 
     @staticmethod
     def _few_experts(x, K, F, C, rows, top) -> bool:
-        """Whether the experts' products of few rows run once per expert (csrc/few_experts.cu): type, sizes and alignment."""
+        """Whether the experts' products of few rows run once per expert (csrc/few_experts.cu): type, sizes and alignment, and
+        pairs enough (16 experts of 1,536 x 3,072, two a row: 2 pairs 27.3 us by pair and 30.8 by expert, 4 pairs 41.5 and
+        46.2, 8 pairs 68 and 58; 64 of 2,048 x 1,408, six a row: 6 pairs 54 and 50)."""
         return (x.dtype == torch.bfloat16 and K % 8 == 0 and F % 8 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
-                and rows * top <= 4096)
+                and 6 <= rows * top <= 4096)
 
     @staticmethod
     def _use_grouped(x, K, F, C, gated, activation) -> bool:
@@ -1043,8 +1045,9 @@ class Kernels:
     # Windowed prompts take the tcgen05 kernel from so many rows (tokens times heads of a group) of the longest sequence and so many
     # keys in a row's sight: a block of it walks two tiles of 128 rows through blocks of 128 keys, which pays where the walk is
     # long (a whole mixer of 16/4 heads of 128 with a window of 1,024, mma.sync and tcgen05: one prompt of 256 tokens 31 and 35 us, of
-    # 512 47 and 45, of 1,024 85 and 67; 64 tokens behind 1,400 62 and 56; 12/4 heads: 512 tokens 86 and 90, 1,024 147 and 134)
-    SINK_TCGEN05_ROWS, SINK_TCGEN05_KEYS = 192, 640
+    # 512 47 and 45, of 1,024 85 and 67; 64 tokens behind 1,400 62 and 56; 12/4 heads: 512 tokens 86 and 90, 1,024 147 and 134;
+    # with capped scores two prompts of 700 88 and 93, 700 tokens behind 700 124 and 116)
+    SINK_TCGEN05_ROWS, SINK_TCGEN05_KEYS = 192, 896
 
     def sink_attention(self, proj, q_col, heads, dim, vdim, sink, scale, window, batch, cache, out, out_col, out_scale,
                        fuse=None, keep_first=0, gate=None, gate_rows=None, slopes=None, softcap=None):
@@ -1285,21 +1288,23 @@ class Kernels:
                                           batch.seq_slot.data_ptr(), _code(h.dtype), self._stream(), int(store)), "token shift")
         return out
 
-    RECURRENCE_CHUNK_MIN = 40  # tokens of a step's longest sequence from which a bfloat16 scan of such mixers may run in chunks
+    RECURRENCE_CHUNK_MIN = 160  # tokens of a step's longest sequence from which a bfloat16 scan of such mixers may run in chunks
     RECURRENCE_SCRATCH = 256 << 20  # bytes
     CHUNK_SCRATCH_MOST = 1 << 30    # a step of so many sequences that one chunk of each takes more is scanned token by token
 
     def _recurrence_in_chunks(self, kind, heads, batch) -> bool:
-        """Time mixing gains at every size measured from 40 tokens on (one sequence of 40 at 24 heads: 60 -> 55 us a layer's mixer, 16
-        of 64: 130 -> 95, one of 2,048 and more: several times). The delta rule has more work a chunk: where sequences and
-        heads fill the SMs, the scan token by token keeps up (8 heads, 16 sequences of 128: 145 us against 157; of 64: 85
-        against 95), so the two are estimated from their measured parts: 0.57 us a token for each round of blocks, against 0.18 us a
-        chunk and head, 0.5 us a chunk of the longest sequence and 12 us."""
+        """Where the scan in chunks pays. It takes more launches, and a short step is bound by issuing them from the host, so the
+        lines lie by the time of a whole mixer as it is called. Time mixing, token by token and in chunks: one sequence of
+        200 tokens at 24 heads 188 us and 198, of 350 210 and 197; four of 200 at 40 heads 229 and 206. The delta rule: one
+        sequence of 110 at 8 heads 134 us and 145, of 200 173 and 143. The delta rule has more work a chunk: where sequences
+        and heads fill the SMs, the scan token by token keeps up (8 heads, 16 sequences of 128: 145 us against 157), so the
+        two are also estimated from their measured parts: 0.57 us a token for each round of blocks, against 0.18 us a chunk
+        and head, 0.5 us a chunk of the longest sequence and 12 us."""
         longest = batch.max_q_len
         if longest < self.RECURRENCE_CHUNK_MIN:
             return False
         if kind == "wkv":
-            return True
+            return longest >= (192 if batch.n_seqs * heads > 148 else 320)
         items = heads * sum(-(-n // 32) for n in batch.q_lens)
         return 0.57 * longest * -(-batch.n_seqs * heads // 148) > 12.0 + 0.18 * items + 0.5 * longest / 32
 
@@ -1507,10 +1512,11 @@ class Kernels:
                                         self._stream()), "state-space scan (a head's state must fit a block's registers)")
         return y
 
-    # tokens of a step's longest sequence from which a bfloat16 scan runs in chunks on the tensor cores (48 heads of 64 x 128, a
-    # whole mixer: one sequence of 33 tokens 41.1 us token by token and 43.1 in chunks, of 64 63 and 53, of 255 188 and 70;
-    # 16 sequences of 64 143 and 135)
-    SSD_TENSOR_MIN = 64
+    # tokens of a step's longest sequence from which a bfloat16 scan runs in chunks on the tensor cores. The kernels alone gain
+    # from 64 tokens on, but a short step is bound by the host, which has more launches to issue (48 heads of 64 x 128, a whole
+    # mixer as it is called: one sequence of 110 tokens 123 us by the other scan and 151 in chunks, of 200 161 and 152, of 700
+    # 241 and 154; four of 110 127 and 154, of 200 183 and 155)
+    SSD_TENSOR_MIN = 192
     SSD_SCRATCH = 256 << 20  # bytes of chunk states
 
     def _ssd_chunks(self, views, dt_bias, a_log, skip, heads, P, N, groups, state, batch, y, tokens) -> bool:
