@@ -320,8 +320,9 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
       if constexpr (WIDE) {
         const int head = kh * G + (valid[t] ? R % G : 0);
         if (ex.sink) {
+          // a sink at minus infinity, or so low that it is in log2 units, is none: nothing is summed before the first key
           m[t] = ex.sink[head] * LOG2E;
-          l[t] = half == 0 ? 1.f : 0.f;  // the two halves' sums are added at the end
+          l[t] = half == 0 && m[t] != -INFINITY ? 1.f : 0.f;  // the two halves' sums are added at the end
         }
         if (SHAPED && ex.slopes) slope[t] = ex.slopes[head] * LOG2E;
       }

@@ -387,6 +387,54 @@ def test_prompt_attention_on_the_tcgen05_cores(options, heads, kv_heads, D, wind
     assert off[True] <= 1.05 * off[False] + 1e-5, off
 
 
+def windowed_prompt(rt, qkv, heads, kv_heads, D, window, sink, cache, slot, start, slopes=None):
+    """One step of one sequence: its keys and values into the cache, then the attention of its queries."""
+    n = qkv.shape[0]
+    cache.reserve(slot, start + n)
+    cache.sync()
+    ctx = context(rt, [slot], [start], [n], cache)
+    out = torch.zeros((n, heads * D), dtype=torch.bfloat16, device="cuda")
+    rt.ops.rotate_norm_write(qkv, 0, heads * D, (heads + kv_heads) * D, heads, kv_heads, D, D, torch.zeros(2, device="cuda"), 0, None,
+                             ctx.batch, cache.view(0))
+    rt.ops.sink_attention(qkv, 0, heads, D, D, sink, 0.3, window, ctx.batch, cache.view(0), out, 0, 1.0, slopes=slopes)
+    cache.advance(slot, n)
+    rt.ops.check()
+    return out
+
+
+def split_qkv(qkv, heads, kv_heads, D):
+    d = qkv.double().cpu()
+    return (d[:, :heads * D].view(-1, heads, D), d[:, heads * D:(heads + kv_heads) * D].view(-1, kv_heads, D),
+            d[:, (heads + kv_heads) * D:].view(-1, kv_heads, D))
+
+
+@pytest.mark.parametrize("tcgen05", [True, False])
+@pytest.mark.parametrize("biased", [False, True])
+@pytest.mark.parametrize("D", [64, 128])
+def test_a_sink_that_is_switched_off_counts_nothing(tcgen05, biased, D, monkeypatch):
+    """A head's sink at minus infinity, or at the lowest number of 32 or 16 bits, which is minus infinity in log2 units: its rows
+    are a plain softmax, beside heads whose sink counts. Few keys and equal ones, where one more weight shows most."""
+    from kernel_rush_kawk_b200.cache import SequenceCache
+    from kernel_rush_kawk_b200.parts.base import KVNeed
+
+    rt = runtime(torch.bfloat16)
+    heads, kv_heads, n = 8, 2, 150
+    low = [-float("inf"), torch.finfo(torch.float32).min, torch.finfo(torch.bfloat16).min, -1e4, 0.0, 2.0, -float("inf"), -2.4e38]
+    sink = torch.tensor(low)
+    slopes = 2.0 ** -torch.arange(1.0, heads + 1) if biased else None
+    monkeypatch.setattr(type(rt.ops), "SINK_TCGEN05_ROWS", 1)
+    monkeypatch.setattr(type(rt.ops), "SINK_TCGEN05_KEYS", 1 if tcgen05 else 1 << 30)
+    for loud in (0.0, 1.0):
+        qkv = rand((n, (heads + 2 * kv_heads) * D), 170)
+        qkv[:, :heads * D] *= loud  # without a query all scores are equal
+        qkv = qkv.to(torch.bfloat16).cuda()
+        cache = SequenceCache([KVNeed(kv_heads, D, None)], 1024, 1, 512, rt.device, torch.bfloat16, step_tokens=512)
+        got = windowed_prompt(rt, qkv, heads, kv_heads, D, None, sink.cuda(), cache, cache.alloc(), 0, slopes if slopes is None else slopes.cuda())
+        q, k, v = split_qkv(qkv, heads, kv_heads, D)
+        want = attention_in_64_bits(q, k, v, 0, 0.3, None, sink.double(), slopes if slopes is None else slopes.double(), None).reshape(n, -1)
+        assert ((got.double().cpu() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all(), loud
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("kind", ["attention", "attention_2"])
 @pytest.mark.parametrize("D", [16, 12])
