@@ -28,7 +28,7 @@
 //
 // e^{-c_s} must stay in range. The delta rule's decay is at least e^{-decay_scale} a token, so a chunk's is bounded by the
 // parameter (the caller asks krk_recurrence_chunk_tokens). Time mixing's has no bound: a chunk in which some channel decays by
-// more than e^-80 forms its pair sums from e^{c_{t-1} - c_s} one by one, right for any decay and slower.
+// more than e^-80 forms its pair sums by decaying each key token by token, right for any decay and slower.
 #include "mma.cuh"  // cp.async
 
 namespace {
@@ -38,7 +38,6 @@ constexpr int N = 64;         // channels of a head
 constexpr int PITCH = N + 4;  // rows on 16-byte boundaries; eight neighbouring rows' pieces fall into different banks
 constexpr int THREADS = 128;
 constexpr float SAFE = 80.f;
-constexpr float FORGOTTEN = 120.f;
 constexpr int WALK_COLS = 4;    // value columns a block of pass 2 walks with
 constexpr int WALK_STAGES = 6;  // chunks whose M are on the way, and the one at hand
 
@@ -57,9 +56,9 @@ struct ChunkArgs {
   int H, R;
   const int *cu_q, *seq_qlen, *seq_slot;
   int chunk0, n_chunks;  // the chunks of every sequence that this launch takes
-  float* scratch;        // per (sequence, chunk, head): delta M, G, Q, O_own; time mixing G, summed decays
+  float* scratch;        // per (sequence, chunk, head): delta M, G, Q, O_own; time mixing G, summed decays and, past e^-SAFE, the decays
 };
-constexpr int ITEM_DELTA = 2 * N * N + 2 * L * N, ITEM_MIX = N * N + L * N;
+constexpr int ITEM_DELTA = 2 * N * N + 2 * L * N, ITEM_MIX = N * N + 2 * L * N;
 
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.0f / (1.0f + expf(-z)); }
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -76,41 +75,42 @@ __device__ __forceinline__ float dot4(float4 a, float4 b, float d) {
   return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, d))));
 }
 
-// The chunk's log decays, summed over its tokens, into cs [L][PITCH] (zero decay beyond the last token). A thread takes
-// one channel of half the tokens; `total` is [2][N]. With `rest` (delta rule) what the running sums round off goes
-// there: a sum of 18 rounds at 1e-6, which e^c would multiply everything by. Ends with a barrier.
+// Log decays of a chunk's tokens, a thread one channel of half of them (zero decay beyond the last token).
+constexpr int HALF = L / 2;
 template <int RULE>
-__device__ __forceinline__ void summed_decays(const ChunkArgs& a, float* cs, float* rest, float* total, const float* th_s, int ch0, int nt) {
-  constexpr int HALF = L / 2;
-  const int ch = threadIdx.x & (N - 1), half = threadIdx.x / N, t0 = half * HALF, RP = (a.R + 7) & ~7;
+__device__ __forceinline__ void log_decays(const ChunkArgs& a, float (&x)[HALF], const float* th_s, int ch0, int nt) {
+  const int ch = threadIdx.x & (N - 1), t0 = threadIdx.x / N * HALF, RP = (a.R + 7) & ~7;
   const bf16* w2 = a.w2 + (size_t)(ch0 + ch) * a.R;
-  float z[HALF];
 #pragma unroll
-  for (int t = 0; t < HALF; ++t) z[t] = 0.f;
+  for (int t = 0; t < HALF; ++t) x[t] = 0.f;
   for (int m = 0; m < RP; m += 8) {
     float w[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) w[i] = m + i < a.R ? __bfloat162float(w2[m + i]) : 0.f;
 #pragma unroll
     for (int t = 0; t < HALF; ++t) {
-      const float4 x = ld4(th_s + (t0 + t) * RP + m), y = ld4(th_s + (t0 + t) * RP + m + 4);
-      z[t] = fmaf(x.w, w[3], fmaf(x.z, w[2], fmaf(x.y, w[1], fmaf(x.x, w[0], z[t]))));
-      z[t] = fmaf(y.w, w[7], fmaf(y.z, w[6], fmaf(y.y, w[5], fmaf(y.x, w[4], z[t]))));
+      const float4 p = ld4(th_s + (t0 + t) * RP + m), q = ld4(th_s + (t0 + t) * RP + m + 4);
+      x[t] = fmaf(p.w, w[3], fmaf(p.z, w[2], fmaf(p.y, w[1], fmaf(p.x, w[0], x[t]))));
+      x[t] = fmaf(q.w, w[7], fmaf(q.z, w[6], fmaf(q.y, w[5], fmaf(q.x, w[4], x[t]))));
     }
   }
   const float w0 = a.w0[ch0 + ch];
-  float run = 0.f, lost = 0.f, low[HALF];
+#pragma unroll
+  for (int t = 0; t < HALF; ++t)
+    x[t] = t0 + t >= nt ? 0.f : RULE == 1 ? -a.decay_scale * sigmoid_f(x[t] + w0) : -expf(x[t] + w0);
+}
+
+// Delta rule: the log decays summed over the chunk's tokens, into cs [L][PITCH]; what the running sums round off goes to
+// `rest`: a sum of 18 rounds at 1e-6, which e^c would multiply everything by. `total` is [2][N]. Ends with a barrier.
+__device__ __forceinline__ void summed_decays(const ChunkArgs& a, float* cs, float* rest, float* total, const float* th_s, int ch0, int nt) {
+  const int ch = threadIdx.x & (N - 1), half = threadIdx.x / N, t0 = half * HALF;
+  float z[HALF], low[HALF], run = 0.f, lost = 0.f;
+  log_decays<1>(a, z, th_s, ch0, nt);
 #pragma unroll
   for (int t = 0; t < HALF; ++t) {
-    float x = RULE == 1 ? -a.decay_scale * sigmoid_f(z[t] + w0) : -expf(z[t] + w0);
-    if (x < -FORGOTTEN) x = -FORGOTTEN;  // a decay that is zero in 32 bits either way; -infinity would not add up
-    if (t0 + t >= nt) x = 0.f;
-    const float sum = run + x;
-    if (RULE == 1) {
-      const float y = sum - run;
-      lost += (run - (sum - y)) + (x - y);
-      low[t] = lost;
-    }
+    const float x = z[t], sum = run + x, y = sum - run;
+    lost += (run - (sum - y)) + (x - y);
+    low[t] = lost;
     z[t] = run = sum;
   }
   if (half == 0) {
@@ -118,15 +118,12 @@ __device__ __forceinline__ void summed_decays(const ChunkArgs& a, float* cs, flo
     total[N + ch] = lost;
   }
   __syncthreads();
-  const float before = half ? total[ch] : 0.f, before_low = half && RULE == 1 ? total[N + ch] : 0.f;
+  const float before = half ? total[ch] : 0.f, before_low = half ? total[N + ch] : 0.f;
 #pragma unroll
   for (int t = 0; t < HALF; ++t) {
-    const float sum = before + z[t];
+    const float sum = before + z[t], y = sum - before;
     cs[(t0 + t) * PITCH + ch] = sum;
-    if (RULE == 1) {
-      const float y = sum - before;
-      rest[(t0 + t) * PITCH + ch] = low[t] + before_low + ((before - (sum - y)) + (z[t] - y));
-    }
+    rest[(t0 + t) * PITCH + ch] = low[t] + before_low + ((before - (sum - y)) + (z[t] - y));
   }
   __syncthreads();
 }
@@ -187,7 +184,7 @@ __global__ void __launch_bounds__(THREADS, 3) delta_chunk_kernel(ChunkArgs a) {
     const float sq = warp_sum(x * x + y * y);
     if (lane == 0) inv[t] = rsqrtf(sq + 1e-6f);
   }
-  summed_decays<1>(a, zs, es, es + L * PITCH, th_s, ch0, nt);
+  summed_decays(a, zs, es, es + L * PITCH, th_s, ch0, nt);
   {
     const int ch = tid & 63;
     const float bias = a.rate_bias[ch0 + ch];
@@ -343,12 +340,14 @@ __global__ void __launch_bounds__(THREADS, 3) delta_chunk_kernel(ChunkArgs a) {
 }
 
 // ---- pass 1, time mixing ---------------------------------------------------------------------------------------
+// A thread has its channel's decays in registers, and sums them from either end: the weights e^{c_last - c_s} from the last token
+// back and the running sums c_t from the first one on. Neither is a difference of sums, in which a small decay after
+// large ones would be lost.
 __global__ void __launch_bounds__(THREADS) mix_chunk_kernel(ChunkArgs a) {
   extern __shared__ __align__(16) float sm[];
   float* ks = sm;                // [L][PITCH] k_s e^{c_last - c_s}
   float* vs = ks + L * PITCH;    // [L][PITCH]
-  float* cs = vs + L * PITCH;    // [L][PITCH]
-  float* th_s = cs + L * PITCH;  // [L][R rounded up]
+  float* th_s = vs + L * PITCH;  // [L][R rounded up]
   float* total = th_s + L * ((a.R + 7) & ~7);  // [2][N]
   const int h = blockIdx.x, ci = blockIdx.y, seq = blockIdx.z, ch0 = h * N;
   grid_dependency_wait();
@@ -359,18 +358,35 @@ __global__ void __launch_bounds__(THREADS) mix_chunk_kernel(ChunkArgs a) {
   load_rows(vs, a.v, a.v_stride, row0, ch0, nt);
   load_tanh(a, th_s, row0, nt);
   __syncthreads();
-  summed_decays<0>(a, cs, nullptr, total, th_s, ch0, nt);
-  grid_launch_dependents();
   float* item = a.scratch + (((size_t)seq * a.n_chunks + ci) * a.H + h) * ITEM_MIX;
-  for (int i = threadIdx.x; i < L * (N / 4); i += THREADS) {
-    const int t = i / (N / 4), n = (i % (N / 4)) * 4;
-    const float4 c = ld4(cs + t * PITCH + n), e = ld4(cs + (L - 1) * PITCH + n);
-    st4(item + N * N + t * N + n, c);
-    float4 k = ld4(ks + t * PITCH + n);
-    k.x *= expf(e.x - c.x); k.y *= expf(e.y - c.y); k.z *= expf(e.z - c.z); k.w *= expf(e.w - c.w);
-    st4(ks + t * PITCH + n, k);
+  {
+    const int ch = threadIdx.x & (N - 1), half = threadIdx.x / N, t0 = half * HALF;
+    float x[HALF], run = 0.f;
+    log_decays<0>(a, x, th_s, ch0, nt);
+#pragma unroll
+    for (int t = 0; t < HALF; ++t) run += x[t];
+    total[half * N + ch] = run;
+    __syncthreads();
+    grid_launch_dependents();
+    const float other = total[(half ^ 1) * N + ch];
+    const float before = half ? other : 0.f;
+    float after = half ? 0.f : other, c = before;
+    run = 0.f;
+#pragma unroll
+    for (int t = 0; t < HALF; ++t) {
+      run += x[t];
+      c = before + run;
+      item[N * N + (t0 + t) * N + ch] = c;
+    }
+#pragma unroll
+    for (int t = HALF - 1; t >= 0; --t) {
+      ks[(t0 + t) * PITCH + ch] *= expf(after);
+      after += x[t];
+    }
+    if (__syncthreads_or(half && !(c > -SAFE)))  // pass 3 will form the pair sums from the decays themselves
+#pragma unroll
+      for (int t = 0; t < HALF; ++t) item[N * N + L * N + (t0 + t) * N + ch] = expf(x[t]);
   }
-  __syncthreads();
   const Place at;
   float4 g[8];
 #pragma unroll
@@ -496,7 +512,7 @@ __global__ void __launch_bounds__(THREADS) chunk_finish_kernel(ChunkArgs a) {
   float* red = qs + L * PITCH;    // [4][L] sums of squares of a warp's columns
   float* ks = red + 4 * L;        // time mixing: [L][PITCH] k_s e^{-c_s}
   float* vs = ks + L * PITCH;     // [L][PITCH]
-  float* cs = vs + L * PITCH;     // [L][PITCH], where a channel forgets too much
+  float* cs = vs + L * PITCH;     // [L][PITCH] decays, where a channel forgets too much
   float* ps = cs + L * PITCH;     // [L][L + 4] pair sums
   constexpr int PP = L + 4;
   grid_launch_dependents();
@@ -542,22 +558,33 @@ __global__ void __launch_bounds__(THREADS) chunk_finish_kernel(ChunkArgs a) {
       b[i] = t ? __ldcg(reinterpret_cast<const float4*>(cum + (t - 1) * N + n)) : zero;
     }
     const bool safe = !__syncthreads_or(!(end.x > -SAFE) || !(end.y > -SAFE) || !(end.z > -SAFE) || !(end.w > -SAFE));
-    if (!safe) {  // pair by pair: a token against every fourth one before it
+    if (!safe) {  // a token's key, as the tokens after it find it: a thread a token and a quarter of the channels
+      const float* decays = cum + L * N;
 #pragma unroll
       for (int i = 0; i < EACH; ++i) {
-        const int at4 = (tid / (N / 4) + i * (THREADS / (N / 4))) * PITCH + n;
+        const int t = tid / (N / 4) + i * (THREADS / (N / 4)), at4 = t * PITCH + n;
         st4(qs + at4, q[i]);
         st4(ks + at4, k[i]);
-        st4(cs + at4, c[i]);
+        st4(cs + at4, __ldcg(reinterpret_cast<const float4*>(decays + t * N + n)));
       }
       __syncthreads();
-      const int t = tid >> 2, piece = tid & 3;
-      for (int s = piece; s < L; s += 4) {
+      const int s = tid >> 2, m0 = (tid & 3) * 4;
+      float4 w[N / 16];
+#pragma unroll
+      for (int j = 0; j < N / 16; ++j) w[j] = ld4(ks + s * PITCH + m0 + 16 * j);
+      for (int t = 0; t < L; ++t) {
         float d = 0.f;
+#pragma unroll
+        for (int j = 0; j < N / 16; ++j) d = dot4(ld4(qs + t * PITCH + m0 + 16 * j), w[j], d);
+        d += __shfl_xor_sync(0xffffffffu, d, 1);
+        d += __shfl_xor_sync(0xffffffffu, d, 2);
+        if (m0 == 0 && s != t) ps[t * PP + s] = s < t ? d : 0.f;
         if (s < t)
-          for (int m = 0; m < N; ++m)
-            d += qs[t * PITCH + m] * ks[s * PITCH + m] * expf(cs[(t - 1) * PITCH + m] - cs[s * PITCH + m]);
-        if (s != t) ps[t * PP + s] = d;
+#pragma unroll
+          for (int j = 0; j < N / 16; ++j) {
+            const float4 e = ld4(cs + t * PITCH + m0 + 16 * j);
+            w[j].x *= e.x; w[j].y *= e.y; w[j].z *= e.z; w[j].w *= e.w;
+          }
       }
       __syncthreads();
     }
@@ -712,7 +739,7 @@ KRK_API int krk_recurrence_chunks(int rule, const void* r, int r_stride, const v
     if ((rc = run(delta_walk_kernel, dim3(N / WALK_COLS, (unsigned)H, (unsigned)n_seqs), THREADS, walk, a, stream))) return rc;
     return run(chunk_finish_kernel<1>, items, THREADS, (size_t)L * PITCH + 4 * L, a, stream);
   }
-  if ((rc = run(mix_chunk_kernel, items, THREADS, 3 * (size_t)L * PITCH + L * RP + 2 * N, a, stream))) return rc;
+  if ((rc = run(mix_chunk_kernel, items, THREADS, 2 * (size_t)L * PITCH + L * RP + 2 * N, a, stream))) return rc;
   if ((rc = run(mix_walk_kernel, dim3(N * N / 4 / 64, (unsigned)H, (unsigned)n_seqs), 64, 0, a, stream))) return rc;
   return run(chunk_finish_kernel<0>, items, THREADS, 4 * (size_t)L * PITCH + 4 * L + (size_t)L * (L + 4), a, stream);
 }

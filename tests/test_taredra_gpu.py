@@ -372,6 +372,45 @@ def test_scans_in_chunks(kind, lens, decays, monkeypatch):
     assert off["chunks"] < 2 * off["tokens"] + 1e-7, off
 
 
+def turning_decays(case, heads):
+    """Rows whose decays change within a chunk of 32 tokens, made by the one low-rank row: e^-e^z with z what ``lora`` says."""
+    lens = [224, 97]
+    rows, HN = sum(lens), heads * 64
+    x = scan_inputs("wkv", lens, heads, "mild", 160)
+    z = {"strong then slow": [(5.0, 8), (1e-3, 24)], "resets": [(60.0, 1), (1e-4, 31)], "forgets all, then slow": [(120.0, 16), (1e-3, 16)],
+         "slow then strong": [(1e-3, 24), (5.0, 8)], "turns within a half": [(3.0, 5), (1e-2, 6), (30.0, 2), (1e-3, 19)]}[case]
+    steps = torch.cat([torch.full((n,), f) for f, n in z]).log()
+    steps = steps.repeat(rows // 32 + 1)[:rows]
+    # tanh(lora) is one bfloat16 number a token; w2 and w0 spread it over -10 .. 5
+    x["lora"] = torch.zeros((rows, 16), device="cuda")
+    x["lora"][:, 0] = torch.atanh(((steps + 2.0) / 8.0).clamp(-0.99, 0.99)).cuda()
+    x["lora"] = x["lora"].to(torch.bfloat16)
+    x["w2"] = torch.zeros((HN, 16), dtype=torch.bfloat16, device="cuda")
+    x["w2"][:, 0] = 8.0
+    x["w0"] = torch.full((HN,), -2.0, device="cuda")
+    return x, lens
+
+
+@pytest.mark.parametrize("case", ["strong then slow", "resets", "forgets all, then slow", "slow then strong", "turns within a half"])
+def test_decays_that_change_within_a_chunk(case, monkeypatch):
+    """Time mixing whose channels forget and then keep, or keep and then forget, inside a chunk: what small decays do after large ones
+    must not be lost in a sum. The 32-bit state no further from 64 bits than twice the scan token by token (and 1e-7, a
+    rounding or two), the outputs within a bfloat16 rounding."""
+    rt = runtime(torch.bfloat16)
+    heads = 3
+    x, lens = turning_decays(case, heads)
+    start = rand((len(lens), heads, 64, 64), 170).cuda()
+    want, want_state = scan_in_64_bits("wkv", x, lens, heads, start)
+    size, off = want.pow(2).mean().sqrt(), {}
+    for name, in_chunks in (("tokens", False), ("chunks", True)):
+        monkeypatch.setattr(type(rt.ops), "_recurrence_in_chunks", lambda *_, yes=in_chunks: yes)
+        state = start.clone()
+        got = run_scan(rt, "wkv", x, lens, heads, state)
+        assert ((got.double().cpu() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-3 * size).all(), name
+        off[name] = ((state.double().cpu() - want_state).norm() / want_state.norm()).item()
+    assert off["chunks"] <= 2 * off["tokens"] + 1e-7, off
+
+
 @pytest.mark.parametrize("kind", ["delta", "wkv"])
 def test_a_tokens_infinities_reach_no_earlier_token(kind, monkeypatch):
     """An infinite value in the middle of a chunk: the tokens before it and the value channels beside it are untouched."""
