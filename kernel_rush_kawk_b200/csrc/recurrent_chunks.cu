@@ -28,7 +28,7 @@
 //
 // e^{-c_s} must stay in range. The delta rule's decay is at least e^{-decay_scale} a token, so a chunk's is bounded by the
 // parameter (the caller asks krk_recurrence_chunk_tokens). Time mixing's has no bound: a chunk in which some channel decays by
-// more than e^-80 forms its pair sums by decaying each key token by token, right for any decay and slower.
+// more than e^-40 forms its pair sums by decaying each key token by token, right for any decay and slower.
 #include "mma.cuh"  // cp.async
 
 namespace {
@@ -37,7 +37,7 @@ constexpr int L = 32;         // tokens per chunk
 constexpr int N = 64;         // channels of a head
 constexpr int PITCH = N + 4;  // rows on 16-byte boundaries; eight neighbouring rows' pieces fall into different banks
 constexpr int THREADS = 128;
-constexpr float SAFE = 80.f;
+constexpr float SAFE = 40.f;  // keys up to 1e21 stay finite times e^SAFE
 constexpr int WALK_COLS = 4;    // value columns a block of pass 2 walks with
 constexpr int WALK_STAGES = 6;  // chunks whose M are on the way, and the one at hand
 

@@ -2,6 +2,7 @@
 tests/plain_taredra.py, then the model through the engine: whole prompts, portions, single
 tokens, unequal batches, reused slots, windows' edges, long decoding, greedy generation."""
 
+import math
 from types import SimpleNamespace
 
 import pytest
@@ -406,6 +407,33 @@ def test_decays_that_change_within_a_chunk(case, monkeypatch):
         monkeypatch.setattr(type(rt.ops), "_recurrence_in_chunks", lambda *_, yes=in_chunks: yes)
         state = start.clone()
         got = run_scan(rt, "wkv", x, lens, heads, state)
+        assert ((got.double().cpu() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-3 * size).all(), name
+        off[name] = ((state.double().cpu() - want_state).norm() / want_state.norm()).item()
+    assert off["chunks"] <= 2 * off["tokens"] + 1e-7, off
+
+
+@pytest.mark.parametrize("total", [38.0, 42.0, 60.0, 79.0])
+def test_large_keys_in_channels_that_forget_much(total, monkeypatch):
+    """Time mixing whose channels decay by e^-total in a chunk's first token and hardly after it, with keys of 30,000 in two of
+    them: finite inputs, finite results, though e^total times such a key may not be."""
+    rt = runtime(torch.bfloat16)
+    heads, lens = 2, [96]
+    x = scan_inputs("wkv", lens, heads, "mild", 190)
+    once = torch.zeros(96, 16, device="cuda")
+    once[::32, 0] = 10.0  # tanh = 1
+    x["lora"], x["w2"] = once.to(torch.bfloat16), torch.zeros((heads * 64, 16), dtype=torch.bfloat16, device="cuda")
+    x["w2"][:, 0] = 8.0
+    x["w0"].fill_(math.log(total) - 8.0)
+    x["k"][:, 7] = 30000.0
+    x["k"][:, 64 + 9] = -30000.0
+    start = rand((1, heads, 64, 64), 191).cuda()
+    want, want_state = scan_in_64_bits("wkv", x, lens, heads, start)
+    off = {}
+    for name, in_chunks in (("tokens", False), ("chunks", True)):
+        monkeypatch.setattr(type(rt.ops), "_recurrence_in_chunks", lambda *_, yes=in_chunks: yes)
+        state = start.clone()
+        got = run_scan(rt, "wkv", x, lens, heads, state)
+        size = want.pow(2).mean().sqrt()
         assert ((got.double().cpu() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-3 * size).all(), name
         off[name] = ((state.double().cpu() - want_state).norm() / want_state.norm()).item()
     assert off["chunks"] <= 2 * off["tokens"] + 1e-7, off
