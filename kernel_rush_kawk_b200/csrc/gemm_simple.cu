@@ -319,8 +319,11 @@ int launch_tile(float* C, const float* A, const float* W, int M, int N, int K, i
 
 template <int RPT, int CPT>
 int launch_few(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
-  const size_t smem = (size_t)FEW_DEPTH * (16 * CPT + M) * FEW_PITCH * sizeof(float);  // 54 to 152 KB
-  cudaFuncSetAttribute(gemm_f32_few_kernel<RPT, CPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  constexpr size_t per_row = (size_t)FEW_DEPTH * FEW_PITCH * sizeof(float);
+  const size_t smem = (16 * CPT + M) * per_row;  // 54 to 152 KB
+  // always the most that a call may need: another thread may be about to launch with more rows than this one
+  cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<RPT, CPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((16 * CPT + 8 * RPT) * per_row));
+  if (e != cudaSuccess) return (int)e;
   gemm_f32_few_kernel<RPT, CPT><<<(N + 16 * CPT - 1) / (16 * CPT), 128, smem, stream>>>(C, A, W, M, N, K, lda, ldw, ldc);
   KRK_CHECK_LAUNCH();
   return 0;

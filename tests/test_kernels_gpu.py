@@ -5,6 +5,7 @@ whose score stands out, a window's edge, pages scattered over the pool."""
 
 import math
 import random
+import threading
 from types import SimpleNamespace
 
 import pytest
@@ -110,6 +111,30 @@ def test_float32_products_sum_in_one_order_whatever_the_rows(ops, nk):
     wide = torch.zeros((40, 2 * k), device="cuda")
     wide[:, :k] = x[:40]
     assert torch.equal(ops.linear(wide[:, :k], w), want[:40]), "rows of a wider buffer"
+
+
+def test_float32_products_of_several_threads(ops):
+    """Threads whose products have one row, eight and sixteen: a launch's shared memory depends on the rows, and no call may lower
+    what another is about to launch with. Straight through the library, which other threads enter while one is in it."""
+    w = rand((64, 2560), torch.float32, 81)
+    xs = {m: rand((m, 2560), torch.float32, 82) for m in (1, 8, 9, 16)}
+    want, outs, failed = {m: ops.linear(x, w) for m, x in xs.items()}, {}, []
+
+    def work(i, m):
+        out = outs[i] = torch.zeros((m, 64), device="cuda")
+        args = (out.data_ptr(), xs[m].data_ptr(), w.data_ptr(), m, 64, 2560, 2560, 2560, 64, 0, 0, torch.cuda.current_stream().cuda_stream)
+        codes = {ops.core.krk_gemm_nt(*args) for _ in range(4000)}
+        if codes != {0}:
+            failed.append((m, codes))
+
+    threads = [threading.Thread(target=work, args=(i, m)) for i, m in enumerate((1, 8, 9, 16, 1, 8))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not failed, failed
+    assert all(torch.equal(out, want[out.shape[0]]) for out in outs.values())
 
 
 @pytest.mark.parametrize("mnk", [(1, 2560, 9728), (8, 2560, 4096), (16, 2560, 9728), (13, 1000, 2080), (3, 48, 2048),
