@@ -900,7 +900,7 @@ class Kernels:
         single = batch is not None and batch.is_decode  # such a step may be replayed from a graph: nothing comes to the host
         if single or rows * top <= max(self.MOE_PAIR_ROWS * top, 2 * E):
             pairs = torch.empty((rows * top, F), dtype=x.dtype, device=x.device)
-            if self._few_experts(x, K, F, C, rows, top):
+            if self._few_experts(x, w_gate_up, w_down, rows, top):
                 # bfloat16: an expert's weights meet all its rows at once; the pairs' results are added up by their rows
                 self._ok(self.moe.krk_few_experts(pairs.data_ptr(), ptr, stride, w_gate_up.data_ptr(), experts.data_ptr(), rows, top,
                                                   E, F, K, int(not gated), act, _ptr(w_in), float(limit), float(slope),
@@ -957,12 +957,13 @@ class Kernels:
         return out
 
     @staticmethod
-    def _few_experts(x, K, F, C, rows, top) -> bool:
-        """Whether the experts' products of few rows run once per expert (csrc/few_experts.cu): type, sizes and alignment, and
-        pairs enough (16 experts of 1,536 x 3,072, two a row: 2 pairs 27.3 us by pair and 30.8 by expert, 4 pairs 41.5 and
-        46.2, 8 pairs 68 and 58; 64 of 2,048 x 1,408, six a row: 6 pairs 54 and 50)."""
-        return (x.dtype == torch.bfloat16 and K % 8 == 0 and F % 8 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
-                and 6 <= rows * top <= 4096)
+    def _few_experts(x, w_first, w_down, rows, top) -> bool:
+        """Whether the experts' products of few rows run once per expert (csrc/few_experts.cu): type, sizes, the alignment of rows
+        and weights, choices that the sum by rows holds, and pairs enough (16 experts of 1,536 x 3,072, two a row: 2 pairs
+        27.3 us by pair and 30.8 by expert, 4 pairs 41.5 and 46.2, 8 pairs 68 and 58; 64 of 2,048 x 1,408, six a row: 6 pairs
+        54 and 50)."""
+        return (x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and w_down.shape[2] % 8 == 0 and x.stride(0) % 8 == 0
+                and (x.data_ptr() | w_first.data_ptr() | w_down.data_ptr()) % 16 == 0 and top <= 32 and 6 <= rows * top <= 4096)
 
     @staticmethod
     def _use_grouped(x, K, F, C, gated, activation) -> bool:

@@ -398,6 +398,32 @@ def test_products_of_few_experts_rows(gated, activation, weigh_input, sizes, row
     assert off[True] < 1e-2, off
 
 
+@pytest.mark.parametrize("odd", ["first", "second", "choices"])
+def test_few_experts_rows_with_weights_off_a_16_byte_boundary_or_many_choices(odd):
+    """What the product per expert does not take goes to the kernels that read an expert per pair: weights that start at an
+    odd element, and more choices a row than the sum by rows holds."""
+    rt = runtime(torch.bfloat16)
+    K, F, C, E, rows, top = 64, 48, 40, 40, 6, 36 if odd == "choices" else 3
+    g = torch.Generator().manual_seed(3)
+
+    def weight(shape, seed, off):
+        flat = torch.zeros(shape[0] * shape[1] * shape[2] + 1, dtype=torch.bfloat16, device="cuda")
+        flat[1:] = rand(shape, seed, 0.2).flatten()
+        return (flat[1:] if off else flat[1:].clone()).view(shape)
+
+    w1, w2 = weight((E, 2 * F, K), 2, odd == "first"), weight((E, C, F), 3, odd == "second")
+    x = rand((rows, K), 1).to(torch.bfloat16).cuda()
+    experts = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(rows)]).to(torch.int32)
+    weights = rand((rows, top), 5).abs().cuda()
+    got = rt.ops.moe_experts(x, w1, w2, experts.cuda(), weights, F, "silu", batch=SimpleNamespace(is_decode=True))
+    want = torch.zeros((rows, C), dtype=torch.float64)
+    for r in range(rows):
+        for j in range(top):
+            z = w1[experts[r, j]].double().cpu() @ x[r].double().cpu()
+            want[r] += weights[r, j].item() * (w2[experts[r, j]].double().cpu() @ (torch.nn.functional.silu(z[:F]) * z[F:]))
+    close(got, want, torch.bfloat16, f"experts, odd {odd}")
+
+
 @pytest.mark.parametrize("rows,top,E", [(1, 1, 1), (40, 3, 7), (1000, 6, 64), (2048, 6, 64), (3000, 8, 33)])
 def test_expert_ordering_is_stable(rows, top, E):
     """Offsets and places of pairs ordered by expert, pairs of one expert in their own order, choices that are no expert left out:
