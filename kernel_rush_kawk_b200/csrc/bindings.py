@@ -1293,6 +1293,17 @@ class Kernels:
     RECURRENCE_SCRATCH = 256 << 20  # bytes
     CHUNK_SCRATCH_MOST = 1 << 30    # a step of so many sequences that one chunk of each takes more is scanned token by token
 
+    @staticmethod
+    def _chunk_scratch(floats, chunks, device, beside=0):
+        """(float32 scratch, chunks that it holds): ``floats`` for a chunk of every sequence, up to ``chunks`` of them at a time,
+        and ``beside`` more; fewer chunks where the device's memory has no room, and (None, 0) where not one fits."""
+        while chunks:
+            try:
+                return torch.empty(chunks * floats + beside, dtype=torch.float32, device=device), chunks
+            except torch.OutOfMemoryError:
+                chunks //= 2
+        return None, 0
+
     def _recurrence_in_chunks(self, kind, heads, batch) -> bool:
         """Where the scan in chunks pays. It takes more launches, and a short step is bound by issuing them from the host, so the
         lines lie by the time of a whole mixer as it is called. Time mixing, token by token and in chunks: one sequence of
@@ -1327,14 +1338,12 @@ class Kernels:
                 and self._recurrence_in_chunks(kind, heads, batch)):
             item = c_int(0)
             tokens = self.scan.krk_recurrence_chunk_tokens(rule, dim, lora.shape[1], float(decay_scale), ctypes.byref(item))
-            if 4 * item.value * batch.n_seqs * heads > self.CHUNK_SCRATCH_MOST:
-                tokens = 0
-            chunks = -(-batch.max_q_len // tokens) if tokens else 0
+            floats = item.value * batch.n_seqs * heads
+            chunks = -(-batch.max_q_len // tokens) if tokens and 4 * floats <= self.CHUNK_SCRATCH_MOST else 0
             # a long step goes through its chunks in portions, so that the scratch stays within RECURRENCE_SCRATCH
-            portion = max(1, min(chunks, self.RECURRENCE_SCRATCH // (4 * item.value * batch.n_seqs * heads)))
-            scratch = torch.empty(portion * batch.n_seqs * heads * item.value if tokens else 0, dtype=torch.float32, device=r.device)
-            rc = 0 if tokens else -2
-            for first in range(0, chunks, portion):
+            scratch, portion = self._chunk_scratch(floats, min(chunks, max(1, self.RECURRENCE_SCRATCH // (4 * floats))), r.device)
+            rc = 0 if portion else -2
+            for first in range(0, chunks, portion) if portion else ():
                 rc = self.scan.krk_recurrence_chunks(
                     rule, *views[0], *views[1], *views[2], *views[3], *rate_v, *lora_v, w2.data_ptr(), w0.data_ptr(),
                     _ptr(rate_bias), _ptr(bonus), norm_w.data_ptr(), state.data_ptr(), last_ptr, last_stride, C,
@@ -1522,24 +1531,27 @@ class Kernels:
 
     def _ssd_chunks(self, views, dt_bias, a_log, skip, heads, P, N, groups, state, batch, y, tokens) -> bool:
         """The scan in chunks on the tensor cores (csrc/matrix_memory_chunks.cu); False, with nothing done, where rows do not
-        start on 16-byte boundaries."""
+        start on 16-byte boundaries or the device's memory has no room for the chunks' states."""
         (xp, xs), (bp, bs), (cp, cs_), (dp, ds) = views
         if (any(p % 16 or s % 8 for p, s in views[:3]) or state.data_ptr() % 16
                 or 4 * batch.n_seqs * heads * N * P > self.CHUNK_SCRATCH_MOST):
             return False
         rows = y.shape[0]
-        steps = torch.empty((rows, heads, 2), dtype=torch.float32, device=y.device)
-        self._ok(self.memory.krk_ssd_steps(steps.data_ptr(), dp, ds, dt_bias.data_ptr(), a_log.data_ptr(), rows, heads,
-                                           self._stream()), "step sizes and decays")
-        chunks = -(-batch.max_q_len // tokens)
+        chunks, state_floats = -(-batch.max_q_len // tokens), batch.n_seqs * heads * N * P
         # a long step goes through its chunks in portions, so that their states stay within SSD_SCRATCH
-        portion = max(1, min(chunks, 65535 // heads, self.SSD_SCRATCH // (4 * batch.n_seqs * heads * N * P)))
-        items = portion * batch.n_seqs * heads
-        sums = torch.empty((items, N * P), dtype=torch.float32, device=y.device)
-        decays = torch.empty((items, N), dtype=torch.float32, device=y.device)
+        portion = max(1, min(chunks, 65535 // heads, self.SSD_SCRATCH // (4 * state_floats)))
+        # the chunks' states, a decay for each of their rows, and every row's step sizes and log decays
+        scratch, portion = self._chunk_scratch(state_floats + batch.n_seqs * heads * N, portion, y.device, beside=2 * rows * heads)
+        if not portion:
+            return False
+        sums = scratch.data_ptr()
+        decays = sums + 4 * portion * state_floats
+        steps = decays + 4 * portion * batch.n_seqs * heads * N
+        self._ok(self.memory.krk_ssd_steps(steps, dp, ds, dt_bias.data_ptr(), a_log.data_ptr(), rows, heads, self._stream()),
+                 "step sizes and decays")
         for first in range(0, chunks, portion):
-            self._ok(self.memory.krk_ssd_chunks(y.data_ptr(), xp, xs, bp, bs, cp, cs_, steps.data_ptr(), skip.data_ptr(),
-                                                state.data_ptr(), sums.data_ptr(), decays.data_ptr(), heads, P, N, groups,
+            self._ok(self.memory.krk_ssd_chunks(y.data_ptr(), xp, xs, bp, bs, cp, cs_, steps, skip.data_ptr(),
+                                                state.data_ptr(), sums, decays, heads, P, N, groups,
                                                 batch.n_seqs, first, min(portion, chunks - first), batch.cu_q.data_ptr(),
                                                 batch.seq_qlen.data_ptr(), batch.seq_slot.data_ptr(), self._stream()),
                      "state-space scan in chunks")

@@ -456,6 +456,35 @@ def test_a_tokens_infinities_reach_no_earlier_token(kind, monkeypatch):
     assert torch.equal(states[1][0, :, :, rest], states[0][0, :, :, rest]) and not torch.isfinite(states[1][0, 0, :, 5]).any()
 
 
+@pytest.mark.parametrize("kind", ["delta", "wkv"])
+def test_a_scan_without_room_for_its_scratch(kind, monkeypatch):
+    """Where the device's memory has no room for the chunks' scratch, a step goes through in smaller portions, and token by token
+    where not even one chunk of each sequence fits: it needed no scratch before it had chunks."""
+    rt = runtime(torch.bfloat16)
+    heads, lens = 3, [200, 65]
+    monkeypatch.setattr(type(rt.ops), "_recurrence_in_chunks", lambda *_: True)
+    x = scan_inputs(kind, lens, heads, "mild", 60)
+    start = rand((len(lens), heads, 64, 64), 70).cuda()
+    runs = {}
+    empty = torch.empty
+    for room in (1 << 30, 1 << 20, 0):
+        def limited(*shape, room=room, **kw):
+            n = math.prod(shape[0]) if isinstance(shape[0], (tuple, list)) else math.prod(shape)
+            if kw.get("dtype") is torch.float32 and 4 * n > room:
+                raise torch.OutOfMemoryError("no room")
+            return empty(*shape, **kw)
+
+        monkeypatch.setattr(torch, "empty", limited)
+        state = start.clone()
+        runs[room] = run_scan(rt, kind, x, lens, heads, state), state
+        monkeypatch.setattr(torch, "empty", empty)
+    monkeypatch.setattr(type(rt.ops), "_recurrence_in_chunks", lambda *_: False)
+    state = start.clone()
+    tokens = run_scan(rt, kind, x, lens, heads, state)
+    assert torch.equal(runs[1 << 20][0], runs[1 << 30][0]) and torch.equal(runs[1 << 20][1], runs[1 << 30][1])
+    assert torch.equal(runs[0][0], tokens) and torch.equal(runs[0][1], state)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_parallel_mixer_alone(dtype):
     """Two branches on one input: one stacked input product, one output product over both branches' columns."""

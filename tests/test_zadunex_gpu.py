@@ -4,6 +4,7 @@ unequal batches, reused slots, far tokens, long decoding, greedy generation and 
 
 import io
 import json
+import math
 from types import SimpleNamespace
 
 import pytest
@@ -273,6 +274,37 @@ def test_a_tokens_infinities_reach_no_earlier_token_of_a_state_space_chunk(monke
     rest = [c for c in range(H * P) if c != 5]
     assert torch.equal(y0[:41], y1[:41]) and torch.equal(y0[:, rest], y1[:, rest]) and not torch.isfinite(y1[41:, 5]).any()
     assert torch.equal(s0[0, 1], s1[0, 1]) and not torch.isfinite(s1[0, 0, :, 5]).any()
+
+
+def test_a_state_space_scan_without_room_for_its_scratch(monkeypatch):
+    """Where the device's memory has no room for the chunks' states, a prompt goes through in smaller portions, and by the other
+    scan where not even one chunk of each sequence fits."""
+    rt = runtime(torch.bfloat16)
+    H, P, N, lens = 4, 64, 128, [240, 70]  # shorter than the other scan's own chunks
+    rows = sum(lens)
+    x, B, C = (rand((rows, n), 40 + i).to(torch.bfloat16).cuda() for i, n in enumerate((H * P, N, N)))
+    dt, vec = rand((rows, H), 43).to(torch.bfloat16).cuda(), rand((H,), 44).cuda()
+    start = rand((2, H, N, P), 45).cuda()
+    ctx = context(rt, [0, 1], [0, 0], lens, None)
+    monkeypatch.setattr(type(rt.ops), "SSD_TENSOR_MIN", 1)
+    empty, runs = torch.empty, {}
+    item = 4 * 2 * H * N * P  # bytes of one chunk's states
+    for name, room in (("all", 1 << 30), ("two chunks", 3 * item), ("none", item - 1)):
+        def limited(*shape, room=room, **kw):
+            n = math.prod(shape[0]) if isinstance(shape[0], (tuple, list)) else math.prod(shape)
+            if kw.get("dtype") is torch.float32 and 4 * n > room and n != rows * H * P:  # the outputs are always there
+                raise torch.OutOfMemoryError("no room")
+            return empty(*shape, **kw)
+
+        monkeypatch.setattr(torch, "empty", limited)
+        state = start.clone()
+        runs[name] = rt.ops.ssd_scan(x, B, C, dt, vec, vec, vec, H, P, N, 1, state, ctx.batch), state
+        monkeypatch.setattr(torch, "empty", empty)
+    monkeypatch.setattr(type(rt.ops), "SSD_TENSOR_MIN", 1 << 30)
+    state = start.clone()
+    runs["tokens"] = rt.ops.ssd_scan(x, B, C, dt, vec, vec, vec, H, P, N, 1, state, ctx.batch), state
+    for a, b in (("two chunks", "all"), ("none", "tokens")):
+        assert torch.equal(runs[a][0], runs[b][0]) and torch.equal(runs[a][1], runs[b][1]), a
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
