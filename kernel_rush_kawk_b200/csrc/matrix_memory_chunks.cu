@@ -788,7 +788,9 @@ __global__ void chunk_decays_kernel(float* __restrict__ cum, const bf16* __restr
   }
 }
 
-// state-space kind: dt = softplus(raw + bias), log decay -exp(A_log) dt
+// state-space kind: dt = softplus(raw + bias), log decay -exp(A_log) dt. Not below FORGOTTEN, whose e^ is zero in 32 bits: sums of
+// minus infinity have no difference, and even 64 bits would lose a later token's decay beside a number that is large enough.
+constexpr float FORGOTTEN = -120.f;
 __global__ void steps_kernel(float2* __restrict__ steps, const bf16* __restrict__ dt, int dt_stride, const float* __restrict__ bias,
                              const float* __restrict__ a_log, int rows, int H) {
   grid_launch_dependents();
@@ -798,7 +800,8 @@ __global__ void steps_kernel(float2* __restrict__ steps, const bf16* __restrict_
   const int r = i / H, h = i % H;
   const float z = __bfloat162float(dt[(size_t)r * dt_stride + h]) + bias[h];
   const float d = z > 20.f ? z : log1pf(expf(z));
-  steps[i] = make_float2(-expf(a_log[h]) * d, d);
+  const float f = -expf(a_log[h]) * d;
+  steps[i] = make_float2(f < FORGOTTEN ? FORGOTTEN : f, d);  // a NaN stays one
 }
 
 size_t sum_smem(int N) { return (3 * (size_t)L * (N + 8) + (size_t)L * VPITCH) * sizeof(bf16); }

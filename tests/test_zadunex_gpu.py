@@ -307,6 +307,28 @@ def test_a_state_space_scan_without_room_for_its_scratch(monkeypatch):
         assert torch.equal(runs[a][0], runs[b][0]) and torch.equal(runs[a][1], runs[b][1]), a
 
 
+def test_state_space_heads_that_forget_everything(monkeypatch):
+    """Rates whose log decay is minus infinity in 32 bits (and so large that a sum of 64 bits would lose a later token's): a decay of
+    zero, as the scan token by token has it, with step sizes that leave single tokens almost undecayed."""
+    rt = runtime(torch.bfloat16)
+    H, P, N, lens = 4, 64, 32, [150, 40]
+    rows = sum(lens)
+    x, B, C = (rand((rows, n), 40 + i).to(torch.bfloat16).cuda() for i, n in enumerate((H * P, N, N)))
+    dt, vec = rand((rows, H), 43).to(torch.bfloat16).cuda(), rand((H,), 44).cuda()
+    dt[::3] = -60.0
+    bias, a_log = torch.zeros(H, device="cuda"), torch.tensor([100.0, 88.0, 57.0, 0.0], device="cuda")
+    start = rand((2, H, N, P), 45).cuda()
+    ctx = context(rt, [0, 1], [0, 0], lens, None)
+    runs = []
+    for least in (1, 1 << 30):
+        monkeypatch.setattr(type(rt.ops), "SSD_TENSOR_MIN", least)
+        state = start.clone()
+        runs.append((rt.ops.ssd_scan(x, B, C, dt, bias, a_log, vec, H, P, N, 1, state, ctx.batch), state))
+    for got, want in zip(*runs):
+        assert torch.isfinite(want).all()
+        assert ((got - want).double().norm() / want.double().norm()).item() < 2e-6
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_a_state_carries_one_loud_token_over_hundreds(dtype):
     """A head whose decay is almost one keeps a token that came hundreds of tokens (and several chunks and
