@@ -127,7 +127,7 @@ _SCAN_SIGNATURES = {
     "krk_recurrence_chunks": [c_int, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, _P, _P, _P, _P, _P, _P,
                               c_int, c_int, _P, _P, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_int, _P, _P, _P,
                               c_int, c_int, _P, _P],
-    "krk_causal_conv_silu": [_P, _P, c_int, _P, _P, _P, c_int, c_int, c_int, c_int, _P, _P, _P, _P, c_int, _P],
+    "krk_causal_conv_silu": [_P, _P, c_int, _P, _P, _P, c_int, c_int, c_int, c_int, _P, _P, _P, _P, c_int, _P, c_int],
     "krk_ssd_scan": [_P, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int,
                      c_int, _P, _P, _P, c_int, _P, _P, c_int, _P],
     "krk_gated_group_norm": [_P, c_int, c_int, c_float, _P, _P, c_int, _P, c_int, c_int, c_int, c_float, c_int, _P],
@@ -1477,6 +1477,16 @@ class Kernels:
     # -- state-space mixer ------------------------------------------------------------------
     SSD_CHUNK = 128  # tokens per chunk where one sequence's step is long enough to be scanned in chunks
 
+    CONV_WALK_BYTES = 12_000_000
+
+    def _conv_walks(self, rows, row_bytes, n_seqs) -> bool:
+        """Whether threads of the short convolution go through sixteen rows each, the rows before in registers. That is one chain of
+        13 us at least (bfloat16; 9 in 32-bit), at a sequence's first row with the loads of its stored rows in it, and pays by
+        bytes: a block a row and sixteen rows a thread, one prompt of 4,096 channels, 256 rows 6.2 and 13.5 us, 1,024 14.2 and
+        17.0, 1,536 18.6 and 17.6, 2,048 23.0 and 18.1; of 1,792 channels 2,048 rows 13.4 and 17.0, 4,096 21.7 and 18.0; 32-bit of
+        4,096 channels 512 rows 9.4 and 10.3, 768 12.5 and 11.8. Single tokens of 64 sequences 10.3 and 24.6, of 2,048 equal."""
+        return rows * row_bytes >= self.CONV_WALK_BYTES and rows >= 2 * n_seqs
+
     def causal_conv_silu(self, x, w, b, tail, batch):
         """silu(b + short causal convolution over each sequence's rows); ``tail`` [slots, taps - 1, channels] holds
         every sequence's last inputs and is brought up to date. x may be a column slice; w [taps, channels] float32."""
@@ -1491,7 +1501,9 @@ class Kernels:
         self._ok(self.scan.krk_causal_conv_silu(out.data_ptr(), ptr, stride, w.data_ptr(), b.data_ptr(), tail.data_ptr(),
                                                taps, ch, rows, batch.n_seqs, batch.row_seq.data_ptr(),
                                                batch.cu_q.data_ptr(), batch.seq_qlen.data_ptr(), batch.seq_slot.data_ptr(),
-                                               _code(x.dtype), self._stream()), "causal convolution + silu")
+                                               _code(x.dtype), self._stream(),
+                                               int(self._conv_walks(rows, ch * x.element_size(), batch.n_seqs))),
+                 "causal convolution + silu")
         self.launches += int(taps > 1)
         return out
 

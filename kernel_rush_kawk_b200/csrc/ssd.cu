@@ -553,9 +553,10 @@ int run_scan(SsdArgs a, int n_seqs, int max_q_len, cudaStream_t stream) {
 
 }  // namespace
 
+// walk: a thread goes through CONV_ROWS rows where it can (the caller's rule), else a block takes a row
 KRK_API int krk_causal_conv_silu(void* out, const void* in, int in_stride, const float* w, const float* bias, void* tail,
                                  int taps, int ch, int rows, int n_seqs, const int* row_seq, const int* cu_q,
-                                 const int* seq_qlen, const int* seq_slot, int dtype, cudaStream_t stream) {
+                                 const int* seq_qlen, const int* seq_slot, int dtype, cudaStream_t stream, int walk) {
   if (rows == 0) return 0;
   if (taps < 1 || taps > MAX_TAPS) return -2;
   const int threads = 256;
@@ -565,7 +566,7 @@ KRK_API int krk_causal_conv_silu(void* out, const void* in, int in_stride, const
                    (((uintptr_t)in | (uintptr_t)out | (uintptr_t)tail | (uintptr_t)w | (uintptr_t)bias) & 15) == 0;
   const int vcols = min(64, (ch / V + threads - 1) / threads);
   int rc;
-  if (vec && taps == 4 && rows >= 64 && rows <= 65535 * CONV_ROWS) {  // fewer rows: a block a row has more in flight
+  if (vec && taps == 4 && walk && rows <= 65535 * CONV_ROWS) {
     const dim3 grid((ch / V + 63) / 64, (rows + CONV_ROWS - 1) / CONV_ROWS);
     if (dtype == KRK_DTYPE_F32)
       rc = (int)launch_pdl(causal_conv4_kernel<float>, grid, dim3(64), 0, stream, (float*)out, (const float*)in, in_stride, w, bias,

@@ -141,3 +141,13 @@ def test_unequal_batch_against_each_alone_and_a_slot_used_again(folders):
         for s in slots:
             eng.cache.free(s)
         eng.cache.check()
+
+
+def test_which_steps_go_through_the_convolutions_rows_in_runs():
+    """By bytes, and never single tokens of many sequences: a run of rows is one chain, which short steps would wait for."""
+    from kernel_rush_kawk_b200.csrc.bindings import Kernels
+
+    walks = lambda n_seqs, rows, row_bytes: Kernels._conv_walks(Kernels, rows, row_bytes, n_seqs)
+    assert not any(walks(n, n, 8192) for n in (1, 63, 64, 65, 200, 2048, 4096))
+    assert not any(walks(1, rows, 8192) for rows in (64, 100, 512, 1024)) and not walks(1, 2048, 3584) and not walks(64, 1024, 8192)
+    assert walks(1, 2048, 8192) and walks(3, 2553, 8192) and walks(1, 1024, 16384) and walks(64, 4096, 8192)

@@ -224,10 +224,11 @@ def test_state_space_scans_on_the_tensor_cores(shape, lens, rate, monkeypatch):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-def test_convolution_of_many_rows(dtype):
-    """64 rows and more with four taps: sequences that start anywhere in a thread's sixteen rows, shorter than the taps, channels
+def test_convolution_of_many_rows(dtype, monkeypatch):
+    """Rows in runs of sixteen a thread, four taps: sequences that start anywhere in a run, shorter than the taps, channels
     that fill no block. The same bits as the kernel of single elements, which rows off a 16-byte boundary take."""
     rt = runtime(dtype)
+    monkeypatch.setattr(type(rt.ops), "_conv_walks", lambda *_: True)
     ch, lens = 520, [15, 1, 2, 33, 48, 7]
     rows = sum(lens)
     x = rand((rows, ch), 50).to(dtype).cuda()
@@ -235,6 +236,26 @@ def test_convolution_of_many_rows(dtype):
     odd[:, 1:] = x
     w, b, tail = rand((4, ch), 51).cuda(), rand((ch,), 52).cuda(), rand((7, 3, ch), 53).to(dtype).cuda()
     ctx = context(rt, [1, 0, 4, 3, 5, 6], [9] * 6, lens, None)
+    tails = [tail.clone(), tail.clone()]
+    got = rt.ops.causal_conv_silu(x, w, b, tails[0], ctx.batch)
+    want = rt.ops.causal_conv_silu(odd[:, 1:], w, b, tails[1], ctx.batch)
+    assert torch.equal(got, want) and torch.equal(tails[0], tails[1])
+
+
+@pytest.mark.parametrize("walks", [True, False])
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("lens", [[1] * 70, [1] * 64 + [500], [15, 1, 2, 33, 48, 7], [3, 17, 300, 1, 16, 64]])
+def test_convolution_rows_in_runs_and_one_by_one(dtype, lens, walks, monkeypatch):
+    """Whichever kernel a step takes: the same bits as the kernel of single elements, outputs and stored inputs, with sequences that start
+    anywhere in a thread's sixteen rows."""
+    rt = runtime(dtype)
+    monkeypatch.setattr(type(rt.ops), "_conv_walks", lambda *_: walks)
+    ch, rows = 520, sum(lens)
+    x = rand((rows, ch), 50).to(dtype).cuda()
+    odd = torch.empty((rows, ch + 1), dtype=dtype, device="cuda")
+    odd[:, 1:] = x
+    w, b, tail = rand((4, ch), 51).cuda(), rand((ch,), 52).cuda(), rand((len(lens), 3, ch), 53).to(dtype).cuda()
+    ctx = context(rt, list(range(len(lens)))[::-1], [9] * len(lens), lens, None)
     tails = [tail.clone(), tail.clone()]
     got = rt.ops.causal_conv_silu(x, w, b, tails[0], ctx.batch)
     want = rt.ops.causal_conv_silu(odd[:, 1:], w, b, tails[1], ctx.batch)
