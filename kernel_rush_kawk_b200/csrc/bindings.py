@@ -119,7 +119,7 @@ _LATENT_SIGNATURES = {
                            _P, _P, _P, _P, _P, c_int, _P],
 }
 _SCAN_SIGNATURES = {
-    "krk_token_shift": [_P, _P, c_int, _P, _P, c_int, c_int, c_int, _P, _P, _P, c_int, _P, c_int],
+    "krk_token_shift": [_P, _P, c_int, _P, _P, c_int, c_int, c_int, _P, _P, _P, c_int, _P, c_int, c_int],
     "krk_linear_recurrence": [c_int, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, _P, _P, _P, _P,
                               _P, _P, c_int, c_int, _P, _P, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_int,
                               c_int, _P, _P, _P, c_int, _P, _P, c_int, _P],
@@ -1276,6 +1276,17 @@ class Kernels:
                                        float(params[0]), float(params[1]), _code(z.dtype), self._stream()), "activation")
         return out
 
+    @staticmethod
+    def _shift_walks(rows, C, n_seqs) -> bool:
+        """Whether threads of the token shift go through sixteen rows each, the blend weights in registers. A chain: 5 us, and
+        about 6 more at every sequence's first row, where the thread waits for the stored one; a block a row takes time by
+        its width (a block a row and sixteen rows a thread, single tokens of 64 sequences: 1,536 channels 6.4 and 11.0 us,
+        2,560 9.6 and 11.4, 4,096 14.1 and 11.7; 64 sequences of two: 1,536 6.4 and 8.3, 2,048 7.8 and 8.3, 2,560 9.5 and 8.3;
+        16 of four: 1,024 4.6 and 6.6, 1,536 6.2 and 6.5, 2,048 7.6 and 6.4; one of 128: 1,024 4.2 and 5.1, 1,536 5.6 and 5.2)
+        and by its rounds over the SMs (one of 256: 1,024 6.6 and 5.1; 256 of two: 1,536 10.9 and 8.6). 32-bit: the same."""
+        least = 3072 if rows < 2 * n_seqs else (2048 if rows < 4 * n_seqs else 1536) - 512 * (rows >= 256)
+        return rows >= 64 and C >= least
+
     def token_shift(self, h, last_state, mu, batch, store=False):
         """[mixes, rows, hidden]: h + (h_prev - h) * mu, the row before a step's first coming from ``last_state``;
         with ``store`` every sequence's last row of the step then takes its place there."""
@@ -1286,7 +1297,8 @@ class Kernels:
         out = torch.empty((mu.shape[0], rows, C), dtype=h.dtype, device=h.device)
         self._ok(self.scan.krk_token_shift(out.data_ptr(), ptr, stride, last_state.data_ptr(), mu.data_ptr(), mu.shape[0],
                                           C, rows, batch.row_seq.data_ptr(), batch.cu_q.data_ptr(),
-                                          batch.seq_slot.data_ptr(), _code(h.dtype), self._stream(), int(store)), "token shift")
+                                          batch.seq_slot.data_ptr(), _code(h.dtype), self._stream(), int(store),
+                                          int(self._shift_walks(rows, C, batch.n_seqs))), "token shift")
         return out
 
     RECURRENCE_CHUNK_MIN = 160  # tokens of a step's longest sequence from which a bfloat16 scan of such mixers may run in chunks

@@ -117,10 +117,9 @@ token_shift_wide_kernel(T* __restrict__ out, const T* __restrict__ h, int h_stri
 
 template <typename T>
 int launch_token_shift(T* out, const T* h, int h_stride, float* last_state, const float* mu, int n_mix, int C, int rows,
-                       const int* row_seq, const int* cu_q, const int* seq_slot, cudaStream_t stream, int store) {
+                       const int* row_seq, const int* cu_q, const int* seq_slot, cudaStream_t stream, int store, int walk) {
   constexpr int V = 16 / (int)sizeof(T);
-  // from 64 rows: below, a block a row has more in flight
-  if (n_mix == SHIFT_MIXES && rows >= 64 && C % V == 0 && h_stride % V == 0 && rows <= 65535 * SHIFT_ROWS &&
+  if (walk && n_mix == SHIFT_MIXES && C % V == 0 && h_stride % V == 0 && rows <= 65535 * SHIFT_ROWS &&
       (((uintptr_t)out | (uintptr_t)h | (uintptr_t)mu) & 15) == 0)
     return (int)launch_pdl(token_shift_wide_kernel<T>, dim3((C / V + 63) / 64, (rows + SHIFT_ROWS - 1) / SHIFT_ROWS), dim3(64), 0,
                            stream, out, h, h_stride, last_state, mu, C, rows, row_seq, cu_q, seq_slot, store);
@@ -691,15 +690,16 @@ int pick_split(const ScanArgs& a, float* prep, float* o_scratch, int rows, cudaS
 
 }  // namespace
 
+// walk: a thread goes through SHIFT_ROWS rows where it can (the caller's rule), else a block takes a row
 KRK_API int krk_token_shift(void* out, const void* h, int h_stride, float* last_state, const float* mu, int n_mix,
                             int C, int rows, const int* row_seq, const int* cu_q, const int* seq_slot, int dtype,
-                            cudaStream_t stream, int store) {
+                            cudaStream_t stream, int store, int walk) {
   if (rows == 0) return 0;
   if (dtype == KRK_DTYPE_F32)
     return launch_token_shift<float>((float*)out, (const float*)h, h_stride, last_state, mu, n_mix, C, rows, row_seq, cu_q, seq_slot,
-                                     stream, store);
+                                     stream, store, walk);
   return launch_token_shift<bf16>((bf16*)out, (const bf16*)h, h_stride, last_state, mu, n_mix, C, rows, row_seq, cu_q, seq_slot, stream,
-                                  store);
+                                  store, walk);
 }
 
 KRK_API int krk_linear_recurrence(int rule, const void* r, int r_stride, const void* k, int k_stride, const void* v,

@@ -261,3 +261,14 @@ def test_routing_within_groups_and_the_dense_activation_against_the_plain_functi
     want = plain.dense_ff(h.double(), {k: v.double() for k, v in wd.items()}, "")
     got = dense.forward(SimpleNamespace(ops=rt.ops), h)
     assert (got.double() - want).abs().max() < 1e-4 * want.abs().max()
+
+
+def test_which_steps_go_through_the_token_shifts_rows_in_runs():
+    """By the rows that a sequence brings and the width: at a sequence's first row a thread waits for the stored one, so single tokens
+    of many sequences keep a block a row unless rows are very wide."""
+    from kernel_rush_kawk_b200.csrc.bindings import Kernels
+
+    walks = Kernels._shift_walks
+    assert not any(walks(n, C, n) for n in (1, 63, 64, 65, 128, 1000) for C in (1024, 1536, 2560))
+    assert not walks(63, 4096, 1) and not walks(128, 1536, 64) and not walks(128, 1024, 1)
+    assert walks(64, 1536, 1) and walks(2553, 2560, 3) and walks(400, 1536, 4) and walks(256, 1024, 1) and walks(64, 4096, 64)

@@ -148,11 +148,12 @@ def test_token_shift_keeps_the_last_row_of_every_sequence(dtype):
 
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("store", [False, True])
-def test_token_shift_of_many_rows(dtype, store):
-    """Five blends of 64 rows and more: 16-byte pieces, sequences that start anywhere in a block's sixteen rows (one of a
+def test_token_shift_of_many_rows(dtype, store, monkeypatch):
+    """Five blends, rows in runs of sixteen a thread and in 16-byte pieces: sequences that start anywhere in a run (one of a
     single row among them), a width that fills no block. The same bits as the kernel of single elements, which rows that
     start off a 16-byte boundary take."""
     rt = runtime(dtype)
+    monkeypatch.setattr(type(rt.ops), "_shift_walks", staticmethod(lambda *_: True))
     C, lens = 520, [15, 1, 33, 48, 7]
     rows = sum(lens)
     h = rand((rows, C), 10).to(dtype).cuda()
@@ -163,6 +164,25 @@ def test_token_shift_of_many_rows(dtype, store):
     ctx = context(rt, [1, 0, 4, 3, 5], [0] * 5, [[0] * n for n in lens], None)
     got = rt.ops.token_shift(h, states[0], mu, ctx.batch, store=store)
     want = rt.ops.token_shift(odd[:, 1:], states[1], mu, ctx.batch, store=store)
+    assert torch.equal(got, want) and torch.equal(states[0], states[1])
+
+
+@pytest.mark.parametrize("walks", [True, False])
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("lens", [[1] * 70, [1] * 64 + [500], [3, 17, 300, 1, 16, 64]])
+def test_token_shift_rows_in_runs_and_one_by_one(dtype, lens, walks, monkeypatch):
+    """Whichever kernel a step takes: the same bits as the kernel of single elements, outputs and stored rows."""
+    rt = runtime(dtype)
+    monkeypatch.setattr(type(rt.ops), "_shift_walks", staticmethod(lambda *_: walks))
+    C, rows = 520, sum(lens)
+    h = rand((rows, C), 10).to(dtype).cuda()
+    odd = torch.empty((rows, C + 1), dtype=dtype, device="cuda")
+    odd[:, 1:] = h
+    mu, start = rand((5, C), 3).cuda(), rand((len(lens), C), 4).cuda()
+    states = [start.clone(), start.clone()]
+    ctx = context(rt, list(range(len(lens)))[::-1], [0] * len(lens), [[0] * n for n in lens], None)
+    got = rt.ops.token_shift(h, states[0], mu, ctx.batch, store=True)
+    want = rt.ops.token_shift(odd[:, 1:], states[1], mu, ctx.batch, store=True)
     assert torch.equal(got, want) and torch.equal(states[0], states[1])
 
 
