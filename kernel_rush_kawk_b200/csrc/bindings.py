@@ -130,7 +130,7 @@ _SCAN_SIGNATURES = {
     "krk_causal_conv_silu": [_P, _P, c_int, _P, _P, _P, c_int, c_int, c_int, c_int, _P, _P, _P, _P, c_int, _P, c_int],
     "krk_ssd_scan": [_P, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int,
                      c_int, _P, _P, _P, c_int, _P, _P, c_int, _P],
-    "krk_gated_group_norm": [_P, c_int, c_int, c_float, _P, _P, c_int, _P, c_int, c_int, c_int, c_float, c_int, _P],
+    "krk_gated_group_norm": [_P, c_int, c_int, c_float, _P, _P, c_int, _P, c_int, c_int, c_int, c_float, c_int, _P, c_int],
 }
 _ACTIVATIONS = {"silu": 0, "gelu_tanh": 1, "sigmoid": 2, "swish_clamped": 3, "xielu": 4, "relu2": 5}
 _ATTN_SIGNATURES = {
@@ -1582,6 +1582,14 @@ class Kernels:
             self.launches += 2
         return True
 
+    @staticmethod
+    def _norm_by_warps(items, n) -> bool:
+        """Whether the gated norm takes a warp for a part of a row instead of a block: where the parts are many enough to fill
+        the SMs either way (a block and a warp, bfloat16, 768 elements a part: 4 parts 1.8 and 3.3 us, 1,024 3.7 and 4.7, 2,048
+        5.5 and 5.3, 8,192 16.8 and 11.4; 256 elements: 1,024 parts 2.5 and 2.5, 2,048 3.8 and 3.5; 128: 16 parts 1.74 and
+        1.84, 512 1.94 and 1.98, 1,024 2.3 and 2.0; 32-bit: the same)."""
+        return items >= (1024 if n <= 128 else 2048)
+
     def gated_group_norm(self, y, gate_rows, weight, parts, eps, out, out_col, out_scale):
         """out[:, out_col:...] = group_norm(y * silu(gate_rows)) * weight * out_scale; y float32, ``parts`` equal parts
         each divided by its own root mean square."""
@@ -1592,7 +1600,8 @@ class Kernels:
             raise KernelError("the gated norm reads float32 rows and a gate of the path's dtype")
         self._ok(self.scan.krk_gated_group_norm(optr, ostride, int(out_col), float(out_scale), y.data_ptr(), zptr, zstride,
                                                weight.data_ptr(), rows, inner, int(parts), float(eps), _code(out.dtype),
-                                               self._stream()), "gated group norm")
+                                               self._stream(), int(self._norm_by_warps(rows * int(parts), inner // int(parts)))),
+                 "gated group norm")
 
     # -- token selection ------------------------------------------------------------
     def select_tokens(self, logits, temperature, seed, requests, step, feed=None, out=None):

@@ -450,7 +450,8 @@ __global__ void gated_group_norm_kernel(T* __restrict__ out, int out_stride, int
 }
 
 // The same with a warp per part of a row: parts of up to 1,024 elements, held in registers between the two passes over
-// them. A block per part spent its time on two barriers around little work: 8,192 parts of 768 21.5 -> 15.6 us.
+// them. A block per part spends its time on two barriers around little work where parts are many (8,192 parts of 768 21.5 ->
+// 15.6 us); where they are few, its threads share what is one lane's chain here.
 template <typename T, int PIECES>
 __global__ void __launch_bounds__(256)
 gated_group_norm_warp_kernel(T* __restrict__ out, int out_stride, int out_col, float out_scale, const float* __restrict__ y,
@@ -608,9 +609,10 @@ KRK_API int krk_ssd_scan(float* y, const void* x, int x_stride, const void* B, i
   return dtype == KRK_DTYPE_F32 ? run_scan<float>(a, n_seqs, max_q_len, stream) : run_scan<bf16>(a, n_seqs, max_q_len, stream);
 }
 
+// warps: a warp per part where sizes and addresses allow (the caller's rule), else a block
 KRK_API int krk_gated_group_norm(void* out, int out_stride, int out_col, float out_scale, const float* y, const void* z,
                                  int z_stride, const float* weight, int rows, int inner, int parts, float eps, int dtype,
-                                 cudaStream_t stream) {
+                                 cudaStream_t stream, int warps) {
   if (rows == 0) return 0;
   if (parts < 1 || inner % parts) return -2;
   const int n = inner / parts;
@@ -621,7 +623,7 @@ KRK_API int krk_gated_group_norm(void* out, int out_stride, int out_col, float o
   const size_t esz = dtype == KRK_DTYPE_F32 ? 4 : 2;
   const bool vec = n % 4 == 0 && z_stride % 4 == 0 && out_stride % 4 == 0 && out_col % 4 == 0 &&
                    ((uintptr_t)y & 15) == 0 && (((uintptr_t)z | (uintptr_t)out) & (4 * esz - 1)) == 0;
-  if (vec && n <= 1024 && ((uintptr_t)weight & 15) == 0) {
+  if (warps && vec && n <= 1024 && ((uintptr_t)weight & 15) == 0) {
     const dim3 grid((unsigned)(((long long)rows * parts + 7) / 8));
     const int pieces = (n + 127) / 128;
     if (dtype == KRK_DTYPE_F32) {

@@ -151,3 +151,12 @@ def test_which_steps_go_through_the_convolutions_rows_in_runs():
     assert not any(walks(n, n, 8192) for n in (1, 63, 64, 65, 200, 2048, 4096))
     assert not any(walks(1, rows, 8192) for rows in (64, 100, 512, 1024)) and not walks(1, 2048, 3584) and not walks(64, 1024, 8192)
     assert walks(1, 2048, 8192) and walks(3, 2553, 8192) and walks(1, 1024, 16384) and walks(64, 4096, 8192)
+
+
+def test_few_norm_parts_take_a_block_each():
+    """A single-token step's parts of a gated norm are few: one lane's chain over a part would be the step's."""
+    from kernel_rush_kawk_b200.csrc.bindings import Kernels
+
+    by_warps = Kernels._norm_by_warps
+    assert not any(by_warps(rows * 4, n) for rows in (1, 8, 64, 256) for n in (256, 768, 1024)) and not by_warps(64, 64)
+    assert by_warps(2048 * 4, 768) and by_warps(2048, 1024) and by_warps(64 * 16, 128)

@@ -278,6 +278,24 @@ def test_gated_norm_of_parts_of_any_size(dtype, n):
     assert not out[:, :4].any() and not out[:, -4:].any()
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n", [4, 124, 256, 260, 768, 772, 1024])
+def test_gated_norm_of_many_parts(dtype, n):
+    """Enough parts for a warp each, and one row less than fills the last block of eight: within an element's rounding and a
+    sum's of n terms."""
+    rt = runtime(dtype)
+    rows, parts = 685, 3
+    assert rt.ops._norm_by_warps(rows * parts, n)
+    y, z = rand((rows, parts * n), 54).cuda(), rand((rows, parts * n), 55).to(dtype).cuda()
+    weight, out = (1 + rand((parts * n,), 56, 0.2)).cuda(), torch.zeros((rows, parts * n + 8), dtype=dtype, device="cuda")
+    rt.ops.gated_group_norm(y, z, weight, parts, 1e-5, out, 4, 0.5)
+    v = (y.double() * torch.nn.functional.silu(z.double())).view(rows, parts, n)
+    want = 0.5 * (v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-5)).view(rows, -1) * weight.double()
+    unit = 2.0 ** -8 if dtype == torch.bfloat16 else 2e-6
+    assert ((out[:, 4:-4].double() - want).abs() <= unit * want.abs() + 1e-12).all()
+    assert not out[:, :4].any() and not out[:, -4:].any()
+
+
 def test_a_tokens_infinities_reach_no_earlier_token_of_a_state_space_chunk(monkeypatch):
     rt = runtime(torch.bfloat16)
     monkeypatch.setattr(type(rt.ops), "SSD_TENSOR_MIN", 1)
