@@ -435,6 +435,43 @@ def test_a_sink_that_is_switched_off_counts_nothing(tcgen05, biased, D, monkeypa
         assert ((got.double().cpu() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all(), loud
 
 
+@pytest.mark.parametrize("tcgen05", [True, False])
+@pytest.mark.parametrize("heads,kv_heads,D", [(8, 2, 64), (6, 2, 128), (1, 1, 64)])
+def test_pages_that_no_row_sees_may_hold_anything(heads, kv_heads, D, tcgen05, monkeypatch):
+    """Values that are not finite in a page beyond the sequence's last one (where the table names another sequence's page) and in a
+    page of its own below the window: a masked weight of zero times infinity must not reach a row."""
+    from kernel_rush_kawk_b200.cache import SequenceCache
+    from kernel_rush_kawk_b200.parts.base import KVNeed
+
+    rt = runtime(torch.bfloat16)
+    monkeypatch.setattr(type(rt.ops), "SINK_TCGEN05_ROWS", 1)
+    monkeypatch.setattr(type(rt.ops), "SINK_TCGEN05_KEYS", 1 if tcgen05 else 1 << 30)
+    W = (heads + 2 * kv_heads) * D
+    # a sequence of three whole pages beside one that holds page 0, which a table row names where nothing is reserved yet
+    cache = SequenceCache([KVNeed(kv_heads, D, None)], 1024, 2, 512, rt.device, torch.bfloat16, step_tokens=512)
+    other, slot = cache.alloc(), cache.alloc()
+    cache.reserve(other, 64)
+    cache.sync()
+    view = cache.view(0)
+    view.v[int(view.table[other, 0])] = float("inf")
+    assert int(view.table[other, 0]) == int(view.table[slot, 3])
+    qkv = rand((192, W), 180).to(torch.bfloat16).cuda()
+    got = windowed_prompt(rt, qkv, heads, kv_heads, D, None, None, cache, slot, 0).double().cpu()
+    want = attention_in_64_bits(*split_qkv(qkv, heads, kv_heads, D), 0, 0.3, None, None, None, None).reshape(192, -1)
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
+    # a window of 70 keys: the rows from 270 on see keys from 201 on, in the fourth page; the third one, half of the same block of
+    # 128 keys, holds infinities
+    cache = SequenceCache([KVNeed(kv_heads, D, 70)], 1024, 1, 512, rt.device, torch.bfloat16, step_tokens=512)
+    slot = cache.alloc()
+    qkv = rand((370, W), 181).to(torch.bfloat16).cuda()
+    qkv[128:192, (heads + kv_heads) * D:] = float("inf")
+    windowed_prompt(rt, qkv[:270].contiguous(), heads, kv_heads, D, 70, None, cache, slot, 0)
+    got = windowed_prompt(rt, qkv[270:].contiguous(), heads, kv_heads, D, 70, None, cache, slot, 270).double().cpu()
+    q, k, v = split_qkv(qkv[192:], heads, kv_heads, D)
+    want = attention_in_64_bits(q, k, v, 0, 0.3, 70, None, None, None).reshape(178, -1)[78:]
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("kind", ["attention", "attention_2"])
 @pytest.mark.parametrize("D", [16, 12])
