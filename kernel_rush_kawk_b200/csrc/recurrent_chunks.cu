@@ -75,40 +75,40 @@ __device__ __forceinline__ float dot4(float4 a, float4 b, float d) {
   return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, d))));
 }
 
-// Log decays of a chunk's tokens, a thread one channel of half of them (zero decay beyond the last token).
+// W2 tanh(lora) of a chunk's tokens, a thread one channel of half of them.
 constexpr int HALF = L / 2;
-template <int RULE>
-__device__ __forceinline__ void log_decays(const ChunkArgs& a, float (&x)[HALF], const float* th_s, int ch0, int nt) {
+__device__ __forceinline__ void low_rank_rows(const ChunkArgs& a, float (&z)[HALF], const float* th_s, int ch0) {
   const int ch = threadIdx.x & (N - 1), t0 = threadIdx.x / N * HALF, RP = (a.R + 7) & ~7;
   const bf16* w2 = a.w2 + (size_t)(ch0 + ch) * a.R;
 #pragma unroll
-  for (int t = 0; t < HALF; ++t) x[t] = 0.f;
+  for (int t = 0; t < HALF; ++t) z[t] = 0.f;
   for (int m = 0; m < RP; m += 8) {
     float w[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) w[i] = m + i < a.R ? __bfloat162float(w2[m + i]) : 0.f;
 #pragma unroll
     for (int t = 0; t < HALF; ++t) {
-      const float4 p = ld4(th_s + (t0 + t) * RP + m), q = ld4(th_s + (t0 + t) * RP + m + 4);
-      x[t] = fmaf(p.w, w[3], fmaf(p.z, w[2], fmaf(p.y, w[1], fmaf(p.x, w[0], x[t]))));
-      x[t] = fmaf(q.w, w[7], fmaf(q.z, w[6], fmaf(q.y, w[5], fmaf(q.x, w[4], x[t]))));
+      const float4 x = ld4(th_s + (t0 + t) * RP + m), y = ld4(th_s + (t0 + t) * RP + m + 4);
+      z[t] = fmaf(x.w, w[3], fmaf(x.z, w[2], fmaf(x.y, w[1], fmaf(x.x, w[0], z[t]))));
+      z[t] = fmaf(y.w, w[7], fmaf(y.z, w[6], fmaf(y.y, w[5], fmaf(y.x, w[4], z[t]))));
     }
   }
-  const float w0 = a.w0[ch0 + ch];
-#pragma unroll
-  for (int t = 0; t < HALF; ++t)
-    x[t] = t0 + t >= nt ? 0.f : RULE == 1 ? -a.decay_scale * sigmoid_f(x[t] + w0) : -expf(x[t] + w0);
 }
 
-// Delta rule: the log decays summed over the chunk's tokens, into cs [L][PITCH]; what the running sums round off goes to
-// `rest`: a sum of 18 rounds at 1e-6, which e^c would multiply everything by. `total` is [2][N]. Ends with a barrier.
+// Delta rule: the log decays summed over the chunk's tokens (zero decay beyond the last), into cs [L][PITCH]; what the
+// running sums round off goes to `rest`: a sum of 18 rounds at 1e-6, which e^c would multiply everything by. `total` is [2][N].
+// Ends with a barrier.
 __device__ __forceinline__ void summed_decays(const ChunkArgs& a, float* cs, float* rest, float* total, const float* th_s, int ch0, int nt) {
   const int ch = threadIdx.x & (N - 1), half = threadIdx.x / N, t0 = half * HALF;
-  float z[HALF], low[HALF], run = 0.f, lost = 0.f;
-  log_decays<1>(a, z, th_s, ch0, nt);
+  float z[HALF];
+  low_rank_rows(a, z, th_s, ch0);
+  const float w0 = a.w0[ch0 + ch];
+  float run = 0.f, lost = 0.f, low[HALF];
 #pragma unroll
   for (int t = 0; t < HALF; ++t) {
-    const float x = z[t], sum = run + x, y = sum - run;
+    float x = -a.decay_scale * sigmoid_f(z[t] + w0);
+    if (t0 + t >= nt) x = 0.f;
+    const float sum = run + x, y = sum - run;
     lost += (run - (sum - y)) + (x - y);
     low[t] = lost;
     z[t] = run = sum;
@@ -362,9 +362,13 @@ __global__ void __launch_bounds__(THREADS) mix_chunk_kernel(ChunkArgs a) {
   {
     const int ch = threadIdx.x & (N - 1), half = threadIdx.x / N, t0 = half * HALF;
     float x[HALF], run = 0.f;
-    log_decays<0>(a, x, th_s, ch0, nt);
+    low_rank_rows(a, x, th_s, ch0);
+    const float w0 = a.w0[ch0 + ch];
 #pragma unroll
-    for (int t = 0; t < HALF; ++t) run += x[t];
+    for (int t = 0; t < HALF; ++t) {
+      x[t] = t0 + t < nt ? -expf(x[t] + w0) : 0.f;  // zero decay beyond the last token
+      run += x[t];
+    }
     total[half * N + ch] = run;
     __syncthreads();
     grid_launch_dependents();
