@@ -589,9 +589,9 @@ __global__ void __launch_bounds__(THREADS) chunk_output_kernel(ChunkArgs a) {
   }
 }
 
-// State-space kind. A block's time is its chain of loads and barriers rather than its products, so four blocks share an SM:
-// the state never passes through shared memory. A warp takes all 64 tokens of eight value columns, whose part of the
-// state is then its own fragment of the product, loaded (from the first instruction on) and split in registers.
+// State-space kind. A block's time is its chain of loads and barriers rather than its products, so three blocks share an SM
+// (80 registers a thread): the state never passes through shared memory. A warp takes all 64 tokens of eight value columns, whose
+// part of the state is then its own fragment of the product, loaded (from the first instruction on) and split in registers.
 // 2,048 tokens of 48 heads: 66 us; with the state's three terms in shared memory and two blocks an SM 87.
 __global__ void __launch_bounds__(THREADS, 3) ssd_output_kernel(ChunkArgs a) {
   extern __shared__ __align__(16) bf16 sm[];

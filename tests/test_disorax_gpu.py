@@ -358,7 +358,8 @@ def test_routed_experts_alone(dtype, shape, rows):
 def test_products_of_few_experts_rows(gated, activation, weigh_input, sizes, rows, top):
     """Single-token steps in bfloat16, an expert's weights read once for all its rows: one row to more than sixteen rows an
     expert, more pairs than experts and fewer, choices that are no expert, sizes off the tiles of 16 and 32; no further from
-    64 bits than the kernels that read an expert per pair are, within a rounding of the result."""
+    64 bits than the kernels that read an expert per pair are (both round an expert's result to bfloat16 before it is weighted and
+    added in float32; only the order of k differs, which moves the distance by a thousandth)."""
     rt = runtime(torch.bfloat16)
     K, F, C, E = sizes
     bf = lambda t: t.to(torch.bfloat16).cuda()
@@ -394,7 +395,7 @@ def test_products_of_few_experts_rows(gated, activation, weigh_input, sizes, row
         finally:
             ops._few_experts = staticmethod(kept)
         off[few] = ((got.double().cpu() - want).norm() / want.norm()).item()
-    assert off[True] <= 1.2 * off[False] + 2.0 ** -10, off
+    assert off[True] <= 1.01 * off[False] + 1e-5, off
     assert off[True] < 1e-2, off
 
 

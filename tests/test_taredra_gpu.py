@@ -351,7 +351,8 @@ def test_scans_in_chunks(kind, lens, decays, monkeypatch):
     """Steps of many tokens in bfloat16 with heads of 64 channels: chunks of 32 tokens, whole and cut into portions of one
     chunk (little scratch), from a state that is not zero; against 64 bits, and no further from it than the scan token by
     token: the outputs within a bfloat16 rounding (2^-8 of a value, and of the row's size for what cancels), the
-    32-bit state within 8e-6 of its size (the decays' sums over a chunk round at 2^-24 of up to 80)."""
+    32-bit state within 1e-6 of its size (the scan token by token, which multiplies by a rounded decay a token, is off by up to
+    4.1e-7)."""
     rt = runtime(torch.bfloat16)
     heads = 3
     x = scan_inputs(kind, lens, heads, decays, 60)
@@ -366,7 +367,7 @@ def test_scans_in_chunks(kind, lens, decays, monkeypatch):
         size = want.pow(2).mean().sqrt()
         assert ((got.double().cpu() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-3 * size).all(), name
         off[name] = ((state.double().cpu() - want_state).norm() / want_state.norm()).item()
-        assert off[name] < 8e-6, (name, off)
+        assert off[name] < 1e-6, (name, off)
         if name == "chunks":
             whole = got, state
     assert torch.equal(got, whole[0]) and torch.equal(state, whole[1]), "portions are the same sums"
