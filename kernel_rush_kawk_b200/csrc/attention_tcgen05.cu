@@ -31,9 +31,9 @@
 //
 // WIDE: attention whose softmax weights are 32-bit quantities (krk_sink_prefill_tcgen05). A weight reaches P V as two bfloat16
 // halves, p = hi + lo (16 bits of mantissa), which take the two halves of S's columns in tensor memory, and each instruction of
-// P V comes twice, for the pages that some row of the tile sees. A row may start from a softmax sink (maximum = its
-// head's sink, sum 1, no value); rows of the output may lie
-// apart, are multiplied by a number and by the sigmoid of a gate per head or per element. SHAPED: scores are capped
+// P V comes twice, for the pages that some row of the tile sees. A row may start from a softmax sink (maximum = its head's
+// sink, sum 1, no value); rows of the output may lie apart, are multiplied by a number and by the sigmoid of a gate per head or
+// per element. SHAPED: scores are capped
 // (c tanh(s / c) = c (1 - 2 / (1 + e^(2 s / c)))) and lose a slope times the distance of query and key before the softmax.
 // 2,048 tokens, a window of 1,024, 16 heads of 128 in groups of four: 45 us against the mma.sync kernel's 116 (of 37 at that
 // instruction's measured rate, 550 TFLOP/s, for 19 GFLOP); 12 heads in groups of three, no slopes, 46 against 75.
@@ -82,20 +82,22 @@ struct TileRange {
   __device__ __forceinline__ bool has(int j) const { return j >= lo && j <= hi; }
 };
 
-// The first and the last key that some row of a tile sees.
-__device__ __forceinline__ int first_key(int row_begin, int G, int start, int window) {
-  return window > 0 ? max(0, start + row_begin / G - window + 1) : 0;
-}
-__device__ __forceinline__ int last_key(int row_begin, int G, int q_len, int start) {
-  return start + min(q_len - 1, (row_begin + ROWS - 1) / G);
-}
-
 __device__ __forceinline__ TileRange tile_range(int row_begin, int n_rows, int G, int q_len, int start, int window) {
   TileRange t;
   if (row_begin >= n_rows) { t.lo = 1; t.hi = 0; return t; }
-  t.lo = first_key(row_begin, G, start, window) / KEYS;
-  t.hi = last_key(row_begin, G, q_len, start) / KEYS;
+  const int first_tok = row_begin / G;
+  const int last_tok = min(q_len - 1, (row_begin + ROWS - 1) / G);
+  t.lo = window > 0 ? max(0, start + first_tok - window + 1) / KEYS : 0;
+  t.hi = (start + last_tok) / KEYS;
   return t;
+}
+
+// The first and the last page that some row of a tile sees, of the sequence's.
+__device__ __forceinline__ int first_page(int row_begin, int G, int start, int window) {
+  return window > 0 ? max(0, start + row_begin / G - window + 1) / KRK_PAGE : 0;
+}
+__device__ __forceinline__ int last_page(int row_begin, int G, int q_len, int start) {
+  return (start + min(q_len - 1, (row_begin + ROWS - 1) / G)) / KRK_PAGE;
 }
 
 // What the wide form adds; see the opening text.
@@ -244,27 +246,35 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
       // stays out of P V: its weights are zero, but its values may be anything (the second page of a sequence's last block
       // may belong to another sequence), and zero times infinity is not zero.
       bool skip_first[2], skip_last[2];
+      if constexpr (WIDE) {
 #pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        const int row = pair * PAIR + t * ROWS;
-        skip_first[t] = WIDE && first_key(row, G, start, window) % KEYS >= KRK_PAGE;
-        skip_last[t] = WIDE && last_key(row, G, q_len, start) % KEYS < KRK_PAGE;
+        for (int t = 0; t < 2; ++t) {
+          skip_first[t] = first_page(pair * PAIR + t * ROWS, G, start, window) & 1;
+          skip_last[t] = !(last_page(pair * PAIR + t * ROWS, G, q_len, start) & 1);
+        }
       }
       auto pv = [&](int t, int i, bool first, bool last) {  // O_t (+)= P_t V_i, 16 keys (8 columns of P) per instruction
         const unsigned char* v = v_s + (i & 1) * TILE_BYTES;
-        const bool skip = first && skip_first[t];
-        auto page = [&](int k0) {
+        if constexpr (WIDE) {
+          const bool skip = first && skip_first[t];
+          auto page = [&](int k0) {
 #pragma unroll
-          for (int ks = k0; ks < k0 + KEYS / 32; ++ks) {
-            umma_bf16_tmem_a(tmem + TMEM_O + t * D, tmem + t * 128 + ks * 8, umma_desc_sw128(v + ks * 16 * 128, SUB, 1024),
-                             idesc_o, (first && ks == 0) || (skip && ks == KEYS / 32) ? 0u : 1u);
-            if constexpr (WIDE)  // the weights' low halves
+            for (int ks = k0; ks < k0 + KEYS / 32; ++ks) {
+              umma_bf16_tmem_a(tmem + TMEM_O + t * D, tmem + t * 128 + ks * 8, umma_desc_sw128(v + ks * 16 * 128, SUB, 1024),
+                               idesc_o, (first && ks == 0) || (skip && ks == KEYS / 32) ? 0u : 1u);
+              // the weights' low halves
               umma_bf16_tmem_a(tmem + TMEM_O + t * D, tmem + t * 128 + 64 + ks * 8, umma_desc_sw128(v + ks * 16 * 128, SUB, 1024),
                                idesc_o, 1u);
-          }
-        };
-        if (!skip) page(0);
-        if (!(last && skip_last[t])) page(KEYS / 32);
+            }
+          };
+          if (!skip) page(0);
+          if (!(last && skip_last[t])) page(KEYS / 32);
+        } else {
+#pragma unroll
+          for (int ks = 0; ks < KEYS / 16; ++ks)
+            umma_bf16_tmem_a(tmem + TMEM_O + t * D, tmem + t * 128 + ks * 8, umma_desc_sw128(v + ks * 16 * 128, SUB, 1024),
+                             idesc_o, (first && ks == 0) ? 0u : 1u);
+        }
       };
       const TileRange rng[2] = {r0, r1};
       if (q_by_tma && !mbar_wait(bars + Q_FULL, 0)) give_up(14);
