@@ -246,13 +246,6 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
       // stays out of P V: its weights are zero, but its values may be anything (the second page of a sequence's last block
       // may belong to another sequence), and zero times infinity is not zero.
       bool skip_first[2], skip_last[2];
-      if constexpr (WIDE) {
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          skip_first[t] = first_page(pair * PAIR + t * ROWS, G, start, window) & 1;
-          skip_last[t] = !(last_page(pair * PAIR + t * ROWS, G, q_len, start) & 1);
-        }
-      }
       auto pv = [&](int t, int i, bool first, bool last) {  // O_t (+)= P_t V_i, 16 keys (8 columns of P) per instruction
         const unsigned char* v = v_s + (i & 1) * TILE_BYTES;
         if constexpr (WIDE) {
@@ -284,6 +277,13 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         if (r0.has(j_lo)) qk(0, 0);
         if (r1.has(j_lo)) qk(1, 0);
         umma_commit(bars + K_FREE);
+      }
+      if constexpr (WIDE) {  // here, while the first scores are on their way
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          skip_first[t] = first_page(pair * PAIR + t * ROWS, G, start, window) & 1;
+          skip_last[t] = !(last_page(pair * PAIR + t * ROWS, G, q_len, start) & 1);
+        }
       }
       for (int i = 0; i < n && ok; ++i) {
         const int j = j_lo + i, b = i & 1;
