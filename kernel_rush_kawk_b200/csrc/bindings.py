@@ -981,17 +981,14 @@ class Kernels:
         pairs = rows * top
         empty = lambda n: torch.empty((pairs, n), dtype=x.dtype, device=x.device)
         xg, h, yg = empty(K), empty(F), empty(C)
-        # blocks of up to 256 rows: experts of more than 128 rows on the average, and blocks enough for two rounds over the
-        # SMs all the same (4,096 rows of 16 experts of 512: 33 against 28 us; 12,288 of 64 of 1,408: 199 against 258 us)
-        tall = lambda n, cols: int(pairs > 128 * E and E * -(-n // cols) >= 296)
         row_w = torch.empty(pairs, dtype=torch.float32, device=x.device) if w_in is not None else None  # in the rows' new order
         self._ok(self.moe.krk_moe_gather(xg.data_ptr(), ptr, stride, place.data_ptr(), experts.data_ptr(), offsets.data_ptr(), 0,
                                          rows, top, K, _ptr(w_in), _ptr(row_w), _code(x.dtype), self._stream()), "expert gather")
         self._ok(self.moe.krk_grouped_gemm(h.data_ptr(), xg.data_ptr(), w_first.data_ptr(), offsets.data_ptr(), pairs, E, F, K,
-                                           _ACTIVATIONS[activation], int(gated), tall(F, 128 if gated else 256), _ptr(row_w), float(act_params[0]),
+                                           _ACTIVATIONS[activation], int(gated), 1, _ptr(row_w), float(act_params[0]),
                                            float(act_params[1]), self.error.data_ptr(), self._stream()), "experts' first product")
         self._ok(self.moe.krk_grouped_gemm(yg.data_ptr(), h.data_ptr(), w_down.data_ptr(), offsets.data_ptr(), pairs, E, C, F, -1,
-                                           0, tall(C, 256), None, 0.0, 0.0, self.error.data_ptr(), self._stream()), "experts' second product")
+                                           0, 1, None, 0.0, 0.0, self.error.data_ptr(), self._stream()), "experts' second product")
         out = torch.empty((rows, C), dtype=x.dtype, device=x.device)
         self._ok(self.moe.krk_moe_combine(out.data_ptr(), _ptr(add), _ptr(add_gate), yg.data_ptr(), place.data_ptr(),
                                           experts.data_ptr(), offsets.data_ptr(), 0, _ptr(w_out), rows, top, C, ptr, stride,

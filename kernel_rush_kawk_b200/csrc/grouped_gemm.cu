@@ -1,32 +1,42 @@
 // The routed experts' products of many rows in one launch on the 5th-generation tensor cores, the rows of an expert
 // wherever the routing put their number: C[r, :] = act(A[r, :] W_e^T) for the rows r of expert e, offsets[e] <= r <
-// offsets[e + 1], W [E, N, K]. GATED: W [E, 2N, K] holds every expert's gate rows and then its up rows; a block streams 128
-// of either, and the epilogue reads both halves of its accumulator: C = act(g, u) with g and u multiplied by the row's weight
-// first where there is one (a router that weighs an expert's input). The offsets stay on the device: the grid holds as many row tiles as the routing could need
-// at most, a block finds its expert and rows by a scan over the experts' tile counts, and blocks beyond the last tile leave
-// at once.
+// offsets[e + 1], W [E, N, K]. Gated: W [E, 2N, K] holds every expert's gate rows and then its up rows, and C = act(g, u) with g
+// and u multiplied by the row's weight first where there is one (a router that weighs an expert's input). The offsets stay on the device.
 //
-// The tile engine is that of gemm_tcgen05.cu: warp 0 drives TMA (128 rows of A, BN rows of W, 64 elements of K a stage,
-// 128-byte swizzle), warp 1 owns tensor memory and issues tcgen05.mma, warps 2..5 read the accumulator back. With MT = 2 a
-// block takes up to 256 of an expert's rows: two tiles of A ride with every tile of W into two accumulators (all 512 columns
-// of tensor memory), which warps 2..5 and 6..9 read back side by side. Where experts have more than one tile of rows, W is
-// then fetched once instead of twice and half as many blocks pay for their start and their epilogue. A tile of A
-// that reaches past its expert's rows reads the next expert's (or zeros beyond the matrix); what it makes of them is not
-// stored. Every wait is bounded: one that runs out sets the error word and the block leaves, after freeing its tensor
-// memory.
+// Bound by the weights' bytes (64 experts of 2,048 x 1,408, 2,048 rows of six: 738 and 369 MB, 113 and 56 us, against 88 and 44 us of
+// products). Blocks work in pairs (cta_group::2): 256 rows of W_e are the product's M, each block's shared memory holding 128 of them,
+// and an expert's rows are its N, 32 to 256 of them, each block holding half. So what a product costs follows the rows that there are,
+// in steps of 32 instead of 128, every weight is fetched once for up to 256 rows, an SM takes in 16 KB of weights and its half of the rows
+// for as much work as a block alone does with 16 and 32 KB, and a tile's accumulator fills half of tensor memory: while its eight
+// reading warps turn one tile into C, the next one is multiplied. Pairs stay and walk the tiles (74 pairs, the tiles of a row tile
+// side by side), so that loads go on over the seams. With a single-block tile of 256 rows by 256 columns, launched per tile,
+// the two products took 195 and 105 us, now 163 and 85; 4,000 rows 352 and 187 -> 280 and 150; 200 rows, where nothing but the weights
+// counts, 163 and 81 -> 120 and 65. Asking weights into L2 ahead of the ring was measured and is slower (eight blocks of k: 219
+// against 189 us, single blocks); rows in copies of 16 instead of 128, 64, 32 and 16: 200 against 167 us.
+//
+// Warp 0 of either block drives TMA (64 elements of K a stage, 128-byte swizzle) and counts on the first block's barriers; warp 1 of
+// the first block issues tcgen05.mma for both; warps 2..9 read the accumulator back. There a lane is a column of C and what a thread
+// holds are rows, so a warp turns 32 x 32 of them through a patch of shared memory. Gated, gate and up rows alternate in the tile, so
+// that neighbouring lanes hold a column's two products. Rows beyond the expert's, the next one's or zeros, are not stored.
+// Every wait is bounded: one that runs out sets the error word, and the blocks leave after freeing their tensor memory.
 #include "tcgen05.cuh"
 
 namespace {
 
 using namespace tc;
 
-constexpr int BM = 128, BK = 64, UMMA_K = 16;
-constexpr uint32_t A_BYTES = BM * BK * 2;
+constexpr int BK = 64, UMMA_K = 16;
+constexpr int SMS = 148;
+constexpr int READERS = 8;  // warps that read accumulators: two to a quarter of tensor memory's lanes
+constexpr int THREADS = 64 + 32 * READERS;
 
-// act 0: silu(g) u of the two products as they would have been stored; act 3: clamped inputs,
+// SILU: silu(g) u of the two products as they would have been stored; CLAMPED:,
 // g' = min(g, limit), u' = clamp(u, -limit, limit), g' sigmoid(slope g') (u' + 1), nothing rounded before the end
-__device__ __forceinline__ float gated_act_of(float g, float u, int act, float limit, float slope) {
-  if (act == 3) {
+enum Form { SILU, CLAMPED, PLAIN, SQUARED };
+
+template <Form FORM>
+__device__ __forceinline__ float gated_act_of(float g, float u, float limit, float slope) {
+  if (FORM == CLAMPED) {
     g = fminf(g, limit);
     u = fminf(fmaxf(u, -limit), limit);
     return __fdividef(g, 1.0f + __expf(-slope * g)) * (u + 1.0f);
@@ -35,197 +45,312 @@ __device__ __forceinline__ float gated_act_of(float g, float u, int act, float l
   return __fdividef(g, 1.0f + __expf(-g)) * round_to<bf16>(u);
 }
 
-template <int BN, int STAGES, bool GATED, int MT>
-__global__ void __launch_bounds__(64 + 128 * MT)
-grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, bf16* __restrict__ C,
-                    const int* __restrict__ offsets, int E, int N, int K, int act, const float* __restrict__ row_weights,
-                    float limit, float slope, int* __restrict__ error) {
-  constexpr int BC = GATED ? BN / 2 : BN;  // columns of C a block makes
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
-  constexpr uint32_t B_BYTES = BN * BK * 2;
-  constexpr uint32_t STAGE_BYTES = MT * A_BYTES + B_BYTES;
-  constexpr uint32_t TMEM_COLS = MT * (BN <= 128 ? 128 : 256);
-  unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(tiles + (size_t)STAGES * STAGE_BYTES);
-  uint64_t* empty_bar = full_bar + STAGES;
-  uint64_t* acc_bar = empty_bar + STAGES;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_bar + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+constexpr uint32_t W_BYTES = 128 * BK * 2;      // a block's half of the pair's weights
+constexpr int BOXES = 4, BIGGEST = 128;         // rows come in copies of 128, 64, 32 and 16: many small ones would bound the kernel
+struct RowMaps { CUtensorMap of[BOXES]; };
+constexpr int BUF_COLS = 256;                   // tensor memory of an accumulator; there are two
+constexpr int PATCH_PITCH = 80;                 // bytes of a row of a warp's patch for the transpose: 16-byte reads of 32 rows meet no bank twice
+constexpr int PATCH_BYTES = 32 * PATCH_PITCH;
+constexpr int RING_BYTES = 200 * 1024, MOST_STAGES = 10;
+constexpr size_t SMEM_BYTES = 1024 + (size_t)RING_BYTES + READERS * PATCH_BYTES + (2 * MOST_STAGES + 5) * 8 + 16;
 
-  // which expert's which tile: every warp scans the experts' tile counts, 32 at a time
-  int e = -1, m0 = 0, row_end = 0;
-  for (int e0 = 0, before = 0; e0 < E && e < 0; e0 += 32) {
-    const int mine = e0 + lane;
-    const int lo = mine < E ? offsets[mine] : 0, hi = mine < E ? offsets[mine + 1] : 0;
-    const int tiles_here = (hi - lo + MT * BM - 1) / (MT * BM);
-    int incl = tiles_here;
+// Which expert and rows the row tile `y` is, over all experts' row tiles in order: an expert's rows in as few equal tiles of up to
+// `most` rows as hold them, in multiples of 32. A warp's own: 32 experts' tile counts at a time, kept between calls, since a
+// block asks for its tiles in ascending order.
+struct RowTiles {
+  const int* offsets;
+  int E, most, e0, before, lo, hi, count, incl;  // experts e0 + lane; `before`: row tiles of the experts before e0
+  __device__ RowTiles(const int* offsets_, int E_, int most_) : offsets(offsets_), E(E_), most(most_), e0(0), before(0) { load(); }
+  __device__ void load() {
+    const int lane = threadIdx.x & 31, mine = e0 + lane;
+    lo = mine < E ? offsets[mine] : 0;
+    hi = mine < E ? offsets[mine + 1] : 0;
+    incl = count = tiles_of(hi - lo);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int p = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += p;
     }
-    const int t = (int)blockIdx.y - before;
-    const unsigned hit = __ballot_sync(0xffffffffu, t < incl && t >= incl - tiles_here);
-    if (hit) {
-      const int src = __ffs(hit) - 1;
-      e = e0 + src;
-      m0 = __shfl_sync(0xffffffffu, lo + (t - (incl - tiles_here)) * (MT * BM), src);
-      row_end = __shfl_sync(0xffffffffu, hi, src);
-    }
-    before += __shfl_sync(0xffffffffu, incl, 31);
   }
-  if (e < 0) return;  // the same for the whole block
-  const int n0 = blockIdx.x * BC;
-  const int k_blocks = (K + BK - 1) / BK;
-  const int live = (MT == 2 && row_end - m0 > BM) ? 2 : 1;  // tiles of A that hold rows of this expert
+  __device__ int tiles_of(int rows) const { return (rows + most - 1) / most; }
+  __device__ int each(int rows) const { return rows ? ((rows + tiles_of(rows) - 1) / tiles_of(rows) + 31) / 32 * 32 : 0; }
+  // rows of the biggest tile
+  __device__ int biggest() const {
+    int n = 32;
+    for (int i = threadIdx.x & 31; i < E; i += 32) n = max(n, each(offsets[i + 1] - offsets[i]));
+    return __reduce_max_sync(0xffffffffu, n);
+  }
+  // false: there are not so many
+  __device__ bool find(int y, int& e, int& m0, int& rows) {
+    for (int all = __shfl_sync(0xffffffffu, incl, 31); y - before >= all; all = __shfl_sync(0xffffffffu, incl, 31)) {
+      if (e0 + 32 >= E) return false;
+      before += all;
+      e0 += 32;
+      load();
+    }
+    const int t = y - before, first = incl - count;
+    const int src = __ffs(__ballot_sync(0xffffffffu, t < incl && t >= first)) - 1;
+    const int rows_each = each(hi - lo), from = lo + (t - first) * rows_each;
+    e = e0 + src;
+    m0 = __shfl_sync(0xffffffffu, from, src);
+    rows = __shfl_sync(0xffffffffu, min(rows_each, hi - from), src);
+    return true;
+  }
+};
+
+template <Form FORM>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS)
+grouped_gemm_kernel(const __grid_constant__ RowMaps maps_a, const __grid_constant__ CUtensorMap map_w, bf16* __restrict__ C,
+                    const int* __restrict__ offsets, int E, int N, int K, int most, const float* __restrict__ row_weights,
+                    float limit, float slope, int* __restrict__ error) {
+  constexpr bool GATED = FORM == SILU || FORM == CLAMPED;
+  constexpr int BC = GATED ? 64 : 128;  // columns of C a block makes of a tile; the pair twice as many
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* patches = tiles + RING_BYTES;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(patches + READERS * PATCH_BYTES);  // the first block's: copies of both have landed
+  uint64_t* empty_bar = full_bar + MOST_STAGES;   // either block's: the products have read a stage
+  uint64_t* acc_full = empty_bar + MOST_STAGES;   // either block's
+  uint64_t* acc_empty = acc_full + 2;        // the first block's: the reading warps of both are through
+  uint64_t* drain_bar = acc_empty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
+  int* issued = reinterpret_cast<int*>(tmem_slot + 1);  // blocks of k that were asked for, where a wait ran out; else -1
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank();
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < MOST_STAGES; ++s) {
       mbar_init(full_bar + s, 1);
       mbar_init(empty_bar + s, 1);
     }
-    mbar_init(acc_bar, 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(acc_full + b, 1);
+      mbar_init(acc_empty + b, 2 * READERS);
+    }
+    mbar_init(drain_bar, 1);
+    *issued = -1;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2 * BUF_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
+  cluster_sync();  // the other block's barriers exist
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_launch_dependents();
+  grid_dependency_wait();
+  RowTiles tiles_of(offsets, E, most);
+  const uint32_t stage_bytes = W_BYTES + (uint32_t)tiles_of.biggest() / 2 * BK * 2;
+  const int stages = min(MOST_STAGES, (int)(RING_BYTES / stage_bytes));
+  const int k_blocks = (K + BK - 1) / BK, cols = (N + 2 * BC - 1) / (2 * BC);
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  int e, m0, rows;
 
-  if (warp == 0 && lane == 0) {
-    for (int kb = 0; kb < k_blocks; ++kb) {
-      const int s = kb % STAGES;
-      if (kb >= STAGES && !mbar_wait(empty_bar + s, ((kb / STAGES) - 1) & 1)) { atomicExch(error, 3); break; }
-      unsigned char* stage = tiles + (size_t)s * STAGE_BYTES;
-      mbar_expect_tx(full_bar + s, live * A_BYTES + B_BYTES);
+  if (warp == 0) {
+    int s = 0, asked = 0;
+    uint32_t parity = 1;  // of the round before: a first round finds its stages empty
+    bool ok = true;
+    for (int t = pair; ok && tiles_of.find(t / cols, e, m0, rows); t += pairs) {
+      if (lane == 0) {
+        const int half = (rows + 31) / 32 * 16;  // rows that each block of the pair brings
+        const int f0 = (t % cols * 2 + (int)rank) * BC, first = m0 + (int)rank * half;
+        const uint32_t bytes = 2 * (W_BYTES + (uint32_t)half * BK * 2);
+        for (int kb = 0; kb < k_blocks; ++kb) {
+          if (!mbar_wait(empty_bar + s, parity)) {
+            atomicExch(error, 3);
+            *issued = asked;
+            ok = false;
+            break;
+          }
+          unsigned char* stage = tiles + s * stage_bytes;
+          const uint32_t bar = cluster_address(full_bar + s, 0);
+          if (rank == 0) mbar_expect_tx(full_bar + s, bytes);
+          if (GATED) tma_load_3d_pair(stage, &map_w, bar, kb * BK, 0, 2 * e * N + f0);
+          else tma_load_2d_pair(stage, &map_w, bar, kb * BK, e * N + f0);
+          int r = 0;
 #pragma unroll
-      for (int t = 0; t < MT; ++t)
-        if (t < live) tma_load_2d(stage + t * A_BYTES, &map_a, full_bar + s, kb * BK, m0 + t * BM);
-#pragma unroll
-      for (int h = 0; h < BN / 128; ++h)
-        tma_load_2d(stage + MT * A_BYTES + h * (128 * BK * 2), &map_w, full_bar + s, kb * BK,
-                    GATED ? (2 * e + h) * N + n0 : e * N + n0 + 128 * h);
-    }
-  } else if (warp == 1 && lane == 0) {
-    constexpr uint32_t idesc = umma_idesc(BM, BN);
-    for (int kb = 0; kb < k_blocks; ++kb) {
-      const int s = kb % STAGES;
-      if (!mbar_wait(full_bar + s, (kb / STAGES) & 1)) { atomicExch(error, 4); break; }
-      tc_fence_after();
-      unsigned char* stage = tiles + (size_t)s * STAGE_BYTES;
-      const uint64_t b_desc = umma_desc(stage + MT * A_BYTES);
-#pragma unroll
-      for (int t = 0; t < MT; ++t) {
-        if (t >= live) break;
-        const uint64_t a_desc = umma_desc(stage + t * A_BYTES);
-#pragma unroll
-        for (int k = 0; k < BK / UMMA_K; ++k) {
-          const uint64_t adv = (uint64_t)((k * UMMA_K * 2) >> 4);
-          umma_bf16(tmem_base + (uint32_t)(t * BN), a_desc + adv, b_desc + adv, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          for (int b = 0; b < BOXES; ++b)
+            if (half & (BIGGEST >> b)) {
+              tma_load_2d_pair(stage + W_BYTES + r * (BK * 2), &maps_a.of[b], bar, kb * BK, first + r);
+              r += BIGGEST >> b;
+            }
+          ++asked;
+          if (++s == stages) { s = 0; parity ^= 1; }
         }
       }
-      umma_commit(empty_bar + s);
+      ok = __shfl_sync(0xffffffffu, ok, 0);
     }
-    umma_commit(acc_bar);  // arrives even after a failed wait, so the epilogue moves on
-  } else if (warp >= 2) {
-    const int quarter = warp & 3, tile = (warp - 2) >> 2;
-    const int row = m0 + tile * BM + quarter * 32 + lane;
-    const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(tile * BN);
-    const bool ok = mbar_wait(acc_bar, 0);
-    if (!ok && lane == 0) atomicExch(error, 5);
-    tc_fence_after();
-    if (ok && tile < live) {
-      const float a = (GATED && row_weights && row < row_end) ? row_weights[row] : 1.f;
-#pragma unroll 1
-      for (int c0 = 0; c0 < BC; c0 += 32) {
-        if (n0 + c0 >= N) break;  // the same for the whole block
-        uint32_t g[32], u[GATED ? 32 : 1];
-        tmem_ld_32x32(acc + (uint32_t)c0, g);
-        if constexpr (GATED) tmem_ld_32x32(acc + (uint32_t)(BC + c0), u);
-        tmem_wait_ld();
-        if (row < row_end) {
-          bf16* dst = C + (size_t)row * N + n0 + c0;
-          float v[32];
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            v[j] = __uint_as_float(g[j]);
-            if constexpr (GATED) {
-              v[j] = gated_act_of(a * v[j], a * __uint_as_float(u[j]), act, limit, slope);
-            } else if (act == 5) {  // squared relu of the product as it would have been stored
-              const float z = round_to<bf16>(v[j]);
-              v[j] = z > 0.f ? z * z : 0.f;
-            }
+    if (lane == 0 && ok)  // the last stages' releases, too, have arrived before the block leaves
+      for (int i = 0; i < stages; ++i) {
+        if (!mbar_wait(empty_bar + s, parity)) {
+          atomicExch(error, 3);
+          *issued = asked;
+          break;
+        }
+        if (++s == stages) { s = 0; parity ^= 1; }
+      }
+  } else if (warp == 1) {
+    int s = 0, buf = 0;
+    uint32_t parity = 0, acc_parity = 1;
+    bool ok = rank == 0;
+    for (int t = pair; ok && tiles_of.find(t / cols, e, m0, rows); t += pairs) {
+      if (lane == 0) {
+        const uint32_t idesc = umma_idesc(256, (rows + 31) / 32 * 32);
+        const uint32_t acc = tmem_base + (uint32_t)buf * BUF_COLS;
+        ok = mbar_wait(acc_empty + buf, acc_parity);  // both blocks have read what was there
+        tc_fence_after();
+        for (int kb = 0; ok && kb < k_blocks; ++kb) {
+          if (!mbar_wait(full_bar + s, parity)) {
+            ok = false;
+            break;
           }
-          if (n0 + c0 + 32 <= N) {  // N is a multiple of 8: 16-byte stores
+          tc_fence_after();
+          unsigned char* stage = tiles + s * stage_bytes;
+          const uint64_t w_desc = umma_desc(stage), r_desc = umma_desc(stage + W_BYTES);
 #pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              uint4 pk;
-              __nv_bfloat162* pp = reinterpret_cast<__nv_bfloat162*>(&pk);
+          for (int k = 0; k < BK / UMMA_K; ++k) {
+            const uint64_t adv = (uint64_t)((k * UMMA_K * 2) >> 4);
+            umma_bf16_pair(acc, w_desc + adv, r_desc + adv, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          }
+          umma_commit_pair(empty_bar + s);
+          if (++s == stages) { s = 0; parity ^= 1; }
+        }
+        if (ok) {
+          umma_commit_pair(acc_full + buf);
+        } else {  // products on their way end before tensor memory is freed
+          atomicExch(error, 4);
+          umma_commit_pair(drain_bar);
+          mbar_wait(drain_bar, 0, WAIT_LIMIT_NS / 20);
+        }
+      }
+      ok = __shfl_sync(0xffffffffu, ok, 0);
+      buf ^= 1;
+      acc_parity ^= buf == 0;
+    }
+  } else {
+    const int quarter = warp & 3;
+    unsigned char* patch = patches + (warp - 2) * PATCH_BYTES;
+    int buf = 0;
+    uint32_t parity = 0;
+    for (int t = pair; tiles_of.find(t / cols, e, m0, rows); t += pairs) {
+      if (!mbar_wait(acc_full + buf, parity)) {
+        if (lane == 0) atomicExch(error, 5);
+        break;
+      }
+      __syncwarp();
+      tc_fence_after();
+      const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * BUF_COLS;
+      constexpr int MINE = BC / 4;  // features of this warp
+      const int f0 = (t % cols * 2 + (int)rank) * BC + quarter * MINE;
+      if (f0 < N) {
+        for (int c0 = (warp - 2) / 4 * 32; c0 < rows; c0 += 32 * (READERS / 4)) {
+          uint32_t v[32];
+          tmem_ld_32x32(acc + (uint32_t)c0, v);
+          const int row = m0 + c0 + lane;
+          const bool live = c0 + lane < rows;
+          float by = 1.f;
+          if (GATED && row_weights && live) by = row_weights[row];
+          tmem_wait_ld();
+          if constexpr (GATED) {
+            // an even lane has a feature's gate and the odd one after it the same feature's up: they share the rows, the even ones to
+            // the even lane
+            const bool odd = lane & 1;
 #pragma unroll
-              for (int q = 0; q < 4; ++q) pp[q] = __floats2bfloat162_rn(v[j + 2 * q], v[j + 2 * q + 1]);
-              *reinterpret_cast<uint4*>(dst + j) = pk;
+            for (int j = 0; j < 16; ++j) {
+              const float a = __uint_as_float(v[2 * j]), b = __uint_as_float(v[2 * j + 1]);
+              const float got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
+              float g = odd ? got : a, u = odd ? b : got;
+              if (row_weights) {
+                const float w = __shfl_sync(0xffffffffu, by, 2 * j + (odd ? 1 : 0));
+                g *= w;
+                u *= w;
+              }
+              *reinterpret_cast<bf16*>(patch + (2 * j + (odd ? 1 : 0)) * PATCH_PITCH + (lane >> 1) * 2) =
+                  from_float<bf16>(gated_act_of<FORM>(g, u, limit, slope));
             }
           } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (n0 + c0 + j < N) dst[j] = from_float<bf16>(v[j]);
+            for (int j = 0; j < 32; ++j) {
+              float z = __uint_as_float(v[j]);
+              if (FORM == SQUARED) {  // squared relu of the product as it would have been stored
+                z = round_to<bf16>(z);
+                z = z > 0.f ? z * z : 0.f;
+              }
+              *reinterpret_cast<bf16*>(patch + j * PATCH_PITCH + lane * 2) = from_float<bf16>(z);
+            }
           }
+          __syncwarp();
+          if (live) {
+            bf16* dst = C + (size_t)row * N + f0;
+#pragma unroll
+            for (int j = 0; j < MINE; j += 8)  // N is a multiple of 8
+              if (f0 + j < N) *reinterpret_cast<uint4*>(dst + j) = *reinterpret_cast<const uint4*>(patch + lane * PATCH_PITCH + j * 2);
+          }
+          __syncwarp();
         }
       }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(cluster_address(acc_empty + buf, 0));
+      buf ^= 1;
+      parity ^= buf == 0;
     }
-    tc_fence_before();
   }
+  __syncwarp();
+  tc_fence_before();
   __syncthreads();
+  if (rank == 0 && threadIdx.x == 0 && *issued >= 0)  // copies on their way end before shared memory is given up
+    for (int i = max(0, *issued - stages); i < *issued; ++i) mbar_wait(full_bar + i % stages, (uint32_t)(i / stages) & 1u, WAIT_LIMIT_NS / 20);
+  __syncthreads();
+  cluster_sync();  // neither block's barriers are signalled any more
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * BUF_COLS) : "memory");
   }
 }
 
-template <int BN, int STAGES, bool GATED, int MT>
-int launch_grouped(bf16* C, const bf16* A, const bf16* W, const int* offsets, int rows, int E, int N, int K, int act,
+template <Form FORM>
+int launch_grouped(bf16* C, const bf16* A, const bf16* W, const int* offsets, int rows, int E, int N, int K, int most,
                    const float* row_weights, float limit, float slope, int* error, cudaStream_t stream) {
-  static_assert(!GATED || BN == 256, "a gate tile and an up tile of 128 rows each");
-  constexpr size_t SMEM = (size_t)STAGES * (MT * A_BYTES + BN * BK * 2) + 1024 + (2 * STAGES + 1) * 8 + 16;
-  CUtensorMap map_a, map_w;
-  int rc = make_map_bf16(&map_a, A, rows, K, K, BM);
+  constexpr bool GATED = FORM == SILU || FORM == CLAMPED;
+  RowMaps maps_a;
+  CUtensorMap map_w;
+  int rc;
+  for (int b = 0; b < BOXES; ++b)
+    if ((rc = make_map_bf16(&maps_a.of[b], A, rows, K, K, BIGGEST >> b))) return rc;
+  // gated: rows [e 2 N + n] and, N rows further on, [e 2 N + N + n]: a box of 64 features brings each gate row and its up row in turn
+  rc = GATED ? make_map_bf16_3d(&map_w, W, K, 2, 2LL * E * N - N, (long long)N * K, K, 2, 64)
+             : make_map_bf16(&map_w, W, (long long)E * N, K, K, 128);
   if (rc) return rc;
-  rc = make_map_bf16(&map_w, W, (long long)E * N * (GATED ? 2 : 1), K, K, 128);
-  if (rc) return rc;
-  auto kern = grouped_gemm_kernel<BN, STAGES, GATED, MT>;
+  auto kern = grouped_gemm_kernel<FORM>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  const long long row_tiles = rows / (MT * BM) + (rows < E ? rows : E);  // an expert leaves at most one tile partly filled
-  if (row_tiles > 65535) return -3;
-  constexpr int BC = GATED ? BN / 2 : BN;
-  kern<<<dim3((N + BC - 1) / BC, (unsigned)row_tiles), 64 + 128 * MT, SMEM, stream>>>(map_a, map_w, C, offsets, E, N, K, act, row_weights,
-                                                                                limit, slope, error);
-  KRK_CHECK_LAUNCH();
-  return 0;
+  const int cols = (N + (GATED ? 127 : 255)) / (GATED ? 128 : 256);
+  const long long work = (rows / most + (long long)(rows < E ? rows : E)) * cols;  // tiles at most: an expert leaves one partly filled
+  if (work + SMS > 0x7fffffffLL) return -3;
+  return (int)launch_pdl(kern, dim3((unsigned)(2 * work < SMS ? 2 * work : SMS)), dim3(THREADS), SMEM_BYTES, stream, maps_a, map_w, C,
+                         offsets, E, N, K, most, row_weights, limit, slope, error);
 }
 
 }  // namespace
 
 // C [rows, N] = act(A [rows, K] W_e^T) over the experts' rows (offsets int32 [E + 1] on the device; rows is the most there
 // can be). act: -1 none, 5 squared relu. N and K multiples of 8, K at least 64, 16-byte aligned bases. `gated`: W [E, 2N, K],
-// act 0 (silu) or 3 (clamped swish with its limit and slope), row_weights [rows] or null. `tall`: blocks of up to 256 rows
-// (N above 128), for experts of more than 128 rows.
+// act 0 (silu) or 3 (clamped swish with its limit and slope), row_weights [rows] or null. `tall`: tiles of up to 256 of an
+// expert's rows, else of 128, which fetches the weights of experts with more rows twice.
 KRK_API int krk_grouped_gemm(void* C, const void* A, const void* W, const int* offsets, int rows, int E, int N, int K, int act,
                              int gated, int tall, const float* row_weights, float limit, float slope, int* error,
                              cudaStream_t stream) {
   if (rows == 0 || N == 0 || E == 0) return 0;
   if (N % 8 || K % 8 || K < 64 || (((uintptr_t)A | (uintptr_t)W | (uintptr_t)C) & 15) || 2LL * E * N > 0x7fffffffLL) return -2;
   if (gated ? (act != 0 && act != 3) : ((act != -1 && act != 5) || row_weights)) return -2;
-  auto go = gated ? (tall ? launch_grouped<256, 3, true, 2> : launch_grouped<256, 4, true, 1>)
-                  : N <= 128 ? launch_grouped<128, 4, false, 1>
-                             : (tall ? launch_grouped<256, 3, false, 2> : launch_grouped<256, 4, false, 1>);
-  return go((bf16*)C, (const bf16*)A, (const bf16*)W, offsets, rows, E, N, K, act, row_weights, limit, slope, error, stream);
+  auto go = gated ? (act == 3 ? launch_grouped<CLAMPED> : launch_grouped<SILU>) : (act == 5 ? launch_grouped<SQUARED> : launch_grouped<PLAIN>);
+  return go((bf16*)C, (const bf16*)A, (const bf16*)W, offsets, rows, E, N, K, tall ? 256 : 128, row_weights, limit, slope, error, stream);
 }
