@@ -62,16 +62,6 @@ struct ChunkArgs {
   const int *cu_q, *seq_qlen, *seq_slot;
 };
 
-// x and y as three pairs of bfloat16 terms each
-__device__ __forceinline__ void split3_pair(float x, float y, uint32_t (&t)[3]) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const float xa = __bfloat162float(__float2bfloat16_rn(x)), ya = __bfloat162float(__float2bfloat16_rn(y));
-    t[i] = pack_bf16x2(xa, ya);
-    x -= xa;
-    y -= ya;
-  }
-}
 // eight consecutive floats as three terms of eight bfloat16 each, 16 bytes a term
 __device__ __forceinline__ void split3_store8(const float (&f)[8], bf16* dst, size_t apart) {
   uint32_t t[4][3];

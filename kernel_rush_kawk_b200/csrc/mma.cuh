@@ -18,6 +18,17 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// x and y as three pairs of bfloat16 terms each, which add up to them (24 bits of mantissa). Two conversions at once and the widening by
+// hand: single conversions run on the unit of the exponentials, a quarter as fast.
+__device__ __forceinline__ void split3_pair(float x, float y, uint32_t (&t)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    t[i] = pack_bf16x2(x, y);
+    x -= __uint_as_float(t[i] << 16);
+    y -= __uint_as_float(t[i] & 0xffff0000u);
+  }
+}
+
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void cp_async_16(void* smem, const void* gmem) {

@@ -2,8 +2,8 @@
 //
 // The scan of recurrent.cu takes a sequence's tokens one after the other: 0.57 us a token (delta rule) or 0.40 (time
 // mixing) whatever the batch, on as many SMs as there are heads and sequences. Here a chunk's tokens become small matrix
-// products, and all chunks but for one walk run side by side. Everything is float32 on the CUDA cores, as it is there; only
-// the order of the sums differs. With the state S before the chunk, c_t the log decays summed from the chunk's first
+// products, and all chunks but for one walk run side by side. The delta rule is float32 on the CUDA cores, as it is there, and
+// time mixing float32 in three bfloat16 terms on the tensor cores; only the order of the sums differs. With the state S before the chunk, c_t the log decays summed from the chunk's first
 // token to t, and rows of the chunk's tokens:
 //
 //   time mixing:  o_t = (r_t e^{c_{t-1}}) . S + sum_{s<t} [sum_n r_tn k_sn e^{c_{t-1,n} - c_{s,n}}] v_s + (r_t . bonus k_t) v_t
@@ -23,8 +23,8 @@
 // weight and gate. Chunks of 32: a chunk of 64 needs twice the multiply-adds a token in pass 1 and halves the walk's steps.
 //
 // Measured: one prompt of 2,048 tokens, delta rule of 8 heads, 1,171 -> 107 us (the passes 62, 34 and 11); three prompts of
-// 2,553 tokens in all, time mixing of 40 heads, 405 -> 180 us (59, 13, 109). Passes 1 and 3 are bound by instruction issue
-// and shared-memory latency (a 0.4 to 0.5 share of the issue slots, 12 to 16 warps an SM), the walk by the chain of its steps.
+// 2,553 tokens in all, time mixing of 40 heads, 405 -> 128 us (45, 15, 68; with float32 on the CUDA cores 57, 15 and 115). Passes 1
+// and 3 are bound by instruction issue and latencies (a 0.4 to 0.5 share of the issue slots, 12 to 32 warps an SM), the walk by the chain of its steps.
 //
 // e^{-c_s} must stay in range. The delta rule's decay is at least e^{-decay_scale} a token, so a chunk's is bounded by the
 // parameter (the caller asks krk_recurrence_chunk_tokens). Time mixing's has no bound: a chunk in which some channel decays by
@@ -80,12 +80,18 @@ constexpr int HALF = L / 2;
 __device__ __forceinline__ void low_rank_rows(const ChunkArgs& a, float (&z)[HALF], const float* th_s, int ch0) {
   const int ch = threadIdx.x & (N - 1), t0 = threadIdx.x / N * HALF, RP = (a.R + 7) & ~7;
   const bf16* w2 = a.w2 + (size_t)(ch0 + ch) * a.R;
+  const bool wide = a.R % 8 == 0 && ((uintptr_t)a.w2 & 7) == 0;  // in pieces of four
 #pragma unroll
   for (int t = 0; t < HALF; ++t) z[t] = 0.f;
   for (int m = 0; m < RP; m += 8) {
     float w[8];
+    if (wide) {
+      st4(w, widen4(w2 + m));
+      st4(w + 4, widen4(w2 + m + 4));
+    } else {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) w[i] = m + i < a.R ? __bfloat162float(w2[m + i]) : 0.f;
+      for (int i = 0; i < 8; ++i) w[i] = m + i < a.R ? __bfloat162float(w2[m + i]) : 0.f;
+    }
 #pragma unroll
     for (int t = 0; t < HALF; ++t) {
       const float4 x = ld4(th_s + (t0 + t) * RP + m), y = ld4(th_s + (t0 + t) * RP + m + 4);
@@ -339,23 +345,54 @@ __global__ void __launch_bounds__(THREADS, 3) delta_chunk_kernel(ChunkArgs a) {
   }
 }
 
+// ---- time mixing's products on the tensor cores ------------------------------------------------------------------
+// mma.sync m16n8k16, float32 accumulate. Values are bfloat16 already; every other operand is handed over as three bfloat16 terms
+// that add up to it, and where both sides are such sums the six products that matter in 32-bit are formed, small ones first.
+constexpr int KP = N + 8;   // bfloat16 rows in shared memory: ldmatrix reads eight of them from different banks
+constexpr int PP = L + 8;
+__device__ __forceinline__ void split3_store(bf16* dst, int apart, float x) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const uint32_t b = pack_bf16x2(x, 0.f);
+    *reinterpret_cast<unsigned short*>(dst + i * apart) = (unsigned short)b;
+    x -= __uint_as_float(b << 16);
+  }
+}
+__device__ __forceinline__ void split3_store4(bf16* dst, int apart, float4 x) {
+  uint32_t lo[3], hi[3];
+  split3_pair(x.x, x.y, lo);
+  split3_pair(x.z, x.w, hi);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(dst + i * apart) = make_uint2(lo[i], hi[i]);
+}
+__device__ __forceinline__ void load_raw(bf16* dst, const bf16* src, int stride, size_t row0, int ch0, int nt) {
+#pragma unroll
+  for (int i = threadIdx.x; i < L * (N / 4); i += THREADS) {
+    const int t = i / (N / 4), c = (i % (N / 4)) * 4;
+    *reinterpret_cast<uint2*>(dst + t * KP + c) =
+        t < nt ? *reinterpret_cast<const uint2*>(src + (row0 + t) * stride + ch0 + c) : make_uint2(0u, 0u);
+  }
+}
+
 // ---- pass 1, time mixing ---------------------------------------------------------------------------------------
 // A thread has its channel's decays in registers, and sums them from either end: the weights e^{c_last - c_s} from the last token
 // back and the running sums c_t from the first one on. Neither is a difference of sums, in which a small decay after
-// large ones would be lost.
-__global__ void __launch_bounds__(THREADS) mix_chunk_kernel(ChunkArgs a) {
+// large ones would be lost. Eight blocks an SM: 45 us where seven take 50 and the float32 form took 57 (2,553 tokens, 40 heads).
+__global__ void __launch_bounds__(THREADS, 8) mix_chunk_kernel(ChunkArgs a) {
   extern __shared__ __align__(16) float sm[];
-  float* ks = sm;                // [L][PITCH] k_s e^{c_last - c_s}
-  float* vs = ks + L * PITCH;    // [L][PITCH]
-  float* th_s = vs + L * PITCH;  // [L][R rounded up]
+  bf16* kt = reinterpret_cast<bf16*>(sm);      // [3][L][KP] k_s e^{c_last - c_s}
+  bf16* vs = kt + 3 * L * KP;                  // [L][KP]
+  bf16* ks = vs + L * KP;                      // [L][KP]
+  float* th_s = reinterpret_cast<float*>(ks + L * KP);  // [L][R rounded up]
   float* total = th_s + L * ((a.R + 7) & ~7);  // [2][N]
   const int h = blockIdx.x, ci = blockIdx.y, seq = blockIdx.z, ch0 = h * N;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   grid_dependency_wait();
   const int first = (a.chunk0 + ci) * L, nt = min(L, a.seq_qlen[seq] - first);
   if (nt <= 0) return;
   const size_t row0 = (size_t)a.cu_q[seq] + first;
-  load_rows(ks, a.k, a.k_stride, row0, ch0, nt);
-  load_rows(vs, a.v, a.v_stride, row0, ch0, nt);
+  load_raw(ks, a.k, a.k_stride, row0, ch0, nt);
+  load_raw(vs, a.v, a.v_stride, row0, ch0, nt);
   load_tanh(a, th_s, row0, nt);
   __syncthreads();
   float* item = a.scratch + (((size_t)seq * a.n_chunks + ci) * a.H + h) * ITEM_MIX;
@@ -384,28 +421,43 @@ __global__ void __launch_bounds__(THREADS) mix_chunk_kernel(ChunkArgs a) {
     }
 #pragma unroll
     for (int t = HALF - 1; t >= 0; --t) {
-      ks[(t0 + t) * PITCH + ch] *= expf(after);
+      const int at = (t0 + t) * KP + ch;
+      split3_store(kt + at, L * KP, __bfloat162float(ks[at]) * expf(after));
       after += x[t];
     }
     if (__syncthreads_or(half && !(c > -SAFE)))  // pass 3 will form the pair sums from the decays themselves
 #pragma unroll
       for (int t = 0; t < HALF; ++t) item[N * N + L * N + (t0 + t) * N + ch] = expf(x[t]);
   }
-  const Place at;
-  float4 g[8];
+  const int m0 = warp * 16;  // key channels of this warp
+  float g[N / 8][4];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-  for (int s = 0; s < L; ++s) {
-    float kr[8];
-    st4(kr, ld4(ks + s * PITCH + 4 * at.ty));
-    st4(kr + 4, ld4(ks + s * PITCH + 32 + 4 * at.ty));
-    const float4 v = ld4(vs + s * PITCH + at.col);
+  for (int n = 0; n < N / 8; ++n)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) fma4(g[i], kr[i], v);
+    for (int c = 0; c < 4; ++c) g[n][c] = 0.f;
+#pragma unroll
+  for (int s = 0; s < L; s += 16) {
+    uint32_t af[3][4];
+#pragma unroll
+    for (int t = 0; t < 3; ++t)  // the transpose of the keys' rows
+      ldmatrix_x4_trans(af[t][0], af[t][1], af[t][2], af[t][3],
+                        kt + (t * L + s + (lane & 7) + ((lane >> 4) & 1) * 8) * KP + m0 + ((lane >> 3) & 1) * 8);
+#pragma unroll
+    for (int n = 0; n < N / 8; n += 2) {
+      uint32_t b[4];
+      ldmatrix_x4_trans(b[0], b[1], b[2], b[3], vs + (s + (lane & 7) + ((lane >> 3) & 1) * 8) * KP + (n + (lane >> 4)) * 8);
+#pragma unroll
+      for (int t = 2; t >= 0; --t) {
+        mma_bf16_16816(g[n], af[t][0], af[t][1], af[t][2], af[t][3], b[0], b[1]);
+        mma_bf16_16816(g[n + 1], af[t][0], af[t][1], af[t][2], af[t][3], b[2], b[3]);
+      }
+    }
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) st4(item + (32 * (i >> 2) + 4 * at.ty + (i & 3)) * N + at.col, g[i]);
+  for (int n = 0; n < N / 8; ++n)
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh)
+      *reinterpret_cast<float2*>(item + (m0 + (lane >> 2) + 8 * hh) * N + n * 8 + 2 * (lane & 3)) = make_float2(g[n][2 * hh], g[n][2 * hh + 1]);
 }
 
 // ---- pass 2 ----------------------------------------------------------------------------------------------------
@@ -508,17 +560,11 @@ __global__ void mix_walk_kernel(ChunkArgs a) {
   st4(st, run);
 }
 
-// ---- pass 3 ----------------------------------------------------------------------------------------------------
-template <int RULE>
-__global__ void __launch_bounds__(THREADS) chunk_finish_kernel(ChunkArgs a) {
+// ---- pass 3, delta rule ----------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(THREADS) delta_finish_kernel(ChunkArgs a) {
   extern __shared__ __align__(16) float sm[];
   float* qs = sm;                 // [L][PITCH] rows that meet the state
   float* red = qs + L * PITCH;    // [4][L] sums of squares of a warp's columns
-  float* ks = red + 4 * L;        // time mixing: [L][PITCH] k_s e^{-c_s}
-  float* vs = ks + L * PITCH;     // [L][PITCH]
-  float* cs = vs + L * PITCH;     // [L][PITCH] decays, where a channel forgets too much
-  float* ps = cs + L * PITCH;     // [L][L + 4] pair sums
-  constexpr int PP = L + 4;
   grid_launch_dependents();
   grid_dependency_wait();
   const int h = blockIdx.x, ci = blockIdx.y, seq = blockIdx.z, ch0 = h * N;
@@ -526,109 +572,21 @@ __global__ void __launch_bounds__(THREADS) chunk_finish_kernel(ChunkArgs a) {
   const int first = (a.chunk0 + ci) * L, qlen = a.seq_qlen[seq], nt = min(L, qlen - first);
   if (nt <= 0) return;
   const size_t row0 = (size_t)a.cu_q[seq] + first;
-  const size_t index = ((size_t)seq * a.n_chunks + ci) * a.H + h;
-  const float* item = a.scratch + index * (RULE == 1 ? ITEM_DELTA : ITEM_MIX);
+  const float* item = a.scratch + (((size_t)seq * a.n_chunks + ci) * a.H + h) * ITEM_DELTA;
   const Place at;
   // the state before the chunk: a value column is one warp's alone, so it is read from memory where it is used
-  const float* start = item + (RULE == 1 ? N * N : 0) + at.col;
+  const float* start = item + N * N + at.col;
   auto state4 = [&](int n) { return __ldcg(reinterpret_cast<const float4*>(start + n * N)); };
   float4 o[4], s0[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) s0[j] = state4(j);
-  if (RULE == 1) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) o[i] = __ldcg(reinterpret_cast<const float4*>(item + 2 * N * N + L * N + (at.ty + 8 * i) * N + at.col));
-    for (int i = tid; i < L * (N / 4); i += THREADS)
-      cp_async_16(qs + (i / (N / 4)) * PITCH + (i % (N / 4)) * 4, item + 2 * N * N + 4 * i);
-    cp_async_commit();
-    cp_async_wait<0>();
-    __syncthreads();
-  } else {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float* cum = item + N * N;
-    const int n = (tid % (N / 4)) * 4;  // this thread's four channels of tokens tid / 16, 8 further on, ...
-    constexpr int EACH = L * (N / 4) / THREADS;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 end = __ldcg(reinterpret_cast<const float4*>(cum + (L - 1) * N + n)), by = ld4(a.bonus + ch0 + n);
-    float4 q[EACH], k[EACH], c[EACH], b[EACH];
-    load_rows(vs, a.v, a.v_stride, row0, ch0, nt);
-#pragma unroll
-    for (int i = 0; i < EACH; ++i) {
-      const int t = tid / (N / 4) + i * (THREADS / (N / 4));
-      q[i] = t < nt ? widen4(a.r + (row0 + t) * a.r_stride + ch0 + n) : zero;
-      k[i] = t < nt ? widen4(a.k + (row0 + t) * a.k_stride + ch0 + n) : zero;
-      c[i] = __ldcg(reinterpret_cast<const float4*>(cum + t * N + n));
-      b[i] = t ? __ldcg(reinterpret_cast<const float4*>(cum + (t - 1) * N + n)) : zero;
-    }
-    const bool safe = !__syncthreads_or(!(end.x > -SAFE) || !(end.y > -SAFE) || !(end.z > -SAFE) || !(end.w > -SAFE));
-    if (!safe) {  // a token's key, as the tokens after it find it: a thread a token and a quarter of the channels
-      const float* decays = cum + L * N;
-#pragma unroll
-      for (int i = 0; i < EACH; ++i) {
-        const int t = tid / (N / 4) + i * (THREADS / (N / 4)), at4 = t * PITCH + n;
-        st4(qs + at4, q[i]);
-        st4(ks + at4, k[i]);
-        st4(cs + at4, __ldcg(reinterpret_cast<const float4*>(decays + t * N + n)));
-      }
-      __syncthreads();
-      const int s = tid >> 2, m0 = (tid & 3) * 4;
-      float4 w[N / 16];
-#pragma unroll
-      for (int j = 0; j < N / 16; ++j) w[j] = ld4(ks + s * PITCH + m0 + 16 * j);
-      for (int t = 0; t < L; ++t) {
-        float d = 0.f;
-#pragma unroll
-        for (int j = 0; j < N / 16; ++j) d = dot4(ld4(qs + t * PITCH + m0 + 16 * j), w[j], d);
-        d += __shfl_xor_sync(0xffffffffu, d, 1);
-        d += __shfl_xor_sync(0xffffffffu, d, 2);
-        if (m0 == 0 && s != t) ps[t * PP + s] = s < t ? d : 0.f;
-        if (s < t)
-#pragma unroll
-          for (int j = 0; j < N / 16; ++j) {
-            const float4 e = ld4(cs + t * PITCH + m0 + 16 * j);
-            w[j].x *= e.x; w[j].y *= e.y; w[j].z *= e.z; w[j].w *= e.w;
-          }
-      }
-      __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < EACH; ++i) {
-      const int t = tid / (N / 4) + i * (THREADS / (N / 4));
-      float bonus = q[i].x * by.x * k[i].x + q[i].y * by.y * k[i].y + q[i].z * by.z * k[i].z + q[i].w * by.w * k[i].w;
-#pragma unroll
-      for (int off = 1; off < N / 4; off <<= 1) bonus += __shfl_xor_sync(0xffffffffu, bonus, off);
-      if (n == 0) ps[t * PP + t] = bonus;
-      st4(qs + t * PITCH + n, make_float4(q[i].x * expf(b[i].x), q[i].y * expf(b[i].y), q[i].z * expf(b[i].z), q[i].w * expf(b[i].w)));
-      if (safe)
-        st4(ks + t * PITCH + n, make_float4(k[i].x * expf(-c[i].x), k[i].y * expf(-c[i].y), k[i].z * expf(-c[i].z), k[i].w * expf(-c[i].w)));
-    }
-    __syncthreads();
-    if (safe) {  // rows ty, ty + 8, ...; columns x, x + 16 of the pair sums
-      const int x = at.col / 4;
-      float e[4][2];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) e[i][0] = e[i][1] = 0.f;
-#pragma unroll 4
-      for (int m = 0; m < N; m += 4) {
-        const float4 k0 = ld4(ks + x * PITCH + m), k1 = ld4(ks + (x + 16) * PITCH + m);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float4 r = ld4(qs + (at.ty + 8 * i) * PITCH + m);
-          e[i][0] = dot4(r, k0, e[i][0]);
-          e[i][1] = dot4(r, k1, e[i][1]);
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int u = at.ty + 8 * i, s = x + 16 * j;
-          if (s != u) ps[u * PP + s] = s < u ? e[i][j] : 0.f;
-        }
-      __syncthreads();
-    }
-  }
+  for (int i = 0; i < 4; ++i) o[i] = __ldcg(reinterpret_cast<const float4*>(item + 2 * N * N + L * N + (at.ty + 8 * i) * N + at.col));
+  for (int i = tid; i < L * (N / 4); i += THREADS)
+    cp_async_16(qs + (i / (N / 4)) * PITCH + (i % (N / 4)) * 4, item + 2 * N * N + 4 * i);
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
 #pragma unroll 2
   for (int n = 0; n < N; n += 4) {
     float4 s1[4];
@@ -644,21 +602,6 @@ __global__ void __launch_bounds__(THREADS) chunk_finish_kernel(ChunkArgs a) {
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) s0[j] = s1[j];
-  }
-  if (RULE == 0) {
-#pragma unroll 2
-    for (int s = 0; s < L; s += 4) {
-      float p[4][4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) st4(p[i], ld4(ps + (at.ty + 8 * i) * PP + s));
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float4 v = ld4(vs + (s + j) * PITCH + at.col);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (s + j <= at.ty + 8 * i) fma4(o[i], p[i][j], v);  // a later token's infinities stay its own
-      }
-    }
   }
   // per head: divide by the root mean square, weight, gate, scale
 #pragma unroll
@@ -677,11 +620,268 @@ __global__ void __launch_bounds__(THREADS) chunk_finish_kernel(ChunkArgs a) {
     const float sum = (red[t] + red[L + t]) + (red[2 * L + t] + red[3 * L + t]);
     const float by = rsqrtf(sum / (float)N + a.eps) * a.out_scale;
     const float4 g = widen4(a.g + (row0 + t) * a.g_stride + ch0 + at.col);
-    auto gate = [](float x) { return RULE == 1 ? sigmoid_f(x) : x * sigmoid_f(x); };
     uint2 raw;
-    raw.x = pack_bf16x2(o[i].x * by * w.x * gate(g.x), o[i].y * by * w.y * gate(g.y));
-    raw.y = pack_bf16x2(o[i].z * by * w.z * gate(g.z), o[i].w * by * w.w * gate(g.w));
+    raw.x = pack_bf16x2(o[i].x * by * w.x * sigmoid_f(g.x), o[i].y * by * w.y * sigmoid_f(g.y));
+    raw.y = pack_bf16x2(o[i].z * by * w.z * sigmoid_f(g.z), o[i].w * by * w.w * sigmoid_f(g.w));
     *reinterpret_cast<uint2*>(a.out + (row0 + t) * a.out_stride + a.out_col + ch0 + at.col) = raw;
+  }
+  if (a.last_rows && h == 0 && first + nt == qlen) {  // the sequence's last row, for the next step's token shift
+    const bf16* row = a.last_rows + (row0 + nt - 1) * a.last_stride;
+    float* dst = a.last_state + (size_t)a.seq_slot[seq] * a.C;
+    for (int c = tid; c < a.C; c += THREADS) dst[c] = __bfloat162float(row[c]);
+  }
+}
+
+// ---- pass 3, time mixing ---------------------------------------------------------------------------------------
+// Bound by what surrounds the products: loads, exponentials, splitting and barriers; the tensor cores are busy a quarter of the time. Five
+// blocks an SM (six spill: 84 us against 72 at 3 sequences of 2,553 tokens, 40 heads; the float32 form 115). A warp makes 16 value columns of all tokens. Of a warp's 16 columns the even ones are one tile of the products and the odd ones
+// another: a row's piece of the state is then one 8-byte load for both, and a thread ends with four neighbouring columns.
+__global__ void __launch_bounds__(THREADS, 5) mix_finish_kernel(ChunkArgs a) {
+  extern __shared__ __align__(16) float sm[];
+  bf16* qt = reinterpret_cast<bf16*>(sm);  // [3][L][KP] r_t e^{c_{t-1}}
+  bf16* kt = qt + 3 * L * KP;              // [3][L][KP] k_s e^{-c_s}; then
+  bf16* pt = kt;                           // [3][L][PP] the pair sums
+  bf16* vs = kt + 3 * L * KP;              // [L][KP], the columns of 16 ordered as the products want them
+  float* red = reinterpret_cast<float*>(vs + L * KP);  // [4][L] sums of squares of a warp's columns
+  float* own = red + 4 * L;                // [L] a token's own share, through the bonus
+  int* bad = reinterpret_cast<int*>(own + L);  // [2][N]: the first token with an infinity in a value column, with a NaN
+  // where a channel forgets too much, as float32, before qt and pt are written
+  float* es = sm;                                  // [L][PITCH] decays
+  float* rs = reinterpret_cast<float*>(kt);        // [L][PITCH] queries
+  float* ps = rs + L * PITCH;                      // [L][L + 4] pair sums
+  static_assert(L * PITCH * 4 <= 3 * L * KP * 2 && (L * PITCH + L * (L + 4)) * 4 <= 3 * L * KP * 2 && 3 * L * PP * 2 <= L * PITCH * 4, "room");
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int h = blockIdx.x, ci = blockIdx.y, seq = blockIdx.z, ch0 = h * N;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
+  const int first = (a.chunk0 + ci) * L, qlen = a.seq_qlen[seq], nt = min(L, qlen - first);
+  if (nt <= 0) return;
+  const size_t row0 = (size_t)a.cu_q[seq] + first;
+  const float* item = a.scratch + (((size_t)seq * a.n_chunks + ci) * a.H + h) * ITEM_MIX;
+  const float* cum = item + N * N;
+  constexpr int EACH = L * (N / 4) / THREADS;
+  const int n = (tid % (N / 4)) * 4, tq = tid / (N / 4);  // this thread's four channels of tokens tq, tq + 8, ...
+  bool safe;
+  {
+    uint2 q[EACH], k[EACH], v[EACH];
+    float4 c[EACH], b[EACH];
+    const float4 end = __ldcg(reinterpret_cast<const float4*>(cum + (L - 1) * N + n)), by = ld4(a.bonus + ch0 + n);
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) {
+      const int t = tq + i * (THREADS / (N / 4));
+      const bool in = t < nt;
+      q[i] = in ? *reinterpret_cast<const uint2*>(a.r + (row0 + t) * a.r_stride + ch0 + n) : make_uint2(0u, 0u);
+      k[i] = in ? *reinterpret_cast<const uint2*>(a.k + (row0 + t) * a.k_stride + ch0 + n) : make_uint2(0u, 0u);
+      v[i] = in ? *reinterpret_cast<const uint2*>(a.v + (row0 + t) * a.v_stride + ch0 + n) : make_uint2(0u, 0u);
+      c[i] = __ldcg(reinterpret_cast<const float4*>(cum + t * N + n));
+      b[i] = t ? __ldcg(reinterpret_cast<const float4*>(cum + (t - 1) * N + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (tid < 2 * N) bad[tid] = L;
+    safe = !__syncthreads_or(!(end.x > -SAFE) || !(end.y > -SAFE) || !(end.z > -SAFE) || !(end.w > -SAFE));
+    auto widen = [](uint2 raw) {
+      const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&raw.x), hi = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
+      return make_float4(__low2float(lo), __high2float(lo), __low2float(hi), __high2float(hi));
+    };
+    if (!safe) {  // a token's key, as the tokens after it find it: a thread a token and a quarter of the channels
+      const float* decays = cum + L * N;
+#pragma unroll
+      for (int i = 0; i < EACH; ++i) {
+        const int t = tq + i * (THREADS / (N / 4)), at4 = t * PITCH + n;
+        st4(rs + at4, widen(q[i]));
+        st4(es + at4, __ldcg(reinterpret_cast<const float4*>(decays + t * N + n)));
+      }
+      const int s = tid >> 2, m0 = (tid & 3) * 4;
+      float4 w[N / 16];
+#pragma unroll
+      for (int j = 0; j < N / 16; ++j)
+        w[j] = s < nt ? widen4(a.k + (row0 + s) * a.k_stride + ch0 + m0 + 16 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+      __syncthreads();
+      for (int t = 0; t < L; ++t) {
+        float d = 0.f;
+#pragma unroll
+        for (int j = 0; j < N / 16; ++j) d = dot4(ld4(rs + t * PITCH + m0 + 16 * j), w[j], d);
+        d += __shfl_xor_sync(0xffffffffu, d, 1);
+        d += __shfl_xor_sync(0xffffffffu, d, 2);
+        if (m0 == 0) ps[t * (L + 4) + s] = s < t ? d : 0.f;
+        if (s < t)
+#pragma unroll
+          for (int j = 0; j < N / 16; ++j) {
+            const float4 e = ld4(es + t * PITCH + m0 + 16 * j);
+            w[j].x *= e.x; w[j].y *= e.y; w[j].z *= e.z; w[j].w *= e.w;
+          }
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) {
+      const int t = tq + i * (THREADS / (N / 4));
+      const float4 qf = widen(q[i]), kf = widen(k[i]);
+      float bonus = qf.x * by.x * kf.x + qf.y * by.y * kf.y + qf.z * by.z * kf.z + qf.w * by.w * kf.w;
+#pragma unroll
+      for (int off = 1; off < N / 4; off <<= 1) bonus += __shfl_xor_sync(0xffffffffu, bonus, off);
+      if (n == 0) own[t] = bonus;
+      split3_store4(qt + t * KP + n, L * KP, make_float4(qf.x * expf(b[i].x), qf.y * expf(b[i].y), qf.z * expf(b[i].z), qf.w * expf(b[i].w)));
+      if (safe)
+        split3_store4(kt + t * KP + n, L * KP, make_float4(kf.x * expf(-c[i].x), kf.y * expf(-c[i].y), kf.z * expf(-c[i].z), kf.w * expf(-c[i].w)));
+      // columns n, n + 2 side by side in the even tile, n + 1, n + 3 in the odd one; what is not finite is set aside, since a product
+      // would hand it, times zero, to the tokens before
+      uint32_t even = __byte_perm(v[i].x, v[i].y, 0x5410), odd = __byte_perm(v[i].x, v[i].y, 0x7632);
+      auto finite = [](uint32_t two) { return (two & 0x7f80u) != 0x7f80u && (two & 0x7f800000u) != 0x7f800000u; };
+      if (!finite(even) || !finite(odd)) {
+        auto aside = [&](uint32_t& two, int col) {
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const uint32_t one = two >> (16 * j) & 0xffffu;
+            if ((one & 0x7f80u) != 0x7f80u) continue;
+            atomicMin(bad + (one & 0x7fu ? N : 0) + col + 2 * j, t);
+            two &= j ? 0x0000ffffu : 0xffff0000u;
+          }
+        };
+        aside(even, n);
+        aside(odd, n + 1);
+      }
+      bf16* to = vs + t * KP + (n & ~15) + ((n & 15) >> 1);
+      *reinterpret_cast<uint32_t*>(to) = even;
+      *reinterpret_cast<uint32_t*>(to + 8) = odd;
+    }
+  }
+  __syncthreads();
+  // the state before the chunk: a value column is one warp's alone, so it comes from memory straight into the products' fragments
+  const float* start = item + warp * 16 + 2 * g;
+  float2 st[N / 16][4];
+#pragma unroll
+  for (int kk = 0; kk < N / 16; ++kk)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      st[kk][i] = __ldcg(reinterpret_cast<const float2*>(start + (kk * 16 + 2 * t4 + (i & 1) + 8 * (i >> 1)) * N));
+  // pair sums: warp 0 tokens 0..15, warps 1 and 2 tokens 16..31, each against 16 of the tokens before
+  const int mt = warp ? 1 : 0, u0 = warp == 2 ? 16 : 0;
+  float e[2][4];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) e[j][c] = 0.f;
+  if (safe && warp < 3) {
+#pragma unroll
+    for (int kk = 0; kk < N; kk += 16) {
+      uint32_t af[3][4], b[3][4];
+#pragma unroll
+      for (int t = 0; t < 3; ++t) {
+        ldmatrix_x4(af[t][0], af[t][1], af[t][2], af[t][3], qt + (t * L + mt * 16 + (lane & 15)) * KP + kk + (lane >> 4) * 8);
+        ldmatrix_x4(b[t][0], b[t][1], b[t][2], b[t][3], kt + (t * L + u0 + ((lane >> 4) << 3) + (lane & 7)) * KP + kk + ((lane >> 3) & 1) * 8);
+      }
+#pragma unroll
+      for (int sum = 2; sum >= 0; --sum)
+#pragma unroll
+        for (int t = 0; t <= sum; ++t) {
+          mma_bf16_16816(e[0], af[t][0], af[t][1], af[t][2], af[t][3], b[sum - t][0], b[sum - t][1]);
+          mma_bf16_16816(e[1], af[t][0], af[t][1], af[t][2], af[t][3], b[sum - t][2], b[sum - t][3]);
+        }
+    }
+  }
+  if (safe) {
+    __syncthreads();  // the keys are no longer read
+    if (warp < 3) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+          const int t = mt * 16 + g + 8 * hh, s = u0 + j * 8 + 2 * t4;
+          float p[2];
+#pragma unroll
+          for (int c = 0; c < 2; ++c) p[c] = s + c < t ? e[j][2 * hh + c] : s + c == t ? own[t] : 0.f;
+          uint32_t three[3];
+          split3_pair(p[0], p[1], three);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(pt + (i * L + t) * PP + s) = three[i];
+        }
+    }
+  } else {
+    for (int i = tid; i < L * (L / 2); i += THREADS) {
+      const int t = i / (L / 2), s = (i % (L / 2)) * 2;
+      uint32_t three[3];
+      split3_pair(s == t ? own[t] : ps[t * (L + 4) + s], s + 1 == t ? own[t] : ps[t * (L + 4) + s + 1], three);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) *reinterpret_cast<uint32_t*>(pt + (j * L + t) * PP + s) = three[j];
+    }
+  }
+  const int col = warp * 16 + 4 * t4;  // this thread's columns, of tokens g, g + 8, g + 16, g + 24
+  uint2 gate[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    gate[i] = g + 8 * i < nt ? *reinterpret_cast<const uint2*>(a.g + (row0 + g + 8 * i) * a.g_stride + ch0 + col) : make_uint2(0u, 0u);
+  float o[2][2][4];  // [16 tokens][even, odd columns]
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) o[m][j][c] = 0.f;
+#pragma unroll
+  for (int kk = 0; kk < N / 16; ++kk) {
+    uint32_t b[2][2][3];
+    split3_pair(st[kk][0].x, st[kk][1].x, b[0][0]);
+    split3_pair(st[kk][2].x, st[kk][3].x, b[0][1]);
+    split3_pair(st[kk][0].y, st[kk][1].y, b[1][0]);
+    split3_pair(st[kk][2].y, st[kk][3].y, b[1][1]);
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      uint32_t af[3][4];
+#pragma unroll
+      for (int t = 0; t < 3; ++t)
+        ldmatrix_x4(af[t][0], af[t][1], af[t][2], af[t][3], qt + (t * L + m * 16 + (lane & 15)) * KP + kk * 16 + (lane >> 4) * 8);
+#pragma unroll
+      for (int sum = 2; sum >= 0; --sum)
+#pragma unroll
+        for (int t = 0; t <= sum; ++t)
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            mma_bf16_16816(o[m][j], af[t][0], af[t][1], af[t][2], af[t][3], b[j][0][sum - t], b[j][1][sum - t]);
+    }
+  }
+  __syncthreads();  // the pair sums are here
+#pragma unroll
+  for (int kk = 0; kk < 2; ++kk) {
+    uint32_t b[4];
+    ldmatrix_x4_trans(b[0], b[1], b[2], b[3], vs + (kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * KP + warp * 16 + (lane >> 4) * 8);
+#pragma unroll
+    for (int m = kk; m < 2; ++m)
+#pragma unroll
+      for (int t = 2; t >= 0; --t) {
+        uint32_t af[4];
+        ldmatrix_x4(af[0], af[1], af[2], af[3], pt + (t * L + m * 16 + (lane & 15)) * PP + kk * 16 + (lane >> 4) * 8);
+        mma_bf16_16816(o[m][0], af[0], af[1], af[2], af[3], b[0], b[1]);
+        mma_bf16_16816(o[m][1], af[0], af[1], af[2], af[3], b[2], b[3]);
+      }
+  }
+  // per head: divide by the root mean square, weight, gate, scale
+  const int4 inf = *reinterpret_cast<const int4*>(bad + col), nan = *reinterpret_cast<const int4*>(bad + N + col);
+  float4 y[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int m = i >> 1, hh = i & 1, t = g + 8 * i;
+    y[i] = make_float4(o[m][0][2 * hh], o[m][1][2 * hh], o[m][0][2 * hh + 1], o[m][1][2 * hh + 1]);
+    auto kept = [&](float x, int inf, int nan) { return t >= nan ? NAN : t >= inf ? INFINITY : x; };
+    y[i] = make_float4(kept(y[i].x, inf.x, nan.x), kept(y[i].y, inf.y, nan.y), kept(y[i].z, inf.z, nan.z), kept(y[i].w, inf.w, nan.w));
+    float sq = y[i].x * y[i].x + y[i].y * y[i].y + y[i].z * y[i].z + y[i].w * y[i].w;
+    sq += __shfl_xor_sync(0xffffffffu, sq, 1);
+    sq += __shfl_xor_sync(0xffffffffu, sq, 2);
+    if (t4 == 0) red[warp * L + t] = sq;
+  }
+  __syncthreads();
+  const float4 w = ld4(a.norm_w + ch0 + col);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int t = g + 8 * i;
+    if (t >= nt) continue;
+    const float sum = (red[t] + red[L + t]) + (red[2 * L + t] + red[3 * L + t]);
+    const float by = rsqrtf(sum / (float)N + a.eps) * a.out_scale;
+    const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&gate[i].x), hi = *reinterpret_cast<const __nv_bfloat162*>(&gate[i].y);
+    auto silu = [](float x) { return __fdividef(x, 1.0f + __expf(-x)); };
+    uint2 raw;
+    raw.x = pack_bf16x2(y[i].x * by * w.x * silu(__low2float(lo)), y[i].y * by * w.y * silu(__high2float(lo)));
+    raw.y = pack_bf16x2(y[i].z * by * w.z * silu(__low2float(hi)), y[i].w * by * w.w * silu(__high2float(hi)));
+    *reinterpret_cast<uint2*>(a.out + (row0 + t) * a.out_stride + a.out_col + ch0 + col) = raw;
   }
   if (a.last_rows && h == 0 && first + nt == qlen) {  // the sequence's last row, for the next step's token shift
     const bf16* row = a.last_rows + (row0 + nt - 1) * a.last_stride;
@@ -741,9 +941,10 @@ KRK_API int krk_recurrence_chunks(int rule, const void* r, int r_stride, const v
     if ((rc = run(delta_chunk_kernel, items, THREADS, 8 * (size_t)L * PITCH + N + L, a, stream))) return rc;
     const size_t walk = (size_t)WALK_STAGES * N * (PITCH + WALK_COLS) + N * WALK_COLS + 4 * N * 4;
     if ((rc = run(delta_walk_kernel, dim3(N / WALK_COLS, (unsigned)H, (unsigned)n_seqs), THREADS, walk, a, stream))) return rc;
-    return run(chunk_finish_kernel<1>, items, THREADS, (size_t)L * PITCH + 4 * L, a, stream);
+    return run(delta_finish_kernel, items, THREADS, (size_t)L * PITCH + 4 * L, a, stream);
   }
-  if ((rc = run(mix_chunk_kernel, items, THREADS, 2 * (size_t)L * PITCH + L * RP + 2 * N, a, stream))) return rc;
+  const size_t rows_bytes = (size_t)L * KP * sizeof(bf16);  // a term of a chunk's rows
+  if ((rc = run(mix_chunk_kernel, items, THREADS, 5 * rows_bytes / sizeof(float) + L * RP + 2 * N, a, stream))) return rc;
   if ((rc = run(mix_walk_kernel, dim3(N * N / 4 / 64, (unsigned)H, (unsigned)n_seqs), 64, 0, a, stream))) return rc;
-  return run(chunk_finish_kernel<0>, items, THREADS, 4 * (size_t)L * PITCH + 4 * L + (size_t)L * (L + 4), a, stream);
+  return run(mix_finish_kernel, items, THREADS, 7 * rows_bytes / sizeof(float) + 5 * L + 2 * N, a, stream);
 }
