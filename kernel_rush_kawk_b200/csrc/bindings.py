@@ -173,6 +173,9 @@ def _ptr(t) -> int | None:
     return None if t is None else t.data_ptr()
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
+
+
 class Kernels:
     """All kernels, for one device. ``head_dims``: the head sizes whose attention
     libraries are needed (compiled at first use)."""
@@ -233,7 +236,9 @@ class Kernels:
 
     # -- plumbing -------------------------------------------------------------
     def _stream(self):
-        return torch.cuda.current_stream(self.device).cuda_stream
+        # the current stream's handle itself: the stream object around it costs 5 us of the host's time, and a prompt's layer, which is
+        # not replayed from a graph, asks ten times
+        return _raw_stream(torch.cuda.current_device() if self.device.index is None else self.device.index)
 
     def _ok(self, code: int, what: str) -> None:
         self.launches += 1
