@@ -109,8 +109,8 @@ _MEMORY_SIGNATURES = {
     "krk_memory_chunk_decays": [_P, _P, c_int, _P, _P, c_float, c_int, c_int, c_int, c_int, _P, _P, _P],
     "krk_memory_chunks": [_P, _P, _P, c_int, _P, c_int, _P, c_int, c_float, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int,
                           _P, _P, _P, _P],
-    "krk_ssd_steps": [_P, _P, c_int, _P, _P, c_int, c_int, _P],
-    "krk_ssd_chunks": [_P, _P, c_int, _P, c_int, _P, c_int, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
+    "krk_ssd_steps": [_P, _P, c_int, _P, _P, c_int, c_int, c_int, c_int, _P, _P, _P],
+    "krk_ssd_chunks": [_P, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                        _P, _P, _P, _P],
     "krk_memory_finish": [_P, c_int, c_int, c_float, _P, _P, _P, _P, c_int, _P, c_int, c_int, c_float, c_int, c_int, _P],
 }
@@ -1567,16 +1567,17 @@ class Kernels:
         # a long step goes through its chunks in portions, so that their states stay within SSD_SCRATCH
         portion = max(1, min(chunks, 65535 // heads, self.SSD_SCRATCH // (4 * state_floats)))
         # the chunks' states, a decay for each of their rows, and every row's step sizes and log decays
-        scratch, portion = self._chunk_scratch(state_floats + batch.n_seqs * heads * N, portion, y.device, beside=2 * rows * heads)
+        scratch, portion = self._chunk_scratch(state_floats + batch.n_seqs * heads * N, portion, y.device, beside=4 * rows * heads)
         if not portion:
             return False
         sums = scratch.data_ptr()
         decays = sums + 4 * portion * state_floats
         steps = decays + 4 * portion * batch.n_seqs * heads * N
-        self._ok(self.memory.krk_ssd_steps(steps, dp, ds, dt_bias.data_ptr(), a_log.data_ptr(), rows, heads, self._stream()),
+        self._ok(self.memory.krk_ssd_steps(steps, dp, ds, dt_bias.data_ptr(), a_log.data_ptr(), rows, heads, batch.n_seqs,
+                                             batch.max_q_len, batch.cu_q.data_ptr(), batch.seq_qlen.data_ptr(), self._stream()),
                  "step sizes and decays")
         for first in range(0, chunks, portion):
-            self._ok(self.memory.krk_ssd_chunks(y.data_ptr(), xp, xs, bp, bs, cp, cs_, steps, skip.data_ptr(),
+            self._ok(self.memory.krk_ssd_chunks(y.data_ptr(), xp, xs, bp, bs, cp, cs_, steps, rows, skip.data_ptr(),
                                                 state.data_ptr(), sums, decays, heads, P, N, groups,
                                                 batch.n_seqs, first, min(portion, chunks - first), batch.cu_q.data_ptr(),
                                                 batch.seq_qlen.data_ptr(), batch.seq_slot.data_ptr(), self._stream()),

@@ -19,10 +19,10 @@
 //
 // A state-space mixer (ssd.cu) is a third kind: q and k are its C and B, one row of each for a group of heads, v its x, the decay
 // one number per head and token, and x_s counts dt_s times: A_ts = (C_t . B_s) e^{F_t - F_s} dt_s, r_t = e^{F_t}, w_s = e^{F_last - F_s} dt_s,
-// plus skip * x_t in the output. Its log decays are as large as the step sizes make them, so they are summed and subtracted in
-// 64-bit: e^{F_t - F_s} is then as exact as the product of the decays that the scan token by token forms. One prompt of 2,048
-// tokens, 48 heads of 64 with 128 rows: the scan's three passes on the CUDA cores
-// 403 us, these 114 (31, 16 and 66).
+// plus skip * x_t in the output. Its log decays are as large as the step sizes make them, so they are summed in 64-bit and kept as two
+// floats: e^{F_t - F_s} is then as exact as the product of the decays that the scan token by token forms. One prompt of 2,048
+// tokens, 48 heads of 64 with 128 rows: the scan's three passes on the CUDA cores 403 us, these 90 (22, 16 and 50; 114 with a block
+// a head: 31, 16 and 66).
 //
 // Three passes: (1) every chunk's own sum_s (w_s k_s) v_s^T; (2) the walk over a sequence's chunks, which leaves every
 // chunk its starting state and the sequence its final one; (3) the outputs. A block takes some slices of 64 value
@@ -31,7 +31,7 @@
 
 namespace {
 
-enum Kind { DECAYS, RUNNING_MAX, STATE_SPACE };
+enum Kind { DECAYS, RUNNING_MAX };
 
 constexpr int L = 64;        // tokens per chunk
 constexpr int PB = 64;       // value columns per block
@@ -55,9 +55,11 @@ struct ChunkArgs {
   float* cd;            // [n_seqs, max_chunks, H, N]: a chunk's decays
   int H, N, P, max_chunks;
   int slices;  // column slices a block walks
-  const float2* steps;  // state-space kind: [rows, H]: (log decay, dt)
+  const float4* steps;  // state-space kind: [H, rows]: log decays summed within the chunk (two floats), dt, e^{F_last - F_s} dt
+  int rows;
   const float* skip;    // state-space kind: [H]
   int per_group;        // heads that share a row of q and k
+  int units, parts;     // state-space kind: (head, column slice) pairs a block takes of those of a group; blocks for a group
   int chunk0;           // the chunks of every sequence that this launch takes start here
   const int *cu_q, *seq_qlen, *seq_slot;
 };
@@ -91,28 +93,6 @@ __device__ __forceinline__ void chunk_sums(float* F, const float* f, int lane) {
   F[2 * lane + 1] = before + b;
 }
 
-// the same sums in 64-bit
-__device__ __forceinline__ void chunk_sums_64(double* F, const float* f, int lane) {
-  const double a = f[2 * lane], b = a + f[2 * lane + 1];
-  double run = b;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const double p = __shfl_up_sync(0xffffffffu, run, o);
-    if (lane >= o) run += p;
-  }
-  F[2 * lane] = (run - b) + a;
-  F[2 * lane + 1] = run;
-}
-
-// state-space kind: log decays and step sizes of the chunk's tokens, zeros beyond the last
-__device__ __forceinline__ void load_steps(const ChunkArgs& a, float* f, float* dt, size_t row0, int h, int nt) {
-  if (threadIdx.x < L) {
-    const float2 s = threadIdx.x < nt ? a.steps[(row0 + threadIdx.x) * a.H + h] : make_float2(0.f, 0.f);
-    f[threadIdx.x] = s.x;
-    dt[threadIdx.x] = s.y;
-  }
-}
-
 __device__ __forceinline__ void load_values(bf16* vs, const ChunkArgs& a, size_t row0, int h, int p0, int nt) {
   for (int i = threadIdx.x; i < L * (PB / 8); i += THREADS) {
     const int s = i / (PB / 8), c = (i % (PB / 8)) * 8;
@@ -122,32 +102,15 @@ __device__ __forceinline__ void load_values(bf16* vs, const ChunkArgs& a, size_t
   }
 }
 
-// Values that are not finite, out of a slice of values in shared memory (a zero in their place): bad[c] becomes the first
-// token that holds one in column c. A matrix product would hand them, times zero, to the tokens before.
-__device__ __forceinline__ void set_aside_infinities(bf16* vs, int* bad) {
-  for (int i = threadIdx.x; i < L * (PB / 2); i += THREADS) {
-    const int s = i / (PB / 2), c = (i % (PB / 2)) * 2;
-    uint32_t* at = reinterpret_cast<uint32_t*>(vs + s * VPITCH + c);
-    const uint32_t two = *at;
-    const bool lo = (two & 0x7f80u) == 0x7f80u, hi = (two & 0x7f800000u) == 0x7f800000u;
-    if (lo) atomicMin(bad + c, s);
-    if (hi) atomicMin(bad + c + 1, s);
-    if (lo || hi) *at = two & (lo ? 0xffff0000u : 0xffffffffu) & (hi ? 0xffffu : 0xffffffffu);
-  }
-}
-
 // ---- pass 1: the chunk's own sum of (w k) v^T, and its decays ------------------------------------------------
 template <Kind KIND>
 __global__ void __launch_bounds__(THREADS) chunk_sum_kernel(ChunkArgs a) {
-  constexpr bool GATED = KIND == RUNNING_MAX, SCALAR = KIND != DECAYS;
+  constexpr bool GATED = KIND == RUNNING_MAX;
   extern __shared__ __align__(16) bf16 sm[];
   __shared__ float fs[L], is_[L], Fs[L], ws[L];
-  __shared__ double Fd[L];
   const int N = a.N, P = a.P, H = a.H, NP = N + 8;
-  // where a token's weight is one number it multiplies the values instead of the keys: they are fewer, and the keys stay exact
-  constexpr int KT = KIND == STATE_SPACE ? 1 : 3, VT = KIND == STATE_SPACE ? 3 : 1;
-  bf16* kt = sm;                          // [KT][L][NP]
-  bf16* vs = kt + KT * (size_t)L * NP;    // [VT][L][VPITCH]
+  bf16* kt = sm;                       // [3][L][NP]
+  bf16* vs = kt + 3 * (size_t)L * NP;  // [L][VPITCH]
   const int h = blockIdx.y % H, chunk = blockIdx.y / H, seq = blockIdx.z;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   grid_launch_dependents();
@@ -173,24 +136,8 @@ __global__ void __launch_bounds__(THREADS) chunk_sum_kernel(ChunkArgs a) {
     }
     __syncthreads();
   }
-  if (KIND == STATE_SPACE) {
-    load_steps(a, fs, is_, row0, h, nt);
-    for (int i = threadIdx.x; i < L * (N / 8); i += THREADS) {
-      const int s = i / (N / 8), n = (i % (N / 8)) * 8;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (s < nt) v = *reinterpret_cast<const uint4*>(a.k + (row0 + s) * a.k_stride + k_col + n);
-      *reinterpret_cast<uint4*>(kt + s * NP + n) = v;
-    }
-    __syncthreads();
-    if (warp == 0) {
-      chunk_sums_64(Fd, fs, lane);
-      __syncwarp();
-      for (int s = lane; s < L; s += 32) ws[s] = expf((float)(Fd[L - 1] - Fd[s])) * is_[s];
-    }
-    __syncthreads();
-  }
-  const float* cum_last = SCALAR ? nullptr : a.cum + (row0 + nt - 1) * H * N + (size_t)h * N;
-  for (int i = threadIdx.x; KIND != STATE_SPACE && i < L * (N / 8); i += THREADS) {
+  const float* cum_last = GATED ? nullptr : a.cum + (row0 + nt - 1) * H * N + (size_t)h * N;
+  for (int i = threadIdx.x; i < L * (N / 8); i += THREADS) {
     const int s = i / (N / 8), n = (i % (N / 8)) * 8;
     float f[8];
     if (s < nt) {
@@ -214,7 +161,7 @@ __global__ void __launch_bounds__(THREADS) chunk_sum_kernel(ChunkArgs a) {
   float* cs = a.cs + at * ((size_t)N * P + (GATED ? N : 0));
   if (blockIdx.x == 0) {
     for (int n = threadIdx.x; n < N; n += THREADS) {
-      a.cd[at * N + n] = GATED ? expf(Fs[L - 1] + m_before - m_last) : SCALAR ? expf((float)Fd[L - 1]) : expf(cum_last[n]);
+      a.cd[at * N + n] = GATED ? expf(Fs[L - 1] + m_before - m_last) : expf(cum_last[n]);
       if (GATED) {
         float d = 0.f;
         for (int s = 0; s < nt; ++s) {
@@ -228,22 +175,7 @@ __global__ void __launch_bounds__(THREADS) chunk_sum_kernel(ChunkArgs a) {
   for (int slice = blockIdx.x * a.slices; slice < (int)(blockIdx.x + 1) * a.slices && slice * PB < P; ++slice) {
   const int p0 = slice * PB;
   __syncthreads();  // the values of the slice before are no longer read
-  if (KIND == STATE_SPACE) {
-    for (int i = threadIdx.x; i < L * (PB / 8); i += THREADS) {
-      const int s = i / (PB / 8), c = (i % (PB / 8)) * 8;
-      float f[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] = 0.f;
-      if (s < nt && p0 + c < P) {
-        widen8(a.v + (row0 + s) * a.v_stride + (size_t)h * P + p0 + c, f);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) f[j] *= ws[s];
-      }
-      split3_store8(f, vs + s * VPITCH + c, (size_t)L * VPITCH);
-    }
-  } else {
-    load_values(vs, a, row0, h, p0, nt);
-  }
+  load_values(vs, a, row0, h, p0, nt);
   __syncthreads();
   for (int m0 = warp * 16; m0 < N; m0 += 16 * (THREADS / 32)) {
     float acc[8][4];
@@ -253,23 +185,19 @@ __global__ void __launch_bounds__(THREADS) chunk_sum_kernel(ChunkArgs a) {
       for (int c = 0; c < 4; ++c) acc[n][c] = 0.f;
 #pragma unroll
     for (int ks = 0; ks < L / 16; ++ks) {
-      uint32_t af[KT][4];
+      uint32_t af[3][4];
 #pragma unroll
-      for (int t = 0; t < KT; ++t)  // the transpose of k's rows
+      for (int t = 0; t < 3; ++t)  // the transpose of k's rows
         ldmatrix_x4_trans(af[t][0], af[t][1], af[t][2], af[t][3],
                           kt + t * (size_t)L * NP + (ks * 16 + (lane & 7) + ((lane >> 4) & 1) * 8) * NP + m0 + ((lane >> 3) & 1) * 8);
 #pragma unroll
       for (int n = 0; n < 8; n += 2) {
-        uint32_t b[VT][4];
-#pragma unroll
-        for (int t = 0; t < VT; ++t)
-          ldmatrix_x4_trans(b[t][0], b[t][1], b[t][2], b[t][3],
-                            vs + t * (size_t)L * VPITCH + (ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * VPITCH + (n + (lane >> 4)) * 8);
+        uint32_t b0, b1, b2, b3;
+        ldmatrix_x4_trans(b0, b1, b2, b3, vs + (ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * VPITCH + (n + (lane >> 4)) * 8);
 #pragma unroll
         for (int t = 2; t >= 0; --t) {  // small terms first
-          const int ta = KT == 3 ? t : 0, tb = VT == 3 ? t : 0;
-          mma_bf16_16816(acc[n], af[ta][0], af[ta][1], af[ta][2], af[ta][3], b[tb][0], b[tb][1]);
-          mma_bf16_16816(acc[n + 1], af[ta][0], af[ta][1], af[ta][2], af[ta][3], b[tb][2], b[tb][3]);
+          mma_bf16_16816(acc[n], af[t][0], af[t][1], af[t][2], af[t][3], b0, b1);
+          mma_bf16_16816(acc[n + 1], af[t][0], af[t][1], af[t][2], af[t][3], b2, b3);
         }
       }
     }
@@ -579,118 +507,257 @@ __global__ void __launch_bounds__(THREADS) chunk_output_kernel(ChunkArgs a) {
   }
 }
 
-// State-space kind. A block's time is its chain of loads and barriers rather than its products, so three blocks share an SM
-// (80 registers a thread): the state never passes through shared memory. A warp takes all 64 tokens of eight value columns, whose
-// part of the state is then its own fragment of the product, loaded (from the first instruction on) and split in registers.
-// 2,048 tokens of 48 heads: 66 us; with the state's three terms in shared memory and two blocks an SM 87.
-__global__ void __launch_bounds__(THREADS, 3) ssd_output_kernel(ChunkArgs a) {
+// ---- state-space kind ----------------------------------------------------------------------------------------
+// A group's heads share the rows of q and k, so a block takes several (head, column slice) units of a group's chunk: what depends on
+// q and k alone is done once, and a unit's values, step sizes and state are on their way while the unit before is multiplied. Two blocks
+// an SM: three leave the outputs 80 registers, which spill (69 us against 58, profiled; a block a head 66).
+
+// What a unit needs of the chunk's tokens: the raw values of a thread's two pieces of eight, the steps of token threadIdx.x
+struct UnitRows {
+  uint4 v[2];
+  float4 step;
+  __device__ __forceinline__ void fetch(const ChunkArgs& a, size_t row0, int h, int p0, int nt) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int s = (threadIdx.x >> 3) + 32 * i, c = (threadIdx.x & 7) * 8;
+      v[i] = s < nt && p0 + c < a.P ? *reinterpret_cast<const uint4*>(a.v + (row0 + s) * a.v_stride + (size_t)h * a.P + p0 + c)
+                                    : make_uint4(0u, 0u, 0u, 0u);
+    }
+    step = threadIdx.x < nt ? a.steps[(size_t)h * a.rows + row0 + threadIdx.x] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+};
+static_assert(L * PB / 8 == 2 * THREADS && PB == 64, "two pieces a thread");
+
+// The chunk's own sum_s k_s (w_s v_s)^T: where a token's weight is one number it multiplies the values instead of the keys: they are
+// fewer, and the keys stay exact. Warps 4 x 2: 32 key rows and 32 columns each, so that a fragment of the values' terms, which
+// bound the kernel (every warp reads them from shared memory), serves two products; the keys' fragments stay in registers.
+__global__ void __launch_bounds__(THREADS, 2) ssd_sum_kernel(ChunkArgs a) {
   extern __shared__ __align__(16) bf16 sm[];
-  __shared__ float fs[L], dts[L];
-  __shared__ double Fd[L];
-  __shared__ int bad[PB];
+  __shared__ float ws[2][L];
   const int N = a.N, P = a.P, H = a.H, NP = N + 8;
-  bf16* qs = sm;                   // [L][NP]
-  bf16* vs = qs + (size_t)L * NP;  // [L][VPITCH]
-  bf16* ks = vs + L * VPITCH;      // [L][NP]; then
-  bf16* as = ks;                   // [3][L][APITCH]: A
-  const int h = blockIdx.y % H, chunk = blockIdx.y / H, seq = blockIdx.z;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int g = lane >> 2, t4 = lane & 3;
+  bf16* ks = sm;                       // [L][NP]
+  bf16* vs = ks + (size_t)L * NP;      // [3][L][VPITCH]
+  const int part = blockIdx.x % a.parts, group = blockIdx.x / a.parts, chunk = blockIdx.y, seq = blockIdx.z;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
   grid_launch_dependents();
   grid_dependency_wait();
   const int first = (a.chunk0 + chunk) * L, nt = min(L, a.seq_qlen[seq] - first);
   if (nt <= 0) return;
   const size_t row0 = (size_t)a.cu_q[seq] + first;
-  const size_t group = (size_t)(h / a.per_group) * N;
-  const float* start = a.cs + (((size_t)seq * a.max_chunks + chunk) * H + h) * (size_t)N * P;
+  const int slices = (P + PB - 1) / PB, all = a.per_group * slices, u1 = min(all, (part + 1) * a.units);
+  int u = part * a.units;
+  UnitRows next;
+  next.fetch(a, row0, group * a.per_group + u / slices, u % slices * PB, nt);
+  for (int s = warp; s < L; s += THREADS / 32)
+    for (int n = lane * 8; n < N; n += 256) {
+      bf16* dst = ks + s * NP + n;
+      if (s < nt) cp_async_16(dst, a.k + (row0 + s) * a.k_stride + (size_t)group * N + n);
+      else *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
+    }
+  cp_async_commit();
+  cp_async_wait<0>();
+  const int c0 = (warp >> 2) * 32;
+  for (; u < u1; ++u) {
+    const int h = group * a.per_group + u / slices, p0 = u % slices * PB, b = u & 1;
+    const UnitRows now = next;
+    if (threadIdx.x < L) ws[b][threadIdx.x] = now.step.w;
+    __syncthreads();  // the weights are here, and the values of the unit before are no longer read
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int s = (threadIdx.x >> 3) + 32 * i, c = (threadIdx.x & 7) * 8;
+      const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&now.v[i]);
+      const float w = ws[b][s];
+      float f[8];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) { f[2 * j] = w * __low2float(h2[j]); f[2 * j + 1] = w * __high2float(h2[j]); }
+      split3_store8(f, vs + s * VPITCH + c, (size_t)L * VPITCH);
+    }
+    if (u + 1 < u1) next.fetch(a, row0, group * a.per_group + (u + 1) / slices, (u + 1) % slices * PB, nt);
+    __syncthreads();
+    const size_t at = ((size_t)seq * a.max_chunks + chunk) * H + h;
+    float* cs = a.cs + at * ((size_t)N * P);
+    if (p0 == 0) {
+      const float4 last = a.steps[(size_t)h * a.rows + row0 + nt - 1];
+      const float decay = expf(last.x + last.y);
+      for (int n = threadIdx.x; n < N; n += THREADS) a.cd[at * N + n] = decay;
+    }
+    for (int m0 = (warp & 3) * 32; m0 < N; m0 += 128) {
+      float acc[2][4][4];
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc[m][n][c] = 0.f;
+#pragma unroll
+      for (int kk = 0; kk < L / 16; ++kk) {
+        uint32_t af[2][4];
+#pragma unroll
+        for (int m = 0; m < 2; ++m)  // the transpose of k's rows (the last 16 columns again where N ends there)
+          ldmatrix_x4_trans(af[m][0], af[m][1], af[m][2], af[m][3],
+                            ks + (kk * 16 + (lane & 7) + ((lane >> 4) & 1) * 8) * NP + min(m0 + 16 * m, N - 16) + ((lane >> 3) & 1) * 8);
+#pragma unroll
+        for (int n = 0; n < 4; n += 2) {
+          uint32_t bf[3][4];
+#pragma unroll
+          for (int t = 0; t < 3; ++t)
+            ldmatrix_x4_trans(bf[t][0], bf[t][1], bf[t][2], bf[t][3],
+                              vs + ((size_t)t * L + kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * VPITCH + c0 + (n + (lane >> 4)) * 8);
+#pragma unroll
+          for (int t = 2; t >= 0; --t)  // small terms first
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+              mma_bf16_16816(acc[m][n], af[m][0], af[m][1], af[m][2], af[m][3], bf[t][0], bf[t][1]);
+              mma_bf16_16816(acc[m][n + 1], af[m][0], af[m][1], af[m][2], af[m][3], bf[t][2], bf[t][3]);
+            }
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        if (m0 + 16 * m >= N) break;
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+          const int p = p0 + c0 + n * 8 + 2 * t4;
+          if (p < P) {
+            float* dst = cs + (size_t)(m0 + 16 * m + g) * P + p;
+            *reinterpret_cast<float2*>(dst) = make_float2(acc[m][n][0], acc[m][n][1]);
+            *reinterpret_cast<float2*>(dst + 8 * (size_t)P) = make_float2(acc[m][n][2], acc[m][n][3]);
+          }
+        }
+      }
+    }
+  }
+}
+
+// The outputs. A warp takes all 64 tokens of eight value columns, whose part of the state is then its own fragment of the product:
+// it never passes through shared memory. C_t . B_s of the chunk, the same for a group's heads, waits in shared memory, each thread's
+// own share side by side.
+__global__ void __launch_bounds__(THREADS, 2) ssd_output_kernel(ChunkArgs a) {
+  extern __shared__ __align__(16) bf16 sm[];
+  __shared__ float2 fs[L];     // the summed decays
+  __shared__ float dts[L];
+  __shared__ int bad[2][PB];   // the first token that holds something infinite in a value column
+  const int N = a.N, P = a.P, H = a.H, NP = N + 8;
+  bf16* qs = sm;                       // [L][NP]
+  bf16* vs = qs + (size_t)L * NP;      // [L][VPITCH]
+  float* dots = reinterpret_cast<float*>(vs + L * VPITCH);  // [16][THREADS] C_t . B_s
+  bf16* ks = reinterpret_cast<bf16*>(dots + 16 * THREADS);  // [L][NP]; then
+  bf16* as = ks;                       // [3][L][APITCH]: A
+  const int part = blockIdx.x % a.parts, group = blockIdx.x / a.parts, chunk = blockIdx.y, seq = blockIdx.z;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int first = (a.chunk0 + chunk) * L, nt = min(L, a.seq_qlen[seq] - first);
+  if (nt <= 0) return;
+  const size_t row0 = (size_t)a.cu_q[seq] + first;
+  const int slices = (P + PB - 1) / PB, all = a.per_group * slices, u1 = min(all, (part + 1) * a.units);
+  int u = part * a.units;
+  const float* starts = a.cs + ((size_t)seq * a.max_chunks + chunk) * H * N * P;
   constexpr int KB = 8;  // 128 rows of the state at a time
   float own[KB][4];
-  auto fetch = [&](int p, int n0) {  // rows n0 .. n0 + 127 of column p, as the product's fragments have them
+  auto fetch = [&](int u, int n0) {  // rows n0 .. n0 + 127 of a column of the unit's state, as the product's fragments have them
+    const int p = u % slices * PB + warp * 8 + g;
+    const float* from = starts + ((size_t)(group * a.per_group + u / slices) * N + n0 + 2 * t4) * P + p;
 #pragma unroll
-    for (int kk = 0; kk < KB; ++kk)
+    for (int kk = 0; kk < KB; ++kk) {
+      const bool in = p < P && n0 + kk * 16 < N;  // N is a multiple of 16
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int n = n0 + kk * 16 + 2 * t4 + (i & 1) + 8 * (i >> 1);
-        own[kk][i] = n < N && p < P ? __ldcg(start + (size_t)n * P + p) : 0.f;
-      }
+      for (int i = 0; i < 4; ++i) own[kk][i] = in ? __ldcg(from + (size_t)(kk * 16 + (i & 1) + 8 * (i >> 1)) * P) : 0.f;
+    }
   };
-  int slice = blockIdx.x * a.slices;
-  fetch(slice * PB + warp * 8 + g, 0);
-  load_steps(a, fs, dts, row0, h, nt);
-  for (int i = threadIdx.x; i < 2 * L * (N / 8); i += THREADS) {
-    const int s = (i / (N / 8)) % L, n = (i % (N / 8)) * 8;
-    const bool is_k = i >= L * (N / 8);
-    bf16* dst = (is_k ? ks : qs) + s * NP + n;
-    if (s < nt) cp_async_16(dst, (is_k ? a.k + (row0 + s) * a.k_stride : a.q + (row0 + s) * a.q_stride) + group + n);
-    else *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
+  UnitRows next;
+  next.fetch(a, row0, group * a.per_group + u / slices, u % slices * PB, nt);
+  for (int s = warp; s < 2 * L; s += THREADS / 32) {
+    const bool is_k = s >= L;
+    const int r = s & (L - 1);
+    for (int n = lane * 8; n < N; n += 256) {
+      bf16* dst = (is_k ? ks : qs) + r * NP + n;
+      if (r < nt) cp_async_16(dst, (is_k ? a.k + (row0 + r) * a.k_stride : a.q + (row0 + r) * a.q_stride) + (size_t)group * N + n);
+      else *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
+    }
   }
   cp_async_commit();
-  load_values(vs, a, row0, h, slice * PB, nt);
-  if (threadIdx.x < PB) bad[threadIdx.x] = L;
+  fetch(u, 0);
+  if (threadIdx.x < 2 * PB) bad[threadIdx.x >> 6][threadIdx.x & 63] = L;
   cp_async_wait<0>();
   __syncthreads();
-  if (warp == 0) chunk_sums_64(Fd, fs, lane);
-  {  // A: the warp's 16 tokens against 32 of the chunk's
-    const int mt = warp & 3, u0 = (warp >> 2) * 32;
+  // A: the warp's 16 tokens against 32 of the chunk's; two warps have later tokens alone, whose tiles are not read
+  const int mt = warp & 3, t0 = (warp >> 2) * 32;
+  if (t0 < mt * 16 + 16) {
     float s[4][4];
 #pragma unroll
     for (int n = 0; n < 4; ++n)
 #pragma unroll
       for (int c = 0; c < 4; ++c) s[n][c] = 0.f;
-    for (int kk = 0; kk < N / 16; ++kk) {
-      if (u0 >= mt * 16 + 16) break;
+    for (int kk = 0; kk < N; kk += 16) {
       uint32_t af[4];
-      ldmatrix_x4(af[0], af[1], af[2], af[3], qs + (mt * 16 + (lane & 15)) * NP + kk * 16 + (lane >> 4) * 8);
+      ldmatrix_x4(af[0], af[1], af[2], af[3], qs + (mt * 16 + (lane & 15)) * NP + kk + (lane >> 4) * 8);
 #pragma unroll
       for (int n = 0; n < 4; n += 2) {
-        if (u0 + n * 8 >= mt * 16 + 16) break;  // later tokens
         uint32_t b[4];
-        ldmatrix_x4(b[0], b[1], b[2], b[3], ks + (u0 + n * 8 + ((lane >> 4) << 3) + (lane & 7)) * NP + kk * 16 + ((lane >> 3) & 1) * 8);
+        ldmatrix_x4(b[0], b[1], b[2], b[3], ks + (t0 + n * 8 + ((lane >> 4) << 3) + (lane & 7)) * NP + kk + ((lane >> 3) & 1) * 8);
         mma_bf16_16816(s[n], af[0], af[1], af[2], af[3], b[0], b[1]);
         mma_bf16_16816(s[n + 1], af[0], af[1], af[2], af[3], b[2], b[3]);
       }
     }
-    __syncthreads();  // the keys are no longer read; the decays' sums are here
-    set_aside_infinities(vs, bad);
 #pragma unroll
-    for (int hh = 0; hh < 2; ++hh) {
-      const int t = mt * 16 + g + 8 * hh;
+    for (int n = 0; n < 4; ++n)
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        float v[2];
+      for (int c = 0; c < 4; ++c) dots[(n * 4 + c) * THREADS + threadIdx.x] = s[n][c];
+  }
+  for (int h_before = -1; u < u1; ++u) {
+    const int h = group * a.per_group + u / slices;
+    int* worst = bad[u & 1];
+    // the values, what is not finite set aside (a zero in its place): a matrix product would hand it, times zero, to the tokens before
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int u = u0 + n * 8 + 2 * t4 + c;
-          v[c] = u <= t && t < nt ? s[n][2 * hh + c] * (expf((float)(Fd[t] - Fd[u])) * dts[u]) : 0.f;
+    for (int i = 0; i < 2; ++i) {
+      const int s = (threadIdx.x >> 3) + 32 * i, c = (threadIdx.x & 7) * 8;
+      uint32_t* two = reinterpret_cast<uint32_t*>(&next.v[i]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const bool lo = (two[j] & 0x7f80u) == 0x7f80u, hi = (two[j] & 0x7f800000u) == 0x7f800000u;
+        if (lo) atomicMin(worst + c + 2 * j, s);
+        if (hi) atomicMin(worst + c + 2 * j + 1, s);
+        if (lo || hi) two[j] &= (lo ? 0xffff0000u : 0xffffffffu) & (hi ? 0xffffu : 0xffffffffu);
+      }
+      *reinterpret_cast<uint4*>(vs + s * VPITCH + c) = next.v[i];
+    }
+    if (threadIdx.x < L) {
+      fs[threadIdx.x] = make_float2(next.step.x, next.step.y);
+      dts[threadIdx.x] = next.step.z;
+    }
+    __syncthreads();  // values and steps are here, and the keys (later A) are no longer read
+    if (h != h_before && t0 < mt * 16 + 16) {
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh) {
+        const int t = mt * 16 + g + 8 * hh;
+        const float2 ft = fs[t];
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+          float v[2];
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const int s = t0 + n * 8 + 2 * t4 + c;
+            const float2 f = fs[s];
+            // the difference of the two-float sums: its largest part is exact or rounded once
+            v[c] = s <= t && t < nt ? dots[(n * 4 + 2 * hh + c) * THREADS + threadIdx.x] * (expf((ft.x - f.x) + (ft.y - f.y)) * dts[s]) : 0.f;
+          }
+          uint32_t p[3];
+          split3_pair(v[0], v[1], p);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(as + (i * L + t) * APITCH + t0 + n * 8 + 2 * t4) = p[i];
         }
-        uint32_t p[3];
-        split3_pair(v[0], v[1], p);
-#pragma unroll
-        for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(as + (i * L + t) * APITCH + u0 + n * 8 + 2 * t4) = p[i];
       }
     }
-  }
-  __syncthreads();
-  const float skip = a.skip[h];
-  for (const int end = slice + a.slices; slice < end && slice * PB < P; ++slice) {
-    const int p0 = slice * PB + warp * 8;
-    if (slice != (int)blockIdx.x * a.slices) {
-      fetch(p0 + g, 0);
-      __syncthreads();  // the values of the slice before are no longer read
-      if (threadIdx.x < PB) bad[threadIdx.x] = L;
-      load_values(vs, a, row0, h, slice * PB, nt);
-      __syncthreads();
-      set_aside_infinities(vs, bad);
-      __syncthreads();
-    }
-    if (p0 >= P) continue;  // the whole warp: P is a multiple of 16
+    h_before = h;
+    const int p0 = u % slices * PB + warp * 8;
     float acc[4][4];
 #pragma unroll
     for (int m = 0; m < 4; ++m)
 #pragma unroll
       for (int c = 0; c < 4; ++c) acc[m][c] = 0.f;
     for (int n0 = 0; n0 < N; n0 += 16 * KB) {
-      if (n0) fetch(p0 + g, n0);
+      if (n0) fetch(u, n0);
 #pragma unroll
       for (int kk = 0; kk < KB; ++kk) {
         if (n0 + kk * 16 >= N) break;
@@ -706,10 +773,20 @@ __global__ void __launch_bounds__(THREADS, 3) ssd_output_kernel(ChunkArgs a) {
         }
       }
     }
+    if (u + 1 < u1) {
+      next.fetch(a, row0, group * a.per_group + (u + 1) / slices, (u + 1) % slices * PB, nt);
+      fetch(u + 1, 0);
+    }
 #pragma unroll
     for (int m = 0; m < 4; ++m)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) acc[m][c] *= expf((float)Fd[m * 16 + g + 8 * (c >> 1)]);
+      for (int hh = 0; hh < 2; ++hh) {
+        const float2 f = fs[m * 16 + g + 8 * hh];
+        const float e = expf(f.x + f.y);
+        acc[m][2 * hh] *= e;
+        acc[m][2 * hh + 1] *= e;
+      }
+    __syncthreads();  // A is here
 #pragma unroll
     for (int kk = 0; kk < 4; kk += 2) {
       uint32_t b[4];  // of 16 tokens, and of the 16 after them
@@ -728,17 +805,22 @@ __global__ void __launch_bounds__(THREADS, 3) ssd_output_kernel(ChunkArgs a) {
         }
     }
     const int c0 = warp * 8 + 2 * t4;
+    const float skip = a.skip[h];
+    if (p0 < P) {  // the whole warp: P is a multiple of 16
 #pragma unroll
-    for (int m = 0; m < 4; ++m)
+      for (int m = 0; m < 4; ++m)
 #pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {
-        const int t = m * 16 + g + 8 * hh;
-        if (t >= nt) continue;
-        const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(vs + t * VPITCH + c0);
-        const float y0 = fmaf(skip, __low2float(x), acc[m][2 * hh]), y1 = fmaf(skip, __high2float(x), acc[m][2 * hh + 1]);
-        *reinterpret_cast<float2*>(a.y + ((row0 + t) * H + h) * P + p0 + 2 * t4) =
-            make_float2(t >= bad[c0] ? NAN : y0, t >= bad[c0 + 1] ? NAN : y1);
-      }
+        for (int hh = 0; hh < 2; ++hh) {
+          const int t = m * 16 + g + 8 * hh;
+          if (t >= nt) continue;
+          const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(vs + t * VPITCH + c0);
+          const float y0 = fmaf(skip, __low2float(x), acc[m][2 * hh]), y1 = fmaf(skip, __high2float(x), acc[m][2 * hh + 1]);
+          *reinterpret_cast<float2*>(a.y + ((row0 + t) * H + h) * P + p0 + 2 * t4) =
+              make_float2(t >= worst[c0] ? NAN : y0, t >= worst[c0 + 1] ? NAN : y1);
+        }
+    }
+    __syncthreads();  // the values, A and the steps make room for the next unit's
+    if (threadIdx.x < PB) worst[threadIdx.x] = L;
   }
 }
 
@@ -779,23 +861,51 @@ __global__ void chunk_decays_kernel(float* __restrict__ cum, const bf16* __restr
 }
 
 // state-space kind: dt = softplus(raw + bias), log decay -exp(A_log) dt. Not below FORGOTTEN, whose e^ is zero in 32 bits: sums of
-// minus infinity have no difference, and even 64 bits would lose a later token's decay beside a number that is large enough.
+// minus infinity have no difference, and even 64 bits would lose a later token's decay beside a number that is large enough. The
+// decays are summed over a chunk's tokens in 64 bits and left as two floats, whose differences are as exact. A warp a chunk and head,
+// a lane two neighbouring tokens.
 constexpr float FORGOTTEN = -120.f;
-__global__ void steps_kernel(float2* __restrict__ steps, const bf16* __restrict__ dt, int dt_stride, const float* __restrict__ bias,
-                             const float* __restrict__ a_log, int rows, int H) {
+__global__ void __launch_bounds__(256) steps_kernel(float4* __restrict__ steps, const bf16* __restrict__ dt, int dt_stride,
+                                                    const float* __restrict__ bias, const float* __restrict__ a_log, int rows, int H,
+                                                    const int* __restrict__ cu_q, const int* __restrict__ seq_qlen) {
   grid_launch_dependents();
   grid_dependency_wait();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows * H) return;
-  const int r = i / H, h = i % H;
-  const float z = __bfloat162float(dt[(size_t)r * dt_stride + h]) + bias[h];
-  const float d = z > 20.f ? z : log1pf(expf(z));
-  const float f = -expf(a_log[h]) * d;
-  steps[i] = make_float2(f < FORGOTTEN ? FORGOTTEN : f, d);  // a NaN stays one
+  const int lane = threadIdx.x & 31, h = blockIdx.x * 8 + (threadIdx.x >> 5), seq = blockIdx.z;
+  const int first = blockIdx.y * L, nt = min(L, seq_qlen[seq] - first);
+  if (nt <= 0 || h >= H) return;
+  const size_t row0 = (size_t)cu_q[seq] + first;
+  const float b = bias[h], rate = expf(a_log[h]);
+  float d[2], f[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int t = 2 * lane + j;
+    d[j] = f[j] = 0.f;
+    if (t < nt) {
+      const float z = __bfloat162float(dt[(row0 + t) * dt_stride + h]) + b;
+      d[j] = z > 20.f ? z : log1pf(expf(z));
+      f[j] = -rate * d[j];
+      if (f[j] < FORGOTTEN) f[j] = FORGOTTEN;  // a NaN stays one
+    }
+  }
+  const double two = (double)f[0] + f[1];
+  double run = two;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double p = __shfl_up_sync(0xffffffffu, run, o);
+    if (lane >= o) run += p;
+  }
+  const double sums[2] = {(run - two) + f[0], run}, last = __shfl_sync(0xffffffffu, run, 31);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int t = 2 * lane + j;
+    if (t >= nt) continue;
+    const float hi = (float)sums[j];
+    steps[(size_t)h * rows + row0 + t] = make_float4(hi, (float)(sums[j] - hi), d[j], expf((float)(last - sums[j])) * d[j]);
+  }
 }
 
 size_t sum_smem(int N) { return (3 * (size_t)L * (N + 8) + (size_t)L * VPITCH) * sizeof(bf16); }
-size_t sum_smem_scalar(int N) { return ((size_t)L * (N + 8) + 3 * (size_t)L * VPITCH) * sizeof(bf16); }
+size_t ssd_sum_smem(int N) { return ((size_t)L * (N + 8) + 3 * (size_t)L * VPITCH) * sizeof(bf16); }
 size_t output_smem(int N, bool gated) {
   const size_t terms = gated ? 1 : 3, rows = terms * L * (N + 8), state = 3 * (size_t)N * VPITCH;
   return (rows + 3 * (size_t)L * APITCH + (size_t)L * VPITCH + (state > rows ? state : rows)) * sizeof(bf16);
@@ -803,13 +913,19 @@ size_t output_smem(int N, bool gated) {
 
 size_t ssd_output_smem(int N) {
   const size_t keys = (size_t)L * (N + 8), sums = 3 * (size_t)L * APITCH;
-  return ((size_t)L * (N + 8) + (size_t)L * VPITCH + (keys > sums ? keys : sums)) * sizeof(bf16);
+  return ((size_t)L * (N + 8) + (size_t)L * VPITCH + (keys > sums ? keys : sums)) * sizeof(bf16) + 16 * THREADS * sizeof(float);
+}
+
+int launch_walk(const ChunkArgs& a, bool gated, int n_seqs, cudaStream_t stream) {
+  const size_t all = (size_t)a.N * a.P + (gated ? a.N : 0);
+  return (int)launch_pdl(gated ? chunk_walk_kernel<true> : chunk_walk_kernel<false>, dim3((unsigned)((all / 4 + 63) / 64), (unsigned)a.H, (unsigned)n_seqs),
+                         dim3(64), 0, stream, a);
 }
 
 template <Kind KIND>
 int launch_chunks(ChunkArgs a, int n_seqs, cudaStream_t stream) {
   constexpr bool GATED = KIND == RUNNING_MAX;
-  const size_t s1 = KIND == STATE_SPACE ? sum_smem_scalar(a.N) : sum_smem(a.N), s3 = KIND == STATE_SPACE ? ssd_output_smem(a.N) : output_smem(a.N, GATED);
+  const size_t s1 = sum_smem(a.N), s3 = output_smem(a.N, GATED);
   const long long heads = (long long)a.H * a.max_chunks;
   if (heads > 65535 || n_seqs > 65535) return -2;
   // what a block does before its first slice is done once per block: as many slices a block as leave every SM three
@@ -818,18 +934,39 @@ int launch_chunks(ChunkArgs a, int n_seqs, cudaStream_t stream) {
   a.slices = (int)(most / 444 < 1 ? 1 : most / 444 > all_slices ? all_slices : most / 444);
   const dim3 grid((unsigned)((all_slices + a.slices - 1) / a.slices), (unsigned)heads, (unsigned)n_seqs);
   cudaFuncSetAttribute(chunk_sum_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1);
-  auto output = [] {
-    if constexpr (KIND == STATE_SPACE) return ssd_output_kernel;
-    else return chunk_output_kernel<KIND>;
-  }();
-  cudaFuncSetAttribute(output, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3);
+  cudaFuncSetAttribute(chunk_output_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3);
   int rc = (int)launch_pdl(chunk_sum_kernel<KIND>, grid, dim3(THREADS), s1, stream, a);
   if (rc) return rc;
-  const size_t all = (size_t)a.N * a.P + (GATED ? a.N : 0);
-  rc = (int)launch_pdl(chunk_walk_kernel<GATED>, dim3((unsigned)((all / 4 + 63) / 64), (unsigned)a.H, (unsigned)n_seqs), dim3(64),
-                       0, stream, a);
+  if ((rc = launch_walk(a, GATED, n_seqs, stream))) return rc;
+  return (int)launch_pdl(chunk_output_kernel<KIND>, grid, dim3(THREADS), s3, stream, a);
+}
+
+int launch_ssd(ChunkArgs a, int n_seqs, cudaStream_t stream) {
+  const size_t s1 = ssd_sum_smem(a.N), s3 = ssd_output_smem(a.N);
+  if (a.max_chunks > 65535 || n_seqs > 65535) return -2;
+  cudaFuncSetAttribute(ssd_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1);
+  cudaFuncSetAttribute(ssd_output_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3);
+  const int groups = a.H / a.per_group, all = a.per_group * ((a.P + PB - 1) / PB);
+  // units a block: the fewest rounds of units over the SMs, a block's start counted as a part of one
+  auto split = [&](int an_sm, float start) {
+    float best = 1e30f;
+    for (int units = 1; units <= all; ++units) {
+      const long long blocks = (long long)((all + units - 1) / units) * groups * a.max_chunks * n_seqs;
+      const float cost = (float)((blocks + 148 * an_sm - 1) / (148 * an_sm)) * (units + start);
+      if (cost < best) {
+        best = cost;
+        a.units = units;
+      }
+    }
+    a.parts = (all + a.units - 1) / a.units;
+    return dim3((unsigned)(a.parts * groups), (unsigned)a.max_chunks, (unsigned)n_seqs);
+  };
+  dim3 grid = split(2, 0.5f);
+  int rc = (int)launch_pdl(ssd_sum_kernel, grid, dim3(THREADS), s1, stream, a);
   if (rc) return rc;
-  return (int)launch_pdl(output, grid, dim3(THREADS), s3, stream, a);
+  if ((rc = launch_walk(a, false, n_seqs, stream))) return rc;
+  grid = split(2, 0.7f);
+  return (int)launch_pdl(ssd_output_kernel, grid, dim3(THREADS), s3, stream, a);
 }
 
 }  // namespace
@@ -866,35 +1003,36 @@ KRK_API int krk_memory_chunks(float* y, float* den, const void* q, int q_stride,
   a.v_stride = v_stride; a.q_scale = q_scale; a.cum = cum; a.gates = (const float4*)gates; a.state = state; a.nm = nm; a.y = y; a.den = den;
   a.cs = cs; a.cd = cd; a.H = H; a.N = N; a.P = P; a.max_chunks = (max_q_len + L - 1) / L; a.slices = 1;
   a.cu_q = cu_q; a.seq_qlen = seq_qlen; a.seq_slot = seq_slot;
-  a.steps = nullptr; a.skip = nullptr; a.per_group = 1; a.chunk0 = 0;
+  a.steps = nullptr; a.rows = 0; a.skip = nullptr; a.per_group = 1; a.units = a.parts = 1; a.chunk0 = 0;
   return gates ? launch_chunks<RUNNING_MAX>(a, n_seqs, stream) : launch_chunks<DECAYS>(a, n_seqs, stream);
 }
 
-// Step sizes and log decays [rows, H] of a state-space mixer's rows (bfloat16), for krk_ssd_chunks.
+// Step sizes and summed log decays [H, rows] of a state-space mixer's rows (bfloat16), four floats each, for krk_ssd_chunks.
 KRK_API int krk_ssd_steps(float* steps, const void* dt, int dt_stride, const float* dt_bias, const float* a_log, int rows, int H,
-                          cudaStream_t stream) {
-  if (rows == 0) return 0;
-  if ((long long)rows * H > 0x7fffff00LL) return -2;
-  return (int)launch_pdl(steps_kernel, dim3((unsigned)((rows * H + 255) / 256)), dim3(256), 0, stream, (float2*)steps, (const bf16*)dt,
-                         dt_stride, dt_bias, a_log, rows, H);
+                          int n_seqs, int max_q_len, const int* cu_q, const int* seq_qlen, cudaStream_t stream) {
+  if (rows == 0 || n_seqs == 0 || max_q_len == 0) return 0;
+  const int chunks = (max_q_len + L - 1) / L;
+  if (chunks > 65535 || n_seqs > 65535 || ((uintptr_t)steps & 15)) return -2;
+  return (int)launch_pdl(steps_kernel, dim3((unsigned)((H + 7) / 8), (unsigned)chunks, (unsigned)n_seqs), dim3(256), 0, stream, (float4*)steps,
+                         (const bf16*)dt, dt_stride, dt_bias, a_log, rows, H, cu_q, seq_qlen);
 }
 
 // The scan of a state-space mixer (krk_ssd_scan) over chunks chunk0 .. chunk0 + n_chunks - 1 of every sequence, from and to the
 // stored state [slots, H, N, P]; the caller goes through a step's chunks in order. x, B and C bfloat16 with rows on 16-byte
 // boundaries; scratch cs and cd for n_chunks chunks a sequence.
 KRK_API int krk_ssd_chunks(float* y, const void* x, int x_stride, const void* B, int b_stride, const void* C, int c_stride,
-                           const float* steps, const float* skip, float* state, float* cs, float* cd, int H, int P, int N, int G,
-                           int n_seqs, int chunk0, int n_chunks, const int* cu_q, const int* seq_qlen, const int* seq_slot,
+                           const float* steps, int rows, const float* skip, float* state, float* cs, float* cd, int H, int P,
+                           int N, int G, int n_seqs, int chunk0, int n_chunks, const int* cu_q, const int* seq_qlen, const int* seq_slot,
                            cudaStream_t stream) {
   if (n_seqs == 0 || n_chunks == 0) return 0;
   if (G < 1 || H % G || !krk_memory_chunk_tokens(N, P, 1) || x_stride % 8 || b_stride % 8 || c_stride % 8 ||
-      (((uintptr_t)x | (uintptr_t)B | (uintptr_t)C | (uintptr_t)state | (uintptr_t)cs) & 15) || ((uintptr_t)steps & 7))
+      (((uintptr_t)x | (uintptr_t)B | (uintptr_t)C | (uintptr_t)state | (uintptr_t)cs) & 15) || ((uintptr_t)steps & 15))
     return -2;
   ChunkArgs a;
   a.q = (const bf16*)C; a.k = (const bf16*)B; a.v = (const bf16*)x; a.q_stride = c_stride; a.k_stride = b_stride;
   a.v_stride = x_stride; a.q_scale = 1.f; a.cum = nullptr; a.gates = nullptr; a.state = state; a.nm = nullptr; a.y = y; a.den = nullptr;
   a.cs = cs; a.cd = cd; a.H = H; a.N = N; a.P = P; a.max_chunks = n_chunks; a.slices = 1;
   a.cu_q = cu_q; a.seq_qlen = seq_qlen; a.seq_slot = seq_slot;
-  a.steps = (const float2*)steps; a.skip = skip; a.per_group = H / G; a.chunk0 = chunk0;
-  return launch_chunks<STATE_SPACE>(a, n_seqs, stream);
+  a.steps = (const float4*)steps; a.rows = rows; a.skip = skip; a.per_group = H / G; a.chunk0 = chunk0;
+  return launch_ssd(a, n_seqs, stream);
 }
