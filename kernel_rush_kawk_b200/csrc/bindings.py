@@ -1491,14 +1491,14 @@ class Kernels:
     # -- state-space mixer ------------------------------------------------------------------
     SSD_CHUNK = 128  # tokens per chunk where one sequence's step is long enough to be scanned in chunks
 
-    CONV_WALK_BYTES = 12_000_000
+    CONV_WALK_BYTES = 5_000_000
 
     def _conv_walks(self, rows, row_bytes, n_seqs) -> bool:
-        """Whether threads of the short convolution go through sixteen rows each, the rows before in registers. That is one chain of
-        13 us at least (bfloat16; 9 in 32-bit), at a sequence's first row with the loads of its stored rows in it, and pays by
-        bytes: a block a row and sixteen rows a thread, one prompt of 4,096 channels, 256 rows 6.2 and 13.5 us, 1,024 14.2 and
-        17.0, 1,536 18.6 and 17.6, 2,048 23.0 and 18.1; of 1,792 channels 2,048 rows 13.4 and 17.0, 4,096 21.7 and 18.0; 32-bit of
-        4,096 channels 512 rows 9.4 and 10.3, 768 12.5 and 11.8. Single tokens of 64 sequences 10.3 and 24.6, of 2,048 equal."""
+        """Whether threads of the short convolution go through eight rows each, the rows before in registers. That is one chain of
+        5.3 us at least, at a sequence's first row with the loads of its stored rows in it, and pays by bytes: a block a row and
+        eight rows a thread, one prompt of 4,096 channels in bfloat16, 64 rows 5.0 and 5.6 us, 256 6.2 and 5.9, 512 8.2 and 7.1,
+        2,048 18.7 and 12.9; of 1,792 channels 512 rows 5.9 and 6.4, 1,024 7.9 and 6.9, 2,048 10.8 and 9.1; 32-bit of 4,096 channels
+        256 rows 6.9 and 7.3, 512 9.5 and 7.7. Single tokens of 64 sequences 9.9 and 12.9, of 2,048 equal."""
         return rows * row_bytes >= self.CONV_WALK_BYTES and rows >= 2 * n_seqs
 
     def causal_conv_silu(self, x, w, b, tail, batch):

@@ -30,6 +30,9 @@ constexpr int TOK = 16;       // tokens staged at a time
 constexpr int MAX_TAPS = 16;  // the convolution's taps
 
 __device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
+// where the result is rounded to T: bfloat16 takes the fast exponential and division, a few units in 2^23 off
+template <typename T> __device__ __forceinline__ float silu_to(float z) { return silu_f(z); }
+template <> __device__ __forceinline__ float silu_to<bf16>(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
 // V consecutive elements as floats, in one access of V * sizeof(T) bytes (the address is aligned to that)
@@ -75,15 +78,16 @@ __global__ void causal_conv_silu_kernel(T* __restrict__ out, const T* __restrict
       for (int i = 0; i < V; ++i) acc[i] += wj[i] * v[i];
     }
 #pragma unroll
-    for (int i = 0; i < V; ++i) acc[i] = silu_f(acc[i]);
+    for (int i = 0; i < V; ++i) acc[i] = silu_to<T>(acc[i]);
     store_run<T, V>(out + (size_t)r * ch + c, acc);
   }
 }
 
 // The same for four taps and 16-byte pieces, CONV_ROWS rows a thread. Bound by bytes (a row in, a row out), which the kernel
 // above does not reach: it reads every row four times and the taps' weights, 20 bytes a channel, for every row. Here the
-// weights and the three rows before stay in registers: 2,048 rows of 4,096 channels 26.0 -> 17.9 us (34 MB, and the exponential and division of silu).
-constexpr int CONV_ROWS = 16;
+// weights and the rows before stay in registers, and all of a thread's rows are asked for before the first is used: 2,048 rows of
+// 4,096 channels 18.7 us a row a block, 12.9 here (sixteen rows a thread, four asked for at a time: 18.1; twelve at once 17.8).
+constexpr int CONV_ROWS = 8;
 
 template <typename T>
 __global__ void __launch_bounds__(64)
@@ -102,9 +106,12 @@ causal_conv4_kernel(T* __restrict__ out, const T* __restrict__ in, int in_stride
     for (int j = 0; j < 4; ++j) load_run<float, 4>(w + (size_t)j * ch + c + i, wj[j] + i);
   }
   grid_dependency_wait();
-  const int r0 = blockIdx.y * CONV_ROWS, r1 = min(rows, r0 + CONV_ROWS);
+  const int r0 = blockIdx.y * CONV_ROWS;
+  Run<T, V> now[CONV_ROWS], at[4];  // this thread's rows; inputs of the three tokens before and of this one
+#pragma unroll
+  for (int u = 0; u < CONV_ROWS; ++u)
+    if (r0 + u < rows) now[u] = *reinterpret_cast<const Run<T, V>*>(in + (size_t)(r0 + u) * in_stride + c);
   int seq = row_seq[r0], first = cu_q[seq], end = cu_q[seq + 1];
-  Run<T, V> at[4];  // inputs of the three tokens before and of this one
   auto before = [&](int r, int back) {  // the input `back` tokens before row r of this sequence
     const T* p = r - back >= first ? in + (size_t)(r - back) * in_stride + c
                                    : tail + ((size_t)seq_slot[seq] * 3 + 3 - (first - (r - back))) * ch + c;
@@ -112,34 +119,28 @@ causal_conv4_kernel(T* __restrict__ out, const T* __restrict__ in, int in_stride
   };
 #pragma unroll
   for (int j = 0; j < 3; ++j) at[j + 1] = before(r0, 3 - j);
-  for (int r = r0; r < r1; r += 4) {
-    Run<T, V> now[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (r + u < r1) now[u] = *reinterpret_cast<const Run<T, V>*>(in + (size_t)(r + u) * in_stride + c);
+  for (int u = 0; u < CONV_ROWS; ++u) {
+    if (r0 + u >= rows) break;
+    if (r0 + u == end) {  // the next sequence begins
+      seq = row_seq[r0 + u];
+      first = r0 + u;
+      end = cu_q[seq + 1];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      if (r + u >= r1) break;
-      if (r + u == end) {  // the next sequence begins
-        seq = row_seq[r + u];
-        first = r + u;
-        end = cu_q[seq + 1];
-#pragma unroll
-        for (int j = 0; j < 3; ++j) at[j + 1] = before(r + u, 3 - j);
-      }
-#pragma unroll
-      for (int j = 0; j < 3; ++j) at[j] = at[j + 1];
-      at[3] = now[u];
-      float acc[V];
-#pragma unroll
-      for (int i = 0; i < V; ++i) {
-        acc[i] = b[i];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i] += wj[j][i] * to_float<T>(at[j].v[i]);
-        acc[i] = silu_f(acc[i]);
-      }
-      store_run<T, V>(out + (size_t)(r + u) * ch + c, acc);
+      for (int j = 0; j < 3; ++j) at[j + 1] = before(r0 + u, 3 - j);
     }
+#pragma unroll
+    for (int j = 0; j < 3; ++j) at[j] = at[j + 1];
+    at[3] = now[u];
+    float acc[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      acc[i] = b[i];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i] += wj[j][i] * to_float<T>(at[j].v[i]);
+      acc[i] = silu_to<T>(acc[i]);
+    }
+    store_run<T, V>(out + (size_t)(r0 + u) * ch + c, acc);
   }
 }
 
@@ -435,7 +436,7 @@ __global__ void gated_group_norm_kernel(T* __restrict__ out, int out_stride, int
     load_run<T, V>(z + (size_t)r * z_stride + c0 + i, zv);
 #pragma unroll
     for (int k = 0; k < V; ++k) {
-      const float v = yv[k] * silu_f(zv[k]);
+      const float v = yv[k] * silu_to<T>(zv[k]);
       row_s[i + k] = v;
       sq += v * v;
     }
@@ -478,7 +479,7 @@ gated_group_norm_warp_kernel(T* __restrict__ out, int out_stride, int out_col, f
     if (4 * (lane + 32 * i) >= n) continue;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      v[i][k] *= silu_f(zv[i][k]);
+      v[i][k] *= silu_to<T>(zv[i][k]);
       sq += v[i][k] * v[i][k];
     }
   }
