@@ -16,8 +16,8 @@
 //   Packed multiply-adds (fma.rn.f32x2) were measured and are slower here (274 to 294 us): the copies that pair an
 //   operand with itself cost more than the pipe's register reads gain.
 // * gemm_f32_few: up to 16 float32 rows. Bound by the weights' bytes: each is read once, by asynchronous 16-byte copies
-//   several slices ahead; a thread owns one or two output columns of one or two rows. One row of 151,936 x 2,560: 252 us,
-//   6.2 TB/s; three rows 361 us, of 2,560 x 4,096 26 us (the general kernel: 1.9 ms and 570 us).
+//   a slice ahead; a thread owns one or two output columns of one or two rows. One row of 151,936 x 2,560: 241 us,
+//   6.5 TB/s; three rows 262 us, of 2,560 x 4,096 22 us, where the chain of K multiply-adds is the bound (the general kernel: 1.9 ms and 570 us).
 // * gemm_nt: everything else (bfloat16 inputs with float32 output at odd sizes, for output-head logits at many
 //   positions; float32 rows whose size or alignment does not allow 16-byte accesses). 64x64 output tile, k in slices of
 //   16, 256 threads with a 4x4 micro-tile each.
@@ -203,11 +203,13 @@ gemm_f32_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const f
 }
 
 // ---- float32, up to 16 rows ------------------------------------------------------------------------------------
-// A block owns 16 * CPT columns (a thread c, c + 16); its 8 groups of 16 threads take RPT rows each. A slice is 128 k of
-// the columns' weights and of the rows; DEPTH slices are on the way, 40 or 80 KB of weights a block, which is what an SM
-// has to have in flight to draw its share of the memory's bandwidth. Beyond 8 rows, where shared-memory reads are the
+// A block owns 16 * CPT columns (a thread c, c + 16); its 8 groups of 16 threads take RPT rows each. A slice is 256 k of
+// the columns' weights and of the rows, and the next one is on its way while one is multiplied. What an SM has in flight is a matter of how
+// many blocks it holds, not of how deep each one's ring is: with two slices of 256 k, 35 KB a block at one row, five or six
+// blocks share an SM; six slices of 128 left room for three, whose waits and chains did not cover each other (three rows of 151,936
+// x 2,560 367 us, now 262; 16 rows of 19,456 x 2,560 114 and 101). Beyond 8 rows, where shared-memory reads are the
 // bound, a thread's two rows of two columns read half as much for a multiply-add as one of one.
-constexpr int FEW_K = 128, FEW_PITCH = FEW_K + 4, FEW_DEPTH = 6;
+constexpr int FEW_K = 256, FEW_PITCH = FEW_K + 4, FEW_DEPTH = 2;
 
 template <int RPT, int CPT>
 __global__ void __launch_bounds__(128)
@@ -222,15 +224,16 @@ gemm_f32_few_kernel(float* __restrict__ C, const float* __restrict__ A, const fl
   const int n0 = blockIdx.x * COLS;
   const int slices = (K + FEW_K - 1) / FEW_K;
   const uint64_t policy = l2_evict_first_policy();
-  const int ck = (tid & 31) * 4, cr = tid >> 5;  // this thread copies k = ck..ck+3 of rows cr, cr + 4, ...
+  constexpr int COPY_ROWS = 128 / (FEW_K / 4);  // rows that the threads copy at a time
+  const int ck = tid % (FEW_K / 4) * 4, cr = tid / (FEW_K / 4);  // this thread copies k = ck..ck+3 of rows cr, cr + COPY_ROWS, ...
   auto request = [&](int s) {
     const int k = s * FEW_K + ck;
     if (k < K) {  // what lies beyond K is never read: the loops below end there
       float* dst = sm + (s % FEW_DEPTH) * stage_floats + ck;
 #pragma unroll
-      for (int r = 0; r < COLS; r += 4)
+      for (int r = 0; r < COLS; r += COPY_ROWS)
         if (n0 + cr + r < N) cp_async_16_stream(dst + (cr + r) * FEW_PITCH, W + (size_t)(n0 + cr + r) * ldw + k, policy);
-      for (int r = cr; r < M; r += 4) cp_async_16(dst + (COLS + r) * FEW_PITCH, A + (size_t)r * lda + k);
+      for (int r = cr; r < M; r += COPY_ROWS) cp_async_16(dst + (COLS + r) * FEW_PITCH, A + (size_t)r * lda + k);
     }
     cp_async_commit();  // one group a slice, empty beyond the last, so that the count of waits holds
   };
@@ -320,7 +323,7 @@ int launch_tile(float* C, const float* A, const float* W, int M, int N, int K, i
 template <int RPT, int CPT>
 int launch_few(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
   constexpr size_t per_row = (size_t)FEW_DEPTH * FEW_PITCH * sizeof(float);
-  const size_t smem = (16 * CPT + M) * per_row;  // 54 to 152 KB
+  const size_t smem = (16 * CPT + M) * per_row;  // 35 to 100 KB
   // always the most that a call may need: another thread may be about to launch with more rows than this one
   cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<RPT, CPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((16 * CPT + 8 * RPT) * per_row));
   if (e != cudaSuccess) return (int)e;
@@ -343,7 +346,7 @@ int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, in
   const long long c22 = cost(64, 128, 120, 89), c21 = cost(64, 64, 88, 47), c12 = cost(32, 128, 96, 49);
   const long long best = min(c22, min(c21, c12));
   if (M <= 8) return launch_few<1, 1>(C, A, W, M, N, K, lda, ldw, ldc, stream);
-  // 9 to 16 rows: 17 cycles a block (115 us at 16 rows of 19,456 x 2,560 against the tiles' 192; 740 against 641 at 151,936)
+  // 9 to 16 rows: 17 cycles a block (101 us at 16 rows of 19,456 x 2,560 against the tiles' 192; 740 against 641 at 151,936)
   if (M <= 16 && ((long long)(N + 31) / 32 + 147) / 148 * 17 <= best) return launch_few<2, 2>(C, A, W, M, N, K, lda, ldw, ldc, stream);
   if (best == c22) return launch_tile<2, 2>(C, A, W, M, N, K, lda, ldw, ldc, stream);
   if (best == c21) return launch_tile<2, 1>(C, A, W, M, N, K, lda, ldw, ldc, stream);
