@@ -2,8 +2,8 @@
 //
 // The scan of recurrent.cu takes a sequence's tokens one after the other: 0.57 us a token (delta rule) or 0.40 (time
 // mixing) whatever the batch, on as many SMs as there are heads and sequences. Here a chunk's tokens become small matrix
-// products, and all chunks but for one walk run side by side. The delta rule is float32 on the CUDA cores, as it is there, and
-// time mixing float32 in three bfloat16 terms on the tensor cores; only the order of the sums differs. With the state S before the chunk, c_t the log decays summed from the chunk's first
+// products, and all chunks but for one walk run side by side. The arithmetic is that of float32, as it is there: on the CUDA cores,
+// and in the products, where operands are three bfloat16 terms each, on the tensor cores; only the order of the sums differs. With the state S before the chunk, c_t the log decays summed from the chunk's first
 // token to t, and rows of the chunk's tokens:
 //
 //   time mixing:  o_t = (r_t e^{c_{t-1}}) . S + sum_{s<t} [sum_n r_tn k_sn e^{c_{t-1,n} - c_{s,n}}] v_s + (r_t . bonus k_t) v_t
@@ -22,7 +22,7 @@
 // its starting state in G's place and the sequence its final one; (3) per (sequence, chunk, head) the outputs with their norm,
 // weight and gate. Chunks of 32: a chunk of 64 needs twice the multiply-adds a token in pass 1 and halves the walk's steps.
 //
-// Measured: one prompt of 2,048 tokens, delta rule of 8 heads, 1,171 -> 107 us (the passes 62, 34 and 11); three prompts of
+// Measured: one prompt of 2,048 tokens, delta rule of 8 heads, 1,171 -> 95 us (the passes 50, 34 and 11); three prompts of
 // 2,553 tokens in all, time mixing of 40 heads, 405 -> 128 us (45, 15, 68; with float32 on the CUDA cores 57, 15 and 115). Passes 1
 // and 3 are bound by instruction issue and latencies (a 0.4 to 0.5 share of the issue slots, 12 to 32 warps an SM), the walk by the chain of its steps.
 //
@@ -36,7 +36,8 @@ namespace {
 constexpr int L = 32;         // tokens per chunk
 constexpr int N = 64;         // channels of a head
 constexpr int PITCH = N + 4;  // rows on 16-byte boundaries; eight neighbouring rows' pieces fall into different banks
-constexpr int THREADS = 128;
+constexpr int THREADS = 128, HALF = L / 2;
+constexpr int DELTA_THREADS = 256, PART = L * N / DELTA_THREADS;  // pass 1 of the delta rule: a thread has PART tokens of a channel
 constexpr float SAFE = 40.f;  // keys up to 1e21 stay finite times e^SAFE
 constexpr int WALK_COLS = 4;    // value columns a block of pass 2 walks with
 constexpr int WALK_STAGES = 6;  // chunks whose M are on the way, and the one at hand
@@ -75,14 +76,14 @@ __device__ __forceinline__ float dot4(float4 a, float4 b, float d) {
   return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, d))));
 }
 
-// W2 tanh(lora) of a chunk's tokens, a thread one channel of half of them.
-constexpr int HALF = L / 2;
-__device__ __forceinline__ void low_rank_rows(const ChunkArgs& a, float (&z)[HALF], const float* th_s, int ch0) {
-  const int ch = threadIdx.x & (N - 1), t0 = threadIdx.x / N * HALF, RP = (a.R + 7) & ~7;
-  const bf16* w2 = a.w2 + (size_t)(ch0 + ch) * a.R;
+// W2 tanh(lora) of tokens t0 .. t0 + T - 1 for one channel
+template <int T>
+__device__ __forceinline__ void low_rank_rows(const ChunkArgs& a, float (&z)[T], const float* th_s, int channel, int t0) {
+  const int RP = (a.R + 7) & ~7;
+  const bf16* w2 = a.w2 + (size_t)channel * a.R;
   const bool wide = a.R % 8 == 0 && ((uintptr_t)a.w2 & 7) == 0;  // in pieces of four
 #pragma unroll
-  for (int t = 0; t < HALF; ++t) z[t] = 0.f;
+  for (int t = 0; t < T; ++t) z[t] = 0.f;
   for (int m = 0; m < RP; m += 8) {
     float w[8];
     if (wide) {
@@ -93,7 +94,7 @@ __device__ __forceinline__ void low_rank_rows(const ChunkArgs& a, float (&z)[HAL
       for (int i = 0; i < 8; ++i) w[i] = m + i < a.R ? __bfloat162float(w2[m + i]) : 0.f;
     }
 #pragma unroll
-    for (int t = 0; t < HALF; ++t) {
+    for (int t = 0; t < T; ++t) {
       const float4 x = ld4(th_s + (t0 + t) * RP + m), y = ld4(th_s + (t0 + t) * RP + m + 4);
       z[t] = fmaf(x.w, w[3], fmaf(x.z, w[2], fmaf(x.y, w[1], fmaf(x.x, w[0], z[t]))));
       z[t] = fmaf(y.w, w[7], fmaf(y.z, w[6], fmaf(y.y, w[5], fmaf(y.x, w[4], z[t]))));
@@ -101,54 +102,13 @@ __device__ __forceinline__ void low_rank_rows(const ChunkArgs& a, float (&z)[HAL
   }
 }
 
-// Delta rule: the log decays summed over the chunk's tokens (zero decay beyond the last), into cs [L][PITCH]; what the
-// running sums round off goes to `rest`: a sum of 18 rounds at 1e-6, which e^c would multiply everything by. `total` is [2][N].
-// Ends with a barrier.
-__device__ __forceinline__ void summed_decays(const ChunkArgs& a, float* cs, float* rest, float* total, const float* th_s, int ch0, int nt) {
-  const int ch = threadIdx.x & (N - 1), half = threadIdx.x / N, t0 = half * HALF;
-  float z[HALF];
-  low_rank_rows(a, z, th_s, ch0);
-  const float w0 = a.w0[ch0 + ch];
-  float run = 0.f, lost = 0.f, low[HALF];
-#pragma unroll
-  for (int t = 0; t < HALF; ++t) {
-    float x = -a.decay_scale * sigmoid_f(z[t] + w0);
-    if (t0 + t >= nt) x = 0.f;
-    const float sum = run + x, y = sum - run;
-    lost += (run - (sum - y)) + (x - y);
-    low[t] = lost;
-    z[t] = run = sum;
-  }
-  if (half == 0) {
-    total[ch] = run;
-    total[N + ch] = lost;
-  }
-  __syncthreads();
-  const float before = half ? total[ch] : 0.f, before_low = half ? total[N + ch] : 0.f;
-#pragma unroll
-  for (int t = 0; t < HALF; ++t) {
-    const float sum = before + z[t], y = sum - before;
-    cs[(t0 + t) * PITCH + ch] = sum;
-    rest[(t0 + t) * PITCH + ch] = low[t] + before_low + ((before - (sum - y)) + (z[t] - y));
-  }
-  __syncthreads();
-}
-
 // tanh of the low-rank input in the path's precision, [L][R rounded up to 8], zeros beyond the tokens and R
 __device__ __forceinline__ void load_tanh(const ChunkArgs& a, float* th_s, size_t row0, int nt) {
   const int RP = (a.R + 7) & ~7;
-  for (int t = threadIdx.x >> 3; t < L; t += THREADS / 8)
+  for (int t = threadIdx.x >> 3; t < L; t += blockDim.x >> 3)
     for (int m = threadIdx.x & 7; m < RP; m += 8)
       th_s[t * RP + m] = t < nt && m < a.R ? round_to<bf16>(tanhf(__bfloat162float(a.lora[(row0 + t) * a.lora_stride + m]))) : 0.f;
 }
-__device__ __forceinline__ void load_rows(float* dst, const bf16* src, int stride, size_t row0, int ch0, int nt) {
-#pragma unroll
-  for (int i = threadIdx.x; i < L * (N / 4); i += THREADS) {
-    const int t = i / (N / 4), c = (i % (N / 4)) * 4;
-    st4(dst + t * PITCH + c, t < nt ? widen4(src + (row0 + t) * stride + ch0 + c) : make_float4(0.f, 0.f, 0.f, 0.f));
-  }
-}
-
 // A warp's place in a product of 64 columns: 16 columns a warp, lanes 8 x 4, neighbouring lanes sharing a row or a column
 // (a warp's 16-byte read of shared memory then takes 2 cycles, not 4).
 struct Place {
@@ -160,192 +120,7 @@ struct Place {
   }
 };
 
-// ---- pass 1, delta rule ----------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(THREADS, 3) delta_chunk_kernel(ChunkArgs a) {
-  extern __shared__ __align__(16) float sm[];
-  float* us = sm;                  // [L][PITCH] u_t e^{c_{t-1}}; then X
-  float* rs = us + L * PITCH;      // [L][PITCH] r_t e^{c_t} (behind us: one matrix of 2 L rows)
-  float* ks = rs + L * PITCH;      // [L][PITCH] k_s e^{-c_s}
-  float* as = ks + L * PITCH;      // [L][PITCH] a_s u_s e^{-c_s} (behind ks)
-  float* vs = as + L * PITCH;      // [L][PITCH]
-  float* zs = vs + L * PITCH;      // [L][PITCH] c, then Z
-  float* es = zs + L * PITCH;      // [2 L][PITCH] products of us, rs with ks, as: B, D above P, R; before, the rest of c
-  float* last = es + 2 * L * PITCH;  // [N] e^{c_last}
-  float* inv = last + N;           // [L] 1 / |k|
-  float* th_s = us;                // [L][R rounded up]; gone before us is written
-  const int h = blockIdx.x, ci = blockIdx.y, seq = blockIdx.z, ch0 = h * N;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  grid_dependency_wait();
-  const int first = (a.chunk0 + ci) * L, nt = min(L, a.seq_qlen[seq] - first);
-  if (nt <= 0) return;
-  const size_t row0 = (size_t)a.cu_q[seq] + first;
-  load_rows(rs, a.r, a.r_stride, row0, ch0, nt);
-  load_rows(ks, a.k, a.k_stride, row0, ch0, nt);
-  load_rows(vs, a.v, a.v_stride, row0, ch0, nt);
-  load_rows(as, a.rate, a.rate_stride, row0, ch0, nt);
-  load_tanh(a, th_s, row0, nt);
-  __syncthreads();
-  for (int t = warp; t < L; t += THREADS / 32) {
-    const float x = ks[t * PITCH + lane], y = ks[t * PITCH + lane + 32];
-    const float sq = warp_sum(x * x + y * y);
-    if (lane == 0) inv[t] = rsqrtf(sq + 1e-6f);
-  }
-  summed_decays(a, zs, es, es + L * PITCH, th_s, ch0, nt);
-  {
-    const int ch = tid & 63;
-    const float bias = a.rate_bias[ch0 + ch];
-#pragma unroll 4
-    for (int t = tid >> 6; t < L; t += 2) {
-      const int at = t * PITCH + ch;
-      const float c = zs[at], c1 = es[at];
-      const float k = ks[at], u = k * inv[t], back = expf(-c) * (1.f - c1);
-      const float before = t ? zs[at - PITCH] : 0.f, before1 = t ? es[at - PITCH] : 0.f;
-      us[at] = u * (expf(before) * (1.f + before1));
-      rs[at] *= expf(c) * (1.f + c1);
-      as[at] = sigmoid_f(as[at] + bias) * u * back;
-      ks[at] = k * back;
-      if (t == L - 1) last[ch] = expf(c) * (1.f + c1);
-    }
-  }
-  __syncthreads();
-  {  // [us; rs] [ks; as]^T, 4 rows (16 apart) x 8 columns (8 apart) a thread; what looks ahead is zeroed
-    const int ty = (warp & 1) * 8 + ((lane & 15) >> 1), tx = (warp >> 1) * 4 + (lane & 1) + 2 * (lane >> 4);
-    float e[4][8];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) e[i][j] = 0.f;
-#pragma unroll 2
-    for (int n = 0; n < N; n += 4) {
-      float4 x[4], y[8];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) x[i] = ld4(us + (ty + 16 * i) * PITCH + n);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) y[j] = ld4(ks + (tx + 8 * j) * PITCH + n);
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) e[i][j] = dot4(x[i], y[j], e[i][j]);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int row = ty + 16 * i, col = tx + 8 * j, t = row & (L - 1), s = col & (L - 1);
-        es[row * PITCH + col] = s < t || (s == t && row >= L) ? e[i][j] : 0.f;
-      }
-  }
-  __syncthreads();
-  {  // forward substitution, a column of [X | Z] a thread; four partial sums a row
-    float x[L];
-    if (warp < 2) {
-#pragma unroll
-      for (int t = 0; t < L; ++t) {
-        float p[4] = {us[t * PITCH + tid], 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int s = 0; s < t; s += 4) {
-          const float4 d = ld4(es + t * PITCH + L + s);
-          p[0] = fmaf(-d.x, x[s], p[0]);
-          if (s + 1 < t) p[1] = fmaf(-d.y, x[s + 1], p[1]);
-          if (s + 2 < t) p[2] = fmaf(-d.z, x[s + 2], p[2]);
-          if (s + 3 < t) p[3] = fmaf(-d.w, x[s + 3], p[3]);
-        }
-        x[t] = (p[0] + p[1]) + (p[2] + p[3]);
-      }
-#pragma unroll
-      for (int t = 0; t < L; ++t) us[t * PITCH + tid] = x[t];
-    } else {
-      const int p0 = tid - N;
-      float v[L];
-#pragma unroll
-      for (int t = 0; t < L; ++t) v[t] = vs[t * PITCH + p0];
-#pragma unroll
-      for (int t = 0; t < L; ++t) {
-        float p[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int s = 0; s < t; s += 4) {
-          const float4 b = ld4(es + t * PITCH + s), d = ld4(es + t * PITCH + L + s);
-          p[0] = fmaf(-d.x, x[s], fmaf(b.x, v[s], p[0]));
-          if (s + 1 < t) p[1] = fmaf(-d.y, x[s + 1], fmaf(b.y, v[s + 1], p[1]));
-          if (s + 2 < t) p[2] = fmaf(-d.z, x[s + 2], fmaf(b.z, v[s + 2], p[2]));
-          if (s + 3 < t) p[3] = fmaf(-d.w, x[s + 3], fmaf(b.w, v[s + 3], p[3]));
-        }
-        x[t] = (p[0] + p[1]) + (p[2] + p[3]);
-      }
-#pragma unroll
-      for (int t = 0; t < L; ++t) zs[t * PITCH + p0] = x[t];
-    }
-  }
-  __syncthreads();
-  // only now: a block of the walk that waited from the start would hold the shared memory that this kernel's blocks need
-  grid_launch_dependents();
-  float* item = a.scratch + (((size_t)seq * a.n_chunks + ci) * a.H + h) * ITEM_DELTA;
-  const Place at;
-  {  // Q and O_own: rows ty, ty + 8, ... of the chunk
-    float4 q[4], o[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      q[i] = ld4(rs + (at.ty + 8 * i) * PITCH + at.col);
-      o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-#pragma unroll 2
-    for (int s = 0; s < L; s += 4) {
-      float p[4][4], r[4][4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        st4(p[i], ld4(es + (L + at.ty + 8 * i) * PITCH + s));
-        st4(r[i], ld4(es + (L + at.ty + 8 * i) * PITCH + L + s));
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float4 x = ld4(us + (s + j) * PITCH + at.col), v = ld4(vs + (s + j) * PITCH + at.col), z = ld4(zs + (s + j) * PITCH + at.col);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (s + j <= at.ty + 8 * i) {  // a later token's infinities stay its own
-            fma4(q[i], -r[i][j], x);
-            fma4(o[i], p[i][j], v);
-            fma4(o[i], -r[i][j], z);
-          }
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      st4(item + 2 * N * N + (at.ty + 8 * i) * N + at.col, q[i]);
-      st4(item + 2 * N * N + L * N + (at.ty + 8 * i) * N + at.col, o[i]);
-    }
-  }
-  {  // M and G: key channels 4 ty .. and 32 + 4 ty ..
-    float4 m[8], g[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) m[i] = g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 2
-    for (int s = 0; s < L; ++s) {
-      float ar[8], kr[8];
-      st4(ar, ld4(as + s * PITCH + 4 * at.ty));
-      st4(ar + 4, ld4(as + s * PITCH + 32 + 4 * at.ty));
-      st4(kr, ld4(ks + s * PITCH + 4 * at.ty));
-      st4(kr + 4, ld4(ks + s * PITCH + 32 + 4 * at.ty));
-      const float4 x = ld4(us + s * PITCH + at.col), v = ld4(vs + s * PITCH + at.col), z = ld4(zs + s * PITCH + at.col);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        fma4(m[i], -ar[i], x);
-        fma4(g[i], kr[i], v);
-        fma4(g[i], -ar[i], z);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int n = 32 * (i >> 2) + 4 * at.ty + (i & 3);
-      const float w = last[n];
-      m[i].x += n == at.col ? 1.f : 0.f; m[i].y += n == at.col + 1 ? 1.f : 0.f;
-      m[i].z += n == at.col + 2 ? 1.f : 0.f; m[i].w += n == at.col + 3 ? 1.f : 0.f;
-      st4(item + n * N + at.col, make_float4(w * m[i].x, w * m[i].y, w * m[i].z, w * m[i].w));
-      st4(item + N * N + n * N + at.col, make_float4(w * g[i].x, w * g[i].y, w * g[i].z, w * g[i].w));
-    }
-  }
-}
-
-// ---- time mixing's products on the tensor cores ------------------------------------------------------------------
+// ---- products on the tensor cores ----------------------------------------------------------------------------------
 // mma.sync m16n8k16, float32 accumulate. Values are bfloat16 already; every other operand is handed over as three bfloat16 terms
 // that add up to it, and where both sides are such sums the six products that matter in 32-bit are formed, small ones first.
 constexpr int KP = N + 8;   // bfloat16 rows in shared memory: ldmatrix reads eight of them from different banks
@@ -374,6 +149,378 @@ __device__ __forceinline__ void load_raw(bf16* dst, const bf16* src, int stride,
   }
 }
 
+// The five small products of two operands that are three terms each, into one tile of 16 x 8. The sixth, of the leading terms, is added
+// after the small ones of all of a sum's k: the tensor cores cut every sum off, and a small product would cost a large one its last bit.
+__device__ __forceinline__ void small33(float (&d)[4], const uint32_t (&x)[3][4], const uint32_t (&y)[3][2]) {
+#pragma unroll
+  for (int sum = 2; sum >= 1; --sum)
+#pragma unroll
+    for (int t = 0; t <= sum; ++t) mma_bf16_16816(d, x[t][0], x[t][1], x[t][2], x[t][3], y[sum - t][0], y[sum - t][1]);
+}
+
+// ---- pass 1, delta rule ----------------------------------------------------------------------------------------
+// Eight warps. A thread makes one channel of eight tokens' rows; six warps multiply [U; Rows] [K; A]^T, a warp four tiles of 16 x 8; four
+// solve for a column of [X | Z] a thread, with float32 multiply-adds, while the other four multiply K^T V; then four multiply A^T X
+// and four A^T Z, and all of them eight columns of Q and O each. X and Z are kept with their signs turned.
+// Two blocks an SM. Bound by its chains and barriers, the substitution's before all. One prompt of 2,048 tokens, 8 heads: 50 us (with
+// float32 on the CUDA cores, three blocks of four warps an SM, 63).
+__global__ void __launch_bounds__(DELTA_THREADS, 2) delta_chunk_kernel(ChunkArgs a) {
+  extern __shared__ __align__(16) float sm[];
+  constexpr int TERM = L * KP, ROWS3 = 3 * TERM;       // elements of one term of a chunk's rows, of three
+  bf16* ut = reinterpret_cast<bf16*>(sm);              // [3][L][KP] u_t e^{c_{t-1}}; then -X
+  bf16* rt = ut + ROWS3;                               // [3][L][KP] r_t e^{c_t}
+  bf16* kt = rt + ROWS3;                               // [3][L][KP] k_s e^{-c_s}
+  bf16* at = kt + ROWS3;                               // [3][L][KP] a_s u_s e^{-c_s}
+  bf16* zt = at + ROWS3;                               // [3][L][KP] -Z
+  bf16* pt = zt + ROWS3;                               // [3][L][KP] P beside R
+  bf16* vs = pt + ROWS3;                               // [L][KP] the values, what is not finite set aside
+  float* us = reinterpret_cast<float*>(vs + TERM);     // [L][PITCH] u_t e^{c_{t-1}}
+  float* es = us + L * PITCH;                          // [L][PITCH] B beside D
+  float* last = es + L * PITCH;                        // [N] e^{c_last}
+  float* sq = last + N;                                // [2][L] |k|^2, of either half of the channels
+  float2* total = reinterpret_cast<float2*>(sq + 2 * L);  // [4][N] a part's decays, summed, and what that rounded off
+  int* bad = reinterpret_cast<int*>(total + 4 * N);    // [3][N]: the first token that is not finite in a column of X, of Z, of the values
+  float* th_s = us;                                    // [L][R rounded up], over us and es; gone before they are written
+  const int h = blockIdx.x, ci = blockIdx.y, seq = blockIdx.z, ch0 = h * N;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
+  grid_dependency_wait();
+  const int first = (a.chunk0 + ci) * L, nt = min(L, a.seq_qlen[seq] - first);
+  if (nt <= 0) return;
+  const size_t row0 = (size_t)a.cu_q[seq] + first;
+  const int ch = tid & (N - 1), part = tid / N, t0 = part * PART;
+  float r[PART], k[PART], rate[PART];
+#pragma unroll
+  for (int i = 0; i < PART; ++i) {
+    const bool in = t0 + i < nt;
+    const size_t row = row0 + t0 + i;
+    r[i] = in ? __bfloat162float(a.r[row * a.r_stride + ch0 + ch]) : 0.f;
+    k[i] = in ? __bfloat162float(a.k[row * a.k_stride + ch0 + ch]) : 0.f;
+    rate[i] = in ? __bfloat162float(a.rate[row * a.rate_stride + ch0 + ch]) : 0.f;
+  }
+  if (tid < 3 * N) bad[tid] = L;
+  load_tanh(a, th_s, row0, nt);
+  __syncthreads();
+  for (int i = tid; i < L * (N / 4); i += DELTA_THREADS) {  // the values
+    const int t = i / (N / 4), c = (i % (N / 4)) * 4;
+    const uint2 raw = t < nt ? *reinterpret_cast<const uint2*>(a.v + (row0 + t) * a.v_stride + ch0 + c) : make_uint2(0u, 0u);
+    uint32_t two[2] = {raw.x, raw.y};
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const bool lo = (two[j] & 0x7f80u) == 0x7f80u, hi = (two[j] & 0x7f800000u) == 0x7f800000u;
+      if (lo) atomicMin(bad + 2 * N + c + 2 * j, t);
+      if (hi) atomicMin(bad + 2 * N + c + 2 * j + 1, t);
+      if (lo || hi) two[j] &= (lo ? 0xffff0000u : 0xffffffffu) & (hi ? 0xffffu : 0xffffffffu);
+    }
+    *reinterpret_cast<uint2*>(vs + t * KP + c) = make_uint2(two[0], two[1]);
+  }
+  float c[PART], rest[PART];  // the log decays summed over the chunk's tokens (zero decay beyond the last), and what the running sums round off:
+                              // a sum of 18 rounds at 1e-6, which e^c would multiply everything by
+  {
+    low_rank_rows<PART>(a, c, th_s, ch0 + ch, t0);
+    const float w0 = a.w0[ch0 + ch];
+    float run = 0.f, lost = 0.f;
+#pragma unroll
+    for (int i = 0; i < PART; ++i) {
+      float x = -a.decay_scale * sigmoid_f(c[i] + w0);
+      if (t0 + i >= nt) x = 0.f;
+      const float sum = run + x, y = sum - run;
+      lost += (run - (sum - y)) + (x - y);
+      rest[i] = lost;
+      c[i] = run = sum;
+    }
+    total[part * N + ch] = make_float2(run, lost);
+#pragma unroll
+    for (int i = 0; i < PART; ++i) {
+      const float s = warp_sum(k[i] * k[i]);
+      if (lane == 0) sq[(warp & 1) * L + t0 + i] = s;
+    }
+  }
+  __syncthreads();  // th_s is no longer read
+  {
+    float before = 0.f, before1 = 0.f;  // the sums of the parts before
+    for (int q = 0; q < part; ++q) {
+      const float2 f = total[q * N + ch];
+      const float sum = before + f.x, y = sum - before;
+      before1 += f.y + ((before - (sum - y)) + (f.x - y));
+      before = sum;
+    }
+    const float bias = a.rate_bias[ch0 + ch];
+    float c_prev = before, c1_prev = before1;
+#pragma unroll
+    for (int i = 0; i < PART; ++i) {
+      const int t = t0 + i, at1 = t * KP + ch;
+      const float sum = before + c[i], y = sum - before;
+      const float c1 = rest[i] + before1 + ((before - (sum - y)) + (c[i] - y));
+      const float u = k[i] * rsqrtf(sq[t] + sq[L + t] + 1e-6f), back = expf(-sum) * (1.f - c1), on = expf(sum) * (1.f + c1);
+      const float ue = u * (expf(c_prev) * (1.f + c1_prev));
+      us[t * PITCH + ch] = ue;
+      split3_store(ut + at1, TERM, ue);
+      split3_store(rt + at1, TERM, r[i] * on);
+      split3_store(kt + at1, TERM, k[i] * back);
+      split3_store(at + at1, TERM, sigmoid_f(rate[i] + bias) * u * back);
+      c_prev = sum;
+      c1_prev = c1;
+      if (t == L - 1) last[ch] = on;
+    }
+  }
+  __syncthreads();
+  if (warp < 6) {  // [U; Rows] [K; A]^T without the tiles that look ahead
+    // warps 0, 3: tokens 0..15 of U, of Rows, against tokens 0..15 of K and A; 1, 4: tokens 16..31 against K; 2, 5: against A
+    const int which = warp % 3;
+    const bool rows = warp >= 3;
+    const int m0 = which ? 16 : 0;
+    const bf16* x = rows ? rt : ut;
+    float e[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) e[j][q] = 0.f;
+#pragma unroll
+    for (int leading = 0; leading < 2; ++leading)
+#pragma unroll
+      for (int kk = 0; kk < N; kk += 16) {
+        uint32_t xf[3][4];
+#pragma unroll
+        for (int t = 0; t < (leading ? 1 : 3); ++t)
+          ldmatrix_x4(xf[t][0], xf[t][1], xf[t][2], xf[t][3], x + t * TERM + (m0 + (lane & 15)) * KP + kk + (lane >> 4) * 8);
+#pragma unroll
+        for (int j = 0; j < 4; j += 2) {  // 16 tokens of K or A
+          const bf16* y = (which == 0 ? j == 2 : which == 2) ? at : kt;
+          const int s0 = which == 0 ? 0 : j * 8;
+          uint32_t y0[3][2], y1[3][2];
+#pragma unroll
+          for (int t = 0; t < (leading ? 1 : 3); ++t)
+            ldmatrix_x4(y0[t][0], y0[t][1], y1[t][0], y1[t][1],
+                        y + t * TERM + (s0 + ((lane >> 4) << 3) + (lane & 7)) * KP + kk + ((lane >> 3) & 1) * 8);
+          if (leading) {
+            mma_bf16_16816(e[j], xf[0][0], xf[0][1], xf[0][2], xf[0][3], y0[0][0], y0[0][1]);
+            mma_bf16_16816(e[j + 1], xf[0][0], xf[0][1], xf[0][2], xf[0][3], y1[0][0], y1[0][1]);
+          } else {
+            small33(e[j], xf, y0);
+            small33(e[j + 1], xf, y1);
+          }
+        }
+      }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int s0 = (which == 0 ? (j & 1) * 8 : j * 8) + 2 * t4;              // the token of K or A
+      const int col = s0 + ((which == 0 ? j >= 2 : which == 2) ? L : 0);       // B or P in front, D or R behind
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh) {
+        const int t = m0 + g + 8 * hh;
+        if (!rows) {
+          *reinterpret_cast<float2*>(es + t * PITCH + col) = make_float2(s0 < t ? e[j][2 * hh] : 0.f, s0 + 1 < t ? e[j][2 * hh + 1] : 0.f);
+        } else {
+          uint32_t three[3];
+          split3_pair(s0 <= t ? e[j][2 * hh] : 0.f, s0 + 1 <= t ? e[j][2 * hh + 1] : 0.f, three);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(pt + i * TERM + t * KP + col) = three[i];
+        }
+      }
+    }
+  }
+  __syncthreads();
+  float* item = a.scratch + (((size_t)seq * a.n_chunks + ci) * a.H + h) * ITEM_DELTA;
+  const int m0 = (warp & 3) * 16;  // key channels of this warp's tiles of M (warps 0..3) or G (4..7)
+  float d[N / 8][4];
+#pragma unroll
+  for (int n = 0; n < N / 8; ++n)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) d[n][q] = 0.f;
+  // 16 rows of the transpose of a term's rows, of tokens s .. s + 15
+  auto transposed = [&](uint32_t (&f)[4], const bf16* rows, int s) {
+    ldmatrix_x4_trans(f[0], f[1], f[2], f[3], rows + (s + (lane & 7) + ((lane >> 4) & 1) * 8) * KP + m0 + ((lane >> 3) & 1) * 8);
+  };
+  auto tokens = [&](uint32_t (&f)[4], const bf16* rows, int s, int n) {  // tokens s .. s + 15 of columns 8 n .. 8 n + 15
+    ldmatrix_x4_trans(f[0], f[1], f[2], f[3], rows + (s + (lane & 7) + ((lane >> 3) & 1) * 8) * KP + (n + (lane >> 4)) * 8);
+  };
+  if (warp < 4) {  // forward substitution, a column of [X | Z] a thread; four partial sums a row
+    const bool is_z = warp >= 2;
+    const int col = tid & (N - 1);
+    float x[L];
+    int nonfinite = L;
+    if (!is_z) {
+#pragma unroll
+      for (int t = 0; t < L; ++t) {
+        float p[4] = {us[t * PITCH + col], 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int s = 0; s < t; s += 4) {
+          const float4 e = ld4(es + t * PITCH + L + s);
+          p[0] = fmaf(-e.x, x[s], p[0]);
+          if (s + 1 < t) p[1] = fmaf(-e.y, x[s + 1], p[1]);
+          if (s + 2 < t) p[2] = fmaf(-e.z, x[s + 2], p[2]);
+          if (s + 3 < t) p[3] = fmaf(-e.w, x[s + 3], p[3]);
+        }
+        x[t] = (p[0] + p[1]) + (p[2] + p[3]);
+      }
+    } else {
+      float v[L];
+#pragma unroll
+      for (int t = 0; t < L; ++t) v[t] = t < nt ? __bfloat162float(a.v[(row0 + t) * a.v_stride + ch0 + col]) : 0.f;
+#pragma unroll
+      for (int t = 0; t < L; ++t) {
+        float p[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int s = 0; s < t; s += 4) {
+          const float4 b = ld4(es + t * PITCH + s), e = ld4(es + t * PITCH + L + s);
+          p[0] = fmaf(-e.x, x[s], fmaf(b.x, v[s], p[0]));
+          if (s + 1 < t) p[1] = fmaf(-e.y, x[s + 1], fmaf(b.y, v[s + 1], p[1]));
+          if (s + 2 < t) p[2] = fmaf(-e.z, x[s + 2], fmaf(b.z, v[s + 2], p[2]));
+          if (s + 3 < t) p[3] = fmaf(-e.w, x[s + 3], fmaf(b.w, v[s + 3], p[3]));
+        }
+        x[t] = (p[0] + p[1]) + (p[2] + p[3]);
+      }
+    }
+    bf16* to = (is_z ? zt : ut) + col;
+#pragma unroll
+    for (int t = L - 1; t >= 0; --t) {
+      const bool in = fabsf(x[t]) < INFINITY;
+      if (!in) nonfinite = t;
+      split3_store(to + t * KP, TERM, in ? -x[t] : 0.f);  // a product would hand what is not finite, times zero, to the tokens before
+    }
+    bad[(is_z ? N : 0) + col] = nonfinite;
+  } else {  // K^T V: the small terms of K
+#pragma unroll
+    for (int s = 0; s < L; s += 16) {
+      uint32_t kf[2][4];
+      transposed(kf[0], kt + TERM, s);
+      transposed(kf[1], kt + 2 * TERM, s);
+#pragma unroll
+      for (int n = 0; n < N / 8; n += 2) {
+        uint32_t b[4];
+        tokens(b, vs, s, n);
+#pragma unroll
+        for (int t = 1; t >= 0; --t) {
+          mma_bf16_16816(d[n], kf[t][0], kf[t][1], kf[t][2], kf[t][3], b[0], b[1]);
+          mma_bf16_16816(d[n + 1], kf[t][0], kf[t][1], kf[t][2], kf[t][3], b[2], b[3]);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  // only now: a block of the walk that waited from the start would hold the shared memory that this kernel's blocks need
+  grid_launch_dependents();
+  {  // M and G: - A^T X, K^T V - A^T Z
+    const bool is_g = warp >= 4;
+    const bf16* y = is_g ? zt : ut;
+#pragma unroll
+    for (int s = 0; s < L; s += 16) {
+      uint32_t af[3][4];
+#pragma unroll
+      for (int t = 0; t < 3; ++t) transposed(af[t], at + t * TERM, s);
+#pragma unroll
+      for (int n = 0; n < N / 8; n += 2) {
+        uint32_t y0[3][2], y1[3][2];
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+          uint32_t f[4];
+          tokens(f, y + t * TERM, s, n);
+          y0[t][0] = f[0]; y0[t][1] = f[1]; y1[t][0] = f[2]; y1[t][1] = f[3];
+        }
+        small33(d[n], af, y0);
+        small33(d[n + 1], af, y1);
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < L; s += 16) {
+      uint32_t af[4], kf[4];
+      transposed(af, at, s);
+      transposed(kf, kt, s);
+#pragma unroll
+      for (int n = 0; n < N / 8; n += 2) {
+        uint32_t f[4];
+        tokens(f, y, s, n);
+        mma_bf16_16816(d[n], af[0], af[1], af[2], af[3], f[0], f[1]);
+        mma_bf16_16816(d[n + 1], af[0], af[1], af[2], af[3], f[2], f[3]);
+        if (is_g) {
+          tokens(f, vs, s, n);
+          mma_bf16_16816(d[n], kf[0], kf[1], kf[2], kf[3], f[0], f[1]);
+          mma_bf16_16816(d[n + 1], kf[0], kf[1], kf[2], kf[3], f[2], f[3]);
+        }
+      }
+    }
+    const int* worst = bad + (is_g ? N : 0);
+#pragma unroll
+    for (int n = 0; n < N / 8; ++n)
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh) {
+        const int row = m0 + g + 8 * hh, col = n * 8 + 2 * t4;
+        const float w = last[row];
+        float v[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          v[j] = d[n][2 * hh + j];
+          if (!is_g && row == col + j) v[j] += 1.f;
+          v[j] = worst[col + j] < L || (is_g && bad[2 * N + col + j] < L) ? NAN : w * v[j];
+        }
+        *reinterpret_cast<float2*>(item + (is_g ? N * N : 0) + row * N + col) = make_float2(v[0], v[1]);
+      }
+  }
+  {  // Q and O: columns 8 warp .. 8 warp + 7 of Rows - R X and of P V - R Z
+    const int c0 = warp * 8, col = c0 + 2 * t4;
+    float q[2][4], o[2][4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) q[m][j] = o[m][j] = 0.f;
+    uint32_t xf[3][4], zf[3][4], vf[4];  // of 32 tokens: two of sixteen
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+      ldmatrix_x4_trans(xf[t][0], xf[t][1], xf[t][2], xf[t][3], ut + t * TERM + lane * KP + c0);
+      ldmatrix_x4_trans(zf[t][0], zf[t][1], zf[t][2], zf[t][3], zt + t * TERM + lane * KP + c0);
+    }
+    ldmatrix_x4_trans(vf[0], vf[1], vf[2], vf[3], vs + lane * KP + c0);
+#pragma unroll
+    for (int leading = 0; leading < 2; ++leading)
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int kk = 0; kk <= m; ++kk) {  // not later tokens
+          uint32_t pf[3][4], rf[3][4];
+#pragma unroll
+          for (int t = 0; t < (leading ? 1 : 3); ++t) {
+            const bf16* from = pt + t * TERM + (m * 16 + (lane & 15)) * KP + kk * 16 + (lane >> 4) * 8;
+            if (leading || t) ldmatrix_x4(pf[t][0], pf[t][1], pf[t][2], pf[t][3], from);
+            ldmatrix_x4(rf[t][0], rf[t][1], rf[t][2], rf[t][3], from + L);
+          }
+          if (leading) {
+            mma_bf16_16816(q[m], rf[0][0], rf[0][1], rf[0][2], rf[0][3], xf[0][2 * kk], xf[0][2 * kk + 1]);
+            mma_bf16_16816(o[m], rf[0][0], rf[0][1], rf[0][2], rf[0][3], zf[0][2 * kk], zf[0][2 * kk + 1]);
+            mma_bf16_16816(o[m], pf[0][0], pf[0][1], pf[0][2], pf[0][3], vf[2 * kk], vf[2 * kk + 1]);
+          } else {
+            uint32_t x2[3][2], z2[3][2];
+#pragma unroll
+            for (int t = 0; t < 3; ++t)
+#pragma unroll
+              for (int j = 0; j < 2; ++j) {
+                x2[t][j] = xf[t][2 * kk + j];
+                z2[t][j] = zf[t][2 * kk + j];
+              }
+            small33(q[m], rf, x2);
+            small33(o[m], rf, z2);
+#pragma unroll
+            for (int t = 2; t >= 1; --t) mma_bf16_16816(o[m], pf[t][0], pf[t][1], pf[t][2], pf[t][3], vf[2 * kk], vf[2 * kk + 1]);
+          }
+        }
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh) {
+        const int t = m * 16 + g + 8 * hh;
+        float v[2], w[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const bf16* from = rt + t * KP + col + j;
+          const float row = __bfloat162float(from[0]) + (__bfloat162float(from[TERM]) + __bfloat162float(from[2 * TERM]));  // r e^c again
+          v[j] = t >= bad[col + j] ? NAN : row + q[m][2 * hh + j];
+          w[j] = t >= bad[N + col + j] ? NAN : t >= bad[2 * N + col + j] ? INFINITY : o[m][2 * hh + j];
+        }
+        *reinterpret_cast<float2*>(item + 2 * N * N + t * N + col) = make_float2(v[0], v[1]);
+        *reinterpret_cast<float2*>(item + 2 * N * N + L * N + t * N + col) = make_float2(w[0], w[1]);
+      }
+  }
+}
+
 // ---- pass 1, time mixing ---------------------------------------------------------------------------------------
 // A thread has its channel's decays in registers, and sums them from either end: the weights e^{c_last - c_s} from the last token
 // back and the running sums c_t from the first one on. Neither is a difference of sums, in which a small decay after
@@ -399,7 +546,7 @@ __global__ void __launch_bounds__(THREADS, 8) mix_chunk_kernel(ChunkArgs a) {
   {
     const int ch = threadIdx.x & (N - 1), half = threadIdx.x / N, t0 = half * HALF;
     float x[HALF], run = 0.f;
-    low_rank_rows(a, x, th_s, ch0);
+    low_rank_rows<HALF>(a, x, th_s, ch0 + ch, t0);
     const float w0 = a.w0[ch0 + ch];
 #pragma unroll
     for (int t = 0; t < HALF; ++t) {
@@ -938,7 +1085,9 @@ KRK_API int krk_recurrence_chunks(int rule, const void* r, int r_stride, const v
   int rc;
   const size_t RP = (size_t)((R + 7) & ~7);
   if (rule == 1) {
-    if ((rc = run(delta_chunk_kernel, items, THREADS, 8 * (size_t)L * PITCH + N + L, a, stream))) return rc;
+    // six times three terms of a chunk's rows and the values; two matrices of float32; the small things
+    const size_t chunk = 19 * (size_t)L * KP / 2 + 2 * (size_t)L * PITCH + N + 2 * L + 8 * N + 3 * N;
+    if ((rc = run(delta_chunk_kernel, items, DELTA_THREADS, chunk, a, stream))) return rc;
     const size_t walk = (size_t)WALK_STAGES * N * (PITCH + WALK_COLS) + N * WALK_COLS + 4 * N * 4;
     if ((rc = run(delta_walk_kernel, dim3(N / WALK_COLS, (unsigned)H, (unsigned)n_seqs), THREADS, walk, a, stream))) return rc;
     return run(delta_finish_kernel, items, THREADS, (size_t)L * PITCH + 4 * L, a, stream);
