@@ -1491,13 +1491,13 @@ class Kernels:
     # -- state-space mixer ------------------------------------------------------------------
     SSD_CHUNK = 128  # tokens per chunk where one sequence's step is long enough to be scanned in chunks
 
-    CONV_WALK_BYTES = 5_000_000
+    CONV_WALK_BYTES = 8_400_000
 
     def _conv_walks(self, rows, row_bytes, n_seqs) -> bool:
         """Whether threads of the short convolution go through eight rows each, the rows before in registers. That is one chain of
         5.3 us at least, at a sequence's first row with the loads of its stored rows in it, and pays by bytes: a block a row and
         eight rows a thread, one prompt of 4,096 channels in bfloat16, 64 rows 5.0 and 5.6 us, 256 6.2 and 5.9, 512 8.2 and 7.1,
-        2,048 18.7 and 12.9; of 1,792 channels 512 rows 5.9 and 6.4, 1,024 7.9 and 6.9, 2,048 10.8 and 9.1; 32-bit of 4,096 channels
+        2,048 18.7 and 12.9 (the line is drawn above 1,024 rows of them); of 1,792 channels 512 rows 5.9 and 6.4, 1,024 7.9 and 6.9, 2,048 10.8 and 9.1; 32-bit of 4,096 channels
         256 rows 6.9 and 7.3, 512 9.5 and 7.7. Single tokens of 64 sequences 9.9 and 12.9, of 2,048 equal."""
         return rows * row_bytes >= self.CONV_WALK_BYTES and rows >= 2 * n_seqs
 
