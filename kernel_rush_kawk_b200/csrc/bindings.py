@@ -903,9 +903,14 @@ class Kernels:
         limit, slope = act_params if act_params is not None else (0.0, 1.0)
         w_in, w_out = (weights, None) if weigh_input else (None, weights)  # which end of an expert the weights multiply
         single = batch is not None and batch.is_decode  # such a step may be replayed from a graph: nothing comes to the host
-        if single or rows * top <= max(self.MOE_PAIR_ROWS * top, 2 * E):
+        by_expert = self._few_experts(x, w_gate_up, w_down, rows, top)
+        if by_expert and self._use_grouped(x, K, F, C, gated, activation):
+            few = rows * top < self._grouped_from(E, F, C, gated)
+        else:
+            few = single or rows * top <= max(self.MOE_PAIR_ROWS * top, 2 * E)
+        if few:
             pairs = torch.empty((rows * top, F), dtype=x.dtype, device=x.device)
-            if self._few_experts(x, w_gate_up, w_down, rows, top):
+            if by_expert:
                 # bfloat16: an expert's weights meet all its rows at once; the pairs' results are added up by their rows
                 self._ok(self.moe.krk_few_experts(pairs.data_ptr(), ptr, stride, w_gate_up.data_ptr(), experts.data_ptr(), rows, top,
                                                   E, F, K, int(not gated), act, _ptr(w_in), float(limit), float(slope),
@@ -969,6 +974,17 @@ class Kernels:
         54 and 50)."""
         return (x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and w_down.shape[2] % 8 == 0 and x.stride(0) % 8 == 0
                 and (x.data_ptr() | w_first.data_ptr() | w_down.data_ptr()) % 16 == 0 and top <= 32 and 6 <= rows * top <= 4096)
+
+    @staticmethod
+    def _grouped_from(E, F, C, gated) -> int:
+        """Pairs from which the two grouped launches, which need the pairs ordered and their rows gathered first, are faster than a
+        block per 32 rows of an expert's matrix. Those read an expert's weights once for sixteen of its rows, at 4.9 TB/s; the
+        grouped ones stream them at 6 where their tiles, of 128 or 256 columns, fill the 74 pairs of blocks some four times
+        (64 experts of 2,048 x 1,408, six a row, a single-token step: 16 rows 160 us and 157, 24 rows 197 and 186, 64 rows 216 and
+        190, 128 rows 252 and 192) and not where the second product is a round and a half (16 of 1,536 x 3,072, two a row: 16
+        rows 74 and 94, 64 rows 98 and 104, 128 rows 124 and 106)."""
+        tiles = E * min(-(-F // (128 if gated else 256)), -(-C // 256))
+        return 9 * E // 4 if tiles >= 296 else 12 * E
 
     @staticmethod
     def _use_grouped(x, K, F, C, gated, activation) -> bool:

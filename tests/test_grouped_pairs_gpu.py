@@ -48,3 +48,36 @@ def test_tiles_of_an_experts_rows_at_their_edges(N, K, counts, gated):
         # float32 sums of up to 640 products of order K^-1/2, and the next order of the roundings
         assert bool(((out.double().cpu() - want).abs() <= 1.02 * bound + 1e-4).all()), f"tall {tall}"
     ops.check()
+
+
+@pytest.mark.parametrize("E, top, F, C, line", [(64, 6, 640, 1280, 24), (8, 2, 96, 72, 48)])
+def test_experts_where_their_products_change_hands(E, top, F, C, line):
+    """Single-token steps and prompts of as many rows as move the experts' products from a block per piece of an expert to the grouped
+    launches, and one row fewer and more: the same sums, within the roundings of each expert's two products."""
+    from types import SimpleNamespace
+
+    from kernel_rush_kawk_b200.csrc import load_kernels
+
+    ops = load_kernels((), "cuda:0")
+    assert ops._grouped_from(E, F, C, True) == line * top
+    g = torch.Generator().manual_seed(2)
+    K = 64
+    w1 = (torch.randn(E, 2 * F, K, generator=g) * K ** -0.5).to(torch.bfloat16)
+    w2 = (torch.randn(E, C, F, generator=g) * F ** -0.5).to(torch.bfloat16)
+    for rows in (line - 1, line, line + 1):
+        x = torch.randn(rows, K, generator=g).to(torch.bfloat16)
+        experts = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(rows)]).int()
+        weights = torch.rand(rows, top, generator=g)
+        want = torch.zeros(rows, C, dtype=torch.float64)
+        for r in range(rows):
+            for j in range(top):
+                e = int(experts[r, j])
+                y = w1[e].double() @ x[r].double()
+                want[r] += weights[r, j].double() * (w2[e].double() @ (y[:F] * torch.sigmoid(y[:F]) * y[F:]))
+        for decode in (False, True):
+            got = ops.moe_experts(x.cuda(), w1.cuda(), w2.cuda(), experts.cuda(), weights.cuda(), F, "silu",
+                                  batch=SimpleNamespace(is_decode=decode))
+            off = (got.double().cpu() - want).norm() / want.norm()
+            # gate, up, their product, each expert's result and the sum are rounded: five times 2^-9 in the mean, added in squares
+            assert off < 5 ** 0.5 * 2.0 ** -8, (rows, decode, float(off))
+    ops.check()
