@@ -411,6 +411,32 @@ __global__ void moe_gather_kernel(T* __restrict__ xg, const T* __restrict__ x, i
   for (int k = threadIdx.x; k < K; k += blockDim.x) dst[k] = src[k];
 }
 
+// The same where a row is copied as it is, in 16-byte pieces: a block a row, which is read once for all the experts that it chose and whose
+// places are looked up at once. 2,048 rows of 2,048, six experts a row: 13.3 us a block a pair, 9.7 here.
+template <typename T>
+__global__ void __launch_bounds__(256)
+moe_gather_row_kernel(T* __restrict__ xg, const T* __restrict__ x, int x_stride, const int* __restrict__ place,
+                      const int* __restrict__ experts, const int* __restrict__ offsets, int cap, int top, int K,
+                      const float* __restrict__ in_weights, float* __restrict__ row_weights) {
+  __shared__ int at[32];
+  grid_dependency_wait();
+  const int row = blockIdx.x, n = K * (int)sizeof(T) / 16;
+  const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)row * x_stride);
+  uint4 piece = make_uint4(0u, 0u, 0u, 0u);
+  if (threadIdx.x < n) piece = src[threadIdx.x];
+  if (threadIdx.x < top) {
+    const int pair = row * top + threadIdx.x, to = row_of_pair(place, experts, offsets, cap, pair);
+    at[threadIdx.x] = to;
+    if (row_weights && to >= 0) row_weights[to] = in_weights[pair];
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < n; k += blockDim.x) {
+    for (int j = 0; j < top; ++j)
+      if (at[j] >= 0) reinterpret_cast<uint4*>(xg + (size_t)at[j] * K)[k] = piece;
+    if (k + blockDim.x < n) piece = src[k + blockDim.x];
+  }
+}
+
 template <typename T>
 __global__ void moe_combine_kernel(T* __restrict__ out, const T* __restrict__ add, const float* __restrict__ add_gate, const T* __restrict__ yg,
                                    const int* __restrict__ place, const int* __restrict__ experts,
@@ -428,7 +454,7 @@ __global__ void moe_combine_kernel(T* __restrict__ out, const T* __restrict__ ad
   if (sizeof(T) == 2 && (C & 7) == 0 && (x_stride & 7) == 0 &&
       ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(add) | reinterpret_cast<uintptr_t>(yg) |
         reinterpret_cast<uintptr_t>(x)) & 15) == 0) {
-    // eight columns a thread, four chosen experts' pieces in flight; the sum in the order of the choice
+    // eight columns a thread, eight chosen experts' pieces in flight; the sum in the order of the choice
     const float ag = add ? (add_gate ? add_gate[row] : 1.f) : 0.f, px = passed ? passed[row] : 0.f;
     auto fma8 = [](float (&t)[8], float w, const uint4& raw) {
       const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
@@ -439,13 +465,13 @@ __global__ void moe_combine_kernel(T* __restrict__ out, const T* __restrict__ ad
       float t[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       if (add) fma8(t, ag, *reinterpret_cast<const uint4*>(add + (size_t)row * C + c));
       if (passed) fma8(t, px, *reinterpret_cast<const uint4*>(x + (size_t)row * x_stride + c));
-      for (int j0 = 0; j0 < top; j0 += 4) {
-        uint4 raw[4];
+      for (int j0 = 0; j0 < top; j0 += 8) {
+        uint4 raw[8];
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int q = 0; q < 8; ++q)
           if (j0 + q < top && src_row[j0 + q] >= 0) raw[q] = *reinterpret_cast<const uint4*>(yg + (size_t)src_row[j0 + q] * C + c);
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int q = 0; q < 8; ++q)
           if (j0 + q < top && src_row[j0 + q] >= 0) fma8(t, src_w[j0 + q], raw[q]);
       }
       uint4 o;
@@ -557,6 +583,14 @@ KRK_API int krk_moe_gather(void* xg, const void* x, int x_stride, const int* pla
   if (rows == 0) return 0;
   if (row_weights && !in_weights) return -2;
   const int pairs = rows * top;
+  const size_t esz = dtype == KRK_DTYPE_F32 ? 4 : 2;
+  if (top <= 32 && !(in_weights && !row_weights) && (K * esz) % 16 == 0 && (x_stride * esz) % 16 == 0 && (((uintptr_t)x | (uintptr_t)xg) & 15) == 0) {
+    if (dtype == KRK_DTYPE_F32)
+      return (int)launch_pdl(moe_gather_row_kernel<float>, dim3(rows), dim3(256), 0, stream, (float*)xg, (const float*)x, x_stride, place, experts,
+                             offsets, cap, top, K, in_weights, row_weights);
+    return (int)launch_pdl(moe_gather_row_kernel<bf16>, dim3(rows), dim3(256), 0, stream, (bf16*)xg, (const bf16*)x, x_stride, place, experts, offsets,
+                           cap, top, K, in_weights, row_weights);
+  }
   if (dtype == KRK_DTYPE_F32)
     return (int)launch_pdl(moe_gather_kernel<float>, dim3(pairs), dim3(128), 0, stream, (float*)xg, (const float*)x,
                            x_stride, place, experts, offsets, cap, top, K, in_weights, row_weights);
