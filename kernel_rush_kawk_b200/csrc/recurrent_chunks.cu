@@ -2,8 +2,11 @@
 //
 // The scan of recurrent.cu takes a sequence's tokens one after the other: 0.57 us a token (delta rule) or 0.40 (time
 // mixing) whatever the batch, on as many SMs as there are heads and sequences. Here a chunk's tokens become small matrix
-// products, and all chunks but for one walk run side by side. The arithmetic is that of float32, as it is there: on the CUDA cores,
-// and in the products, where operands are three bfloat16 terms each, on the tensor cores; only the order of the sums differs. With the state S before the chunk, c_t the log decays summed from the chunk's first
+// products, and all chunks but for one walk run side by side. The state, the decays and all sums are float32, as they are there. Products
+// on the tensor cores take operands as three bfloat16 terms (24 bits), leave out those of two terms that are below 2^-24 of the
+// leading one's, and add all of a sum's small products before its leading ones, because the tensor cores cut every sum off: outputs that are
+// not the correctly rounded ones, of 1,033 tokens of 8 heads, 2.3e-4 with float32 multiply-adds on the CUDA cores, 1.4e-4 here
+// (3.5e-4 with the small products of a slice of k after the leading ones of the slice before). With the state S before the chunk, c_t the log decays summed from the chunk's first
 // token to t, and rows of the chunk's tokens:
 //
 //   time mixing:  o_t = (r_t e^{c_{t-1}}) . S + sum_{s<t} [sum_n r_tn k_sn e^{c_{t-1,n} - c_{s,n}}] v_s + (r_t . bonus k_t) v_t
@@ -582,24 +585,27 @@ __global__ void __launch_bounds__(THREADS, 8) mix_chunk_kernel(ChunkArgs a) {
   for (int n = 0; n < N / 8; ++n)
 #pragma unroll
     for (int c = 0; c < 4; ++c) g[n][c] = 0.f;
+  // the small terms of all tokens before the leading ones: the tensor cores cut every sum off
 #pragma unroll
-  for (int s = 0; s < L; s += 16) {
-    uint32_t af[3][4];
+  for (int leading = 0; leading < 2; ++leading)
 #pragma unroll
-    for (int t = 0; t < 3; ++t)  // the transpose of the keys' rows
-      ldmatrix_x4_trans(af[t][0], af[t][1], af[t][2], af[t][3],
-                        kt + (t * L + s + (lane & 7) + ((lane >> 4) & 1) * 8) * KP + m0 + ((lane >> 3) & 1) * 8);
+    for (int s = 0; s < L; s += 16) {
+      uint32_t af[2][4];
 #pragma unroll
-    for (int n = 0; n < N / 8; n += 2) {
-      uint32_t b[4];
-      ldmatrix_x4_trans(b[0], b[1], b[2], b[3], vs + (s + (lane & 7) + ((lane >> 3) & 1) * 8) * KP + (n + (lane >> 4)) * 8);
+      for (int t = 0; t < (leading ? 1 : 2); ++t)  // the transpose of the keys' rows
+        ldmatrix_x4_trans(af[t][0], af[t][1], af[t][2], af[t][3],
+                          kt + ((leading ? 0 : 2 - t) * L + s + (lane & 7) + ((lane >> 4) & 1) * 8) * KP + m0 + ((lane >> 3) & 1) * 8);
 #pragma unroll
-      for (int t = 2; t >= 0; --t) {
-        mma_bf16_16816(g[n], af[t][0], af[t][1], af[t][2], af[t][3], b[0], b[1]);
-        mma_bf16_16816(g[n + 1], af[t][0], af[t][1], af[t][2], af[t][3], b[2], b[3]);
+      for (int n = 0; n < N / 8; n += 2) {
+        uint32_t b[4];
+        ldmatrix_x4_trans(b[0], b[1], b[2], b[3], vs + (s + (lane & 7) + ((lane >> 3) & 1) * 8) * KP + (n + (lane >> 4)) * 8);
+#pragma unroll
+        for (int t = 0; t < (leading ? 1 : 2); ++t) {
+          mma_bf16_16816(g[n], af[t][0], af[t][1], af[t][2], af[t][3], b[0], b[1]);
+          mma_bf16_16816(g[n + 1], af[t][0], af[t][1], af[t][2], af[t][3], b[2], b[3]);
+        }
       }
     }
-  }
 #pragma unroll
   for (int n = 0; n < N / 8; ++n)
 #pragma unroll
@@ -910,21 +916,24 @@ __global__ void __launch_bounds__(THREADS, 5) mix_finish_kernel(ChunkArgs a) {
     for (int c = 0; c < 4; ++c) e[j][c] = 0.f;
   if (safe && warp < 3) {
 #pragma unroll
-    for (int kk = 0; kk < N; kk += 16) {
-      uint32_t af[3][4], b[3][4];
+    for (int leading = 0; leading < 2; ++leading)
 #pragma unroll
-      for (int t = 0; t < 3; ++t) {
-        ldmatrix_x4(af[t][0], af[t][1], af[t][2], af[t][3], qt + (t * L + mt * 16 + (lane & 15)) * KP + kk + (lane >> 4) * 8);
-        ldmatrix_x4(b[t][0], b[t][1], b[t][2], b[t][3], kt + (t * L + u0 + ((lane >> 4) << 3) + (lane & 7)) * KP + kk + ((lane >> 3) & 1) * 8);
-      }
+      for (int kk = 0; kk < N; kk += 16) {
+        uint32_t af[3][4], b0[3][2], b1[3][2];
 #pragma unroll
-      for (int sum = 2; sum >= 0; --sum)
-#pragma unroll
-        for (int t = 0; t <= sum; ++t) {
-          mma_bf16_16816(e[0], af[t][0], af[t][1], af[t][2], af[t][3], b[sum - t][0], b[sum - t][1]);
-          mma_bf16_16816(e[1], af[t][0], af[t][1], af[t][2], af[t][3], b[sum - t][2], b[sum - t][3]);
+        for (int t = 0; t < (leading ? 1 : 3); ++t) {
+          ldmatrix_x4(af[t][0], af[t][1], af[t][2], af[t][3], qt + (t * L + mt * 16 + (lane & 15)) * KP + kk + (lane >> 4) * 8);
+          ldmatrix_x4(b0[t][0], b0[t][1], b1[t][0], b1[t][1],
+                      kt + (t * L + u0 + ((lane >> 4) << 3) + (lane & 7)) * KP + kk + ((lane >> 3) & 1) * 8);
         }
-    }
+        if (leading) {
+          mma_bf16_16816(e[0], af[0][0], af[0][1], af[0][2], af[0][3], b0[0][0], b0[0][1]);
+          mma_bf16_16816(e[1], af[0][0], af[0][1], af[0][2], af[0][3], b1[0][0], b1[0][1]);
+        } else {
+          small33(e[0], af, b0);
+          small33(e[1], af, b1);
+        }
+      }
   }
   if (safe) {
     __syncthreads();  // the keys are no longer read
@@ -964,6 +973,7 @@ __global__ void __launch_bounds__(THREADS, 5) mix_finish_kernel(ChunkArgs a) {
     for (int j = 0; j < 2; ++j)
 #pragma unroll
       for (int c = 0; c < 4; ++c) o[m][j][c] = 0.f;
+  // q . S and the pair sums' products: the small terms of both before the leading ones of both
 #pragma unroll
   for (int kk = 0; kk < N / 16; ++kk) {
     uint32_t b[2][2][3];
@@ -978,7 +988,7 @@ __global__ void __launch_bounds__(THREADS, 5) mix_finish_kernel(ChunkArgs a) {
       for (int t = 0; t < 3; ++t)
         ldmatrix_x4(af[t][0], af[t][1], af[t][2], af[t][3], qt + (t * L + m * 16 + (lane & 15)) * KP + kk * 16 + (lane >> 4) * 8);
 #pragma unroll
-      for (int sum = 2; sum >= 0; --sum)
+      for (int sum = 2; sum >= 1; --sum)
 #pragma unroll
         for (int t = 0; t <= sum; ++t)
 #pragma unroll
@@ -987,20 +997,32 @@ __global__ void __launch_bounds__(THREADS, 5) mix_finish_kernel(ChunkArgs a) {
     }
   }
   __syncthreads();  // the pair sums are here
+  auto pairs = [&](int t) {  // a term of the pair sums against the values
 #pragma unroll
-  for (int kk = 0; kk < 2; ++kk) {
-    uint32_t b[4];
-    ldmatrix_x4_trans(b[0], b[1], b[2], b[3], vs + (kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * KP + warp * 16 + (lane >> 4) * 8);
+    for (int kk = 0; kk < 2; ++kk) {
+      uint32_t b[4];
+      ldmatrix_x4_trans(b[0], b[1], b[2], b[3], vs + (kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * KP + warp * 16 + (lane >> 4) * 8);
 #pragma unroll
-    for (int m = kk; m < 2; ++m)
-#pragma unroll
-      for (int t = 2; t >= 0; --t) {
+      for (int m = kk; m < 2; ++m) {
         uint32_t af[4];
         ldmatrix_x4(af[0], af[1], af[2], af[3], pt + (t * L + m * 16 + (lane & 15)) * PP + kk * 16 + (lane >> 4) * 8);
         mma_bf16_16816(o[m][0], af[0], af[1], af[2], af[3], b[0], b[1]);
         mma_bf16_16816(o[m][1], af[0], af[1], af[2], af[3], b[2], b[3]);
       }
-  }
+    }
+  };
+  pairs(2);
+  pairs(1);
+#pragma unroll
+  for (int kk = 0; kk < N / 16; ++kk)
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      uint32_t af[4];
+      ldmatrix_x4(af[0], af[1], af[2], af[3], qt + (m * 16 + (lane & 15)) * KP + kk * 16 + (lane >> 4) * 8);
+      mma_bf16_16816(o[m][0], af[0], af[1], af[2], af[3], pack_bf16x2(st[kk][0].x, st[kk][1].x), pack_bf16x2(st[kk][2].x, st[kk][3].x));
+      mma_bf16_16816(o[m][1], af[0], af[1], af[2], af[3], pack_bf16x2(st[kk][0].y, st[kk][1].y), pack_bf16x2(st[kk][2].y, st[kk][3].y));
+    }
+  pairs(0);
   // per head: divide by the root mean square, weight, gate, scale
   const int4 inf = *reinterpret_cast<const int4*>(bad + col), nan = *reinterpret_cast<const int4*>(bad + N + col);
   float4 y[4];

@@ -374,6 +374,23 @@ def test_scans_in_chunks(kind, lens, decays, monkeypatch):
     assert off["chunks"] < 2 * off["tokens"] + 1e-7, off
 
 
+@pytest.mark.parametrize("decays", ["mild", "spread"])
+@pytest.mark.parametrize("kind", ["delta", "wkv"])
+def test_chunks_sum_as_exactly_as_32_bit_multiply_adds(kind, decays, monkeypatch):
+    """Outputs next to the correctly rounded ones, of half a million: a sum that is 2^-24 off in a few places more shows there long before
+    it shows in a distance, which a bfloat16's own rounding fills. With float32 multiply-adds on the CUDA cores the same chunks leave up to
+    2.72e-4 of them; time mixing with its small products among the leading ones, which the tensor cores' sums then cut off, 3.65e-4."""
+    rt = runtime(torch.bfloat16)
+    monkeypatch.setattr(type(rt.ops), "_recurrence_in_chunks", lambda *_: True)
+    heads, lens = 8, [700, 333]
+    x = scan_inputs(kind, lens, heads, decays, 260)
+    start = rand((2, heads, 64, 64), 270).cuda()
+    want, _ = scan_in_64_bits(kind, x, lens, heads, start)
+    got = run_scan(rt, kind, x, lens, heads, start.clone()).cpu()
+    share = (got != want.to(torch.bfloat16)).double().mean().item()
+    assert share < 2.8e-4, share
+
+
 def turning_decays(case, heads):
     """Rows whose decays change within a chunk of 32 tokens, made by the one low-rank row: e^-e^z with z what ``lora`` says."""
     lens = [224, 97]
