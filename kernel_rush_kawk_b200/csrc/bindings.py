@@ -1511,10 +1511,12 @@ class Kernels:
 
     def _conv_walks(self, rows, row_bytes, n_seqs) -> bool:
         """Whether threads of the short convolution go through eight rows each, the rows before in registers. That is one chain of
-        5.3 us at least, at a sequence's first row with the loads of its stored rows in it, and pays by bytes: a block a row and
-        eight rows a thread, one prompt of 4,096 channels in bfloat16, 64 rows 5.0 and 5.6 us, 256 6.2 and 5.9, 512 8.2 and 7.1,
-        2,048 18.7 and 12.9 (the line is drawn above 1,024 rows of them); of 1,792 channels 512 rows 5.9 and 6.4, 1,024 7.9 and 6.9, 2,048 10.8 and 9.1; 32-bit of 4,096 channels
-        256 rows 6.9 and 7.3, 512 9.5 and 7.7. Single tokens of 64 sequences 9.9 and 12.9, of 2,048 equal."""
+        6 us at least, at a sequence's first row with the loads of its stored rows in it, and pays by bytes: a block a row and
+        eight rows a thread, one prompt of 4,096 channels in bfloat16, with the stored rows' update, 64 rows 5.1 and 6.2 us, 256 6.7
+        and 6.7, 512 8.5 and 7.6, 1,024 12.5 and 10.4, 2,048 22.3 and 15.7; of 1,792 channels 512 rows 6.4 and 7.0, 1,024 8.1 and
+        7.5, 2,048 11.6 and 10.2; 32-bit of 4,096 channels 256 rows 6.9 and 7.3, 512 9.5 and 7.8. So one long sequence's two kernels meet
+        between 2 and 5 MB; the line lies above, at 1,024 rows of 4,096 channels, for steps of many short sequences, whose
+        first rows each wait for their stored ones."""
         return rows * row_bytes >= self.CONV_WALK_BYTES and rows >= 2 * n_seqs
 
     def causal_conv_silu(self, x, w, b, tail, batch):

@@ -2,12 +2,12 @@
 //
 // The scan of recurrent.cu takes a sequence's tokens one after the other: 0.57 us a token (delta rule) or 0.40 (time
 // mixing) whatever the batch, on as many SMs as there are heads and sequences. Here a chunk's tokens become small matrix
-// products, and all chunks but for one walk run side by side. The state, the decays and all sums are float32, as they are there. Products
-// on the tensor cores take operands as three bfloat16 terms (24 bits), leave out those of two terms that are below 2^-24 of the
-// leading one's, and add all of a sum's small products before its leading ones, because the tensor cores cut every sum off: outputs that are
-// not the correctly rounded ones, of 1,033 tokens of 8 heads, 2.3e-4 with float32 multiply-adds on the CUDA cores, 1.4e-4 here
-// (3.5e-4 with the small products of a slice of k after the leading ones of the slice before). With the state S before the chunk, c_t the log decays summed from the chunk's first
-// token to t, and rows of the chunk's tokens:
+// products, and all chunks but for one walk run side by side. The state, the decays and all sums are float32, as they are there.
+// Products on the tensor cores take operands as three bfloat16 terms (24 bits), leave out those of two terms that are below
+// 2^-24 of the leading one's, and add all of a sum's small products before its leading ones, because the tensor cores cut every sum
+// off: outputs that are not the correctly rounded ones, of 1,033 tokens of 8 heads, 2.3e-4 with float32 multiply-adds on the CUDA
+// cores, 1.4e-4 here (3.5e-4 with the small products of a slice of k after the leading ones of the slice before). With the state S
+// before the chunk, c_t the log decays summed from the chunk's first token to t, and rows of the chunk's tokens:
 //
 //   time mixing:  o_t = (r_t e^{c_{t-1}}) . S + sum_{s<t} [sum_n r_tn k_sn e^{c_{t-1,n} - c_{s,n}}] v_s + (r_t . bonus k_t) v_t
 //                 S' = e^{c_last} S + sum_s (k_s e^{c_last - c_s}) v_s^T
@@ -1046,10 +1046,9 @@ __global__ void __launch_bounds__(THREADS, 5) mix_finish_kernel(ChunkArgs a) {
     const float sum = (red[t] + red[L + t]) + (red[2 * L + t] + red[3 * L + t]);
     const float by = rsqrtf(sum / (float)N + a.eps) * a.out_scale;
     const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&gate[i].x), hi = *reinterpret_cast<const __nv_bfloat162*>(&gate[i].y);
-    auto silu = [](float x) { return __fdividef(x, 1.0f + __expf(-x)); };
     uint2 raw;
-    raw.x = pack_bf16x2(y[i].x * by * w.x * silu(__low2float(lo)), y[i].y * by * w.y * silu(__high2float(lo)));
-    raw.y = pack_bf16x2(y[i].z * by * w.z * silu(__low2float(hi)), y[i].w * by * w.w * silu(__high2float(hi)));
+    raw.x = pack_bf16x2(y[i].x * by * w.x * silu_near(__low2float(lo)), y[i].y * by * w.y * silu_near(__high2float(lo)));
+    raw.y = pack_bf16x2(y[i].z * by * w.z * silu_near(__low2float(hi)), y[i].w * by * w.w * silu_near(__high2float(hi)));
     *reinterpret_cast<uint2*>(a.out + (row0 + t) * a.out_stride + a.out_col + ch0 + col) = raw;
   }
   if (a.last_rows && h == 0 && first + nt == qlen) {  // the sequence's last row, for the next step's token shift

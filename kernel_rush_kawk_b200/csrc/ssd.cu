@@ -30,9 +30,8 @@ constexpr int TOK = 16;       // tokens staged at a time
 constexpr int MAX_TAPS = 16;  // the convolution's taps
 
 __device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
-// where the result is rounded to T: bfloat16 takes the fast exponential and division, a few units in 2^23 off
-template <typename T> __device__ __forceinline__ float silu_to(float z) { return silu_f(z); }
-template <> __device__ __forceinline__ float silu_to<bf16>(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
+// the same number, rounded to T after
+template <typename T> __device__ __forceinline__ float silu_to(float z) { return sizeof(T) == 2 ? silu_near(z) : silu_f(z); }
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
 // V consecutive elements as floats, in one access of V * sizeof(T) bytes (the address is aligned to that)
@@ -86,7 +85,8 @@ __global__ void causal_conv_silu_kernel(T* __restrict__ out, const T* __restrict
 // The same for four taps and 16-byte pieces, CONV_ROWS rows a thread. Bound by bytes (a row in, a row out), which the kernel
 // above does not reach: it reads every row four times and the taps' weights, 20 bytes a channel, for every row. Here the
 // weights and the rows before stay in registers, and all of a thread's rows are asked for before the first is used: 2,048 rows of
-// 4,096 channels 18.7 us a row a block, 12.9 here (sixteen rows a thread, four asked for at a time: 18.1; twelve at once 17.8).
+// 4,096 channels, with the stored rows brought up to date, 22.3 us a block a row, 15.7 here (sixteen rows a thread, four asked for at a
+// time: 19.1).
 constexpr int CONV_ROWS = 8;
 
 template <typename T>

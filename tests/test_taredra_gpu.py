@@ -391,6 +391,22 @@ def test_chunks_sum_as_exactly_as_32_bit_multiply_adds(kind, decays, monkeypatch
     assert share < 2.8e-4, share
 
 
+@pytest.mark.parametrize("kind", ["delta", "wkv"])
+def test_gates_that_close(kind, monkeypatch):
+    """Gates down to where e^-g still is a number: an output of 1e-36 is as exact as any other, a bfloat16's rounding (2^-134 where those are
+    subnormal, and what 32-bit sums leave of an o that cancels)."""
+    rt = runtime(torch.bfloat16)
+    monkeypatch.setattr(type(rt.ops), "_recurrence_in_chunks", lambda *_: True)
+    lens, heads = [64], 2
+    x = scan_inputs(kind, lens, heads, "mild", 280)
+    x["g"] = -torch.linspace(20.0, 88.5, 64 * 128, device="cuda").view(64, 128).to(torch.bfloat16)
+    start = rand((1, heads, 64, 64), 281).cuda()
+    want, _ = scan_in_64_bits(kind, x, lens, heads, start)
+    got = run_scan(rt, kind, x, lens, heads, start.clone()).double().cpu()
+    gate = torch.sigmoid(x["g"].double().cpu())
+    assert ((got - want).abs() <= 1.01 * 2.0 ** -8 * want.abs() + 2.0 ** -134 + 1e-4 * gate).all()
+
+
 def turning_decays(case, heads):
     """Rows whose decays change within a chunk of 32 tokens, made by the one low-rank row: e^-e^z with z what ``lora`` says."""
     lens = [224, 97]

@@ -296,6 +296,27 @@ def test_gated_norm_of_many_parts(dtype, n):
     assert not out[:, :4].any() and not out[:, -4:].any()
 
 
+@pytest.mark.parametrize("walks", [True, False])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_silu_of_the_most_negative(dtype, walks, monkeypatch):
+    """Down to where e^-z still is a number: 1e-36 is as exact as any other result of the convolution and of the gated norm."""
+    rt = runtime(dtype)
+    monkeypatch.setattr(type(rt.ops), "_conv_walks", lambda *_: walks)
+    ch, rows = 1024, 24
+    z = -torch.linspace(20.0, 88.5, ch, device="cuda")
+    zero = lambda *s: torch.zeros(s, dtype=dtype, device="cuda")
+    got = rt.ops.causal_conv_silu(zero(rows, ch), zero(4, ch).float(), z, zero(1, 3, ch), context(rt, [0], [0], [rows], None).batch)
+    silu = lambda t: t.double() * torch.sigmoid(t.double())
+    unit = 1.01 * 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -21
+    assert ((got.double() - silu(z)).abs() <= unit * silu(z).abs()).all()
+    for rows in (24, 4096):  # a block a part, a warp a part
+        y, gates, out = torch.ones((rows, ch), device="cuda"), z.to(dtype).repeat(rows, 1), zero(rows, ch)
+        rt.ops.gated_group_norm(y, gates, torch.ones(ch, device="cuda"), 1, 1e-5, out, 0, 1.0)
+        v = silu(gates)
+        want = v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-5)
+        assert ((out.double() - want).abs() <= unit * want.abs()).all()
+
+
 def test_a_tokens_infinities_reach_no_earlier_token_of_a_state_space_chunk(monkeypatch):
     rt = runtime(torch.bfloat16)
     monkeypatch.setattr(type(rt.ops), "SSD_TENSOR_MIN", 1)
