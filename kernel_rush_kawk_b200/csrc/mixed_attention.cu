@@ -154,7 +154,7 @@ __global__ void norm_write_kernel(T* proj, int stride, int q_col, int k_col, int
   }
 }
 
-// The same for bfloat16 steps of many rows, heads of one size for keys and values: a block a row, 16 bytes a lane. A warp a head is
+// The same for bfloat16 steps of many rows, heads of one size up to 128 for keys and values: a block a row, 16 bytes a lane. A warp a head is
 // a chain of four dependent loads in front of 256 bytes; here a row's page is looked up once and its heads are asked for before.
 // 2,048 rows of 24 heads of 128: 15.7 us a warp a head, 11.1 here; 512 rows 5.4 and 4.2, 256 3.7 and 3.3, 128 2.7 and 3.1. Two rows a
 // block 10.7 and 4.7 (512 rows), four 14.2 and 6.7.
@@ -191,15 +191,27 @@ norm_write_row_kernel(bf16* proj, int stride, int q_col, int k_col, int v_col, i
     for (int u = 0; u < U; ++u) {
       const int h = h0 + u * groups;
       const bool query = h < HQ, value = h >= HQ + HKV;
-      float x[8], sq = 0.f;
+      float x[8];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const __nv_bfloat162 two = reinterpret_cast<const __nv_bfloat162*>(&raw[u])[j];
         x[2 * j] = __low2float(two);
         x[2 * j + 1] = __high2float(two);
-        sq += x[2 * j] * x[2 * j] + x[2 * j + 1] * x[2 * j + 1];
       }
-      for (int o = lph >> 1; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+      // squares in the order of the kernel above, where a lane has four elements and the lanes are added from the most distant pairs
+      // on: the same bits whichever kernel a step takes
+      auto squares = [&](int i) {
+        float s = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s = fmaf(x[i + j], x[i + j], s);
+        return s;
+      };
+      float lo = squares(0), hi = squares(4);
+      for (int o = lph >> 1; o > 0; o >>= 1) {
+        lo += __shfl_xor_sync(0xffffffffu, lo, o);
+        hi += __shfl_xor_sync(0xffffffffu, hi, o);
+      }
+      const float sq = lo + hi;
       if (h >= heads) continue;
       float f = normed && !value ? rsqrtf(sq / (float)D + eps) : 1.f;
       if (query) f *= temp;
@@ -680,7 +692,7 @@ KRK_API int krk_bias_norm_rotate_write(void* proj, int stride, int q_col, int k_
       return (int)launch_pdl(norm_write_kernel<float>, dim3((unsigned)blocks), dim3(warps * 32), 0, stream, (float*)proj,
                              stride, q_col, k_col, v_col, HQ, HKV, D, DV, gain, eps, unit, temp_coef, temp_every, row_seq,
                              row_pos, seq_slot, table, width, (float*)k_cache, (float*)v_cache, rows, keep_pages);
-    if (rows >= ROW_MIN && D == DV && D >= 8 && (D & (D - 1)) == 0 && stride % 8 == 0 && q_col % 8 == 0 && k_col % 8 == 0 && v_col % 8 == 0 &&
+    if (rows >= ROW_MIN && D == DV && D >= 8 && D <= 128 && (D & (D - 1)) == 0 && stride % 8 == 0 && q_col % 8 == 0 && k_col % 8 == 0 && v_col % 8 == 0 &&
         (((uintptr_t)proj | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0) {
       // as many groups of lanes as take all heads at once, up to 256 threads
       const int all = (D / 8 * ((HQ + 2 * HKV + ROW_HEADS - 1) / ROW_HEADS) + 31) / 32 * 32;
