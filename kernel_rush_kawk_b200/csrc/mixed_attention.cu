@@ -156,9 +156,10 @@ __global__ void norm_write_kernel(T* proj, int stride, int q_col, int k_col, int
 
 // The same for bfloat16 steps of many rows, heads of one size up to 128 for keys and values: a block a row, 16 bytes a lane. A warp a head is
 // a chain of four dependent loads in front of 256 bytes; here a row's page is looked up once and its heads are asked for before.
-// 2,048 rows of 24 heads of 128: 15.7 us a warp a head, 11.1 here; 512 rows 5.4 and 4.2, 256 3.7 and 3.3, 128 2.7 and 3.1. Two rows a
-// block 10.7 and 4.7 (512 rows), four 14.2 and 6.7.
-constexpr int ROW_MIN = 256, ROW_HEADS = 2;
+// That pays where the rows give every SM some blocks and the heads are many in all: a warp a head and a block a row, 24 heads of 128, 256 rows
+// 2.6 and 3.6 us, 384 3.6 and 3.8, 448 4.0 and 3.8, 2,048 13.8 and 7.9; 56 heads, 256 rows 5.0 and 5.6, 512 8.6 and 6.4; 11 heads of 64,
+// 768 rows 3.4 and 3.4, 1,024 4.1 and 3.8, 2,048 7.1 and 4.2; 10 heads, 1,024 rows 3.8 and 3.8. Heads of 256, 2,048 rows of 15: 9.3 and 9.4.
+constexpr int ROW_MIN = 448, ROW_ITEMS = 10000, ROW_HEADS = 2;
 
 __global__ void __launch_bounds__(256)
 norm_write_row_kernel(bf16* proj, int stride, int q_col, int k_col, int v_col, int HQ, int HKV, int D, const float* __restrict__ gain, float eps,
@@ -692,7 +693,7 @@ KRK_API int krk_bias_norm_rotate_write(void* proj, int stride, int q_col, int k_
       return (int)launch_pdl(norm_write_kernel<float>, dim3((unsigned)blocks), dim3(warps * 32), 0, stream, (float*)proj,
                              stride, q_col, k_col, v_col, HQ, HKV, D, DV, gain, eps, unit, temp_coef, temp_every, row_seq,
                              row_pos, seq_slot, table, width, (float*)k_cache, (float*)v_cache, rows, keep_pages);
-    if (rows >= ROW_MIN && D == DV && D >= 8 && D <= 128 && (D & (D - 1)) == 0 && stride % 8 == 0 && q_col % 8 == 0 && k_col % 8 == 0 && v_col % 8 == 0 &&
+    if (rows >= ROW_MIN && items >= ROW_ITEMS && D == DV && D >= 8 && D <= 128 && (D & (D - 1)) == 0 && stride % 8 == 0 && q_col % 8 == 0 && k_col % 8 == 0 && v_col % 8 == 0 &&
         (((uintptr_t)proj | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0) {
       // as many groups of lanes as take all heads at once, up to 256 threads
       const int all = (D / 8 * ((HQ + 2 * HKV + ROW_HEADS - 1) / ROW_HEADS) + 31) / 32 * 32;

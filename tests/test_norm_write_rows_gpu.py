@@ -1,5 +1,5 @@
-"""Head norms and cache writes of bfloat16 steps of many rows, which take a block a row: the same as the step one row shorter, which
-takes a warp a head, and within roundings of 64 bits; the same bits however a prompt was cut; more heads than lanes take at once, odd counts of them, one and many sequences."""
+"""Head norms and cache writes of bfloat16 steps of many rows, which take a block a row, and of fewer, which take a warp a head: within
+roundings of 64 bits; the same bits however a prompt was cut; more heads than lanes take at once, odd counts of them, one and many sequences."""
 
 import pytest
 import torch
