@@ -19,8 +19,8 @@
 //
 // A state-space mixer (ssd.cu) is a third kind: q and k are its C and B, one row of each for a group of heads, v its x, the decay
 // one number per head and token, and x_s counts dt_s times: A_ts = (C_t . B_s) e^{F_t - F_s} dt_s, r_t = e^{F_t}, w_s = e^{F_last - F_s} dt_s,
-// plus skip * x_t in the output. Its log decays are as large as the step sizes make them, so they are summed in 64-bit and kept as two
-// floats: e^{F_t - F_s} is then as exact as the product of the decays that the scan token by token forms. One prompt of 2,048
+// plus skip * x_t in the output. Its log decays are as large as the step sizes make them, so they are summed, kept and subtracted in
+// 64-bit: e^{F_t - F_s} is then as exact as the product of the decays that the scan token by token forms. One prompt of 2,048
 // tokens, 48 heads of 64 with 128 rows: the scan's three passes on the CUDA cores 403 us, these 90 (22, 16 and 50; 114 with a block
 // a head: 31, 16 and 66).
 //
@@ -42,6 +42,12 @@ constexpr float SAFE = 40.f;
 
 __device__ __forceinline__ float log_sigmoid_f(float z) { return fminf(z, 0.f) - log1pf(expf(-fabsf(z))); }
 
+// state-space kind: the log decays summed from the chunk's first token to this one, its step size, e^{F_last - F_s} dt
+struct __align__(16) Step {
+  double sum;
+  float dt, weight;
+};
+
 struct ChunkArgs {
   const bf16 *q, *k, *v;
   int q_stride, k_stride, v_stride;
@@ -55,7 +61,7 @@ struct ChunkArgs {
   float* cd;            // [n_seqs, max_chunks, H, N]: a chunk's decays
   int H, N, P, max_chunks;
   int slices;  // column slices a block walks
-  const float4* steps;  // state-space kind: [H, rows]: log decays summed within the chunk (two floats), dt, e^{F_last - F_s} dt
+  const Step* steps;    // state-space kind: [H, rows]
   int rows;
   const float* skip;    // state-space kind: [H]
   int per_group;        // heads that share a row of q and k
@@ -515,7 +521,7 @@ __global__ void __launch_bounds__(THREADS) chunk_output_kernel(ChunkArgs a) {
 // What a unit needs of the chunk's tokens: the raw values of a thread's two pieces of eight, the steps of token threadIdx.x
 struct UnitRows {
   uint4 v[2];
-  float4 step;
+  Step step;
   __device__ __forceinline__ void fetch(const ChunkArgs& a, size_t row0, int h, int p0, int nt) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -523,7 +529,8 @@ struct UnitRows {
       v[i] = s < nt && p0 + c < a.P ? *reinterpret_cast<const uint4*>(a.v + (row0 + s) * a.v_stride + (size_t)h * a.P + p0 + c)
                                     : make_uint4(0u, 0u, 0u, 0u);
     }
-    step = threadIdx.x < nt ? a.steps[(size_t)h * a.rows + row0 + threadIdx.x] : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (threadIdx.x < nt) step = a.steps[(size_t)h * a.rows + row0 + threadIdx.x];
+    else step = {0.0, 0.f, 0.f};
   }
 };
 static_assert(L * PB / 8 == 2 * THREADS && PB == 64, "two pieces a thread");
@@ -560,7 +567,7 @@ __global__ void __launch_bounds__(THREADS, 2) ssd_sum_kernel(ChunkArgs a) {
   for (; u < u1; ++u) {
     const int h = group * a.per_group + u / slices, p0 = u % slices * PB, b = u & 1;
     const UnitRows now = next;
-    if (threadIdx.x < L) ws[b][threadIdx.x] = now.step.w;
+    if (threadIdx.x < L) ws[b][threadIdx.x] = now.step.weight;
     __syncthreads();  // the weights are here, and the values of the unit before are no longer read
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -577,8 +584,7 @@ __global__ void __launch_bounds__(THREADS, 2) ssd_sum_kernel(ChunkArgs a) {
     const size_t at = ((size_t)seq * a.max_chunks + chunk) * H + h;
     float* cs = a.cs + at * ((size_t)N * P);
     if (p0 == 0) {
-      const float4 last = a.steps[(size_t)h * a.rows + row0 + nt - 1];
-      const float decay = expf(last.x + last.y);
+      const float decay = expf((float)a.steps[(size_t)h * a.rows + row0 + nt - 1].sum);
       for (int n = threadIdx.x; n < N; n += THREADS) a.cd[at * N + n] = decay;
     }
     for (int m0 = (warp & 3) * 32; m0 < N; m0 += 128) {
@@ -634,7 +640,7 @@ __global__ void __launch_bounds__(THREADS, 2) ssd_sum_kernel(ChunkArgs a) {
 // own share side by side.
 __global__ void __launch_bounds__(THREADS, 2) ssd_output_kernel(ChunkArgs a) {
   extern __shared__ __align__(16) bf16 sm[];
-  __shared__ float2 fs[L];     // the summed decays
+  __shared__ double fs[L];     // the summed decays
   __shared__ float dts[L];
   __shared__ int bad[2][PB];   // the first token that holds something infinite in a value column
   const int N = a.N, P = a.P, H = a.H, NP = N + 8;
@@ -723,24 +729,22 @@ __global__ void __launch_bounds__(THREADS, 2) ssd_output_kernel(ChunkArgs a) {
       *reinterpret_cast<uint4*>(vs + s * VPITCH + c) = next.v[i];
     }
     if (threadIdx.x < L) {
-      fs[threadIdx.x] = make_float2(next.step.x, next.step.y);
-      dts[threadIdx.x] = next.step.z;
+      fs[threadIdx.x] = next.step.sum;
+      dts[threadIdx.x] = next.step.dt;
     }
     __syncthreads();  // values and steps are here, and the keys (later A) are no longer read
     if (h != h_before && t0 < mt * 16 + 16) {
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
         const int t = mt * 16 + g + 8 * hh;
-        const float2 ft = fs[t];
+        const double ft = fs[t];
 #pragma unroll
         for (int n = 0; n < 4; ++n) {
           float v[2];
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             const int s = t0 + n * 8 + 2 * t4 + c;
-            const float2 f = fs[s];
-            // the difference of the two-float sums: its largest part is exact or rounded once
-            v[c] = s <= t && t < nt ? dots[(n * 4 + 2 * hh + c) * THREADS + threadIdx.x] * (expf((ft.x - f.x) + (ft.y - f.y)) * dts[s]) : 0.f;
+            v[c] = s <= t && t < nt ? dots[(n * 4 + 2 * hh + c) * THREADS + threadIdx.x] * (expf((float)(ft - fs[s])) * dts[s]) : 0.f;
           }
           uint32_t p[3];
           split3_pair(v[0], v[1], p);
@@ -781,8 +785,7 @@ __global__ void __launch_bounds__(THREADS, 2) ssd_output_kernel(ChunkArgs a) {
     for (int m = 0; m < 4; ++m)
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
-        const float2 f = fs[m * 16 + g + 8 * hh];
-        const float e = expf(f.x + f.y);
+        const float e = expf((float)fs[m * 16 + g + 8 * hh]);
         acc[m][2 * hh] *= e;
         acc[m][2 * hh + 1] *= e;
       }
@@ -862,10 +865,9 @@ __global__ void chunk_decays_kernel(float* __restrict__ cum, const bf16* __restr
 
 // state-space kind: dt = softplus(raw + bias), log decay -exp(A_log) dt. Not below FORGOTTEN, whose e^ is zero in 32 bits: sums of
 // minus infinity have no difference, and even 64 bits would lose a later token's decay beside a number that is large enough. The
-// decays are summed over a chunk's tokens in 64 bits and left as two floats, whose differences are as exact. A warp a chunk and head,
-// a lane two neighbouring tokens.
+// decays are summed over a chunk's tokens in 64 bits. A warp a chunk and head, a lane two neighbouring tokens.
 constexpr float FORGOTTEN = -120.f;
-__global__ void __launch_bounds__(256) steps_kernel(float4* __restrict__ steps, const bf16* __restrict__ dt, int dt_stride,
+__global__ void __launch_bounds__(256) steps_kernel(Step* __restrict__ steps, const bf16* __restrict__ dt, int dt_stride,
                                                     const float* __restrict__ bias, const float* __restrict__ a_log, int rows, int H,
                                                     const int* __restrict__ cu_q, const int* __restrict__ seq_qlen) {
   grid_launch_dependents();
@@ -899,8 +901,7 @@ __global__ void __launch_bounds__(256) steps_kernel(float4* __restrict__ steps, 
   for (int j = 0; j < 2; ++j) {
     const int t = 2 * lane + j;
     if (t >= nt) continue;
-    const float hi = (float)sums[j];
-    steps[(size_t)h * rows + row0 + t] = make_float4(hi, (float)(sums[j] - hi), d[j], expf((float)(last - sums[j])) * d[j]);
+    steps[(size_t)h * rows + row0 + t] = {sums[j], d[j], expf((float)(last - sums[j])) * d[j]};
   }
 }
 
@@ -1007,13 +1008,13 @@ KRK_API int krk_memory_chunks(float* y, float* den, const void* q, int q_stride,
   return gates ? launch_chunks<RUNNING_MAX>(a, n_seqs, stream) : launch_chunks<DECAYS>(a, n_seqs, stream);
 }
 
-// Step sizes and summed log decays [H, rows] of a state-space mixer's rows (bfloat16), four floats each, for krk_ssd_chunks.
+// Step sizes and summed log decays [H, rows] of a state-space mixer's rows (bfloat16), a Step of 16 bytes each, for krk_ssd_chunks.
 KRK_API int krk_ssd_steps(float* steps, const void* dt, int dt_stride, const float* dt_bias, const float* a_log, int rows, int H,
                           int n_seqs, int max_q_len, const int* cu_q, const int* seq_qlen, cudaStream_t stream) {
   if (rows == 0 || n_seqs == 0 || max_q_len == 0) return 0;
   const int chunks = (max_q_len + L - 1) / L;
   if (chunks > 65535 || n_seqs > 65535 || ((uintptr_t)steps & 15)) return -2;
-  return (int)launch_pdl(steps_kernel, dim3((unsigned)((H + 7) / 8), (unsigned)chunks, (unsigned)n_seqs), dim3(256), 0, stream, (float4*)steps,
+  return (int)launch_pdl(steps_kernel, dim3((unsigned)((H + 7) / 8), (unsigned)chunks, (unsigned)n_seqs), dim3(256), 0, stream, (Step*)steps,
                          (const bf16*)dt, dt_stride, dt_bias, a_log, rows, H, cu_q, seq_qlen);
 }
 
@@ -1033,6 +1034,6 @@ KRK_API int krk_ssd_chunks(float* y, const void* x, int x_stride, const void* B,
   a.v_stride = x_stride; a.q_scale = 1.f; a.cum = nullptr; a.gates = nullptr; a.state = state; a.nm = nullptr; a.y = y; a.den = nullptr;
   a.cs = cs; a.cd = cd; a.H = H; a.N = N; a.P = P; a.max_chunks = n_chunks; a.slices = 1;
   a.cu_q = cu_q; a.seq_qlen = seq_qlen; a.seq_slot = seq_slot;
-  a.steps = (const float4*)steps; a.rows = rows; a.skip = skip; a.per_group = H / G; a.chunk0 = chunk0;
+  a.steps = (const Step*)steps; a.rows = rows; a.skip = skip; a.per_group = H / G; a.chunk0 = chunk0;
   return launch_ssd(a, n_seqs, stream);
 }

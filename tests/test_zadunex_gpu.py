@@ -223,6 +223,31 @@ def test_state_space_scans_on_the_tensor_cores(shape, lens, rate, monkeypatch):
     assert all(c <= 2 * t + 2e-7 for c, t in zip(off["chunks"], off["tokens"])), off
 
 
+def test_a_state_space_token_after_its_decay(monkeypatch):
+    """One token in front of a chunk, alone: what is left of it later in the chunk is e^d times it, d the difference of two sums of 64
+    bits rounded once, so off by a rounding of d: a unit of its last place over the root of 12. A difference rounded twice would be off by
+    the root of 2 more. Beside it e^ and the products are rounded to 2^-24 each: of d between 16 and 32 a twentieth."""
+    rt = runtime(torch.bfloat16)
+    monkeypatch.setattr(type(rt.ops), "SSD_TENSOR_MIN", 1)
+    H, P, N, rows = 64, 16, 16, 64
+    x, B, C = torch.zeros((rows, H * P)), torch.zeros((rows, N)), torch.zeros((rows, N))
+    x[3], B[3, 0], C[:, 0] = 1.0, 1.0, 1.0
+    x, B, C = (t.to(torch.bfloat16).cuda() for t in (x, B, C))
+    dt = rand((rows, H), 71, 0.3).to(torch.bfloat16).cuda()
+    bias, a_log, skip = rand((H,), 72).cuda(), torch.zeros(H, device="cuda"), torch.zeros(H, device="cuda")
+    state = torch.zeros((1, H, N, P), device="cuda")
+    ctx = context(rt, [0], [0], [rows], None)
+    y = rt.ops.ssd_scan(x, B, C, dt, bias, a_log, skip, H, P, N, 1, state, ctx.batch).view(rows, H, P)[:, :, 0].double()
+    d = torch.nn.functional.softplus(dt.float() + bias)  # the step sizes and log decays are numbers of 32 bits
+    f = -(torch.exp(a_log) * d).double().cumsum(0)
+    want = torch.exp(f - f[3]) * d[3].double()
+    seen = (f - f[3] < -16) & (f - f[3] > -32)
+    assert seen.sum() > 900
+    off = ((y - want) / want)[seen].pow(2).mean().sqrt().item()
+    # the kernel's own softplus may differ from torch's by a unit or two of 2^-24, which moves d by as much again
+    assert off < 1.2 * 2.0 ** -19 / 12 ** 0.5, off
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_convolution_of_many_rows(dtype, monkeypatch):
     """Rows in runs of sixteen a thread, four taps: sequences that start anywhere in a run, shorter than the taps, channels
