@@ -111,7 +111,7 @@ _MEMORY_SIGNATURES = {
                           _P, _P, _P, _P],
     "krk_ssd_steps": [_P, _P, c_int, _P, _P, c_int, c_int, c_int, c_int, _P, _P, _P],
     "krk_ssd_chunks": [_P, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                       _P, _P, _P, _P],
+                       c_int, _P, _P, _P, _P],
     "krk_memory_finish": [_P, c_int, c_int, c_float, _P, _P, _P, _P, c_int, _P, c_int, c_int, c_float, c_int, c_int, _P],
 }
 _LATENT_SIGNATURES = {
@@ -1595,9 +1595,11 @@ class Kernels:
                                              batch.max_q_len, batch.cu_q.data_ptr(), batch.seq_qlen.data_ptr(), self._stream()),
                  "step sizes and decays")
         for first in range(0, chunks, portion):
+            count = min(portion, chunks - first)
+            live = sum(min(max(-(-n // tokens) - first, 0), count) for n in batch.q_lens)
             self._ok(self.memory.krk_ssd_chunks(y.data_ptr(), xp, xs, bp, bs, cp, cs_, steps, rows, skip.data_ptr(),
                                                 state.data_ptr(), sums, decays, heads, P, N, groups,
-                                                batch.n_seqs, first, min(portion, chunks - first), batch.cu_q.data_ptr(),
+                                                batch.n_seqs, first, count, live, batch.cu_q.data_ptr(),
                                                 batch.seq_qlen.data_ptr(), batch.seq_slot.data_ptr(), self._stream()),
                      "state-space scan in chunks")
             self.launches += 2

@@ -223,6 +223,46 @@ def test_state_space_scans_on_the_tensor_cores(shape, lens, rate, monkeypatch):
     assert all(c <= 2 * t + 2e-7 for c, t in zip(off["chunks"], off["tokens"])), off
 
 
+@pytest.mark.parametrize("shape, lens", [
+    ((48, 64, 128, 4), [450]),            # more blocks than the SMs hold two of, not more than three
+    ((48, 64, 128, 4), [600, 400, 300]),  # several heads a block, sequences that end before others
+    ((24, 80, 32, 2), [1100]),            # a head's second slice of columns in the block of the first
+    ((40, 64, 272, 2), [700]),            # more rows of the state than are fetched at a time
+])
+def test_state_space_scans_of_many_heads(shape, lens, monkeypatch):
+    """Enough heads and chunks that a block takes several units of a group's chunk one after the other, or that three share an SM: from 64
+    bits no further than twice the scan token by token, portions the same bits, and an infinite value of one head reaches no earlier
+    token, no other column and no other head."""
+    rt = runtime(torch.bfloat16)
+    H, P, N, G = shape
+    rows = sum(lens)
+    x, B, C = (rand((rows, n), 61 + i).to(torch.bfloat16).cuda() for i, n in enumerate((H * P, G * N, G * N)))
+    dt, bias = rand((rows, H), 64).to(torch.bfloat16).cuda(), rand((H,), 65).cuda() - 2
+    a_log, skip = rand((H,), 66, 0.5).cuda(), rand((H,), 67).cuda()
+    start = rand((len(lens), H, N, P), 68).cuda()
+    ctx = context(rt, list(range(len(lens))), [0] * len(lens), lens, None)
+
+    def scan(x, least, scratch=1 << 28):
+        monkeypatch.setattr(type(rt.ops), "SSD_TENSOR_MIN", least)
+        monkeypatch.setattr(type(rt.ops), "SSD_SCRATCH", scratch)
+        state = start.clone()
+        return rt.ops.ssd_scan(x, B, C, dt, bias, a_log, skip, H, P, N, G, state, ctx.batch), state
+
+    want = ssd_in_64_bits(x, B, C, dt, bias, a_log, skip, G, lens, start)
+    tokens, chunks, portions = scan(x, 1 << 30), scan(x, 1), scan(x, 1, 12 * start.numel())  # three chunks at a time
+    assert all(torch.equal(a, b) for a, b in zip(chunks, portions))
+    off = lambda got: [((a.double() - b).norm() / b.norm()).item() for a, b in zip(got, want)]
+    assert all(c <= 2 * t + 2e-7 for c, t in zip(off(chunks), off(tokens))), (off(chunks), off(tokens))
+    at, col = 250, 3 * P + 5  # the fourth head
+    x[at, col] = float("-inf")
+    y, state = scan(x, 1)
+    rest = [c for c in range(H * P) if c != col]
+    assert torch.equal(y[:at], chunks[0][:at]) and torch.equal(y[:, rest], chunks[0][:, rest]) and not torch.isfinite(y[at:lens[0], col]).any()
+    clean = torch.ones_like(start, dtype=torch.bool)
+    clean[0, 3, :, 5] = False
+    assert torch.equal(state[clean], chunks[1][clean]) and not torch.isfinite(state[~clean]).any()
+
+
 def test_a_state_space_token_after_its_decay(monkeypatch):
     """One token in front of a chunk, alone: what is left of it later in the chunk is e^d times it, d the difference of two sums of 64
     bits rounded once, so off by a rounding of d: a unit of its last place over the root of 12. A difference rounded twice would be off by
