@@ -515,8 +515,10 @@ __global__ void __launch_bounds__(THREADS) chunk_output_kernel(ChunkArgs a) {
 
 // ---- state-space kind ----------------------------------------------------------------------------------------
 // A group's heads share the rows of q and k, so a block takes several (head, column slice) units of a group's chunk: what depends on
-// q and k alone is done once, and a unit's values, step sizes and state are on their way while the unit before is multiplied. Two blocks
-// an SM: three leave the outputs 80 registers, which spill (69 us against 58, profiled; a block a head 66).
+// q and k alone is done once, and a unit's values, step sizes and state are on their way while the unit before is multiplied (MANY). Two
+// blocks an SM: three leave the outputs 80 registers, which spill (69 us against 58, profiled; a block a head 66). Where the units
+// are more than two blocks an SM hold and not more than three, a block takes one of them, with no next unit's registers: 450 tokens
+// of 48 heads 39.6 us with two units a block, 35.2 here.
 
 // What a unit needs of the chunk's tokens: the raw values of a thread's two pieces of eight, the steps of token threadIdx.x
 struct UnitRows {
@@ -538,7 +540,8 @@ static_assert(L * PB / 8 == 2 * THREADS && PB == 64, "two pieces a thread");
 // The chunk's own sum_s k_s (w_s v_s)^T: where a token's weight is one number it multiplies the values instead of the keys: they are
 // fewer, and the keys stay exact. Warps 4 x 2: 32 key rows and 32 columns each, so that a fragment of the values' terms, which
 // bound the kernel (every warp reads them from shared memory), serves two products; the keys' fragments stay in registers.
-__global__ void __launch_bounds__(THREADS, 2) ssd_sum_kernel(ChunkArgs a) {
+template <bool MANY>
+__global__ void __launch_bounds__(THREADS, MANY ? 2 : 3) ssd_sum_kernel(ChunkArgs a) {
   extern __shared__ __align__(16) bf16 sm[];
   __shared__ float ws[2][L];
   const int N = a.N, P = a.P, H = a.H, NP = N + 8;
@@ -551,8 +554,8 @@ __global__ void __launch_bounds__(THREADS, 2) ssd_sum_kernel(ChunkArgs a) {
   const int first = (a.chunk0 + chunk) * L, nt = min(L, a.seq_qlen[seq] - first);
   if (nt <= 0) return;
   const size_t row0 = (size_t)a.cu_q[seq] + first;
-  const int slices = (P + PB - 1) / PB, all = a.per_group * slices, u1 = min(all, (part + 1) * a.units);
-  int u = part * a.units;
+  const int slices = (P + PB - 1) / PB, u1 = MANY ? min(a.per_group * slices, (part + 1) * a.units) : part + 1;
+  int u = MANY ? part * a.units : part;
   UnitRows next;
   next.fetch(a, row0, group * a.per_group + u / slices, u % slices * PB, nt);
   for (int s = warp; s < L; s += THREADS / 32)
@@ -579,7 +582,7 @@ __global__ void __launch_bounds__(THREADS, 2) ssd_sum_kernel(ChunkArgs a) {
       for (int j = 0; j < 4; ++j) { f[2 * j] = w * __low2float(h2[j]); f[2 * j + 1] = w * __high2float(h2[j]); }
       split3_store8(f, vs + s * VPITCH + c, (size_t)L * VPITCH);
     }
-    if (u + 1 < u1) next.fetch(a, row0, group * a.per_group + (u + 1) / slices, (u + 1) % slices * PB, nt);
+    if (MANY && u + 1 < u1) next.fetch(a, row0, group * a.per_group + (u + 1) / slices, (u + 1) % slices * PB, nt);
     __syncthreads();
     const size_t at = ((size_t)seq * a.max_chunks + chunk) * H + h;
     float* cs = a.cs + at * ((size_t)N * P);
@@ -637,8 +640,9 @@ __global__ void __launch_bounds__(THREADS, 2) ssd_sum_kernel(ChunkArgs a) {
 
 // The outputs. A warp takes all 64 tokens of eight value columns, whose part of the state is then its own fragment of the product:
 // it never passes through shared memory. C_t . B_s of the chunk, the same for a group's heads, waits in shared memory, each thread's
-// own share side by side.
-__global__ void __launch_bounds__(THREADS, 2) ssd_output_kernel(ChunkArgs a) {
+// own share side by side (or in registers, for one unit).
+template <bool MANY>
+__global__ void __launch_bounds__(THREADS, MANY ? 2 : 3) ssd_output_kernel(ChunkArgs a) {
   extern __shared__ __align__(16) bf16 sm[];
   __shared__ double fs[L];     // the summed decays
   __shared__ float dts[L];
@@ -656,8 +660,8 @@ __global__ void __launch_bounds__(THREADS, 2) ssd_output_kernel(ChunkArgs a) {
   const int first = (a.chunk0 + chunk) * L, nt = min(L, a.seq_qlen[seq] - first);
   if (nt <= 0) return;
   const size_t row0 = (size_t)a.cu_q[seq] + first;
-  const int slices = (P + PB - 1) / PB, all = a.per_group * slices, u1 = min(all, (part + 1) * a.units);
-  int u = part * a.units;
+  const int slices = (P + PB - 1) / PB, u1 = MANY ? min(a.per_group * slices, (part + 1) * a.units) : part + 1;
+  int u = MANY ? part * a.units : part;
   const float* starts = a.cs + ((size_t)seq * a.max_chunks + chunk) * H * N * P;
   constexpr int KB = 8;  // 128 rows of the state at a time
   float own[KB][4];
@@ -689,8 +693,9 @@ __global__ void __launch_bounds__(THREADS, 2) ssd_output_kernel(ChunkArgs a) {
   __syncthreads();
   // A: the warp's 16 tokens against 32 of the chunk's; two warps have later tokens alone, whose tiles are not read
   const int mt = warp & 3, t0 = (warp >> 2) * 32;
+  float own_dots[4][4];
   if (t0 < mt * 16 + 16) {
-    float s[4][4];
+    auto& s = own_dots;
 #pragma unroll
     for (int n = 0; n < 4; ++n)
 #pragma unroll
@@ -706,10 +711,11 @@ __global__ void __launch_bounds__(THREADS, 2) ssd_output_kernel(ChunkArgs a) {
         mma_bf16_16816(s[n + 1], af[0], af[1], af[2], af[3], b[2], b[3]);
       }
     }
+    if (MANY)
 #pragma unroll
-    for (int n = 0; n < 4; ++n)
+      for (int n = 0; n < 4; ++n)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) dots[(n * 4 + c) * THREADS + threadIdx.x] = s[n][c];
+        for (int c = 0; c < 4; ++c) dots[(n * 4 + c) * THREADS + threadIdx.x] = s[n][c];
   }
   for (int h_before = -1; u < u1; ++u) {
     const int h = group * a.per_group + u / slices;
@@ -744,7 +750,8 @@ __global__ void __launch_bounds__(THREADS, 2) ssd_output_kernel(ChunkArgs a) {
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             const int s = t0 + n * 8 + 2 * t4 + c;
-            v[c] = s <= t && t < nt ? dots[(n * 4 + 2 * hh + c) * THREADS + threadIdx.x] * (expf((float)(ft - fs[s])) * dts[s]) : 0.f;
+            const float dot = MANY ? dots[(n * 4 + 2 * hh + c) * THREADS + threadIdx.x] : own_dots[n][2 * hh + c];
+            v[c] = s <= t && t < nt ? dot * (expf((float)(ft - fs[s])) * dts[s]) : 0.f;
           }
           uint32_t p[3];
           split3_pair(v[0], v[1], p);
@@ -777,7 +784,7 @@ __global__ void __launch_bounds__(THREADS, 2) ssd_output_kernel(ChunkArgs a) {
         }
       }
     }
-    if (u + 1 < u1) {
+    if (MANY && u + 1 < u1) {
       next.fetch(a, row0, group * a.per_group + (u + 1) / slices, (u + 1) % slices * PB, nt);
       fetch(u + 1, 0);
     }
@@ -945,30 +952,41 @@ int launch_chunks(ChunkArgs a, int n_seqs, cudaStream_t stream) {
 int launch_ssd(ChunkArgs a, int n_seqs, int live, cudaStream_t stream) {
   const size_t s1 = ssd_sum_smem(a.N), s3 = ssd_output_smem(a.N);
   if (a.max_chunks > 65535 || n_seqs > 65535) return -2;
-  cudaFuncSetAttribute(ssd_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1);
-  cudaFuncSetAttribute(ssd_output_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3);
+  auto room = [](auto kernel, size_t bytes) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); };
+  room(ssd_sum_kernel<true>, s1);
+  room(ssd_sum_kernel<false>, s1);
+  room(ssd_output_kernel<true>, s3);
+  room(ssd_output_kernel<false>, s3);
   const int groups = a.H / a.per_group, all = a.per_group * ((a.P + PB - 1) / PB);
   // units a block: the fewest rounds of units over the SMs, a block's start counted as a part of one. Blocks of chunks that a shorter
-  // sequence does not have leave at once and are not counted (48 heads, sequences of 600, 400 and 300 tokens: 93 us counted, 71)
-  auto split = [&](int an_sm, float start) {
+  // sequence does not have leave at once and are not counted (48 heads, sequences of 600, 400 and 300 tokens: 93 us counted, 71).
+  // Three blocks an SM of one unit each take 1.4 times as long as two (48 heads, 330 tokens: 33.5 us and 28).
+  // The starts, 0.5 for the sums and 0.7 for the outputs, choose the fastest or within 1 % of it of 1, 2, 3, 4 and 6 units for one prompt of
+  // 192 to 3,000 tokens of 48 heads in four groups (2,048 tokens, the outputs by 1, 2, 3, 4, 6, 8 and 12: 112, 103, 100, 103, 97, 113 and 142 us).
+  // Returns whether it is the form of many.
+  auto split = [&](float start) {
     float best = 1e30f;
-    for (int units = 1; units <= all; ++units) {
-      const long long blocks = (long long)((all + units - 1) / units) * groups * live;
-      const float cost = (float)((blocks + 148 * an_sm - 1) / (148 * an_sm)) * (units + start);
+    bool many = true;
+    for (int units = 0; units <= all; ++units) {  // 0: three blocks an SM, one unit each
+      const int each = units ? units : 1;
+      const long long blocks = (long long)((all + each - 1) / each) * groups * live, at_once = units ? 296 : 444;
+      const float cost = (float)((blocks + at_once - 1) / at_once) * (each + start) * (units ? 1.f : 1.4f);
       if (cost < best) {
         best = cost;
-        a.units = units;
+        a.units = each;
+        many = units > 0;
       }
     }
     a.parts = (all + a.units - 1) / a.units;
-    return dim3((unsigned)(a.parts * groups), (unsigned)a.max_chunks, (unsigned)n_seqs);
+    return many;
   };
-  dim3 grid = split(2, 0.5f);
-  int rc = (int)launch_pdl(ssd_sum_kernel, grid, dim3(THREADS), s1, stream, a);
+  auto grid = [&] { return dim3((unsigned)(a.parts * groups), (unsigned)a.max_chunks, (unsigned)n_seqs); };
+  const bool many_sums = split(0.5f);
+  int rc = (int)launch_pdl(many_sums ? ssd_sum_kernel<true> : ssd_sum_kernel<false>, grid(), dim3(THREADS), s1, stream, a);
   if (rc) return rc;
   if ((rc = launch_walk(a, false, n_seqs, stream))) return rc;
-  grid = split(2, 0.7f);
-  return (int)launch_pdl(ssd_output_kernel, grid, dim3(THREADS), s3, stream, a);
+  const bool many = split(0.7f);
+  return (int)launch_pdl(many ? ssd_output_kernel<true> : ssd_output_kernel<false>, grid(), dim3(THREADS), s3, stream, a);
 }
 
 }  // namespace
