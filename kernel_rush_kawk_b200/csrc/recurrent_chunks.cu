@@ -182,7 +182,8 @@ __global__ void __launch_bounds__(DELTA_THREADS, 2) delta_chunk_kernel(ChunkArgs
   float* last = es + L * PITCH;                        // [N] e^{c_last}
   float* sq = last + N;                                // [2][L] |k|^2, of either half of the channels
   float2* total = reinterpret_cast<float2*>(sq + 2 * L);  // [4][N] a part's decays, summed, and what that rounded off
-  int* bad = reinterpret_cast<int*>(total + 4 * N);    // [3][N]: the first token that is not finite in a column of X, of Z, of the values
+  int* bad = reinterpret_cast<int*>(total + 4 * N);    // [4][N]: the first token that is not finite in a column of X, of Z; with an
+                                                       // infinity in a column of the values, with a NaN
   float* th_s = us;                                    // [L][R rounded up], over us and es; gone before they are written
   const int h = blockIdx.x, ci = blockIdx.y, seq = blockIdx.z, ch0 = h * N;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
@@ -200,7 +201,7 @@ __global__ void __launch_bounds__(DELTA_THREADS, 2) delta_chunk_kernel(ChunkArgs
     k[i] = in ? __bfloat162float(a.k[row * a.k_stride + ch0 + ch]) : 0.f;
     rate[i] = in ? __bfloat162float(a.rate[row * a.rate_stride + ch0 + ch]) : 0.f;
   }
-  if (tid < 3 * N) bad[tid] = L;
+  if (tid < 4 * N) bad[tid] = L;
   load_tanh(a, th_s, row0, nt);
   __syncthreads();
   for (int i = tid; i < L * (N / 4); i += DELTA_THREADS) {  // the values
@@ -210,8 +211,8 @@ __global__ void __launch_bounds__(DELTA_THREADS, 2) delta_chunk_kernel(ChunkArgs
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const bool lo = (two[j] & 0x7f80u) == 0x7f80u, hi = (two[j] & 0x7f800000u) == 0x7f800000u;
-      if (lo) atomicMin(bad + 2 * N + c + 2 * j, t);
-      if (hi) atomicMin(bad + 2 * N + c + 2 * j + 1, t);
+      if (lo) atomicMin(bad + (two[j] & 0x7fu ? 3 * N : 2 * N) + c + 2 * j, t);
+      if (hi) atomicMin(bad + (two[j] & 0x7f0000u ? 3 * N : 2 * N) + c + 2 * j + 1, t);
       if (lo || hi) two[j] &= (lo ? 0xffff0000u : 0xffffffffu) & (hi ? 0xffffu : 0xffffffffu);
     }
     *reinterpret_cast<uint2*>(vs + t * KP + c) = make_uint2(two[0], two[1]);
@@ -454,7 +455,7 @@ __global__ void __launch_bounds__(DELTA_THREADS, 2) delta_chunk_kernel(ChunkArgs
         for (int j = 0; j < 2; ++j) {
           v[j] = d[n][2 * hh + j];
           if (!is_g && row == col + j) v[j] += 1.f;
-          v[j] = worst[col + j] < L || (is_g && bad[2 * N + col + j] < L) ? NAN : w * v[j];
+          v[j] = worst[col + j] < L || (is_g && min(bad[2 * N + col + j], bad[3 * N + col + j]) < L) ? NAN : w * v[j];
         }
         *reinterpret_cast<float2*>(item + (is_g ? N * N : 0) + row * N + col) = make_float2(v[0], v[1]);
       }
@@ -516,7 +517,7 @@ __global__ void __launch_bounds__(DELTA_THREADS, 2) delta_chunk_kernel(ChunkArgs
           const bf16* from = rt + t * KP + col + j;
           const float row = __bfloat162float(from[0]) + (__bfloat162float(from[TERM]) + __bfloat162float(from[2 * TERM]));  // r e^c again
           v[j] = t >= bad[col + j] ? NAN : row + q[m][2 * hh + j];
-          w[j] = t >= bad[N + col + j] ? NAN : t >= bad[2 * N + col + j] ? INFINITY : o[m][2 * hh + j];
+          w[j] = t >= min(bad[N + col + j], bad[3 * N + col + j]) ? NAN : t >= bad[2 * N + col + j] ? INFINITY : o[m][2 * hh + j];
         }
         *reinterpret_cast<float2*>(item + 2 * N * N + t * N + col) = make_float2(v[0], v[1]);
         *reinterpret_cast<float2*>(item + 2 * N * N + L * N + t * N + col) = make_float2(w[0], w[1]);
@@ -1107,7 +1108,7 @@ KRK_API int krk_recurrence_chunks(int rule, const void* r, int r_stride, const v
   const size_t RP = (size_t)((R + 7) & ~7);
   if (rule == 1) {
     // six times three terms of a chunk's rows and the values; two matrices of float32; the small things
-    const size_t chunk = 19 * (size_t)L * KP / 2 + 2 * (size_t)L * PITCH + N + 2 * L + 8 * N + 3 * N;
+    const size_t chunk = 19 * (size_t)L * KP / 2 + 2 * (size_t)L * PITCH + N + 2 * L + 8 * N + 4 * N;
     if ((rc = run(delta_chunk_kernel, items, DELTA_THREADS, chunk, a, stream))) return rc;
     const size_t walk = (size_t)WALK_STAGES * N * (PITCH + WALK_COLS) + N * WALK_COLS + 4 * N * 4;
     if ((rc = run(delta_walk_kernel, dim3(N / WALK_COLS, (unsigned)H, (unsigned)n_seqs), THREADS, walk, a, stream))) return rc;

@@ -490,6 +490,28 @@ def test_a_tokens_infinities_reach_no_earlier_token(kind, monkeypatch):
     assert torch.equal(states[1][0, :, :, rest], states[0][0, :, :, rest]) and not torch.isfinite(states[1][0, 0, :, 5]).any()
 
 
+@pytest.mark.parametrize("token", [41, 64, 95])
+@pytest.mark.parametrize("kind", ["delta", "wkv"])
+def test_a_value_that_is_no_number(kind, token, monkeypatch):
+    """A NaN in one value channel leaves the whole head's outputs NaN from its token on, through the head's norm, as token by token; nothing
+    before it, no other head and no other channel of the state."""
+    rt = runtime(torch.bfloat16)
+    x = scan_inputs(kind, [96], 2, "mild", 80)
+    start = rand((1, 2, 64, 64), 90).cuda()
+    clean, clean_state = None, start.clone()
+    for in_chunks in (False, True):
+        monkeypatch.setattr(type(rt.ops), "_recurrence_in_chunks", lambda *_, yes=in_chunks: yes)
+        clean_state, state = start.clone(), start.clone()
+        clean = run_scan(rt, kind, x, [96], 2, clean_state)
+        y = dict(x, v=x["v"].clone())
+        y["v"][token, 5] = float("nan")
+        got = run_scan(rt, kind, y, [96], 2, state)
+        assert torch.equal(got[:token], clean[:token]) and torch.equal(got[:, 64:], clean[:, 64:])
+        assert torch.isnan(got[token:, :64]).all(), f"in chunks {in_chunks}"
+        rest = [p for p in range(64) if p != 5]
+        assert torch.equal(state[0, :, :, rest], clean_state[0, :, :, rest]) and torch.isnan(state[0, 0, :, 5]).all()
+
+
 @pytest.mark.parametrize("kind", ["delta", "wkv"])
 def test_a_scan_without_room_for_its_scratch(kind, monkeypatch):
     """Where the device's memory has no room for the chunks' scratch, a step goes through in smaller portions, and token by token
