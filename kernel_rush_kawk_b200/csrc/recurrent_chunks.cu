@@ -143,13 +143,17 @@ __device__ __forceinline__ void split3_store4(bf16* dst, int apart, float4 x) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(dst + i * apart) = make_uint2(lo[i], hi[i]);
 }
-__device__ __forceinline__ void load_raw(bf16* dst, const bf16* src, int stride, size_t row0, int ch0, int nt) {
+// Returns whether one of this thread's is not finite: an exponent of ones, to which its lowest bit is added, leaves its field.
+__device__ __forceinline__ bool load_raw(bf16* dst, const bf16* src, int stride, size_t row0, int ch0, int nt) {
+  uint32_t over = 0u;
 #pragma unroll
   for (int i = threadIdx.x; i < L * (N / 4); i += THREADS) {
     const int t = i / (N / 4), c = (i % (N / 4)) * 4;
-    *reinterpret_cast<uint2*>(dst + t * KP + c) =
-        t < nt ? *reinterpret_cast<const uint2*>(src + (row0 + t) * stride + ch0 + c) : make_uint2(0u, 0u);
+    const uint2 four = t < nt ? *reinterpret_cast<const uint2*>(src + (row0 + t) * stride + ch0 + c) : make_uint2(0u, 0u);
+    *reinterpret_cast<uint2*>(dst + t * KP + c) = four;
+    over |= ((four.x & 0x7f807f80u) + 0x00800080u) | ((four.y & 0x7f807f80u) + 0x00800080u);
   }
+  return over & 0x80008000u;
 }
 
 // The five small products of two operands that are three terms each, into one tile of 16 x 8. The sixth, of the leading terms, is added
@@ -455,7 +459,13 @@ __global__ void __launch_bounds__(DELTA_THREADS, 2) delta_chunk_kernel(ChunkArgs
         for (int j = 0; j < 2; ++j) {
           v[j] = d[n][2 * hh + j];
           if (!is_g && row == col + j) v[j] += 1.f;
-          v[j] = worst[col + j] < L || (is_g && min(bad[2 * N + col + j], bad[3 * N + col + j]) < L) ? NAN : w * v[j];
+          if (is_g && min(bad[2 * N + col + j], bad[3 * N + col + j]) < L) {
+            // a value that is not finite: the tokens after it have read it (NaN), unless it is the chunk's last
+            const bf16* key = kt + (nt - 1) * KP + row;
+            const float k0 = __bfloat162float(key[0]), k1 = k0 + (__bfloat162float(key[TERM]) + __bfloat162float(key[2 * TERM]));
+            v[j] = fmaf(fabsf(k0) < INFINITY ? k1 : k0, __bfloat162float(a.v[(row0 + nt - 1) * a.v_stride + ch0 + col + j]), v[j]);
+          }
+          v[j] = worst[col + j] < nt ? NAN : w * v[j];
         }
         *reinterpret_cast<float2*>(item + (is_g ? N * N : 0) + row * N + col) = make_float2(v[0], v[1]);
       }
@@ -542,10 +552,9 @@ __global__ void __launch_bounds__(THREADS, 8) mix_chunk_kernel(ChunkArgs a) {
   const int first = (a.chunk0 + ci) * L, nt = min(L, a.seq_qlen[seq] - first);
   if (nt <= 0) return;
   const size_t row0 = (size_t)a.cu_q[seq] + first;
-  load_raw(ks, a.k, a.k_stride, row0, ch0, nt);
-  load_raw(vs, a.v, a.v_stride, row0, ch0, nt);
+  const bool odd_key = load_raw(ks, a.k, a.k_stride, row0, ch0, nt), odd_value = load_raw(vs, a.v, a.v_stride, row0, ch0, nt);
   load_tanh(a, th_s, row0, nt);
-  __syncthreads();
+  const bool odd = __syncthreads_or(odd_key || odd_value);
   float* item = a.scratch + (((size_t)seq * a.n_chunks + ci) * a.H + h) * ITEM_MIX;
   {
     const int ch = threadIdx.x & (N - 1), half = threadIdx.x / N, t0 = half * HALF;
@@ -612,6 +621,21 @@ __global__ void __launch_bounds__(THREADS, 8) mix_chunk_kernel(ChunkArgs a) {
 #pragma unroll
     for (int hh = 0; hh < 2; ++hh)
       *reinterpret_cast<float2*>(item + (m0 + (lane >> 2) + 8 * hh) * N + n * 8 + 2 * (lane & 3)) = make_float2(g[n][2 * hh], g[n][2 * hh + 1]);
+  if (odd) {  // the terms of an infinity do not add up to it: what came out not finite, again with multiply-adds
+#pragma unroll 1
+    for (int i = 0; i < N / 2; ++i) {
+      const int n = m0 + (lane >> 2) + (i & 2) * 4, p = (i >> 2) * 8 + 2 * (lane & 3) + (i & 1);  // this thread's own sums
+      if (fabsf(item[n * N + p]) < INFINITY) continue;
+      float sum = 0.f;
+#pragma unroll 1
+      for (int t = 0; t < nt; ++t) {
+        const bf16* key = kt + t * KP + n;
+        const float k0 = __bfloat162float(key[0]), k1 = k0 + (__bfloat162float(key[L * KP]) + __bfloat162float(key[2 * L * KP]));
+        sum = fmaf(fabsf(k0) < INFINITY ? k1 : k0, __bfloat162float(vs[t * KP + p]), sum);
+      }
+      item[n * N + p] = sum;
+    }
+  }
 }
 
 // ---- pass 2 ----------------------------------------------------------------------------------------------------

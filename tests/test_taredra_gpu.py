@@ -512,6 +512,33 @@ def test_a_value_that_is_no_number(kind, token, monkeypatch):
         assert torch.equal(state[0, :, :, rest], clean_state[0, :, :, rest]) and torch.isnan(state[0, 0, :, 5]).all()
 
 
+@pytest.mark.parametrize("value", [float("inf"), float("-inf")])
+@pytest.mark.parametrize("kind, what, token, rows", [
+    ("delta", "v", 95, 96), ("delta", "v", 89, 90), ("delta", "v", 64, 65), ("delta", "k", 95, 96), ("delta", "k", 41, 96), ("delta", "r", 41, 96),
+    ("wkv", "v", 41, 96), ("wkv", "v", 95, 96), ("wkv", "k", 41, 96), ("wkv", "k", 64, 65), ("wkv", "r", 41, 96)])
+def test_an_infinity_leaves_the_state_that_it_leaves_token_by_token(kind, what, token, rows, value, monkeypatch):
+    """An infinite value, key or query: infinities of the same sign and NaNs in the same places of the state, the rest of it within the
+    rounding of its sums; the outputs before it and those of other heads the same bits as without it."""
+    rt = runtime(torch.bfloat16)
+    x = scan_inputs(kind, [rows], 2, "mild", 80)
+    start = rand((1, 2, 64, 64), 90).cuda()
+    states = []
+    for in_chunks in (False, True):
+        monkeypatch.setattr(type(rt.ops), "_recurrence_in_chunks", lambda *_, yes=in_chunks: yes)
+        clean_state, state = start.clone(), start.clone()
+        clean = run_scan(rt, kind, x, [rows], 2, clean_state)
+        y = dict(x, **{what: x[what].clone()})
+        y[what][token, 5] = value
+        got = run_scan(rt, kind, y, [rows], 2, state)
+        assert torch.equal(got[:token], clean[:token]) and torch.equal(got[:, 64:], clean[:, 64:])
+        assert not torch.isfinite(got[token, :64]).all() and torch.equal(state[0, 1], clean_state[0, 1])
+        states.append(state)
+    tokens, chunks = states
+    assert torch.equal(torch.isnan(tokens), torch.isnan(chunks))
+    assert torch.equal(tokens.isposinf(), chunks.isposinf()) and torch.equal(tokens.isneginf(), chunks.isneginf())
+    assert (tokens - chunks)[torch.isfinite(tokens)].abs().max() < 1e-5 if torch.isfinite(tokens).any() else True
+
+
 @pytest.mark.parametrize("kind", ["delta", "wkv"])
 def test_a_scan_without_room_for_its_scratch(kind, monkeypatch):
     """Where the device's memory has no room for the chunks' scratch, a step goes through in smaller portions, and token by token
