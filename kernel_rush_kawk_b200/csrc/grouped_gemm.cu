@@ -19,6 +19,7 @@
 // holds are rows, so a warp turns 32 x 32 of them through a patch of shared memory. Gated, gate and up rows alternate in the tile, so
 // that neighbouring lanes hold a column's two products. Rows beyond the expert's, the next one's or zeros, are not stored.
 // Every wait is bounded: one that runs out sets the error word, and the blocks leave after freeing their tensor memory.
+#include "mma.cuh"  // times_logistic
 #include "tcgen05.cuh"
 
 namespace {
@@ -30,18 +31,26 @@ constexpr int SMS = 148;
 constexpr int READERS = 8;  // warps that read accumulators: two to a quarter of tensor memory's lanes
 constexpr int THREADS = 64 + 32 * READERS;
 
-// SILU: silu(g) u of the two products as they would have been stored; CLAMPED:,
+// SILU: silu(g) u of the two products as they would have been stored; CLAMPED:
 // g' = min(g, limit), u' = clamp(u, -limit, limit), g' sigmoid(slope g') (u' + 1), nothing rounded before the end
 enum Form { SILU, CLAMPED, PLAIN, SQUARED };
 
-template <Form FORM>
+// SHORT: single-token steps, which may come here or, with fewer pairs, to few_experts.cu, are as exact here as there. There eight warps share
+// a sum's k, and the activation is expf and a division. The tensor cores cut off every sum: one accumulator for all of 2,048 k left 2.0e-3
+// of the activations next to the correctly rounded ones. So tiles are of up to 32 rows and have eight accumulators, a block of k each in
+// turn, which are added when they are read back.
+constexpr int SHORT_ROWS = 32, SHORT_SUMS = 8;
+
+template <Form FORM, bool SHORT>
 __device__ __forceinline__ float gated_act_of(float g, float u, float limit, float slope) {
   if (FORM == CLAMPED) {
     g = fminf(g, limit);
     u = fminf(fmaxf(u, -limit), limit);
+    if (SHORT) return times_logistic(g, slope * g) * (u + 1.0f);
     return __fdividef(g, 1.0f + __expf(-slope * g)) * (u + 1.0f);
   }
   g = round_to<bf16>(g);
+  if (SHORT) return silu_near(g) * round_to<bf16>(u);
   return __fdividef(g, 1.0f + __expf(-g)) * round_to<bf16>(u);
 }
 
@@ -98,7 +107,7 @@ struct RowTiles {
   }
 };
 
-template <Form FORM>
+template <Form FORM, bool SHORT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS)
 grouped_gemm_kernel(const __grid_constant__ RowMaps maps_a, const __grid_constant__ CUtensorMap map_w, bf16* __restrict__ C,
                     const int* __restrict__ offsets, int E, int N, int K, int most, const float* __restrict__ row_weights,
@@ -213,7 +222,8 @@ grouped_gemm_kernel(const __grid_constant__ RowMaps maps_a, const __grid_constan
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
             const uint64_t adv = (uint64_t)((k * UMMA_K * 2) >> 4);
-            umma_bf16_pair(acc, w_desc + adv, r_desc + adv, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            if (SHORT) umma_bf16_pair(acc + kb % SHORT_SUMS * SHORT_ROWS, w_desc + adv, r_desc + adv, idesc, (kb >= SHORT_SUMS || k > 0) ? 1u : 0u);
+            else umma_bf16_pair(acc, w_desc + adv, r_desc + adv, idesc, (kb > 0 || k > 0) ? 1u : 0u);
           }
           umma_commit_pair(empty_bar + s);
           if (++s == stages) { s = 0; parity ^= 1; }
@@ -254,6 +264,16 @@ grouped_gemm_kernel(const __grid_constant__ RowMaps maps_a, const __grid_constan
           float by = 1.f;
           if (GATED && row_weights && live) by = row_weights[row];
           tmem_wait_ld();
+          if constexpr (SHORT) {
+#pragma unroll 1
+            for (int i = 1; i < min(SHORT_SUMS, k_blocks); ++i) {
+              uint32_t more[32];
+              tmem_ld_32x32(acc + (uint32_t)(i * SHORT_ROWS), more);
+              tmem_wait_ld();
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(more[j]));
+            }
+          }
           if constexpr (GATED) {
             // an even lane has a feature's gate and the odd one after it the same feature's up: they share the rows, the even ones to
             // the even lane
@@ -269,7 +289,7 @@ grouped_gemm_kernel(const __grid_constant__ RowMaps maps_a, const __grid_constan
                 u *= w;
               }
               *reinterpret_cast<bf16*>(patch + (2 * j + (odd ? 1 : 0)) * PATCH_PITCH + (lane >> 1) * 2) =
-                  from_float<bf16>(gated_act_of<FORM>(g, u, limit, slope));
+                  from_float<bf16>(gated_act_of<FORM, SHORT>(g, u, limit, slope));
             }
           } else {
 #pragma unroll
@@ -312,9 +332,10 @@ grouped_gemm_kernel(const __grid_constant__ RowMaps maps_a, const __grid_constan
   }
 }
 
-template <Form FORM>
-int launch_grouped(bf16* C, const bf16* A, const bf16* W, const int* offsets, int rows, int E, int N, int K, int most,
+template <Form FORM, bool SHORT = false>
+int launch_grouped(bf16* C, const bf16* A, const bf16* W, const int* offsets, int rows, int E, int N, int K, int tall,
                    const float* row_weights, float limit, float slope, int* error, cudaStream_t stream) {
+  const int most = SHORT ? SHORT_ROWS : tall ? 256 : 128;
   constexpr bool GATED = FORM == SILU || FORM == CLAMPED;
   RowMaps maps_a;
   CUtensorMap map_w;
@@ -325,7 +346,7 @@ int launch_grouped(bf16* C, const bf16* A, const bf16* W, const int* offsets, in
   rc = GATED ? make_map_bf16_3d(&map_w, W, K, 2, 2LL * E * N - N, (long long)N * K, K, 2, 64)
              : make_map_bf16(&map_w, W, (long long)E * N, K, K, 128);
   if (rc) return rc;
-  auto kern = grouped_gemm_kernel<FORM>;
+  auto kern = grouped_gemm_kernel<FORM, SHORT>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
@@ -343,14 +364,18 @@ int launch_grouped(bf16* C, const bf16* A, const bf16* W, const int* offsets, in
 
 // C [rows, N] = act(A [rows, K] W_e^T) over the experts' rows (offsets int32 [E + 1] on the device; rows is the most there
 // can be). act: -1 none, 5 squared relu. N and K multiples of 8, K at least 64, 16-byte aligned bases. `gated`: W [E, 2N, K],
-// act 0 (silu) or 3 (clamped swish with its limit and slope), row_weights [rows] or null. `tall`: tiles of up to 256 of an
-// expert's rows, else of 128, which fetches the weights of experts with more rows twice.
+// act 0 (silu) or 3 (clamped swish with its limit and slope), row_weights [rows] or null. `tall` 1: tiles of up to 256 of an
+// expert's rows; 0: of 128, which fetches the weights of experts with more rows twice; 2: a single-token step's, of 32.
 KRK_API int krk_grouped_gemm(void* C, const void* A, const void* W, const int* offsets, int rows, int E, int N, int K, int act,
                              int gated, int tall, const float* row_weights, float limit, float slope, int* error,
                              cudaStream_t stream) {
   if (rows == 0 || N == 0 || E == 0) return 0;
   if (N % 8 || K % 8 || K < 64 || (((uintptr_t)A | (uintptr_t)W | (uintptr_t)C) & 15) || 2LL * E * N > 0x7fffffffLL) return -2;
   if (gated ? (act != 0 && act != 3) : ((act != -1 && act != 5) || row_weights)) return -2;
-  auto go = gated ? (act == 3 ? launch_grouped<CLAMPED> : launch_grouped<SILU>) : (act == 5 ? launch_grouped<SQUARED> : launch_grouped<PLAIN>);
-  return go((bf16*)C, (const bf16*)A, (const bf16*)W, offsets, rows, E, N, K, tall ? 256 : 128, row_weights, limit, slope, error, stream);
+  const Form form = gated ? (act == 3 ? CLAMPED : SILU) : (act == 5 ? SQUARED : PLAIN);
+  auto go = tall == 2 ? (form == CLAMPED ? launch_grouped<CLAMPED, true> : form == SILU ? launch_grouped<SILU, true>
+                         : form == SQUARED ? launch_grouped<SQUARED, true> : launch_grouped<PLAIN, true>)
+                      : (form == CLAMPED ? launch_grouped<CLAMPED> : form == SILU ? launch_grouped<SILU>
+                         : form == SQUARED ? launch_grouped<SQUARED> : launch_grouped<PLAIN>);
+  return go((bf16*)C, (const bf16*)A, (const bf16*)W, offsets, rows, E, N, K, tall, row_weights, limit, slope, error, stream);
 }

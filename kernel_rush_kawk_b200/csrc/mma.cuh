@@ -18,18 +18,19 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// z / (1 + e^-z) for results that are rounded to bfloat16, as exact as expf and a division leave it: the quotient is a product with the
+// z / (1 + e^-y) for results that are rounded to bfloat16, as exact as expf and a division leave it: the quotient is a product with the
 // approximate reciprocal (an error of about 2^-23), corrected once by what it leaves of z (Newton's step), which squares that error. The
 // division branches for divisors beyond 2^126, whose reciprocals are subnormal; here both sides are taken a quarter, an infinite divisor has
 // zero for a reciprocal, and what is left beside an infinity is no number and counts as any. 8.4 million of them, with the short convolution
 // around: 23.5 us by the division, 15.7 here.
-__device__ __forceinline__ float silu_near(float z) {
-  const float divisor = 0.25f * (1.0f + expf(-z)), part = 0.25f * z;
+__device__ __forceinline__ float times_logistic(float z, float y) {
+  const float divisor = 0.25f * (1.0f + expf(-y)), part = 0.25f * z;
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(divisor));
   const float q = part * r;
   return fmaf(fminf(fmaf(-q, divisor, part), 3e38f), r, q);
 }
+__device__ __forceinline__ float silu_near(float z) { return times_logistic(z, z); }
 
 // x and y as three pairs of bfloat16 terms each, which add up to them (24 bits of mantissa). Two conversions at once and the widening by
 // hand: single conversions run on the unit of the exponentials, a quarter as fast.

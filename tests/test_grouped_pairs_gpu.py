@@ -81,3 +81,88 @@ def test_experts_where_their_products_change_hands(E, top, F, C, line):
             # gate, up, their product, each expert's result and the sum are rounded: five times 2^-9 in the mean, added in squares
             assert off < 5 ** 0.5 * 2.0 ** -8, (rows, decode, float(off))
     ops.check()
+
+
+@pytest.mark.parametrize("activation, act_params, weigh_input", [("silu", None, False), ("swish_clamped", (7.0, 1.702), True)])
+def test_single_token_steps_are_as_exact_by_either_route(activation, act_params, weigh_input, monkeypatch):
+    """Outputs next to the correctly rounded ones, where every product, activation and result is rounded as the path rounds it: by pieces of an
+    expert half a percent or less, and no more by the grouped launches (4 % with one accumulator for all of k, whose last bits the
+    tensor cores cut off)."""
+    from types import SimpleNamespace
+
+    from kernel_rush_kawk_b200.csrc import load_kernels
+    from kernel_rush_kawk_b200.csrc.bindings import Kernels
+
+    ops = load_kernels((), "cuda:0")
+    g = torch.Generator("cuda").manual_seed(3)
+    E, top, F, K, C, rows = 64, 6, 640, 2048, 1280, 64
+    normal = lambda *s, std=1.0: torch.empty(s, device="cuda").normal_(0, std, generator=g)
+    x, w1, w2 = (t.to(torch.bfloat16) for t in (normal(rows, K), normal(E, 2 * F, K, std=K ** -0.5), normal(E, C, F, std=F ** -0.5)))
+    experts = torch.rand((rows, E), device="cuda", generator=g).topk(top, 1).indices.int()
+    weights = torch.rand((rows, top), device="cuda", generator=g)
+    rounded = lambda t: t.float().to(torch.bfloat16).double()
+    want = torch.zeros((rows, C), dtype=torch.float64, device="cuda")
+    for e in range(E):
+        r, j = (experts == e).nonzero(as_tuple=True)
+        y, w = x[r].double() @ w1[e].double().t(), weights[r, j].double()[:, None]
+        if activation == "silu":
+            y = rounded(y)
+            h = y[:, :F] * torch.sigmoid(y[:, :F]) * y[:, F:]
+        else:
+            gate, up = (w * y)[:, :F].clamp(max=7.0), (w * y)[:, F:].clamp(-7.0, 7.0)
+            h = gate * torch.sigmoid(1.702 * gate) * (up + 1)
+        out = rounded(rounded(h) @ w2[e].double().t())
+        want.index_add_(0, r, out if weigh_input else out * w)
+    share = {}
+    for route, line in (("pieces", 1 << 30), ("grouped", 0)):
+        monkeypatch.setattr(Kernels, "_grouped_from", staticmethod(lambda *_, line=line: line))
+        got = ops.moe_experts(x, w1, w2, experts, weights, F, activation, batch=SimpleNamespace(is_decode=True), act_params=act_params,
+                              weigh_input=weigh_input)
+        share[route] = (got != want.float().to(torch.bfloat16)).double().mean().item()
+    ops.check()
+    assert share["grouped"] < 1.5 * share["pieces"] + 1e-3 and share["pieces"] < 0.01, share
+
+
+def test_gates_of_the_most_negative_in_a_single_token_step():
+    """Gates down to where e^-g still is a number: activations of 1e-36 as exact as any other."""
+    from kernel_rush_kawk_b200.csrc import load_kernels
+
+    ops = load_kernels((), "cuda:0")
+    N, K = 128, 64
+    z = -torch.linspace(20.0, 87.5, N).to(torch.bfloat16)
+    w = torch.zeros(1, 2 * N, K, dtype=torch.bfloat16)
+    w[0, :N, 0], w[0, N:, 1] = z, 1.0
+    a = torch.zeros(7, K, dtype=torch.bfloat16)
+    a[:, :2] = 1.0
+    out, offsets = torch.empty(7, N, dtype=torch.bfloat16, device="cuda"), torch.tensor([0, 7], dtype=torch.int32, device="cuda")
+    a_d, w_d = a.cuda(), w.cuda()
+    ops._ok(ops.moe.krk_grouped_gemm(out.data_ptr(), a_d.data_ptr(), w_d.data_ptr(), offsets.data_ptr(), 7, 1, N, K, 0, 1, 2, None, 0.0, 0.0,
+                                     ops.error.data_ptr(), ops._stream()), "grouped product")
+    want = z.double() * torch.sigmoid(z.double())
+    assert ((out.double().cpu() - want).abs() <= 1.01 * 2.0 ** -8 * want.abs()).all()
+
+
+@pytest.mark.parametrize("gated", [0, 1])
+@pytest.mark.parametrize("N, K, counts", [(8, 64, [31, 32, 33, 0, 1]), (136, 200, [65, 0, 0, 97]), (264, 640, [2, 5]), (384, 520, [0] * 40 + [1] + [0] * 30 + [300])])
+def test_single_token_tiles_at_their_edges(N, K, counts, gated):
+    """Tiles of 32 rows in up to eight partial sums, fewer where k has fewer blocks of 64: within the rounding of the result and of a
+    float32 sum, rows beyond the last expert's as they were."""
+    from kernel_rush_kawk_b200.csrc import load_kernels
+
+    ops = load_kernels((), "cuda:0")
+    g = torch.Generator().manual_seed(4)
+    offsets = torch.tensor([0] + counts).cumsum(0).to(torch.int32)
+    rows, E = int(offsets[-1]), len(counts)
+    a = torch.randn(rows + 3, K, generator=g).to(torch.bfloat16)
+    w = (torch.randn(E, (2 if gated else 1) * N, K, generator=g) * K ** -0.5).to(torch.bfloat16)
+    a_d, w_d, o_d = a.cuda(), w.cuda(), offsets.cuda()
+    outs = []
+    for tiles in (1, 2):
+        out = torch.full((rows + 3, N), 7.0, dtype=torch.bfloat16, device="cuda")
+        ops._ok(ops.moe.krk_grouped_gemm(out.data_ptr(), a_d.data_ptr(), w_d.data_ptr(), o_d.data_ptr(), rows + 3, E, N, K,
+                                         0 if gated else -1, gated, tiles, None, 0.0, 0.0, ops.error.data_ptr(), ops._stream()), "grouped product")
+        outs.append(out.double().cpu())
+    ops.check()
+    # one rounding of the result, gated of either product too (a gate's through silu's slope, at most 1.1)
+    assert ((outs[0] - outs[1]).abs() <= (3.1 if gated else 1.0) * 2.0 ** -7 * outs[0].abs() + (2.0 ** -7 if gated else 1e-4)).all()
+    assert (outs[1][rows:] == 7.0).all()
