@@ -992,9 +992,9 @@ class Kernels:
         return ((not gated or activation in ("swish_clamped", "silu")) and x.dtype == torch.bfloat16 and K % 8 == 0 and F % 8 == 0 and C % 8 == 0 and min(K, F) >= 64)
 
     def _grouped_experts(self, x, w_first, w_down, experts, w_in, w_out, activation, act_params, add, add_gate, gated, add_input,
-                         offsets, place, tiles):
+                         offsets, place, route):
         """``moe_experts`` for many rows with the experts' row counts left on the device: rows ordered by expert, the first
-        product (weights of the input and the activation in its epilogue), the second, and the weighted sum. ``tiles``: 1, or 2 for
+        product (weights of the input and the activation in its epilogue), the second, and the weighted sum. ``route``: 1, or 2 for
         a single-token step, whose sums are as exact as those of fewer pairs."""
         rows, top = experts.shape
         E, C, F = w_down.shape
@@ -1007,10 +1007,10 @@ class Kernels:
         self._ok(self.moe.krk_moe_gather(xg.data_ptr(), ptr, stride, place.data_ptr(), experts.data_ptr(), offsets.data_ptr(), 0,
                                          rows, top, K, _ptr(w_in), _ptr(row_w), _code(x.dtype), self._stream()), "expert gather")
         self._ok(self.moe.krk_grouped_gemm(h.data_ptr(), xg.data_ptr(), w_first.data_ptr(), offsets.data_ptr(), pairs, E, F, K,
-                                           _ACTIVATIONS[activation], int(gated), tiles, _ptr(row_w), float(act_params[0]),
+                                           _ACTIVATIONS[activation], int(gated), route, _ptr(row_w), float(act_params[0]),
                                            float(act_params[1]), self.error.data_ptr(), self._stream()), "experts' first product")
         self._ok(self.moe.krk_grouped_gemm(yg.data_ptr(), h.data_ptr(), w_down.data_ptr(), offsets.data_ptr(), pairs, E, C, F, -1,
-                                           0, tiles, None, 0.0, 0.0, self.error.data_ptr(), self._stream()), "experts' second product")
+                                           0, route, None, 0.0, 0.0, self.error.data_ptr(), self._stream()), "experts' second product")
         out = torch.empty((rows, C), dtype=x.dtype, device=x.device)
         self._ok(self.moe.krk_moe_combine(out.data_ptr(), _ptr(add), _ptr(add_gate), yg.data_ptr(), place.data_ptr(),
                                           experts.data_ptr(), offsets.data_ptr(), 0, _ptr(w_out), rows, top, C, ptr, stride,

@@ -9,8 +9,8 @@
 // in steps of 32 instead of 128, every weight is fetched once for up to 256 rows, an SM takes in 16 KB of weights and its half of the rows
 // for as much work as a block alone does with 16 and 32 KB, and a tile's accumulator fills half of tensor memory: while its eight
 // reading warps turn one tile into C, the next one is multiplied. Pairs stay and walk the tiles (74 pairs, the tiles of a row tile
-// side by side), so that loads go on over the seams. With a single-block tile of 256 rows by 256 columns, launched per tile,
-// the two products took 195 and 105 us, now 163 and 85; 4,000 rows 352 and 187 -> 280 and 150; 200 rows, where nothing but the weights
+// side by side), so that loads go on over the seams; products of few tiles take single blocks (by_blocks, below). With a single-block tile of
+// 256 rows by 256 columns, launched per tile, the two products took 195 and 105 us, now 163 and 85; 4,000 rows 352 and 187 -> 280 and 150; 200 rows, where nothing but the weights
 // counts, 163 and 81 -> 120 and 65. Asking weights into L2 ahead of the ring was measured and is slower (eight blocks of k: 219
 // against 189 us, single blocks); rows in copies of 16 instead of 128, 64, 32 and 16: 200 against 167 us.
 //
@@ -332,10 +332,181 @@ grouped_gemm_kernel(const __grid_constant__ RowMaps maps_a, const __grid_constan
   }
 }
 
-template <Form FORM, bool SHORT = false>
-int launch_grouped(bf16* C, const bf16* A, const bf16* W, const int* offsets, int rows, int E, int N, int K, int tall,
-                   const float* row_weights, float limit, float slope, int* error, cudaStream_t stream) {
-  const int most = SHORT ? SHORT_ROWS : tall ? 256 : 128;
+// The same by single blocks, 128 of an expert's rows against BN rows of its weights (gated: 128 gate rows and their up rows), a tile each: for
+// products of few tiles, which pairs would do in fewer and larger pieces than the SMs are (by_blocks). The rows are the product's M here, so a
+// lane is a row of C. Tile for tile the sums are the same bits.
+constexpr int BLOCK_THREADS = 192, BLOCK_STAGES = 4;
+constexpr uint32_t A_BYTES = 128 * BK * 2;
+
+template <int BN> constexpr size_t block_smem() { return (size_t)BLOCK_STAGES * (A_BYTES + BN * BK * 2) + 1024 + (2 * BLOCK_STAGES + 1) * 8 + 16; }
+
+template <Form FORM, int BN>
+__global__ void __launch_bounds__(BLOCK_THREADS)
+grouped_block_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, bf16* __restrict__ C,
+                     const int* __restrict__ offsets, int E, int N, int K, const float* __restrict__ row_weights, float limit,
+                     float slope, int* __restrict__ error) {
+  constexpr bool GATED = FORM == SILU || FORM == CLAMPED;
+  static_assert(!GATED || BN == 256, "a gate tile and an up tile of 128 rows each");
+  constexpr int BC = GATED ? BN / 2 : BN;  // columns of C a block makes
+  constexpr uint32_t STAGE_BYTES = A_BYTES + BN * BK * 2;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(tiles + (size_t)BLOCK_STAGES * STAGE_BYTES);
+  uint64_t* empty_bar = full_bar + BLOCK_STAGES;
+  uint64_t* acc_bar = empty_bar + BLOCK_STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_bar + 1);
+  int* issued = reinterpret_cast<int*>(tmem_slot + 1);  // blocks of k that were asked for, where a wait ran out; else -1
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  grid_dependency_wait();
+  RowTiles tiles_of(offsets, E, 128);
+  int e, m0, rows;
+  if (!tiles_of.find(blockIdx.y, e, m0, rows)) return;  // the same for the whole block
+  const int n0 = blockIdx.x * BC, k_blocks = (K + BK - 1) / BK;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < BLOCK_STAGES; ++s) {
+      mbar_init(full_bar + s, 1);
+      mbar_init(empty_bar + s, 1);
+    }
+    mbar_init(acc_bar, 1);
+    *issued = -1;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(BN) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  grid_launch_dependents();
+
+  if (warp == 0 && lane == 0) {
+    for (int kb = 0; kb < k_blocks; ++kb) {
+      const int s = kb % BLOCK_STAGES;
+      if (kb >= BLOCK_STAGES && !mbar_wait(empty_bar + s, ((kb / BLOCK_STAGES) - 1) & 1)) {
+        atomicExch(error, 3);
+        *issued = kb;
+        break;
+      }
+      unsigned char* stage = tiles + (size_t)s * STAGE_BYTES;
+      mbar_expect_tx(full_bar + s, STAGE_BYTES);
+      tma_load_2d(stage, &map_a, full_bar + s, kb * BK, m0);
+#pragma unroll
+      for (int h = 0; h < BN / 128; ++h)
+        tma_load_2d(stage + A_BYTES + h * (128 * BK * 2), &map_w, full_bar + s, kb * BK, GATED ? (2 * e + h) * N + n0 : e * N + n0 + 128 * h);
+    }
+  } else if (warp == 1 && lane == 0) {
+    constexpr uint32_t idesc = umma_idesc(128, BN);
+    for (int kb = 0; kb < k_blocks; ++kb) {
+      const int s = kb % BLOCK_STAGES;
+      if (!mbar_wait(full_bar + s, (kb / BLOCK_STAGES) & 1)) {
+        atomicExch(error, 4);
+        break;
+      }
+      tc_fence_after();
+      unsigned char* stage = tiles + (size_t)s * STAGE_BYTES;
+      const uint64_t a_desc = umma_desc(stage), b_desc = umma_desc(stage + A_BYTES);
+#pragma unroll
+      for (int k = 0; k < BK / UMMA_K; ++k) {
+        const uint64_t adv = (uint64_t)((k * UMMA_K * 2) >> 4);
+        umma_bf16(tmem_base, a_desc + adv, b_desc + adv, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+      }
+      umma_commit(empty_bar + s);
+    }
+    umma_commit(acc_bar);  // arrives even after a failed wait, so the epilogue moves on
+  } else if (warp >= 2) {
+    const int quarter = warp & 3, row = quarter * 32 + lane;
+    const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    const bool ok = mbar_wait(acc_bar, 0);
+    if (!ok && lane == 0) atomicExch(error, 5);
+    __syncwarp();
+    tc_fence_after();
+    if (ok) {
+      const float by = GATED && row_weights && row < rows ? row_weights[m0 + row] : 1.f;
+#pragma unroll 1
+      for (int c0 = 0; c0 < BC && n0 + c0 < N; c0 += 32) {
+        uint32_t g[32], u[GATED ? 32 : 1];
+        tmem_ld_32x32(acc + (uint32_t)c0, g);
+        if constexpr (GATED) tmem_ld_32x32(acc + (uint32_t)(BC + c0), u);
+        tmem_wait_ld();
+        if (row < rows) {
+          bf16* dst = C + (size_t)(m0 + row) * N + n0 + c0;
+#pragma unroll
+          for (int j = 0; j < 32; j += 8) {
+            float v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              v[i] = __uint_as_float(g[j + i]);
+              if constexpr (GATED) {
+                v[i] = gated_act_of<FORM, false>(by * v[i], by * __uint_as_float(u[j + i]), limit, slope);
+              } else if (FORM == SQUARED) {  // squared relu of the product as it would have been stored
+                const float z = round_to<bf16>(v[i]);
+                v[i] = z > 0.f ? z * z : 0.f;
+              }
+            }
+            uint4 pk;
+            __nv_bfloat162* two = reinterpret_cast<__nv_bfloat162*>(&pk);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) two[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+            if (n0 + c0 + j < N) *reinterpret_cast<uint4*>(dst + j) = pk;  // N is a multiple of 8
+          }
+        }
+        __syncwarp();
+      }
+    }
+    tc_fence_before();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && *issued >= 0)  // copies on their way end before shared memory is given up
+    for (int i = max(0, *issued - BLOCK_STAGES); i < *issued; ++i)
+      mbar_wait(full_bar + i % BLOCK_STAGES, (uint32_t)(i / BLOCK_STAGES) & 1u, WAIT_LIMIT_NS / 20);
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(BN) : "memory");
+  }
+}
+
+// Whether single blocks are the faster ones: where their tiles, an expert's last one half filled, are one round over the SMs (two of a
+// short k), and the pairs' larger ones would be a second round that is nearly empty (gated, whose epilogue takes a single block's lanes longer), or
+// leave SMs idle: an expert's rows are a tile's or nearly, or its columns half of one. Pairs and blocks, us: gated, 8 experts of 512 x 1,024,
+// 2,048 rows 13.9 and 17.1, 4,096 rows 20.8 and 13.4, of 16 22.2 and 35.7; plain, 16 of 512 x 1,024, 1,024 rows 10.4 and 11.2, 2,048 11.9
+// and 10.3, 4,096 14.5 and 11.7, 8,192 21.4 and 14.2; 16 of 1,024 x 512, 8,192 rows 23.7 and 18.7; of 1,024 x 1,024 27.8 and 26.7; 8 of
+// 1,024 x 512, 4,096 rows 16.6 and 8.4; 64 of 128 x 512, 64 rows 7.7 and 5.6, 8,192 10.4 and 6.5.
+bool by_blocks(int rows, int E, int N, int K, bool gated) {
+  const int experts = rows < E ? rows : E;
+  const long long cols = (N + (gated || N <= 128 ? 127 : 255)) / (gated || N <= 128 ? 128 : 256);
+  const long long blocks = (rows / 128 + (experts + 1) / 2) * cols;
+  if (blocks > (!gated && K <= 512 ? 2 * SMS : SMS)) return false;
+  if (gated) return (rows / 256 + experts / 2) * cols > SMS / 2;
+  return N <= 128 || rows >= 96LL * E;
+}
+
+template <Form FORM, int BN>
+int launch_blocks(bf16* C, const bf16* A, const bf16* W, const int* offsets, int rows, int E, int N, int K, const float* row_weights,
+                  float limit, float slope, int* error, cudaStream_t stream) {
+  constexpr bool GATED = FORM == SILU || FORM == CLAMPED;
+  CUtensorMap map_a, map_w;
+  int rc = make_map_bf16(&map_a, A, rows, K, K, 128);
+  if (rc) return rc;
+  rc = make_map_bf16(&map_w, W, (long long)E * N * (GATED ? 2 : 1), K, K, 128);
+  if (rc) return rc;
+  auto kern = grouped_block_kernel<FORM, BN>;
+  const cudaError_t set = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem<BN>());
+  if (set != cudaSuccess) return (int)set;
+  constexpr int BC = GATED ? BN / 2 : BN;
+  const long long row_tiles = rows / 128 + (rows < E ? rows : E);  // an expert leaves at most one tile partly filled
+  if (row_tiles > 65535) return -3;
+  return (int)launch_pdl(kern, dim3((unsigned)((N + BC - 1) / BC), (unsigned)row_tiles), dim3(BLOCK_THREADS), block_smem<BN>(), stream, map_a,
+                         map_w, C, offsets, E, N, K, row_weights, limit, slope, error);
+}
+
+template <Form FORM, bool SHORT>
+int launch_pairs(bf16* C, const bf16* A, const bf16* W, const int* offsets, int rows, int E, int N, int K, const float* row_weights,
+                 float limit, float slope, int* error, cudaStream_t stream) {
+  constexpr int most = SHORT ? SHORT_ROWS : 256;
   constexpr bool GATED = FORM == SILU || FORM == CLAMPED;
   RowMaps maps_a;
   CUtensorMap map_w;
@@ -364,18 +535,19 @@ int launch_grouped(bf16* C, const bf16* A, const bf16* W, const int* offsets, in
 
 // C [rows, N] = act(A [rows, K] W_e^T) over the experts' rows (offsets int32 [E + 1] on the device; rows is the most there
 // can be). act: -1 none, 5 squared relu. N and K multiples of 8, K at least 64, 16-byte aligned bases. `gated`: W [E, 2N, K],
-// act 0 (silu) or 3 (clamped swish with its limit and slope), row_weights [rows] or null. `tall` 1: tiles of up to 256 of an
-// expert's rows; 0: of 128, which fetches the weights of experts with more rows twice; 2: a single-token step's, of 32.
+// act 0 (silu) or 3 (clamped swish with its limit and slope), row_weights [rows] or null. `route` 0: pairs of blocks; 1: pairs or
+// single blocks, by sizes; 2: a single-token step's tiles.
 KRK_API int krk_grouped_gemm(void* C, const void* A, const void* W, const int* offsets, int rows, int E, int N, int K, int act,
-                             int gated, int tall, const float* row_weights, float limit, float slope, int* error,
+                             int gated, int route, const float* row_weights, float limit, float slope, int* error,
                              cudaStream_t stream) {
   if (rows == 0 || N == 0 || E == 0) return 0;
   if (N % 8 || K % 8 || K < 64 || (((uintptr_t)A | (uintptr_t)W | (uintptr_t)C) & 15) || 2LL * E * N > 0x7fffffffLL) return -2;
   if (gated ? (act != 0 && act != 3) : ((act != -1 && act != 5) || row_weights)) return -2;
-  const Form form = gated ? (act == 3 ? CLAMPED : SILU) : (act == 5 ? SQUARED : PLAIN);
-  auto go = tall == 2 ? (form == CLAMPED ? launch_grouped<CLAMPED, true> : form == SILU ? launch_grouped<SILU, true>
-                         : form == SQUARED ? launch_grouped<SQUARED, true> : launch_grouped<PLAIN, true>)
-                      : (form == CLAMPED ? launch_grouped<CLAMPED> : form == SILU ? launch_grouped<SILU>
-                         : form == SQUARED ? launch_grouped<SQUARED> : launch_grouped<PLAIN>);
-  return go((bf16*)C, (const bf16*)A, (const bf16*)W, offsets, rows, E, N, K, tall, row_weights, limit, slope, error, stream);
+  auto with = [&](auto go) { return go((bf16*)C, (const bf16*)A, (const bf16*)W, offsets, rows, E, N, K, row_weights, limit, slope, error, stream); };
+  const bool blocks = route == 1 && by_blocks(rows, E, N, K, gated), narrow = N <= 128, single = route == 2;
+  if (gated && act == 3) return with(blocks ? launch_blocks<CLAMPED, 256> : single ? launch_pairs<CLAMPED, true> : launch_pairs<CLAMPED, false>);
+  if (gated) return with(blocks ? launch_blocks<SILU, 256> : single ? launch_pairs<SILU, true> : launch_pairs<SILU, false>);
+  if (act == 5)
+    return with(blocks ? (narrow ? launch_blocks<SQUARED, 128> : launch_blocks<SQUARED, 256>) : single ? launch_pairs<SQUARED, true> : launch_pairs<SQUARED, false>);
+  return with(blocks ? (narrow ? launch_blocks<PLAIN, 128> : launch_blocks<PLAIN, 256>) : single ? launch_pairs<PLAIN, true> : launch_pairs<PLAIN, false>);
 }

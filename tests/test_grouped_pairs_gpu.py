@@ -1,5 +1,6 @@
 """The grouped products of the routed experts at the edges of their tiles: rows of an expert around multiples of 32 and 256,
-more experts than a warp has lanes, empty ones, and widths at which the second block of a pair has part of a tile or nothing."""
+more experts than a warp has lanes, empty ones, and widths at which the second block of a pair has part of a tile or nothing; by pairs of
+blocks, by single ones and in a single-token step's small tiles."""
 
 import pytest
 import torch
@@ -166,3 +167,28 @@ def test_single_token_tiles_at_their_edges(N, K, counts, gated):
     # one rounding of the result, gated of either product too (a gate's through silu's slope, at most 1.1)
     assert ((outs[0] - outs[1]).abs() <= (3.1 if gated else 1.0) * 2.0 ** -7 * outs[0].abs() + (2.0 ** -7 if gated else 1e-4)).all()
     assert (outs[1][rows:] == 7.0).all()
+
+
+@pytest.mark.parametrize("gated, act", [(0, -1), (0, 5), (1, 0), (1, 3)])
+@pytest.mark.parametrize("E, N, K, rows", [(8, 512, 128, 4100), (40, 128, 72, 500), (40, 72, 200, 3000), (8, 328, 640, 900), (4, 1032, 136, 2100)])
+def test_single_blocks_and_pairs_are_the_same_bits(E, N, K, rows, gated, act):
+    """Products of few tiles take single blocks (of these all plain ones, of the gated ones the first and the last): the same bits as by
+    pairs, row weights and an expert without rows among them."""
+    from kernel_rush_kawk_b200.csrc import load_kernels
+
+    ops = load_kernels((), "cuda:0")
+    g = torch.Generator().manual_seed(7)
+    counts = torch.bincount(torch.randint(0, E - 1, (rows,), generator=g), minlength=E)
+    offsets = torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)]).int().cuda()
+    a = torch.randn(rows, K, generator=g).to(torch.bfloat16).cuda()
+    w = (torch.randn(E, (2 if gated else 1) * N, K, generator=g) * K ** -0.5).to(torch.bfloat16).cuda()
+    weights = torch.rand(rows, generator=g).cuda() if act == 3 else None
+    outs = []
+    for route in (0, 1):
+        out = torch.full((rows, N), 7.0, dtype=torch.bfloat16, device="cuda")
+        ops._ok(ops.moe.krk_grouped_gemm(out.data_ptr(), a.data_ptr(), w.data_ptr(), offsets.data_ptr(), rows, E, N, K, act, gated, route,
+                                         None if weights is None else weights.data_ptr(), 7.0, 1.702, ops.error.data_ptr(), ops._stream()),
+                "grouped product")
+        outs.append(out)
+    ops.check()
+    assert torch.equal(*outs)
