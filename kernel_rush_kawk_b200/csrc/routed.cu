@@ -437,7 +437,12 @@ moe_gather_row_kernel(T* __restrict__ xg, const T* __restrict__ x, int x_stride,
   }
 }
 
-template <typename T>
+// AHEAD chosen experts' pieces in flight a thread: eight while all blocks share the SMs by threes, which is what eight's registers allow and
+// where one block's chain of loads is the time (rows of 2,048, six experts: 128 rows 2.8 us by four, 2.4 by eight, 384 rows 3.3 and 3.0), four
+// beyond (512 rows 3.9 and 4.5 us; 4,096 rows of 1,024, two experts, 13.7 and 19.7).
+constexpr int COMBINE_FEW_ROWS = 3 * 148;
+
+template <typename T, int AHEAD>
 __global__ void moe_combine_kernel(T* __restrict__ out, const T* __restrict__ add, const float* __restrict__ add_gate, const T* __restrict__ yg,
                                    const int* __restrict__ place, const int* __restrict__ experts,
                                    const int* __restrict__ offsets, int cap, const float* __restrict__ weights, int top,
@@ -454,7 +459,7 @@ __global__ void moe_combine_kernel(T* __restrict__ out, const T* __restrict__ ad
   if (sizeof(T) == 2 && (C & 7) == 0 && (x_stride & 7) == 0 &&
       ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(add) | reinterpret_cast<uintptr_t>(yg) |
         reinterpret_cast<uintptr_t>(x)) & 15) == 0) {
-    // eight columns a thread, eight chosen experts' pieces in flight; the sum in the order of the choice
+    // eight columns a thread; the sum in the order of the choice
     const float ag = add ? (add_gate ? add_gate[row] : 1.f) : 0.f, px = passed ? passed[row] : 0.f;
     auto fma8 = [](float (&t)[8], float w, const uint4& raw) {
       const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
@@ -465,13 +470,13 @@ __global__ void moe_combine_kernel(T* __restrict__ out, const T* __restrict__ ad
       float t[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       if (add) fma8(t, ag, *reinterpret_cast<const uint4*>(add + (size_t)row * C + c));
       if (passed) fma8(t, px, *reinterpret_cast<const uint4*>(x + (size_t)row * x_stride + c));
-      for (int j0 = 0; j0 < top; j0 += 8) {
-        uint4 raw[8];
+      for (int j0 = 0; j0 < top; j0 += AHEAD) {
+        uint4 raw[AHEAD];
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
+        for (int q = 0; q < AHEAD; ++q)
           if (j0 + q < top && src_row[j0 + q] >= 0) raw[q] = *reinterpret_cast<const uint4*>(yg + (size_t)src_row[j0 + q] * C + c);
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
+        for (int q = 0; q < AHEAD; ++q)
           if (j0 + q < top && src_row[j0 + q] >= 0) fma8(t, src_w[j0 + q], raw[q]);
       }
       uint4 o;
@@ -604,8 +609,8 @@ KRK_API int krk_moe_combine(void* out, const void* add, const float* add_gate, c
   if (rows == 0) return 0;
   if (top > 32) return -2;
   if (dtype == KRK_DTYPE_F32)
-    return (int)launch_pdl(moe_combine_kernel<float>, dim3(rows), dim3(256), 0, stream, (float*)out, (const float*)add, add_gate,
+    return (int)launch_pdl(moe_combine_kernel<float, 4>, dim3(rows), dim3(256), 0, stream, (float*)out, (const float*)add, add_gate,
                            (const float*)yg, place, experts, offsets, cap, weights, top, C, (const float*)x, x_stride, passed);
-  return (int)launch_pdl(moe_combine_kernel<bf16>, dim3(rows), dim3(256), 0, stream, (bf16*)out, (const bf16*)add, add_gate,
+  return (int)launch_pdl(rows <= COMBINE_FEW_ROWS ? moe_combine_kernel<bf16, 8> : moe_combine_kernel<bf16, 4>, dim3(rows), dim3(256), 0, stream, (bf16*)out, (const bf16*)add, add_gate,
                          (const bf16*)yg, place, experts, offsets, cap, weights, top, C, (const bf16*)x, x_stride, passed);
 }

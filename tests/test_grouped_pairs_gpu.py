@@ -192,3 +192,30 @@ def test_single_blocks_and_pairs_are_the_same_bits(E, N, K, rows, gated, act):
         outs.append(out)
     ops.check()
     assert torch.equal(*outs)
+
+
+@pytest.mark.parametrize("top, C", [(1, 64), (3, 72), (8, 2056), (11, 128)])
+def test_the_sum_of_many_rows_is_that_of_few(top, C):
+    """A row's chosen results added four or eight at a time: the same bits in a step of 445 rows as in one of 444, in the order of the choice."""
+    from kernel_rush_kawk_b200.csrc import load_kernels
+
+    ops = load_kernels((), "cuda:0")
+    g = torch.Generator().manual_seed(8)
+    rows, E = 445, 16
+    x, yg = torch.randn(rows, C, generator=g).to(torch.bfloat16), torch.randn(rows * top, C, generator=g).to(torch.bfloat16)
+    experts = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(rows)]).int()
+    experts[torch.rand(rows, top, generator=g) < 0.1] = -1
+    weights, passed = torch.rand(rows, top, generator=g), torch.rand(rows, generator=g)
+    want = passed[:, None].double() * x.double()
+    for j in range(top):
+        want += torch.where(experts[:, j] < 0, 0.0, weights[:, j])[:, None].double() * yg.view(rows, top, C)[:, j].double()
+    x_d, y_d, e_d, w_d, p_d = x.cuda(), yg.cuda(), experts.cuda(), weights.cuda(), passed.cuda()
+    outs = []
+    for n in (rows, rows - 1):
+        out = torch.empty((rows, C), dtype=torch.bfloat16, device="cuda")
+        ops._ok(ops.moe.krk_moe_combine(out.data_ptr(), None, None, y_d.data_ptr(), None, e_d.data_ptr(), None, 0, w_d.data_ptr(), n, top, C,
+                                        x_d.data_ptr(), C, p_d.data_ptr(), 1, ops._stream()), "experts' sum")
+        outs.append(out[:rows - 1])
+    assert torch.equal(*outs)
+    # one rounding to bfloat16, and float32 sums of up to twelve products of order one
+    assert ((outs[0].double().cpu() - want[:-1]).abs() <= 1.01 * 2.0 ** -8 * want[:-1].abs() + 1e-5).all()
