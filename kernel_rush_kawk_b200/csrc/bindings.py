@@ -904,8 +904,9 @@ class Kernels:
         w_in, w_out = (weights, None) if weigh_input else (None, weights)  # which end of an expert the weights multiply
         single = batch is not None and batch.is_decode  # such a step may be replayed from a graph: nothing comes to the host
         by_expert = self._few_experts(x, w_gate_up, w_down, rows, top)
-        if by_expert and self._use_grouped(x, K, F, C, gated, activation):
-            few = rows * top < self._grouped_from(E, F, C, gated)
+        if self._use_grouped(x, K, F, C, gated, activation) and (
+                by_expert or rows * top > self.FEW_EXPERTS_PAIRS and top <= 32 and (w_gate_up.data_ptr() | w_down.data_ptr()) % 16 == 0):
+            few = by_expert and rows * top < self._grouped_from(E, F, C, gated)
         else:
             few = single or rows * top <= max(self.MOE_PAIR_ROWS * top, 2 * E)
         if few:
@@ -929,8 +930,8 @@ class Kernels:
                                                  experts.data_ptr(), _ptr(w_out), rows, top, C, F, ptr, stride,
                                                  _ptr(add_input), _code(x.dtype), self._stream()), "experts' down")
             return out
-        # many rows: ordered by expert on the device; the experts' row counts come to the host (a step of many
-        # tokens is never replayed from a graph)
+        # many rows: ordered by expert on the device, where the grouped launches, which single-token steps may take, find the experts'
+        # row counts; for the other products they come to the host (a step of many tokens is never replayed from a graph)
         offsets = torch.empty(E + 1, dtype=torch.int32, device=x.device)
         place = torch.empty(rows * top, dtype=torch.int32, device=x.device)
         self._ok(self.moe.krk_moe_sort(offsets.data_ptr(), place.data_ptr(), experts.data_ptr(), rows, top, E,
@@ -966,6 +967,8 @@ class Kernels:
                                           _ptr(add_input), _code(x.dtype), self._stream()), "experts' sum")
         return out
 
+    FEW_EXPERTS_PAIRS = 4096  # that krk_few_experts takes
+
     @staticmethod
     def _few_experts(x, w_first, w_down, rows, top) -> bool:
         """Whether the experts' products of few rows run once per expert (csrc/few_experts.cu): type, sizes, the alignment of rows
@@ -973,7 +976,7 @@ class Kernels:
         27.3 us by pair and 30.8 by expert, 4 pairs 41.5 and 46.2, 8 pairs 68 and 58; 64 of 2,048 x 1,408, six a row: 6 pairs
         54 and 50)."""
         return (x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and w_down.shape[2] % 8 == 0 and x.stride(0) % 8 == 0
-                and (x.data_ptr() | w_first.data_ptr() | w_down.data_ptr()) % 16 == 0 and top <= 32 and 6 <= rows * top <= 4096)
+                and (x.data_ptr() | w_first.data_ptr() | w_down.data_ptr()) % 16 == 0 and top <= 32 and 6 <= rows * top <= Kernels.FEW_EXPERTS_PAIRS)
 
     @staticmethod
     def _grouped_from(E, F, C, gated) -> int:

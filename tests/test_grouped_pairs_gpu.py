@@ -219,3 +219,67 @@ def test_the_sum_of_many_rows_is_that_of_few(top, C):
     assert torch.equal(*outs)
     # one rounding to bfloat16, and float32 sums of up to twelve products of order one
     assert ((outs[0].double().cpu() - want[:-1]).abs() <= 1.01 * 2.0 ** -8 * want[:-1].abs() + 1e-5).all()
+
+
+def test_single_token_steps_of_more_pairs_than_a_piece_holds(monkeypatch):
+    """From 4,097 pairs on the kernel that reads an expert's weights once for its rows is out of bounds; the grouped launches, which take
+    steps of fewer pairs, take those too, and the sums are as near 64 bits as by pairs, each of which reads its expert's weights itself."""
+    from types import SimpleNamespace
+
+    from kernel_rush_kawk_b200.csrc import load_kernels
+
+    ops = load_kernels((), "cuda:0")
+    g = torch.Generator().manual_seed(9)
+    E, top, F, K, C = 32, 6, 96, 128, 72
+    w1, w2 = (torch.randn(E, 2 * F, K, generator=g) * K ** -0.5).to(torch.bfloat16), (torch.randn(E, C, F, generator=g) * F ** -0.5).to(torch.bfloat16)
+    grouped = []
+    gemm = ops._grouped_experts
+    monkeypatch.setattr(ops, "_grouped_experts", lambda *a: grouped.append(a[-1]) or gemm(*a))
+    for rows in (682, 683):  # 4,092 and 4,098 pairs
+        x = torch.randn(rows, K, generator=g).to(torch.bfloat16)
+        experts = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(rows)]).int()
+        weights = torch.rand(rows, top, generator=g)
+        y = torch.einsum("rk,enk->ren", x.double(), w1.double())
+        h = y[..., :F] * torch.sigmoid(y[..., :F]) * y[..., F:]
+        each = torch.einsum("ref,ecf->rec", h, w2.double())
+        want = (each.gather(1, experts.long()[..., None].expand(-1, -1, C)) * weights.double()[..., None]).sum(1)
+        got = ops.moe_experts(x.cuda(), w1.cuda(), w2.cuda(), experts.cuda(), weights.cuda(), F, "silu", batch=SimpleNamespace(is_decode=True))
+        off = (got.double().cpu() - want).norm() / want.norm()
+        # gate, up, their product, each expert's result and the sum are rounded: five times 2^-9 in the mean, added in squares
+        assert off < 5 ** 0.5 * 2.0 ** -8, (rows, float(off))
+    ops.check()
+    assert grouped == [2, 2], "both by the grouped launches, in a single-token step's tiles"
+
+
+def test_a_captured_step_of_the_grouped_experts():
+    """A single-token step by the grouped launches, captured and replayed over other rows, choices and weights: what the direct call returns."""
+    from types import SimpleNamespace
+
+    from kernel_rush_kawk_b200.csrc import load_kernels
+
+    ops = load_kernels((), "cuda:0")
+    g = torch.Generator().manual_seed(10)
+    E, top, F, K, C, rows = 64, 6, 640, 128, 1280, 40
+    w1, w2 = ((torch.randn(s, generator=g) * 0.06).to(torch.bfloat16).cuda() for s in ((E, 2 * F, K), (E, C, F)))
+
+    def inputs():
+        return (torch.randn(rows, K, generator=g).to(torch.bfloat16).cuda(),
+                torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(rows)]).int().cuda(), torch.rand(rows, top, generator=g).cuda())
+
+    step = lambda x, experts, weights: ops.moe_experts(x, w1, w2, experts, weights, F, "silu", batch=SimpleNamespace(is_decode=True))
+    assert rows * top >= ops._grouped_from(E, F, C, True)
+    held = inputs()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        step(*held)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = step(*held)
+    for _ in range(3):
+        fresh = inputs()
+        for a, b in zip(held, fresh):
+            a.copy_(b)
+        graph.replay()
+        assert torch.equal(out, step(*fresh))
+    ops.check()
