@@ -981,13 +981,21 @@ class Kernels:
     @staticmethod
     def _grouped_from(E, F, C, gated) -> int:
         """Pairs from which the two grouped launches, which need the pairs ordered and their rows gathered first, are faster than a
-        block per 32 rows of an expert's matrix. Those read an expert's weights once for sixteen of its rows, at 4.9 TB/s; the
-        grouped ones stream them at 6 where their tiles, of 128 or 256 columns, fill the 74 pairs of blocks some four times
-        (64 experts of 2,048 x 1,408, six a row, a single-token step: 16 rows 160 us and 157, 24 rows 197 and 186, 64 rows 216 and
-        190, 128 rows 252 and 192) and not where the second product is a round and a half (16 of 1,536 x 3,072, two a row: 16
-        rows 74 and 94, 64 rows 98 and 104, 128 rows 124 and 106)."""
+        block per 32 rows of an expert's matrix. Those read an expert's weights once for sixteen of its rows, at 4.9 TB/s where a
+        block has 64 KB of them and more; the grouped ones stream them at 6 where their tiles, of 128 or 256 columns, fill the rounds
+        of 74 pairs of blocks. Pairs an expert at which they meet in a single-token step, and both sides below and above:
+        128 experts of 768 x 2,048 (tiles 768) 0.6: at 0.5 101 and 106 us, 1 161 and 142; 64 of 1,408 x 2,048 (512) 0.6: 0.75 117 and
+        114, 3 193 and 183, 6 216 and 188; 32 of 2,048 x 1,024 (128, two rounds nearly full) 2.2: 2 78 and 81, 6 97 and 85; 32 of
+        768 x 1,536 (192) 10: 8 56 and 61, 12 67 and 61; 16 of 3,072 x 1,536 (96) 11: 8 91 and 103, 12 109 and 104; 16 of 1,024 x
+        1,024 13, of 512 x 1,024 17, 8 of 2,048 x 1,024 16. Blocks of 20 to 40 KB in many rounds of their own: 128 of 128 x 1,024 1: 4
+        58 and 48, 8 68 and 49; 64 of 256 x 1,024 5: 4 39 and 41, 8 45 and 42; not 64 of 128 x 512, 1,280 blocks in all, 12."""
         tiles = E * min(-(-F // (128 if gated else 256)), -(-C // 256))
-        return 9 * E // 4 if tiles >= 296 else 12 * E
+        if tiles >= 296:
+            return 9 * E // 4
+        blocks, size = E * -(-(F + C) // 32), 2 * E * F * C * (3 if gated else 2)
+        if (tiles >= 111 and size >= 300e6) or (blocks >= 16 * 148 and size < 65536 * blocks):
+            return 5 * E
+        return 12 * E
 
     @staticmethod
     def _use_grouped(x, K, F, C, gated, activation) -> bool:

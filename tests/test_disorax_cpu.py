@@ -134,3 +134,13 @@ def test_unequal_batch_against_each_alone(folders):
         for i, (s, ids) in enumerate(live):
             ref = plain_logits(folders["da"], ids)
             assert_logits(got[i:i + 1], ref[len(ids) - back:len(ids) - back + 1], "float32", f"batched token of sequence {i}")
+
+
+@pytest.mark.parametrize("E, F, C, below, above", [
+    (128, 768, 2048, 0.5, 3), (64, 1408, 2048, 0.375, 3), (32, 2048, 1024, 2, 6), (32, 768, 1536, 8, 16), (16, 3072, 1536, 8, 16),
+    (128, 128, 1024, 0.75, 8), (64, 256, 1024, 4, 8), (64, 128, 512, 6, 12)])
+def test_where_the_grouped_launches_begin(E, F, C, below, above):
+    """Pairs an expert at which the products by pieces were measured the faster ones, and at which the grouped launches were."""
+    from kernel_rush_kawk_b200.csrc.bindings import Kernels
+
+    assert below * E < Kernels._grouped_from(E, F, C, True) <= above * E
