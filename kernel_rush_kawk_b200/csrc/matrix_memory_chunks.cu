@@ -879,8 +879,8 @@ __global__ void __launch_bounds__(256) steps_kernel(Step* __restrict__ steps, co
                                                     const int* __restrict__ cu_q, const int* __restrict__ seq_qlen) {
   grid_launch_dependents();
   grid_dependency_wait();
-  const int lane = threadIdx.x & 31, h = blockIdx.x * 8 + (threadIdx.x >> 5), seq = blockIdx.z;
-  const int first = blockIdx.y * L, nt = min(L, seq_qlen[seq] - first);
+  const int lane = threadIdx.x & 31, h = blockIdx.y * 8 + (threadIdx.x >> 5), seq = blockIdx.z;
+  const int first = blockIdx.x * L, nt = min(L, seq_qlen[seq] - first);
   if (nt <= 0 || h >= H) return;
   const size_t row0 = (size_t)cu_q[seq] + first;
   const float b = bias[h], rate = expf(a_log[h]);
@@ -1032,8 +1032,8 @@ KRK_API int krk_ssd_steps(float* steps, const void* dt, int dt_stride, const flo
                           int n_seqs, int max_q_len, const int* cu_q, const int* seq_qlen, cudaStream_t stream) {
   if (rows == 0 || n_seqs == 0 || max_q_len == 0) return 0;
   const int chunks = (max_q_len + L - 1) / L;
-  if (chunks > 65535 || n_seqs > 65535 || ((uintptr_t)steps & 15)) return -2;
-  return (int)launch_pdl(steps_kernel, dim3((unsigned)((H + 7) / 8), (unsigned)chunks, (unsigned)n_seqs), dim3(256), 0, stream, (Step*)steps,
+  if (H > 8 * 65535 || n_seqs > 65535 || ((uintptr_t)steps & 15)) return -2;
+  return (int)launch_pdl(steps_kernel, dim3((unsigned)chunks, (unsigned)((H + 7) / 8), (unsigned)n_seqs), dim3(256), 0, stream, (Step*)steps,
                          (const bf16*)dt, dt_stride, dt_bias, a_log, rows, H, cu_q, seq_qlen);
 }
 

@@ -263,6 +263,24 @@ def test_state_space_scans_of_many_heads(shape, lens, monkeypatch):
     assert torch.equal(state[clean], chunks[1][clean]) and not torch.isfinite(state[~clean]).any()
 
 
+def test_step_sizes_of_a_prompt_of_millions(monkeypatch):
+    """4,194,305 tokens of one head are 65,537 chunks, more than a grid has rows: their step sizes and summed decays all the same (the scan itself
+    goes through them in portions)."""
+    rt = runtime(torch.bfloat16)
+    rows, L = 65536 * 64 + 1, 64
+    dt = torch.linspace(-3, 1, 64).repeat(65537)[:rows].to(torch.bfloat16).cuda()
+    one = torch.zeros(1, device="cuda")
+    steps = torch.empty((rows, 4), dtype=torch.float32, device="cuda")
+    cu, qlen = (torch.tensor(t, dtype=torch.int32, device="cuda") for t in ([0, rows], [rows]))
+    rt.ops._ok(rt.ops.memory.krk_ssd_steps(steps.data_ptr(), dt.data_ptr(), 1, one.data_ptr(), one.data_ptr(), rows, 1, 1, rows, cu.data_ptr(),
+                                           qlen.data_ptr(), rt.ops._stream()), "step sizes and decays")
+    whole = steps[:-1].view(-1, L, 4)
+    d = torch.nn.functional.softplus(dt[:L].float())
+    assert torch.equal(whole, whole[:1].expand_as(whole))
+    assert ((steps[:L, 2] - d).abs() <= 1e-6 * d).all() and ((steps[-1, 2] - d[0]).abs() <= 1e-6 * d[0]) and torch.isfinite(steps[-1]).all()
+    assert torch.equal(steps[-1, 2:3], steps[-1, 3:]), "the last token's weight is its step size: nothing comes after it"
+
+
 def test_a_state_space_token_after_its_decay(monkeypatch):
     """One token in front of a chunk, alone: what is left of it later in the chunk is e^d times it, d the difference of two sums of 64
     bits rounded once, so off by a rounding of d: a unit of its last place over the root of 12. A difference rounded twice would be off by
