@@ -106,7 +106,8 @@ causal_conv4_kernel(T* __restrict__ out, const T* __restrict__ in, int in_stride
     for (int j = 0; j < 4; ++j) load_run<float, 4>(w + (size_t)j * ch + c + i, wj[j] + i);
   }
   grid_dependency_wait();
-  const int r0 = blockIdx.y * CONV_ROWS;
+  const int r0 = (blockIdx.z * gridDim.y + blockIdx.y) * CONV_ROWS;
+  if (r0 >= rows) return;
   Run<T, V> now[CONV_ROWS], at[4];  // this thread's rows; inputs of the three tokens before and of this one
 #pragma unroll
   for (int u = 0; u < CONV_ROWS; ++u)
@@ -568,8 +569,9 @@ KRK_API int krk_causal_conv_silu(void* out, const void* in, int in_stride, const
                    (((uintptr_t)in | (uintptr_t)out | (uintptr_t)tail | (uintptr_t)w | (uintptr_t)bias) & 15) == 0;
   const int vcols = min(64, (ch / V + threads - 1) / threads);
   int rc;
-  if (vec && taps == 4 && walk && rows <= 65535 * CONV_ROWS) {
-    const dim3 grid((ch / V + 63) / 64, (rows + CONV_ROWS - 1) / CONV_ROWS);
+  if (vec && taps == 4 && walk) {
+    const int runs = (rows + CONV_ROWS - 1) / CONV_ROWS, layers = (runs + 65534) / 65535;  // of the grid, which has 65,535 rows
+    const dim3 grid((ch / V + 63) / 64, (runs + layers - 1) / layers, layers);
     if (dtype == KRK_DTYPE_F32)
       rc = (int)launch_pdl(causal_conv4_kernel<float>, grid, dim3(64), 0, stream, (float*)out, (const float*)in, in_stride, w, bias,
                            (const float*)tail, ch, rows, row_seq, cu_q, seq_slot);

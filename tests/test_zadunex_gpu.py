@@ -345,6 +345,23 @@ def test_convolution_rows_in_runs_and_one_by_one(dtype, lens, walks, monkeypatch
     assert torch.equal(got, want) and torch.equal(tails[0], tails[1])
 
 
+def test_convolution_of_more_runs_of_rows_than_a_grid_has(monkeypatch):
+    """A step of 524,300 rows, 65,538 runs of eight: the same bits as a block a row."""
+    rt = runtime(torch.bfloat16)
+    ch, lens = 8, [524000, 300]
+    x = rand((sum(lens), ch), 50).to(torch.bfloat16).cuda()
+    w, b, tail = rand((4, ch), 51).cuda(), rand((ch,), 52).cuda(), rand((2, 3, ch), 53).to(torch.bfloat16).cuda()
+    batch = SimpleNamespace(n_seqs=2, row_seq=torch.repeat_interleave(torch.arange(2), torch.tensor(lens)).int().cuda(),
+                            cu_q=torch.tensor([0, lens[0], sum(lens)], dtype=torch.int32, device="cuda"),
+                            seq_qlen=torch.tensor(lens, dtype=torch.int32, device="cuda"), seq_slot=torch.tensor([1, 0], dtype=torch.int32, device="cuda"))
+    runs = []
+    for walks in (True, False):
+        monkeypatch.setattr(type(rt.ops), "_conv_walks", lambda *_, walks=walks: walks)
+        stored = tail.clone()
+        runs.append((rt.ops.causal_conv_silu(x, w, b, stored, batch), stored))
+    assert all(torch.equal(a, b) for a, b in zip(*runs))
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n", [4, 32, 124, 256, 260, 768, 772, 1024, 1028])
 def test_gated_norm_of_parts_of_any_size(dtype, n):
