@@ -1519,16 +1519,15 @@ class Kernels:
     # -- state-space mixer ------------------------------------------------------------------
     SSD_CHUNK = 128  # tokens per chunk where one sequence's step is long enough to be scanned in chunks
 
-    CONV_WALK_BYTES = 8_400_000
+    CONV_WALK_BYTES = 3_500_000
 
     def _conv_walks(self, rows, row_bytes, n_seqs) -> bool:
         """Whether threads of the short convolution go through eight rows each, the rows before in registers. That is one chain of
         6 us at least, at a sequence's first row with the loads of its stored rows in it, and pays by bytes: a block a row and
-        eight rows a thread, one prompt of 4,096 channels in bfloat16, with the stored rows' update, 64 rows 5.1 and 6.2 us, 256 6.7
-        and 6.7, 512 8.5 and 7.6, 1,024 12.5 and 10.4, 2,048 22.3 and 15.7; of 1,792 channels 512 rows 6.4 and 7.0, 1,024 8.1 and
-        7.5, 2,048 11.6 and 10.2; 32-bit of 4,096 channels 256 rows 6.9 and 7.3, 512 9.5 and 7.8. So one long sequence's two kernels meet
-        between 2 and 5 MB; the line lies above, at 1,024 rows of 4,096 channels, for steps of many short sequences, whose
-        first rows each wait for their stored ones."""
+        eight rows a thread, with the stored rows' update, one prompt of 4,096 channels in bfloat16, 64 rows 5.2 and 6.1 us, 256 6.8
+        and 6.6, 512 8.5 and 7.5, 1,024 12.5 and 9.7, 2,048 22.3 and 14.9; of 1,792 channels 512 rows 6.5 and 6.9, 1,024 8.2 and
+        7.3; 32-bit of 4,096 channels 128 rows 5.3 and 6.5, 256 6.9 and 6.8, 512 9.4 and 8.3. Sequences of 1,024 rows in all: of 128
+        rows 12.6 and 10.3, 16 rows 17.2 and 14.8, 4 rows 32.3 and 30.6, 2 rows 54 and 54; single tokens 96 and 101."""
         return rows * row_bytes >= self.CONV_WALK_BYTES and rows >= 2 * n_seqs
 
     def causal_conv_silu(self, x, w, b, tail, batch):

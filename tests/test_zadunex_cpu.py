@@ -144,13 +144,16 @@ def test_unequal_batch_against_each_alone_and_a_slot_used_again(folders):
 
 
 def test_which_steps_go_through_the_convolutions_rows_in_runs():
-    """By bytes, and never single tokens of many sequences: a run of rows is one chain, which short steps would wait for."""
+    """By bytes, and never single tokens of many sequences: a run of rows is one chain, which short steps would wait for. On either side of
+    the line, sizes at which that side was measured the faster one."""
     from kernel_rush_kawk_b200.csrc.bindings import Kernels
 
     walks = lambda n_seqs, rows, row_bytes: Kernels._conv_walks(Kernels, rows, row_bytes, n_seqs)
     assert not any(walks(n, n, 8192) for n in (1, 63, 64, 65, 200, 2048, 4096))
-    assert not any(walks(1, rows, 8192) for rows in (64, 100, 512, 1024)) and not walks(1, 2048, 3584) and not walks(64, 1024, 8192)
+    assert not any(walks(1, rows, 8192) for rows in (64, 100, 256)) and not walks(1, 512, 3584) and not walks(1, 128, 16384)
+    assert walks(1, 512, 8192) and walks(1, 1024, 8192) and walks(1, 2048, 3584) and walks(64, 1024, 8192) and walks(1, 512, 16384)
     assert walks(1, 2048, 8192) and walks(3, 2553, 8192) and walks(1, 1024, 16384) and walks(64, 4096, 8192)
+    assert [walks(1, rows, 8192) for rows in range(1, 3000)] == sorted(walks(1, rows, 8192) for rows in range(1, 3000)), "one line"
 
 
 def test_few_norm_parts_take_a_block_each():

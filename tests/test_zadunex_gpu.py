@@ -308,7 +308,7 @@ def test_a_state_space_token_after_its_decay(monkeypatch):
 
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_convolution_of_many_rows(dtype, monkeypatch):
-    """Rows in runs of sixteen a thread, four taps: sequences that start anywhere in a run, shorter than the taps, channels
+    """Rows in runs of eight a thread, four taps: sequences that start anywhere in a run, shorter than the taps, channels
     that fill no block. The same bits as the kernel of single elements, which rows off a 16-byte boundary take."""
     rt = runtime(dtype)
     monkeypatch.setattr(type(rt.ops), "_conv_walks", lambda *_: True)
@@ -330,7 +330,7 @@ def test_convolution_of_many_rows(dtype, monkeypatch):
 @pytest.mark.parametrize("lens", [[1] * 70, [1] * 64 + [500], [15, 1, 2, 33, 48, 7], [3, 17, 300, 1, 16, 64]])
 def test_convolution_rows_in_runs_and_one_by_one(dtype, lens, walks, monkeypatch):
     """Whichever kernel a step takes: the same bits as the kernel of single elements, outputs and stored inputs, with sequences that start
-    anywhere in a thread's sixteen rows."""
+    anywhere in a thread's eight rows."""
     rt = runtime(dtype)
     monkeypatch.setattr(type(rt.ops), "_conv_walks", lambda *_: walks)
     ch, rows = 520, sum(lens)
