@@ -1331,7 +1331,7 @@ class Kernels:
                                           int(self._shift_walks(rows, C, batch.n_seqs))), "token shift")
         return out
 
-    RECURRENCE_CHUNK_MIN = 160  # tokens of a step's longest sequence from which a bfloat16 scan of such mixers may run in chunks
+    RECURRENCE_CHUNK_MIN = 128  # tokens of a step's longest sequence from which a bfloat16 scan of such mixers may run in chunks
     RECURRENCE_SCRATCH = 256 << 20  # bytes
     CHUNK_SCRATCH_MOST = 1 << 30    # a step of so many sequences that one chunk of each takes more is scanned token by token
 
@@ -1347,20 +1347,22 @@ class Kernels:
         return None, 0
 
     def _recurrence_in_chunks(self, kind, heads, batch) -> bool:
-        """Where the scan in chunks pays. It takes more launches, and a short step is bound by issuing them from the host, so the
-        lines lie by the time of a whole mixer as it is called. Time mixing, token by token and in chunks: one sequence of
-        200 tokens at 24 heads 188 us and 198, of 350 210 and 197; four of 200 at 40 heads 229 and 206. The delta rule: one
-        sequence of 110 at 8 heads 134 us and 145, of 200 173 and 143. The delta rule has more work a chunk: where sequences
-        and heads fill the SMs, the scan token by token keeps up (8 heads, 16 sequences of 128: 145 us against 157), so the
-        two are also estimated from their measured parts: 0.57 us a token for each round of blocks, against 0.18 us a chunk
-        and head, 0.5 us a chunk of the longest sequence and 12 us."""
+        """Where the scan in chunks pays. It takes more launches, and a short step among others is bound by issuing them from the host,
+        so the lines lie by the time of a whole mixer as it is called, token by token and in chunks (alone, with the device waited
+        for, chunks are ahead from 64 tokens on). Time mixing: one sequence of 192 tokens at 24 heads 154 us and 162, of 256 160 and 162,
+        of 320 184 and 162, at 40 heads of 192 155 and 165, of 256 177 and 164; four at 40 heads, of 128 164 and 171, of 192 193 and 166.
+        The delta rule: one sequence at 8 heads, of 96 tokens 109 and 118, of 128 118 and 118, of 160 140 and 119; at 16 heads of 128 132
+        and 119; four at 8 heads of 96 109 and 119, of 128 130 and 121. It has more work a chunk: where sequences and heads fill the
+        SMs, the scan token by token keeps up (on the device, 8 heads, 16 sequences of 128: 85 us and 91, of 256 158 and 172, of 512 304
+        and 305; 16 heads, 8 of 200 125 and 154), so the two are also estimated from their measured parts: 0.6 us a token for each
+        round of blocks, against 0.15 us a chunk and head, 0.5 us a chunk of the longest sequence and 12 us."""
         longest = batch.max_q_len
         if longest < self.RECURRENCE_CHUNK_MIN:
             return False
         if kind == "wkv":
-            return longest >= (192 if batch.n_seqs * heads > 148 else 320)
+            return longest >= (160 if batch.n_seqs * heads > 148 else 256)
         items = heads * sum(-(-n // 32) for n in batch.q_lens)
-        return 0.57 * longest * -(-batch.n_seqs * heads // 148) > 12.0 + 0.18 * items + 0.5 * longest / 32
+        return 0.6 * longest * -(-batch.n_seqs * heads // 148) > 12.0 + 0.15 * items + 0.5 * longest / 32
 
     def linear_recurrence(self, kind, r, k, v, gate, lora, w2, w0, heads, dim, norm_w, eps, state, batch, out, out_col,
                           out_scale, rate=None, rate_bias=None, decay_scale=1.0, bonus=None, last_rows=None):
@@ -1578,10 +1580,10 @@ class Kernels:
         return y
 
     # tokens of a step's longest sequence from which a bfloat16 scan runs in chunks on the tensor cores. The kernels alone gain
-    # from 64 tokens on, but a short step is bound by the host, which has more launches to issue (48 heads of 64 x 128, a whole
-    # mixer as it is called: one sequence of 110 tokens 123 us by the other scan and 151 in chunks, of 200 161 and 152, of 700
-    # 241 and 154; four of 110 127 and 154, of 200 183 and 155)
-    SSD_TENSOR_MIN = 192
+    # from 64 tokens on, but a short step among others is bound by the host, which has more launches to issue (48 heads of 64 x 128, a
+    # whole mixer as it is called: one sequence of 128 tokens 104 us by the other scan and 122 in chunks, of 160 130 and 122, of 192 151
+    # and 122, of 256 212 and 122; four of 96 106 and 125, of 128 132 and 127, of 200 186 and 126)
+    SSD_TENSOR_MIN = 160
     SSD_SCRATCH = 256 << 20  # bytes of chunk states
 
     def _ssd_chunks(self, views, dt_bias, a_log, skip, heads, P, N, groups, state, batch, y, tokens) -> bool:
