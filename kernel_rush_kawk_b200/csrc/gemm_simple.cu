@@ -16,8 +16,8 @@
 //   Packed multiply-adds (fma.rn.f32x2) were measured and are slower here (274 to 294 us): the copies that pair an
 //   operand with itself cost more than the pipe's register reads gain.
 // * gemm_f32_few: up to 16 float32 rows. Bound by the weights' bytes: each is read once, by asynchronous 16-byte copies
-//   a slice ahead; a thread owns one or two output columns of one or two rows. One row of 151,936 x 2,560: 241 us,
-//   6.5 TB/s; three rows 262 us, of 2,560 x 4,096 22 us, where the chain of K multiply-adds is the bound (the general kernel: 1.9 ms and 570 us).
+//   a slice ahead; a thread owns one or two output columns of one or two rows. One row of 151,936 x 2,560: 235 us,
+//   6.6 TB/s; three rows 258 us, of 2,560 x 4,096 21 us, where the chain of K multiply-adds is the bound (the general kernel: 1.9 ms and 570 us).
 // * gemm_nt: everything else (bfloat16 inputs with float32 output at odd sizes, for output-head logits at many
 //   positions; float32 rows whose size or alignment does not allow 16-byte accesses). 64x64 output tile, k in slices of
 //   16, 256 threads with a 4x4 micro-tile each.
@@ -207,7 +207,7 @@ gemm_f32_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const f
 // the columns' weights and of the rows, and the next one is on its way while one is multiplied. What an SM has in flight is a matter of how
 // many blocks it holds, not of how deep each one's ring is: with two slices of 256 k, 35 KB a block at one row, five or six
 // blocks share an SM; six slices of 128 left room for three, whose waits and chains did not cover each other (three rows of 151,936
-// x 2,560 367 us, now 262; 16 rows of 19,456 x 2,560 114 and 101). Beyond 8 rows, where shared-memory reads are the
+// x 2,560 355 us, now 258; 16 rows of 19,456 x 2,560 113 and 98). Beyond 8 rows, where shared-memory reads are the
 // bound, a thread's two rows of two columns read half as much for a multiply-add as one of one.
 constexpr int FEW_K = 256, FEW_PITCH = FEW_K + 4, FEW_DEPTH = 2;
 
@@ -336,6 +336,9 @@ int launch_few(float* C, const float* A, const float* W, int M, int N, int K, in
 int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
   if (M == 0 || N == 0) return 0;
   if (K < 4 || K % 4 || lda % 4 || ldw % 4 || (((uintptr_t)A | (uintptr_t)W | (uintptr_t)C) & 15)) return -2;
+  // 16 rows: 98 us of 19,456 x 2,560 and 161 by the tiles below, 558 and 647 of 151,936 x 2,560, 2.5 and 4.0 of 128 x 64
+  if (M <= 8) return launch_few<1, 1>(C, A, W, M, N, K, lda, ldw, ldc, stream);
+  if (M <= 16) return launch_few<2, 2>(C, A, W, M, N, K, lda, ldw, ldc, stream);
   // Cycles per k on the busiest SM, from the times measured at 17 to 1,024 rows of five matrices: a block alone is bound by
   // its own latency (the first number), several by what a block takes of the SM.
   auto cost = [&](int tm, int tn, int alone, int each) {
@@ -345,9 +348,6 @@ int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, in
   };
   const long long c22 = cost(64, 128, 120, 89), c21 = cost(64, 64, 88, 47), c12 = cost(32, 128, 96, 49);
   const long long best = min(c22, min(c21, c12));
-  if (M <= 8) return launch_few<1, 1>(C, A, W, M, N, K, lda, ldw, ldc, stream);
-  // 9 to 16 rows: 17 cycles a block (101 us at 16 rows of 19,456 x 2,560 against the tiles' 192; 740 against 641 at 151,936)
-  if (M <= 16 && ((long long)(N + 31) / 32 + 147) / 148 * 17 <= best) return launch_few<2, 2>(C, A, W, M, N, K, lda, ldw, ldc, stream);
   if (best == c22) return launch_tile<2, 2>(C, A, W, M, N, K, lda, ldw, ldc, stream);
   if (best == c21) return launch_tile<2, 1>(C, A, W, M, N, K, lda, ldw, ldc, stream);
   return launch_tile<1, 2>(C, A, W, M, N, K, lda, ldw, ldc, stream);
