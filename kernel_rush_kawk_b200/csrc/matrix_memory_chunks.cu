@@ -21,8 +21,8 @@
 // one number per head and token, and x_s counts dt_s times: A_ts = (C_t . B_s) e^{F_t - F_s} dt_s, r_t = e^{F_t}, w_s = e^{F_last - F_s} dt_s,
 // plus skip * x_t in the output. Its log decays are as large as the step sizes make them, so they are summed, kept and subtracted in
 // 64-bit: e^{F_t - F_s} is then as exact as the product of the decays that the scan token by token forms. One prompt of 2,048
-// tokens, 48 heads of 64 with 128 rows: the scan's three passes on the CUDA cores 403 us, these 90 (22, 16 and 50; 114 with a block
-// a head: 31, 16 and 66).
+// tokens, 48 heads of 64 with 128 rows: the scan's three passes on the CUDA cores 403 us, these 97 (25, 30 and 57, each from a
+// cold cache; 111 with a block a head).
 //
 // Three passes: (1) every chunk's own sum_s (w_s k_s) v_s^T; (2) the walk over a sequence's chunks, which leaves every
 // chunk its starting state and the sequence its final one; (3) the outputs. A block takes some slices of 64 value

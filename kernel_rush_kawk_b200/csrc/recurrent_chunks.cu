@@ -25,9 +25,10 @@
 // its starting state in G's place and the sequence its final one; (3) per (sequence, chunk, head) the outputs with their norm,
 // weight and gate. Chunks of 32: a chunk of 64 needs twice the multiply-adds a token in pass 1 and halves the walk's steps.
 //
-// Measured: one prompt of 2,048 tokens, delta rule of 8 heads, 1,171 -> 95 us (the passes 50, 34 and 11); three prompts of
-// 2,553 tokens in all, time mixing of 40 heads, 405 -> 128 us (45, 15, 68; with float32 on the CUDA cores 57, 15 and 115). Passes 1
-// and 3 are bound by instruction issue and latencies (a 0.4 to 0.5 share of the issue slots, 12 to 32 warps an SM), the walk by the chain of its steps.
+// Measured: one prompt of 2,048 tokens, delta rule of 8 heads, 1,171 us token by token, 110 here (the passes 57, 36 and 17, each from a
+// cold cache); three prompts of 2,553 tokens in all, time mixing of 40 heads, 405 -> 117 us (48, 17 and 66; with float32 on the
+// CUDA cores 175). Passes 1 and 3 are bound by instruction issue and latencies (a 0.4 to 0.5 share of the issue slots, 12 to 32 warps an
+// SM), the walk by the chain of its steps.
 //
 // e^{-c_s} must stay in range. The delta rule's decay is at least e^{-decay_scale} a token, so a chunk's is bounded by the
 // parameter (the caller asks krk_recurrence_chunk_tokens). Time mixing's has no bound: a chunk in which some channel decays by
@@ -169,8 +170,8 @@ __device__ __forceinline__ void small33(float (&d)[4], const uint32_t (&x)[3][4]
 // Eight warps. A thread makes one channel of eight tokens' rows; six warps multiply [U; Rows] [K; A]^T, a warp four tiles of 16 x 8; four
 // solve for a column of [X | Z] a thread, with float32 multiply-adds, while the other four multiply K^T V; then four multiply A^T X
 // and four A^T Z, and all of them eight columns of Q and O each. X and Z are kept with their signs turned.
-// Two blocks an SM. Bound by its chains and barriers, the substitution's before all. One prompt of 2,048 tokens, 8 heads: 50 us (with
-// float32 on the CUDA cores, three blocks of four warps an SM, 63).
+// Two blocks an SM. Bound by its chains and barriers, the substitution's before all. One prompt of 2,048 tokens, 8 heads: 50 us (57 from
+// a cold cache; with float32 on the CUDA cores, three blocks of four warps an SM, 63).
 __global__ void __launch_bounds__(DELTA_THREADS, 2) delta_chunk_kernel(ChunkArgs a) {
   extern __shared__ __align__(16) float sm[];
   constexpr int TERM = L * KP, ROWS3 = 3 * TERM;       // elements of one term of a chunk's rows, of three
@@ -812,7 +813,7 @@ __global__ void __launch_bounds__(THREADS) delta_finish_kernel(ChunkArgs a) {
 
 // ---- pass 3, time mixing ---------------------------------------------------------------------------------------
 // Bound by what surrounds the products: loads, exponentials, splitting and barriers; the tensor cores are busy a quarter of the time. Five
-// blocks an SM (six spill: 84 us against 72 at 3 sequences of 2,553 tokens, 40 heads; the float32 form 115). A warp makes 16 value columns of all tokens. Of a warp's 16 columns the even ones are one tile of the products and the odd ones
+// blocks an SM (six spill: 84 us against 72 in one measurement, 3 sequences of 2,553 tokens, 40 heads; the float32 form 115). A warp makes 16 value columns of all tokens. Of a warp's 16 columns the even ones are one tile of the products and the odd ones
 // another: a row's piece of the state is then one 8-byte load for both, and a thread ends with four neighbouring columns.
 __global__ void __launch_bounds__(THREADS, 5) mix_finish_kernel(ChunkArgs a) {
   extern __shared__ __align__(16) float sm[];
