@@ -984,14 +984,16 @@ class Kernels:
         block per 32 rows of an expert's matrix. Those read an expert's weights once for sixteen of its rows, at 4.9 TB/s where a
         block has 64 KB of them and more; the grouped ones stream them at 6 where their tiles, of 128 or 256 columns, fill the rounds
         of 74 pairs of blocks. Pairs an expert at which they meet in a single-token step, and both sides below and above:
-        128 experts of 768 x 2,048 (tiles 768) 0.6: at 0.5 101 and 106 us, 1 161 and 142; 64 of 1,408 x 2,048 (512) 0.6: 0.75 117 and
-        114, 3 193 and 183, 6 216 and 188; 32 of 2,048 x 1,024 (128, two rounds nearly full) 2.2: 2 78 and 81, 6 97 and 85; 32 of
-        768 x 1,536 (192) 10: 8 56 and 61, 12 67 and 61; 16 of 3,072 x 1,536 (96) 11: 8 91 and 103, 12 109 and 104; 16 of 1,024 x
-        1,024 13, of 512 x 1,024 17, 8 of 2,048 x 1,024 16. Blocks of 20 to 40 KB in many rounds of their own: 128 of 128 x 1,024 1: 4
-        58 and 48, 8 68 and 49; 64 of 256 x 1,024 5: 4 39 and 41, 8 45 and 42; not 64 of 128 x 512, 1,280 blocks in all, 12."""
+        128 experts of 768 x 2,048 (tiles 768) 0.6: at 0.5 101 and 106 us, 1 161 and 142; 128 of 512 x 1,024 (512) 0.75: 0.5 49 and 53,
+        1 78 and 71; 64 of 1,408 x 2,048 (512) 0.6: 0.75 117 and 114, 3 193 and 183, 6 216 and 188; 64 of 768 x 1,536 (384) 4.5: 3 89
+        and 92, 9 118 and 100; 64 of 640 x 1,280 (320) 4: 3 73 and 78, 4.5 80 and 78, 9 93 and 78; 48 of 1,024 x 1,536 (288) 5;
+        32 of 1,536 x 2,048 (256) 7, of 3,072 x 2,048 (256) 0.9, of 2,048 x 1,024 (128, two rounds nearly full) 2.2: 2 78 and 81, 6 97
+        and 85; of 768 x 1,536 (192) 10: 8 56 and 61, 12 67 and 61; 16 of 3,072 x 1,536 (96) 11: 8 91 and 103, 12 109 and 104; 16
+        of 1,024 x 1,024 13, of 512 x 1,024 17, 8 of 2,048 x 1,024 16. Blocks of 20 to 40 KB in many rounds of their own: 128 of 128 x
+        1,024 1: 4 58 and 48, 8 68 and 49; 64 of 256 x 1,024 5: 4 39 and 41, 8 45 and 42; not 64 of 128 x 512, 1,280 blocks in all, 12."""
         tiles = E * min(-(-F // (128 if gated else 256)), -(-C // 256))
-        if tiles >= 296:
-            return 9 * E // 4
+        if tiles >= 296:  # four rounds; six
+            return E if tiles >= 444 else 9 * E // 2
         blocks, size = E * -(-(F + C) // 32), 2 * E * F * C * (3 if gated else 2)
         if (tiles >= 111 and size >= 300e6) or (blocks >= 16 * 148 and size < 65536 * blocks):
             return 5 * E
