@@ -470,16 +470,18 @@ grouped_block_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 }
 
 // Whether single blocks are the faster ones: where their tiles, an expert's last one half filled, are one round over the SMs (two of a
-// short k), and the pairs' larger ones would be a second round that is nearly empty (gated, whose epilogue takes a single block's lanes longer), or
-// leave SMs idle: an expert's rows are a tile's or nearly, or its columns half of one. Pairs and blocks, us: gated, 8 experts of 512 x 1,024,
-// 2,048 rows 13.9 and 17.1, 4,096 rows 20.8 and 13.4, of 16 22.2 and 35.7; plain, 16 of 512 x 1,024, 1,024 rows 10.4 and 11.2, 2,048 11.9
-// and 10.3, 4,096 14.5 and 11.7, 8,192 21.4 and 14.2; 16 of 1,024 x 512, 8,192 rows 23.7 and 18.7; of 1,024 x 1,024 27.8 and 26.7; 8 of
-// 1,024 x 512, 4,096 rows 16.6 and 8.4; 64 of 128 x 512, 64 rows 7.7 and 5.6, 8,192 10.4 and 6.5.
+// short k, or of up to 1,024 where the second is nearly full), and the pairs' larger ones would be a second round that is nearly empty
+// (gated, whose epilogue takes a single block's lanes longer), or leave SMs idle: an expert's rows are a tile's or nearly, or its
+// columns half of one. Pairs and blocks, us: gated, 8 experts of 512 x 1,024, 2,048 rows 13.9 and 17.1, 4,096 rows 20.8 and 13.4, of 16
+// 22.2 and 35.7; plain, 16 of 512 x 1,024, 1,024 rows 10.4 and 11.2, 2,048 11.9 and 10.3, 4,096 14.5 and 11.7, 8,192 21.4 and 14.2; 16
+// of 1,024 x 512, 8,192 rows 23.7 and 18.7; of 1,024 x 1,024, 4,096 rows 23.2 and 24.4, 8,192 27.8 and 25.4; 8 of 1,024 x 512,
+// 4,096 rows 16.6 and 8.4; 64 of 128 x 512, 64 rows 7.7 and 5.6, 8,192 10.4 and 6.5.
 bool by_blocks(int rows, int E, int N, int K, bool gated) {
   const int experts = rows < E ? rows : E;
   const long long cols = (N + (gated || N <= 128 ? 127 : 255)) / (gated || N <= 128 ? 128 : 256);
   const long long blocks = (rows / 128 + (experts + 1) / 2) * cols;
-  if (blocks > (!gated && K <= 512 ? 2 * SMS : SMS)) return false;
+  const bool second = !gated && (K <= 512 || (K <= 1024 && blocks > 9 * SMS / 5));
+  if (blocks > (second ? 2 * SMS : SMS)) return false;
   if (gated) return (rows / 256 + experts / 2) * cols > SMS / 2;
   return N <= 128 || rows >= 96LL * E;
 }
