@@ -6,13 +6,21 @@
 //   64 columns of S_t (two keys per 32-bit column) and is the A operand of O_t += P_t V.
 //   shared memory: Q0, Q1, and K and V double-buffered (128-byte swizzle, filled by TMA).
 //
-// Warps 0..7 run the softmax of tile 0 and of tile 1 in turn (thread = query row = tensor-memory lane,
-// and one half of the block's keys: warps w and w + 4 share their rows); lane 0 of warp 8 issues every
-// MMA (lane 0 of warp 9 the TMA loads), in the order
+// Warps 0..3 run the softmax of tile 0 and warps 4..7 that of tile 1 (thread = query row = tensor-memory lane, all 128 keys
+// of a block); lane 0 of warp 8 issues every MMA, lane 0 of warp 9 the TMA loads, in the order
 //   ... PV0(j-1) QK0(j) PV1(j-1) QK1(j) PV0(j) QK0(j+1) ...
-// so that while one tile's rows are in the softmax the tensor core works for the other tile. A tile's
-// next MMAs wait for its softmax, so all eight warps on one tile (half the time per block) shorten the
-// chain that bounds the kernel: softmax of a block, its P V, the next block's Q K^T.
+// so that while one tile's rows are in the softmax the tensor core works for the other tile.
+//
+// What bounds it is a tile's chain: softmax of a block, its P V, the next block's Q K^T (tensor memory has no room for a
+// second S per tile). Per block of 128 keys a tile spends 1,800 clocks in the softmax (reading S 50, maximum 370,
+// exponentials and packing 1,260 where the special-function unit alone takes 1,024, storing P 120), 1,030 in its 16 MMAs and
+// about 600 on the barriers between them. A thread keeps its 128 scores in registers: the softmax warps take 216 each and the
+// other four warps 72 (setmaxnreg; of the 168 that 384 threads start with). With 168 the compiler spilled some 100 bytes a
+// thread, and the exponentials took 2,000 clocks, twice the rate of the unit, in every arrangement of the warps that was
+// tried; a path of its own for blocks that some row sees in part cost as much (the compiler moved the exponentials of both
+// paths in front of the branch), so scores that a row does not see become minus infinity first and there is one path.
+// 2,048 tokens, 32 heads in groups of four: 45 us (49 before); four prompts of 957 to 1,531, 40 heads in groups of five:
+// 120 (167, of which two thirds of the difference are the query tiles, which come by TMA at any group size now).
 // Per key block of 128 keys (two cache pages) and tile:
 //   S = Q K^T                                   [issuer]   -> s_full
 //   row max; p = exp2(S*c - m) rounded to bfloat16 -> tensor memory  [softmax]  -> p_ready
@@ -35,8 +43,9 @@
 // sink, sum 1, no value); rows of the output may lie apart, are multiplied by a number and by the sigmoid of a gate per head or
 // per element. SHAPED: scores are capped
 // (c tanh(s / c) = c (1 - 2 / (1 + e^(2 s / c)))) and lose a slope times the distance of query and key before the softmax.
-// 2,048 tokens, a window of 1,024, 16 heads of 128 in groups of four: 45 us against the mma.sync kernel's 116 (of 37 at that
-// instruction's measured rate, 550 TFLOP/s, for 19 GFLOP); 12 heads in groups of three, no slopes, 46 against 75.
+// 2,048 tokens, a window of 1,024, 16 heads of 128 in groups of four: 37 us (45 with the softmax of both tiles in all eight
+// warps; the mma.sync kernel 116, of 37 at that instruction's measured rate, 550 TFLOP/s, for 19 GFLOP); 12 heads in groups of
+// three, no slopes, 39 (43; 75).
 //
 // Compiled once per head size, for head sizes 64 and 128: -DKRK_HEAD_DIM=<D>.
 #include "tcgen05.cuh"
@@ -53,11 +62,9 @@ using namespace tc;
 
 constexpr int D = KRK_HEAD_DIM;
 constexpr int ROWS = 128;              // query rows per tile
-constexpr int PAIR = 2 * ROWS;         // query rows per block
 constexpr int KEYS = 128;              // keys per block iteration: two pages
-constexpr int HALF = KEYS / 2;         // score columns a softmax thread holds at a time
 constexpr int DB = D / 64;             // 64-wide blocks of the head dimension
-constexpr int THREADS = 320;           // 8 softmax warps, the warp that issues the MMAs, the warp that loads
+constexpr int THREADS = 384;           // 8 softmax warps, the warps that issue the MMAs, load and allocate, one idle
 constexpr uint32_t SUB = 128 * 128;    // bytes of a [128 rows x 64 bf16] swizzled sub-tile
 constexpr uint32_t TILE_BYTES = DB * SUB;  // a Q, K or V tile
 constexpr uint32_t TMEM_COLS = 512;
@@ -82,11 +89,11 @@ struct TileRange {
   __device__ __forceinline__ bool has(int j) const { return j >= lo && j <= hi; }
 };
 
-__device__ __forceinline__ TileRange tile_range(int row_begin, int n_rows, int G, int q_len, int start, int window) {
+__device__ __forceinline__ TileRange tile_range(int row_begin, int rows, int n_rows, int G, int q_len, int start, int window) {
   TileRange t;
   if (row_begin >= n_rows) { t.lo = 1; t.hi = 0; return t; }
   const int first_tok = row_begin / G;
-  const int last_tok = min(q_len - 1, (row_begin + ROWS - 1) / G);
+  const int last_tok = min(q_len - 1, (row_begin + rows - 1) / G);
   t.lo = window > 0 ? max(0, start + first_tok - window + 1) / KEYS : 0;
   t.hi = (start + last_tok) / KEYS;
   return t;
@@ -96,8 +103,8 @@ __device__ __forceinline__ TileRange tile_range(int row_begin, int n_rows, int G
 __device__ __forceinline__ int first_page(int row_begin, int G, int start, int window) {
   return window > 0 ? max(0, start + row_begin / G - window + 1) / KRK_PAGE : 0;
 }
-__device__ __forceinline__ int last_page(int row_begin, int G, int q_len, int start) {
-  return (start + min(q_len - 1, (row_begin + ROWS - 1) / G)) / KRK_PAGE;
+__device__ __forceinline__ int last_page(int row_begin, int rows, int G, int q_len, int start) {
+  return (start + min(q_len - 1, (row_begin + rows - 1) / G)) / KRK_PAGE;
 }
 
 // What the wide form adds; see the opening text.
@@ -110,13 +117,14 @@ struct Extras {
   int out_stride;
 };
 
-template <bool WIDE, bool SHAPED>
+template <bool WIDE, int SHAPE>
 __global__ void __launch_bounds__(THREADS, 1)
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                         const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_o, int q_by_tma, bf16* __restrict__ out, const bf16* __restrict__ qkv, int q_stride, int HQ, int HKV,
+                         const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_o, int q_by_tma, int rows, bf16* __restrict__ out, const bf16* __restrict__ qkv, int q_stride, int HQ, int HKV,
                          const int* __restrict__ seq_slot, const int* __restrict__ seq_start,
                          const int* __restrict__ seq_qlen, const int* __restrict__ cu_q, const int* __restrict__ table,
                          int width, float scale_log2, int window, int* __restrict__ error, const Extras ex) {
+  constexpr bool SHAPED = SHAPE != 0;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* q_s = base;                    // two tiles
@@ -125,9 +133,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
   uint64_t* bars = reinterpret_cast<uint64_t*>(v_s + 2 * TILE_BYTES);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + N_BARS);
   int* pages_s = reinterpret_cast<int*>(tmem_slot + 2);  // [PAGE_IDS] the block's page-table entries, from page 2 * j_lo on
-  float* xchg = reinterpret_cast<float*>(pages_s + PAGE_IDS);  // [2 copies][2 halves][ROWS] partial row maxima of the softmax warps
-  float* xsum = xchg + 4 * ROWS;                               // [2 tiles][2 halves][ROWS] their partial row sums
-  volatile int* gave_up = reinterpret_cast<volatile int*>(xsum + 4 * ROWS);  // [4] per pair of softmax warps
+  volatile int* gave_up = pages_s + PAGE_IDS;  // [2] per tile
 
   // blockIdx.x counts (row pair, kv head) with the pair as the slow index, descending: blocks start in
   // launch order, so the pairs with the most key blocks, of every kv head, run first and the short ones
@@ -135,14 +141,15 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
   const int seq = blockIdx.y, kh = blockIdx.x % HKV;
   const int pair = gridDim.x / HKV - 1 - blockIdx.x / HKV;
   const int G = HQ / HKV;
-  const int q_len = seq_qlen[seq];
+  // all four before the first is used: one trip to memory
+  const int q_len = seq_qlen[seq], start = seq_start[seq], slot = seq_slot[seq], row0 = cu_q[seq];
   const int n_rows = q_len * G;
-  if (pair * PAIR >= n_rows) return;
-  const int start = seq_start[seq], slot = seq_slot[seq], row0 = cu_q[seq];
+  const int pair_row = pair * 2 * rows;
+  if (pair_row >= n_rows) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  const TileRange r0 = tile_range(pair * PAIR, n_rows, G, q_len, start, window);
-  const TileRange r1 = tile_range(pair * PAIR + ROWS, n_rows, G, q_len, start, window);
+  const TileRange r0 = tile_range(pair_row, rows, n_rows, G, q_len, start, window);
+  const TileRange r1 = tile_range(pair_row + rows, rows, n_rows, G, q_len, start, window);
   const int j_lo = r0.lo;                                   // tile 0 exists and starts no later than tile 1
   const int j_hi = r1.lo <= r1.hi ? max(r0.hi, r1.hi) : r0.hi;
   const int n = j_hi - j_lo + 1;
@@ -163,6 +170,10 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
   auto load_k = [&](int i) { load_tile(k_s + (i & 1) * TILE_BYTES, &map_k, bars + K_FULL + (i & 1), i); };
   auto load_v = [&](int i) { load_tile(v_s + (i & 1) * TILE_BYTES, &map_v, bars + V_FULL + (i & 1), i); };
 
+  if (warp == 9 && lane < 4) {
+    const CUtensorMap* map = lane == 0 ? &map_k : lane == 1 ? &map_v : lane == 2 ? &map_q : &map_o;
+    asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+  }
   if (warp == 8) {
     // The block's first loads in the order of what they wait for: the error word and the page-table entries are
     // requested together, the query tiles (which need neither) go out before either has arrived.
@@ -176,18 +187,18 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
       page_here[q] = i < min(2 * n, PAGE_IDS) ? table[(size_t)slot * width + (2 * j_lo + i) % width] : 0;
     }
     if (lane == 0) {
-      for (int i = 0; i < N_BARS; ++i) mbar_init(bars + i, (i == P_READY || i == P_READY + 1) ? 2 * ROWS : 1);
+      for (int i = 0; i < N_BARS; ++i) mbar_init(bars + i, (i == P_READY || i == P_READY + 1) ? ROWS / 32 : 1);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-      for (int i = 0; i < 4; ++i) gave_up[i] = 0;
+      gave_up[0] = gave_up[1] = 0;
       if (q_by_tma) {
-        // a query tile is a box of 128 / G tokens x G heads x 64 dims per 64-wide block of the head: its rows
-        // land in (token, group member) order, which is the tile's row order
+        // a query tile is a box of whole tokens x G heads x 64 dims per 64-wide block of the head: its rows land in
+        // (token, group member) order, which is the tile's row order
         const int tiles_here = r1.lo <= r1.hi ? 2 : 1;
-        mbar_expect_tx(bars + Q_FULL, tiles_here * TILE_BYTES);
+        mbar_expect_tx(bars + Q_FULL, tiles_here * DB * rows * 128);
         for (int t = 0; t < tiles_here; ++t)
 #pragma unroll
           for (int h = 0; h < DB; ++h)
-            tma_load_3d(q_s + t * TILE_BYTES + h * SUB, &map_q, bars + Q_FULL, h * 64, kh * G, row0 + (pair * PAIR + t * ROWS) / G);
+            tma_load_3d(q_s + t * TILE_BYTES + h * SUB, &map_q, bars + Q_FULL, h * 64, kh * G, row0 + (pair_row + t * rows) / G);
       }
     }
 #pragma unroll
@@ -201,15 +212,15 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
       load_v(0);
       if (n > 1) load_k(1);
     }
-    __syncwarp();
+  } else if (warp == 10) {  // beside the loads of warp 8
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (!q_by_tma) {
     // the query tiles by hand: row r, 16-byte piece c -> swizzled K-major sub-tiles; rows past the end are zero
-    for (int i = threadIdx.x; i < PAIR * (D / 8); i += THREADS) {
+    for (int i = threadIdx.x; i < 2 * ROWS * (D / 8); i += THREADS) {
       const int r = i / (D / 8), c = i % (D / 8);
-      const int R = pair * PAIR + r;
+      const int R = pair_row + r;
       uint4 v = make_uint4(0, 0, 0, 0);
       if (R < n_rows) v = *reinterpret_cast<const uint4*>(qkv + (size_t)(row0 + R / G) * q_stride + (size_t)(kh * G + R % G) * D + c * 8);
       *reinterpret_cast<uint4*>(q_s + (r / ROWS) * TILE_BYTES + (c / 8) * SUB + swz(r % ROWS, c % 8)) = v;
@@ -224,7 +235,9 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
 
   if (dead) {
     // nothing to do
-  } else if (warp == 8) {
+  } else if (warp >= 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    if (warp == 8) {
     if (lane == 0) {
       // ---- issuer: TMA loads and MMAs ----
       constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(KEYS >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
@@ -281,8 +294,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
       if constexpr (WIDE) {  // here, while the first scores are on their way
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
-          skip_first[t] = first_page(pair * PAIR + t * ROWS, G, start, window) & 1;
-          skip_last[t] = !(last_page(pair * PAIR + t * ROWS, G, q_len, start) & 1);
+          skip_first[t] = first_page(pair_row + t * rows, G, start, window) & 1;
+          skip_last[t] = !(last_page(pair_row + t * rows, rows, G, q_len, start) & 1);
         }
       }
       for (int i = 0; i < n && ok; ++i) {
@@ -315,7 +328,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         }
       }
     }
-  } else if (warp == 9) {
+    } else if (warp == 9) {
     if (lane == 0) {
       // ---- loader: the TMA loads after the first ones. A thread of its own: issuing a load takes the time of
       // several MMAs, and the issuer's instruction stream is what bounds the kernel.
@@ -330,229 +343,216 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         }
       }
     }
+    }
   } else {
-    // ---- softmax: all eight warps work on one tile at a time, tile 0 and tile 1 in turn. Thread = query row r of
-    // both tiles (its tensor-memory lane) and one half of a block's keys: warps w and w + 4 share the rows
-    // 32 (w & 3) .. + 31 and exchange their partial row maxima (and, at the end, sums) through shared memory.
-    // A tile's block is through the softmax in half the time, which is what the other tile's MMAs wait for.
-    const int quad = warp & 3, half = warp >> 2;
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+    // ---- softmax: warps 0..3 have tile 0, warps 4..7 tile 1; thread = query row (its tensor-memory lane), whole key blocks.
+    const int t = warp >> 2, quad = warp & 3;
     const int r = quad * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
-    const TileRange rng[2] = {r0, r1};
-    bool valid[2];
-    int tok[2], pos[2], lo[2];
-    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, slope[2] = {0.f, 0.f};
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-      const int R = pair * PAIR + t * ROWS + r;
-      valid[t] = R < n_rows;
-      tok[t] = valid[t] ? R / G : 0;
-      pos[t] = valid[t] ? start + tok[t] : -1;  // -1: sees nothing
-      lo[t] = (valid[t] && window > 0) ? max(0, pos[t] - window + 1) : 0;
-      if constexpr (WIDE) {
-        const int head = kh * G + (valid[t] ? R % G : 0);
-        if (ex.sink) {
-          // a sink at minus infinity, or so low that it is in log2 units, is none: nothing is summed before the first key
-          m[t] = ex.sink[head] * LOG2E;
-          l[t] = half == 0 && m[t] != -INFINITY ? 1.f : 0.f;  // the two halves' sums are added at the end
-        }
-        if (SHAPED && ex.slopes) slope[t] = ex.slopes[head] * LOG2E;
+    const TileRange rng = t ? r1 : r0;
+    const uint32_t tmem_s = tmem + t * 128 + lane_addr, tmem_o = tmem + TMEM_O + t * D + lane_addr;
+    const int R = pair_row + t * rows + r;
+    const bool valid = r < rows && R < n_rows;
+    const int tok = valid ? R / G : 0;
+    const int pos = valid ? start + tok : -1;  // -1: sees nothing
+    const int low = (valid && window > 0) ? max(0, pos - window + 1) : 0;
+    const int head = kh * G + (valid ? R % G : 0);
+    float m = -INFINITY, slope = 0.f;
+    float2 l2 = make_float2(0.f, 0.f);
+    if constexpr (WIDE) {
+      if (ex.sink) {
+        // a sink at minus infinity, or so low that it is in log2 units, is none: nothing is summed before the first key
+        m = ex.sink[head] * LOG2E;
+        l2.x = m != -INFINITY ? 1.f : 0.f;
       }
+      if (SHAPED && ex.slopes) slope = ex.slopes[head] * LOG2E;
     }
-    auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory"); };
-    bool ok = true, stores_pending = false;
-    uint32_t step = 0;
-    for (int j = j_lo; j <= j_hi && ok; ++j) {
+    const float2 scale2 = make_float2(scale_log2, scale_log2);
+    const uint32_t unseen = scale_log2 < 0.f ? 0x7f800000u : 0xff800000u;  // a score whose weight is zero
+    bool ok = true;
+    for (int j = rng.lo; j <= rng.hi; ++j) {
+      const int key0 = j * KEYS;
+      // the row sees keys first..first + span of the block: (unsigned)(i - first) <= span; none of them: no i passes
+      const bool none = pos < max(low, key0);
+      const unsigned first = none ? (unsigned)KEYS : (unsigned)max(low - key0, 0);
+      const unsigned span = none ? 0u : (unsigned)(pos - key0) - first;
+      const bool whole = __all_sync(0xffffffffu, key0 + KEYS - 1 <= pos && key0 >= low);
+      // tensor-memory loads and stores are warp-wide: a warp gives up as a whole
+      if (!__all_sync(0xffffffffu, mbar_wait(bars + S_FULL + t, (j - rng.lo) & 1))) {
+        if (lane == 0) atomicExch(error, 12);
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      uint32_t s[KEYS];
 #pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        if (j < rng[t].lo || j > rng[t].hi) continue;  // the same for every thread of the block
-        const uint32_t c = (uint32_t)(j - rng[t].lo);
-        const int key0 = j * KEYS + half * HALF;  // this thread's first key
-        const uint32_t tmem_s = tmem + t * 128 + lane_addr;
-        const uint32_t tmem_o = tmem + TMEM_O + t * D + lane_addr;
-        float* xm = xchg + (step & 1) * 2 * ROWS;  // [half][row], two copies used in turn
-        ++step;
-        // the row sees keys first..first + span of its half: (unsigned)(i - first) <= span; none of them: no i passes
-        const bool whole = key0 + HALF - 1 <= pos[t] && key0 >= lo[t];
-        const bool none = pos[t] < max(lo[t], key0);
-        const unsigned first = none ? (unsigned)HALF : (unsigned)max(lo[t] - key0, 0);
-        const unsigned span = none ? 0u : (unsigned)(pos[t] - key0) - first;
-        // tensor-memory loads and stores are warp-wide, and the two warps of a row meet at a barrier that has no
-        // time limit: a warp that gives up says so in shared memory and both leave after the barrier
-        const bool arrived = __all_sync(0xffffffffu, mbar_wait(bars + S_FULL + t, c & 1));
-        uint32_t s[HALF];
-        float mx = -INFINITY;
-        if (arrived) {
-          tc_fence_after();
+      for (int q = 0; q < KEYS / 32; ++q) tmem_ld_32x32(tmem_s + 32 * q, *reinterpret_cast<uint32_t(*)[32]>(s + 32 * q));
+      tmem_wait_ld();
+      if constexpr (SHAPED) {  // in log2 units from here on; the slope's distance counted from the block's first key
+        const float away = slope * (float)(pos - key0);
+        const float2 slope2 = make_float2(slope, slope), away2 = make_float2(-away, -away);
 #pragma unroll
-          for (int q = 0; q < HALF / 32; ++q) tmem_ld_32x32(tmem_s + HALF * half + 32 * q, *reinterpret_cast<uint32_t(*)[32]>(s + 32 * q));
-          tmem_wait_ld();
-          if constexpr (SHAPED) {  // in log2 units from here on; the slope's distance counted from the half's first key
-            const float away = slope[t] * (float)(pos[t] - key0);
-            if (ex.in_cap > 0.f) {
-#pragma unroll
-              for (int i = 0; i < HALF; ++i) {
-                const float x = __uint_as_float(s[i]) * scale_log2;
-                const float y = ex.cap_log2 * (1.f - __fdividef(2.f, 1.f + fast_exp2(x * ex.in_cap)));
-                s[i] = __float_as_uint(fmaf(slope[t], (float)i, y - away));
-              }
-            } else {
-#pragma unroll
-              for (int i = 0; i < HALF; ++i)
-                s[i] = __float_as_uint(fmaf(slope[t], (float)i, fmaf(__uint_as_float(s[i]), scale_log2, -away)));
-            }
-          }
-          if (whole) {
-#pragma unroll
-            for (int i = 0; i < HALF; ++i) mx = fmaxf(mx, __uint_as_float(s[i]));
+        for (int i = 0; i < KEYS; i += 2) {
+          float2 x = make_float2(__uint_as_float(s[i]), __uint_as_float(s[i + 1]));
+          if constexpr (SHAPE == 2) {
+            x = __fmul2_rn(x, scale2);
+            x.x = ex.cap_log2 * (1.f - __fdividef(2.f, 1.f + fast_exp2(x.x * ex.in_cap)));
+            x.y = ex.cap_log2 * (1.f - __fdividef(2.f, 1.f + fast_exp2(x.y * ex.in_cap)));
+            x = __fadd2_rn(x, away2);
           } else {
-#pragma unroll
-            for (int i = 0; i < HALF; ++i)
-              if ((unsigned)i - first <= span) mx = fmaxf(mx, __uint_as_float(s[i]));
+            x = __ffma2_rn(x, scale2, away2);
           }
-          xm[half * ROWS + r] = mx;
-        } else if (lane == 0) {
-          atomicExch(error, 12);
-          gave_up[quad] = 1;
+          x = __ffma2_rn(slope2, make_float2((float)i, (float)(i + 1)), x);
+          s[i] = __float_as_uint(x.x);
+          s[i + 1] = __float_as_uint(x.y);
         }
-        pair_sync();
-        if (gave_up[quad]) { ok = false; break; }
-        mx = fmaxf(mx, xm[(half ^ 1) * ROWS + r]);
-        const float m_new = fmaxf(m[t], SHAPED ? mx : mx * scale_log2);
-        const bool outgrown = m[t] != -INFINITY && m_new - m[t] > RESCALE_STEP;
-        if (__any_sync(0xffffffffu, outgrown)) {
-          // the warp moves its rows' reference maxima (its partner, with the same rows and maxima, decides the
-          // same) and scales its half of the columns of O; the block's P.V has not been issued and the one
-          // before it is complete (S of this block came after it), so nothing else touches these rows of O
-          const float alpha = m[t] == -INFINITY ? 1.f : fast_exp2(m[t] - m_new);
-          // a row that starts from a sink may outgrow it in the tile's first block, when there is no O yet
+      }
+      if (!whole) {
 #pragma unroll
-          for (int c0 = 0; c0 < ((WIDE && c == 0) ? 0 : D / 2); c0 += 32) {
-            uint32_t o[32];
-            tmem_ld_32x32(tmem_o + half * (D / 2) + c0, o);
-            tmem_wait_ld();
+        for (int i = 0; i < KEYS; ++i)
+          if ((unsigned)i - first > span) s[i] = unseen;
+      }
+      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st_32x32(tmem_o + half * (D / 2) + c0, o);
-          }
-          l[t] *= alpha;
-          m[t] = m_new;
-        } else if (m[t] == -INFINITY) {
-          m[t] = m_new;  // no key seen before this block: O and l are still zero
+        for (int i = 0; i < KEYS; i += 8)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) mx4[q] = fmaxf(fmaxf(mx4[q], __uint_as_float(s[i + q])), __uint_as_float(s[i + 4 + q]));
+      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      const float m_new = fmaxf(m, SHAPED ? mx : mx * scale_log2);
+      const bool outgrown = m != -INFINITY && m_new - m > RESCALE_STEP;
+      if (__any_sync(0xffffffffu, outgrown)) {
+        // the warp moves its rows' reference maxima and scales its rows of O; the block's P.V has not been issued and the
+        // one before it is complete (S of this block came after it), so nothing else touches these rows of O
+        const float alpha = m == -INFINITY ? 1.f : fast_exp2(m - m_new);
+        // a row that starts from a sink may outgrow it in the tile's first block, when there is no O yet
+#pragma unroll 1
+        for (int c0 = 0; c0 < ((WIDE && j == rng.lo) ? 0 : D); c0 += 32) {
+          uint32_t o[32];
+          tmem_ld_32x32(tmem_o + c0, o);
+          tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          tmem_st_32x32(tmem_o + c0, o);
         }
-        const float m_safe = m[t] == -INFINITY ? 0.f : m[t];
-        float sum = 0.f;
-        uint32_t pk[HALF / 2], pl[WIDE ? HALF / 2 : 1];
-        auto weight = [&](int i) {
-          return fast_exp2(SHAPED ? __uint_as_float(s[i]) - m_safe : fmaf(__uint_as_float(s[i]), scale_log2, -m_safe));
-        };
-        auto keep = [&](int i, float p0, float p1) {
-          sum += p0 + p1;
-          const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
+        l2.x *= alpha;
+        l2.y *= alpha;
+        m = m_new;
+      } else if (m == -INFINITY) {
+        m = m_new;  // no key seen before this block: O and the sums are still zero
+      }
+      const float m_safe = m == -INFINITY ? 0.f : m;
+      const float2 minus_m = make_float2(-m_safe, -m_safe);
+#pragma unroll
+      for (int i0 = 0; i0 < KEYS; i0 += 32) {
+        uint32_t pk[16], pl[WIDE ? 16 : 1];
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          float2 x = make_float2(__uint_as_float(s[i0 + i]), __uint_as_float(s[i0 + i + 1]));
+          x = SHAPED ? __fadd2_rn(x, minus_m) : __ffma2_rn(x, scale2, minus_m);
+          const float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+          l2 = __fadd2_rn(l2, p);
+          const __nv_bfloat162 h = __floats2bfloat162_rn(p.x, p.y);
           const uint32_t hi = *reinterpret_cast<const uint32_t*>(&h);
           pk[i / 2] = hi;
           if constexpr (WIDE) {
-            const __nv_bfloat162 d = __floats2bfloat162_rn(p0 - __uint_as_float(hi << 16), p1 - __uint_as_float(hi & 0xffff0000u));
+            const float2 rest = __fadd2_rn(p, make_float2(-__uint_as_float(hi << 16), -__uint_as_float(hi & 0xffff0000u)));
+            const __nv_bfloat162 d = __floats2bfloat162_rn(rest.x, rest.y);
             pl[i / 2] = *reinterpret_cast<const uint32_t*>(&d);
           }
-        };
-        if (whole) {
-#pragma unroll
-          for (int i = 0; i < HALF; i += 2) keep(i, weight(i), weight(i + 1));
-        } else {
-#pragma unroll
-          for (int i = 0; i < HALF; i += 2)
-            keep(i, ((unsigned)i - first <= span) ? weight(i) : 0.f, ((unsigned)(i + 1) - first <= span) ? weight(i + 1) : 0.f);
         }
-        l[t] += sum;
-        __syncwarp();  // rows that see their whole half and rows at its edge took different paths
-        // P's second half lands on score columns of the partner warp, which holds them in registers since the barrier
-        tmem_st_32x32(tmem_s + (HALF / 2) * half, pk);
-        if constexpr (WIDE) tmem_st_32x32(tmem_s + HALF + (HALF / 2) * half, pl);
-        tmem_wait_st();
-        tc_fence_before();
-        mbar_arrive(bars + P_READY + t);
+        tmem_st_32x16(tmem_s + i0 / 2, pk);
+        if constexpr (WIDE) tmem_st_32x16(tmem_s + KEYS / 2 + i0 / 2, pl);
       }
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bars + P_READY + t);
     }
-    // the row's sum is the two halves' sums; every thread comes here exactly once, whatever happened before
-    xsum[half * ROWS + r] = l[0];
-    xsum[2 * ROWS + half * ROWS + r] = l[1];
-    pair_sync();
-    l[0] += xsum[(half ^ 1) * ROWS + r];
-    l[1] += xsum[2 * ROWS + (half ^ 1) * ROWS + r];
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-      if (rng[t].lo > rng[t].hi) continue;  // the same for every thread of the block
-      // O_t, divided by the row sums and rounded, goes through shared memory: a thread holds half a row, and rows
-      // are 2 * D bytes apart at best in the output. It is staged in the tile's query buffer, which its MMAs are
-      // done with, in the query tile's own layout (128-byte swizzle), and leaves as the query tile came: one
-      // tiled store per 64-wide block of the head when the tile is whole, else 16-byte pieces by all threads,
-      // consecutive threads storing consecutive pieces (the rows of a token lie side by side in the output).
+    if (rng.lo <= rng.hi) {  // the same for every thread of the tile's four warps
+      // O_t, divided by the row sums and rounded, goes through shared memory: a thread holds a row, and rows are 2 * D bytes
+      // apart at best in the output. It is staged in the tile's query buffer, which its MMAs are done with, in the query
+      // tile's own layout (128-byte swizzle), and leaves as the query tile came: one tiled store per 64-wide block of the
+      // head when the tile is whole, else 16-byte pieces by all threads of the tile, consecutive threads storing consecutive
+      // pieces (the rows of a token lie side by side in the output).
       const bool fine = ok && __all_sync(0xffffffffu, mbar_wait(bars + O_DONE + t, 0));
       unsigned char* stage = q_s + t * TILE_BYTES;
       if (fine) {
         tc_fence_after();
-        const uint32_t tmem_o = tmem + TMEM_O + t * D + lane_addr;
-        float inv = valid[t] ? (WIDE ? ex.out_scale : 1.0f) / l[t] : 0.f;
-        const bf16* gp = nullptr;  // this row's gates, one per element
-        if constexpr (WIDE) {
-          if (ex.gate_mode && valid[t]) {
-            const int head = kh * G + (pair * PAIR + t * ROWS + r) % G;
-            const bf16* g = ex.gate + (size_t)(row0 + tok[t]) * ex.gate_stride;
-            if (ex.gate_mode == 1) inv /= 1.0f + expf(-__bfloat162float(g[head]));
-            else gp = g + (size_t)head * D;
-          }
-        }
-#pragma unroll
-        for (int c0 = 0; c0 < D / 2; c0 += 32) {
-          uint32_t o[32];
-          tmem_ld_32x32(tmem_o + half * (D / 2) + c0, o);
-          tmem_wait_ld();
-#pragma unroll
-          for (int c = 0; c < 32; c += 8) {
-            if constexpr (WIDE) {
-              if (gp)
-#pragma unroll
-                for (int e = 0; e < 8; ++e)
-                  o[c + e] = __float_as_uint(__uint_as_float(o[c + e]) / (1.0f + expf(-__bfloat162float(gp[half * (D / 2) + c0 + c + e]))));
+        float inv = valid ? (WIDE ? ex.out_scale : 1.0f) / (l2.x + l2.y) : 0.f;
+        if (WIDE && ex.gate_mode == 1 && valid)
+          inv /= 1.0f + expf(-__bfloat162float(ex.gate[(size_t)(row0 + tok) * ex.gate_stride + head]));
+        if (WIDE && ex.gate_mode == 2) {
+          // a gate per element: eight columns at a time, a loop of its own (unrolled into the other one it was code of 50 KB
+          // that every block jumped over, 3 to 9 us)
+          const bf16* g = ex.gate + (size_t)(row0 + tok) * ex.gate_stride + (size_t)head * D;
+          const bool pieces = valid && ex.gate_stride % 8 == 0 && ((uintptr_t)ex.gate & 15) == 0;
+#pragma unroll 2
+          for (int c0 = 0; c0 < D; c0 += 8) {
+            uint32_t o[8];
+            tmem_ld_32x8(tmem_o + c0, o);
+            uint4 gv = make_uint4(0, 0, 0, 0);
+            if (pieces) gv = *reinterpret_cast<const uint4*>(g + c0);
+            else if (valid) {
+              bf16* e = reinterpret_cast<bf16*>(&gv);
+              for (int i = 0; i < 8; ++i) e[i] = g[c0 + i];
             }
+            tmem_wait_ld();
+            const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&gv);
             uint4 pk;
             __nv_bfloat162* pp = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-              pp[e] = __floats2bfloat162_rn(__uint_as_float(o[c + 2 * e]) * inv, __uint_as_float(o[c + 2 * e + 1]) * inv);
-            const int piece = (half * (D / 2) + c0 + c) / 8;
-            *reinterpret_cast<uint4*>(stage + (piece / 8) * SUB + swz(r, piece % 8)) = pk;
+              pp[e] = __floats2bfloat162_rn(__uint_as_float(o[2 * e]) / (1.0f + expf(-__low2float(g2[e]))) * inv,
+                                            __uint_as_float(o[2 * e + 1]) / (1.0f + expf(-__high2float(g2[e]))) * inv);
+            *reinterpret_cast<uint4*>(stage + (c0 / 64) * SUB + swz(r, (c0 / 8) % 8)) = pk;
+          }
+        } else {
+#pragma unroll
+          for (int c0 = 0; c0 < D; c0 += 32) {
+            uint32_t o[32];
+            tmem_ld_32x32(tmem_o + c0, o);
+            tmem_wait_ld();
+#pragma unroll
+            for (int c = 0; c < 32; c += 8) {
+              uint4 pk;
+              __nv_bfloat162* pp = reinterpret_cast<__nv_bfloat162*>(&pk);
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                pp[e] = __floats2bfloat162_rn(__uint_as_float(o[c + 2 * e]) * inv, __uint_as_float(o[c + 2 * e + 1]) * inv);
+              const int piece = (c0 + c) / 8;
+              *reinterpret_cast<uint4*>(stage + (piece / 8) * SUB + swz(r, piece % 8)) = pk;
+            }
           }
         }
         fence_async_smem();
       } else if (lane == 0) {
         if (ok) atomicExch(error, 13);
-        gave_up[quad] = 1;
+        gave_up[t] = 1;
       }
-      asm volatile("bar.sync 5, 256;" ::: "memory");  // the eight softmax warps
-      if (gave_up[0] | gave_up[1] | gave_up[2] | gave_up[3]) continue;
-      const int row_begin = pair * PAIR + t * ROWS;
-      if (q_by_tma && row_begin + ROWS <= n_rows) {
-        if (threadIdx.x == 0) {
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + t) : "memory");  // the tile's four warps
+      if (!gave_up[t]) {
+        const int row_begin = pair_row + t * rows;
+        if (q_by_tma && row_begin + rows <= n_rows) {
+          if (quad == 0 && lane == 0) {
 #pragma unroll
-          for (int h = 0; h < DB; ++h) tma_store_3d(&map_o, stage + h * SUB, h * 64, kh * G, row0 + row_begin / G);
-          tma_store_commit();
-          stores_pending = true;
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < ROWS * (D / 8) / 256; ++k) {
-          const int p = threadIdx.x + 256 * k;
-          const int row = p / (D / 8), piece = p % (D / 8);
-          const int R = row_begin + row;
-          if (R < n_rows)
-            *reinterpret_cast<uint4*>(out + (size_t)(row0 + R / G) * (WIDE ? ex.out_stride : HQ * D) + (size_t)(kh * G + R % G) * D + piece * 8) =
-                *reinterpret_cast<const uint4*>(stage + (piece / 8) * SUB + swz(row, piece % 8));
+            for (int h = 0; h < DB; ++h) tma_store_3d(&map_o, stage + h * SUB, h * 64, kh * G, row0 + row_begin / G);
+            tma_store_commit();
+            tma_store_wait_read();  // shared memory is given up when the block ends
+          }
+        } else {
+#pragma unroll 4
+          for (int k = 0; k < ROWS * (D / 8) / 128; ++k) {
+            const int p = quad * 32 + lane + 128 * k;
+            const int row = p / (D / 8), piece = p % (D / 8);
+            const int R = row_begin + row;
+            if (row < rows && R < n_rows)
+              *reinterpret_cast<uint4*>(out + (size_t)(row0 + R / G) * (WIDE ? ex.out_stride : HQ * D) + (size_t)(kh * G + R % G) * D + piece * 8) =
+                  *reinterpret_cast<const uint4*>(stage + (piece / 8) * SUB + swz(row, piece % 8));
+          }
         }
       }
     }
-    if (stores_pending) tma_store_wait_read();  // shared memory is given up when the block ends
   }
   tc_fence_before();
   __syncthreads();
@@ -562,15 +562,21 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
   }
 }
 
-constexpr size_t SMEM_BYTES = 6 * TILE_BYTES + 1024 + N_BARS * 8 + 64 + PAGE_IDS * sizeof(int) + 8 * ROWS * sizeof(float) + 16;
+constexpr size_t SMEM_BYTES = 6 * TILE_BYTES + 1024 + N_BARS * 8 + 64 + PAGE_IDS * sizeof(int) + 16;
 
-template <bool WIDE, bool SHAPED>
+template <bool WIDE, int SHAPE>
 int launch_tcgen05(bf16* out, const bf16* q, int q_stride, int HQ, int HKV, const int* seq_slot, const int* seq_start,
                    const int* seq_qlen, const int* cu_q, const int* table, int width, const void* k_cache, const void* v_cache,
                    int n_pages, int n_seqs, int max_q_len, int total_rows, float scale, int window, int* error, const Extras& ex,
                    cudaStream_t stream) {
   const int G = HQ / HKV;
-  const long long tiles = ((long long)max_q_len * G + PAIR - 1) / PAIR;
+  // The query tiles come and go by TMA where whole tokens (G rows each) fill at least three quarters of a tile; a tile then has
+  // that many rows. Fetched by the threads, the two tiles take 8 us at G of 5 where TMA takes 2 (of 30 for a block with twelve
+  // blocks of keys), so the rows left empty (3 of 128 at G of 5) cost less.
+  const int whole = G <= ROWS ? ROWS / G * G : 0;
+  const int q_by_tma = whole >= ROWS * 3 / 4 ? 1 : 0;
+  const int tile_rows = q_by_tma ? whole : ROWS;
+  const long long tiles = ((long long)max_q_len * G + 2 * tile_rows - 1) / (2 * tile_rows);
   if (tiles * HKV > 0x7fffffffLL || n_seqs > 65535) return -3;
   CUtensorMap map_k, map_v;
   const long long rows = (long long)n_pages * HKV * KRK_PAGE;
@@ -578,16 +584,15 @@ int launch_tcgen05(bf16* out, const bf16* q, int q_stride, int HQ, int HKV, cons
   if (rc) return rc;
   rc = make_map_bf16(&map_v, v_cache, rows, D, D, 64);
   if (rc) return rc;
-  // the query tiles come by TMA when a tile is a whole number of tokens (the group size divides 128)
-  const int q_by_tma = (ROWS % G == 0) ? 1 : 0;
   CUtensorMap map_q = map_k, map_o = map_k;
   if (q_by_tma) {
-    rc = make_map_bf16_3d(&map_q, q, D, HQ, total_rows, D, q_stride, G, ROWS / G);
+    rc = make_map_bf16_3d(&map_q, q, D, HQ, total_rows, D, q_stride, G, tile_rows / G);
     if (rc) return rc;
-    rc = make_map_bf16_3d(&map_o, out, D, HQ, total_rows, D, ex.out_stride, G, ROWS / G);
+    rc = make_map_bf16_3d(&map_o, out, D, HQ, total_rows, D, ex.out_stride, G, tile_rows / G);
     if (rc) return rc;
   }
-  auto kern = attention_tcgen05_kernel<WIDE, SHAPED>;
+  if (scale == 0.f) scale = 1e-30f;  // weights of zero are made by scores of minus infinity: the scale must not be zero
+  auto kern = attention_tcgen05_kernel<WIDE, SHAPE>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
@@ -595,7 +600,7 @@ int launch_tcgen05(bf16* out, const bf16* q, int q_stride, int HQ, int HKV, cons
     configured = true;
   }
   kern<<<dim3((unsigned)(tiles * HKV), n_seqs, 1), THREADS, SMEM_BYTES, stream>>>(
-      map_k, map_v, map_q, map_o, q_by_tma, out, q, q_stride, HQ, HKV, seq_slot, seq_start, seq_qlen, cu_q, table, width,
+      map_k, map_v, map_q, map_o, q_by_tma, tile_rows, out, q, q_stride, HQ, HKV, seq_slot, seq_start, seq_qlen, cu_q, table, width,
       scale * LOG2E, window, error, ex);
   KRK_CHECK_LAUNCH();
   return 0;
@@ -614,7 +619,7 @@ KRK_API int krk_attention_prefill_tcgen05(void* out, const void* qkv, int q_stri
   if ((q_stride % 8) || ((uintptr_t)qkv & 15) || ((uintptr_t)out & 15)) return -2;
   Extras ex = {};
   ex.out_stride = HQ * D;
-  return launch_tcgen05<false, false>((bf16*)out, (const bf16*)qkv, q_stride, HQ, HKV, seq_slot, seq_start, seq_qlen, cu_q, table, width,
+  return launch_tcgen05<false, 0>((bf16*)out, (const bf16*)qkv, q_stride, HQ, HKV, seq_slot, seq_start, seq_qlen, cu_q, table, width,
                                       k_cache, v_cache, n_pages, n_seqs, max_q_len, total_rows, scale, window, error, ex, stream);
 }
 
@@ -633,7 +638,7 @@ KRK_API int krk_sink_prefill_tcgen05(void* out, int out_stride, float out_scale,
   ex.sink = sink; ex.slopes = slopes; ex.out_scale = out_scale; ex.out_stride = out_stride;
   ex.cap_log2 = softcap * LOG2E; ex.in_cap = softcap > 0.f ? 2.f / softcap : 0.f;
   ex.gate = (const bf16*)gate; ex.gate_stride = gate_stride; ex.gate_mode = gate ? gate_mode : 0;
-  auto go = slopes || softcap > 0.f ? launch_tcgen05<true, true> : launch_tcgen05<true, false>;
+  auto go = softcap > 0.f ? launch_tcgen05<true, 2> : slopes ? launch_tcgen05<true, 1> : launch_tcgen05<true, 0>;
   return go((bf16*)out, (const bf16*)q, q_stride, HQ, HKV, seq_slot, seq_start, seq_qlen, cu_q, table, width, k_cache, v_cache, n_pages,
             n_seqs, max_q_len, total_rows, scale, window, error, ex, stream);
 }

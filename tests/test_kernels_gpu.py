@@ -615,6 +615,27 @@ def test_tcgen05_prefill_attention(ops, shape, window):
         close(got, other, dtype, "tcgen05 against mma.sync")
 
 
+@pytest.mark.parametrize("group", [3, 5, 20, 42, 43, 64, 100, 129])
+@pytest.mark.parametrize("scale,size", [(1.0 / 8.0, 1.0), (1.0 / 8.0, 6.0), (0.0, 1.0), (-1.0 / 16.0, 0.5)])
+def test_tcgen05_prefill_attention_of_any_group(ops, group, scale, size):
+    """Tiles of whole tokens where those fill three quarters of 128 rows (3, 5, 20, 42, 64 and 100 heads a kv head), of 128 rows
+    that threads fetch elsewhere (43, 129); sequences whose last tile holds one token, and more keys than a block; scores that
+    outgrow the reference maximum by far, none at all (the mean of the values) and of a negative scale."""
+    D, kv_heads, dtype = 64, 2, torch.bfloat16
+    ref = TorchOps(dtype)
+    heads = group * kv_heads
+    cache = make_cache(24, kv_heads, D, 3, 7, dtype, 90)
+    tokens = 128 // group if group <= 128 else 1
+    lens = [2 * max(tokens, 2) + 1, 259, -(-130 // group)]
+    starts = [0, 150, 77]
+    batch = make_batch([1, 2, 0], starts, lens)
+    qkv = rand((batch.n_rows, (heads + 2 * kv_heads) * D), dtype, 91, size)
+    ops.qk_norm_rope_write(qkv, heads, kv_heads, D, None, None, 1e-6, None, None, batch, cache)
+    got = ops.attention(qkv, heads, kv_heads, D, batch, cache, scale, None)
+    ops.check()
+    close(got, ref.attention(qkv, heads, kv_heads, D, batch, cache, scale, None), dtype, f"group {group} scale {scale}")
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("q_len", [1, 37])
 def test_one_far_key_among_hundreds_decides(ops, dtype, q_len):
