@@ -15,13 +15,15 @@
 //   (measured with independent chains); 360 rows of 6,144 x 2,560: 259 us, 44 TFLOP/s (the general kernel: 2.0 ms).
 //   Packed multiply-adds (fma.rn.f32x2) were measured and are slower here (274 to 294 us): the copies that pair an
 //   operand with itself cost more than the pipe's register reads gain.
-// * gemm_f32_few: up to 16 float32 rows. Bound by the weights' bytes: each is read once, by asynchronous 16-byte copies
-//   a slice ahead; a thread owns one or two output columns of one or two rows. One row of 151,936 x 2,560: 235 us,
-//   6.6 TB/s; three rows 258 us, of 2,560 x 4,096 21 us, where the chain of K multiply-adds is the bound (the general kernel: 1.9 ms and 570 us).
+// * gemm_f32_few: up to 16 float32 rows. Bound by the weights' bytes: each is read once, by bulk copies a slice or two ahead; a
+//   thread owns one or two output columns of one or two rows. One row of 151,936 x 2,560: 235 us, 6.6 TB/s; three rows 239,
+//   of 2,560 x 9,728 41 us, where the chain of K multiply-adds is the bound (20 us at four clocks each; copies of 16 bytes by
+//   all threads: 265 and 50; the general kernel: 1.9 ms and 570 us of 2,560 x 4,096).
 // * gemm_nt: everything else (bfloat16 inputs with float32 output at odd sizes, for output-head logits at many
 //   positions; float32 rows whose size or alignment does not allow 16-byte accesses). 64x64 output tile, k in slices of
 //   16, 256 threads with a 4x4 micro-tile each.
-#include "mma.cuh"  // cp.async
+#include "mma.cuh"      // the cache policy of streamed weights
+#include "tcgen05.cuh"  // mbarriers
 
 namespace {
 
@@ -203,112 +205,135 @@ gemm_f32_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const f
 }
 
 // ---- float32, up to 16 rows ------------------------------------------------------------------------------------
-// A block owns 16 * CPT columns (a thread c, c + 16); its 8 groups of 16 threads take RPT rows each. A slice is 256 k of
-// the columns' weights and of the rows, and the next one is on its way while one is multiplied. What an SM has in flight is a matter of how
-// many blocks it holds, not of how deep each one's ring is: with two slices of 256 k, 35 KB a block at one row, five or six
-// blocks share an SM; six slices of 128 left room for three, whose waits and chains did not cover each other (three rows of 151,936
-// x 2,560 355 us, now 258; 16 rows of 19,456 x 2,560 113 and 98). Beyond 8 rows, where shared-memory reads are the
-// bound, a thread's two rows of two columns read half as much for a multiply-add as one of one.
-constexpr int FEW_K = 256, FEW_PITCH = FEW_K + 4, FEW_DEPTH = 2;
+// A block owns 16 * CPT columns (a thread c, c + 16); a group of 16 threads takes RPT rows, a warp has two groups, and there are as many
+// warps as the rows ask for. A slice is SLICE k of the columns' weights and of the rows. One more warp asks for slices, a bulk copy a
+// column (1 KB), as far ahead as the ring is deep, so that the others only wait and multiply: with 16-byte copies by all threads, asking
+// for a slice took 600 to 1,200 clocks of the 1,200 that its 256 multiply-adds take in their chain (256 x 4, and the reads).
+// Beyond 8 rows, where shared-memory reads are the bound, a thread's two rows of two columns read half as much for a
+// multiply-add as one of one.
+constexpr int FEW_MAX_DEPTH = 3;
+constexpr int FEW_BARS = 2 * FEW_MAX_DEPTH * 8;  // bytes before the ring: slice is here, slice is free
 
-template <int RPT, int CPT>
-__global__ void __launch_bounds__(128)
+template <int RPT, int CPT, int SLICE>
+__global__ void __launch_bounds__(160)
 gemm_f32_few_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W, int M, int N, int K,
-                    int lda, int ldw, int ldc) {
-  constexpr int COLS = 16 * CPT;
-  extern __shared__ __align__(16) float sm[];
-  const int stage_floats = (COLS + M) * FEW_PITCH;
-  // neighbouring lanes share a column and differ in their rows: a warp's 16-byte reads of W and of x then take 2 cycles
-  // of the SM's shared memory each, 4 where neighbours' columns differ
-  const int tid = threadIdx.x, col = (tid & 31) >> 1, group = 2 * (tid >> 5) + (tid & 1);
+                    int lda, int ldw, int ldc, int depth, int* __restrict__ error) {
+  constexpr int COLS = 16 * CPT, PITCH = SLICE + 4;
+  extern __shared__ __align__(16) unsigned char smem[];
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem);
+  uint64_t* free_ = full + FEW_MAX_DEPTH;
+  float* ring = reinterpret_cast<float*>(smem + FEW_BARS);
+  const int stage_floats = (COLS + M) * PITCH;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, readers = (blockDim.x >> 5) - 1;
   const int n0 = blockIdx.x * COLS;
-  const int slices = (K + FEW_K - 1) / FEW_K;
-  const uint64_t policy = l2_evict_first_policy();
-  constexpr int COPY_ROWS = 128 / (FEW_K / 4);  // rows that the threads copy at a time
-  const int ck = tid % (FEW_K / 4) * 4, cr = tid / (FEW_K / 4);  // this thread copies k = ck..ck+3 of rows cr, cr + COPY_ROWS, ...
-  auto request = [&](int s) {
-    const int k = s * FEW_K + ck;
-    if (k < K) {  // what lies beyond K is never read: the loops below end there
-      float* dst = sm + (s % FEW_DEPTH) * stage_floats + ck;
-#pragma unroll
-      for (int r = 0; r < COLS; r += COPY_ROWS)
-        if (n0 + cr + r < N) cp_async_16_stream(dst + (cr + r) * FEW_PITCH, W + (size_t)(n0 + cr + r) * ldw + k, policy);
-      for (int r = cr; r < M; r += COPY_ROWS) cp_async_16(dst + (COLS + r) * FEW_PITCH, A + (size_t)r * lda + k);
+  const int slices = (K + SLICE - 1) / SLICE;
+  if (tid == 0) {
+    for (int i = 0; i < depth; ++i) {
+      tc::mbar_init(full + i, 1);
+      tc::mbar_init(free_ + i, readers);
     }
-    cp_async_commit();  // one group a slice, empty beyond the last, so that the count of waits holds
-  };
-  for (int s = 0; s < FEW_DEPTH - 1; ++s) request(s);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  if (warp == readers) {  // the copies: a lane has columns (or rows) lane, lane + 32 of a slice
+    const int cols = min(COLS, N - n0);
+    const uint64_t policy = l2_evict_first_policy();
+    for (int s = 0, b = 0, round = 0; s < slices; ++s) {
+      if (round > 0 && !__all_sync(0xffffffffu, tc::mbar_wait(free_ + b, (round - 1) & 1))) return;  // the readers say so
+      const int bytes = min(SLICE, K - s * SLICE) * 4;
+      if (lane == 0) tc::mbar_expect_tx(full + b, (cols + M) * bytes);
+      __syncwarp();
+      float* dst = ring + b * stage_floats;
+      for (int r = lane; r < cols; r += 32)
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+                     ::"r"(tc::smem_u32(dst + r * PITCH)), "l"(W + (size_t)(n0 + r) * ldw + s * SLICE), "r"(bytes), "r"(tc::smem_u32(full + b)), "l"(policy)
+                     : "memory");
+      if (lane < M)
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     ::"r"(tc::smem_u32(dst + (COLS + lane) * PITCH)), "l"(A + (size_t)lane * lda + s * SLICE), "r"(bytes), "r"(tc::smem_u32(full + b))
+                     : "memory");
+      if (++b == depth) { b = 0; ++round; }
+    }
+    return;
+  }
+  // neighbouring lanes share a column and differ in their rows
+  const int col = lane >> 1, group = 2 * warp + (lane & 1);
   float acc[RPT][CPT];
 #pragma unroll
   for (int r = 0; r < RPT; ++r)
 #pragma unroll
     for (int c = 0; c < CPT; ++c) acc[r][c] = 0.f;
   const int row0 = group * RPT;
-  const bool live = row0 < M;
   int xat[RPT];
 #pragma unroll
-  for (int r = 0; r < RPT; ++r) xat[r] = (COLS + min(row0 + r, M - 1)) * FEW_PITCH;
-  for (int s = 0; s < slices; ++s) {
-    cp_async_wait<FEW_DEPTH - 2>();
-    __syncthreads();  // slice s is here for everyone, and the slice before it is no longer read
-    request(s + FEW_DEPTH - 1);
-    if (!live) continue;
-    const float* base = sm + (s % FEW_DEPTH) * stage_floats;
-    const float* w = base + col * FEW_PITCH;
+  for (int r = 0; r < RPT; ++r) xat[r] = (COLS + min(row0 + r, M - 1)) * PITCH;
+  bool here = true;
+  for (int s = 0, b = 0, round = 0; s < slices; ++s) {
+    // a wait that runs out: the block's outputs are NaN
+    here = __all_sync(0xffffffffu, tc::mbar_wait(full + b, round & 1));
+    if (!here) {
+      tc::mbar_wait(full + b, round & 1);  // the copy may still be on its way into this block's memory: as long again
+      break;
+    }
+    const float* base = ring + b * stage_floats;
+    const float* w = base + col * PITCH;
     constexpr int AHEAD = 4;  // pieces of four k in registers while as many are multiplied
-    const int kn = min(FEW_K, K - s * FEW_K);
+    const int kn = min(SLICE, K - s * SLICE);
     float4 w4[2][AHEAD][CPT], x4[2][AHEAD][RPT];
-    auto read = [&](int b, int k0) {
+    auto read = [&](int f, int k0) {
 #pragma unroll
       for (int i = 0; i < AHEAD; ++i) {
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) w4[b][i][c] = *reinterpret_cast<const float4*>(w + 16 * c * FEW_PITCH + k0 + 4 * i);
+        for (int c = 0; c < CPT; ++c) w4[f][i][c] = *reinterpret_cast<const float4*>(w + 16 * c * PITCH + k0 + 4 * i);
 #pragma unroll
-        for (int r = 0; r < RPT; ++r) x4[b][i][r] = *reinterpret_cast<const float4*>(base + xat[r] + k0 + 4 * i);
+        for (int r = 0; r < RPT; ++r) x4[f][i][r] = *reinterpret_cast<const float4*>(base + xat[r] + k0 + 4 * i);
       }
     };
-    auto multiply = [&](int b, int i) {
+    auto multiply = [&](int f, int i) {
 #pragma unroll
       for (int r = 0; r < RPT; ++r)
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) acc[r][c] = fmaf(x4[b][i][r].x, w4[b][i][c].x, acc[r][c]);
+        for (int c = 0; c < CPT; ++c) acc[r][c] = fmaf(x4[f][i][r].x, w4[f][i][c].x, acc[r][c]);
 #pragma unroll
       for (int r = 0; r < RPT; ++r)
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) acc[r][c] = fmaf(x4[b][i][r].y, w4[b][i][c].y, acc[r][c]);
+        for (int c = 0; c < CPT; ++c) acc[r][c] = fmaf(x4[f][i][r].y, w4[f][i][c].y, acc[r][c]);
 #pragma unroll
       for (int r = 0; r < RPT; ++r)
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) acc[r][c] = fmaf(x4[b][i][r].z, w4[b][i][c].z, acc[r][c]);
+        for (int c = 0; c < CPT; ++c) acc[r][c] = fmaf(x4[f][i][r].z, w4[f][i][c].z, acc[r][c]);
 #pragma unroll
       for (int r = 0; r < RPT; ++r)
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) acc[r][c] = fmaf(x4[b][i][r].w, w4[b][i][c].w, acc[r][c]);
+        for (int c = 0; c < CPT; ++c) acc[r][c] = fmaf(x4[f][i][r].w, w4[f][i][c].w, acc[r][c]);
     };
-    if (kn == FEW_K) {
+    if (kn == SLICE) {
       read(0, 0);
 #pragma unroll
-      for (int p = 0; p < FEW_K / (4 * AHEAD); ++p) {
-        if (p + 1 < FEW_K / (4 * AHEAD)) read((p + 1) & 1, (p + 1) * 4 * AHEAD);
+      for (int p = 0; p < SLICE / (4 * AHEAD); ++p) {
+        if (p + 1 < SLICE / (4 * AHEAD)) read((p + 1) & 1, (p + 1) * 4 * AHEAD);
 #pragma unroll
         for (int i = 0; i < AHEAD; ++i) multiply(p & 1, i);
       }
     } else {
       for (int k = 0; k < kn; k += 4) {
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) w4[0][0][c] = *reinterpret_cast<const float4*>(w + 16 * c * FEW_PITCH + k);
+        for (int c = 0; c < CPT; ++c) w4[0][0][c] = *reinterpret_cast<const float4*>(w + 16 * c * PITCH + k);
 #pragma unroll
         for (int r = 0; r < RPT; ++r) x4[0][0][r] = *reinterpret_cast<const float4*>(base + xat[r] + k);
         multiply(0, 0);
       }
     }
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(free_ + b);
+    if (++b == depth) { b = 0; ++round; }
   }
-  cp_async_wait<0>();
+  if (!here && lane == 0 && error) atomicExch(error, 20);
 #pragma unroll
   for (int r = 0; r < RPT; ++r)
 #pragma unroll
     for (int c = 0; c < CPT; ++c)
-      if (row0 + r < M && n0 + col + 16 * c < N) C[(size_t)(row0 + r) * ldc + n0 + col + 16 * c] = acc[r][c];
+      if (row0 + r < M && n0 + col + 16 * c < N) C[(size_t)(row0 + r) * ldc + n0 + col + 16 * c] = here ? acc[r][c] : NAN;
 }
 
 template <int MG, int NG>
@@ -320,25 +345,43 @@ int launch_tile(float* C, const float* A, const float* W, int M, int N, int K, i
   return 0;
 }
 
-template <int RPT, int CPT>
-int launch_few(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
-  constexpr size_t per_row = (size_t)FEW_DEPTH * FEW_PITCH * sizeof(float);
-  const size_t smem = (16 * CPT + M) * per_row;  // 35 to 100 KB
+template <int RPT, int CPT, int SLICE>
+int launch_few(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, int* error, cudaStream_t stream) {
+  constexpr size_t per_row = (SLICE + 4) * sizeof(float);
+  const size_t stage = (16 * CPT + M) * per_row;  // 17 to 50 KB
+  const int blocks = (N + 16 * CPT - 1) / (16 * CPT);
+  // Two slices of the ring leave an SM more blocks than three, three cover more of a slice's way. What decides is how many blocks
+  // the SMs take in full rounds (three rows of K 2,560, two slices and three: N of 2,560 17.8 and 16.4 us, 6,144 20.3 and 19.0,
+  // 8,192 22.6 and 29.3, 12,288 (K 4,096) 51.6 and 44.3, 19,456 43.0 and 44.0, 151,936 239 and 256).
+  auto rounds = [&](int depth) {
+    const long long held = max(1LL, (long long)(227 * 1024 / (FEW_BARS + depth * stage + 1024)));
+    return (blocks + 148 * held - 1) / (148 * held) * held;
+  };
+  const int depth = rounds(3) < rounds(2) ? 3 : 2;
   // always the most that a call may need: another thread may be about to launch with more rows than this one
-  cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<RPT, CPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((16 * CPT + 8 * RPT) * per_row));
+  cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<RPT, CPT, SLICE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(FEW_BARS + FEW_MAX_DEPTH * (16 * CPT + 8 * RPT) * per_row));
   if (e != cudaSuccess) return (int)e;
-  gemm_f32_few_kernel<RPT, CPT><<<(N + 16 * CPT - 1) / (16 * CPT), 128, smem, stream>>>(C, A, W, M, N, K, lda, ldw, ldc);
+  const int readers = (M + 2 * RPT - 1) / (2 * RPT);
+  gemm_f32_few_kernel<RPT, CPT, SLICE><<<blocks, 32 * (readers + 1), FEW_BARS + depth * stage, stream>>>(
+      C, A, W, M, N, K, lda, ldw, ldc, depth, error);
   KRK_CHECK_LAUNCH();
   return 0;
 }
 
 // float32 in and out with 16-byte rows. -2: not of that kind.
-int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
+int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, int* error, cudaStream_t stream) {
   if (M == 0 || N == 0) return 0;
   if (K < 4 || K % 4 || lda % 4 || ldw % 4 || (((uintptr_t)A | (uintptr_t)W | (uintptr_t)C) & 15)) return -2;
-  // 16 rows: 98 us of 19,456 x 2,560 and 161 by the tiles below, 558 and 647 of 151,936 x 2,560, 2.5 and 4.0 of 128 x 64
-  if (M <= 8) return launch_few<1, 1>(C, A, W, M, N, K, lda, ldw, ldc, stream);
-  if (M <= 16) return launch_few<2, 2>(C, A, W, M, N, K, lda, ldw, ldc, stream);
+  // 16 rows: 84 us of 19,456 x 2,560 and 161 by the tiles below, 453 and 647 of 151,936 x 2,560, 2.5 and 4.0 of 128 x 64.
+  // One row of one column a thread reads most of shared memory for a multiply-add and has the most blocks; from five rows
+  // on the reads bound it where there are columns enough (eight rows, two by two in slices of 128 and one by one: N of 19,456
+  // 50 and 63 us, 151,936 287 and 367; 8,192 38 and 31; five rows 49 and 53, 281 and 287; 12,288 63 and 55). Beyond eight rows two by
+  // two always: in slices of 128 to 12 rows of many columns (nine rows: N of 12,288 66 and 85, 151,936 327 and 420; 8,192 39 and 33;
+  // sixteen 441 and 453, but 94 and 84 of 19,456).
+  if (M <= 8 && (M < 5 || N < 16384)) return launch_few<1, 1, 256>(C, A, W, M, N, K, lda, ldw, ldc, error, stream);
+  if (M <= 8 || (M <= 12 && N >= 12288)) return launch_few<2, 2, 128>(C, A, W, M, N, K, lda, ldw, ldc, error, stream);
+  if (M <= 16) return launch_few<2, 2, 256>(C, A, W, M, N, K, lda, ldw, ldc, error, stream);
   // Cycles per k on the busiest SM, from the times measured at 17 to 1,024 rows of five matrices: a block alone is bound by
   // its own latency (the first number), several by what a block takes of the SM.
   auto cost = [&](int tm, int tn, int alone, int each) {
@@ -355,11 +398,12 @@ int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, in
 
 }  // namespace
 
-// in_dtype / out_dtype: KRK_DTYPE_F32 or KRK_DTYPE_BF16. Supported: f32->f32, bf16->f32, bf16->bf16.
-KRK_API int krk_gemm_nt(void* C, const void* A, const void* W, int M, int N, int K, int lda, int ldw, int ldc,
-                        int in_dtype, int out_dtype, cudaStream_t stream) {
+// in_dtype / out_dtype: KRK_DTYPE_F32 or KRK_DTYPE_BF16. Supported: f32->f32, bf16->f32, bf16->bf16. `error` (device, may be null)
+// is set to 20 should a product of few rows give up on a wait, whose outputs are then NaN.
+KRK_API int krk_gemm_nt_checked(void* C, const void* A, const void* W, int M, int N, int K, int lda, int ldw, int ldc,
+                                int in_dtype, int out_dtype, int* error, cudaStream_t stream) {
   if (in_dtype == KRK_DTYPE_F32 && out_dtype == KRK_DTYPE_F32) {
-    const int rc = launch_f32((float*)C, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldc, stream);
+    const int rc = launch_f32((float*)C, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldc, error, stream);
     if (rc != -2) return rc;
   }
   if (in_dtype == KRK_DTYPE_F32 && out_dtype == KRK_DTYPE_F32)
@@ -369,4 +413,9 @@ KRK_API int krk_gemm_nt(void* C, const void* A, const void* W, int M, int N, int
   if (in_dtype == KRK_DTYPE_BF16 && out_dtype == KRK_DTYPE_BF16)
     return launch<bf16, bf16>(C, A, W, M, N, K, lda, ldw, ldc, stream);
   return -4;
+}
+
+KRK_API int krk_gemm_nt(void* C, const void* A, const void* W, int M, int N, int K, int lda, int ldw, int ldc,
+                        int in_dtype, int out_dtype, cudaStream_t stream) {
+  return krk_gemm_nt_checked(C, A, W, M, N, K, lda, ldw, ldc, in_dtype, out_dtype, nullptr, stream);
 }

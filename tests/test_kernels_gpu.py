@@ -113,6 +113,20 @@ def test_float32_products_sum_in_one_order_whatever_the_rows(ops, nk):
     assert torch.equal(ops.linear(wide[:, :k], w), want[:40]), "rows of a wider buffer"
 
 
+@pytest.mark.parametrize("nk", [(16383, 132), (16384, 132), (12288, 260), (12273, 388), (4741, 516), (21003, 4)])
+def test_float32_products_of_few_rows_and_many_columns(ops, nk):
+    """Around the column counts and rows at which the kernel of few rows takes other slices, more columns a thread or a deeper ring:
+    the same chain still, equal to the bit to the general kernel's (rows off 16-byte boundaries)."""
+    n, k = nk
+    x, w = rand((16, k), torch.float32, 73), rand((n, k), torch.float32, 74)
+    odd = torch.empty((16, k + 1), device="cuda")
+    odd[:, 1:] = x
+    want = ops.linear(odd[:, 1:], w)
+    for m in (1, 3, 4, 5, 8, 9, 12, 13, 16):
+        assert torch.equal(ops.linear(x[:m], w), want[:m]), f"{m} rows"
+    ops.check()
+
+
 def test_float32_products_of_several_threads(ops):
     """Threads whose products have one row, eight and sixteen: a launch's shared memory depends on the rows, and no call may lower
     what another is about to launch with. Straight through the library, which other threads enter while one is in it."""
