@@ -127,7 +127,7 @@ _SCAN_SIGNATURES = {
     "krk_recurrence_chunk_tokens": [c_int, c_int, c_int, c_float, _P],
     "krk_recurrence_chunks": [c_int, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, _P, _P, _P, _P, _P, _P,
                               c_int, c_int, _P, _P, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_int, _P, _P, _P,
-                              c_int, c_int, _P, _P],
+                              c_int, c_int, _P, _P, _P],
     "krk_causal_conv_silu": [_P, _P, c_int, _P, _P, _P, c_int, c_int, c_int, c_int, _P, _P, _P, _P, c_int, _P, c_int],
     "krk_ssd_scan": [_P, _P, c_int, _P, c_int, _P, c_int, _P, c_int, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int,
                      c_int, _P, _P, _P, c_int, _P, _P, c_int, _P],
@@ -266,6 +266,7 @@ class Kernels:
                  3: "a tensor-core GEMM gave up waiting for a free shared-memory stage",
                  4: "a tensor-core GEMM gave up waiting for a TMA load",
                  5: "a tensor-core GEMM gave up waiting for its accumulator",
+                 24: "the delta rule's walk gave up waiting for its copies",
                  20: "a 32-bit product of few rows gave up waiting for its copies",
                  21: "the wait of the self-test kernel ran out (as it is meant to)"}
         if flag in known:
@@ -1397,7 +1398,7 @@ class Kernels:
                     _ptr(rate_bias), _ptr(bonus), norm_w.data_ptr(), state.data_ptr(), last_ptr, last_stride, C,
                     _ptr(last_state), optr, ostride, out_col, float(out_scale), float(eps), float(decay_scale), heads,
                     lora.shape[1], batch.n_seqs, batch.cu_q.data_ptr(), batch.seq_qlen.data_ptr(), batch.seq_slot.data_ptr(),
-                    first, min(portion, chunks - first), scratch.data_ptr(), self._stream())
+                    first, min(portion, chunks - first), scratch.data_ptr(), self.error.data_ptr(), self._stream())
                 if rc == -2:  # odd strides or offsets: the first portion already says so, and nothing was done
                     break
                 self._ok(rc, f"{kind} recurrence in chunks")

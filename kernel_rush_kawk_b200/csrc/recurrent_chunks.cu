@@ -25,7 +25,7 @@
 // its starting state in G's place and the sequence its final one; (3) per (sequence, chunk, head) the outputs with their norm,
 // weight and gate. Chunks of 32: a chunk of 64 needs twice the multiply-adds a token in pass 1 and halves the walk's steps.
 //
-// Measured: one prompt of 2,048 tokens, delta rule of 8 heads, 1,171 us token by token, 110 here (the passes 57, 36 and 17, each from a
+// Measured: one prompt of 2,048 tokens, delta rule of 8 heads, 1,171 us token by token, 97 here (the passes 57, 22 and 17, each from a
 // cold cache); three prompts of 2,553 tokens in all, time mixing of 40 heads, 405 -> 117 us (48, 17 and 66; with float32 on the
 // CUDA cores 175). Passes 1 and 3 are bound by instruction issue and latencies (a 0.4 to 0.5 share of the issue slots, 12 to 32 warps an
 // SM), the walk by the chain of its steps.
@@ -33,7 +33,8 @@
 // e^{-c_s} must stay in range. The delta rule's decay is at least e^{-decay_scale} a token, so a chunk's is bounded by the
 // parameter (the caller asks krk_recurrence_chunk_tokens). Time mixing's has no bound: a chunk in which some channel decays by
 // more than e^-40 forms its pair sums by decaying each key token by token, right for any decay and slower.
-#include "mma.cuh"  // cp.async
+#include "mma.cuh"
+#include "tcgen05.cuh"  // tiled copies and their barriers
 
 namespace {
 
@@ -61,6 +62,7 @@ struct ChunkArgs {
   int H, R;
   const int *cu_q, *seq_qlen, *seq_slot;
   int chunk0, n_chunks;  // the chunks of every sequence that this launch takes
+  int* error;
   float* scratch;        // per (sequence, chunk, head): delta M, G, Q, O_own; time mixing G, summed decays and, past e^-SAFE, the decays
 };
 constexpr int ITEM_DELTA = 2 * N * N + 2 * L * N, ITEM_MIX = N * N + 2 * L * N;
@@ -640,71 +642,120 @@ __global__ void __launch_bounds__(THREADS, 8) mix_chunk_kernel(ChunkArgs a) {
 }
 
 // ---- pass 2 ----------------------------------------------------------------------------------------------------
-// Delta rule: a block walks WALK_COLS value columns of one (sequence, head). A lane holds the sums of two key channels over
-// its warp's quarter of M's columns; the warps' shares meet in shared memory. M comes by asynchronous copies, five chunks ahead.
-__global__ void __launch_bounds__(THREADS) delta_walk_kernel(ChunkArgs a) {
+// Delta rule: a block walks WALK_COLS value columns of one (sequence, head). Four warps have sixteen of the 64 key channels' rows
+// each; a lane takes four rows against eight channels, and eight lanes hand their shares round until each has two numbers of
+// the new state: one barrier a chunk. A fifth warp asks for the chunks' M and columns of G five chunks ahead, as tiled copies, and waits
+// for them. Bound by the chain of a step: the state from shared memory, 32 multiply-adds of four columns, three exchanges, the
+// barrier. One prompt of 2,048 tokens, 8 heads: 36 us with 16-byte copies by the walkers (32 a step, which took half of it) and
+// two barriers, 22 here; M read before the state is there 3 us of that, a wait for a copy by the walkers themselves 5 more.
+constexpr int WALKERS = 128, WALK_THREADS = WALKERS + 32;
+constexpr int WALK_M = N * N, WALK_G = N * WALK_COLS;         // floats of a chunk's M and of its columns of G
+constexpr int WALK_SP = 36;                                   // floats from eight channels of the state to the next eight: other banks
+__global__ void __launch_bounds__(WALK_THREADS)
+delta_walk_kernel(const __grid_constant__ CUtensorMap map_m, const __grid_constant__ CUtensorMap map_g, ChunkArgs a) {
   extern __shared__ __align__(16) float sm[];
-  float* ms = sm;                                          // [WALK_STAGES][N][PITCH]
-  float* gs = ms + WALK_STAGES * N * PITCH;                // [WALK_STAGES][N][4]
-  float* ss = gs + WALK_STAGES * N * WALK_COLS;            // [N][4] the state's columns
-  float* part = ss + N * WALK_COLS;                        // [4][N][4]
-  grid_dependency_wait();
+  float* ms = reinterpret_cast<float*>(((uintptr_t)sm + 1023) & ~(uintptr_t)1023);  // [WALK_STAGES][2][N][32], 128-byte swizzle
+  float* gs = ms + WALK_STAGES * WALK_M;                                            // [WALK_STAGES][N][WALK_COLS]
+  float* ss = gs + WALK_STAGES * WALK_G;                                            // [2][N / 8][WALK_SP] the state's columns, in turn
+  __shared__ uint64_t full[WALK_STAGES];
   const int p0 = blockIdx.x * WALK_COLS, h = blockIdx.y, seq = blockIdx.z;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) {
+    for (int i = 0; i < WALK_STAGES; ++i) tc::mbar_init(full + i, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  grid_dependency_wait();
   const int n_chunks = min(a.n_chunks, (a.seq_qlen[seq] + L - 1) / L - a.chunk0);
   if (n_chunks <= 0) return;
-  float* items = a.scratch + ((size_t)seq * a.n_chunks * a.H + h) * ITEM_DELTA;
-  const size_t step = (size_t)a.H * ITEM_DELTA;
-  float* st = a.state + ((size_t)a.seq_slot[seq] * a.H + h) * N * N + p0;
-  auto request = [&](int c) {
-    if (c < n_chunks) {
-      const float* m = items + c * step;
-      const int b = c % WALK_STAGES;
-#pragma unroll
-      for (int i = 0; i < N * N / 4 / THREADS; ++i) {
-        const int e = i * THREADS + tid, n = e / (N / 4), j = (e % (N / 4)) * 4;
-        cp_async_16(ms + (b * N + n) * PITCH + j, m + n * N + j);
-      }
-      if (tid < N) cp_async_16(gs + (b * N + tid) * WALK_COLS, m + N * N + tid * N + p0);
+  auto step_sync = [] { asm volatile("bar.sync 1, 160;" ::: "memory"); };
+  if (warp == WALKERS / 32) {
+    // The fifth warp waits for the copies, so that no walker has to: at a step's barrier the next chunk but one is here. A
+    // chunk's place is free when the step before it is over, since the walkers read a chunk a step ahead.
+    auto request = [&](int c) {
+      if (c >= n_chunks || lane != 0) return;
+      const int b = c % WALK_STAGES, row = ((seq * a.n_chunks + c) * a.H + h) * (ITEM_DELTA / N);
+      tc::mbar_expect_tx(full + b, (WALK_M + WALK_G) * sizeof(float));
+      tc::tma_load_2d(ms + b * WALK_M, &map_m, full + b, 0, row);
+      tc::tma_load_2d(ms + b * WALK_M + N * 32, &map_m, full + b, 32, row);
+      tc::tma_load_2d(gs + b * WALK_G, &map_g, full + b, p0, row + N);
+    };
+    auto wait = [&](int c) {
+      // a wait that runs out: the step's results are not to be used, which the error word says; the copy may still be on its way: as long again
+      if (c >= n_chunks || __all_sync(0xffffffffu, tc::mbar_wait(full + c % WALK_STAGES, (c / WALK_STAGES) & 1))) return;
+      if (lane == 0) atomicExch(a.error, 24);
+      tc::mbar_wait(full + c % WALK_STAGES, (c / WALK_STAGES) & 1);
+    };
+    for (int c = 0; c < WALK_STAGES; ++c) request(c);
+    wait(0);
+    wait(1);
+    step_sync();
+    for (int c = 0; c < n_chunks; ++c) {
+      if (c) request(c + WALK_STAGES - 1);
+      wait(c + 2);
+      step_sync();
     }
-    cp_async_commit();
-  };
-  for (int c = 0; c < WALK_STAGES - 1; ++c) request(c);
-  if (tid < N) st4(ss + tid * WALK_COLS, ld4(st + (size_t)tid * N));
-  for (int c = 0; c < n_chunks; ++c) {
-    cp_async_wait<WALK_STAGES - 2>();
-    __syncthreads();  // chunk c's M and G and the state are here; the buffers of the chunk before are no longer read
-    request(c + WALK_STAGES - 1);
-    const int b = c % WALK_STAGES;
-    float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
-#pragma unroll
-    for (int j = 0; j < N / 4; j += 4) {
-      const int k = warp * (N / 4) + j;
-      float x[4], y[4];
-      st4(x, ld4(ms + (b * N + lane) * PITCH + k));
-      st4(y, ld4(ms + (b * N + 32 + lane) * PITCH + k));
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float4 s = ld4(ss + (k + i) * WALK_COLS);
-        fma4(lo, x[i], s);
-        fma4(hi, y[i], s);
-      }
-    }
-    st4(part + (warp * N + lane) * 4, lo);
-    st4(part + (warp * N + 32 + lane) * 4, hi);
-    __syncthreads();
-    if (tid < N) {
-      const float4 p = ld4(part + tid * 4), q = ld4(part + (N + tid) * 4), r = ld4(part + (2 * N + tid) * 4), s = ld4(part + (3 * N + tid) * 4);
-      const float4 g = ld4(gs + (b * N + tid) * WALK_COLS);
-      st4(items + c * step + N * N + tid * N + p0, ld4(ss + tid * WALK_COLS));  // the chunk's starting state, in G's place
-      st4(ss + tid * WALK_COLS, make_float4(g.x + ((p.x + q.x) + (r.x + s.x)), g.y + ((p.y + q.y) + (r.y + s.y)),
-                                            g.z + ((p.z + q.z) + (r.z + s.z)), g.w + ((p.w + q.w) + (r.w + s.w))));
-    }
+    return;
   }
-  cp_async_wait<0>();
-  __syncthreads();
+  const int kg = lane & 7, half = kg >> 2, r0 = warp * 16 + (lane >> 3) * 4;
+  const int row = r0 + 2 * half + ((lane >> 1) & 1), col = 2 * (lane & 1);  // what this lane has of the state: two columns of a channel
+  float* items = a.scratch + ((size_t)seq * a.n_chunks * a.H + h) * ITEM_DELTA + N * N + row * N + p0 + col;
+  const size_t step = (size_t)a.H * ITEM_DELTA;
+  float2* st = reinterpret_cast<float2*>(a.state + ((size_t)a.seq_slot[seq] * a.H + h) * N * N + row * N + p0 + col);
+  const int at = (row >> 3) * WALK_SP + (row & 7) * WALK_COLS + col;
+  float2 mine = *st;
+  *reinterpret_cast<float2*>(ss + at) = mine;
+  step_sync();
+  int b = 0;
+  float4 x[4][2];  // a chunk's M, in registers before the state that it meets is there
+  float2 own;
+  auto fetch = [&] {
+    const float* m = ms + b * WALK_M + half * (N * 32);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = r0 + i;
+#pragma unroll
+      for (int j = 0; j < 2; ++j)  // the upper channels' lanes take their second four first, for the banks' sake
+        x[i][j] = ld4(m + r * 32 + ((((kg & 3) * 2 + (j ^ half)) ^ (r & 7)) << 2));
+    }
+    own = *reinterpret_cast<const float2*>(gs + b * WALK_G + row * WALK_COLS + col);
+  };
+  fetch();
+  for (int c = 0; c < n_chunks; ++c) {
+    const float* s = ss + (c & 1) * (N / 8) * WALK_SP + kg * WALK_SP;
+    float4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float* sj = s + (j ^ half) * 16;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float4 state = ld4(sj + 4 * e);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) fma4(v[i], e == 0 ? x[i][j].x : e == 1 ? x[i][j].y : e == 2 ? x[i][j].z : x[i][j].w, state);
+      }
+    }
+    const float2 g = own;
+    if (++b == WALK_STAGES) b = 0;
+    if (c + 1 < n_chunks) fetch();
+    *reinterpret_cast<float2*>(items + c * step) = mine;  // the chunk's starting state, in G's place
+    auto exchange = [](float keep, float send, int by) { return keep + __shfl_xor_sync(0xffffffffu, send, by); };
+    const bool up = half, up1 = lane & 2, up2 = lane & 1;
+    float4 w[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float4 k = up ? v[2 + i] : v[i], d = up ? v[i] : v[2 + i];
+      w[i] = make_float4(exchange(k.x, d.x, 4), exchange(k.y, d.y, 4), exchange(k.z, d.z, 4), exchange(k.w, d.w, 4));
+    }
+    const float4 k = up1 ? w[1] : w[0], d = up1 ? w[0] : w[1];
+    const float4 y = make_float4(exchange(k.x, d.x, 2), exchange(k.y, d.y, 2), exchange(k.z, d.z, 2), exchange(k.w, d.w, 2));
+    mine = make_float2(g.x + exchange(up2 ? y.z : y.x, up2 ? y.x : y.z, 1), g.y + exchange(up2 ? y.w : y.y, up2 ? y.y : y.w, 1));
+    *reinterpret_cast<float2*>(ss + ((c + 1) & 1) * (N / 8) * WALK_SP + at) = mine;
+    step_sync();  // the new state is here, and the old one is no longer read
+  }
   grid_launch_dependents();
-  if (tid < N) st4(st + (size_t)tid * N, ld4(ss + tid * WALK_COLS));
+  *st = mine;
 }
 
 // Time mixing: every element of the state by itself, four neighbours a thread.
@@ -1110,7 +1161,7 @@ KRK_API int krk_recurrence_chunks(int rule, const void* r, int r_stride, const v
                                   const float* norm_w, float* state, const void* last_rows, int last_stride, int C,
                                   float* last_state, void* out, int out_stride, int out_col, float out_scale, float eps,
                                   float decay_scale, int H, int R, int n_seqs, const int* cu_q, const int* seq_qlen,
-                                  const int* seq_slot, int chunk0, int n_chunks, float* scratch, cudaStream_t stream) {
+                                  const int* seq_slot, int chunk0, int n_chunks, float* scratch, int* error, cudaStream_t stream) {
   if (n_seqs == 0 || n_chunks == 0) return 0;
   int item;
   const uintptr_t rows = (uintptr_t)r | (uintptr_t)k | (uintptr_t)v | (uintptr_t)g | (uintptr_t)rate | (uintptr_t)out;
@@ -1127,7 +1178,7 @@ KRK_API int krk_recurrence_chunks(int rule, const void* r, int r_stride, const v
   a.bonus = bonus; a.norm_w = norm_w; a.state = state; a.last_rows = (const bf16*)last_rows; a.last_stride = last_stride;
   a.C = C; a.last_state = last_state; a.out = (bf16*)out; a.out_stride = out_stride; a.out_col = out_col; a.out_scale = out_scale;
   a.eps = eps; a.decay_scale = decay_scale; a.H = H; a.R = R; a.cu_q = cu_q; a.seq_qlen = seq_qlen; a.seq_slot = seq_slot;
-  a.chunk0 = chunk0; a.n_chunks = n_chunks; a.scratch = scratch;
+  a.chunk0 = chunk0; a.n_chunks = n_chunks; a.scratch = scratch; a.error = error;
   const dim3 items((unsigned)H, (unsigned)n_chunks, (unsigned)n_seqs);
   int rc;
   const size_t RP = (size_t)((R + 7) & ~7);
@@ -1135,8 +1186,16 @@ KRK_API int krk_recurrence_chunks(int rule, const void* r, int r_stride, const v
     // six times three terms of a chunk's rows and the values; two matrices of float32; the small things
     const size_t chunk = 19 * (size_t)L * KP / 2 + 2 * (size_t)L * PITCH + N + 2 * L + 8 * N + 4 * N;
     if ((rc = run(delta_chunk_kernel, items, DELTA_THREADS, chunk, a, stream))) return rc;
-    const size_t walk = (size_t)WALK_STAGES * N * (PITCH + WALK_COLS) + N * WALK_COLS + 4 * N * 4;
-    if ((rc = run(delta_walk_kernel, dim3(N / WALK_COLS, (unsigned)H, (unsigned)n_seqs), THREADS, walk, a, stream))) return rc;
+    // the scratch as rows of N floats: an item's M, then its G
+    CUtensorMap map_m, map_g;
+    const long long scratch_rows = (long long)n_seqs * n_chunks * H * (ITEM_DELTA / N);
+    if (scratch_rows > 0x7fffffffLL) return -2;
+    if ((rc = tc::make_map_f32(&map_m, scratch, scratch_rows, N, N, 32, N, true))) return rc;
+    if ((rc = tc::make_map_f32(&map_g, scratch, scratch_rows, N, N, WALK_COLS, N, false))) return rc;
+    const size_t walk = (WALK_STAGES * (size_t)(WALK_M + WALK_G) + 2 * (N / 8) * WALK_SP) * sizeof(float) + 1024;
+    cudaFuncSetAttribute(delta_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk);
+    if ((rc = (int)launch_pdl(delta_walk_kernel, dim3(N / WALK_COLS, (unsigned)H, (unsigned)n_seqs), dim3(WALK_THREADS), walk, stream, map_m, map_g, a)))
+      return rc;
     return run(delta_finish_kernel, items, THREADS, (size_t)L * PITCH + 4 * L, a, stream);
   }
   const size_t rows_bytes = (size_t)L * KP * sizeof(bf16);  // a term of a chunk's rows

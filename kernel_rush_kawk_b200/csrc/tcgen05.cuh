@@ -247,6 +247,21 @@ inline int make_map_bf16(CUtensorMap* map, const void* base, long long rows, int
   return r == CUDA_SUCCESS ? 0 : -7;
 }
 
+// A row-major [rows, cols] float32 matrix with row stride ld elements, read in boxes of box_rows x box_cols, with the 128-byte
+// swizzle (then box_cols is 32) or as it is.
+inline int make_map_f32(CUtensorMap* map, const void* base, long long rows, int cols, long long ld, int box_cols, int box_rows, bool swizzle) {
+  EncodeTiled fn = encode_fn();
+  if (!fn) return -6;
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
+  cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
+  cuuint32_t elem[2] = {1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, elem,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -7;
+}
+
 // A bfloat16 tensor [n2][n1][n0] (n0 contiguous; strides in elements) read in boxes of box2 x box1 x 64 with
 // the 128-byte swizzle: in shared memory the box is box2 * box1 rows of 128 bytes, the middle index fastest.
 inline int make_map_bf16_3d(CUtensorMap* map, const void* base, long long n0, long long n1, long long n2, long long stride1,

@@ -374,6 +374,27 @@ def test_scans_in_chunks(kind, lens, decays, monkeypatch):
     assert off["chunks"] < 2 * off["tokens"] + 1e-7, off
 
 
+@pytest.mark.parametrize("lens", [[32], [33], [160, 1, 191], [192, 193, 224], [417]])
+def test_the_walk_over_chunks_rounds_its_ring(lens, monkeypatch):
+    """The delta rule's walk, whose ring holds six chunks: sequences of one chunk, of the ring's five to seven, of more than two rounds
+    of it, side by side; the state as the same chunks give it one launch at a time."""
+    rt = runtime(torch.bfloat16)
+    heads = 2
+    x = scan_inputs("delta", lens, heads, "spread", 61)
+    start = rand((len(lens), heads, 64, 64), 71).cuda()
+    want, want_state = scan_in_64_bits("delta", x, lens, heads, start)
+    monkeypatch.setattr(type(rt.ops), "_recurrence_in_chunks", lambda *_: True)
+    got = []
+    for scratch in (1 << 28, 1):
+        monkeypatch.setattr(type(rt.ops), "RECURRENCE_SCRATCH", scratch)
+        state = start.clone()
+        got.append((run_scan(rt, "delta", x, lens, heads, state), state))
+    rt.ops.check()
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert ((got[0][0].double().cpu() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-3 * want.pow(2).mean().sqrt()).all()
+    assert ((got[0][1].double().cpu() - want_state).norm() / want_state.norm()).item() < 1e-6
+
+
 @pytest.mark.parametrize("decays", ["mild", "spread"])
 @pytest.mark.parametrize("kind", ["delta", "wkv"])
 def test_chunks_sum_as_exactly_as_32_bit_multiply_adds(kind, decays, monkeypatch):
