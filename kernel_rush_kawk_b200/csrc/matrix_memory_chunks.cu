@@ -37,7 +37,7 @@ constexpr int L = 64;        // tokens per chunk
 constexpr int PB = 64;       // value columns per block
 constexpr int VPITCH = PB + 8;
 constexpr int APITCH = L + 8;
-constexpr int THREADS = 256;
+constexpr int THREADS = 256, OUT_THREADS = 512;
 constexpr float SAFE = 40.f;
 
 __device__ __forceinline__ float log_sigmoid_f(float z) { return fminf(z, 0.f) - log1pf(expf(-fabsf(z))); }
@@ -100,7 +100,7 @@ __device__ __forceinline__ void chunk_sums(float* F, const float* f, int lane) {
 }
 
 __device__ __forceinline__ void load_values(bf16* vs, const ChunkArgs& a, size_t row0, int h, int p0, int nt) {
-  for (int i = threadIdx.x; i < L * (PB / 8); i += THREADS) {
+  for (int i = threadIdx.x; i < L * (PB / 8); i += blockDim.x) {
     const int s = i / (PB / 8), c = (i % (PB / 8)) * 8;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (s < nt && p0 + c < a.P) v = *reinterpret_cast<const uint4*>(a.v + (row0 + s) * a.v_stride + (size_t)h * a.P + p0 + c);
@@ -268,13 +268,15 @@ __global__ void chunk_walk_kernel(ChunkArgs a) {
 }
 
 // ---- pass 3: the outputs -------------------------------------------------------------------------------------
-// A is formed once per block, each warp one quarter of the tokens against one half of the earlier ones, and left in shared
-// memory; then the block walks its column slices.
+// A is formed once per block, each warp one quarter of the tokens against one quarter of the earlier ones, and left in shared
+// memory; then the block walks its column slices. A block's 109 to 144 KB of shared memory leave an SM two or one: sixteen warps
+// cover one another's reads and barriers, where eight took 73 us (per-channel
+// decays) and 42 (gated) of 1,500 tokens of 8 heads of 128 x 256 and sixteen take 61 and 36.
 template <Kind KIND>
-__global__ void __launch_bounds__(THREADS) chunk_output_kernel(ChunkArgs a) {
+__global__ void __launch_bounds__(OUT_THREADS, KIND == RUNNING_MAX ? 2 : 1) chunk_output_kernel(ChunkArgs a) {
   constexpr bool GATED = KIND == RUNNING_MAX;
   extern __shared__ __align__(16) bf16 sm[];
-  __shared__ float fs[L], is_[L], Fs[L], ms[L], den[2][L];
+  __shared__ float fs[L], is_[L], Fs[L], ms[L], den[4][L];
   const int N = a.N, P = a.P, H = a.H, NP = N + 8;
   constexpr int TERMS = GATED ? 1 : 3;  // of a query's and a key's row in shared memory
   const size_t q_apart = (size_t)L * NP, s_apart = (size_t)N * VPITCH;
@@ -285,7 +287,7 @@ __global__ void __launch_bounds__(THREADS) chunk_output_kernel(ChunkArgs a) {
   bf16* ss = ks;                       // [3][N][VPITCH]
   const int h = blockIdx.y % H, chunk = blockIdx.y / H, seq = blockIdx.z;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int mt = warp & 3, half = warp >> 2;  // 16 tokens; 32 earlier tokens, later 32 of a slice's columns
+  const int mt = warp & 3, part = warp >> 2;  // 16 tokens; 16 earlier tokens, later 16 of a slice's columns
   const int g = lane >> 2, t4 = lane & 3;
   grid_launch_dependents();
   grid_dependency_wait();
@@ -304,7 +306,7 @@ __global__ void __launch_bounds__(THREADS) chunk_output_kernel(ChunkArgs a) {
       ms[threadIdx.x] = gt.w;
     }
     m_before = a.gates[row0 * H + h].z;
-    for (int i = threadIdx.x; i < 2 * L * (N / 8); i += THREADS) {
+    for (int i = threadIdx.x; i < 2 * L * (N / 8); i += OUT_THREADS) {
       const int s = (i / (N / 8)) % L, n = (i % (N / 8)) * 8;
       const bool is_k = i >= L * (N / 8);
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
@@ -316,9 +318,9 @@ __global__ void __launch_bounds__(THREADS) chunk_output_kernel(ChunkArgs a) {
   } else {
     const float* cl = a.cum + (row0 + nt - 1) * H * N + (size_t)h * N;
     int over = 0;
-    for (int n = threadIdx.x; n < N; n += THREADS) over |= !(cl[n] > -SAFE);
+    for (int n = threadIdx.x; n < N; n += OUT_THREADS) over |= !(cl[n] > -SAFE);
     safe = !__syncthreads_or(over);
-    for (int i = threadIdx.x; i < L * (N / 8); i += THREADS) {
+    for (int i = threadIdx.x; i < L * (N / 8); i += OUT_THREADS) {
       const int s = i / (N / 8), n = (i % (N / 8)) * 8;
       float f[8], k8[8];
 #pragma unroll
@@ -342,13 +344,13 @@ __global__ void __launch_bounds__(THREADS) chunk_output_kernel(ChunkArgs a) {
   }
   __syncthreads();
 
-  // A: the warp's 16 tokens against 32 of the chunk's (a tile of later tokens stays zero and is not read)
-  float s[4][4];
+  // A: the warp's 16 tokens against 16 of the chunk's (a tile of later tokens stays zero and is not read)
+  float s[2][4];
 #pragma unroll
-  for (int n = 0; n < 4; ++n)
+  for (int n = 0; n < 2; ++n)
 #pragma unroll
     for (int c = 0; c < 4; ++c) s[n][c] = 0.f;
-  const int u0 = half * 32;
+  const int u0 = part * 16;
   if (safe) {
     for (int kk = 0; kk < N / 16; ++kk) {
       if (u0 >= mt * 16 + 16) break;
@@ -356,26 +358,22 @@ __global__ void __launch_bounds__(THREADS) chunk_output_kernel(ChunkArgs a) {
 #pragma unroll
       for (int t = 0; t < TERMS; ++t)
         ldmatrix_x4(af[t][0], af[t][1], af[t][2], af[t][3], qs + t * q_apart + (mt * 16 + (lane & 15)) * NP + kk * 16 + (lane >> 4) * 8);
+      uint32_t b[TERMS][4];
 #pragma unroll
-      for (int n = 0; n < 4; n += 2) {
-        if (u0 + n * 8 >= mt * 16 + 16) break;  // later tokens
-        uint32_t b[TERMS][4];
+      for (int t = 0; t < TERMS; ++t)
+        ldmatrix_x4(b[t][0], b[t][1], b[t][2], b[t][3],
+                    ks + t * q_apart + (u0 + ((lane >> 4) << 3) + (lane & 7)) * NP + kk * 16 + ((lane >> 3) & 1) * 8);
 #pragma unroll
-        for (int t = 0; t < TERMS; ++t)
-          ldmatrix_x4(b[t][0], b[t][1], b[t][2], b[t][3],
-                      ks + t * q_apart + (u0 + n * 8 + ((lane >> 4) << 3) + (lane & 7)) * NP + kk * 16 + ((lane >> 3) & 1) * 8);
+      for (int sum = TERMS == 1 ? 0 : 2; sum >= 0; --sum)  // small terms first
 #pragma unroll
-        for (int sum = TERMS == 1 ? 0 : 2; sum >= 0; --sum)  // small terms first
-#pragma unroll
-          for (int t = 0; t <= sum; ++t) {
-            mma_bf16_16816(s[n], af[t][0], af[t][1], af[t][2], af[t][3], b[sum - t][0], b[sum - t][1]);
-            mma_bf16_16816(s[n + 1], af[t][0], af[t][1], af[t][2], af[t][3], b[sum - t][2], b[sum - t][3]);
-          }
-      }
+        for (int t = 0; t <= sum; ++t) {
+          mma_bf16_16816(s[0], af[t][0], af[t][1], af[t][2], af[t][3], b[sum - t][0], b[sum - t][1]);
+          mma_bf16_16816(s[1], af[t][0], af[t][1], af[t][2], af[t][3], b[sum - t][2], b[sum - t][3]);
+        }
     }
   } else {
 #pragma unroll
-    for (int n = 0; n < 4; ++n)
+    for (int n = 0; n < 2; ++n)
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const int t = mt * 16 + g + 8 * (c >> 1), u = u0 + n * 8 + 2 * t4 + (c & 1);
@@ -395,7 +393,7 @@ __global__ void __launch_bounds__(THREADS) chunk_output_kernel(ChunkArgs a) {
     const int t = mt * 16 + g + 8 * hh;
     float sum = 0.f;
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
+    for (int n = 0; n < 2; ++n) {
       float v[2];
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
@@ -417,25 +415,25 @@ __global__ void __launch_bounds__(THREADS) chunk_output_kernel(ChunkArgs a) {
       rows[hh] *= t < nt ? expf(Fs[t] + m_before - ms[t]) : 0.f;
       sum += __shfl_xor_sync(0xffffffffu, sum, 1);
       sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-      if (t4 == 0) den[half][t] = sum;
+      if (t4 == 0) den[part][t] = sum;
     }
   }
   __syncthreads();  // A is complete, and the keys are no longer read
   if (GATED && blockIdx.x == 0) {
     const float* n0 = start + (size_t)N * P;
-    for (int t = warp; t < nt; t += THREADS / 32) {
+    for (int t = warp; t < nt; t += OUT_THREADS / 32) {
       float d = 0.f;
       for (int n = lane; n < N; n += 32) d += __bfloat162float(qs[t * NP + n]) * n0[n];
       d = warp_sum(d);
       if (lane == 0)
-        a.den[(row0 + t) * H + h] = den[0][t] + den[1][t] + a.q_scale * expf(Fs[t] + m_before - ms[t]) * d;
+        a.den[(row0 + t) * H + h] = ((den[0][t] + den[1][t]) + (den[2][t] + den[3][t])) + a.q_scale * expf(Fs[t] + m_before - ms[t]) * d;
     }
   }
 
   for (int slice = blockIdx.x * a.slices; slice < (int)(blockIdx.x + 1) * a.slices && slice * PB < P; ++slice) {
     const int p0 = slice * PB;
     load_values(vs, a, row0, h, p0, nt);
-    for (int i = threadIdx.x; i < N * (PB / 8); i += THREADS) {
+    for (int i = threadIdx.x; i < N * (PB / 8); i += OUT_THREADS) {
       const int n = i / (PB / 8), c = (i % (PB / 8)) * 8;
       float f[8];
       if (p0 + c < P) {
@@ -449,9 +447,9 @@ __global__ void __launch_bounds__(THREADS) chunk_output_kernel(ChunkArgs a) {
       split3_store8(f, ss + n * VPITCH + c, s_apart);
     }
     __syncthreads();
-    float acc[4][4];
+    float acc[2][4];
 #pragma unroll
-    for (int n = 0; n < 4; ++n)
+    for (int n = 0; n < 2; ++n)
 #pragma unroll
       for (int c = 0; c < 4; ++c) acc[n][c] = 0.f;
     for (int kk = 0; kk < N / 16; ++kk) {
@@ -459,25 +457,22 @@ __global__ void __launch_bounds__(THREADS) chunk_output_kernel(ChunkArgs a) {
 #pragma unroll
       for (int t = 0; t < TERMS; ++t)
         ldmatrix_x4(af[t][0], af[t][1], af[t][2], af[t][3], qs + t * q_apart + (mt * 16 + (lane & 15)) * NP + kk * 16 + (lane >> 4) * 8);
+      uint32_t b[3][4];
 #pragma unroll
-      for (int n = 0; n < 4; n += 2) {
-        uint32_t b[3][4];
+      for (int t = 0; t < 3; ++t)
+        ldmatrix_x4_trans(b[t][0], b[t][1], b[t][2], b[t][3],
+                          ss + t * s_apart + (kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * VPITCH + (part * 2 + (lane >> 4)) * 8);
 #pragma unroll
-        for (int t = 0; t < 3; ++t)
-          ldmatrix_x4_trans(b[t][0], b[t][1], b[t][2], b[t][3],
-                            ss + t * s_apart + (kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * VPITCH + (half * 4 + n + (lane >> 4)) * 8);
+      for (int sum = 2; sum >= 0; --sum)
 #pragma unroll
-        for (int sum = 2; sum >= 0; --sum)
-#pragma unroll
-          for (int t = 0; t < TERMS; ++t) {
-            if (sum - t < 0) continue;
-            mma_bf16_16816(acc[n], af[t][0], af[t][1], af[t][2], af[t][3], b[sum - t][0], b[sum - t][1]);
-            mma_bf16_16816(acc[n + 1], af[t][0], af[t][1], af[t][2], af[t][3], b[sum - t][2], b[sum - t][3]);
-          }
-      }
+        for (int t = 0; t < TERMS; ++t) {
+          if (sum - t < 0) continue;
+          mma_bf16_16816(acc[0], af[t][0], af[t][1], af[t][2], af[t][3], b[sum - t][0], b[sum - t][1]);
+          mma_bf16_16816(acc[1], af[t][0], af[t][1], af[t][2], af[t][3], b[sum - t][2], b[sum - t][3]);
+        }
     }
 #pragma unroll
-    for (int n = 0; n < 4; ++n)
+    for (int n = 0; n < 2; ++n)
 #pragma unroll
       for (int c = 0; c < 4; ++c) acc[n][c] *= rows[c >> 1];
 #pragma unroll
@@ -487,15 +482,12 @@ __global__ void __launch_bounds__(THREADS) chunk_output_kernel(ChunkArgs a) {
 #pragma unroll
       for (int t = 0; t < 3; ++t)
         ldmatrix_x4(af[t][0], af[t][1], af[t][2], af[t][3], as + (t * L + mt * 16 + (lane & 15)) * APITCH + kk * 16 + (lane >> 4) * 8);
+      uint32_t b0, b1, b2, b3;
+      ldmatrix_x4_trans(b0, b1, b2, b3, vs + (kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * VPITCH + (part * 2 + (lane >> 4)) * 8);
 #pragma unroll
-      for (int n = 0; n < 4; n += 2) {
-        uint32_t b0, b1, b2, b3;
-        ldmatrix_x4_trans(b0, b1, b2, b3, vs + (kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * VPITCH + (half * 4 + n + (lane >> 4)) * 8);
-#pragma unroll
-        for (int t = 2; t >= 0; --t) {
-          mma_bf16_16816(acc[n], af[t][0], af[t][1], af[t][2], af[t][3], b0, b1);
-          mma_bf16_16816(acc[n + 1], af[t][0], af[t][1], af[t][2], af[t][3], b2, b3);
-        }
+      for (int t = 2; t >= 0; --t) {
+        mma_bf16_16816(acc[0], af[t][0], af[t][1], af[t][2], af[t][3], b0, b1);
+        mma_bf16_16816(acc[1], af[t][0], af[t][1], af[t][2], af[t][3], b2, b3);
       }
     }
 #pragma unroll
@@ -504,8 +496,8 @@ __global__ void __launch_bounds__(THREADS) chunk_output_kernel(ChunkArgs a) {
       if (t >= nt) continue;
       float* yr = a.y + ((row0 + t) * H + h) * P;
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        const int p = p0 + half * 32 + n * 8 + 2 * t4;
+      for (int n = 0; n < 2; ++n) {
+        const int p = p0 + part * 16 + n * 8 + 2 * t4;
         if (p < P) *reinterpret_cast<float2*>(yr + p) = make_float2(acc[n][2 * hh], acc[n][2 * hh + 1]);
       }
     }
@@ -835,39 +827,66 @@ __global__ void __launch_bounds__(THREADS, MANY ? 2 : 3) ssd_output_kernel(Chunk
 }
 
 // ---- log decays summed within chunks -------------------------------------------------------------------------
-// cum[row, c]: sum over the chunk's tokens up to the row's of logsigmoid(z) / tau, z = W2 lora + bias
-__global__ void chunk_decays_kernel(float* __restrict__ cum, const bf16* __restrict__ lora, int lora_stride,
-                                    const bf16* __restrict__ w2, const float* __restrict__ bias, float inv_tau, int channels,
-                                    int R, const int* __restrict__ cu_q, const int* __restrict__ seq_qlen) {
-  extern __shared__ __align__(16) float ls[];  // [L][R]
+// cum[row, c]: sum over the chunk's tokens up to the row's of logsigmoid(z) / tau, z = W2 lora + bias. A warp has 32 channels of
+// sixteen tokens, a block the chunk: bound by the chain of a token's logarithm, so the tokens are spread (a thread with all 64 of a
+// channel: 19 us for 1,500 rows of 1,024 channels, 12 here).
+constexpr int DECAY_TOKENS = 16;
+__global__ void __launch_bounds__(32 * L / DECAY_TOKENS)
+chunk_decays_kernel(float* __restrict__ cum, const bf16* __restrict__ lora, int lora_stride, const bf16* __restrict__ w2,
+                    const float* __restrict__ bias, float inv_tau, int channels, int R, const int* __restrict__ cu_q,
+                    const int* __restrict__ seq_qlen) {
+  extern __shared__ __align__(16) float ls[];  // [R][L]
+  __shared__ float total[L / DECAY_TOKENS][32];
   grid_launch_dependents();
   grid_dependency_wait();
-  const int chunk = blockIdx.y, seq = blockIdx.z;
+  const int chunk = blockIdx.y, seq = blockIdx.z, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nt = min(L, seq_qlen[seq] - chunk * L);
   if (nt <= 0) return;
   const size_t row0 = (size_t)cu_q[seq] + chunk * L;
-  for (int i = threadIdx.x; i < nt * R; i += blockDim.x) ls[i] = __bfloat162float(lora[(row0 + i / R) * lora_stride + i % R]);
+  for (int i = threadIdx.x; i < L * R; i += blockDim.x)
+    ls[(i % R) * L + i / R] = i / R < nt ? __bfloat162float(lora[(row0 + i / R) * lora_stride + i % R]) : 0.f;
+  const int c = blockIdx.x * 32 + lane, t0 = warp * DECAY_TOKENS;
+  const bool mine = c < channels;
   __syncthreads();
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= channels) return;
-  const float b = bias[c];
-  float run = 0.f;
-  for (int t0 = 0; t0 < nt; t0 += 16) {
-    float z[16];
+  float z[DECAY_TOKENS];
+  const float b = mine ? bias[c] : 0.f;
 #pragma unroll
-    for (int t = 0; t < 16; ++t) z[t] = b;
-    for (int m = 0; m < R; ++m) {
-      const float w = __bfloat162float(w2[(size_t)c * R + m]);
+  for (int t = 0; t < DECAY_TOKENS; ++t) z[t] = b;
+  const bool wide = R % 8 == 0 && ((uintptr_t)w2 & 15) == 0;
+  for (int m0 = 0; m0 < R; m0 += 8) {
+    float w[8];
 #pragma unroll
-      for (int t = 0; t < 16; ++t) z[t] += w * ls[min(t0 + t, nt - 1) * R + m];
+    for (int j = 0; j < 8; ++j) w[j] = 0.f;
+    if (mine && wide) {
+      widen8(w2 + (size_t)c * R + m0, w);
+    } else if (mine) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (m0 + j < R) w[j] = __bfloat162float(w2[(size_t)c * R + m0 + j]);
     }
 #pragma unroll
-    for (int t = 0; t < 16; ++t)
-      if (t0 + t < nt) {
-        run += log_sigmoid_f(z[t]) * inv_tau;
-        cum[(row0 + t0 + t) * channels + c] = run;
+    for (int j = 0; j < 8; ++j) {
+      if (m0 + j >= R) break;
+#pragma unroll
+      for (int t = 0; t < DECAY_TOKENS; t += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(ls + (m0 + j) * L + t0 + t);
+        z[t] += w[j] * x.x; z[t + 1] += w[j] * x.y; z[t + 2] += w[j] * x.z; z[t + 3] += w[j] * x.w;
       }
+    }
   }
+  float run = 0.f;
+#pragma unroll
+  for (int t = 0; t < DECAY_TOKENS; ++t) {
+    if (t0 + t < nt) run += log_sigmoid_f(z[t]) * inv_tau;
+    z[t] = run;
+  }
+  total[warp][lane] = run;
+  __syncthreads();
+  float before = 0.f;
+  for (int w = 0; w < warp; ++w) before += total[w][lane];
+#pragma unroll
+  for (int t = 0; t < DECAY_TOKENS; ++t)
+    if (mine && t0 + t < nt) cum[(row0 + t0 + t) * channels + c] = before + z[t];
 }
 
 // state-space kind: dt = softplus(raw + bias), log decay -exp(A_log) dt. Not below FORGOTTEN, whose e^ is zero in 32 bits: sums of
@@ -946,7 +965,7 @@ int launch_chunks(ChunkArgs a, int n_seqs, cudaStream_t stream) {
   int rc = (int)launch_pdl(chunk_sum_kernel<KIND>, grid, dim3(THREADS), s1, stream, a);
   if (rc) return rc;
   if ((rc = launch_walk(a, GATED, n_seqs, stream))) return rc;
-  return (int)launch_pdl(chunk_output_kernel<KIND>, grid, dim3(THREADS), s3, stream, a);
+  return (int)launch_pdl(chunk_output_kernel<KIND>, grid, dim3(OUT_THREADS), s3, stream, a);
 }
 
 int launch_ssd(ChunkArgs a, int n_seqs, int live, cudaStream_t stream) {
@@ -1003,8 +1022,9 @@ KRK_API int krk_memory_chunk_decays(float* cum, const void* lora, int lora_strid
   const size_t smem = (size_t)L * R * sizeof(float);
   const int chunks = (max_q_len + L - 1) / L;
   if (smem > 48 * 1024 || chunks > 65535 || n_seqs > 65535) return -2;
-  const dim3 grid((unsigned)((channels + 127) / 128), (unsigned)chunks, (unsigned)n_seqs);
-  return (int)launch_pdl(chunk_decays_kernel, grid, dim3(128), smem, stream, cum, (const bf16*)lora, lora_stride, (const bf16*)w2,
+  cudaFuncSetAttribute(chunk_decays_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024);  // beside the kernel's own
+  const dim3 grid((unsigned)((channels + 31) / 32), (unsigned)chunks, (unsigned)n_seqs);
+  return (int)launch_pdl(chunk_decays_kernel, grid, dim3(32 * L / DECAY_TOKENS), smem, stream, cum, (const bf16*)lora, lora_stride, (const bf16*)w2,
                          bias, 1.0f / tau, channels, R, cu_q, seq_qlen);
 }
 

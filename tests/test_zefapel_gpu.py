@@ -631,3 +631,30 @@ def test_command_line_writes_a_random_model_and_generates_from_it(tmp_path, caps
     assert cli.main(["generate", "--random", "zefapel_tiny", "--weights-seed", "3"] + common) == 0
     from_preset = [json.loads(line) for line in capsys.readouterr().out.strip().splitlines()]
     assert from_folder == from_preset and [len(r["tokens"]) for r in from_folder] == [6, 6]
+
+
+@pytest.mark.parametrize("channels,R", [(32, 16), (40, 5), (1024, 24), (31, 1), (64, 192)])
+def test_log_decays_summed_within_chunks(channels, R):
+    """Widths of the low-rank input that are read in pieces of eight and ones that are not, up to the most that a block holds; channels
+    that do not fill a warp; chunks of 64 tokens, of fewer than a warp's sixteen, and of one: within the rounding of a
+    sum of 64 decays and of R + 1 products each."""
+    rt = runtime(torch.bfloat16)
+    lens = [64, 1, 130, 79]
+    rows = sum(lens)
+    lora, w2 = rand((rows, R + 3), 80).to(torch.bfloat16).cuda(), rand((channels, R), 81, 0.2).to(torch.bfloat16).cuda()
+    bias = rand((channels,), 82).cuda()
+    cu = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device="cuda")
+    n = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    got = torch.zeros((rows, channels), device="cuda")
+    rt.ops._ok(rt.ops.memory.krk_memory_chunk_decays(got.data_ptr(), lora.data_ptr(), R + 3, w2.data_ptr(), bias.data_ptr(), 16.0, channels, R,
+                                                     len(lens), max(lens), cu.data_ptr(), n.data_ptr(), rt.ops._stream()), "decays")
+    z = lora[:, :R].double() @ w2.double().T + bias.double()
+    size = lora[:, :R].double().abs() @ w2.double().T.abs() + bias.double().abs()
+    f = torch.nn.functional.logsigmoid(z) / 16.0
+    at = 0
+    for i in lens:
+        for c in range(at, at + i, 64):
+            e = min(c + 64, at + i)
+            want, most = f[c:e].cumsum(0), (f[c:e].abs() + size[c:e] / 16.0).cumsum(0)
+            assert ((got[c:e].double() - want).abs() <= most * (64 + R + 8) * 2.0 ** -24).all()
+        at += i
