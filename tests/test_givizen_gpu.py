@@ -387,6 +387,43 @@ def test_prompt_attention_on_the_tcgen05_cores(options, heads, kv_heads, D, wind
     assert off[True] <= 1.05 * off[False] + 1e-5, off
 
 
+@pytest.mark.parametrize("cap", [2.0, 30.0, 400.0])
+@pytest.mark.parametrize("D,window", [(128, None), (64, 200)])
+def test_capped_scores_near_and_far_from_the_cap(cap, D, window, monkeypatch):
+    """Tangents by the series (all of a block's scores up to 0.65 of the cap), by the exponential (some beyond) and of both kinds in
+    one sequence: the first 150 tokens' queries are a hundredth of the others'. No further from 64 bits than the mma.sync kernel is, and
+    within the output's rounding."""
+    from kernel_rush_kawk_b200.cache import SequenceCache
+    from kernel_rush_kawk_b200.parts.base import KVNeed
+
+    rt = runtime(torch.bfloat16)
+    heads, kv_heads, n = 4, 2, 290
+    qkv = rand((n, (heads + 2 * kv_heads) * D), 76)
+    qkv[:150, :heads * D] *= 0.01
+    qkv = qkv.to(torch.bfloat16).cuda()
+    slopes = (2.0 ** -torch.arange(1.0, heads + 1)).cuda()
+    monkeypatch.setattr(type(rt.ops), "SINK_TCGEN05_ROWS", 1)
+    q, k, v = split_qkv(qkv, heads, kv_heads, D)
+    want = attention_in_64_bits(q, k, v, 0, 0.3, window, None, slopes.double().cpu(), cap).reshape(n, -1)
+    off = {}
+    for tcgen05 in (True, False):
+        monkeypatch.setattr(type(rt.ops), "SINK_TCGEN05_KEYS", 1 if tcgen05 else 1 << 30)
+        cache = SequenceCache([KVNeed(kv_heads, D, window)], 512, 1, 512, rt.device, torch.bfloat16, step_tokens=n)
+        slot = cache.alloc()
+        cache.reserve(slot, n)
+        cache.sync()
+        ctx = context(rt, [slot], [0], [n], cache)
+        out = torch.zeros((n, heads * D), dtype=torch.bfloat16, device="cuda")
+        rt.ops.rotate_norm_write(qkv, 0, heads * D, (heads + kv_heads) * D, heads, kv_heads, D, D, torch.zeros(2, device="cuda"), 0, None,
+                                 ctx.batch, cache.view(0))
+        rt.ops.sink_attention(qkv, 0, heads, D, D, None, 0.3, window, ctx.batch, cache.view(0), out, 0, 1.0, slopes=slopes, softcap=cap)
+        rt.ops.check()
+        diff = out.double().cpu() - want
+        assert (diff.abs() <= 2.0 ** -8 * want.abs() + 1e-4).all(), (tcgen05, diff.abs().max())
+        off[tcgen05] = (diff.norm() / want.norm()).item()
+    assert off[True] <= 1.05 * off[False] + 1e-5, off
+
+
 def windowed_prompt(rt, qkv, heads, kv_heads, D, window, sink, cache, slot, start, slopes=None):
     """One step of one sequence: its keys and values into the cache, then the attention of its queries."""
     n = qkv.shape[0]
