@@ -48,7 +48,7 @@ _SIGNATURES = {
     "krk_select_tokens": [_P, _P, c_int, c_int, c_float, c_uint, _P, c_uint, _P, _P, _P, _P, _P],
     "krk_gemm_tcgen05": [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, _P],
     "krk_selftest_wait_runs_out": [_P, c_int, _P],
-    "krk_skinny_linear": [_P, _P, _P, _P, _P, _P, c_int, _P, c_int, c_int, c_int, c_float, c_int, c_int, _P],
+    "krk_skinny_linear": [_P, _P, _P, c_int, c_int, c_int, c_float, c_int, c_int, _P],
     "krk_lt_gemm_bf16": [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, _P],
     "krk_lt_gemm_report": [_P, _P],
 }
@@ -182,9 +182,6 @@ class Kernels:
     libraries are needed (compiled at first use)."""
 
     SKINNY_MAX_ROWS = 16  # rows up to which the fused skinny kernels serve a bfloat16 product
-    # Every block of a skinny product redoes the norm of all rows in its prologue. That is
-    # cheaper than a separate norm kernel for one or two rows and dearer beyond.
-    FUSED_NORM_MAX_ROWS = 2
 
     def __init__(self, head_dims=(), device="cuda:0"):
         if not torch.cuda.is_available():
@@ -345,22 +342,12 @@ class Kernels:
         return out
 
     def _skinny(self, x, w, out_dtype, swiglu_rows=0, gate_act=1, act_limit=0.0):
-        """x: a tensor or a Normed not yet computed (then the add and the norm run in
-        the kernel's prologue)."""
-        lazy = not isinstance(x, torch.Tensor)
-        src = x.x if lazy else x
-        M, K = src.shape
+        M, K = x.shape
         N = swiglu_rows if swiglu_rows else w.shape[0]
-        out = torch.empty((M, N), dtype=out_dtype, device=src.device)
-        branch = x.branch if lazy else None
-        gain = x.gain if lazy else None
-        x_new = x.x_new if lazy and x.branch is not None else None
+        out = torch.empty((M, N), dtype=out_dtype, device=x.device)
         self._ok(self.core.krk_skinny_linear(
-            out.data_ptr(), src.data_ptr(), w.data_ptr(), _ptr(branch), _ptr(gain), _ptr(x_new),
-            int(gain is not None and gain.dtype == torch.float32), None, M, N, K, float(x.eps) if lazy else float(act_limit),
+            out.data_ptr(), x.data_ptr(), w.data_ptr(), M, N, K, float(act_limit),
             int(gate_act if swiglu_rows > 0 or gate_act == 4 else 0), _code(out_dtype), self._stream()), "skinny product")
-        if lazy:
-            x.mark_fused()
         return out
 
     def _use_skinny(self, x, w) -> bool:
@@ -368,29 +355,11 @@ class Kernels:
         return (self.has_skinny and w.dtype == torch.bfloat16 and 0 < rows <= self.SKINNY_MAX_ROWS
                 and w.shape[1] % 32 == 0 and w.is_contiguous())
 
-    @staticmethod
-    def _fits_prologue(x) -> bool:
-        """Whether the normalised rows fit the fused kernel's shared memory."""
-        rows, k = x.shape
-        if rows > Kernels.FUSED_NORM_MAX_ROWS:
-            return False
-        tiles = 1 if rows <= 8 else 2
-        return 65536 + rows * (k + 64) * 2 + 8 * 2 * tiles * 512 <= 216 * 1024
-
-    def _skinny_input(self, x):
-        """A Normed goes to the kernel as it is if its norm is still to be done and fits
-        the prologue; otherwise its rows are computed first."""
-        if isinstance(x, torch.Tensor):
-            return x
-        if x.done or not self._fits_prologue(x):
-            return x.tensor()
-        return x
-
     def linear(self, x, w, out_float32=False):
         """y = x W^T; W is [out, in]. x may be a Normed (see parts/norm.py)."""
         out_dtype = torch.float32 if out_float32 else w.dtype
         if self._use_skinny(x, w):
-            return self._skinny(self._skinny_input(x), w, out_dtype)
+            return self._skinny(self._resolve(x), w, out_dtype)
         x = self._resolve(x)
         if x.shape[0] == 0:
             return torch.empty((0, w.shape[0]), dtype=out_dtype, device=x.device)
@@ -425,7 +394,7 @@ class Kernels:
 
     def gate_up_swiglu(self, h, w_gate_up, intermediate):
         if self._use_skinny(h, w_gate_up):
-            return self._skinny(self._skinny_input(h), w_gate_up, w_gate_up.dtype, swiglu_rows=intermediate)
+            return self._skinny(self._resolve(h), w_gate_up, w_gate_up.dtype, swiglu_rows=intermediate)
         return self.swiglu(self.linear(h, w_gate_up), intermediate)
 
     # -- attention ------------------------------------------------------------------

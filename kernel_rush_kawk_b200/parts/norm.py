@@ -15,10 +15,8 @@ from .base import Norm, Stream, TensorSpec, register_norm
 class Normed:
     """Rows that a norm produces, computed on demand.
 
-    A consumer either calls ``tensor()`` (the norm kernel runs once) or hands the
-    object to ``ops.linear`` and friends, which may fold the add and the norm
-    into their own prologue when few rows are in flight. Either way the new
-    residual stream ``x_new`` is written exactly once."""
+    A consumer calls ``tensor()`` or hands the object to ``ops.linear`` and friends, which do. The norm kernel
+    runs once, however many ask, and the new residual stream ``x_new`` is written exactly once."""
 
     __slots__ = ("ops", "x", "branch", "gain", "eps", "x_new", "_rows")
 
@@ -48,7 +46,7 @@ class Normed:
         return self._rows
 
     def mark_fused(self, rows=True) -> None:
-        """Called by a kernel wrapper that did the add and the norm itself."""
+        """Called by whoever did the add and the norm itself."""
         self._rows = rows
 
 

@@ -115,7 +115,7 @@ class WideRMSNorm(Norm):
         out = []
         for r, g in zip(rows if gain2 is not None else (rows,), (self.gain, gain2)):
             normed = Normed(ctx.ops, x, branch, g, self.eps, x_new)
-            normed.mark_fused(r)  # computed here and now: a product never folds this norm into its prologue
+            normed.mark_fused(r)  # computed here and now
             out.append(normed)
         stream.x = x_new
         stream.rows = None
