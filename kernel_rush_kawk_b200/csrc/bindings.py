@@ -430,14 +430,18 @@ class Kernels:
             n = batch.n_seqs
             out = torch.empty((n, heads * head_dim), dtype=qkv.dtype, device=qkv.device)
             row_tiles = -(-(heads // cache.kv_heads) // 16)
-            # key splits (blocks per cluster) by the number of (sequence, kv head, row tile) items alone,
-            # never by lengths, so a captured step stays valid; measured best on B200 at 1, 2 to 4, 8, 16 and 32 or
-            # 64 sequences of the 4B shape: 16, 8, 4, 2 and 1 (one block per item runs a deeper page pipeline). One
-            # sequence has eight items: sixteen splits are 128 blocks where eight are 64, and what bounds the
-            # kernel is the bytes its blocks have in flight (one step of the 4B shape at 32,000 tokens of context:
-            # 4.41 -> 3.14 ms, at 8,000: 2.51 -> 2.17, at 1,000: 1.93 -> 1.91; at two sequences sixteen gain nothing)
+            # key splits (blocks per cluster) by the number of (sequence, kv head, row tile) items alone, never by
+            # lengths, so a captured step stays valid: as many as one wave of the kernel's blocks has room for. Two
+            # blocks share an SM, so 148 items split in two still start at once; a layer of the 4B shape at 19, 20
+            # and 24 sequences of 500 tokens takes 84.6, 86.4 and 85.0 us in two splits and 77.5, 77.9 and 79.2 in
+            # one (18 sequences: 76.0 and 77.4; after 100 tokens 78.4 against 68.3 at 20, after 1,500 102.2 against
+            # 96.4). Clusters of four do not fill every SM: 8 sequences 51.3 us in four splits, 53.0 in two; 9 take
+            # 61.6 and 56.7 (after 100 tokens 57.4 and 52.0, after 1,500 70.2 and 65.6). Four sequences 48.7 us in four,
+            # 47.3 in eight; five 49.4 and 53.4. One sequence has eight items: sixteen splits are 128 blocks where
+            # eight are 64, and what bounds the kernel is the bytes its blocks have in flight (one step of the 4B
+            # shape at 32,000 tokens of context: 4.41 -> 3.14 ms, at 8,000: 2.51 -> 2.17, at 1,500 the same)
             items = n * cache.kv_heads * row_tiles
-            splits = 16 if items <= 9 else 8 if items <= 37 else 4 if items <= 74 else 2 if items <= 192 else 1
+            splits = 16 if items <= 9 else 8 if items <= 37 else 4 if items <= 64 else 2 if items <= 148 else 1
             gain = q_gain if q_gain is not None else k_gain
             n_pos = cos.shape[0] if cos is not None else 0x7fffffff
             if (splits in self.tma_decode_splits and self.use_tma_decode_attention and head_dim % 64 == 0
