@@ -319,9 +319,19 @@ int launch(void* out, const void* x, const void* W, int M, int N, int K, float l
 
 template <int NT, int SWIGLU, typename TOut>
 int pick_rt(void* out, const void* x, const void* W, int M, int N, int K, float limit, cudaStream_t stream) {
-  // two row tiles per block when that still leaves a few blocks for each of the 148 SMs
-  if (!SWIGLU && N >= 16 * 2 * 296)
-    return launch<NT, 2, SWIGLU, TOut>(out, x, W, M, N, K, limit, stream);
+  if constexpr (!SWIGLU) {
+    // Two row tiles a block where the blocks of one tile would be more than three an SM: a block asks for the batch rows' pieces beside
+    // every weight tile's, and two tiles share them. us at 16 rows, one tile / two: 7,168 outputs of 5,120 19.5 / 15.7, 8,192 of
+    // 2,560 11.3 / 8.7, 9,216 of 12,288 47.6 / 42.3; at 8 rows 16.4 / 13.9, 9.3 / 7.9, 42.6 / 40.1; at one 13.5 / 12.9, 7.8 / 7.3, 39.4 / 39.2.
+    const int tiles = (N + 15) / 16, pairs = (N + 31) / 32;
+    if (tiles > 3 * 148) return launch<NT, 2, SWIGLU, TOut>(out, x, W, M, N, K, limit, stream);
+    // Between two and three blocks of one tile an SM, and long rows: two tiles a block as well, and K split three ways over a cluster, while
+    // that leaves room for the clusters' placing (500 of 592 blocks; 528 ran over). us, one tile / two split: 5,120 outputs of 5,120 at 16
+    // rows 13.6 / 11.8, at 8 11.9 / 10.4, at one 10.3 / 10.0; of 17,408 43.9 / 37.7, 36.7 / 34.3, 33.1 / 33.0. (Two ways, for 6,144 outputs,
+    // gained alone, 7.2 -> 6.7 at 8 rows of 2,560, and lost in a step, 51.6 -> 52.4 a layer.)
+    if (tiles > 2 * 148 && pairs * 3 <= 500 && K >= 5120)
+      return launch_warps<4, NT, 2, SWIGLU, TOut, false, 3, (NT == 1 ? 8 : 6)>(out, x, W, M, N, K, limit, stream);
+  }
   return launch<NT, 1, SWIGLU, TOut>(out, x, W, M, N, K, limit, stream);
 }
 

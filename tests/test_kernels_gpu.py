@@ -151,6 +151,20 @@ def test_float32_products_of_several_threads(ops):
     assert all(torch.equal(out, want[out.shape[0]]) for out in outs.values())
 
 
+@pytest.mark.parametrize("rows", [1, 8, 9, 16])
+@pytest.mark.parametrize("nk", [(4752, 5120), (4753, 5152), (5312, 5120), (5313, 5120), (7104, 96), (7105, 96), (9457, 2080)])
+def test_few_row_products_of_two_tiles_a_block(ops, rows, nk):
+    """Output counts on both sides of each line of the few-row products' forms (two row tiles a block, K split three ways), with
+    sums of whole numbers below 2^24: they are exact in any order, so a tile, a slice or a row in the wrong place shows."""
+    n, k = nk
+    g = torch.Generator("cuda").manual_seed(n + rows)
+    x = torch.randint(-2, 3, (rows, k), generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randint(-2, 3, (n, k), generator=g, device="cuda").to(torch.bfloat16)
+    want = (x.double() @ w.double().t()).float()
+    assert torch.equal(ops.linear(x, w, out_float32=True), want)
+    assert torch.equal(ops.linear(x, w), want.to(torch.bfloat16))
+
+
 @pytest.mark.parametrize("mnk", [(1, 2560, 9728), (8, 2560, 4096), (16, 2560, 9728), (13, 1000, 2080), (3, 48, 2048),
                                  (9, 2000, 4128)])
 def test_few_row_products_that_split_k_over_a_cluster(ops, mnk):
