@@ -948,31 +948,33 @@ class Kernels:
     @staticmethod
     def _few_experts(x, w_first, w_down, rows, top) -> bool:
         """Whether the experts' products of few rows run once per expert (csrc/few_experts.cu): type, sizes, the alignment of rows
-        and weights, choices that the sum by rows holds, and pairs enough (16 experts of 1,536 x 3,072, two a row: 2 pairs
-        27.3 us by pair and 30.8 by expert, 4 pairs 41.5 and 46.2, 8 pairs 68 and 58; 64 of 2,048 x 1,408, six a row: 6 pairs
-        54 and 50)."""
+        and weights, choices that the sum by rows holds, and more than one pair (by pair and by expert, us: 16 experts of 1,536 x
+        3,072, two a row, 2 pairs 23 and 16, 4 pairs 36 and 26; 64 of 2,048 x 1,408, two a row, 2 pairs 17 and 13; 64 of 1,024 x 256 8.6 and
+        8.6; one pair of 16 of 1,024 x 1,024 8 and 9, of 64 of 2,048 x 1,408 14 and 11)."""
         return (x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and w_down.shape[2] % 8 == 0 and x.stride(0) % 8 == 0
-                and (x.data_ptr() | w_first.data_ptr() | w_down.data_ptr()) % 16 == 0 and top <= 32 and 6 <= rows * top <= Kernels.FEW_EXPERTS_PAIRS)
+                and (x.data_ptr() | w_first.data_ptr() | w_down.data_ptr()) % 16 == 0 and top <= 32 and 2 <= rows * top <= Kernels.FEW_EXPERTS_PAIRS)
 
     @staticmethod
     def _grouped_from(E, F, C, gated) -> int:
-        """Pairs from which the two grouped launches, which need the pairs ordered and their rows gathered first, are faster than a
-        block per 32 rows of an expert's matrix. Those read an expert's weights once for sixteen of its rows, at 4.9 TB/s where a
-        block has 64 KB of them and more; the grouped ones stream them at 6 where their tiles, of 128 or 256 columns, fill the rounds
-        of 74 pairs of blocks. Pairs an expert at which they meet in a single-token step, and both sides below and above:
-        128 experts of 768 x 2,048 (tiles 768) 0.6: at 0.5 101 and 106 us, 1 161 and 142; 128 of 512 x 1,024 (512) 0.75: 0.5 49 and 53,
-        1 78 and 71; 64 of 1,408 x 2,048 (512) 0.6: 0.75 117 and 114, 3 193 and 183, 6 216 and 188; 64 of 768 x 1,536 (384) 4.5: 3 89
-        and 92, 9 118 and 100; 64 of 640 x 1,280 (320) 4: 3 73 and 78, 4.5 80 and 78, 9 93 and 78; 48 of 1,024 x 1,536 (288) 5;
-        32 of 1,536 x 2,048 (256) 7, of 3,072 x 2,048 (256) 0.9, of 2,048 x 1,024 (128, two rounds nearly full) 2.2: 2 78 and 81, 6 97
-        and 85; of 768 x 1,536 (192) 10: 8 56 and 61, 12 67 and 61; 16 of 3,072 x 1,536 (96) 11: 8 91 and 103, 12 109 and 104; 16
-        of 1,024 x 1,024 13, of 512 x 1,024 17, 8 of 2,048 x 1,024 16. Blocks of 20 to 40 KB in many rounds of their own: 128 of 128 x
-        1,024 1: 4 58 and 48, 8 68 and 49; 64 of 256 x 1,024 5: 4 39 and 41, 8 45 and 42; not 64 of 128 x 512, 1,280 blocks in all, 12."""
+        """Pairs from which the two grouped launches, which need the pairs ordered and their rows gathered first, are faster than
+        blocks that walk over 32 rows of an expert's matrix at a time. Those read an expert's weights once for sixteen of its rows, at
+        5.7 TB/s and more beyond a hundred MB; the grouped ones stream them at 6 where their tiles, of 128 or 256 columns, fill the rounds
+        of 74 pairs of blocks. Pairs an expert at which they meet in a single-token step, and both sides (walk and grouped, us) below and
+        above: 64 experts of 1,408 x 2,048 (tiles 512) 4: at 3 167 and 174, 6 194 and 187; of 2,112 x 2,048 (512) 3.5: 3 244 and 249, 4.5 266
+        and 261; 128 of 768 x 2,048 (768) 3: 2 174 and 193, 4.5 211 and 209; 128 of 512 x 1,024 (512) 4.5: 3 88 and 92, 6 99 and 92; 256 of
+        512 x 2,048 (1,024) 2.3: 2 229 and 239, 3 270 and 257; 64 of 768 x 1,536 (384) 11: 9 99 and 102, 12 105 and 103; 64 of 640 x 1,280
+        (320) 10: 9 78 and 80, 12 85 and 80; 48 of 1,024 x 1,536 (288) 10; 32 of 1,536 x 2,048 (256) 11, of 3,072 x 2,048 (256) 9, of
+        2,048 x 1,024 (128) 9: 8 86 and 87, 12 95 and 87; 16 of 6,144 x 2,048 (128) 6; of 3,072 x 1,536 (96) 13: 12 92 and 105, 16 113 and
+        105; 32 of 768 x 1,536 (192) 13; 16 of 1,024 x 1,024 13, 8 of 2,048 x 1,024 15. Many units of 20 to 40 KB: 128 of 128 x 1,024 2.5:
+        2 40 and 45, 4.5 53 and 48; 64 of 256 x 1,024 4.7: 3 33 and 40, 6 43 and 41; not 64 of 128 x 512, 1,280 units in all, 8."""
         tiles = E * min(-(-F // (128 if gated else 256)), -(-C // 256))
-        if tiles >= 296:  # four rounds; six
-            return E if tiles >= 444 else 9 * E // 2
-        blocks, size = E * -(-(F + C) // 32), 2 * E * F * C * (3 if gated else 2)
-        if (tiles >= 111 and size >= 300e6) or (blocks >= 16 * 148 and size < 65536 * blocks):
-            return 5 * E
+        if tiles >= 444:  # six rounds
+            return 7 * E // 2
+        units, size = E * -(-(F + C) // 32), 2 * E * F * C * (3 if gated else 2)
+        if units >= 16 * 148 and size < 65536 * units:
+            return 4 * E
+        if tiles >= 111 and size >= 300e6:
+            return 9 * E
         return 12 * E
 
     @staticmethod

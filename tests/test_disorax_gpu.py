@@ -399,6 +399,27 @@ def test_products_of_few_experts_rows(gated, activation, weigh_input, sizes, row
     assert off[True] < 1e-2, off
 
 
+@pytest.mark.parametrize("rows,top,E", [(32, 1, 2), (11, 3, 40), (16, 2, 5), (200, 2, 5), (512, 8, 3), (129, 31, 70), (1000, 4, 3000)])
+@pytest.mark.parametrize("K,F", [(8, 33), (776, 40), (1544, 70)])
+def test_units_of_few_experts_rows(rows, top, E, K, F):
+    """Every block finds its own share of the units (32 rows of an expert's matrix and up to sixteen of its pairs): up to 32 pairs
+    and more, the same expert in many passes and in none, choices that are none, shares that end within an expert. Sums of whole
+    numbers below 2^24, exact in any order: a pair or a tile left out or in another block's place shows."""
+    ops = runtime(torch.bfloat16).ops
+    g = torch.Generator("cuda").manual_seed(rows + K)
+    x = torch.randint(-2, 3, (rows * top, K), generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randint(-2, 3, (min(E, 70), F, K), generator=g, device="cuda").to(torch.bfloat16)
+    experts = torch.randint(-1, min(E, 70), (rows, top), generator=g, device="cuda").to(torch.int32)
+    got = torch.full((rows * top, F), 7.0, dtype=torch.bfloat16, device="cuda")
+    assert ops.moe.krk_few_experts(got.data_ptr(), x.data_ptr(), K, w.data_ptr(), experts.data_ptr(), rows, top, E, F, K, 2, 0, None, 0.0,
+                                   0.0, ops._stream()) == 0
+    flat, want = experts.view(-1).long(), torch.full((rows * top, F), 7.0, device="cuda")
+    for e in range(w.shape[0]):
+        mine = flat == e
+        want[mine] = (x[mine].double() @ w[e].double().t()).float()
+    assert torch.equal(got, want.to(torch.bfloat16))
+
+
 @pytest.mark.parametrize("odd", ["first", "second", "choices"])
 def test_few_experts_rows_with_weights_off_a_16_byte_boundary_or_many_choices(odd):
     """What the product per expert does not take goes to the kernels that read an expert per pair: weights that start at an
