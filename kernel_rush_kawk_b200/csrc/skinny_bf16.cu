@@ -15,7 +15,7 @@
 // Epilogue (swiglu): rows n and N + n of W are gate and up; out = round(round(silu(round(g))) * round(u))
 // (gemm.py:108-113).
 //
-// The residual add and the RMSNorm before a product stay a kernel of their own (rows.cu), although the reference
+// The residual add and the RMSNorm before a product stay a kernel of their own (elementwise.cu), although the reference
 // folds them into its product (gemm.py:22-51): done in every block's prologue they stand between the block's first
 // weights and its first use of them, while the separate kernel runs under the ring-fulls that these blocks have asked
 // for already. Measured, a captured layer after 500 tokens, prologue against kernel: 4B shape 47.3 / 45.3 us at one
