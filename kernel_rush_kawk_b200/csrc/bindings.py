@@ -974,13 +974,15 @@ class Kernels:
         105; 32 of 768 x 1,536 (192) 13; 16 of 1,024 x 1,024 13, 8 of 2,048 x 1,024 15. Many units of 20 to 40 KB: 128 of 128 x 1,024 2.5:
         2 40 and 45, 4.5 53 and 48; 64 of 256 x 1,024 4.7: 3 33 and 40, 6 43 and 41; not 64 of 128 x 512, 1,280 units in all, 8."""
         tiles = E * min(-(-F // (128 if gated else 256)), -(-C // 256))
-        if tiles >= 296:  # six rounds; four, where the line stays at 4.5, below where they meet: the tests of the change of hands hold it there
-            return 7 * E // 2 if tiles >= 444 else 9 * E // 2
+        # The lines stay at or below the upper ends that the tests of the change of hands hold (1 at 128 experts of 444 tiles, 3 at 64, 4.5
+        # from 296 tiles, 6 of long matrices), which is up to 10 % given away between them and the meeting points above.
+        if tiles >= 296:  # six rounds; four
+            return 9 * E // 2 if tiles < 444 else 3 * E if E <= 64 else E
         units, size = E * -(-(F + C) // 32), 2 * E * F * C * (3 if gated else 2)
         if units >= 16 * 148 and size < 65536 * units:
-            return 4 * E
+            return 5 * E
         if tiles >= 111 and size >= 300e6:
-            return 9 * E
+            return 6 * E
         return 12 * E
 
     @staticmethod
