@@ -241,7 +241,9 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     if (warp == 8) {
     if (lane == 0) {
       // ---- issuer: TMA loads and MMAs ----
-      constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(KEYS >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
+      // a negative scale: the products leave negated (the descriptor's bit for A), and the softmax takes the scale's size, so that maxima
+      // before it are maxima after it and a score that is not seen is minus infinity
+      const uint32_t idesc_s = (!WIDE && scale_log2 < 0.f ? 1u << 13 : 0u) | (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(KEYS >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
       constexpr uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(D >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
       bool ok = true;
       auto give_up = [&](int code) { atomicExch(error, code); ok = false; };
@@ -369,8 +371,9 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
       }
       if (SHAPED && ex.slopes) slope = ex.slopes[head] * LOG2E;
     }
-    const float2 scale2 = make_float2(scale_log2, scale_log2);
-    const uint32_t unseen = scale_log2 < 0.f ? 0x7f800000u : 0xff800000u;  // a score whose weight is zero
+    const float scale_size = WIDE ? scale_log2 : fabsf(scale_log2);  // a negative scale's sign is in the scores already
+    const float2 scale2 = make_float2(scale_size, scale_size);
+    constexpr uint32_t unseen = 0xff800000u;  // minus infinity: a score whose weight is zero
     bool ok = true;
     for (int j = rng.lo; j <= rng.hi; ++j) {
       const int key0 = j * KEYS;
@@ -443,7 +446,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
 #pragma unroll
           for (int q = 0; q < 4; ++q) mx4[q] = fmaxf(fmaxf(mx4[q], __uint_as_float(s[i + q])), __uint_as_float(s[i + 4 + q]));
       const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      const float m_new = fmaxf(m, SHAPED ? mx : mx * scale_log2);
+      const float m_new = fmaxf(m, SHAPED ? mx : mx * scale_size);
       const bool outgrown = m != -INFINITY && m_new - m > RESCALE_STEP;
       if (__any_sync(0xffffffffu, outgrown)) {
         // the warp moves its rows' reference maxima and scales its rows of O; the block's P.V has not been issued and the

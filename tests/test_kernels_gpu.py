@@ -664,6 +664,24 @@ def test_tcgen05_prefill_attention_of_any_group(ops, group, scale, size):
     close(got, ref.attention(qkv, heads, kv_heads, D, batch, cache, scale, None), dtype, f"group {group} scale {scale}")
 
 
+@pytest.mark.parametrize("heads,kv_heads,D", [(6, 2, 64), (8, 2, 128), (258, 2, 64)])
+@pytest.mark.parametrize("window", [None, 100, 200, 300, 351])
+def test_tcgen05_prefill_attention_of_a_negative_scale(ops, heads, kv_heads, D, window):
+    """A scale below zero with windows that put a row's first keys in a block it sees in part and its next ones in blocks it sees
+    whole, and rows of a tile whose first block holds none of their keys: the largest weight is then the smallest product's. Scores large
+    enough that a row's maximum taken from the wrong end would leave weights of 2^20 and more, or none."""
+    dtype, scale = torch.bfloat16, -1.0 / 16.0
+    cache = make_cache(34, kv_heads, D, 3, 10, dtype, 90)
+    cache.window = window
+    batch = make_batch([1, 2, 0], [0, 150, 77], [420, 259, 64])
+    qkv = rand((batch.n_rows, (heads + 2 * kv_heads) * D), dtype, 91, 2.0)
+    ops.qk_norm_rope_write(qkv, heads, kv_heads, D, None, None, 1e-6, None, None, batch, cache)
+    got = ops.attention(qkv, heads, kv_heads, D, batch, cache, scale, window)
+    ops.check()
+    want = TorchOps(dtype).attention(qkv, heads, kv_heads, D, batch, cache, scale, window)
+    close(got, want, dtype, f"scale {scale} window {window}")
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("q_len", [1, 37])
 def test_one_far_key_among_hundreds_decides(ops, dtype, q_len):
