@@ -404,6 +404,11 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         };
         if constexpr (SHAPE == 2) {
           float most = 0.f;
+          if (!whole) {  // by the scores that count alone: a row's bits do not depend on what lies in pages and rows that it does not see
+#pragma unroll
+            for (int i = 0; i < KEYS; ++i)
+              if ((unsigned)i - first > span) s[i] = 0u;
+          }
 #pragma unroll
           for (int i = 0; i < KEYS; i += 2) most = fmaxf(fmaxf(most, fabsf(__uint_as_float(s[i]))), fabsf(__uint_as_float(s[i + 1])));
           if (__any_sync(0xffffffffu, most > ex.small)) {

@@ -445,6 +445,57 @@ def split_qkv(qkv, heads, kv_heads, D):
             d[:, (heads + kv_heads) * D:].view(-1, kv_heads, D))
 
 
+@pytest.mark.parametrize("heads,kv_heads,D", [(6, 2, 128), (8, 2, 64), (86, 2, 64)])
+@pytest.mark.parametrize("unseen", ["page tail", "next sequence", "later keys", "before the window"])
+def test_capped_scores_do_not_depend_on_what_a_row_does_not_see(heads, kv_heads, D, unseen, monkeypatch):
+    """Which form of the tangent a block of scores takes is decided by the scores that count: the same bits whatever lies in the
+    rest of the last page, with or without another sequence's loud queries in the tile, whatever keys come after a warp's rows, and
+    whatever lies before their window. All scores that count are far below the cap, those that don't far above it."""
+    from kernel_rush_kawk_b200.cache import SequenceCache
+    from kernel_rush_kawk_b200.parts.base import KVNeed
+
+    rt = runtime(torch.bfloat16)
+    monkeypatch.setattr(type(rt.ops), "SINK_TCGEN05_ROWS", 1)
+    monkeypatch.setattr(type(rt.ops), "SINK_TCGEN05_KEYS", 1)
+    window, n, W = 200, 290, (heads + 2 * kv_heads) * D
+    same = slice(0, n)
+    quiet = rand((n, W), 77)
+    quiet[:, :heads * D] *= 0.01
+    keys = slice(heads * D, (heads + kv_heads) * D)
+
+    def run(rows, stale, beside):
+        lens = [n] + ([70] if beside else [])
+        qkv = rows
+        if beside:
+            loud = rand((70, W), 78)
+            loud[:, :heads * D] *= 20.0
+            qkv = torch.cat([rows, loud])
+        qkv = qkv.to(torch.bfloat16).cuda()
+        cache = SequenceCache([KVNeed(kv_heads, D, window)], 512, 2, 512, rt.device, torch.bfloat16, step_tokens=512)
+        slots = [cache.alloc() for _ in lens]
+        for slot, a in zip(slots, lens):
+            cache.reserve(slot, a)
+        cache.sync()
+        ctx = context(rt, slots, [0] * len(lens), lens, cache)
+        cache.view(0).k.fill_(stale)
+        out = torch.zeros((qkv.shape[0], heads * D), dtype=torch.bfloat16, device="cuda")
+        rt.ops.rotate_norm_write(qkv, 0, heads * D, (heads + kv_heads) * D, heads, kv_heads, D, D, torch.zeros(2, device="cuda"), 0, None,
+                                 ctx.batch, cache.view(0))
+        rt.ops.sink_attention(qkv, 0, heads, D, D, None, 0.3, window, ctx.batch, cache.view(0), out, 0, 1.0, softcap=30.0)
+        rt.ops.check()
+        return out[:n]
+
+    want, other = run(quiet, 0.0, False), quiet.clone()
+    if unseen == "later keys":
+        other[100:128, keys] = 200.0  # the warps' rows of tokens up to 63 see none of them
+        same = slice(0, 64)
+    if unseen == "before the window":
+        other[:20, keys] = 200.0  # tokens from 220 on see none of them; 31 tokens are the most that share a warp with one that does
+        same = slice(256, n)
+    got = run(other, 300.0 if unseen == "page tail" else 0.0, unseen == "next sequence")
+    assert torch.equal(got[same], want[same])
+
+
 @pytest.mark.parametrize("tcgen05", [True, False])
 @pytest.mark.parametrize("biased", [False, True])
 @pytest.mark.parametrize("D", [64, 128])
