@@ -496,6 +496,44 @@ def test_capped_scores_do_not_depend_on_what_a_row_does_not_see(heads, kv_heads,
     assert torch.equal(got[same], want[same])
 
 
+@pytest.mark.parametrize("total", [2048, 8192, 16384])
+def test_row_sums_over_many_equal_scores(total, monkeypatch):
+    """Thousands of equal weights: every addition to a row's sum rounds the same way while the sum is between two powers of two, so
+    one chain of them drifts by up to 1e-4 here, up with a first key ahead of the others by 0.24 and down with 0.6. A column's values are all
+    alike, so the output is that value times the quotient of the sum in the matrix products and the row's own; the mean over columns and
+    factors shows it beside the output's rounding (2^-9 of each of 32,768 numbers: 2e-5 in all), and the two cases' difference is free
+    of what both share. A weight's two bfloat16 halves may be off by 2^-17."""
+    from kernel_rush_kawk_b200.cache import SequenceCache
+    from kernel_rush_kawk_b200.parts.base import KVNeed
+
+    rt = runtime(torch.bfloat16)
+    monkeypatch.setattr(type(rt.ops), "SINK_TCGEN05_ROWS", 1)
+    monkeypatch.setattr(type(rt.ops), "SINK_TCGEN05_KEYS", 1)
+    heads, D = 16, 128
+    drift = []
+    for ahead in (0.8046875, 1.984375):
+        qkv = torch.zeros((total, 3 * heads * D))
+        qkv[:, :heads * D:D] = 1.0
+        qkv[0, heads * D:2 * heads * D:D] = ahead  # times the scale of 0.3
+        qkv[:, 2 * heads * D:] = 1.0 + rand((heads * D,), 79).abs()
+        qkv = qkv.to(torch.bfloat16).cuda()
+        cache = SequenceCache([KVNeed(heads, D, None)], 16384, 1, 16384, rt.device, torch.bfloat16, step_tokens=total)
+        slot = cache.alloc()
+        cache.reserve(slot, total)
+        cache.sync()
+        ctx = context(rt, [slot], [0], [total], cache)
+        rt.ops.rotate_norm_write(qkv, 0, heads * D, 2 * heads * D, heads, heads, D, D, torch.zeros(2, device="cuda"), 0, None, ctx.batch,
+                                 cache.view(0))
+        off, out = [], torch.zeros((total, heads * D), dtype=torch.bfloat16, device="cuda")
+        for i in range(16):
+            by = 0.5 + 0.0417 * i
+            rt.ops.sink_attention(qkv, 0, heads, D, D, None, 0.3, None, ctx.batch, cache.view(0), out, 0, by)
+            off.append(out[-1].double() / (qkv[0, 2 * heads * D:].double() * by) - 1)
+        rt.ops.check()
+        drift.append(torch.stack(off).mean().item())
+    assert abs(drift[0] - drift[1]) < 2.0 ** -16 + 3e-5, drift
+
+
 @pytest.mark.parametrize("tcgen05", [True, False])
 @pytest.mark.parametrize("biased", [False, True])
 @pytest.mark.parametrize("D", [64, 128])
