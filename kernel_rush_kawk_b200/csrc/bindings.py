@@ -45,6 +45,7 @@ _SIGNATURES = {
                                c_int, c_float, c_int, _P, c_int, _P],
     "krk_gemm_nt": [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P],
     "krk_gemm_nt_checked": [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, _P],
+    "krk_selftest_wait_for_copies": [_P, _P, c_int, c_int, c_int, _P, c_int, _P],
     "krk_select_tokens": [_P, _P, c_int, c_int, c_float, c_uint, _P, c_uint, _P, _P, _P, _P, _P],
     "krk_gemm_tcgen05": [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, _P],
     "krk_selftest_wait_runs_out": [_P, c_int, _P],
@@ -276,6 +277,17 @@ class Kernels:
         """Launch a kernel whose only wait, on a barrier nobody arrives at, runs out after ``limit_us``
         and sets the error word; ``check`` then raises. For the tests of the error path."""
         self._ok(self.core.krk_selftest_wait_runs_out(self.error.data_ptr(), int(limit_us), self._stream()), "self-test wait")
+
+    def selftest_wait_for_copies(self, src, depth: int, asked: int, withheld: int = 0, limit_us: int = 1000):
+        """The ring of ``depth`` slices of 256 float32 numbers as a kernel sees it that asked for the first ``asked`` slices of
+        ``src``, read none and waited for its copies before it ended; ``withheld``: and for one that it never asked for, which sets the
+        error word after ``limit_us``. For the tests of that wait."""
+        if src.dtype != torch.float32 or not src.is_contiguous() or src.numel() < asked * 256:
+            raise KernelError("the self-test copies slices of 256 contiguous float32 numbers")
+        out = torch.empty((depth, 256), dtype=torch.float32, device=src.device)
+        self._ok(self.core.krk_selftest_wait_for_copies(out.data_ptr(), src.data_ptr(), int(depth), int(asked), int(withheld),
+                                                        self.error.data_ptr(), int(limit_us), self._stream()), "self-test copies")
+        return out
 
     def empty_like(self, x):
         return torch.empty_like(x)

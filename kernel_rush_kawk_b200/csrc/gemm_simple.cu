@@ -239,7 +239,10 @@ gemm_f32_few_kernel(float* __restrict__ C, const float* __restrict__ A, const fl
     const int cols = min(COLS, N - n0);
     const uint64_t policy = l2_evict_first_policy();
     for (int s = 0, b = 0, round = 0; s < slices; ++s) {
-      if (round > 0 && !__all_sync(0xffffffffu, tc::mbar_wait(free_ + b, (round - 1) & 1))) return;  // the readers say so
+      if (round > 0 && !__all_sync(0xffffffffu, tc::mbar_wait(free_ + b, (round - 1) & 1))) {  // a reader has given up, and says so
+        tc::wait_for_copies(full, depth, s);
+        return;
+      }
       const int bytes = min(SLICE, K - s * SLICE) * 4;
       if (lane == 0) tc::mbar_expect_tx(full + b, (cols + M) * bytes);
       __syncwarp();
@@ -254,7 +257,7 @@ gemm_f32_few_kernel(float* __restrict__ C, const float* __restrict__ A, const fl
                      : "memory");
       if (++b == depth) { b = 0; ++round; }
     }
-    return;
+    return;  // what has been asked for is read, or waited for by the reader that gives up
   }
   // neighbouring lanes share a column and differ in their rows
   const int col = lane >> 1, group = 2 * warp + (lane & 1);
@@ -269,10 +272,10 @@ gemm_f32_few_kernel(float* __restrict__ C, const float* __restrict__ A, const fl
   for (int r = 0; r < RPT; ++r) xat[r] = (COLS + min(row0 + r, M - 1)) * PITCH;
   bool here = true;
   for (int s = 0, b = 0, round = 0; s < slices; ++s) {
-    // a wait that runs out: the block's outputs are NaN
+    // a wait that runs out: the warp's outputs are NaN
     here = __all_sync(0xffffffffu, tc::mbar_wait(full + b, round & 1));
-    if (!here) {
-      tc::mbar_wait(full + b, round & 1);  // the copy may still be on its way into this block's memory: as long again
+    if (!here) {  // a place that it hands back no more is not filled again: what may be on its way is a ring from here
+      tc::wait_for_copies(full, depth, min(slices, s + depth));
       break;
     }
     const float* base = ring + b * stage_floats;
@@ -418,4 +421,44 @@ KRK_API int krk_gemm_nt_checked(void* C, const void* A, const void* W, int M, in
 KRK_API int krk_gemm_nt(void* C, const void* A, const void* W, int M, int N, int K, int lda, int ldw, int ldc,
                         int in_dtype, int out_dtype, cudaStream_t stream) {
   return krk_gemm_nt_checked(C, A, W, M, N, K, lda, ldw, ldc, in_dtype, out_dtype, nullptr, stream);
+}
+
+// For the tests of tc::wait_for_copies: a warp asks for `asked` slices of 256 numbers of src into a ring of `depth` places, reads none,
+// and leaves the ring in out once the last copies are said to be here. `withheld`: it counts on one more, which it never asks for;
+// that wait runs out after limit_us, which the error word says (21). Slice i is in place i % depth.
+namespace {
+__global__ void copies_kernel(float* out, const float* src, int depth, int asked, int withheld, int* error, unsigned long long limit_ns) {
+  __shared__ __align__(16) float ring[8][256];
+  __shared__ uint64_t full[8];
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < depth; ++i) tc::mbar_init(full + i, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  for (int i = threadIdx.x; i < depth * 256; i += 32) ring[i / 256][i % 256] = 0.f;
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < asked + withheld; ++i) {
+      if (i >= depth && !tc::mbar_wait(full + i % depth, (uint32_t)(i / depth - 1) & 1u)) { asked = i; withheld = 0; break; }
+      if (i == asked) break;
+      tc::mbar_expect_tx(full + i % depth, 1024);
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], 1024, [%2];"
+                   ::"r"(tc::smem_u32(ring[i % depth])), "l"(src + i * 256), "r"(tc::smem_u32(full + i % depth)) : "memory");
+    }
+  }
+  asked = __shfl_sync(0xffffffffu, asked, 0);
+  withheld = __shfl_sync(0xffffffffu, withheld, 0);
+  if (!__all_sync(0xffffffffu, tc::wait_for_copies(full, depth, asked + withheld, limit_ns)) && threadIdx.x == 0) atomicExch(error, 21);
+  for (int i = threadIdx.x; i < depth * 256; i += 32) out[i] = ring[i / 256][i % 256];
+}
+}  // namespace
+
+KRK_API int krk_selftest_wait_for_copies(float* out, const float* src, int depth, int asked, int withheld, int* error, int limit_us,
+                                         cudaStream_t stream) {
+  if (depth < 1 || depth > 8 || asked < 0 || asked > 64 || withheld < 0 || withheld > 1 || limit_us < 1 || limit_us > 100000 ||
+      (uintptr_t)src % 16)
+    return -2;
+  copies_kernel<<<1, 32, 0, stream>>>(out, src, depth, asked, withheld, error, (unsigned long long)limit_us * 1000ull);
+  KRK_CHECK_LAUNCH();
+  return 0;
 }

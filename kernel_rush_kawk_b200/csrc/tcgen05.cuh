@@ -45,6 +45,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsign
   }
 }
 
+// For a warp of a block that has asked for `asked` slices into a ring of `depth` places, a phase of full[place] each, and is about to give
+// up: copies write into the block's memory, which goes to another block when this one has ended. Waits for the slices that may still
+// be on their way, the last one of each place, within a limit each; false if some did not come.
+__device__ __forceinline__ bool wait_for_copies(uint64_t* full, int depth, int asked, unsigned long long limit_ns = WAIT_LIMIT_NS) {
+  bool here = true;
+  for (int i = max(0, asked - depth); i < asked; ++i) here &= mbar_wait(full + i % depth, (uint32_t)(i / depth) & 1u, limit_ns);
+  return here;
+}
+
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"

@@ -93,3 +93,23 @@ def test_rebuilding_the_cache_gives_its_memory_back(folders):
     growth_cache = sizes[-1][0] - sizes[0][0]
     growth_alloc = sizes[-1][1] - sizes[0][1]
     assert growth_alloc <= growth_cache + (8 << 20), f"allocated memory grew by {growth_alloc}, the cache itself by {growth_cache}"
+
+
+@pytest.mark.parametrize("depth,asked", [(2, 0), (2, 1), (2, 2), (2, 3), (3, 2), (3, 7), (3, 9), (6, 5), (6, 13), (8, 64)])
+def test_a_block_that_gives_up_waits_for_the_copies_that_it_asked_for(folders, depth, asked):
+    """What a kernel with a ring of copies calls before it ends early: every slice asked for and read by nobody is in shared memory
+    afterwards, from a ring that is not full to one that has gone round, and a copy that never comes costs its limit and no more."""
+    from kernel_rush_kawk_b200.csrc import KernelError
+
+    ops = engine_of(folders).ops
+    ops.check()
+    src = torch.randn(64 * 256, device="cuda")
+    want = torch.zeros((depth, 256), device="cuda")
+    for i in range(asked):
+        want[i % depth] = src[i * 256:(i + 1) * 256]
+    assert torch.equal(ops.selftest_wait_for_copies(src, depth, asked), want)
+    ops.check()
+    assert torch.equal(ops.selftest_wait_for_copies(src, depth, asked, withheld=1), want)
+    with pytest.raises(KernelError, match="ran out"):
+        ops.check()
+    ops.check()
