@@ -672,8 +672,12 @@ delta_walk_kernel(const __grid_constant__ CUtensorMap map_m, const __grid_consta
   if (warp == WALKERS / 32) {
     // The fifth warp waits for the copies, so that no walker has to: at a step's barrier the next chunk but one is here. A
     // chunk's place is free when the step before it is over, since the walkers read a chunk a step ahead.
+    int asked = 0;
+    bool late = false;  // a wait has run out: the step's results are not to be used, which the error word says; no more is asked for or waited for
     auto request = [&](int c) {
-      if (c >= n_chunks || lane != 0) return;
+      if (c >= n_chunks || late) return;
+      asked = c + 1;
+      if (lane != 0) return;
       const int b = c % WALK_STAGES, row = ((seq * a.n_chunks + c) * a.H + h) * (ITEM_DELTA / N);
       tc::mbar_expect_tx(full + b, (WALK_M + WALK_G) * sizeof(float));
       tc::tma_load_2d(ms + b * WALK_M, &map_m, full + b, 0, row);
@@ -681,10 +685,9 @@ delta_walk_kernel(const __grid_constant__ CUtensorMap map_m, const __grid_consta
       tc::tma_load_2d(gs + b * WALK_G, &map_g, full + b, p0, row + N);
     };
     auto wait = [&](int c) {
-      // a wait that runs out: the step's results are not to be used, which the error word says; the copy may still be on its way: as long again
-      if (c >= n_chunks || __all_sync(0xffffffffu, tc::mbar_wait(full + c % WALK_STAGES, (c / WALK_STAGES) & 1))) return;
+      if (c >= n_chunks || late || __all_sync(0xffffffffu, tc::mbar_wait(full + c % WALK_STAGES, (c / WALK_STAGES) & 1))) return;
+      late = true;
       if (lane == 0) atomicExch(a.error, 24);
-      tc::mbar_wait(full + c % WALK_STAGES, (c / WALK_STAGES) & 1);
     };
     for (int c = 0; c < WALK_STAGES; ++c) request(c);
     wait(0);
@@ -695,6 +698,7 @@ delta_walk_kernel(const __grid_constant__ CUtensorMap map_m, const __grid_consta
       wait(c + 2);
       step_sync();
     }
+    if (late) tc::wait_for_copies(full, WALK_STAGES, asked);
     return;
   }
   const int kg = lane & 7, half = kg >> 2, r0 = warp * 16 + (lane >> 3) * 4;
