@@ -949,6 +949,11 @@ int launch_walk(const ChunkArgs& a, bool gated, int n_seqs, cudaStream_t stream)
                          dim3(64), 0, stream, a);
 }
 
+template <typename Kernel>
+int room(Kernel kernel, size_t bytes) {
+  return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
 template <Kind KIND>
 int launch_chunks(ChunkArgs a, int n_seqs, cudaStream_t stream) {
   constexpr bool GATED = KIND == RUNNING_MAX;
@@ -960,10 +965,9 @@ int launch_chunks(ChunkArgs a, int n_seqs, cudaStream_t stream) {
   const long long most = heads * n_seqs * all_slices;
   a.slices = (int)(most / 444 < 1 ? 1 : most / 444 > all_slices ? all_slices : most / 444);
   const dim3 grid((unsigned)((all_slices + a.slices - 1) / a.slices), (unsigned)heads, (unsigned)n_seqs);
-  cudaFuncSetAttribute(chunk_sum_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1);
-  cudaFuncSetAttribute(chunk_output_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3);
-  int rc = (int)launch_pdl(chunk_sum_kernel<KIND>, grid, dim3(THREADS), s1, stream, a);
-  if (rc) return rc;
+  int rc;
+  if ((rc = room(chunk_sum_kernel<KIND>, s1)) || (rc = room(chunk_output_kernel<KIND>, s3))) return rc;
+  if ((rc = (int)launch_pdl(chunk_sum_kernel<KIND>, grid, dim3(THREADS), s1, stream, a))) return rc;
   if ((rc = launch_walk(a, GATED, n_seqs, stream))) return rc;
   return (int)launch_pdl(chunk_output_kernel<KIND>, grid, dim3(OUT_THREADS), s3, stream, a);
 }
@@ -971,11 +975,10 @@ int launch_chunks(ChunkArgs a, int n_seqs, cudaStream_t stream) {
 int launch_ssd(ChunkArgs a, int n_seqs, int live, cudaStream_t stream) {
   const size_t s1 = ssd_sum_smem(a.N), s3 = ssd_output_smem(a.N);
   if (a.max_chunks > 65535 || n_seqs > 65535) return -2;
-  auto room = [](auto kernel, size_t bytes) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); };
-  room(ssd_sum_kernel<true>, s1);
-  room(ssd_sum_kernel<false>, s1);
-  room(ssd_output_kernel<true>, s3);
-  room(ssd_output_kernel<false>, s3);
+  int rc;
+  if ((rc = room(ssd_sum_kernel<true>, s1)) || (rc = room(ssd_sum_kernel<false>, s1)) || (rc = room(ssd_output_kernel<true>, s3)) ||
+      (rc = room(ssd_output_kernel<false>, s3)))
+    return rc;
   const int groups = a.H / a.per_group, all = a.per_group * ((a.P + PB - 1) / PB);
   // units a block: the fewest rounds of units over the SMs, a block's start counted as a part of one. Blocks of chunks that a shorter
   // sequence does not have leave at once and are not counted (48 heads, sequences of 600, 400 and 300 tokens: 93 us counted, 71).
@@ -1001,7 +1004,7 @@ int launch_ssd(ChunkArgs a, int n_seqs, int live, cudaStream_t stream) {
   };
   auto grid = [&] { return dim3((unsigned)(a.parts * groups), (unsigned)a.max_chunks, (unsigned)n_seqs); };
   const bool many_sums = split(0.5f);
-  int rc = (int)launch_pdl(many_sums ? ssd_sum_kernel<true> : ssd_sum_kernel<false>, grid(), dim3(THREADS), s1, stream, a);
+  rc = (int)launch_pdl(many_sums ? ssd_sum_kernel<true> : ssd_sum_kernel<false>, grid(), dim3(THREADS), s1, stream, a);
   if (rc) return rc;
   if ((rc = launch_walk(a, false, n_seqs, stream))) return rc;
   const bool many = split(0.7f);
@@ -1022,7 +1025,7 @@ KRK_API int krk_memory_chunk_decays(float* cum, const void* lora, int lora_strid
   const size_t smem = (size_t)L * R * sizeof(float);
   const int chunks = (max_q_len + L - 1) / L;
   if (smem > 48 * 1024 || chunks > 65535 || n_seqs > 65535) return -2;
-  cudaFuncSetAttribute(chunk_decays_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024);  // beside the kernel's own
+  if (const int rc = room(chunk_decays_kernel, 48 * 1024)) return rc;  // beside the kernel's own
   const dim3 grid((unsigned)((channels + 31) / 32), (unsigned)chunks, (unsigned)n_seqs);
   return (int)launch_pdl(chunk_decays_kernel, grid, dim3(32 * L / DECAY_TOKENS), smem, stream, cum, (const bf16*)lora, lora_stride, (const bf16*)w2,
                          bias, 1.0f / tau, channels, R, cu_q, seq_qlen);

@@ -1142,7 +1142,10 @@ __global__ void __launch_bounds__(THREADS, 5) mix_finish_kernel(ChunkArgs a) {
 template <typename Kernel>
 int run(Kernel kernel, dim3 grid, int threads, size_t floats, const ChunkArgs& a, cudaStream_t stream) {
   const size_t smem = floats * sizeof(float);
-  if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+  }
   return (int)launch_pdl(kernel, grid, dim3(threads), smem, stream, a);
 }
 
@@ -1197,7 +1200,7 @@ KRK_API int krk_recurrence_chunks(int rule, const void* r, int r_stride, const v
     if ((rc = tc::make_map_f32(&map_m, scratch, scratch_rows, N, N, 32, N, true))) return rc;
     if ((rc = tc::make_map_f32(&map_g, scratch, scratch_rows, N, N, WALK_COLS, N, false))) return rc;
     const size_t walk = (WALK_STAGES * (size_t)(WALK_M + WALK_G) + 2 * (N / 8) * WALK_SP) * sizeof(float) + 1024;
-    cudaFuncSetAttribute(delta_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk);
+    if ((rc = (int)cudaFuncSetAttribute(delta_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk))) return rc;
     if ((rc = (int)launch_pdl(delta_walk_kernel, dim3(N / WALK_COLS, (unsigned)H, (unsigned)n_seqs), dim3(WALK_THREADS), walk, stream, map_m, map_g, a)))
       return rc;
     return run(delta_finish_kernel, items, THREADS, (size_t)L * PITCH + 4 * L, a, stream);
