@@ -448,22 +448,13 @@ class Kernels:
             n = batch.n_seqs
             out = torch.empty((n, heads * head_dim), dtype=qkv.dtype, device=qkv.device)
             row_tiles = -(-(heads // cache.kv_heads) // 16)
-            # key splits (blocks per cluster) by the number of (sequence, kv head, row tile) items alone, never by
-            # lengths, so a captured step stays valid: as many as one wave of the kernel's blocks has room for. Two
-            # blocks share an SM, so 148 items split in two still start at once; a layer of the 4B shape at 19, 20
-            # and 24 sequences of 500 tokens takes 84.6, 86.4 and 85.0 us in two splits and 77.5, 77.9 and 79.2 in
-            # one (18 sequences: 76.0 and 77.4; after 100 tokens 78.4 against 68.3 at 20, after 1,500 102.2 against
-            # 96.4). Clusters of four do not fill every SM: 8 sequences 51.3 us in four splits, 53.0 in two; 9 take
-            # 61.6 and 56.7 (after 100 tokens 57.4 and 52.0, after 1,500 70.2 and 65.6). Four sequences 48.7 us in four,
-            # 47.3 in eight; five 49.4 and 53.4. One sequence has eight items: sixteen splits are 128 blocks where
-            # eight are 64, and what bounds the kernel is the bytes its blocks have in flight (one step of the 4B
-            # shape at 32,000 tokens of context: 4.41 -> 3.14 ms, at 8,000: 2.51 -> 2.17, at 1,500 the same)
             items = n * cache.kv_heads * row_tiles
-            splits = 16 if items <= 9 else 8 if items <= 37 else 4 if items <= 64 else 2 if items <= 148 else 1
+            # what the TMA-fed kernel takes; the same for either kernel where a switch below gives the step to the other one
+            fed = head_dim % 64 == 0 and cache.width <= 1024 and hasattr(lib, "krk_attention_decode_fused_tma")
+            splits = self._decode_splits(items, head_dim, fed)
             gain = q_gain if q_gain is not None else k_gain
             n_pos = cos.shape[0] if cos is not None else 0x7fffffff
-            if (splits in self.tma_decode_splits and self.use_tma_decode_attention and head_dim % 64 == 0
-                    and cache.width <= 1024 and hasattr(lib, "krk_attention_decode_fused_tma")):
+            if fed and splits in self.tma_decode_splits and self.use_tma_decode_attention:
                 # many sequences: one block or two per (sequence, kv head), pages by TMA into a ring of half page-pairs
                 rc = lib.krk_attention_decode_fused_tma(
                     out.data_ptr(), qkv.data_ptr(), qkv.stride(0), heads, cache.kv_heads, _ptr(q_gain), _ptr(k_gain),
@@ -474,6 +465,7 @@ class Kernels:
                 if rc != -2:  # -2: the shapes do not fit this kernel's shared memory; the kernel below takes them
                     self._ok(rc, "fused decode attention (TMA)")
                     return out
+                splits = self._decode_splits(items, head_dim, False)
             self._ok(lib.krk_attention_decode_fused(
                 out.data_ptr(), qkv.data_ptr(), qkv.stride(0), heads, cache.kv_heads, _ptr(q_gain), _ptr(k_gain),
                 int(gain is not None and gain.dtype == torch.float32), _ptr(cos), _ptr(sin), eps,
@@ -483,6 +475,31 @@ class Kernels:
             return out
         self.qk_norm_rope_write(qkv, heads, kv_in_row, head_dim, q_gain, k_gain, eps, cos, sin, batch, cache)
         return self.attention(qkv, heads, kv_in_row, head_dim, batch, cache, scale, window)
+
+    @staticmethod
+    def _decode_splits(items, head_dim, fed) -> int:
+        """Key splits (blocks per cluster) of a single-token step's attention, by the number of (sequence, kv head, row tile) items,
+        the head size and whether pages come by TMA from two splits down (``fed``), never by lengths, so a captured step stays valid.
+
+        One sequence of the 4B shape has eight items: sixteen splits are 128 blocks where eight are 64, and what bounds the kernel is the
+        bytes its blocks have in flight (one step at 32,000 tokens of context: 4.41 -> 3.14 ms, at 8,000: 2.51 -> 2.17, at 1,500 the
+        same). A layer of four sequences 48.7 us in four, 47.3 in eight; five 49.4 and 53.4.
+
+        Fed, as many as one wave of the kernel's blocks has room for. Two blocks share an SM, so 148 items split in two still start at
+        once, and clusters of four do not fill every SM. The attention alone, eight kv heads of 128, us after 100, 500, 1,500, 8,000 and
+        32,000 tokens: 9 sequences in four 10.5, 12.4, 21.9, 76 and 277, in two 7.4, 10.0, 17.4, 63 and 231 (8 sequences, 500 and 8,000: 8.1
+        and 44 in four, 9.5 and 62); 19 in two 12.7, 19.6, 36.1, 143 and 533, in one 6.8, 13.3, 30.2, 136 and 531 (18, 500 and 8,000:
+        12.7 and 95 in two, 12.8 and 115). Heads of 64 the same way (19, after 1,500 tokens: 26.6 in two, 23.0). A block alone with an item of
+        heads of 256 has too little on the way behind long contexts (19, after 1,500 and 8,000: 69 and 270 in two, 67 and 299).
+
+        Otherwise a block's own pace over its pages bounds a step, and more blocks are worth a second wave: heads of 80, after 500, 1,500 and
+        8,000 tokens, 9 sequences 7.4, 14.8 and 60 in four, 8.3, 19.6 and 84 in two; 20 sequences 11.8, 26.8 and 117 in two, 14.5, 37.1 and
+        181 in one; heads of 128 behind page tables of more than 1,024 entries, 20 sequences, 12.3, 24.6 and 103 in two, 13.8, 31.6 and 146."""
+        if items <= 37:
+            return 16 if items <= 9 else 8
+        if not fed:
+            return 4 if items <= 74 else 2 if items <= 192 else 1
+        return 4 if items <= 64 else 2 if items <= (148 if head_dim <= 128 else 192) else 1
 
     def attention(self, qkv, heads, kv_in_row, head_dim, batch, cache, scale, window):
         lib = self._attn_lib(head_dim)

@@ -150,3 +150,17 @@ def test_attention_part_with_a_rotation_of_part_of_the_head_on_the_stand_in():
             cache.advance(slot, n)
             start += n
         assert_close(torch.cat(got), want, "float32", f"partial rotation on the stand-in, pieces {pieces}")
+
+
+@pytest.mark.parametrize("head_dim, fed, items, splits", [
+    (128, True, 8, 16), (128, True, 16, 8), (128, True, 32, 8), (128, True, 40, 4), (128, True, 64, 4), (128, True, 72, 2), (128, True, 144, 2),
+    (128, True, 152, 1), (128, True, 512, 1), (64, True, 72, 2), (64, True, 152, 1), (256, True, 72, 2), (256, True, 152, 2),
+    (256, True, 192, 2), (80, False, 64, 4), (80, False, 72, 4), (80, False, 80, 2), (80, False, 192, 2), (80, False, 200, 1),
+    (128, False, 72, 4), (128, False, 160, 2), (48, False, 8, 16)])
+def test_key_splits_of_single_token_attention(head_dim, fed, items, splits):
+    """The kernel whose pages come by TMA has a wave of its own; the other one (head sizes that are no multiple of 64, page tables of
+    more than 1,024 entries) was measured slower with its lines: each on the side where it was the faster, or as fast, at most
+    contexts from 100 to 32,000 tokens and nowhere slower by more than a few microseconds."""
+    from kernel_rush_kawk_b200.csrc.bindings import Kernels
+
+    assert Kernels._decode_splits(items, head_dim, fed) == splits
