@@ -992,27 +992,40 @@ class Kernels:
     @staticmethod
     def _grouped_from(E, F, C, gated) -> int:
         """Pairs from which the two grouped launches, which need the pairs ordered and their rows gathered first, are faster than
-        blocks that walk over 32 rows of an expert's matrix at a time. Those read an expert's weights once for sixteen of its rows, at
-        5.7 TB/s and more beyond a hundred MB; the grouped ones stream them at 6 where their tiles, of 128 or 256 columns, fill the rounds
-        of 74 pairs of blocks. Pairs an expert at which they meet in a single-token step, and both sides (walk and grouped, us) below and
-        above: 64 experts of 1,408 x 2,048 (tiles 512) 4: at 3 167 and 174, 6 194 and 187; of 2,112 x 2,048 (512) 3.5: 3 244 and 249, 4.5 266
-        and 261; 128 of 768 x 2,048 (768) 3: 2 174 and 193, 4.5 211 and 209; 128 of 512 x 1,024 (512) 4.5: 3 88 and 92, 6 99 and 92; 256 of
-        512 x 2,048 (1,024) 2.3: 2 229 and 239, 3 270 and 257; 64 of 768 x 1,536 (384) 11: 9 99 and 102, 12 105 and 103; 64 of 640 x 1,280
-        (320) 10: 9 78 and 80, 12 85 and 80; 48 of 1,024 x 1,536 (288) 10; 32 of 1,536 x 2,048 (256) 11, of 3,072 x 2,048 (256) 9, of
-        2,048 x 1,024 (128) 9: 8 86 and 87, 12 95 and 87; 16 of 6,144 x 2,048 (128) 6; of 3,072 x 1,536 (96) 13: 12 92 and 105, 16 113 and
-        105; 32 of 768 x 1,536 (192) 13; 16 of 1,024 x 1,024 13, 8 of 2,048 x 1,024 15. Many units of 20 to 40 KB: 128 of 128 x 1,024 2.5:
-        2 40 and 45, 4.5 53 and 48; 64 of 256 x 1,024 4.7: 3 33 and 40, 6 43 and 41; not 64 of 128 x 512, 1,280 units in all, 8."""
+        blocks that walk over 32 rows of an expert's matrix at a time (a unit). Those read an expert's weights once for sixteen of its rows, at
+        5.7 TB/s and more beyond a hundred MB, and the pairs' own rows once a unit, from L2; the grouped ones stream the weights at 6 where
+        their tiles, of 128 or 256 columns, fill the rounds of 74 pairs of blocks. Pairs an expert at which the two meet in a single-token
+        step (experts of F x C, top 2 to 8 of them, random choices), and the walk's and the grouped time (us) below and above:
+
+        From six rounds of tiles (444) on, where the rows that the walk reads again come to 150 MB, 4.5 at most (units of little more than
+        64 KB reach their own cost first), 2.5 where there are 128 units an SM. 64 experts of 1,408 x 2,048 5: at 3.5 183 and 188, 6 192 and
+        189; of 1,792 x 2,048 3.3: 3 212 and 221, 3.5 234 and 224; of 2,112 x 2,048 3: 2 228 and 231, 4.5 272 and 264; 72 of 1,024 x 2,048 5: 4.5
+        156 and 162, 6 168 and 162; 96 of 768 x 2,048 4: 3 154 and 163, 6 173 and 165; of 768 x 1,536 4.6; of 640 x 1,280 5.8; 128 of 768 x
+        2,048 4.6: 3.5 201 and 210, 5 221 and 212; of 512 x 1,024 4: 3 90 and 92, 4.5 96 and 91; of 1,408 x 2,048 2 to 3.2: 1.5 282 and 287, 3.5 345
+        and 338; 160 of 1,536 x 2,560 1.3: 1 380 and 382, 2 509 and 496; 192 of 768 x 2,048 2.7: 2.5 270 and 282, 3 290 and 283; 256 of 512 x
+        2,048 2.3: 2 233 and 241, 3 279 and 259; of 768 x 1,024 3.
+
+        From four rounds (296) on 9: 48 of 2,048 x 2,048 9: 6 207 and 211, 12 237 and 215; of 1,024 x 2,048 11; 64 of 768 x 2,048 9; of 768 x
+        1,536 10: 8 98 and 102, 11 104 and 103; of 640 x 1,280 10: 8 76 and 79, 11 85 and 80; 80 of 640 x 1,280 8: 6 88 and 93, 9 95 and 93; but 96
+        of 512 x 1,024 5.5: 4.5 79 and 81, 9 88 and 81. From a round and a half (111) and 300 MB on 8: 32 of 3,072 x 2,048 9.5, of 1,536 x
+        2,048 13, of 2,048 x 1,024 6.5: 5 83 and 86, 9 90 and 87; 16 of 6,144 x 2,048 7.7: 6 205 and 207, 9 218 and 207; of 4,096 x 2,048 7.8; 24 of
+        3,072 x 1,536 9; 48 of 1,024 x 1,536 10.5. Fewer 12: 32 of 768 x 1,536 12; 16 of 3,072 x 1,536 13: 12 93 and 105, 16 113 and 106.
+
+        Units of less than 64 KB, which cost more than their bytes, by how many an SM has: from 60 on 2.5: 256 of 256 x 2,048 1.6: 1 123 and 127, 2
+        153 and 148; 512 of 128 x 1,024 1.6, of 256 x 1,024 2; 160 of 128 x 2,048 2.5; 256 of 128 x 1,024 2.5: 2 68 and 70, 3 87 and 78. From 28
+        on 3.5: 128 of 128 x 1,024 2.5: 2 42 and 44, 4 54 and 48; 256 of 128 x 512 2.7; 64 of 256 x 2,048 3.8: 3 53 and 62, 4 65 and 62. From 14 on
+        4.5: 64 of 256 x 1,024 4: 3.5 39 and 41, 6 44 and 41; 96 of 256 x 512 3.7; 32 of 256 x 2,048 5. From 6 on 6: 64 of 512 x 512 6, of 128 x
+        512 4.8: 3.5 23 and 24, 7 27 and 24; 32 of 512 x 512 8.3; 40 of 256 x 1,024 10; 48 of 128 x 1,024 4.5. Fewer 12: 16 of 256 x 1,024 16."""
         tiles = E * min(-(-F // (128 if gated else 256)), -(-C // 256))
-        # The lines stay at or below the upper ends that the tests of the change of hands hold (1 at 128 experts of 444 tiles, 3 at 64, 4.5
-        # from 296 tiles, 6 of long matrices), which is up to 10 % given away between them and the meeting points above.
-        if tiles >= 296:  # six rounds; four
-            return 9 * E // 2 if tiles < 444 else 3 * E if E <= 64 else E
         units, size = E * -(-(F + C) // 32), 2 * E * F * C * (3 if gated else 2)
-        if units >= 16 * 148 and size < 65536 * units:
-            return 5 * E
-        if tiles >= 111 and size >= 300e6:
-            return 6 * E
-        return 12 * E
+        if size < 65536 * units:
+            return 5 * E // 2 if units >= 60 * 148 else 7 * E // 2 if units >= 28 * 148 else 9 * E // 2 if units >= 14 * 148 else 6 * E if units >= 6 * 148 else 12 * E
+        if tiles >= 444 or (tiles >= 296 and size < 80000 * units):
+            again = F * C * (3 if gated else 2) // 16  # bytes of a pair's rows that the walk's units read: K F / 8 + F C / 16 (no gate: K F / 16)
+            return min((5 if units >= 128 * 148 else 9) * E // 2, int(150e6) // again)
+        if tiles >= 296:
+            return 9 * E
+        return 8 * E if tiles >= 111 and size >= 300e6 else 12 * E
 
     @staticmethod
     def _use_grouped(x, K, F, C, gated, activation) -> bool:

@@ -51,7 +51,7 @@ def test_tiles_of_an_experts_rows_at_their_edges(N, K, counts, gated):
     ops.check()
 
 
-@pytest.mark.parametrize("E, top, F, C, line", [(64, 6, 640, 1280, 48), (8, 2, 96, 72, 48)])
+@pytest.mark.parametrize("E, top, F, C, line", [(64, 6, 640, 1280, 96), (8, 2, 96, 72, 48)])
 def test_experts_where_their_products_change_hands(E, top, F, C, line):
     """Single-token steps and prompts of as many rows as move the experts' products from a block per piece of an expert to the grouped
     launches, and one row fewer and more: the same sums, within the roundings of each expert's two products."""
@@ -259,7 +259,7 @@ def test_a_captured_step_of_the_grouped_experts():
 
     ops = load_kernels((), "cuda:0")
     g = torch.Generator().manual_seed(10)
-    E, top, F, K, C, rows = 64, 6, 640, 128, 1280, 50
+    E, top, F, K, C, rows = 64, 6, 640, 128, 1280, 100
     w1, w2 = ((torch.randn(s, generator=g) * 0.06).to(torch.bfloat16).cuda() for s in ((E, 2 * F, K), (E, C, F)))
 
     def inputs():
