@@ -326,10 +326,14 @@ int pick_rt(void* out, const void* x, const void* W, int M, int N, int K, float 
     const int tiles = (N + 15) / 16, pairs = (N + 31) / 32;
     if (tiles > 3 * 148) return launch<NT, 2, SWIGLU, TOut>(out, x, W, M, N, K, limit, stream);
     // Between two and three blocks of one tile an SM, and long rows: two tiles a block as well, and K split three ways over a cluster, while
-    // that leaves room for the clusters' placing (500 of 592 blocks; 528 ran over). us, one tile / two split: 5,120 outputs of 5,120 at 16
-    // rows 13.6 / 11.8, at 8 11.9 / 10.4, at one 10.3 / 10.0; of 17,408 43.9 / 37.7, 36.7 / 34.3, 33.1 / 33.0. (Two ways, for 6,144 outputs,
-    // gained alone, 7.2 -> 6.7 at 8 rows of 2,560, and lost in a step, 51.6 -> 52.4 a layer.)
-    if (tiles > 2 * 148 && pairs * 3 <= 500 && K >= 5120)
+    // that leaves room for the clusters' placing (500 of 592 blocks, 5,312 outputs; 528 ran over). us, one tile / two split: 5,120 outputs
+    // of 5,120 at 16 rows 14.7 / 11.5, at 8 11.5 / 10.0, at one 9.9 / 9.6; of 17,408 42.7 / 36.9, 36.0 / 33.8, 32.9 / 32.8. The clusters' start
+    // and meeting is a fixed cost, so short rows lose: from K of 4,608 on every width at 1, 8, 9 and 16 rows gains (5,312 outputs 9.2 / 9.1,
+    // 10.8 / 9.5, 12.2 / 10.2, 13.4 / 12.5; 4,752 8.8 / 8.5, 10.5 / 8.9, 10.2 / 9.7, 13.9 / 10.2), at 4,352 5,312 outputs of 16 rows lose (11.0 /
+    // 12.5), at 4,096 of 9 as well (9.7 / 11.4), at 2,048 all but 16 rows of the narrowest, at 1,024 all (5,120 outputs 2.7 / 3.5, 2.9 /
+    // 3.7, 3.2 / 4.5, 3.9 / 5.0). (Two ways, for 6,144 outputs, gained alone, 7.2 -> 6.7 at 8 rows of 2,560, and lost in a step, 51.6 ->
+    // 52.4 a layer.)
+    if (tiles > 2 * 148 && pairs * 3 <= 500 && K >= 4608)
       return launch_warps<4, NT, 2, SWIGLU, TOut, false, 3, (NT == 1 ? 8 : 6)>(out, x, W, M, N, K, limit, stream);
   }
   return launch<NT, 1, SWIGLU, TOut>(out, x, W, M, N, K, limit, stream);

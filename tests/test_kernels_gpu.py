@@ -152,7 +152,8 @@ def test_float32_products_of_several_threads(ops):
 
 
 @pytest.mark.parametrize("rows", [1, 8, 9, 16])
-@pytest.mark.parametrize("nk", [(4752, 5120), (4753, 5152), (5312, 5120), (5313, 5120), (7104, 96), (7105, 96), (9457, 2080)])
+@pytest.mark.parametrize("nk", [(4752, 5120), (4753, 5152), (5312, 5120), (5313, 5120), (7104, 96), (7105, 96), (9457, 2080),
+                                (4737, 4608), (5312, 4608), (5312, 4576)])
 def test_few_row_products_of_two_tiles_a_block(ops, rows, nk):
     """Output counts on both sides of each line of the few-row products' forms (two row tiles a block, K split three ways), with
     sums of whole numbers below 2^24: they are exact in any order, so a tile, a slice or a row in the wrong place shows."""
