@@ -43,8 +43,7 @@ _SIGNATURES = {
     "krk_swiglu": [_P, _P, c_int, c_int, c_int, _P],
     "krk_qk_norm_rope_write": [_P, _P, _P, c_int, _P, _P, _P, _P, _P, _P, c_int, _P, _P, c_int, c_int, c_int, c_int,
                                c_int, c_float, c_int, _P, c_int, _P],
-    "krk_gemm_nt": [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P],
-    "krk_gemm_nt_checked": [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, _P],
+    "krk_gemm_nt": [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, _P],
     "krk_selftest_wait_for_copies": [_P, _P, c_int, c_int, c_int, _P, c_int, _P],
     "krk_select_tokens": [_P, _P, c_int, c_int, c_float, c_uint, _P, c_uint, _P, _P, _P, _P, _P],
     "krk_gemm_tcgen05": [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, _P],
@@ -336,8 +335,8 @@ class Kernels:
         M, K = x.shape
         N = w.shape[0]
         out = torch.empty((M, N), dtype=out_dtype, device=x.device)
-        self._ok(self.core.krk_gemm_nt_checked(out.data_ptr(), x.data_ptr(), w.data_ptr(), M, N, K, x.stride(0), w.stride(0), N,
-                                               _code(x.dtype), _code(out_dtype), self.error.data_ptr(), self._stream()), "gemm")
+        self._ok(self.core.krk_gemm_nt(out.data_ptr(), x.data_ptr(), w.data_ptr(), M, N, K, x.stride(0), w.stride(0), N,
+                                       _code(x.dtype), _code(out_dtype), self.error.data_ptr(), self._stream()), "gemm")
         return out
 
     def gemm_tcgen05(self, x, w, swiglu_rows=0, variant=0, out_float32=False):

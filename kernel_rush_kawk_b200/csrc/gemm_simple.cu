@@ -403,8 +403,8 @@ int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, in
 
 // in_dtype / out_dtype: KRK_DTYPE_F32 or KRK_DTYPE_BF16. Supported: f32->f32, bf16->f32, bf16->bf16. `error` (device, may be null)
 // is set to 20 should a product of few rows give up on a wait, whose outputs are then NaN.
-KRK_API int krk_gemm_nt_checked(void* C, const void* A, const void* W, int M, int N, int K, int lda, int ldw, int ldc,
-                                int in_dtype, int out_dtype, int* error, cudaStream_t stream) {
+KRK_API int krk_gemm_nt(void* C, const void* A, const void* W, int M, int N, int K, int lda, int ldw, int ldc,
+                        int in_dtype, int out_dtype, int* error, cudaStream_t stream) {
   if (in_dtype == KRK_DTYPE_F32 && out_dtype == KRK_DTYPE_F32) {
     const int rc = launch_f32((float*)C, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldc, error, stream);
     if (rc != -2) return rc;
@@ -416,11 +416,6 @@ KRK_API int krk_gemm_nt_checked(void* C, const void* A, const void* W, int M, in
   if (in_dtype == KRK_DTYPE_BF16 && out_dtype == KRK_DTYPE_BF16)
     return launch<bf16, bf16>(C, A, W, M, N, K, lda, ldw, ldc, stream);
   return -4;
-}
-
-KRK_API int krk_gemm_nt(void* C, const void* A, const void* W, int M, int N, int K, int lda, int ldw, int ldc,
-                        int in_dtype, int out_dtype, cudaStream_t stream) {
-  return krk_gemm_nt_checked(C, A, W, M, N, K, lda, ldw, ldc, in_dtype, out_dtype, nullptr, stream);
 }
 
 // For the tests of tc::wait_for_copies: a warp asks for `asked` slices of 256 numbers of src into a ring of `depth` places, reads none,

@@ -35,7 +35,7 @@
 namespace {
 
 constexpr int CHUNK = 32;        // k values per fragment load
-constexpr int RING_LOADS = 8;    // 16-row tile chunks in flight per thread (32 bytes each); DEEP doubles it
+constexpr int RING_LOADS = 8;    // 16-row tile chunks in flight per thread (32 bytes each)
 // With two batch tiles whose rows ride in the ring (9 to 16 rows) a stage is a third larger, and
 // at 8 loads an 8-warp block takes 131 KB of shared memory: one block per SM. Six keep two blocks per SM;
 // a decode step at 16 sequences of the 4B shape: 2.79 ms against 3.08 ms with 8 (and 2.96 / 3.06 / 3.30 ms
@@ -43,10 +43,10 @@ constexpr int RING_LOADS = 8;    // 16-row tile chunks in flight per thread (32 
 constexpr int RING_LOADS_TWO_TILES = 6;
 // five 4-warp blocks of a K-split product share an SM: 40 KB each with the ring, the reduction buffer and the inbox
 constexpr int RING_LOADS_KSPLIT = 6, RING_LOADS_KSPLIT_TWO_TILES = 4;
-template <int NT, bool DEEP, int KSPLIT = 1, int RING = 0>
+template <int NT, int KSPLIT = 1, int RING = 0>
 __host__ __device__ constexpr int ring_loads() {
   return RING > 0 ? RING : (KSPLIT > 1) ? (NT == 2 ? RING_LOADS_KSPLIT_TWO_TILES : RING_LOADS_KSPLIT)
-                      : NT == 2 ? RING_LOADS_TWO_TILES : (DEEP ? 2 : 1) * RING_LOADS;
+                      : NT == 2 ? RING_LOADS_TWO_TILES : RING_LOADS;
 }
 
 // NT: 8-row batch tiles (1 or 2). RT: 16-row weight tiles per block; with SWIGLU the
@@ -58,7 +58,7 @@ __host__ __device__ constexpr int ring_loads() {
 // ring-full of copies is issued before anything else (before the wait on the
 // previous kernel), so the memory system is busy from the
 // block's first instruction.
-template <int WARPS, int NT, int RT, int SWIGLU, typename TOut, bool DEEP = false, int KSPLIT = 1, int RING = 0>
+template <int WARPS, int NT, int RT, int SWIGLU, typename TOut, int KSPLIT = 1, int RING = 0>
 __global__ void __launch_bounds__(WARPS * 32)
 skinny_kernel(TOut* __restrict__ out, const bf16* __restrict__ x, const bf16* __restrict__ W,
               int M, int N, int K, float limit) {
@@ -66,7 +66,7 @@ skinny_kernel(TOut* __restrict__ out, const bf16* __restrict__ x, const bf16* __
   KRK_TRACE_DECL
   constexpr int THREADS = WARPS * 32;
   constexpr int TILES = SWIGLU ? 2 * RT : RT;  // 16-row weight tiles this block streams
-  constexpr int STAGES = ring_loads<NT, DEEP, KSPLIT, RING>() / TILES;
+  constexpr int STAGES = ring_loads<NT, KSPLIT, RING>() / TILES;
   constexpr int SLOTS = TILES * 2 + NT;          // 16-byte pieces per thread and stage: weights, and the batch rows
   constexpr size_t RING_BYTES = (size_t)STAGES * SLOTS * THREADS * 16;
   uint4* ring = reinterpret_cast<uint4*>(smem_raw);                                 // [STAGES][SLOTS][THREADS]
@@ -250,17 +250,17 @@ skinny_kernel(TOut* __restrict__ out, const bf16* __restrict__ x, const bf16* __
   KRK_TRACE_END(K)
 }
 
-template <int WARPS, int NT, int RT, int SWIGLU, typename TOut, bool DEEP = false, int KSPLIT = 1, int RING = 0>
+template <int WARPS, int NT, int RT, int SWIGLU, typename TOut, int KSPLIT = 1, int RING = 0>
 int launch_warps(void* out, const void* x, const void* W, int M, int N, int K, float limit,
            cudaStream_t stream) {
   constexpr int THREADS = WARPS * 32;
   constexpr int TILES = SWIGLU ? 2 * RT : RT;
-  constexpr int STAGES = ring_loads<NT, DEEP, KSPLIT, RING>() / TILES;
+  constexpr int STAGES = ring_loads<NT, KSPLIT, RING>() / TILES;
   constexpr int SLOTS = TILES * 2 + NT;
   size_t smem = (size_t)STAGES * SLOTS * THREADS * 16 + (size_t)WARPS * TILES * NT * 4 * 32 * sizeof(float) +
                 (size_t)(KSPLIT - 1) * RT * 16 * NT * 8 * sizeof(float);
   if (smem > 220 * 1024) return -2;
-  auto kern = skinny_kernel<WARPS, NT, RT, SWIGLU, TOut, DEEP, KSPLIT, RING>;
+  auto kern = skinny_kernel<WARPS, NT, RT, SWIGLU, TOut, KSPLIT, RING>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
@@ -302,7 +302,7 @@ int launch(void* out, const void* x, const void* W, int M, int N, int K, float l
   // eight loads against eleven at eight rows, six against eight at sixteen, each within 0.3 %).
   if constexpr (!SWIGLU && RT == 1) {
     if (blocks > 2 * 148 && blocks <= 3 * 148)
-      return launch_warps<4, NT, RT, SWIGLU, TOut, false, 1, (NT == 1 ? 11 : 8)>(out, x, W, M, N, K, limit, stream);
+      return launch_warps<4, NT, RT, SWIGLU, TOut, 1, (NT == 1 ? 11 : 8)>(out, x, W, M, N, K, limit, stream);
   }
   if (blocks > 2 * 148 && blocks <= 5 * 148)
     return launch_warps<4, NT, RT, SWIGLU, TOut>(out, x, W, M, N, K, limit, stream);
@@ -310,7 +310,7 @@ int launch(void* out, const void* x, const void* W, int M, int N, int K, float l
   // have their bytes in flight instead of one large one
   if constexpr (!SWIGLU && RT == 1) {
     if (blocks * 4 <= 5 * 148 && K >= 4 * 4 * CHUNK * 4)
-      return launch_warps<4, NT, RT, SWIGLU, TOut, false, 4>(out, x, W, M, N, K, limit, stream);
+      return launch_warps<4, NT, RT, SWIGLU, TOut, 4>(out, x, W, M, N, K, limit, stream);
   }
   // (a ring twice as deep for kernels of about one block per SM was measured: slower, because the
   // next kernel's blocks then no longer fit beside it to prefetch their weights)
@@ -334,7 +334,7 @@ int pick_rt(void* out, const void* x, const void* W, int M, int N, int K, float 
     // 3.7, 3.2 / 4.5, 3.9 / 5.0). (Two ways, for 6,144 outputs, gained alone, 7.2 -> 6.7 at 8 rows of 2,560, and lost in a step, 51.6 ->
     // 52.4 a layer.)
     if (tiles > 2 * 148 && pairs * 3 <= 500 && K >= 4608)
-      return launch_warps<4, NT, 2, SWIGLU, TOut, false, 3, (NT == 1 ? 8 : 6)>(out, x, W, M, N, K, limit, stream);
+      return launch_warps<4, NT, 2, SWIGLU, TOut, 3, (NT == 1 ? 8 : 6)>(out, x, W, M, N, K, limit, stream);
   }
   return launch<NT, 1, SWIGLU, TOut>(out, x, W, M, N, K, limit, stream);
 }

@@ -30,10 +30,6 @@ class Normed:
         self._rows = None
 
     @property
-    def done(self) -> bool:
-        return self._rows is not None
-
-    @property
     def shape(self):
         return self.x.shape
 
@@ -45,8 +41,8 @@ class Normed:
                 self._rows = self.ops.add_rmsnorm(self.x, self.branch, self.gain, self.eps, self.x_new)
         return self._rows
 
-    def mark_fused(self, rows=True) -> None:
-        """Called by whoever did the add and the norm itself."""
+    def mark_fused(self, rows) -> None:
+        """Called by a norm that does the add and the norm itself, here and now."""
         self._rows = rows
 
 

@@ -136,7 +136,8 @@ def test_float32_products_of_several_threads(ops):
 
     def work(i, m):
         out = outs[i] = torch.zeros((m, 64), device="cuda")
-        args = (out.data_ptr(), xs[m].data_ptr(), w.data_ptr(), m, 64, 2560, 2560, 2560, 64, 0, 0, torch.cuda.current_stream().cuda_stream)
+        args = (out.data_ptr(), xs[m].data_ptr(), w.data_ptr(), m, 64, 2560, 2560, 2560, 64, 0, 0, ops.error.data_ptr(),
+                torch.cuda.current_stream().cuda_stream)
         codes = {ops.core.krk_gemm_nt(*args) for _ in range(4000)}
         if codes != {0}:
             failed.append((m, codes))
@@ -258,7 +259,7 @@ def test_tcgen05_gemm_with_swiglu_epilogue(ops, mik):
 @pytest.mark.parametrize("rows", [1, 3, 8, 13, 16])
 @pytest.mark.parametrize("nk", [(96, 64), (160, 2560), (301, 96), (2560, 9728)])
 def test_fused_norm_linear_bfloat16(ops, rows, nk):
-    """The decode-time product with the residual add and the norm in its prologue."""
+    """A norm with a pending branch, computed when the decode-time product of its rows asks for them: the sum written once, to both sides' bits."""
     from kernel_rush_kawk_b200.parts.norm import Normed
 
     n, k = nk
