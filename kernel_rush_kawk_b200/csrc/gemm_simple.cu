@@ -353,14 +353,17 @@ int launch_few(float* C, const float* A, const float* W, int M, int N, int K, in
   constexpr size_t per_row = (SLICE + 4) * sizeof(float);
   const size_t stage = (16 * CPT + M) * per_row;  // 17 to 50 KB
   const int blocks = (N + 16 * CPT - 1) / (16 * CPT);
-  // Two slices of the ring leave an SM more blocks than three, three cover more of a slice's way. What decides is how many blocks
-  // the SMs take in full rounds (three rows of K 2,560, two slices and three: N of 2,560 17.8 and 16.4 us, 6,144 20.3 and 19.0,
-  // 8,192 22.6 and 29.3, 12,288 (K 4,096) 51.6 and 44.3, 19,456 43.0 and 44.0, 151,936 239 and 256).
+  // Two slices of the ring leave an SM more blocks than three, three cover more of a slice's way. Where a thread has one output, what
+  // decides is how many blocks the SMs take in full rounds (three rows of K 2,560, two slices and three: N of 2,560 17.8 and 16.4 us, 6,144
+  // 20.3 and 19.0, 8,192 22.6 and 29.3, 12,288 (K 4,096) 51.6 and 44.3, 19,456 43.0 and 44.0, 151,936 239 and 256). Two rows by two columns are
+  // bound by the multiplying warps' own reads, which only other blocks cover: two slices at every size measured, where three were within 2 %
+  // or worse (K 2,560, two and three: five rows in slices of 128, N of 151,936 277 and 365 us; sixteen rows in slices of 256, one
+  // block an SM with three, 19,456 79 and 108, 151,936 438 and 698; twelve of 9,728 48 and 61).
   auto rounds = [&](int depth) {
     const long long held = max(1LL, (long long)(227 * 1024 / (FEW_BARS + depth * stage + 1024)));
     return (blocks + 148 * held - 1) / (148 * held) * held;
   };
-  const int depth = rounds(3) < rounds(2) ? 3 : 2;
+  const int depth = RPT == 1 && rounds(3) < rounds(2) ? 3 : 2;
   // always the most that a call may need: another thread may be about to launch with more rows than this one
   cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<RPT, CPT, SLICE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)(FEW_BARS + FEW_MAX_DEPTH * (16 * CPT + 8 * RPT) * per_row));
