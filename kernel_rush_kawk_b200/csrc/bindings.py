@@ -1013,12 +1013,12 @@ class Kernels:
         Units of less than 64 KB, which cost more than their bytes, by how many an SM has: from 60 on 2.5: 256 of 256 x 2,048 1.6: 1 123 and 127, 2
         153 and 148; 512 of 128 x 1,024 1.6, of 256 x 1,024 2; 160 of 128 x 2,048 2.5; 256 of 128 x 1,024 2.5: 2 68 and 70, 3 87 and 78. From 28
         on 3.5: 128 of 128 x 1,024 2.5: 2 42 and 44, 4 54 and 48; 256 of 128 x 512 2.7; 64 of 256 x 2,048 3.8: 3 53 and 62, 4 65 and 62. From 14 on
-        4.5: 64 of 256 x 1,024 4: 3.5 39 and 41, 6 44 and 41; 96 of 256 x 512 3.7; 32 of 256 x 2,048 5. From 6 on 6: 64 of 512 x 512 6, of 128 x
-        512 4.8: 3.5 23 and 24, 7 27 and 24; 32 of 512 x 512 8.3; 40 of 256 x 1,024 10; 48 of 128 x 1,024 4.5. Fewer 12: 16 of 256 x 1,024 16."""
+        4.5: 64 of 256 x 1,024 4: 3.5 39 and 41, 6 44 and 41; 96 of 256 x 512 3.7; 32 of 256 x 2,048 5. From 6 on 7: 64 of 512 x 512 6, of 128 x
+        512 8: 5 23 and 24, 9 26 and 25; 32 of 512 x 512 13; 40 of 256 x 1,024 12; 48 of 128 x 1,024 6.5. Fewer 12: 16 of 256 x 1,024 16."""
         tiles = E * min(-(-F // (128 if gated else 256)), -(-C // 256))
         units, size = E * -(-(F + C) // 32), 2 * E * F * C * (3 if gated else 2)
         if size < 65536 * units:
-            return 5 * E // 2 if units >= 60 * 148 else 7 * E // 2 if units >= 28 * 148 else 9 * E // 2 if units >= 14 * 148 else 6 * E if units >= 6 * 148 else 12 * E
+            return 5 * E // 2 if units >= 60 * 148 else 7 * E // 2 if units >= 28 * 148 else 9 * E // 2 if units >= 14 * 148 else 7 * E if units >= 6 * 148 else 12 * E
         if tiles >= 444 or (tiles >= 296 and size < 80000 * units):
             again = F * C * (3 if gated else 2) // 16  # bytes of a pair's rows that the walk's units read: K F / 8 + F C / 16 (no gate: K F / 16)
             return min((5 if units >= 128 * 148 else 9) * E // 2, int(150e6) // again)

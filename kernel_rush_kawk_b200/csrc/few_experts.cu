@@ -11,9 +11,10 @@
 // instruction, four the next, and neither side passes through shared memory (each is read by one warp alone). The warps' sums meet
 // in shared memory, in the order of the warps. An expert chosen by more than 16 rows goes over its weights again, from L2.
 //
-// A unit is short: 2,048 elements of a row are eight pieces a warp, and a block of one unit spent much of its life with nothing on the
+// A unit is short: 2,048 elements of a row are eight pieces a warp, and a block of one unit spends much of its life with nothing on the
 // way, before its first weights and behind its last. So two blocks an SM share all units out, each a run of neighbours, and a warp asks
-// for a piece of the next unit as soon as it has multiplied one of this.
+// for a piece of the next unit as soon as it has multiplied one of this. Where all units start at once, or nearly, a block of
+// one is left (few_experts_unit_kernel), which needs no tables of the other experts' pairs.
 //
 // 64 experts of 2,048 x 1,408 of which a row takes 6, the gated and the down product (a block a unit / this, us): one row 25.3 / 23.5, 2
 // rows 44.0 / 38.7, 8 rows 114 / 102 (588 MB at 5.75 TB/s), 16 rows 156 / 143, 64 rows 207 / 191; 128 of 1,024 x 512, 8 a row: one row
@@ -220,19 +221,58 @@ __device__ __forceinline__ Tables tables(const FewArgs& a, int* at0, int* warp_s
   return t;
 }
 
-// `steps` units from (pass, tile) on, a unit being a pass over one tile of columns. A warp's pieces of k follow one another over the
-// units' ends: a piece's registers are asked to be filled again as soon as it has been multiplied.
+// The passes of one expert alone, `e`: each warp looks through a run of the pairs. `first`: the pair without which they are none.
+__device__ __forceinline__ Tables tables_of(const FewArgs& a, int e, int early, int first, int* at0, int* counts) {
+  Tables t;
+  const int most = (a.pairs + ROWS - 1) / ROWS;
+  t.list = at0;
+  t.pass_expert = t.list + a.pairs;
+  t.pass_first = t.pass_expert + most;
+  t.pass_rows = t.pass_first + most;
+  t.passes = 0;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int run = ((a.pairs + WARPS - 1) / WARPS + 31) / 32 * 32, lo = warp * run, hi = min(a.pairs, lo + run);
+  auto found = [&](int i) { return __ballot_sync(0xffffffffu, (i == lo ? early : i + lane < hi ? a.experts[i + lane] : -1) == e); };
+  int mine = 0;
+  for (int i = lo; i < hi; i += 32) mine += __popc(found(i));
+  if (lane == 0) counts[warp] = mine;
+  __syncthreads();
+  int m = 0, at = 0;
+#pragma unroll
+  for (int v = 0; v < WARPS; ++v) {
+    if (v == warp) at = m;
+    m += counts[v];
+  }
+  if (m == 0) return t;
+  for (int i = lo; i < hi; i += 32) {
+    const unsigned all = found(i);
+    if (all >> lane & 1u) t.list[at + __popc(all & ((1u << lane) - 1u))] = i + lane;
+    at += __popc(all);
+  }
+  const int passes = (m + ROWS - 1) / ROWS;
+  if (tid < passes) {  // up to 256
+    t.pass_expert[tid] = e;
+    t.pass_first[tid] = tid * ROWS;
+    t.pass_rows[tid] = min(ROWS, m - tid * ROWS);
+  }
+  __syncthreads();
+  if (first < 0 || t.list[0] == first) t.passes = passes;
+  return t;
+}
+
+// `steps` units from (pass, tile) on, a unit being a pass over one of `tiles` tiles of columns from f_base on. A warp's pieces of k follow
+// one another over the units' ends: a piece's registers are asked to be filled again as soon as it has been multiplied.
 template <Form FORM, int NT>
-__device__ __forceinline__ void walk(const FewArgs& a, const Tables& t, float (*sums)[2][ROWS][17], int pass, int tile, int steps) {
+__device__ __forceinline__ void walk(const FewArgs& a, const Tables& t, float (*sums)[2][ROWS][17], int pass, int tile, int steps, int tiles,
+                                     int f_base) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
   const int F = a.F, K = a.K;
   constexpr int COLS = FORM == GATED ? 16 : 32;
-  const int tiles = (F + COLS - 1) / COLS;
 
   const bf16 *w[4], *x[NT];
   auto aim = [&](int pass, int tile) {
     const bf16* we = a.w + (size_t)t.pass_expert[pass] * (FORM == GATED ? 2 : 1) * F * K;
-    const int f0 = tile * COLS, first = t.pass_first[pass], rows = t.pass_rows[pass];
+    const int f0 = f_base + tile * COLS, first = t.pass_first[pass], rows = t.pass_rows[pass];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int f = f0 + g + 8 * (i & 1) + (FORM == GATED ? 0 : 16 * (i >> 1));
@@ -293,7 +333,7 @@ __device__ __forceinline__ void walk(const FewArgs& a, const Tables& t, float (*
 #pragma unroll
         for (int c = 0; c < 4; ++c) sums[warp][i][8 * n + 2 * t4 + (c & 1)][g + 8 * (c >> 1)] = acc[i][n][c];
     __syncthreads();
-    const int r = tid >> 4, f = tid & 15, f0 = tile * COLS;
+    const int r = tid >> 4, f = tid & 15, f0 = f_base + tile * COLS;
     if (r < t.pass_rows[pass]) {
       const int pair = t.list[t.pass_first[pass] + r];
       float s[2] = {0.f, 0.f};
@@ -328,6 +368,28 @@ __device__ __forceinline__ void walk(const FewArgs& a, const Tables& t, float (*
   }
 }
 
+// A block a tile of one expert's columns: blockIdx.y is the expert, or a pair, whose block works if no pair before it has its expert.
+template <Form FORM>
+__global__ void __launch_bounds__(THREADS, 2) few_experts_unit_kernel(FewArgs a) {
+  extern __shared__ int tables_s[];
+  __shared__ float sums[WARPS][2][ROWS][17];
+  __shared__ int counts[WARPS];
+  grid_launch_dependents();
+  grid_dependency_wait();
+  // the first choices of a warp's run are asked for together with the expert's number: a block's time before its first weights is a
+  // sixth of its life
+  const bool by_expert = a.pairs > a.E;
+  const int lane = threadIdx.x & 31, run = ((a.pairs + WARPS - 1) / WARPS + 31) / 32 * 32, i = (threadIdx.x >> 5) * run + lane;
+  const int early = i < a.pairs ? a.experts[i] : -1;
+  const int e = by_expert ? (int)blockIdx.y : a.experts[blockIdx.y];
+  if ((unsigned)e >= (unsigned)a.E) return;
+  const Tables t = tables_of(a, e, early, by_expert ? -1 : (int)blockIdx.y, tables_s, counts);
+  if (t.passes == 0) return;
+  const int f_base = blockIdx.x * (FORM == GATED ? 16 : 32);
+  if (t.pass_rows[0] > 8) walk<FORM, 2>(a, t, sums, 0, 0, t.passes, 1, f_base);
+  else walk<FORM, 1>(a, t, sums, 0, 0, t.passes, 1, f_base);
+}
+
 template <Form FORM>
 __global__ void __launch_bounds__(THREADS, 2) few_experts_kernel(FewArgs a) {
   extern __shared__ int tables_s[];
@@ -357,22 +419,31 @@ __global__ void __launch_bounds__(THREADS, 2) few_experts_kernel(FewArgs a) {
   const int tile0 = (int)(u0 - (long long)p0 * tiles);
   bool many = false;
   for (int p = p0; p <= p1; ++p) many |= t.pass_rows[p] > 8;
-  if (many) walk<FORM, 2>(a, t, sums, p0, tile0, (int)(u1 - u0));
-  else walk<FORM, 1>(a, t, sums, p0, tile0, (int)(u1 - u0));
+  if (many) walk<FORM, 2>(a, t, sums, p0, tile0, (int)(u1 - u0), tiles, 0);
+  else walk<FORM, 1>(a, t, sums, p0, tile0, (int)(u1 - u0), tiles, 0);
 }
 
 template <Form FORM>
 int launch(const FewArgs& a, cudaStream_t stream) {
-  const size_t bytes = Tables::bytes(a.pairs, a.E);  // 160 KB at 4,096 pairs of 65,535 experts
+  const int tiles = (a.F + (FORM == GATED ? 16 : 32) - 1) / (FORM == GATED ? 16 : 32);
+  const int groups = a.pairs > a.E ? a.E : a.pairs;  // experts that may be chosen
+  // A block a tile of an expert where that is no more blocks than start at once, and, beyond 32 pairs, where a walking block's tables of
+  // all pairs cost 2 us, up to 768: walk / tile, us, the gated and the down product of 8 experts of 128 x 256 3.4 / 2.8 and 3.1 / 2.5 at
+  // 32 pairs, 5.5 / 3.4 and 5.2 / 3.2 at 64; 16 of 256 x 1,024 (256 and 512 blocks) 4.8 / 4.2 and 5.0 / 4.8, 7.1 / 4.9 and 7.5 / 5.1; 128
+  // of 128 x 512 at 48 pairs (384 and 768) 7.4 / 5.8 and 8.0 / 6.7; 16 of 1,536 x 1,536 at 64, the down product (768) 14.1 / 12.4. Beyond:
+  // 12 pairs in 384 blocks of K 1,024 5.1 / 5.4; 64 of 256 x 1,024 at 64 (1,024) 11.8 / 11.8, 16 of 1,024 x 1,024 (1,024) 18.4 / 18.9.
+  const long long blocks = (long long)groups * tiles;
+  const bool unit = blocks <= 2 * 148 || (a.pairs > 32 && blocks <= 768);
+  // the list alone and 16 bytes a pass, 20 KB at most; or 160 KB at 4,096 pairs of 65,535 experts
+  const size_t bytes = unit ? ((size_t)a.pairs + 3 * ((a.pairs + ROWS - 1) / ROWS)) * 4 : Tables::bytes(a.pairs, a.E);
   if (bytes > 24 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(few_experts_kernel<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)Tables::bytes(4096, 65535));  // one value, whichever thread sets it
     if (e != cudaSuccess) return (int)e;
   }
-  const int tiles = (a.F + (FORM == GATED ? 16 : 32) - 1) / (FORM == GATED ? 16 : 32);
   const long long most = (long long)(a.pairs < a.E ? a.pairs : a.E + a.pairs / ROWS) * tiles;  // units that there can be
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(most < 2 * 148 ? most : 2 * 148));
+  cfg.gridDim = unit ? dim3((unsigned)tiles, (unsigned)groups) : dim3((unsigned)(most < 2 * 148 ? most : 2 * 148));
   cfg.blockDim = dim3(THREADS);
   cfg.dynamicSmemBytes = bytes;
   cfg.stream = stream;
@@ -389,7 +460,7 @@ int launch(const FewArgs& a, cudaStream_t stream) {
   static const bool plain = getenv("KRK_NO_PDL") != nullptr;  // measurement switch: ordinary stream order
   cfg.attrs = attr;
   cfg.numAttrs = plain ? 1 : 2;
-  return (int)cudaLaunchKernelEx(&cfg, few_experts_kernel<FORM>, a);
+  return (int)cudaLaunchKernelEx(&cfg, unit ? few_experts_unit_kernel<FORM> : few_experts_kernel<FORM>, a);
 }
 
 }  // namespace

@@ -420,6 +420,26 @@ def test_units_of_few_experts_rows(rows, top, E, K, F):
     assert torch.equal(got, want.to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("rows,top,E,K,F", [(5, 2, 4, 264, 1000), (16, 2, 6, 1544, 500), (17, 2, 6, 776, 500), (40, 2, 6, 1544, 520), (300, 4, 10, 72, 1000), (9, 3, 3, 8, 1500)])
+@pytest.mark.parametrize("form", [0, 1, 2])
+def test_a_block_an_expert_and_blocks_that_walk_give_the_same_bits(rows, top, E, K, F, form):
+    """Few units take a block a tile of an expert, many take blocks that walk over a share of them: said to come from 60,000 experts, the
+    same choices are many. Experts in no pass, in one of up to eight rows, of sixteen and in several; up to 32 pairs and more."""
+    ops = runtime(torch.bfloat16).ops
+    g = torch.Generator("cuda").manual_seed(rows + K)
+    x = torch.randn((rows * top, K), generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn((E, (2 if form == 0 else 1) * F, K), generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    experts = torch.randint(-1, E, (rows, top), generator=g, device="cuda").to(torch.int32)
+    by = torch.rand((rows, top), generator=g, device="cuda") if form != 2 else None
+    got = []
+    for said in (E, 60000):
+        out = torch.full((rows * top, F), 7.0, dtype=torch.bfloat16, device="cuda")
+        assert ops.moe.krk_few_experts(out.data_ptr(), x.data_ptr(), K, w.data_ptr(), experts.data_ptr(), rows, top, said, F, K, form, 0,
+                                       None if by is None else by.data_ptr(), 0.0, 0.0, ops._stream()) == 0
+        got.append(out)
+    assert torch.equal(*got)
+
+
 @pytest.mark.parametrize("odd", ["first", "second", "choices"])
 def test_few_experts_rows_with_weights_off_a_16_byte_boundary_or_many_choices(odd):
     """What the product per expert does not take goes to the kernels that read an expert per pair: weights that start at an
