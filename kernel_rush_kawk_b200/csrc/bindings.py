@@ -982,11 +982,15 @@ class Kernels:
     @staticmethod
     def _few_experts(x, w_first, w_down, rows, top) -> bool:
         """Whether the experts' products of few rows run once per expert (csrc/few_experts.cu): type, sizes, the alignment of rows
-        and weights, choices that the sum by rows holds, and more than one pair (by pair and by expert, us: 16 experts of 1,536 x
-        3,072, two a row, 2 pairs 23 and 16, 4 pairs 36 and 26; 64 of 2,048 x 1,408, two a row, 2 pairs 17 and 13; 64 of 1,024 x 256 8.6 and
-        8.6; one pair of 16 of 1,024 x 1,024 8 and 9, of 64 of 2,048 x 1,408 14 and 11)."""
+        and weights, choices that the sum by rows holds, and pairs enough: six, or two of experts of 2 MB and more, whose bytes outweigh the
+        third launch (by pair and by expert, us, 2, 4 and 6 pairs: 16 experts of 1,536 x 3,072 26 and 18, 44 and 24, 61 and 30; of 384 x
+        1,024 (2.4 MB) 8.2 and 8.0, 9.7 and 8.2, 11.4 and 8.5; of 512 x 512 (1.6) 6.5 and 7.2, 7.3 and 7.5, 7.7 and 8.0; of 256 x 1,024 (1.6) 7.3
+        and 7.9, 8.2 and 8.0, 9.2 and 8.2; 8 of 128 x 256 4.9 and 6.7, 5.1 and 6.7, 5.5 and 6.8; one pair of 16 of 512 x 1,024 6.8 and 7.9, of 64 of
+        1,408 x 2,048 16 and 12)."""
+        pairs, size = rows * top, 2 * (w_first.shape[1] * w_first.shape[2] + w_down.shape[1] * w_down.shape[2])
         return (x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and w_down.shape[2] % 8 == 0 and x.stride(0) % 8 == 0
-                and (x.data_ptr() | w_first.data_ptr() | w_down.data_ptr()) % 16 == 0 and top <= 32 and 2 <= rows * top <= Kernels.FEW_EXPERTS_PAIRS)
+                and (x.data_ptr() | w_first.data_ptr() | w_down.data_ptr()) % 16 == 0 and top <= 32
+                and (6 if size < 2 << 20 else 2) <= pairs <= Kernels.FEW_EXPERTS_PAIRS)
 
     @staticmethod
     def _grouped_from(E, F, C, gated) -> int:

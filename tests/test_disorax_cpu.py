@@ -144,3 +144,16 @@ def test_where_the_grouped_launches_begin(E, F, C, below, above):
     from kernel_rush_kawk_b200.csrc.bindings import Kernels
 
     assert below * E < Kernels._grouped_from(E, F, C, True) <= above * E
+
+
+@pytest.mark.parametrize("F, C, pairs, by_expert", [
+    (3072, 1536, 1, False), (3072, 1536, 2, True), (1408, 2048, 2, True), (384, 1024, 2, True), (256, 1024, 2, False), (256, 1024, 4, False),
+    (256, 1024, 6, True), (512, 512, 4, False), (128, 256, 2, False), (128, 256, 6, True), (1408, 2048, 4096, True), (1408, 2048, 4098, False)])
+def test_where_the_products_by_expert_begin(F, C, pairs, by_expert):
+    """Pairs and sizes on the side of the line where either way was measured the faster one; small experts of a few pairs read each
+    pair's weights by itself."""
+    from kernel_rush_kawk_b200.csrc.bindings import Kernels
+
+    top = 2 if pairs % 2 == 0 else 1
+    empty = lambda *shape: torch.empty(shape, dtype=torch.bfloat16)
+    assert Kernels._few_experts(empty(pairs // top, C), empty(2, 2 * F, C), empty(2, C, F), pairs // top, top) == by_expert
