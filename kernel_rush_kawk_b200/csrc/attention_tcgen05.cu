@@ -355,15 +355,17 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
     const TileRange rng = t ? r1 : r0;
     const uint32_t tmem_s = tmem + t * 128 + lane_addr, tmem_o = tmem + TMEM_O + t * D + lane_addr;
-    const int R = pair_row + t * rows + r;
-    const bool valid = r < rows && R < n_rows;
-    const int tok = valid ? R / G : 0;
-    const int pos = valid ? start + tok : -1;  // -1: sees nothing
-    const int low = (valid && window > 0) ? max(0, pos - window + 1) : 0;
-    const int head = kh * G + (valid ? R % G : 0);
+    // a thread without a row (a tile of fewer than 128, or the sequence's last) is where the last row is, so that its warp's blocks are seen
+    // whole when its rows see them whole: its scores are anything, decide nothing and go nowhere
+    const int rows_here = min(rows, n_rows - pair_row - t * rows);
+    const int R = pair_row + t * rows + min(r, rows_here - 1);
+    const bool valid = r < rows_here;
+    const int pos = start + R / G;
+    const int low = window > 0 ? max(0, pos - window + 1) : 0;
     float m = -INFINITY, slope = 0.f;
     float2 l2 = make_float2(0.f, 0.f);
     if constexpr (WIDE) {
+      const int head = kh * G + R % G;
       if (ex.sink) {
         // a sink at minus infinity, or so low that it is in log2 units, is none: nothing is summed before the first key
         m = ex.sink[head] * LOG2E;
@@ -411,7 +413,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
           }
 #pragma unroll
           for (int i = 0; i < KEYS; i += 2) most = fmaxf(fmaxf(most, fabsf(__uint_as_float(s[i]))), fabsf(__uint_as_float(s[i + 1])));
-          if (__any_sync(0xffffffffu, most > ex.small)) {
+          if (__any_sync(0xffffffffu, valid && most > ex.small)) {
 #pragma unroll
             for (int i = 0; i < KEYS; i += 2) {
               float2 x = __fmul2_rn(two(i), scale2);
@@ -452,7 +454,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
           for (int q = 0; q < 4; ++q) mx4[q] = fmaxf(fmaxf(mx4[q], __uint_as_float(s[i + q])), __uint_as_float(s[i + 4 + q]));
       const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       const float m_new = fmaxf(m, SHAPED ? mx : mx * scale_size);
-      const bool outgrown = m != -INFINITY && m_new - m > RESCALE_STEP;
+      const bool outgrown = valid && m != -INFINITY && m_new - m > RESCALE_STEP;
       if (__any_sync(0xffffffffu, outgrown)) {
         // the warp moves its rows' reference maxima and scales its rows of O; the block's P.V has not been issued and the
         // one before it is complete (S of this block came after it), so nothing else touches these rows of O
@@ -515,6 +517,9 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
       unsigned char* stage = q_s + t * TILE_BYTES;
       if (fine) {
         tc_fence_after();
+        int row = R;
+        asm volatile("" : "+r"(row));  // its token and head are worked out again: they are not kept in registers through the walk
+        const int tok = row / G, head = kh * G + row % G;
         float inv = valid ? (WIDE ? ex.out_scale : 1.0f) / (l2.x + l2.y) : 0.f;
         if (WIDE && ex.gate_mode == 1 && valid)
           inv /= 1.0f + expf(-__bfloat162float(ex.gate[(size_t)(row0 + tok) * ex.gate_stride + head]));
