@@ -376,7 +376,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     const float scale_size = WIDE ? scale_log2 : fabsf(scale_log2);  // a negative scale's sign is in the scores already
     const float2 scale2 = make_float2(scale_size, scale_size);
     constexpr uint32_t unseen = 0xff800000u;  // minus infinity: a score whose weight is zero
-    bool ok = true;
+    bool ok = true, loud = false;  // a block of the warp had a capped score beyond the series' range: it is not looked for again
     for (int j = rng.lo; j <= rng.hi; ++j) {
       const int key0 = j * KEYS;
       // the row sees keys first..first + span of the block: (unsigned)(i - first) <= span; none of them: no i passes
@@ -405,15 +405,18 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
           s[i + 1] = __float_as_uint(x.y);
         };
         if constexpr (SHAPE == 2) {
-          float most = 0.f;
-          if (!whole) {  // by the scores that count alone: a row's bits do not depend on what lies in pages and rows that it does not see
+          if (!loud) {
+            float most = 0.f;
+            if (!whole) {  // by the scores that count alone: a row's bits do not depend on what lies in pages and rows that it does not see
 #pragma unroll
-            for (int i = 0; i < KEYS; ++i)
-              if ((unsigned)i - first > span) s[i] = 0u;
+              for (int i = 0; i < KEYS; ++i)
+                if ((unsigned)i - first > span) s[i] = 0u;
+            }
+#pragma unroll
+            for (int i = 0; i < KEYS; i += 2) most = fmaxf(fmaxf(most, fabsf(__uint_as_float(s[i]))), fabsf(__uint_as_float(s[i + 1])));
+            loud = __any_sync(0xffffffffu, valid && most > ex.small);
           }
-#pragma unroll
-          for (int i = 0; i < KEYS; i += 2) most = fmaxf(fmaxf(most, fabsf(__uint_as_float(s[i]))), fabsf(__uint_as_float(s[i + 1])));
-          if (__any_sync(0xffffffffu, valid && most > ex.small)) {
+          if (loud) {
 #pragma unroll
             for (int i = 0; i < KEYS; i += 2) {
               float2 x = __fmul2_rn(two(i), scale2);
