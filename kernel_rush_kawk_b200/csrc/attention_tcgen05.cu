@@ -614,11 +614,14 @@ int launch_tcgen05(bf16* out, const bf16* q, int q_stride, int HQ, int HKV, cons
                    int n_pages, int n_seqs, int max_q_len, int total_rows, float scale, int window, int* error, const Extras& ex,
                    cudaStream_t stream) {
   const int G = HQ / HKV;
-  // The query tiles come and go by TMA where whole tokens (G rows each) fill at least three quarters of a tile; a tile then has
-  // that many rows. Fetched by the threads, the two tiles take 8 us at G of 5 where TMA takes 2 (of 30 for a block with twelve
-  // blocks of keys), so the rows left empty (3 of 128 at G of 5) cost less.
+  // The query tiles come and go by TMA where whole tokens (G rows each) fill most of a tile; a tile then has that many rows.
+  // Fetched by the threads, the two tiles take 8 us at G of 5 where TMA takes 2 (of 30 for a block with twelve blocks of keys), so the
+  // rows left empty cost less down to 112 of 128, and down to 96 where the shorter tiles make no more rounds of one block an SM. One
+  // prompt of 2,048, one kv head of 128, threads / TMA: G of 5 (125 rows, 8 kv heads) 80 / 61 us, 25 (125) 45 / 41, 28 (112) 50 / 45, 22 (110) 45 /
+  // 41, 26 (104) 47 / 45; three rounds for two: 37 (111) 61 / 63, 33 (99) 57 / 63 (heads of 64: 47 / 57), but 700 tokens, one round, 26 / 21.
   const int whole = G <= ROWS ? ROWS / G * G : 0;
-  const int q_by_tma = whole >= ROWS * 3 / 4 ? 1 : 0;
+  auto rounds = [&](int rows_a_tile) { return (((long long)max_q_len * G + 2 * rows_a_tile - 1) / (2 * rows_a_tile) * HKV * n_seqs + 147) / 148; };
+  const int q_by_tma = whole >= 112 || (whole >= 96 && rounds(whole) <= rounds(ROWS)) ? 1 : 0;
   const int tile_rows = q_by_tma ? whole : ROWS;
   const long long tiles = ((long long)max_q_len * G + 2 * tile_rows - 1) / (2 * tile_rows);
   if (tiles * HKV > 0x7fffffffLL || n_seqs > 65535) return -3;

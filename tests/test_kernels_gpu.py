@@ -684,6 +684,20 @@ def test_tcgen05_prefill_attention_of_a_negative_scale(ops, heads, kv_heads, D, 
     close(got, want, dtype, f"scale {scale} window {window}")
 
 
+@pytest.mark.parametrize("group,n", [(33, 1500), (33, 2048), (26, 2048), (37, 2048), (28, 300)])
+def test_tcgen05_prefill_attention_of_groups_that_leave_much_of_a_tile_empty(ops, group, n):
+    """Groups whose whole tokens fill 96 to 112 rows of a tile, on both sides of the line between query tiles by TMA and by threads
+    (by the rounds of blocks); one kv head."""
+    D, dtype = 64, torch.bfloat16
+    cache = make_cache(40, 1, D, 1, 34, dtype, 90)
+    batch = make_batch([0], [70], [n])
+    qkv = rand((n, (group + 2) * D), dtype, 91)
+    ops.qk_norm_rope_write(qkv, group, 1, D, None, None, 1e-6, None, None, batch, cache)
+    got = ops.attention(qkv, group, 1, D, batch, cache, 1.0 / 8.0, None)
+    ops.check()
+    close(got, TorchOps(dtype).attention(qkv, group, 1, D, batch, cache, 1.0 / 8.0, None), dtype, f"group {group} tokens {n}")
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("q_len", [1, 37])
 def test_one_far_key_among_hundreds_decides(ops, dtype, q_len):
