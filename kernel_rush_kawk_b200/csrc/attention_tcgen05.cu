@@ -20,7 +20,8 @@
 // tried; a path of its own for blocks that some row sees in part cost as much (the compiler moved the exponentials of both
 // paths in front of the branch), so scores that a row does not see become minus infinity first and there is one path.
 // 2,048 tokens, 32 heads in groups of four: 45 us (49 before); four prompts of 957 to 1,531, 40 heads in groups of five:
-// 120 (167, of which two thirds of the difference are the query tiles, which come by TMA at any group size now).
+// 105 (166 with query tiles of 128 rows fetched by the threads; 120 while the three rows that whole tokens leave empty counted as
+// rows that see nothing, so that their warp masked every block).
 // Per key block of 128 keys (two cache pages) and tile:
 //   S = Q K^T                                   [issuer]   -> s_full
 //   row max; p = exp2(S*c - m) rounded to bfloat16 -> tensor memory  [softmax]  -> p_ready
@@ -45,7 +46,7 @@
 // (c tanh(s / c) = c (1 - 2 / (1 + e^(2 s / c)))) and lose a slope times the distance of query and key before the softmax.
 // 2,048 tokens, a window of 1,024, 16 heads of 128 in groups of four: 37 us (45 with the softmax of both tiles in all eight
 // warps; the mma.sync kernel 116, of 37 at that instruction's measured rate, 550 TFLOP/s, for 19 GFLOP); 12 heads in groups of
-// three, no slopes, 39 (43; 75).
+// three, no slopes, 37 (43; 75).
 //
 // Compiled once per head size, for head sizes 64 and 128: -DKRK_HEAD_DIM=<D>.
 #include "tcgen05.cuh"
@@ -428,7 +429,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
             // tanh(u) = u + u z P(z), z = u^2, for |u| up to 0.65: the series' terms from u^3 on divided by u^3, fitted in Chebyshev
             // points over z; off by at most 9.4e-8 of tanh(u) in float32 (the form above by 1.7e-7 of 1). Scores that are small beside the
             // cap are the rule where queries and keys are normalised, and the exponentials' unit, which would do three things a score, does
-            // one: 2,048 tokens of 16 heads behind a cap of 30, 99 us and 86 here.
+            // one: 2,048 tokens of 16 heads behind a cap of 30, 94 us and 84 here.
             const float2 into = make_float2(ex.in_tanh, ex.in_tanh), cap2 = make_float2(ex.cap_log2, ex.cap_log2);
             constexpr float P[5] = {-0.333333284f, 0.133326009f, -0.0538258478f, 0.0208813194f, -0.00593298022f};
 #pragma unroll

@@ -16,9 +16,9 @@
 //   Packed multiply-adds (fma.rn.f32x2) were measured and are slower here (274 to 294 us): the copies that pair an
 //   operand with itself cost more than the pipe's register reads gain.
 // * gemm_f32_few: up to 16 float32 rows. Bound by the weights' bytes: each is read once, by bulk copies a slice or two ahead; a
-//   thread owns one or two output columns of one or two rows. One row of 151,936 x 2,560: 235 us, 6.6 TB/s; three rows 239,
-//   of 2,560 x 9,728 41 us, where the chain of K multiply-adds is the bound (20 us at four clocks each; copies of 16 bytes by
-//   all threads: 265 and 50; the general kernel: 1.9 ms and 570 us of 2,560 x 4,096).
+//   thread owns one or two output columns of one or two rows. One row of 151,936 x 2,560: 235 us, 6.6 TB/s; three rows 226,
+//   of 2,560 x 9,728 35 us, where the chain of K multiply-adds is the bound (20 us at four clocks each; copies of 16 bytes by
+//   all threads: 265 and 46; the general kernel: 1.9 ms and 570 us of 2,560 x 4,096).
 // * gemm_nt: everything else (bfloat16 inputs with float32 output at odd sizes, for output-head logits at many
 //   positions; float32 rows whose size or alignment does not allow 16-byte accesses). 64x64 output tile, k in slices of
 //   16, 256 threads with a 4x4 micro-tile each.
@@ -379,12 +379,12 @@ int launch_few(float* C, const float* A, const float* W, int M, int N, int K, in
 int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, int* error, cudaStream_t stream) {
   if (M == 0 || N == 0) return 0;
   if (K < 4 || K % 4 || lda % 4 || ldw % 4 || (((uintptr_t)A | (uintptr_t)W | (uintptr_t)C) & 15)) return -2;
-  // 16 rows: 84 us of 19,456 x 2,560 and 161 by the tiles below, 453 and 647 of 151,936 x 2,560, 2.5 and 4.0 of 128 x 64.
+  // 16 rows: 79 us of 19,456 x 2,560 and 161 by the tiles below, 438 and 647 of 151,936 x 2,560, 2.5 and 4.0 of 128 x 64.
   // One row of one column a thread reads most of shared memory for a multiply-add and has the most blocks; from five rows
   // on the reads bound it where there are columns enough (eight rows, two by two in slices of 128 and one by one: N of 19,456
-  // 50 and 63 us, 151,936 287 and 367; 8,192 38 and 31; five rows 49 and 53, 281 and 287; 12,288 63 and 55). Beyond eight rows two by
-  // two always: in slices of 128 to 12 rows of many columns (nine rows: N of 12,288 66 and 85, 151,936 327 and 420; 8,192 39 and 33;
-  // sixteen 441 and 453, but 94 and 84 of 19,456).
+  // 45 and 57 us, 151,936 283 and 366; 8,192 27 and 22; five rows 44 and 48, 277 and 284; 12,288 31 and 28). Beyond eight rows two by
+  // two always: in slices of 128 to 12 rows of many columns (nine rows: N of 12,288 32 and 41, 151,936 322 and 399; 8,192 28 and 22;
+  // sixteen 437 and 438, but 89 and 79 of 19,456).
   if (M <= 8 && (M < 5 || N < 16384)) return launch_few<1, 1, 256>(C, A, W, M, N, K, lda, ldw, ldc, error, stream);
   if (M <= 8 || (M <= 12 && N >= 12288)) return launch_few<2, 2, 128>(C, A, W, M, N, K, lda, ldw, ldc, error, stream);
   if (M <= 16) return launch_few<2, 2, 256>(C, A, W, M, N, K, lda, ldw, ldc, error, stream);

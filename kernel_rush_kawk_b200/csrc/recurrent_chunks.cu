@@ -25,8 +25,8 @@
 // its starting state in G's place and the sequence its final one; (3) per (sequence, chunk, head) the outputs with their norm,
 // weight and gate. Chunks of 32: a chunk of 64 needs twice the multiply-adds a token in pass 1 and halves the walk's steps.
 //
-// Measured: one prompt of 2,048 tokens, delta rule of 8 heads, 1,171 us token by token, 97 here (the passes 57, 22 and 17, each from a
-// cold cache); three prompts of 2,553 tokens in all, time mixing of 40 heads, 405 -> 117 us (48, 17 and 66; with float32 on the
+// Measured: one prompt of 2,048 tokens, delta rule of 8 heads, 1,171 us token by token, 101 here back to back (the passes 58, 33 and 17, each
+// alone and from a cold cache); three prompts of 2,553 tokens in all, time mixing of 40 heads, 405 -> 117 us (48, 17 and 66; with float32 on the
 // CUDA cores 175). Passes 1 and 3 are bound by instruction issue and latencies (a 0.4 to 0.5 share of the issue slots, 12 to 32 warps an
 // SM), the walk by the chain of its steps.
 //
@@ -646,8 +646,8 @@ __global__ void __launch_bounds__(THREADS, 8) mix_chunk_kernel(ChunkArgs a) {
 // each; a lane takes four rows against eight channels, and eight lanes hand their shares round until each has two numbers of
 // the new state: one barrier a chunk. A fifth warp asks for the chunks' M and columns of G five chunks ahead, as tiled copies, and waits
 // for them. Bound by the chain of a step: the state from shared memory, 32 multiply-adds of four columns, three exchanges, the
-// barrier. One prompt of 2,048 tokens, 8 heads: 36 us with 16-byte copies by the walkers (32 a step, which took half of it) and
-// two barriers, 22 here; M read before the state is there 3 us of that, a wait for a copy by the walkers themselves 5 more.
+// barrier. One prompt of 2,048 tokens, 8 heads, the three passes back to back: 111 us with 16-byte copies by the walkers (32 a step)
+// and two barriers, 101 here; the walk by itself 34.0 and 31.6 us, from a cold cache 35.6 and 33.1.
 constexpr int WALKERS = 128, WALK_THREADS = WALKERS + 32;
 constexpr int WALK_M = N * N, WALK_G = N * WALK_COLS;         // floats of a chunk's M and of its columns of G
 constexpr int WALK_SP = 36;                                   // floats from eight channels of the state to the next eight: other banks
