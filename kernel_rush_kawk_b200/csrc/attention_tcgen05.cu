@@ -210,9 +210,13 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     __syncwarp();
     if (lane == 0) {
       tmem_slot[1] = (uint32_t)(error_now >= 3);
-      load_k(0);
-      load_v(0);
-      if (n > 1) load_k(1);
+      if (error_now < 3) {
+        load_k(0);
+        load_v(0);
+        if (n > 1) load_k(1);
+      } else if (q_by_tma) {
+        mbar_wait(bars + Q_FULL, 0);  // nothing else is asked for, and the block, which has nothing to do, stays until the query tiles are here
+      }
     }
   } else if (warp == 10) {  // beside the loads of warp 8
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");

@@ -113,3 +113,40 @@ def test_a_block_that_gives_up_waits_for_the_copies_that_it_asked_for(folders, d
     with pytest.raises(KernelError, match="ran out"):
         ops.check()
     ops.check()
+
+
+@pytest.mark.parametrize("rows", [130, 700])
+def test_attention_blocks_that_find_a_give_up_code_leave_and_the_next_kernels_are_right(rows):
+    """Blocks of the prompt attention that find a code of an earlier kernel in the error word have asked for their query tiles already: they
+    wait for those, write nothing and leave, launch after launch, and what runs right behind them on the same SMs (products with
+    rings of copies and barriers of their own, then the same attention) gives its usual bits."""
+    from test_kernels_gpu import make_batch, make_cache, rand
+
+    from kernel_rush_kawk_b200.csrc import KernelError, load_kernels
+
+    ops = load_kernels((128,), "cuda:0")
+    heads, kv_heads, D = 32, 8, 128
+    cache = make_cache(24, kv_heads, D, 1, 20, torch.bfloat16, 90)
+    batch = make_batch([0], [300], [rows])
+    qkv = rand((rows, (heads + 2 * kv_heads) * D), torch.bfloat16, 91)
+    ops.qk_norm_rope_write(qkv, heads, kv_heads, D, None, None, 1e-6, None, None, batch, cache)
+    x, w = rand((8, 1024), torch.float32, 92), rand((4096, 1024), torch.float32, 93)
+    attend = lambda out: ops.attn[D].krk_attention_prefill_tcgen05(
+        out.data_ptr(), qkv.data_ptr(), qkv.stride(0), heads, kv_heads, batch.seq_slot.data_ptr(), batch.seq_start.data_ptr(),
+        batch.seq_qlen.data_ptr(), batch.cu_q.data_ptr(), cache.table.data_ptr(), cache.width, cache.k.data_ptr(), cache.v.data_ptr(),
+        cache.k.shape[0], 1, rows, rows, D ** -0.5, 0, ops.error.data_ptr(), ops._stream())
+    out = torch.zeros((rows, heads * D), dtype=torch.bfloat16, device="cuda")
+    assert attend(out) == 0
+    want = out.clone(), ops.linear(x, w)
+    ops.check()
+    for _ in range(20):
+        out.fill_(7.0)
+        ops.error.fill_(8)
+        assert attend(out) == 0
+        got = ops.linear(x, w)
+        assert torch.equal(out, torch.full_like(out, 7.0)) and torch.equal(got, want[1])
+        with pytest.raises(KernelError, match="barrier wait"):
+            ops.check()
+        assert attend(out) == 0
+        ops.check()
+        assert torch.equal(out, want[0])
